@@ -216,10 +216,11 @@ typedef struct insg_gemv_op {
     int tokens;                 /* 0 or 1: one token.  More: consecutive tokens of one sequence in one call (the weights are
                                    streamed once per pass): in, aux and x_out are [tokens][cols], every out is
                                    [tokens][rows]; the convolution history is advanced token by token.  layout 0: 2 or 4
-                                   tokens (one launch of the mma.sync kernel); layout 1: any count up to 4096, sixteen tokens
-                                   per tcgen05 instruction (needs umma_scratch).  Not with INSG_PRO_PREPARED, prepared
+                                   tokens (one launch of the mma.sync kernel); layout 1: any count up to 4096, up to eight
+                                   in one launch of the GEMV kernel, more through the GEMM kernel, sixteen tokens per
+                                   tcgen05 instruction (needs umma_scratch).  Not with INSG_PRO_PREPARED, prepared
                                    outputs or INSG_EPI_LOGITS. */
-    void *umma_scratch;         /* layout 1 with tokens > 1: device scratch of insg_umma_gemm_scratch_bytes(cols, tokens) for
+    void *umma_scratch;         /* layout 1 with tokens > 8: device scratch of insg_umma_gemm_scratch_bytes(cols, tokens) for
                                    the activations' digit image, rewritten by every call                                      */
     size_t umma_scratch_bytes;
 } insg_gemv_op;

@@ -33,13 +33,13 @@ struct DecodeOptions {
                                    // dependent-launch chain costs, and its phases cannot overlap one another's tails)
     bool use_graph = true;         // launch per operation: replay the token step from a CUDA graph
     bool use_pdl = true;           // programmatic dependent launch between kernels
-    bool gemv_tcgen05 = false;     // true: weights through tcgen05.mma kind::mxf4 (TMA-fed); false: the mma.sync streaming kernel
-    bool prepared_inputs = true;   // a GEMV that writes the residual stream or the SwiGLU output also leaves the next GEMV's
-                                   // input ready as fp16 pieces (and its sum of squares), so that one starts streaming
-                                   // without normalising or converting anything; false: every GEMV prepares its own input
-    bool prefill_tcgen05 = true;   // forward_tokens with 16 or more tokens: passes of up to 256 tokens through the tcgen05
-                                   // kernel (kind::mxf4, sixteen tokens per instruction; needs a second, tile-layout copy of
-                                   // the weights); false: always passes of four tokens through the mma.sync kernel
+    bool gemv_tcgen05 = false;     // true: the tcgen05 kernels whatever the two options below and `persistent` say
+    bool prepared_inputs = true;   // true: the matrix products run on tcgen05.mma kind::mxf4 (weights fed by bulk copies, one
+                                   // tile-layout copy for every pass size).  With `persistent` they stay on the mma.sync
+                                   // kernel, whose producers leave the next product's input ready as fp16 pieces.
+                                   // false: the mma.sync kernel, every product preparing its own input
+    bool prefill_tcgen05 = true;   // prompts: passes of up to 256 tokens through the tcgen05 GEMM (sixteen tokens per
+                                   // instruction); false: passes of eight (tcgen05) or four (mma.sync) tokens
     int n_layers = Qwen35Shape::layers;
     int vocab = Qwen35Shape::vocab;
 };

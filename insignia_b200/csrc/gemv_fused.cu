@@ -199,7 +199,7 @@ size_t insg_gemv_argmax_scratch_bytes(void) { return 64 + size_t(8) * 512; }
 
 int insg_gemv_fused(const insg_gemv_op *op, insg_stream_t stream)
 {
-    if (op && op->layout == 1) return op->tokens > 1 ? gemm_umma_launch(op, stream) : gemv_umma_launch(op, stream);
+    if (op && op->layout == 1) return op->tokens > 8 ? gemm_umma_launch(op, stream) : gemv_umma_launch(op, stream);
     return gemv_fused_launch(op, op && op->tokens > 1 ? op->tokens : 1, stream);
 }
 

@@ -1,6 +1,6 @@
-// Helpers shared by the tcgen05 kernels (umma_gemv.cu: one token, activation image resident in shared memory;
-// umma_gemm.cu: eight tokens per MMA, activation image streamed): shared-memory descriptors, mbarrier waits with a
-// bound, bulk copies, and the split of an fp32 activation into exact E2M1 digits.
+// Helpers shared by the tcgen05 kernels (umma_gemv.cu: one to eight tokens, activation image resident in shared memory;
+// umma_gemm.cu: more tokens, activation image streamed): shared-memory descriptors, mbarrier waits with a bound,
+// and bulk copies.
 #pragma once
 #include "common.cuh"
 
@@ -43,28 +43,26 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *b, uint32_t parity, volatile
     return false;
 }
 
+// A poll that never suspends the thread.
+__device__ __forceinline__ bool mbar_test(uint64_t *b, uint32_t parity)
+{
+    uint32_t done;
+    asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(done) : "r"(smem_u32(b)), "r"(parity) : "memory");
+    return done != 0;
+}
+// One lane of a converged warp (the same one every time).
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t e;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(e));
+    return e != 0;
+}
+
 __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
 {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
-
-// Twelve base-4 digits of |v| (24 bits) as E2M1 codes, one per nibble: digits 0..7 in lo, 8..11 in hi; sign in bit 3.
-__device__ __forceinline__ void digit_codes(float x, float alpha, uint32_t &lo, uint32_t &hi)
-{
-    const float sc = fabsf(x) * alpha;                      // < 2^24
-    const uint32_t v = min(__float2uint_rn(sc), 0xFFFFFFu);
-    const uint32_t sgn = (__float_as_uint(x) >> 31) * 0x88888888u;
-    uint32_t t = v & 0xFFFFu;                               // 16 bits -> eight 2-bit digits, one per nibble
-    t = (t | (t << 8)) & 0x00FF00FFu;
-    t = (t | (t << 4)) & 0x0F0F0F0Fu;
-    t = (t | (t << 2)) & 0x33333333u;
-    uint32_t u = v >> 16;                                   // 8 bits -> four digits
-    u = (u | (u << 4)) & 0x0F0F0F0Fu;
-    u = (u | (u << 2)) & 0x33333333u;
-    // digit d -> E2M1 code of the value d: 0,1,2,3 -> 0,2,4,5 = 2d - (d == 3)
-    lo = ((t << 1) - ((t >> 1) & t & 0x11111111u)) | sgn;
-    hi = ((u << 1) - ((u >> 1) & u & 0x11111111u)) | (sgn & 0x0000FFFFu);
 }
 
 } // namespace insg

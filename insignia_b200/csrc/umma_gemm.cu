@@ -696,6 +696,8 @@ size_t umma_gemm_scratch(int cols, int tokens)
     return image_bytes(cols, tokens) + ((groups * tpg * sizeof(float) + 255) & ~size_t(255)) + kPartialBytes + kGMaxGrid * sizeof(int);
 }
 
+int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st); // 1..8 tokens (umma_gemv.cu)
+
 int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
 {
     if (!op || !op->in) return fail(INSG_E_ARG, "gemm: null operand");
@@ -834,7 +836,7 @@ int insg_mxfp4_gemm_umma(const void *packed_umma, const float *x, float *y, int 
     op.layout = 1;
     op.umma_scratch = scratch;
     op.umma_scratch_bytes = scratch_bytes;
-    return gemm_umma_launch(&op, stream);
+    return M <= 8 ? gemv_umma_launch(&op, stream) : gemm_umma_launch(&op, stream);
 }
 
 } // extern "C"

@@ -1,31 +1,31 @@
-// MXFP4 GEMV on the 5th-generation tensor cores (tcgen05, sm_100a), batch 1.
+// MXFP4 weights x one to eight tokens on the 5th-generation tensor cores (tcgen05, sm_100a): the decode-step matrix product.
 //
-// y[r] = sum_k e2m1(code(r,k)) * 2^(s(r,k/32)-127) * x[k]            (reference: src/mxfp4.cu:41-66)
+// y[m][r] = sum_k e2m1(code(r,k)) * 2^(s(r,k/32)-127) * x[m][k]                 (reference: src/mxfp4.cu:41-66)
 //
-// The checkpoint's weights ARE the A operand of tcgen05.mma kind::mxf4.block_scale: packed E2M1 with
-// one UE8M0 scale per 32 values along K.  Nothing is dequantised in registers: weights go
-// HBM -> shared memory with cp.async.bulk (TMA, mbarrier completion) and are read from there by the
-// tensor core, with their scale bytes copied shared -> tensor memory by tcgen05.cp.  The stream is HBM
-// bound (17 bytes per 32 weights) and the SM's instruction slots stay free.
+// What bounds it: the weight stream (17 bytes per 32 weights, each read once), and, because a token is a chain of some
+// 160 of these products, everything between two streams.  The kernel is built so that neither costs instruction slots:
+//   * weights go HBM -> shared memory by cp.async.bulk (17 KB per copy: 8.7 KB copies stream at 4.7 TB/s from one issuing
+//     thread, 17 KB ones at 6.3) and from there straight into tcgen05.mma.kind::mxf4.block_scale as the A operand, in
+//     their packed form; nothing is dequantised in registers;
+//   * the activation is the B operand.  kind::mxf4 wants E2M1 there too, so each fp32 value is written as a 25-bit signed
+//     fixed-point number relative to the largest of its 32-element group (the group's UE8M0 scale) in balanced base 9:
+//     eight digits -4..4, each exact in E2M1.  Column j of a token holds digit j; the epilogue adds 9^j D_j in fp32;
+//   * a cluster of four CTAs shares a 128-row tile, each multiplying a quarter of K: a CTA converts only a quarter of the
+//     activation, 4096 rows still occupy 128 SMs, and the four partial sums meet through distributed shared memory
+//     (st.async with mbarrier completion), added in rank order by the CTA that owns those 32 rows -- no ticket, no
+//     global-memory exchange, and the same bits whatever the timing;
+//   * a CTA keeps its ring within half an SM's shared memory, so the next launch of the chain (programmatic dependent
+//     launch) is resident and has its first ~100 KB of weights per SM on the way while this one finishes.
 //
-// The activation is the B operand, which for kind::mxf4 must be E2M1 as well.  It is written as a
-// 24-bit fixed-point number (relative to the largest element of the vector) cut into twelve base-4
-// digits: a digit 0..3 is exactly representable in E2M1, so column j of B holds digit j of every
-// element with the column's block scale set to 4^j, and y = sum_j D[:, j] / alpha is an exact
-// positional recombination in fp32.  (N = 16 columns are required by the M = 128 instruction shape;
-// the last four are zero.)
+// CTA roles (320 threads): warps 0-7 run the activation prologue (fused RMSNorm / gates, digits); then warps 0-3 read the
+// accumulators (tcgen05.ld, tensor-memory lane = row) and send the partial sums to the rows' owners, warps 4-7 add the
+// four parts and run the fused epilogue; warp 8 issues tcgen05.cp / tcgen05.mma, warp 9 the bulk copies.  Every wait is
+// bounded: on expiry a flag is raised in global memory and all roles drain.
 //
-// Layout of the weights for this kernel (insg_mxfp4_repack_umma), same 17 bytes per 32 weights: rows
-// in tiles of 128, K in blocks of 128; one (tile, block) record is 8704 contiguous bytes = the shared
-// memory image the MMA reads: 2 K-steps of 64 x [16 row groups][2 k cores][8 rows][16 bytes]
-// (canonical K-major, no swizzle: leading byte offset 128, stride byte offset 256), then the 512-byte
-// scale block [32 rows][4 row quarters][4 groups] that tcgen05.cp.32x128b.warpx4 expects.
-//
-// CTA roles (512 threads): every warp takes part in the activation prologue; then one thread issues
-// bulk copies into a ring of stages, one thread issues tcgen05.cp + tcgen05.mma and commits stage
-// releases, warps 0-3 read the accumulators (tcgen05.ld, TMEM lane = output row) and run the fused
-// epilogue.  Accumulators are double buffered so a tile's epilogue overlaps the next tile's MMAs.
-// Every wait is bounded: on expiry a flag is raised in global memory and all roles drain.
+// Layout of the weights (insg_mxfp4_repack_umma): rows in tiles of 128, K in blocks of 128; one (tile, block) record is 8704
+// contiguous bytes = the shared-memory image the MMA reads: 2 K-steps of 64 x [16 row groups][2 k cores][8 rows][16 bytes]
+// (canonical K-major, no swizzle: leading byte offset 128, stride byte offset 256), then the 512-byte scale block
+// [32 rows][4 row quarters][4 groups] that tcgen05.cp.32x128b.warpx4 expects.
 #include "gemv_prologue.cuh"
 #include "umma_common.cuh"
 #include "host_util.h"
@@ -35,26 +35,34 @@
 
 namespace insg {
 
-constexpr int kUThreads = kProThreads;
-constexpr int kBImgPerKb = 1024;     // activation digits: 16 columns x 128 k x 4 bit
-constexpr int kAccMax = 8;           // independent accumulators per tile: consecutive MMAs must not wait on each other's result
-constexpr int kSfaBufs = 8;          // scale-factor column sets cycled by k-block
-constexpr int kTmemCols = 512;       // D set 0 [0,128) D set 1 [128,256) SFA [256,288) SFB [288,292)
+constexpr int kDCl = 4;                    // CTAs per cluster = parts K is cut into = 32-row blocks of a tile
+constexpr int kDThreads = 320;
+constexpr int kDStage = 2 * kURec;         // one ring stage: two consecutive k-blocks of a tile
+constexpr int kDMaxStages = 8;
+constexpr int kDMaxKb = 24;                // k-blocks per CTA: 12288 / 128 / 4
+constexpr int kDDigits = 8;                // digits per activation = N columns per token
+constexpr uint32_t kDSfaCol = 128, kDSfbCol = 160, kDTmemCols = 256; // accumulators [0,128), weight scales [128,160), digit scales [160,256)
+// A CTA takes at most this much dynamic shared memory unless its operands need more: two of them (this launch and the next)
+// then fit an SM's 228 KB with their static part and the 1 KB the hardware keeps per CTA.
+constexpr int kDHalfSm = 112 * 1024;
 
-struct USeg {
+struct DSeg {
     const uint8_t *packed, *packed2;
     float *out;
     float *conv_state;
     const uint16_t *conv_w;
     const float *A_log;
     const uint16_t *dt_bias;
-    int tile_begin, ntiles, nmat, epilogue, rows;
+    long long conv_stride; // 0: the tokens are one sequence (history carried through them in order), else token m's history at + m * stride
+    int tile_begin, epilogue, rows;
 };
 
-struct UParams {
-    ProIn pro;
-    int nkb, nseg, total_tiles, stages, nacc, prefetch;
-    USeg seg[4];
+struct DParams {
+    const float *in, *aux;
+    const uint16_t *norm_w;
+    float *x_out;
+    int cols, nkb, prologue, nseg, units, nmat, tokens, stages;
+    DSeg seg[4];
     float2 *argmax_partial;
     unsigned *argmax_ticket;
     int *token_out, *token_feedback, *token_log, *position_inout;
@@ -62,296 +70,613 @@ struct UParams {
     int token_log_capacity;
 };
 
-// kblock i of this CTA's sequence -> global address of its record and its place in the tile sequence
-struct URun {
-    const uint8_t *rec;
-    int run;  // index of the (tile, matrix) run inside this CTA
-    int kb;
-};
+// ---- cluster helpers -----------------------------------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t saddr, uint32_t rank)
+{
+    uint32_t d;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(saddr), "r"(rank));
+    return d;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ void remote_arrive(uint32_t bar)
+{
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// T floats to another CTA's shared memory; their bytes complete on that CTA's barrier.
+template <int T> __device__ __forceinline__ void send_floats(uint32_t dst, const float (&v)[T], uint32_t bar)
+{
+    if constexpr (T == 1) {
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(dst), "f"(v[0]), "r"(bar) : "memory");
+    } else if constexpr (T == 2) {
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(dst), "f"(v[0]), "f"(v[1]), "r"(bar) : "memory");
+    } else {
+#pragma unroll
+        for (int t = 0; t < T; t += 4)
+            asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
+                         ::"r"(dst + 4 * t), "f"(v[t]), "f"(v[t + 1]), "f"(v[t + 2]), "f"(v[t + 3]), "r"(bar) : "memory");
+    }
+}
+// A wait on data other CTAs of the cluster send (acquire at cluster scope).
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *b, uint32_t parity, volatile int *abort_flag)
+{
+    for (uint32_t it = 0; it < kSpinLimit; it++) {
+        uint32_t done;
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(done) : "r"(smem_u32(b)), "r"(parity) : "memory");
+        if (done) return true;
+        if ((it & 1023u) == 1023u && *abort_flag) return false;
+    }
+    *abort_flag = 1;
+    return false;
+}
 
-__device__ __forceinline__ int useg_of(const UParams &p, int tile)
+// Eight balanced base-9 digits of round(x * alpha) (|.| < 2^24) as E2M1 codes, digit j in nibble j.  u = v + 4 * (9^8 - 1) / 8
+// has plain base-9 digits 0..8 (the balanced digit + 4); they are taken in pairs (base 81) through an 81-byte table, which
+// costs a third of the instructions of eight divisions by 9.
+__device__ __forceinline__ uint32_t digit_codes81(float x, float alpha, const uint8_t *lut)
+{
+    const int v = max(-0xFFFFFF, min(__float2int_rn(x * alpha), 0xFFFFFF));
+    const uint32_t u = uint32_t(v + 21523360);
+    const uint32_t hi = u / 6561u, lo = u - 6561u * hi;
+    const uint32_t h1 = (hi * 6473u) >> 19, h0 = hi - 81u * h1; // n / 81 for n < 6562 (6473 / 2^19 = 1/81 + 1.7e-7)
+    const uint32_t l1 = (lo * 6473u) >> 19, l0 = lo - 81u * l1;
+    return uint32_t(lut[l0]) | (uint32_t(lut[l1]) << 8) | (uint32_t(lut[h0]) << 16) | (uint32_t(lut[h1]) << 24);
+}
+__device__ __forceinline__ uint8_t digit_pair_code(int n) // table entry: digits n % 9 - 4 (low nibble) and n / 9 - 4 (high nibble)
+{
+    uint32_t r = 0;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int d = (h ? n / 9 : n % 9) - 4, mag = d < 0 ? -d : d; // 0..4 -> E2M1 codes 0, 2, 4, 5, 6
+        r |= uint32_t((mag < 3 ? 2 * mag : mag + 2) | (d < 0 ? 8 : 0)) << (4 * h);
+    }
+    return uint8_t(r);
+}
+
+__device__ __forceinline__ int dseg_of(const DParams &p, int unit)
 {
     int s = 0;
 #pragma unroll
     for (int i = 1; i < 4; i++)
-        if (i < p.nseg && tile >= p.seg[i].tile_begin) s = i;
+        if (i < p.nseg && unit >= p.seg[i].tile_begin) s = i;
     return s;
 }
 
-// Run r of CTA c: tile = c + (r / nmat) * G, matrix r % nmat (nmat is the same for all segments of a launch).
-__device__ __forceinline__ const uint8_t *run_base(const UParams &p, int tile, int mat)
+__device__ __forceinline__ void copy_scales(uint32_t taddr, uint64_t desc)
 {
-    const USeg &s = p.seg[useg_of(p, tile)];
-    return (mat ? s.packed2 : s.packed) + size_t(tile - s.tile_begin) * p.nkb * kURec;
+    asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(desc) : "memory");
+}
+__device__ __forceinline__ void mma_step(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, bool accumulate, uint32_t sa, uint32_t sb)
+{
+    asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %4, 0;\n"
+                 "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%5], [%6], q;\n}"
+                 ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"(uint32_t(accumulate)), "r"(sa), "r"(sb) : "memory");
+}
+__device__ __forceinline__ void commit_to(uint64_t *bar)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-__global__ void __launch_bounds__(kUThreads, 1) umma_gemv_kernel(const __grid_constant__ UParams p)
+// The digits of one 128-element k-block of one token (four elements per lane) into the B image, and their group scales.
+// Image of a k-block: [2 K-steps][T column groups][2 k cores][8 columns][16 B]; a token's eight digit columns are one group.
+template <int T>
+__device__ __forceinline__ void store_digits(float4 x, int m, uint8_t *bkb, uint8_t *sfkb, const uint8_t *lut, int lane)
+{
+    float mx = fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w)));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1)); // a group of 32 elements = 8 lanes
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+    int eb = int((__float_as_uint(mx) >> 23) & 0xffu);
+    eb = min(max(eb, 24), 230);
+    const float alpha = __uint_as_float(uint32_t(277 - eb) << 23); // largest element * alpha in [2^23, 2^24)
+    const uint32_t c0 = digit_codes81(x.x, alpha, lut), c1 = digit_codes81(x.y, alpha, lut);
+    const uint32_t c2 = digit_codes81(x.z, alpha, lut), c3 = digit_codes81(x.w, alpha, lut);
+    // columns 0, 2, 4, 6 sit in the low nibbles of the four bytes, 1, 3, 5, 7 in the high ones
+    const uint32_t e01 = (c0 & 0x0F0F0F0Fu) | ((c1 & 0x0F0F0F0Fu) << 4), e23 = (c2 & 0x0F0F0F0Fu) | ((c3 & 0x0F0F0F0Fu) << 4);
+    const uint32_t o01 = ((c0 >> 4) & 0x0F0F0F0Fu) | (c1 & 0xF0F0F0F0u), o23 = ((c2 >> 4) & 0x0F0F0F0Fu) | (c3 & 0xF0F0F0F0u);
+    uint8_t *base = bkb + (lane >> 4) * (256 * T) + m * 256 + ((lane >> 3) & 1) * 128 + (lane & 7) * 2;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        *reinterpret_cast<uint16_t *>(base + (2 * j) * 16) = uint16_t(((e01 >> (8 * j)) & 0xffu) | (((e23 >> (8 * j)) & 0xffu) << 8));
+        *reinterpret_cast<uint16_t *>(base + (2 * j + 1) * 16) = uint16_t(((o01 >> (8 * j)) & 0xffu) | (((o23 >> (8 * j)) & 0xffu) << 8));
+    }
+    const int n = 8 * m + (lane & 7); // scale block: row = column n of B (32 rows, then the next quarter), byte = group
+    sfkb[(n & 31) * 16 + (n >> 5) * 4 + (lane >> 3)] = uint8_t(eb - 23);
+}
+
+// One accumulator: the eight digit columns of each token, digits combined (least significant first; 9^j is exact in fp32).
+template <int T> __device__ __forceinline__ void load_partial(uint32_t taddr, float (&y)[T])
+{
+    uint32_t d[8 * T];
+    if constexpr (T == 1) {
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]) : "r"(taddr));
+    } else {
+#pragma unroll
+        for (int h = 0; h < T / 2; h++)
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                         : "=r"(d[16 * h]), "=r"(d[16 * h + 1]), "=r"(d[16 * h + 2]), "=r"(d[16 * h + 3]), "=r"(d[16 * h + 4]), "=r"(d[16 * h + 5]),
+                           "=r"(d[16 * h + 6]), "=r"(d[16 * h + 7]), "=r"(d[16 * h + 8]), "=r"(d[16 * h + 9]), "=r"(d[16 * h + 10]), "=r"(d[16 * h + 11]),
+                           "=r"(d[16 * h + 12]), "=r"(d[16 * h + 13]), "=r"(d[16 * h + 14]), "=r"(d[16 * h + 15])
+                         : "r"(taddr + 16 * h));
+    }
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int t = 0; t < T; t++) {
+        const uint32_t *q = d + 8 * t;
+        float ya = __uint_as_float(q[0]);
+        ya = fmaf(__uint_as_float(q[1]), 9.f, ya);
+        ya = fmaf(__uint_as_float(q[2]), 81.f, ya);
+        ya = fmaf(__uint_as_float(q[3]), 729.f, ya);
+        ya = fmaf(__uint_as_float(q[4]), 6561.f, ya);
+        ya = fmaf(__uint_as_float(q[5]), 59049.f, ya);
+        ya = fmaf(__uint_as_float(q[6]), 531441.f, ya);
+        ya = fmaf(__uint_as_float(q[7]), 4782969.f, ya);
+        y[t] = ya;
+    }
+}
+
+template <int T>
+__global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_constant__ DParams p)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nkb = p.nkb, S = p.stages;
-    uint8_t *ring = smem;                                   // S stages of kURec bytes
-    uint8_t *bimg = ring + size_t(S) * kURec;               // nkb x 1024 bytes of activation digits
-    uint8_t *sfb = bimg + size_t(nkb) * kBImgPerKb;         // 512 bytes
-    float *scratch = reinterpret_cast<float *>(sfb + 512);  // 64 floats
-    __shared__ __align__(8) uint64_t full[32], empty[32], dfull[2], dempty[2];
+    constexpr int kBKb = 512 * T;       // digit bytes per k-block
+    constexpr int N = kDDigits * T;
+    constexpr int kSlot = kDCl * 32 * T; // floats of one exchange slot: [source rank][32 rows][T]
+    __shared__ __align__(8) uint64_t full[kDMaxStages], empty[kDMaxStages], dfull[2], dempty[2], xfull[8], xempty[8], ssfull, image[kDMaxKb / 8];
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort, s_last;
+    __shared__ float s_ssq[T * kDMaxKb], s_rss[kDCl * T], s_best[4];
+    __shared__ int s_bidx[4];
+    __shared__ uint8_t s_lut[84];
 
-    pdl_launch_dependents();
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int rank = int(blockIdx.x) & (kDCl - 1), cl = int(blockIdx.x) / kDCl, C = int(gridDim.x) / kDCl;
+    const int nkb = p.nkb, S = p.stages, nmat = p.nmat;
+    const int kb0 = (nkb * rank) >> 2, len = ((nkb * (rank + 1)) >> 2) - kb0; // this CTA's k-blocks
+    const int spt = (len + 1) >> 1;                                            // ring stages per (tile, matrix)
+    const int nun = cl < p.units ? (p.units - cl + C - 1) / C : 0;             // units of this cluster: cl, cl + C, ...
+    const int nruns = nun * nmat, nstages = nruns * spt;
+    uint8_t *ring = smem;                                // S stages
+    uint8_t *bimg = ring + size_t(S) * kDStage;          // len x kBKb bytes of digits
+    uint8_t *sfb = bimg + size_t((nkb + 3) >> 2) * kBKb; // len x 512 bytes of their scales
+    float *xslot = reinterpret_cast<float *>(sfb + size_t((nkb + 3) >> 2) * 512); // 4 * nmat exchange slots
 
-    const int G = int(gridDim.x), c = int(blockIdx.x);
-    const int nmat = p.seg[0].nmat;
-    const int my_tiles = c < p.total_tiles ? (p.total_tiles - c + G - 1) / G : 0;
-    const int nruns = my_tiles * nmat;
-    const int total_kb = nruns * nkb;
-
-    if (tid == 0) {
-        for (int i = 0; i < S; i++) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-        for (int i = 0; i < 2; i++) { mbar_init(&dfull[i], 1); mbar_init(&dempty[i], 4); }
-        s_abort = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(kTmemCols));
+    // ---- the weight stream starts first: it depends on nothing ----------------------------------------------------------
+    auto run_src = [&](int run) -> const uint8_t * { // this CTA's records of the run (tile, matrix)
+        const int unit = cl + (nmat == 2 ? run >> 1 : run) * C;
+        const DSeg &s = p.seg[dseg_of(p, unit)];
+        return (nmat == 2 && (run & 1) ? s.packed2 : s.packed) + (size_t(unit - s.tile_begin) * nkb + kb0) * kURec;
+    };
+    auto load_stage = [&](int slot, const uint8_t *src, int st) { // stage st of a run: two records, or the last one of an odd count
+        const uint32_t bytes = uint32_t(min(2, len - 2 * st)) * kURec;
+        mbar_expect_tx(&full[slot], bytes);
+        bulk_load(ring + size_t(slot) * kDStage, src + size_t(st) * kDStage, bytes, &full[slot]);
+    };
+    if (warp == 9) {
+        if (lane == 0) {
+            for (int i = 0; i < S; i++) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+        __syncwarp();
+        if (lane < S && lane < nstages) { // the first ring: one lane per stage
+            const int run = lane / spt;
+            load_stage(lane, run_src(run), lane - run * spt);
+        }
+    } else if (warp == 8) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(kDTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    } else if (tid == 0) {
+        for (int i = 0; i < 2; i++) { mbar_init(&dfull[i], 1); mbar_init(&dempty[i], 4); }
+        for (int i = 0; i < 8; i++) { mbar_init(&xfull[i], 1); mbar_init(&xempty[i], kDCl); }
+        mbar_init(&ssfull, 1);
+        for (int i = 0; i < kDMaxKb / 8; i++) mbar_init(&image[i], uint32_t(T * max(1, min(8, len - 8 * i)))); // one arrival per (token, k-block)
+        s_abort = 0;
+        mbar_expect_tx(&ssfull, kDCl * T * 4);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    } else if (tid >= 128 && tid < 128 + 81) {
+        s_lut[tid - 128] = digit_pair_code(tid - 128);
     }
-    __syncthreads();
-
-    // weights do not depend on the previous kernel: start the stream before the dependency wait
-    if (warp == 5 && lane == 0) {
-        for (int i = 0; i < p.prefetch && i < total_kb; i++) {
-            const int run = i / nkb, kb = i - run * nkb;
-            const uint8_t *src = run_base(p, c + (run / nmat) * G, run % nmat) + size_t(kb) * kURec;
-            mbar_expect_tx(&full[i], kURec);
-            bulk_load(ring + size_t(i) * kURec, src, kURec, &full[i]);
-        }
-    }
-    uint2 wpre[kPreVec];
-    preload_norm_weights(p.pro, wpre);
-    pdl_wait();
-
-    // ---- activation prologue: fp32 vector -> 24-bit fixed point -> twelve E2M1 digit columns ---------
-    float4 v[kMaxVec];
-    load_activation(p.pro, 0, v);
-    const float tmax = transform_activation(p.pro, 0, v, wpre, scratch);
-    int eb = int((__float_as_uint(tmax) >> 23) & 0xffu);
-    eb = min(max(eb, 24), 230);
-    const float alpha = __uint_as_float(uint32_t(127 + 23 - (eb - 127)) << 23); // max * alpha in [2^23, 2^24)
-    const float inv_alpha = __uint_as_float(uint32_t(eb - 23) << 23);
-    {
-        const int nvec = p.pro.cols >> 2;
-#pragma unroll
-        for (int j = 0; j < kMaxVec; j++) {
-            const int i = tid + j * kUThreads;
-            if (i < nvec) {
-                uint32_t lo[4], hi[4];
-                digit_codes(v[j].x, alpha, lo[0], hi[0]);
-                digit_codes(v[j].y, alpha, lo[1], hi[1]);
-                digit_codes(v[j].z, alpha, lo[2], hi[2]);
-                digit_codes(v[j].w, alpha, lo[3], hi[3]);
-                // 4 consecutive k -> 2 bytes per column; image: [kblock][2 steps][2 col groups][2 k cores][8 cols][16 B]
-                const int k = i << 2, kb = k >> 7, kk = k & 127;
-                uint8_t *base = bimg + size_t(kb) * kBImgPerKb + (kk >> 6) * 512 + (((kk & 63) >> 1) >> 4) * 128 + (((kk & 63) >> 1) & 15);
-#pragma unroll
-                for (int col = 0; col < 12; col++) {
-                    const int sh = (col & 7) * 4;
-                    const uint32_t *w = col < 8 ? lo : hi;
-                    const uint32_t two = ((w[0] >> sh) & 0xFu) | (((w[1] >> sh) & 0xFu) << 4) | (((w[2] >> sh) & 0xFu) << 8) |
-                                         (((w[3] >> sh) & 0xFu) << 12);
-                    *reinterpret_cast<uint16_t *>(base + (col >> 3) * 256 + (col & 7) * 16) = uint16_t(two);
-                }
-#pragma unroll
-                for (int col = 12; col < 16; col++) *reinterpret_cast<uint16_t *>(base + 256 + (col & 7) * 16) = 0;
-            }
-        }
-        // column block scales: 4^j for the digit columns, 1 elsewhere; [32 rows][16 B], row = column, byte = (quarter, group)
-        if (tid < 128) reinterpret_cast<uint32_t *>(sfb)[tid] = ((tid >> 2) < 12 && (tid & 3) == 0) ? 0x01010101u * uint32_t(127 + 2 * (tid >> 2)) : 0x7F7F7F7Fu;
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-
+    // The next launch may become resident now, not earlier: were it to take tensor memory before every CTA here has its own,
+    // a CTA could wait for memory held by a CTA that waits for this grid.
+    pdl_launch_dependents();
+    cluster_arrive();
+    cluster_wait(); // the peers' barriers exist from here on
     const uint32_t tmem = s_tmem;
     volatile int *abort_flag = &s_abort;
+    bool arrived = false; // at the closing cluster barrier
 
-    if (warp == 5) {
-        // ---- producer: refill a stage as soon as the MMAs that read it have retired ------------------
-        if (lane == 0) {
-            for (int i = p.prefetch; i < total_kb; i++) {
-                const int st = i % S;
-                if (i >= S && !mbar_wait(&empty[st], ((i / S) - 1) & 1, abort_flag)) break;
-                const int run = i / nkb, kb = i - run * nkb;
-                const uint8_t *src = run_base(p, c + (run / nmat) * G, run % nmat) + size_t(kb) * kURec;
-                mbar_expect_tx(&full[st], kURec);
-                bulk_load(ring + size_t(st) * kURec, src, kURec, &full[st]);
+    if (warp < 8) {
+        // ---- activation prologue: this CTA's quarter of the columns ---------------------------------------------------------
+        constexpr int kBatch = 3;
+        const int items = len * T; // (token, k-block) pairs, dealt to the eight warps
+        const bool rms = p.prologue == INSG_PRO_RMSNORM;
+        float4 x[kBatch], a[kBatch];
+        uint2 w[kBatch];
+        auto place = [&](int it, int &m, int &kb) { m = T == 1 ? 0 : it / len; kb = T == 1 ? it : it - m * len; };
+        auto load_weights = [&](int b0) {
+#pragma unroll
+            for (int j = 0; j < kBatch; j++) {
+                int m, kb;
+                place(b0 + 8 * j, m, kb);
+                w[j] = make_uint2(0u, 0u);
+                if (b0 + 8 * j < items) {
+                    if (rms) w[j] = reinterpret_cast<const uint2 *>(p.norm_w)[(kb0 + kb) * 32 + lane];
+                    else if (p.prologue == INSG_PRO_GATED_RMSNORM) w[j] = reinterpret_cast<const uint2 *>(p.norm_w)[lane];
+                }
+            }
+        };
+        load_weights(warp); // parameters: may be read before the producer of the activation is done
+        pdl_wait();
+        for (int b0 = warp; b0 < items; b0 += 8 * kBatch) {
+            if (b0 != warp) load_weights(b0);
+#pragma unroll
+            for (int j = 0; j < kBatch; j++) { // all loads of the batch in flight together; through L2 (see gemv_prologue.cuh)
+                int m, kb;
+                place(b0 + 8 * j, m, kb);
+                x[j] = a[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (b0 + 8 * j < items && m < p.tokens) {
+                    const int k = (kb0 + kb) * 128 + lane * 4;
+                    x[j] = __ldcg(reinterpret_cast<const float4 *>(p.in + size_t(m) * p.cols + k));
+                    switch (p.prologue) {
+                    case INSG_PRO_GATED_RMSNORM:
+                    case INSG_PRO_SIGMOID_GATE: a[j] = __ldcg(reinterpret_cast<const float4 *>(p.aux + size_t(m) * p.cols + k)); break;
+                    case INSG_PRO_SIGMOID_GATE_HEAD0: a[j].x = __ldcg(p.aux + size_t(m) * 2 * p.cols + (k >> 8) * 512 + 256); break;
+                    case INSG_PRO_SIGMOID_GATE_QPROJ:
+                        a[j] = __ldcg(reinterpret_cast<const float4 *>(p.aux + size_t(m) * 2 * p.cols + (k >> 8) * 512 + 256 + (k & 255)));
+                        break;
+                    default: break;
+                    }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < kBatch; j++) {
+                if (b0 + 8 * j >= items) break; // warp-uniform
+                int m, kb;
+                place(b0 + 8 * j, m, kb);
+                float4 v = x[j];
+                switch (p.prologue) {
+                case INSG_PRO_RMSNORM: { // the factor 1/rms is one number per token: the epilogue applies it
+                    const float ss = warp_sum(fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w))));
+                    if (lane == 0) s_ssq[m * kDMaxKb + kb] = ss;
+                    v.x *= bf16_bits_to_float(w[j].x & 0xffff);
+                    v.y *= bf16_bits_to_float(w[j].x >> 16);
+                    v.z *= bf16_bits_to_float(w[j].y & 0xffff);
+                    v.w *= bf16_bits_to_float(w[j].y >> 16);
+                    break;
+                }
+                case INSG_PRO_GATED_RMSNORM: { // a head is one k-block
+                    const float hs = warp_sum(fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w))));
+                    const float inv = rsqrtf(hs / 128.f + 1e-6f);
+                    v.x = v.x * inv * bf16_bits_to_float(w[j].x & 0xffff) * fast_silu(a[j].x);
+                    v.y = v.y * inv * bf16_bits_to_float(w[j].x >> 16) * fast_silu(a[j].y);
+                    v.z = v.z * inv * bf16_bits_to_float(w[j].y & 0xffff) * fast_silu(a[j].z);
+                    v.w = v.w * inv * bf16_bits_to_float(w[j].y >> 16) * fast_silu(a[j].w);
+                    break;
+                }
+                case INSG_PRO_SIGMOID_GATE:
+                case INSG_PRO_SIGMOID_GATE_QPROJ:
+                    v.x *= fast_sigmoid(a[j].x); v.y *= fast_sigmoid(a[j].y); v.z *= fast_sigmoid(a[j].z); v.w *= fast_sigmoid(a[j].w);
+                    break;
+                case INSG_PRO_SIGMOID_GATE_HEAD0: {
+                    const float g = fast_sigmoid(a[j].x);
+                    v.x *= g; v.y *= g; v.z *= g; v.w *= g;
+                    break;
+                }
+                default: break;
+                }
+                if (p.x_out && cl == 0 && !rms && m < p.tokens)
+                    reinterpret_cast<float4 *>(p.x_out + size_t(m) * p.cols)[(kb0 + kb) * 32 + lane] = v;
+                store_digits<T>(v, m, bimg + size_t(kb) * kBKb, sfb + size_t(kb) * 512, s_lut, lane);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // the tensor core reads the image through the async proxy
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&image[kb >> 3]);
             }
         }
-    } else if (warp == 4) {
-        // ---- MMA issuer ------------------------------------------------------------------------------
-        if (lane == 0) {
-            const uint32_t idesc_base = (1u << 7) | (1u << 10) | ((16u >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
-            asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem + 288), "l"(umma_desc(smem_u32(sfb), 16, 128)));
-            int i = 0;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (warp == 4 && lane < kDCl * T) { // this quarter's sum of squares of each token to the four CTAs
+            const int dst = lane / T, m = lane - dst * T;
+            float ss[1] = {0.f};
+            if (rms)
+                for (int kb = 0; kb < len; kb++) ss[0] += s_ssq[m * kDMaxKb + kb];
+            send_floats<1>(map_to_rank(smem_u32(&s_rss[rank * T + m]), uint32_t(dst)), ss, map_to_rank(smem_u32(&ssfull), uint32_t(dst)));
+        }
+    }
+
+    if (warp == 9) {
+        // ---- producer ----------------------------------------------------------------------------------------------------------
+        {
+            const bool one = elect_one();
+            int i = 0, slot = 0;
+            uint32_t phase = 1; // of the empty barriers: slot reuse n waits for the n-th release
             bool ok = true;
             for (int run = 0; run < nruns && ok; run++) {
+                const uint8_t *src = run_src(run);
+                for (int st = 0; st < spt; st++, i++) {
+                    if (i >= S) {
+                        ok = mbar_wait(&empty[slot], phase, abort_flag);
+                        if (!ok) break;
+                        if (one) load_stage(slot, src, st);
+                    }
+                    if (++slot == S) { slot = 0; phase ^= 1; }
+                }
+            }
+        }
+    } else if (warp == 8) {
+        // ---- MMA issuer --------------------------------------------------------------------------------------------------------
+        // The whole warp walks the loop and one elected lane issues: every operand is then warp-uniform and lives in uniform
+        // registers.  A loop of one lane costs twice as much per instruction (measured per stage: 258 cycles against 594),
+        // which is more than a stage of weights takes to arrive.  Descriptors advance by adding to their address field, and
+        // the next stage's barrier is polled before this stage's multiplies are issued.
+        if (len > 0 && nruns > 0) {
+            const bool one = elect_one();
+            // E2M1 x E2M1, UE8M0 scales, N columns, M = 128; K-step s of a block uses scale bytes 2s, 2s+1 of both operands
+            constexpr uint32_t idesc0 = (1u << 7) | (1u << 10) | ((uint32_t(N) >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
+            constexpr uint32_t idesc1 = idesc0 | (2u << 29) | (2u << 4);
+            const uint64_t da0 = umma_desc(smem_u32(ring), 128, 256), dsf0 = umma_desc(smem_u32(ring) + 8192, 16, 128), db0 = umma_desc(smem_u32(bimg), 128, 256);
+            const uint64_t dsb0 = umma_desc(smem_u32(sfb), 16, 128);
+            bool ok = true;
+            int st = 0, sfa = 0;
+            uint32_t phase = 0;
+            bool here = mbar_test(&full[0], 0), room = true;
+            for (int run = 0; run < nruns && ok; run++) {
                 const int buf = run & 1;
-                ok = mbar_wait(&dempty[buf], ((run >> 1) & 1) ^ 1, abort_flag); // first use of each buffer passes at once
+                const uint32_t dcol = tmem + uint32_t(64 * buf);
+                if (!room) ok = mbar_wait(&dempty[buf], ((run >> 1) & 1) ^ 1, abort_flag); // first use of each buffer passes at once
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int kb = 0; kb < nkb; kb++, i++) {
-                    const int st = i % S;
-                    ok = mbar_wait(&full[st], (i / S) & 1, abort_flag);
-                    if (!ok) break;
+                uint64_t db = db0;
+                uint32_t sb = tmem + kDSfbCol;
+                for (int kb = 0; kb < len; kb += 2) {
+                    if (!here && !mbar_wait(&full[st], phase, abort_flag)) { ok = false; break; }
+                    if (run == 0 && (kb & 7) == 0 && !mbar_wait(&image[kb >> 3], 0, abort_flag)) { ok = false; break; } // the digits of eight k-blocks
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t sbase = smem_u32(ring + size_t(st) * kURec);
-                    const uint32_t t_sfa = tmem + 256 + 4 * (i % kSfaBufs);
-                    asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(t_sfa), "l"(umma_desc(sbase + 8192, 16, 128)));
-                    const uint32_t bbase = smem_u32(bimg + size_t(kb) * kBImgPerKb);
-#pragma unroll
-                    for (int s = 0; s < 2; s++) {
-                        const uint64_t da = umma_desc(sbase + s * 4096, 128, 256), db = umma_desc(bbase + s * 512, 128, 256);
-                        const uint32_t idesc = idesc_base | (uint32_t(2 * s) << 29); // A scales: bytes 2s, 2s+1; B scales: byte 0 (all equal)
-                        const int a = (2 * kb + s) % p.nacc;               // accumulator of this MMA
-                        const uint32_t acc = (2 * kb + s) >= p.nacc ? 1u : 0u;  // its first use overwrites
-                        asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %4, 0;\n"
-                                     "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%5], [%6], q;\n}"
-                                     ::"r"(tmem + 128 * buf + 16 * a), "l"(da), "l"(db), "r"(idesc), "r"(acc), "r"(t_sfa), "r"(tmem + 288)
-                                     : "memory");
+                    const uint64_t da = da0 + uint64_t(uint32_t(st) * uint32_t(kDStage >> 4)), dsf = dsf0 + uint64_t(uint32_t(st) * uint32_t(kDStage >> 4));
+                    const uint32_t sa = tmem + kDSfaCol + 8 * sfa;
+                    const int cur = st;
+                    if (++st == S) { st = 0; phase ^= 1; }
+                    here = mbar_test(&full[st], phase);
+                    if (kb + 2 >= len) room = mbar_test(&dempty[buf ^ 1], (((run + 1) >> 1) & 1) ^ 1);
+                    if (one) {
+                        const bool two = kb + 1 < len;
+                        if (run == 0) { // the digits' scales stay in tensor memory for all tiles
+                            copy_scales(sb, dsb0 + uint64_t(kb * (512 >> 4)));
+                            if (two) copy_scales(sb + 4, dsb0 + uint64_t((kb + 1) * (512 >> 4)));
+                        }
+                        copy_scales(sa, dsf);
+                        if (two) copy_scales(sa + 4, dsf + (kURec >> 4));
+                        mma_step(dcol, da, db, idesc0, kb > 0, sa, sb);
+                        mma_step(dcol, da + 256, db + (kBKb >> 5), idesc1, true, sa, sb);
+                        if (two) {
+                            mma_step(dcol, da + (kURec >> 4), db + (kBKb >> 4), idesc0, true, sa + 4, sb + 4);
+                            mma_step(dcol, da + (kURec >> 4) + 256, db + (kBKb >> 4) + (kBKb >> 5), idesc1, true, sa + 4, sb + 4);
+                        }
+                        commit_to(&empty[cur]);
                     }
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&empty[st])) : "memory");
+                    db += 2 * (kBKb >> 4);
+                    sb += 8;
+                    sfa = (sfa + 1) & 3;
                 }
-                if (ok) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&dfull[buf])) : "memory");
+                if (ok && one) commit_to(&dfull[buf]);
             }
         }
     } else if (warp < 4) {
-        // ---- epilogue: TMEM lane = row of the tile; 16 columns = 12 digit sums (already weighted by 4^j) ----
-        float best = -3.402823466e38f;
-        int best_idx = 0x7fffffff;
-        float gate_val = 0.f;
+        // ---- accumulators -> partial sums -> the CTA that owns these 32 rows (rank = warp) ------------------------------------
+        const uint32_t dst = map_to_rank(smem_u32(xslot) + uint32_t((rank * 32 + lane) * T * 4), uint32_t(warp));
+        const uint32_t dbar = map_to_rank(smem_u32(xfull), uint32_t(warp));
+        const int nslots = 4 * nmat;
         bool ok = true;
         for (int run = 0; run < nruns && ok; run++) {
             const int buf = run & 1;
-            ok = mbar_wait(&dfull[buf], (run >> 1) & 1, abort_flag);
+            float y[T];
+#pragma unroll
+            for (int t = 0; t < T; t++) y[t] = 0.f;
+            if (len > 0) {
+                ok = __all_sync(0xffffffffu, mbar_wait(&dfull[buf], (run >> 1) & 1, abort_flag));
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                load_partial<T>(tmem + uint32_t(64 * buf) + (uint32_t(warp * 32) << 16), y);
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&dempty[buf]);
+            }
+            const int slot = run % nslots;
+            if (run >= nslots) { // the slot's previous content must have been added up by its owner
+                ok = __all_sync(0xffffffffu, mbar_wait_cluster(&xempty[slot], ((run / nslots) - 1) & 1, abort_flag));
+                if (!ok) break;
+            }
+            send_floats<T>(dst + uint32_t(slot * kSlot * 4), y, dbar + uint32_t(slot * 8));
+        }
+    } else if (warp < 8) {
+        // ---- owner of 32 rows of every tile: add the four parts in rank order, fused epilogue ----------------------------------
+        const int fw = warp - 4;
+        float best = -3.402823466e38f, scale[T];
+        int best_idx = 0x7fffffff;
+        bool ok = true;
+#pragma unroll
+        for (int t = 0; t < T; t++) scale[t] = 1.f;
+        // The quarters' sums of squares arrive while the weights are still being multiplied.  Every CTA waits for all four
+        // (also where they are not needed), so that nobody leaves while a peer still writes into its shared memory.
+        ok = __all_sync(0xffffffffu, mbar_wait_cluster(&ssfull, 0, abort_flag));
+        if (ok && p.prologue == INSG_PRO_RMSNORM) {
+#pragma unroll
+            for (int t = 0; t < T; t++) scale[t] = rsqrtf((s_rss[t] + s_rss[T + t] + s_rss[2 * T + t] + s_rss[3 * T + t]) / float(p.cols) + 1e-6f);
+            if (p.x_out && cl == 0) {
+                for (int m = 0; m < p.tokens; m++) {
+                    float sc = scale[0];
+#pragma unroll
+                    for (int t = 1; t < T; t++) sc = t == m ? scale[t] : sc;
+                    for (int k = kb0 * 128 + fw * 32 + lane; k < (kb0 + len) * 128; k += 128)
+                        p.x_out[size_t(m) * p.cols + k] = __ldcg(p.in + size_t(m) * p.cols + k) * sc * bf16_bits_to_float(p.norm_w[k]);
+                }
+            }
+        }
+        for (int i = fw; i < nun && ok; i += 4) {
+            const int unit = cl + i * C;
+            const DSeg &s = p.seg[dseg_of(p, unit)];
+            const int row = (unit - s.tile_begin) * 128 + rank * 32 + lane;
+            const bool on = row < s.rows;
+            const size_t ld = size_t(s.rows);
+            float *out = s.out + row;
+            // the epilogue's other operands are fetched before the wait for the sums
+            float pre[T], h0 = 0.f, h1 = 0.f, h2 = 0.f;
+            float cw0 = 0.f, cw1 = 0.f, cw2 = 0.f, cw3 = 0.f;
+#pragma unroll
+            for (int t = 0; t < T; t++) pre[t] = 0.f;
+            if (on && s.epilogue == INSG_EPI_RESIDUAL) {
+#pragma unroll
+                for (int t = 0; t < T; t++)
+                    if (t < p.tokens) pre[t] = __ldcg(out + t * ld);
+            } else if (on && s.epilogue == INSG_EPI_CONV_SILU) {
+                const uint2 wv = reinterpret_cast<const uint2 *>(s.conv_w)[row];
+                cw0 = bf16_bits_to_float(wv.x & 0xffff); cw1 = bf16_bits_to_float(wv.x >> 16);
+                cw2 = bf16_bits_to_float(wv.y & 0xffff); cw3 = bf16_bits_to_float(wv.y >> 16);
+                const float *hist = s.conv_state + size_t(row) * 3;
+                h0 = __ldcg(hist); h1 = __ldcg(hist + 1); h2 = __ldcg(hist + 2);
+            } else if (on && s.epilogue == INSG_EPI_DECAY) {
+                h0 = bf16_bits_to_float(s.dt_bias[row]);
+                h1 = -__expf(s.A_log[row]);
+            }
+            float y[2][T];
+#pragma unroll
+            for (int mat = 0; mat < 2; mat++) {
+                if (mat >= nmat) break;
+                const int slot = fw * nmat + mat;
+                if (lane == 0) mbar_expect_tx(&xfull[slot], kSlot * 4);
+                ok = __all_sync(0xffffffffu, mbar_wait_cluster(&xfull[slot], (i >> 2) & 1, abort_flag));
+                if (!ok) break;
+                const float *src = xslot + size_t(slot) * kSlot + lane * T;
+#pragma unroll
+                for (int t = 0; t < T; t++) {
+                    float z = src[t];
+#pragma unroll
+                    for (int r = 1; r < kDCl; r++) z += src[r * 32 * T + t];
+                    y[mat][t] = z * scale[t];
+                }
+                if (i + 4 < nun) { // the slot will be used again: tell the four senders
+                    __syncwarp();
+                    if (lane < kDCl) remote_arrive(map_to_rank(smem_u32(&xempty[slot]), uint32_t(lane)));
+                }
+            }
             if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            float y = 0.f;
-            const int nused = min(p.nacc, 2 * nkb);
-            for (int a = 0; a < nused; a++) { // fixed order: accumulator 0 first, least significant digit first
-                uint32_t r[16];
-                const uint32_t taddr = tmem + 128 * buf + 16 * a + (uint32_t(warp * 32) << 16);
-                asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-                               "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                             : "r"(taddr));
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                float ya = 0.f;
-#pragma unroll
-                for (int j = 0; j < 12; j++) ya += __uint_as_float(r[j]);
-                y += ya;
+            if (i + 4 >= nun) { // nothing more comes in for this warp: the peers need not wait for its epilogue
+                cluster_arrive();
+                arrived = true;
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&dempty[buf]);
-            y *= inv_alpha;
-            const int tile = c + (run / nmat) * G, mat = run % nmat;
-            const USeg &s = p.seg[useg_of(p, tile)];
-            const int row = (tile - s.tile_begin) * 128 + tid;
-            if (row < s.rows) {
-                float *out = s.out;
-                switch (s.epilogue) {
-                case INSG_EPI_STORE: out[row] = y; break;
-                case INSG_EPI_RESIDUAL: out[row] = __ldcg(out + row) + y; break;
-                case INSG_EPI_CONV_SILU: {
-                    float *st = s.conv_state + size_t(row) * 3;
-                    const uint2 wv = reinterpret_cast<const uint2 *>(s.conv_w)[row];
-                    const float w0 = bf16_bits_to_float(wv.x & 0xffff), w1 = bf16_bits_to_float(wv.x >> 16);
-                    const float w2 = bf16_bits_to_float(wv.y & 0xffff), w3 = bf16_bits_to_float(wv.y >> 16);
-                    const float s0 = __ldcg(st), s1 = __ldcg(st + 1), s2 = __ldcg(st + 2);
-                    const float z = fmaf(s0, w0, fmaf(s1, w1, fmaf(s2, w2, y * w3)));
-                    st[0] = s1; st[1] = s2; st[2] = y;
-                    out[row] = fast_silu(z);
-                    break;
+            if (!on) continue;
+            switch (s.epilogue) {
+            case INSG_EPI_STORE:
+#pragma unroll
+                for (int t = 0; t < T; t++)
+                    if (t < p.tokens) out[t * ld] = y[0][t];
+                break;
+            case INSG_EPI_RESIDUAL:
+#pragma unroll
+                for (int t = 0; t < T; t++)
+                    if (t < p.tokens) out[t * ld] = pre[t] + y[0][t];
+                break;
+            case INSG_EPI_CONV_SILU: {
+                float *hist = s.conv_state + size_t(row) * 3;
+#pragma unroll
+                for (int t = 0; t < T; t++) {
+                    if (t < p.tokens) {
+                        if (t > 0 && s.conv_stride != 0) { // independent sequences: each token has its own history
+                            hist += s.conv_stride;
+                            h0 = __ldcg(hist); h1 = __ldcg(hist + 1); h2 = __ldcg(hist + 2);
+                        }
+                        const float z = fmaf(h0, cw0, fmaf(h1, cw1, fmaf(h2, cw2, y[0][t] * cw3)));
+                        h0 = h1; h1 = h2; h2 = y[0][t];
+                        out[t * ld] = fast_silu(z);
+                        if (s.conv_stride != 0 || t + 1 == p.tokens) { hist[0] = h0; hist[1] = h1; hist[2] = h2; }
+                    }
                 }
-                case INSG_EPI_BETA: out[row] = fast_sigmoid(y); break;
-                case INSG_EPI_DECAY: {
-                    const float z = y + bf16_bits_to_float(s.dt_bias[row]);
-                    const float soft = z > 20.f ? z : log1pf(__expf(z));
-                    out[row] = -__expf(s.A_log[row]) * soft;
-                    break;
+                break;
+            }
+            case INSG_EPI_BETA:
+#pragma unroll
+                for (int t = 0; t < T; t++)
+                    if (t < p.tokens) out[t * ld] = fast_sigmoid(y[0][t]);
+                break;
+            case INSG_EPI_DECAY:
+#pragma unroll
+                for (int t = 0; t < T; t++) {
+                    const float z = y[0][t] + h0;
+                    if (t < p.tokens) out[t * ld] = h1 * (z > 20.f ? z : log1pf(__expf(z)));
                 }
-                case INSG_EPI_SWIGLU:
-                    if (mat == 0) gate_val = y;
-                    else out[row] = fast_silu(gate_val) * y;
-                    break;
-                case INSG_EPI_LOGITS:
-                    out[row] = y;
-                    if (y > best || (y == best && row < best_idx)) { best = y; best_idx = row; }
-                    break;
-                default: break;
-                }
+                break;
+            case INSG_EPI_SWIGLU:
+#pragma unroll
+                for (int t = 0; t < T; t++)
+                    if (t < p.tokens) out[t * ld] = fast_silu(y[0][t]) * y[1][t];
+                break;
+            case INSG_EPI_LOGITS:
+                out[0] = y[0][0];
+                if (y[0][0] > best || (y[0][0] == best && row < best_idx)) { best = y[0][0]; best_idx = row; }
+                break;
+            default: break;
             }
         }
-        // per-warp arg-max candidates for the logits epilogue
         if (p.argmax_partial) {
+            // per-CTA arg-max, then the last CTA of the grid folds the CTAs' (lowest index on ties)
+            auto fold = [&] {
 #pragma unroll
-            for (int mk = 16; mk; mk >>= 1) {
-                const float ov = __shfl_xor_sync(0xffffffffu, best, mk);
-                const int oi = __shfl_xor_sync(0xffffffffu, best_idx, mk);
-                if (ov > best || (ov == best && oi < best_idx)) { best = ov; best_idx = oi; }
-            }
-            if (lane == 0) { scratch[32 + warp] = best; reinterpret_cast<int *>(scratch)[40 + warp] = best_idx; }
-        }
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
-    if (tid == 0 && s_abort && p.error_flag) *p.error_flag = 1;
-
-    if (p.argmax_partial) {
-        if (tid == 0) {
-            float bv = scratch[32];
-            int bi = reinterpret_cast<int *>(scratch)[40];
-            for (int w = 1; w < 4; w++) {
-                const float ov = scratch[32 + w];
-                const int oi = reinterpret_cast<int *>(scratch)[40 + w];
-                if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-            }
-            p.argmax_partial[blockIdx.x] = make_float2(bv, __int_as_float(bi));
-            __threadfence();
-            const unsigned ticket = atomicAdd(p.argmax_ticket, 1u);
-            s_last = (ticket == gridDim.x - 1);
-        }
-        __syncthreads();
-        if (s_last && warp == 0) {
-            __threadfence();
-            float bv = -3.402823466e38f;
-            int bi = 0x7fffffff;
-            for (int i = lane; i < G; i += 32) {
-                const float ev = __ldcg(reinterpret_cast<const float *>(p.argmax_partial + i));
-                const int idx = __float_as_int(__ldcg(reinterpret_cast<const float *>(p.argmax_partial + i) + 1));
-                if (ev > bv || (ev == bv && idx < bi)) { bv = ev; bi = idx; }
-            }
-#pragma unroll
-            for (int mk = 16; mk; mk >>= 1) {
-                const float ov = __shfl_xor_sync(0xffffffffu, bv, mk);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, mk);
-                if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-            }
-            if (lane == 0) {
-                *p.token_out = bi;
-                if (p.token_feedback) *p.token_feedback = bi;
-                if (p.position_inout) {
-                    const int pos = *p.position_inout;
-                    if (p.token_log && pos >= 0 && pos < p.token_log_capacity) p.token_log[pos] = bi;
-                    *p.position_inout = pos + 1;
+                for (int mk = 16; mk; mk >>= 1) {
+                    const float ov = __shfl_xor_sync(0xffffffffu, best, mk);
+                    const int oi = __shfl_xor_sync(0xffffffffu, best_idx, mk);
+                    if (ov > best || (ov == best && oi < best_idx)) { best = ov; best_idx = oi; }
                 }
-                *p.argmax_ticket = 0u;
+            };
+            __syncwarp();
+            fold();
+            if (lane == 0) { s_best[fw] = best; s_bidx[fw] = best_idx; }
+            asm volatile("bar.sync 2, 128;" ::: "memory");
+            if (fw == 0) {
+                if (lane == 0) {
+                    for (int w = 1; w < 4; w++)
+                        if (s_best[w] > best || (s_best[w] == best && s_bidx[w] < best_idx)) { best = s_best[w]; best_idx = s_bidx[w]; }
+                    p.argmax_partial[blockIdx.x] = make_float2(best, __int_as_float(best_idx));
+                    __threadfence();
+                    s_last = atomicAdd(p.argmax_ticket, 1u) == gridDim.x - 1;
+                }
+                __syncwarp();
+                if (s_last) {
+                    __threadfence();
+                    best = -3.402823466e38f;
+                    best_idx = 0x7fffffff;
+                    for (int i = lane; i < int(gridDim.x); i += 32) {
+                        const float2 e = __ldcg(p.argmax_partial + i);
+                        const int idx = __float_as_int(e.y);
+                        if (e.x > best || (e.x == best && idx < best_idx)) { best = e.x; best_idx = idx; }
+                    }
+                    fold();
+                    if (lane == 0) {
+                        *p.token_out = best_idx;
+                        if (p.token_feedback) *p.token_feedback = best_idx;
+                        if (p.position_inout) {
+                            const int pos = __ldcg(p.position_inout);
+                            if (p.token_log && pos >= 0 && pos < p.token_log_capacity) p.token_log[pos] = best_idx;
+                            *p.position_inout = pos + 1;
+                        }
+                        *p.argmax_ticket = 0u;
+                    }
+                }
             }
         }
     }
+    // Nobody leaves while a peer may still write into its shared memory (after an expired wait too).
+    __syncwarp();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (!arrived) cluster_arrive();
+    cluster_wait();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    __syncwarp();
+    if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kDTmemCols));
+    if (tid == 0 && s_abort && p.error_flag) *p.error_flag = 1;
 }
 
 // ---- repack: MLX layout -> shared-memory images ----------------------------------------------------
@@ -385,47 +710,80 @@ __global__ void repack_umma_kernel(const uint32_t *__restrict__ w, const uint8_t
 }
 
 namespace {
-// fixed launch shape (measured best; no process-wide knobs: engines and threads share this library)
-constexpr int kUStages = 16, kUNacc = 8, kUPrefetch = 8;
-
 std::mutex g_attr_mutex;
-bool g_attr_done[64] = {false}; // the shared-memory opt-in is a per-device function attribute
-} // namespace
+int g_max_clusters[64] = {0}; // per device: clusters that run at once with one CTA per SM (0 = not asked yet)
 
+// The shared-memory opt-in is a per-device function attribute; the cluster count is a property of the device's layout.
+int device_clusters(int *out)
+{
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
+    if (dev < 0 || dev >= 64) return fail(INSG_E_LIMIT, "gemv: device ordinal beyond 63");
+    std::lock_guard<std::mutex> lock(g_attr_mutex);
+    if (!g_max_clusters[dev]) {
+        for (auto k : {umma_gemv_kernel<1>, umma_gemv_kernel<2>, umma_gemv_kernel<4>, umma_gemv_kernel<8>}) {
+            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
+            if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(umma gemv)");
+        }
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kDCl);
+        cfg.blockDim = dim3(kDThreads);
+        cfg.dynamicSmemBytes = 200 * 1024;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = kDCl;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        e = cudaOccupancyMaxActiveClusters(&n, umma_gemv_kernel<1>, &cfg);
+        if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveClusters");
+        g_max_clusters[dev] = std::max(1, std::min(n, 128)); // 128 clusters: the arg-max partials are sized for 512 CTAs
+    }
+    *out = g_max_clusters[dev];
+    return INSG_OK;
+}
+} // namespace
 
 int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
 {
     if (!op || !op->in) return fail(INSG_E_ARG, "gemv: null operand");
-    if (op->cols <= 0 || (op->cols & 127) || op->cols > kMaxVec * kUThreads * 4) return fail(INSG_E_SHAPE, "gemv: cols must be a multiple of 128, <= 12288");
+    const int tokens = op->tokens > 1 ? op->tokens : 1;
+    if (tokens > 8) return fail(INSG_E_SHAPE, "gemv: 1..8 tokens");
+    if (op->cols <= 0 || (op->cols & 127) || op->cols > kDMaxKb * kDCl * 128) return fail(INSG_E_SHAPE, "gemv: cols must be a multiple of 128, <= 12288");
     if (op->n_segments < 1 || op->n_segments > 4) return fail(INSG_E_SHAPE, "gemv: 1..4 segments");
+    if (op->prologue < 0 || op->prologue >= INSG_PRO_PREPARED) return fail(INSG_E_ARG, "gemv: a prepared input belongs to the mma.sync layout");
     if ((op->prologue == INSG_PRO_RMSNORM || op->prologue == INSG_PRO_GATED_RMSNORM) && !op->norm_w) return fail(INSG_E_ARG, "gemv: norm weight missing");
     if (op->prologue >= INSG_PRO_GATED_RMSNORM && !op->aux) return fail(INSG_E_ARG, "gemv: prologue operand missing");
-    UParams p = {};
-    p.pro = ProIn{op->in, op->aux, op->norm_w, op->x_out, op->cols, op->prologue};
+    DParams p = {};
+    p.in = op->in; p.aux = op->aux; p.norm_w = op->norm_w; p.x_out = op->x_out;
+    p.cols = op->cols; p.prologue = op->prologue;
     p.nkb = op->cols >> 7;
     p.nseg = op->n_segments;
-    int tiles = 0, nmat_all = 0;
+    p.tokens = tokens;
     bool logits = false;
     for (int i = 0; i < op->n_segments; i++) {
         const insg_gemv_segment &s = op->seg[i];
         if (!s.packed || !s.out || s.rows <= 0) return fail(INSG_E_SHAPE, "gemv: bad segment");
+        if (s.prep) return fail(INSG_E_SHAPE, "gemv: a prepared output belongs to the mma.sync layout");
         if (s.epilogue == INSG_EPI_SWIGLU && !s.packed2) return fail(INSG_E_ARG, "gemv: SwiGLU needs two matrices");
         if (s.epilogue == INSG_EPI_CONV_SILU && (!s.conv_state || !s.conv_w)) return fail(INSG_E_ARG, "gemv: conv operands missing");
         if (s.epilogue == INSG_EPI_DECAY && (!s.A_log || !s.dt_bias)) return fail(INSG_E_ARG, "gemv: decay operands missing");
-        USeg &d = p.seg[i];
+        DSeg &d = p.seg[i];
         d.packed = static_cast<const uint8_t *>(s.packed);
         d.packed2 = static_cast<const uint8_t *>(s.packed2);
         d.out = s.out; d.conv_state = s.conv_state; d.conv_w = s.conv_w; d.A_log = s.A_log; d.dt_bias = s.dt_bias;
-        d.nmat = s.epilogue == INSG_EPI_SWIGLU ? 2 : 1;
-        if (nmat_all && nmat_all != d.nmat) return fail(INSG_E_SHAPE, "gemv: SwiGLU segments cannot be mixed with others");
-        nmat_all = d.nmat;
-        d.tile_begin = tiles; d.ntiles = (s.rows + 127) >> 7; tiles += d.ntiles; d.epilogue = s.epilogue; d.rows = s.rows;
+        d.conv_stride = s.conv_token_stride;
+        const int nmat = s.epilogue == INSG_EPI_SWIGLU ? 2 : 1;
+        if (p.nmat && p.nmat != nmat) return fail(INSG_E_SHAPE, "gemv: SwiGLU segments cannot be mixed with others");
+        p.nmat = nmat;
+        d.tile_begin = p.units; p.units += (s.rows + 127) >> 7; d.epilogue = s.epilogue; d.rows = s.rows;
         logits |= s.epilogue == INSG_EPI_LOGITS;
     }
-    p.total_tiles = tiles;
-    const int grid = std::max(1, std::min(std::min(sm_count(), 256), tiles));
     if (logits) {
         if (op->n_segments != 1) return fail(INSG_E_SHAPE, "gemv: the logits epilogue takes one segment");
+        if (tokens != 1) return fail(INSG_E_SHAPE, "gemv: the logits epilogue takes one token");
         if (!op->argmax_scratch || !op->token_out) return fail(INSG_E_ARG, "gemv: arg-max scratch/token missing");
         p.argmax_ticket = static_cast<unsigned *>(op->argmax_scratch);
         p.argmax_partial = reinterpret_cast<float2 *>(static_cast<uint8_t *>(op->argmax_scratch) + 64);
@@ -434,26 +792,36 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
         if (op->token_log && op->token_log_capacity <= 0) return fail(INSG_E_ARG, "gemv: token_log needs its capacity");
     }
     p.error_flag = static_cast<int *>(op->error_flag);
-    const size_t fixed = size_t(p.nkb) * kBImgPerKb + 512 + 64 * 4 + 1024;
-    int stages = std::min(kUStages, int((size_t(220) * 1024 - fixed) / kURec));
-    stages = std::max(2, std::min(stages, 24));
-    p.stages = stages;
-    p.nacc = kUNacc;
-    p.prefetch = std::min(kUPrefetch, stages);
-    const size_t smem = size_t(stages) * kURec + fixed;
-    {
-        int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
-        if (dev < 0 || dev >= 64) return fail(INSG_E_LIMIT, "gemv: device ordinal beyond 63");
-        std::lock_guard<std::mutex> lock(g_attr_mutex);
-        if (!g_attr_done[dev]) {
-            e = cudaFuncSetAttribute(umma_gemv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
-            if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(umma gemv)");
-            g_attr_done[dev] = true;
-        }
-    }
-    return launch(umma_gemv_kernel, dim3(grid), dim3(kUThreads), smem, st, op->pdl != 0, p);
+    int max_clusters = 0;
+    const int rc = device_clusters(&max_clusters);
+    if (rc != INSG_OK) return rc;
+    const int clusters = std::min(p.units, max_clusters);
+    const int T = tokens == 1 ? 1 : tokens == 2 ? 2 : tokens <= 4 ? 4 : 8;
+    const int kbq = (p.nkb + 3) >> 2;
+    const size_t fixed = size_t(kbq) * (512 * T + 512) + size_t(4) * p.nmat * kDCl * 32 * T * sizeof(float);
+    // ring: no more stages than the launch has, within half an SM when that leaves at least four, else whatever fits
+    const int need = ((p.units + clusters - 1) / clusters) * p.nmat * ((kbq + 1) / 2);
+    int stages = fixed < size_t(kDHalfSm) ? int((kDHalfSm - fixed) / kDStage) : 0;
+    if (stages < 4) stages = int((size_t(222) * 1024 - fixed) / kDStage);
+    p.stages = std::max(1, std::min({stages, need, kDMaxStages}));
+    const size_t smem = fixed + size_t(p.stages) * kDStage;
+
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(clusters * kDCl));
+    cfg.blockDim = dim3(kDThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kDCl;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = op->pdl ? 2 : 1;
+    auto kernel = T == 1 ? umma_gemv_kernel<1> : T == 2 ? umma_gemv_kernel<2> : T == 4 ? umma_gemv_kernel<4> : umma_gemv_kernel<8>;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
+    return e == cudaSuccess ? INSG_OK : cuda_fail(e, "umma gemv launch");
 }
 
 } // namespace insg

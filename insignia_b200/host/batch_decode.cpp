@@ -26,8 +26,7 @@ void insg_check(int rc)
 } // namespace
 
 struct Qwen35BatchDecode::Impl {
-    int B = 0;      // sequences the kernels run (1 and 2 on the mma.sync kernel, 3..8 on the tcgen05 kernel)
-    int layout = 0; // weight layout: 0 mma.sync records (B <= 2), 1 tcgen05 tiles (B >= 3)
+    int B = 0; // sequences = tokens of each launch of the tcgen05 GEMV
     std::vector<DecodeBlock> layers;
     const uint16_t *final_norm{};
     PackedMatrix lm_head;
@@ -44,8 +43,7 @@ struct Qwen35BatchDecode::Impl {
     float *delta_state{}, *conv_state{}; // [B][24][...]
     void *kv_keys{}, *kv_values{};       // [B][8][ctx][1024]
     void *attn_scratch{};                // [B][insg_gqa_scratch_bytes]
-    void *umma_scratch{};
-    size_t umma_scratch_bytes = 0, attn_scratch_each = 0, kv_seq_bytes = 0;
+    size_t attn_scratch_each = 0, kv_seq_bytes = 0;
     int *d_tokens{}, *d_next{}, *d_position{}, *d_error{}, *d_log{}; // log [ctx + 1][B]
     int *host_tokens{};                  // pinned
     std::vector<void *> allocs;
@@ -63,7 +61,6 @@ Qwen35BatchDecode::Qwen35BatchDecode(Qwen35Weights &weights, int sequences, int 
     if (max_context <= 0) throw std::runtime_error("max_context must be positive");
     Impl &m = *impl_;
     m.B = sequences;
-    m.layout = sequences >= 3 ? 1 : 0; // measured: four sequences cost the mma.sync kernel 4.6 ms a step, the tcgen05 kernel less
     if (stream) {
         m.stream = stream;
     } else {
@@ -89,8 +86,6 @@ Qwen35BatchDecode::Qwen35BatchDecode(Qwen35Weights &weights, int sequences, int 
     m.alloc(&m.kv_values, B * m.kv_seq_bytes, "cudaMalloc batch KV cache");
     m.attn_scratch_each = (insg_gqa_scratch_bytes(max_context) + 255) / 256 * 256;
     m.alloc(&m.attn_scratch, B * m.attn_scratch_each, "cudaMalloc batch attention scratch");
-    m.umma_scratch_bytes = insg_umma_gemm_scratch_bytes(kInter, m.B);
-    m.alloc(&m.umma_scratch, m.umma_scratch_bytes, "cudaMalloc batch activation image");
     m.alloc(&m.d_tokens, (3 * B + 8) * sizeof(int), "cudaMalloc batch scalars");
     m.d_next = m.d_tokens + B;
     m.d_position = m.d_next + B;
@@ -145,29 +140,25 @@ void Qwen35BatchDecode::enqueue_step()
     const int n = options_.n_layers, B = m.B;
     if (!m.loaded) {
         m.layers.resize(size_t(n));
-        Loader L{w_, m.pinned, m.layout};
+        Loader L{w_, m.pinned, 1};
         for (int l = 0; l < n; l++) {
             const std::string name = std::string(kLM) + ".model.layers." + std::to_string(l);
             if (Qwen35Shape::full_attention(l)) load_attention(L, name, m.layers[size_t(l)]);
             else load_delta(L, name, m.layers[size_t(l)]);
         }
         m.final_norm = L.bf16(std::string(kLM) + ".model.norm.weight", kHidden);
-        m.lm_head = w_.packed(std::string(kLM) + ".lm_head", m.layout);
+        m.lm_head = w_.packed(std::string(kLM) + ".lm_head", 1);
         m.embed = w_.matrix(std::string(kLM) + ".model.embed_tokens");
         m.loaded = true;
     }
     cudaStream_t st = m.stream;
     auto gemv = [&](insg_gemv_op &op) {
         op.tokens = B;
-        op.layout = m.layout;
+        op.layout = 1;
         op.error_flag = m.d_error;
         op.pdl = 1; // every kernel of the step waits for its predecessor before it reads activations
-        if (m.layout == 1 && B > 1) {
-            op.umma_scratch = m.umma_scratch;
-            op.umma_scratch_bytes = m.umma_scratch_bytes;
-        }
         insg_check(insg_gemv_fused(&op, st));
-        launches_ += (m.layout == 1 && B > 1) ? 2 : 1;
+        launches_++;
     };
     auto mlp = [&](const DecodeBlock &blk) {
         insg_gemv_op up = {};

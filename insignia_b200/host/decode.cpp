@@ -28,7 +28,8 @@ constexpr size_t kPrepHidden = 0, kPrepAct = size_t(2) * kHidden * 2, kPrepSums 
 constexpr int kMultiSteps = 8; // token steps per graph in Qwen35Decode::generate
 // DecodeWorkspace::multi: activations of up to kChunk consecutive tokens for Qwen35Decode::forward_tokens, [token][width] each
 constexpr int kChunk = 4;     // tokens per pass of the mma.sync kernel
-constexpr int kBigChunk = 256; // tokens per pass of the tcgen05 kernel (sixteen groups of sixteen)
+constexpr int kSmallChunk = 8; // tokens per pass of the tcgen05 GEMV
+constexpr int kBigChunk = 256; // tokens per pass of the tcgen05 GEMM (sixteen groups of sixteen)
 constexpr size_t kMultiHidden = 0, kMultiQkv = kMultiHidden + size_t(kBigChunk) * 4096, kMultiZ = kMultiQkv + size_t(kBigChunk) * 8192,
                  kMultiA = kMultiZ + size_t(kBigChunk) * 4096, kMultiB = kMultiA + size_t(kBigChunk) * 32,
                  kMultiCore = kMultiB + size_t(kBigChunk) * 32, kMultiQg = kMultiCore + size_t(kBigChunk) * 4096,
@@ -196,6 +197,10 @@ Qwen35Decode::Plan &Qwen35Decode::plan()
 
 // --------------------------------------------------------------- enqueue helpers
 namespace {
+// The engine's weight layout.  The tcgen05 kernels carry every pass (one token to prompts) on one tile-layout copy of the
+// weights; the persistent program and prepared_inputs = false run the mma.sync kernel on its own record layout.
+bool tcgen05_engine(const DecodeOptions &o) { return o.gemv_tcgen05 || (o.prepared_inputs && !o.persistent); }
+
 struct Ctx {
     DecodeWorkspace &x;
     cudaStream_t st;
@@ -210,7 +215,8 @@ struct Ctx {
     void *prep_hidden() const { return static_cast<uint8_t *>(x.prep) + kPrepHidden; }
     void *prep_act() const { return static_cast<uint8_t *>(x.prep) + kPrepAct; }
     float *prep_sums() const { return reinterpret_cast<float *>(static_cast<uint8_t *>(x.prep) + kPrepSums); }
-    bool prepared() const { return x.options.prepared_inputs && !x.options.gemv_tcgen05; }
+    bool tcgen05() const { return tcgen05_engine(x.options); }
+    bool prepared() const { return x.options.prepared_inputs && !tcgen05(); }
 };
 
 // The block's first GEMV: RMSNorm of the residual stream, from the fp32 vector or from the image the previous block left.
@@ -227,7 +233,7 @@ void rmsnorm_input(const Ctx &c, insg_gemv_op &op, const uint16_t *norm_w)
     } else {
         op.in = c.x.hidden;
         op.norm_w = norm_w;
-        op.x_out = c.x.norm;
+        op.x_out = c.hidden_prepared ? nullptr : c.x.norm; // inside a token step nobody reads the normalised vector
         op.prologue = INSG_PRO_RMSNORM;
     }
 }
@@ -252,9 +258,9 @@ uint64_t gemv_weight_bytes(const insg_gemv_op &op)
 void run_gemv(Ctx &c, insg_gemv_op &op)
 {
     op.pdl = c.pdl ? 1 : 0;
-    op.layout = c.layout >= 0 ? c.layout : (c.x.options.gemv_tcgen05 ? 1 : 0);
+    op.layout = c.layout >= 0 ? c.layout : (c.tcgen05() ? 1 : 0);
     op.error_flag = c.x.d_token + 3;
-    if (op.layout == 1 && op.tokens > 1) {
+    if (op.layout == 1 && op.tokens > kSmallChunk) {
         op.umma_scratch = c.x.umma_scratch;
         op.umma_scratch_bytes = c.x.umma_scratch_bytes;
     }
@@ -591,7 +597,7 @@ void Qwen35Decode::load_block(int l)
     Plan::Block &b = p.layers[l];
     if (b.ready) return;
     prefetch_block(l + 1);
-    Loader L{w_, p.pinned, x_.options.gemv_tcgen05 ? 1 : 0};
+    Loader L{w_, p.pinned, tcgen05_engine(x_.options) ? 1 : 0};
     const std::string name = std::string(kLM) + ".model.layers." + std::to_string(l);
     if (Qwen35Shape::full_attention(l)) load_attention(L, name, b);
     else load_delta(L, name, b);
@@ -601,9 +607,9 @@ void Qwen35Decode::load_head()
 {
     Plan &p = plan();
     if (p.head_ready) return;
-    Loader L{w_, p.pinned, x_.options.gemv_tcgen05 ? 1 : 0};
+    Loader L{w_, p.pinned, tcgen05_engine(x_.options) ? 1 : 0};
     p.final_norm = L.bf16(std::string(kLM) + ".model.norm.weight", kHidden);
-    p.lm_head = w_.packed(std::string(kLM) + ".lm_head", x_.options.gemv_tcgen05 ? 1 : 0);
+    p.lm_head = w_.packed(std::string(kLM) + ".lm_head", L.layout);
     if (p.lm_head.cols != kHidden || p.lm_head.rows < x_.options.vocab) throw std::runtime_error("unexpected matrix shape: language_model.lm_head");
     p.head_ready = true;
 }
@@ -755,7 +761,7 @@ bool Qwen35Decode::selftest_barrier_timeout()
     return gave_up;
 }
 
-bool Qwen35Decode::persistent() const { return x_.options.persistent && !x_.options.gemv_tcgen05; }
+bool Qwen35Decode::persistent() const { return x_.options.persistent && !tcgen05_engine(x_.options); }
 
 void Qwen35Decode::replay_token_step()
 {
@@ -831,29 +837,26 @@ void Qwen35Decode::forward_tokens(const int *tokens, int count)
     for (int i = 0; i < count; i++)
         if (tokens[i] < 0 || tokens[i] >= Qwen35Shape::vocab) throw std::runtime_error("token out of range");
     if (x_.position + count > x_.max_context) throw std::runtime_error("KV cache full");
-    if (x_.options.gemv_tcgen05) { // that layout takes one token per launch
-        for (int i = 0; i < count; i++) forward_token(tokens[i]);
-        return;
-    }
     Plan &p = plan();
     const int n = x_.options.n_layers;
     for (int l = 0; l < n; l++) load_block(l);
     load_head();
     load_embed();
     Ctx c{x_, p.stream, x_.options.use_pdl, launches_, false, nullptr, nullptr};
-    // Long prompts go through the tcgen05 kernel in passes of up to kBigChunk tokens (sixteen tokens per instruction); what
-    // is left, and short prompts, through the mma.sync kernel in passes of four.
-    const bool big = x_.options.prefill_tcgen05 && count >= 16;
-    if (big)
+    // Long prompts go through the tcgen05 GEMM in passes of up to kBigChunk tokens (sixteen tokens per instruction); what is
+    // left, and short prompts, through the engine's own GEMV: up to eight tokens a pass on tcgen05, four on mma.sync.
+    const bool one_layout = tcgen05_engine(x_.options);
+    const bool big = x_.options.prefill_tcgen05 && count > (one_layout ? kSmallChunk : 15);
+    if (big && !one_layout)
         for (int l = 0; l < n; l++) load_block_umma(l);
     for (int done = 0; done < count;) {
         const int left = count - done;
-        const bool use_umma = big && left >= 8;
-        const int T = use_umma ? std::min(left, kBigChunk) : (left >= 4 ? 4 : (left >= 2 ? 2 : 1));
+        const bool use_umma = big && left > (one_layout ? kSmallChunk : 7);
+        const int T = use_umma ? std::min(left, kBigChunk) : one_layout ? std::min(left, kSmallChunk) : (left >= 4 ? 4 : (left >= 2 ? 2 : 1));
         c.layout = use_umma ? 1 : -1;
-        const std::vector<Plan::Block> &blocks = use_umma ? p.layers_umma : p.layers;
+        const std::vector<Plan::Block> &blocks = use_umma && !one_layout ? p.layers_umma : p.layers;
         Multi u(x_, T);
-        if (use_umma) u.rows_hint = x_.position + T; // eager passes only: a replayed graph must not bake the context length in
+        if (use_umma || one_layout) u.rows_hint = x_.position + T; // eager passes only: a replayed graph must not bake the context length in
         sync_scalars(-1); // the chunk's first position; token m of the chunk sits at position + m
         cuda_check(cudaMemcpyAsync(u.tokens, tokens + done, size_t(T) * sizeof(int), cudaMemcpyHostToDevice, p.stream), "copy tokens");
         auto enqueue_chunk = [&] {
@@ -871,7 +874,7 @@ void Qwen35Decode::forward_tokens(const int *tokens, int count)
                 }
             }
         };
-        if (!use_umma && T == kChunk && x_.options.use_graph && p.chunk_warm) {
+        if (!one_layout && !use_umma && T == kChunk && x_.options.use_graph && p.chunk_warm) {
             // full chunks replay one graph (tokens and position are read from device memory); the first full chunk ran
             // eagerly (first launches of a kernel variant set function attributes)
             const uint64_t before = launches_;
@@ -895,7 +898,7 @@ void Qwen35Decode::forward_tokens(const int *tokens, int count)
             cuda_check(cudaGraphLaunch(p.exec_chunk, p.stream), "launch graph");
         } else {
             enqueue_chunk();
-            p.chunk_warm |= !use_umma && T == kChunk;
+            p.chunk_warm |= !one_layout && !use_umma && T == kChunk;
         }
         x_.position += T;
         done += T;
@@ -1125,7 +1128,7 @@ int Qwen35Decode::mtp_step(int token, bool draft)
     Plan &p = plan();
     const std::string m = std::string(kLM) + ".mtp";
     if (!p.mtp_ready) {
-        Loader L{w_, p.pinned, x_.options.gemv_tcgen05 ? 1 : 0};
+        Loader L{w_, p.pinned, tcgen05_engine(x_.options) ? 1 : 0};
         p.mtp_fc = L.bf16(m + ".fc.weight", size_t(kHidden) * 2 * kHidden);
         p.mtp_norm_e = L.bf16(m + ".pre_fc_norm_embedding.weight", kHidden);
         p.mtp_norm_h = L.bf16(m + ".pre_fc_norm_hidden.weight", kHidden);
@@ -1191,7 +1194,6 @@ std::vector<int> Qwen35Decode::generate_speculative(int first_token, int count, 
     if (count <= 0) return out;
     if (first_token < 0 || first_token >= Qwen35Shape::vocab) throw std::runtime_error("token out of range");
     if (x_.position + count > x_.max_context) throw std::runtime_error("KV cache full");
-    if (x_.options.gemv_tcgen05) throw std::runtime_error("speculative decode runs on the mma.sync weight layout");
     Plan &p = plan();
     const int n = x_.options.n_layers;
     for (int l = 0; l < n; l++) load_block(l);
@@ -1206,7 +1208,6 @@ std::vector<int> Qwen35Decode::generate_speculative(int first_token, int count, 
         cuda_check(cudaMallocHost(&p.spec_host, 4 * sizeof(int)), "cudaMallocHost");
     }
     Ctx c{x_, p.stream, x_.options.use_pdl, launches_, false, nullptr, nullptr};
-    c.layout = 0;
     float *cur = x_.delta_state, *alt = p.spec_state;
     int tok = first_token, hits = 0;
     out.reserve(size_t(count));
