@@ -65,4 +65,20 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t b
                  ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 
+// ---- tcgen05 instructions as the kernels issue them ----
+__device__ __forceinline__ void copy_scales(uint32_t taddr, uint64_t desc)
+{
+    asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(desc) : "memory");
+}
+__device__ __forceinline__ void mma_step(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, bool accumulate, uint32_t sa, uint32_t sb)
+{
+    asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %4, 0;\n"
+                 "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%5], [%6], q;\n}"
+                 ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"(uint32_t(accumulate)), "r"(sa), "r"(sb) : "memory");
+}
+__device__ __forceinline__ void commit_to(uint64_t *bar)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 } // namespace insg

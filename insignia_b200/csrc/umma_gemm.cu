@@ -40,7 +40,7 @@ namespace insg {
 constexpr int kGThreads = kProThreads;     // digitize kernel: the activation prologue is written for this many threads
 constexpr int kGemmThreads = 192;          // GEMM kernel: four epilogue warps, the MMA issuer, the producer
 constexpr int kDigits = 8;                 // balanced base-9 digits per activation = N columns per token
-constexpr int kGSfaBufs = 8;               // scale-factor column sets cycled by k-block
+constexpr int kGSfaBufs = 8;               // scale-factor column sets cycled by stage (a power of two)
 constexpr int kGTmemCols = 512;            // accumulators [0,256), weight scale factors [256,320), digit scale factors [320,324)
 constexpr int kGMaxStages = 16;
 constexpr int kGMaxGrid = 256;             // partial-sum slots and tickets are sized for this many CTAs
@@ -77,7 +77,7 @@ struct GParams {
     const float *inv_alpha; // [ngroups * tpg]
     float *partials;        // [grid][2 cut units][2 matrices][2 tiles][128 rows][tpg]
     int *tickets;           // [grid], zero between launches
-    int nkb, nseg, total_tiles, stages, ngroups, tokens, sfa_lookahead, tpg, nmat;
+    int nkb, nseg, total_tiles, stages, ngroups, tokens, tpg, nmat;
     int total_stages, share, share_rem; // CTA c owns stages [share * c + share_rem * c / G, ...): all products stay in 32 bits
     GSeg seg[4];
     int *error_flag;
@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
     // weights' scale factors at [256, 320) (8 k-blocks x 2 tiles x 4 columns), the digits' (all 1) at [320, 324).
     constexpr int NB = TPG == 8 ? 2 : 1;
     constexpr uint32_t kSfaCol = 256, kSfbCol = 320;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int nkb = p.nkb, S = p.stages;
     uint8_t *ring = smem;                          // S stages of kGStage bytes
     uint8_t *sfb = ring + size_t(S) * kGStage;     // 512 bytes
@@ -439,23 +439,30 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
         asm volatile("griddepcontrol.wait;" ::: "memory");
         if (tid == 160) GEMM_STAMP(3);
         if (lane < first) bulk_load(dst0 + 2 * kURec, b0, kBBlock, &full[lane]);
-        if (lane == 0) {
-            int g = begin + first, i = first;
-            bool ok = true;
+        {   // from here on the whole warp walks the loop and one elected lane issues: warp-uniform operands issue twice as fast
+            const bool one = elect_one();
+            int g = begin + first, st = first == S ? 0 : first;
+            uint32_t phase = 0; // of the empty barriers
+            bool ok = true, room = g < end && mbar_test(&empty[st], phase);
             while (g < end && ok) {
                 const GRun r = run_at(p, g, end);
                 const int pair = r.unit / p.ngroups, grp = r.unit - pair * p.ngroups;
                 const PairSrc q = pair_src(p, pair, r.mat, r.kb0);
-                const uint8_t *b_src = p.bimg + (size_t(r.kb0) * p.ngroups + grp) * kBBlock;
+                const uint8_t *a0 = q.a0, *a1 = q.a1, *b = p.bimg + (size_t(r.kb0) * p.ngroups + grp) * kBBlock;
+                const size_t bstep = size_t(p.ngroups) * kBBlock;
                 const uint32_t bytes = (q.has1 ? 2 : 1) * kURec + kBBlock;
-                for (int k = 0; k < r.len; k++, i++) {
-                    const int st = i % S;
-                    if (!mbar_wait(&empty[st], ((i / S) - 1) & 1, abort_flag)) { ok = false; break; }
-                    uint8_t *dst = ring + size_t(st) * kGStage;
-                    mbar_expect_tx(&full[st], bytes);
-                    bulk_load(dst, q.a0 + size_t(k) * kURec, kURec, &full[st]);
-                    if (q.has1) bulk_load(dst + kURec, q.a1 + size_t(k) * kURec, kURec, &full[st]);
-                    bulk_load(dst + 2 * kURec, b_src + size_t(k) * p.ngroups * kBBlock, kBBlock, &full[st]);
+                for (int k = 0; k < r.len; k++, a0 += kURec, a1 += kURec, b += bstep) {
+                    if (!room && !mbar_wait(&empty[st], phase, abort_flag)) { ok = false; break; }
+                    const int cur = st;
+                    if (++st == S) { st = 0; phase ^= 1; }
+                    room = mbar_test(&empty[st], phase);
+                    if (one) {
+                        uint8_t *dst = ring + size_t(cur) * kGStage;
+                        mbar_expect_tx(&full[cur], bytes);
+                        bulk_load(dst, a0, kURec, &full[cur]);
+                        if (q.has1) bulk_load(dst + kURec, a1, kURec, &full[cur]);
+                        bulk_load(dst + 2 * kURec, b, kBBlock, &full[cur]);
+                    }
                 }
                 g += r.len;
             }
@@ -463,67 +470,52 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
         }
     } else if (warp == 4) {
         // ---- MMA issuer --------------------------------------------------------------------------------------------------
-        if (lane == 0) {
-            asm volatile("griddepcontrol.wait;" ::: "memory");
-            // E2M1 x E2M1, UE8M0 scales, N columns, M = 128
-            const uint32_t idesc_base = (1u << 7) | (1u << 10) | ((uint32_t(N) >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
-            asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem + kSfbCol), "l"(umma_desc(smem_u32(sfb), 16, 128)));
-            // The scale-factor copies of a k-block are issued `la` k-blocks ahead of its MMAs: the tensor pipe runs its
-            // work in order, and a copy placed right in front of the MMAs that need it puts its whole latency on the chain.
-            // (A missing second tile's copy and MMAs read ring bytes nobody wrote; their results are never looked at.)
-            const int la = p.sfa_lookahead;
-            int i = 0, j = 0; // next stage to multiply, next stage whose scale factors are copied
-            bool ok = true;
-            auto copy_scales = [&](int upto) {
-                for (; j <= upto && j < total_kb && ok; j++) {
-                    const int st = j % S;
-                    ok = mbar_wait(&full[st], (j / S) & 1, abort_flag);
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t sbase = smem_u32(ring + size_t(st) * kGStage);
-#pragma unroll
-                    for (int h = 0; h < 2; h++)
-                        asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem + kSfaCol + 8 * (j % kGSfaBufs) + 4 * h),
-                                     "l"(umma_desc(sbase + h * kURec + 8192, 16, 128)));
-                }
-            };
-            int g = begin;
-            for (int run = 0; g < end && ok; run++) {
-                const GRun r = run_at(p, g, end);
-                const bool has1 = 2 * (r.unit / p.ngroups) + 1 < p.total_tiles;
-                const int buf = run % NB;
-                ok = mbar_wait(&dempty[buf], ((run / NB) & 1) ^ 1, abort_flag); // first use of each set passes at once
-                if (!ok) break;
+        // The whole warp walks the loop and one elected lane issues (see umma_gemv.cu: operands in uniform registers); the next
+        // stage's barrier is polled before this stage's multiplies go out.
+        const bool one = elect_one();
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        // E2M1 x E2M1, UE8M0 scales, N columns, M = 128; K-step s of a block uses the weight scale bytes 2s, 2s+1 and byte 0 of the digits' (all equal)
+        constexpr uint32_t idesc0 = (1u << 7) | (1u << 10) | ((uint32_t(N) >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
+        constexpr uint32_t idesc1 = idesc0 | (2u << 29);
+        if (one) copy_scales(tmem + kSfbCol, umma_desc(smem_u32(sfb), 16, 128));
+        const uint64_t da0 = umma_desc(smem_u32(ring), 128, 256), dsf0 = umma_desc(smem_u32(ring) + 8192, 16, 128);
+        // (A missing second tile's copy and MMAs read ring bytes nobody wrote; their results are never looked at.)
+        int st = 0, sfa = 0;
+        uint32_t phase = 0;
+        bool ok = true, here = mbar_test(&full[0], 0);
+        int g = begin;
+        for (int run = 0; g < end && ok; run++) {
+            const GRun r = run_at(p, g, end);
+            const bool has1 = 2 * (r.unit / p.ngroups) + 1 < p.total_tiles;
+            const int buf = run % NB;
+            ok = mbar_wait(&dempty[buf], ((run / NB) & 1) ^ 1, abort_flag); // first use of each set passes at once
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t d0 = tmem + uint32_t(buf * 2 * N), d1 = d0 + uint32_t(N);
+            for (int k = 0; k < r.len; k++) {
+                if (!here && !mbar_wait(&full[st], phase, abort_flag)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int k = 0; k < r.len; k++, i++) {
-                    copy_scales(i + la);
-                    if (!ok) break;
-                    if (i == 0) GEMM_STAMP(5);
-                    const int st = i % S;
-                    const uint32_t sbase = smem_u32(ring + size_t(st) * kGStage);
-#pragma unroll
-                    for (int s = 0; s < 2; s++) {
-                        const uint64_t db = umma_desc(sbase + 2 * kURec + s * (kBBlock / 2), 128, 256);
-                        const uint32_t idesc = idesc_base | (uint32_t(2 * s) << 29); // A scales: bytes 2s, 2s+1; B scales: byte 0 (all equal)
-                        const uint32_t acc = (k > 0 || s > 0) ? 1u : 0u;             // the run's first MMA overwrites
-#pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            if (h == 1 && !has1) break;
-                            const uint64_t da = umma_desc(sbase + h * kURec + s * 4096, 128, 256);
-                            asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %4, 0;\n"
-                                         "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%5], [%6], q;\n}"
-                                         ::"r"(tmem + uint32_t((buf * 2 + h) * N)), "l"(da), "l"(db), "r"(idesc), "r"(acc),
-                                           "r"(tmem + kSfaCol + 8 * (i % kGSfaBufs) + 4 * h), "r"(tmem + kSfbCol)
-                                         : "memory");
-                        }
-                    }
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&empty[st])) : "memory");
+                const uint64_t off = uint64_t(uint32_t(st) * uint32_t(kGStage >> 4));
+                const uint64_t da = da0 + off, dsf = dsf0 + off, db = da + uint64_t((2 * kURec) >> 4);
+                const uint32_t sa = tmem + kSfaCol + 8 * sfa;
+                const int cur = st;
+                if (++st == S) { st = 0; phase ^= 1; }
+                here = mbar_test(&full[st], phase);
+                if (one) {
+                    copy_scales(sa, dsf);
+                    if (has1) copy_scales(sa + 4, dsf + (kURec >> 4));
+                    mma_step(d0, da, db, idesc0, k > 0, sa, tmem + kSfbCol); // the run's first MMA overwrites
+                    if (has1) mma_step(d1, da + (kURec >> 4), db, idesc0, k > 0, sa + 4, tmem + kSfbCol);
+                    mma_step(d0, da + 256, db + (kBBlock >> 5), idesc1, true, sa, tmem + kSfbCol);
+                    if (has1) mma_step(d1, da + (kURec >> 4) + 256, db + (kBBlock >> 5), idesc1, true, sa + 4, tmem + kSfbCol);
+                    commit_to(&empty[cur]);
                 }
-                if (ok) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&dfull[buf])) : "memory");
-                g += r.len;
+                sfa = (sfa + 1) & (kGSfaBufs - 1);
             }
-            GEMM_STAMP(6);
+            if (ok && one) commit_to(&dfull[buf]);
+            g += r.len;
         }
+        GEMM_STAMP(6);
     } else if (warp < 4) {
         // ---- epilogue: tensor-memory lane = row of the tile; token t of the group = columns 8t .. 8t+7 --------------------
         float gate_val[NMAT == 2 ? 2 : 1][NMAT == 2 ? TPG : 1], zero[TPG];
@@ -674,7 +666,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
 namespace {
 std::mutex g_gemm_attr_mutex;
 bool g_gemm_attr_done[64] = {false}; // the shared-memory opt-in is a per-device function attribute
-constexpr int kGemmLookahead = 4; // k-blocks the scale-factor copies run ahead of the MMAs (0, 1, 2, 4, 6 measured alike within 2 %)
 
 int tokens_per_group(int tokens) { return tokens <= 8 ? 8 : 16; }
 size_t image_bytes(int cols, int tokens)
@@ -762,7 +753,6 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     p.error_flag = op->error_flag;
     const int stage_bytes = 2 * kURec + 512 * tpg;
     p.stages = std::min(kGMaxStages, (224 * 1024 - 512) / stage_bytes);
-    p.sfa_lookahead = std::max(0, std::min(kGemmLookahead, kGSfaBufs - 2));
     const size_t smem = size_t(p.stages) * stage_bytes + 512;
     auto kernel = tpg == 8 ? (nmat_all == 2 ? umma_gemm_kernel<8, 2> : umma_gemm_kernel<8, 1>) : (nmat_all == 2 ? umma_gemm_kernel<16, 2> : umma_gemm_kernel<16, 1>);
     {
