@@ -504,6 +504,9 @@ template <bool BF16> __global__ void __launch_bounds__(kAtThreads) attn_chunk_pr
 
 size_t attn_scratch_bytes() { return 64 + size_t(4) * kSplits * kPartFloats * sizeof(float); }
 
+int attn_tile_launch(const AttnParams &p, const float *qn, int tokens, bool bf16, cudaStream_t st, bool pdl);
+constexpr int kTileFromTokens = 32;
+
 int attn_plain_launch(const float *q, const void *kc, const void *vc, float *out, int tokens, int kv_dtype, void *scratch,
                       cudaStream_t st)
 {
@@ -589,6 +592,9 @@ int insg_attention_chunk(const insg_attn_op *op, int tokens, float *q_scratch, i
     int rc = bf16 ? launch(attn_chunk_prepare_kernel<true>, dim3(tokens), dim3(kAtThreads), 0, stream, false, p, q_scratch)
                   : launch(attn_chunk_prepare_kernel<false>, dim3(tokens), dim3(kAtThreads), 0, stream, false, p, q_scratch);
     if (rc != INSG_OK) return rc;
+    // More than 32 tokens: query tiles on the tensor cores.  Fewer: the token-by-token form below, whose results are those of
+    // single steps bit for bit (at 33 tokens the tile kernel still has only twelve CTAs; the two take the same time near 24).
+    if (tokens > kTileFromTokens) return attn_tile_launch(p, q_scratch, tokens, bf16, stream, false);
     // step two: every (kv head, split, token) CTA is the plain split-K decode of its token over the rows up to its own
     p.q = q_scratch; p.q_stride = 4096; p.out_stride = 4096; p.scratch_stride = attn_scratch_bytes();
     p.counters = static_cast<unsigned *>(op->scratch);

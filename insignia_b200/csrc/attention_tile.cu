@@ -1,0 +1,348 @@
+// Attention of a prompt pass on the tensor cores: tiles of query tokens against tiles of cached rows (sm_100a).
+//
+// Math (reference: src/attention.cu:4, once per token): score_t = (q_h . K[t][h>>2]) / 16 over the rows up to the token's own,
+// softmax, out_h = sum_t p_t V[t][h>>2].  The split-K decode kernel (attention.cu) streams the whole cache once per token; a
+// pass of hundreds of tokens reads the same rows hundreds of times (2048 tokens: 79 ms of a 192 ms prompt).  Here a CTA takes
+// one kv head and 16 consecutive tokens = 64 query rows (row = token * 4 + query head of the group), walks the cached rows
+// in tiles of 32 and keeps an online softmax: every row fetched serves 64 query rows.
+//
+// Precision: the products run on mma.sync.m16n8k16 (fp16 in, fp32 accumulate).  Every fp32 operand is scaled by a power of two
+// that puts the largest element of its tile in [2^12, 2^13) and cut into two fp16 pieces hi + lo (22 bits and more of it);
+// the products hi*hi + hi*lo + lo*hi are accumulated, the missing lo*lo is below 2^-22 of the result.  A bf16 cache needs one
+// piece (8 significant bits fit fp16 exactly).  The value tiles share one running scale, so that the output accumulators are
+// rescaled (with the softmax correction, by a power of two) when a tile brings a larger element.
+//
+// Eight warps: warp & 3 = 16 of the query rows, warp >> 2 = which half of the 32 keys; the two halves are merged at the end.
+// Per tile of 32 keys a warp issues 96 + 96 MMAs (fp32 cache) and reads 48 KB of fragments from shared memory: the two are
+// about equal, which is what bounds it.  Rows of 528 bytes keep ldmatrix free of bank conflicts.
+#include "attention_body.cuh"
+#include "host_util.h"
+
+#include <mutex>
+
+namespace insg {
+
+constexpr int kTileTokens = 16, kTileRows = 4 * kTileTokens, kTileKeys = 32;
+constexpr int kTThreads = 256;
+constexpr int kPitch = 528; // bytes per row of fp16 pieces: 512 + 16
+
+template <bool BF16> struct TileSmem {
+    static constexpr int pieces = BF16 ? 1 : 2;                                // of keys and values
+    static constexpr int raw_row = BF16 ? 512 : 1024;                          // bytes of a cached row of one kv head
+    static constexpr int q = 0;                                                // [2][64] rows
+    static constexpr int k = q + 2 * kTileRows * kPitch;                       // [pieces][32] rows
+    static constexpr int v = k + pieces * kTileKeys * kPitch;                  // [pieces][32] rows
+    static constexpr int raw = v + pieces * kTileKeys * kPitch;                // [K, V][32] rows as cached
+    static constexpr int bytes = raw + 2 * kTileKeys * raw_row;
+    // the merge of the two key halves reuses the front: four warps x 16 rows x 256 floats
+    static_assert(bytes >= 4 * 16 * 256 * 4, "merge buffer");
+};
+
+__device__ __forceinline__ uint32_t saddr32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], uint32_t addr)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
+{
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// hi and lo fp16 pieces of two scaled values
+__device__ __forceinline__ void split2(float a, float b, uint32_t &hi, uint32_t &lo)
+{
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
+    hi = *reinterpret_cast<const uint32_t *>(&h);
+    lo = *reinterpret_cast<const uint32_t *>(&l);
+}
+// Biased exponent of a tile's largest magnitude, kept where both 2^(12 - e) and its inverse are normal numbers.
+__device__ __forceinline__ int tile_exponent(uint32_t max_bits) { return min(max(int(max_bits >> 23), 24), 230); }
+__device__ __forceinline__ float scale_up(int e) { return __uint_as_float(uint32_t(127 + 12 + 127 - e) << 23); }   // 2^(12 - (e - 127))
+__device__ __forceinline__ float scale_down(int e) { return __uint_as_float(uint32_t(e - 12) << 23); }             // its inverse
+
+template <bool BF16>
+__global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_constant__ AttnParams p, const float *__restrict__ qn, int tokens)
+{
+    using L = TileSmem<BF16>;
+    extern __shared__ __align__(128) uint8_t sm[];
+    __shared__ uint32_t s_max[3][2]; // largest magnitude bits of [tile buffer][K, V]; [2][0]: the query rows
+    __shared__ float s_ml[4][2][16];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int kvh = blockIdx.x, q0 = (int(gridDim.y) - 1 - int(blockIdx.y)) * kTileTokens; // the longest rows first
+    const int rg = warp & 3, kg = warp >> 2, g = lane >> 2, t = lane & 3;
+
+    pdl_launch_dependents();
+    if (tid < 6) s_max[tid >> 1][tid & 1] = 0u;
+    pdl_wait();
+    __syncthreads();
+    const int pos0 = __ldcg(p.position) + p.position_offset;
+    if (pos0 < 0 || pos0 + tokens > p.max_context) return; // the prepare kernel refuses the same
+    const int nkeys = pos0 + min(q0 + kTileTokens, tokens); // rows the tile's last token attends
+    const int ntiles = (nkeys + kTileKeys - 1) / kTileKeys;
+
+    auto fetch = [&](int tile) { // both raw tiles of 32 cached rows by 16-byte asynchronous copies; rows past the end repeat the last
+        constexpr int per_row = L::raw_row / 16;
+        for (int i = tid; i < 2 * kTileKeys * per_row; i += kTThreads) {
+            const int kv = i / (kTileKeys * per_row), r = (i / per_row) % kTileKeys, c = i % per_row;
+            const int row = min(tile * kTileKeys + r, nkeys - 1);
+            const uint8_t *src = static_cast<const uint8_t *>(kv ? p.vc : p.kc) + (size_t(row) * 4 + kvh) * L::raw_row + c * 16;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(saddr32(sm + L::raw + (kv * kTileKeys + r) * L::raw_row + c * 16)), "l"(src) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0);
+
+    // ---- query rows: scaled by 1/16 and the tile's power of two, two pieces ----
+    float invq;
+    {
+        uint32_t mx = 0;
+        for (int i = tid; i < kTileRows * 64; i += kTThreads) {
+            const int r = i >> 6, c = i & 63, tok = q0 + (r >> 2);
+            if (tok < tokens) {
+                const float4 x = __ldcg(reinterpret_cast<const float4 *>(qn + (size_t(tok) * 16 + kvh * 4 + (r & 3)) * 256) + c);
+                mx = max(mx, __float_as_uint(fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w)))));
+            }
+        }
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        if (lane == 0) atomicMax(&s_max[2][0], mx);
+        __syncthreads();
+        const int e = tile_exponent(s_max[2][0]);
+        const float up = scale_up(e);
+        invq = scale_down(e) * 0.0625f;
+        for (int i = tid; i < kTileRows * 64; i += kTThreads) {
+            const int r = i >> 6, c = i & 63, tok = q0 + (r >> 2);
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (tok < tokens) x = __ldcg(reinterpret_cast<const float4 *>(qn + (size_t(tok) * 16 + kvh * 4 + (r & 3)) * 256) + c);
+            uint2 hi, lo;
+            split2(x.x * up, x.y * up, hi.x, lo.x);
+            split2(x.z * up, x.w * up, hi.y, lo.y);
+            *reinterpret_cast<uint2 *>(sm + L::q + r * kPitch + c * 8) = hi;
+            *reinterpret_cast<uint2 *>(sm + L::q + (kTileRows + r) * kPitch + c * 8) = lo;
+        }
+    }
+
+    float o[32][4]; // [8 dims each][row g: dims 2t, 2t+1 | row g + 8: dims 2t, 2t+1]
+#pragma unroll
+    for (int j = 0; j < 32; j++) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
+    float m_run[2] = {-3.0e38f, -3.0e38f}, l_run[2] = {0.f, 0.f}; // rows g and g + 8 (l as this thread's partial sum)
+    int ev = 24;                                                  // exponent of the running value scale
+    const int limit0 = pos0 + q0 + ((rg * 16 + g) >> 2), limit1 = pos0 + q0 + ((rg * 16 + g + 8) >> 2); // last row each query row sees
+    const uint32_t qaddr = saddr32(sm + L::q) + (rg * 16 + (lane & 15)) * kPitch + (lane >> 4) * 16;
+    const uint32_t kaddr = saddr32(sm + L::k) + (kg * 16 + ((lane >> 4) & 1) * 8 + (lane & 7)) * kPitch + ((lane >> 3) & 1) * 16;
+    const uint32_t vaddr = saddr32(sm + L::v) + (kg * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * kPitch + ((lane >> 4) & 1) * 16;
+
+    for (int tile = 0; tile < ntiles; tile++) {
+        const int buf = tile & 1;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads(); // the raw tile is complete; everybody is done with the previous tile's pieces and maxima
+        // ---- largest magnitudes of the two raw tiles ----
+        if (tid < 2) s_max[buf ^ 1][tid] = 0u;
+        constexpr int per = 2 * kTileKeys * L::raw_row / 16 / kTThreads; // 16-byte cells per thread, the first half keys
+        uint4 cell[per];
+#pragma unroll
+        for (int i = 0; i < per; i++) cell[i] = *reinterpret_cast<const uint4 *>(sm + L::raw + (tid + i * kTThreads) * 16);
+#pragma unroll
+        for (int kv = 0; kv < 2; kv++) {
+            uint32_t mx = 0;
+#pragma unroll
+            for (int i = kv * per / 2; i < (kv + 1) * per / 2; i++) {
+                const uint32_t w[4] = {cell[i].x, cell[i].y, cell[i].z, cell[i].w};
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    if (BF16) mx = max(mx, max((w[q] << 16) & 0x7fffffffu, w[q] & 0x7fff0000u));
+                    else mx = max(mx, w[q] & 0x7fffffffu);
+                }
+            }
+            mx = __reduce_max_sync(0xffffffffu, mx);
+            if (lane == 0) atomicMax(&s_max[buf][kv], mx);
+        }
+        __syncthreads(); // maxima complete, the raw tile is in registers
+        if (tile + 1 < ntiles) fetch(tile + 1);
+        const int ek = tile_exponent(s_max[buf][0]), ev_new = max(ev, tile_exponent(s_max[buf][1]));
+        const float fv = __uint_as_float(uint32_t(max(127 + ev - ev_new, 0)) << 23); // rescales what was accumulated so far
+        ev = ev_new;
+        {
+            const float up[2] = {scale_up(ek), scale_up(ev)};
+#pragma unroll
+            for (int i = 0; i < per; i++) {
+                const int at = tid + i * kTThreads, kv = i >= per / 2;
+                if (BF16) { // eight values of one row
+                    const int r = (at >> 5) & 31, c = at & 31;
+                    const uint32_t w[4] = {cell[i].x, cell[i].y, cell[i].z, cell[i].w};
+                    uint32_t h[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        const __half2 x = __floats2half2_rn(__uint_as_float(w[q] << 16) * up[kv], __uint_as_float(w[q] & 0xffff0000u) * up[kv]);
+                        h[q] = *reinterpret_cast<const uint32_t *>(&x);
+                    }
+                    *reinterpret_cast<uint4 *>(sm + (kv ? L::v : L::k) + r * kPitch + c * 16) = make_uint4(h[0], h[1], h[2], h[3]);
+                } else { // four values of one row
+                    const int r = (at >> 6) & 31, c = at & 63;
+                    uint2 hi, lo;
+                    split2(__uint_as_float(cell[i].x) * up[kv], __uint_as_float(cell[i].y) * up[kv], hi.x, lo.x);
+                    split2(__uint_as_float(cell[i].z) * up[kv], __uint_as_float(cell[i].w) * up[kv], hi.y, lo.y);
+                    uint8_t *dst = sm + (kv ? L::v : L::k) + r * kPitch + c * 8;
+                    *reinterpret_cast<uint2 *>(dst) = hi;
+                    *reinterpret_cast<uint2 *>(dst + kTileKeys * kPitch) = lo;
+                }
+            }
+        }
+        __syncthreads(); // the pieces are complete
+        const int key0 = tile * kTileKeys + kg * 16;
+        if (key0 < nkeys) { // warp-uniform; a half tile past the last row has nothing to add
+            // ---- scores of 16 rows x 16 keys ----
+            float s[2][4];
+#pragma unroll
+            for (int n = 0; n < 2; n++) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
+#pragma unroll 4
+            for (int i = 0; i < 16; i++) {
+                uint32_t qh[4], ql[4], kh[4];
+                ldsm4(qh, qaddr + 32 * i);
+                ldsm4(ql, qaddr + kTileRows * kPitch + 32 * i);
+                ldsm4(kh, kaddr + 32 * i);
+                mma_f16(s[0], qh, kh[0], kh[1]);
+                mma_f16(s[1], qh, kh[2], kh[3]);
+                mma_f16(s[0], ql, kh[0], kh[1]);
+                mma_f16(s[1], ql, kh[2], kh[3]);
+                if (!BF16) {
+                    uint32_t kl[4];
+                    ldsm4(kl, kaddr + kTileKeys * kPitch + 32 * i);
+                    mma_f16(s[0], qh, kl[0], kl[1]);
+                    mma_f16(s[1], qh, kl[2], kl[3]);
+                }
+            }
+            // ---- online softmax (rows g and g + 8; a row's 16 keys sit in the four lanes of a quad) ----
+            const float sc = invq * scale_down(ek);
+            float pr[2][4], corr[2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int limit = h ? limit1 : limit0;
+                float mx = -3.0e38f;
+#pragma unroll
+                for (int n = 0; n < 2; n++)
+#pragma unroll
+                    for (int c = 0; c < 2; c++) {
+                        const float x = s[n][2 * h + c] * sc;
+                        s[n][2 * h + c] = x;
+                        if (key0 + n * 8 + 2 * t + c <= limit) mx = fmaxf(mx, x);
+                    }
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+                const float m_new = fmaxf(m_run[h], mx);
+                corr[h] = __expf(m_run[h] - m_new);
+                m_run[h] = m_new;
+                float sum = 0.f;
+#pragma unroll
+                for (int n = 0; n < 2; n++)
+#pragma unroll
+                    for (int c = 0; c < 2; c++) {
+                        const float e = key0 + n * 8 + 2 * t + c <= limit ? __expf(s[n][2 * h + c] - m_new) : 0.f;
+                        pr[n][2 * h + c] = e * 4096.f;
+                        sum += e;
+                    }
+                l_run[h] = fmaf(l_run[h], corr[h], sum);
+            }
+            uint32_t ph[4], pl[4]; // the weights as the A operand: keys as k
+            split2(pr[0][0], pr[0][1], ph[0], pl[0]);
+            split2(pr[0][2], pr[0][3], ph[1], pl[1]);
+            split2(pr[1][0], pr[1][1], ph[2], pl[2]);
+            split2(pr[1][2], pr[1][3], ph[3], pl[3]);
+            const float c0 = corr[0] * fv, c1 = corr[1] * fv;
+            // ---- values ----
+#pragma unroll
+            for (int j = 0; j < 16; j++) { // 16 dims each
+                uint32_t vh[4];
+                ldsm4t(vh, vaddr + 32 * j);
+#pragma unroll
+                for (int n = 0; n < 2; n++) {
+                    float (&a)[4] = o[2 * j + n];
+                    a[0] *= c0; a[1] *= c0; a[2] *= c1; a[3] *= c1;
+                    mma_f16(a, ph, vh[2 * n], vh[2 * n + 1]);
+                    mma_f16(a, pl, vh[2 * n], vh[2 * n + 1]);
+                }
+                if (!BF16) {
+                    uint32_t vl[4];
+                    ldsm4t(vl, vaddr + kTileKeys * kPitch + 32 * j);
+                    mma_f16(o[2 * j], ph, vl[0], vl[1]);
+                    mma_f16(o[2 * j + 1], ph, vl[2], vl[3]);
+                }
+            }
+        } else if (fv != 1.f) {
+#pragma unroll
+            for (int j = 0; j < 32; j++) { o[j][0] *= fv; o[j][1] *= fv; o[j][2] *= fv; o[j][3] *= fv; }
+        }
+    }
+    // ---- merge the two key halves and write the rows ----
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 1);
+        l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 2);
+    }
+    __syncthreads(); // the pieces are no longer needed
+    float2 *merge = reinterpret_cast<float2 *>(sm) + size_t(rg) * 32 * 64; // [j][2 rows][lane]
+    if (kg == 1) {
+#pragma unroll
+        for (int j = 0; j < 32; j++) {
+            merge[(2 * j) * 32 + lane] = make_float2(o[j][0], o[j][1]);
+            merge[(2 * j + 1) * 32 + lane] = make_float2(o[j][2], o[j][3]);
+        }
+        if (t == 0) {
+            s_ml[rg][0][g] = m_run[0]; s_ml[rg][0][g + 8] = m_run[1];
+            s_ml[rg][1][g] = l_run[0]; s_ml[rg][1][g + 8] = l_run[1];
+        }
+    }
+    __syncthreads();
+    if (kg == 0) {
+        const float inv_v = scale_down(ev) * (1.f / 4096.f);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int r = rg * 16 + g + 8 * h, tok = q0 + (r >> 2);
+            const float mb = s_ml[rg][0][g + 8 * h], lb = s_ml[rg][1][g + 8 * h];
+            const float mg = fmaxf(m_run[h], mb), ea = __expf(m_run[h] - mg), eb = lb > 0.f ? __expf(mb - mg) : 0.f;
+            const float inv = inv_v / fmaf(l_run[h], ea, lb * eb);
+            if (tok < tokens) {
+                float *dst = p.out + (size_t(tok) * 16 + kvh * 4 + (r & 3)) * 256 + 2 * t;
+#pragma unroll
+                for (int j = 0; j < 32; j++) {
+                    const float2 b = merge[(2 * j + h) * 32 + lane];
+                    *reinterpret_cast<float2 *>(dst + 8 * j) =
+                        make_float2(fmaf(o[j][2 * h], ea, b.x * eb) * inv, fmaf(o[j][2 * h + 1], ea, b.y * eb) * inv);
+                }
+            }
+        }
+    }
+}
+
+template <bool BF16> static int launch_tile(const AttnParams &p, const float *qn, int tokens, cudaStream_t st, bool pdl)
+{
+    static std::mutex mu;
+    static bool done[64] = {false};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
+    if (dev < 0 || dev >= 64) return fail(INSG_E_LIMIT, "attention: device ordinal beyond 63");
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!done[dev]) {
+            e = cudaFuncSetAttribute(attn_tile_kernel<BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, TileSmem<BF16>::bytes);
+            if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(attention tiles)");
+            done[dev] = true;
+        }
+    }
+    return launch(attn_tile_kernel<BF16>, dim3(4, (tokens + kTileTokens - 1) / kTileTokens), dim3(kTThreads), TileSmem<BF16>::bytes, st, pdl, p, qn, tokens);
+}
+
+// p: the caches, the device position and the output rows; qn [tokens][16][256]: the normalised, rotated queries.
+int attn_tile_launch(const AttnParams &p, const float *qn, int tokens, bool bf16, cudaStream_t st, bool pdl)
+{
+    return bf16 ? launch_tile<true>(p, qn, tokens, st, pdl) : launch_tile<false>(p, qn, tokens, st, pdl);
+}
+
+} // namespace insg

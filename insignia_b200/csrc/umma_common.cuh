@@ -1,6 +1,6 @@
 // Helpers shared by the tcgen05 kernels (umma_gemv.cu: one to eight tokens, activation image resident in shared memory;
 // umma_gemm.cu: more tokens, activation image streamed): shared-memory descriptors, mbarrier waits with a bound,
-// and bulk copies.
+// bulk copies, the tcgen05 instructions, and the split of an fp32 activation into exact E2M1 digits.
 #pragma once
 #include "common.cuh"
 
@@ -79,6 +79,44 @@ __device__ __forceinline__ void mma_step(uint32_t d, uint64_t da, uint64_t db, u
 __device__ __forceinline__ void commit_to(uint64_t *bar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// Eight balanced base-9 digits of round(x * alpha) (|.| < 2^24) as E2M1 codes, digit j in nibble j.  u = v + 4 * (9^8 - 1) / 8
+// has plain base-9 digits 0..8 (the balanced digit + 4); they are taken in pairs (base 81) through an 81-byte table, which
+// costs a third of the instructions of eight divisions by 9.
+__device__ __forceinline__ uint32_t digit_codes81(float x, float alpha, const uint8_t *lut)
+{
+    const int v = max(-0xFFFFFF, min(__float2int_rn(x * alpha), 0xFFFFFF));
+    const uint32_t u = uint32_t(v + 21523360);
+    const uint32_t hi = u / 6561u, lo = u - 6561u * hi;
+    const uint32_t h1 = (hi * 6473u) >> 19, h0 = hi - 81u * h1; // n / 81 for n < 6562 (6473 / 2^19 = 1/81 + 1.7e-7)
+    const uint32_t l1 = (lo * 6473u) >> 19, l0 = lo - 81u * l1;
+    return uint32_t(lut[l0]) | (uint32_t(lut[l1]) << 8) | (uint32_t(lut[h0]) << 16) | (uint32_t(lut[h1]) << 24);
+}
+__device__ __forceinline__ uint8_t digit_pair_code(int n) // table entry: digits n % 9 - 4 (low nibble) and n / 9 - 4 (high nibble)
+{
+    uint32_t r = 0;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int d = (h ? n / 9 : n % 9) - 4, mag = d < 0 ? -d : d; // 0..4 -> E2M1 codes 0, 2, 4, 5, 6
+        r |= uint32_t((mag < 3 ? 2 * mag : mag + 2) | (d < 0 ? 8 : 0)) << (4 * h);
+    }
+    return uint8_t(r);
+}
+
+// The digits of four consecutive elements: two bytes in each of the eight digit columns (16 bytes apart) from `base` on.
+__device__ __forceinline__ void pack_digits(float4 x, float alpha, const uint8_t *lut, uint8_t *base)
+{
+    const uint32_t c0 = digit_codes81(x.x, alpha, lut), c1 = digit_codes81(x.y, alpha, lut);
+    const uint32_t c2 = digit_codes81(x.z, alpha, lut), c3 = digit_codes81(x.w, alpha, lut);
+    // columns 0, 2, 4, 6 sit in the low nibbles of the four bytes, 1, 3, 5, 7 in the high ones
+    const uint32_t e01 = (c0 & 0x0F0F0F0Fu) | ((c1 & 0x0F0F0F0Fu) << 4), e23 = (c2 & 0x0F0F0F0Fu) | ((c3 & 0x0F0F0F0Fu) << 4);
+    const uint32_t o01 = ((c0 >> 4) & 0x0F0F0F0Fu) | (c1 & 0xF0F0F0F0u), o23 = ((c2 >> 4) & 0x0F0F0F0Fu) | (c3 & 0xF0F0F0F0u);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        *reinterpret_cast<uint16_t *>(base + (2 * j) * 16) = uint16_t(__byte_perm(e01, e23, j | ((4 + j) << 4)));
+        *reinterpret_cast<uint16_t *>(base + (2 * j + 1) * 16) = uint16_t(__byte_perm(o01, o23, j | ((4 + j) << 4)));
+    }
 }
 
 } // namespace insg

@@ -91,30 +91,14 @@ struct DigitizeParams {
     int tokens, ngroups, tpg, parts; // a token's digits are written by `parts` CTAs, each a slice of the columns
 };
 
-// Eight balanced base-9 digits of round(x * alpha) (|.| < 2^24) as E2M1 codes, digit j in nibble j.
-__device__ __forceinline__ uint32_t digit_codes9(float x, float alpha)
-{
-    const int v = max(-0xFFFFFF, min(__float2int_rn(x * alpha), 0xFFFFFF));
-    uint32_t u = uint32_t(v + 21523360); // + 4 * (9^8 - 1) / 8: plain base-9 digits 0..8 of u are the balanced digits + 4
-    uint32_t codes = 0;
-#pragma unroll
-    for (int j = 0; j < kDigits; j++) {
-        const uint32_t q = u / 9u, e = u - 9u * q; // digit + 4
-        u = q;
-        const int d = int(e) - 4;
-        const uint32_t mag = uint32_t(d < 0 ? -d : d);                         // 0..4 -> E2M1 codes 0, 2, 4, 5, 6 (0, 1, 2, 3, 4)
-        const uint32_t code = (mag < 3u ? 2u * mag : mag + 2u) | (d < 0 ? 8u : 0u);
-        codes |= code << (4 * j);
-    }
-    return codes;
-}
-
 // `parts` CTAs per token slot (slots beyond `tokens` are written as zeros so that their columns contribute nothing).  Every
 // CTA of a token runs the whole prologue (the norm and the token's largest element need all columns; that part is a few
 // loads and one reduction) and writes the digits of its slice of the columns only: the digit extraction is the long part.
 __global__ void __launch_bounds__(kGThreads, 2) umma_digitize_kernel(const __grid_constant__ DigitizeParams p)
 {
     __shared__ float scratch[64];
+    __shared__ uint8_t lut[84];
+    if (threadIdx.x < 81) lut[threadIdx.x] = digit_pair_code(threadIdx.x); // read after the prologue's barriers
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); // the GEMM may set itself up and fetch weights meanwhile
 #ifdef INSG_PHASE_TIMES
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -126,7 +110,6 @@ __global__ void __launch_bounds__(kGThreads, 2) umma_digitize_kernel(const __gri
     const int m = blockIdx.x / p.parts, part = blockIdx.x - m * p.parts, grp = m / p.tpg, ms = m - grp * p.tpg;
     const int tid = threadIdx.x;
     const bool live = m < p.tokens;
-    if (blockIdx.x == 0 && tid < kGMaxGrid) p.tickets[tid] = 0;
     float4 v[kMaxVec];
     float alpha = 0.f;
     if (live) {
@@ -134,6 +117,7 @@ __global__ void __launch_bounds__(kGThreads, 2) umma_digitize_kernel(const __gri
         pin.x_out = nullptr;
         uint2 wpre[kPreVec];
         preload_norm_weights(pin, wpre);
+        pdl_wait();
         load_activation(pin, m, v);
         const float tmax = transform_activation(pin, m, v, wpre, scratch);
         int eb = int((__float_as_uint(tmax) >> 23) & 0xffu);
@@ -141,10 +125,13 @@ __global__ void __launch_bounds__(kGThreads, 2) umma_digitize_kernel(const __gri
         alpha = __uint_as_float(uint32_t(127 + 23 - (eb - 127)) << 23); // max * alpha in [2^23, 2^24)
         if (tid == 0 && part == 0) p.inv_alpha[m] = __uint_as_float(uint32_t(eb - 23) << 23);
     } else {
+        pdl_wait();
 #pragma unroll
         for (int j = 0; j < kMaxVec; j++) v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (tid == 0 && part == 0) p.inv_alpha[m] = 0.f;
+        __syncthreads(); // the table
     }
+    if (blockIdx.x == 0 && tid < kGMaxGrid) p.tickets[tid] = 0;
     const int nvec = p.pro.cols >> 2;
     const int block = 512 * p.tpg, kstep = 256 * p.tpg;
     const int per = (nvec + p.parts - 1) / p.parts, v0 = part * per, v1 = min(nvec, v0 + per);
@@ -152,22 +139,11 @@ __global__ void __launch_bounds__(kGThreads, 2) umma_digitize_kernel(const __gri
     for (int j = 0; j < kMaxVec; j++) {
         const int i = tid + j * kGThreads;
         if (i >= v0 && i < v1) {
-            uint32_t c[4];
-            c[0] = digit_codes9(v[j].x, alpha);
-            c[1] = digit_codes9(v[j].y, alpha);
-            c[2] = digit_codes9(v[j].z, alpha);
-            c[3] = digit_codes9(v[j].w, alpha);
             // 4 consecutive k -> 2 bytes per column.  Block image: [2 K-steps][tpg column groups][2 k cores][8 columns][16 B];
             // the token's eight digit columns are one column group.
             const int k = i << 2, kb = k >> 7, kk = k & 127;
             const int half = (kk & 63) >> 1; // byte index of these k inside the 32-byte row of a K-step
-            uint8_t *base = p.bimg + (size_t(kb) * p.ngroups + grp) * block + (kk >> 6) * kstep + ms * 256 + (half >> 4) * 128 + (half & 15);
-#pragma unroll
-            for (int col = 0; col < kDigits; col++) {
-                const int sh = col * 4;
-                const uint32_t two = ((c[0] >> sh) & 0xFu) | (((c[1] >> sh) & 0xFu) << 4) | (((c[2] >> sh) & 0xFu) << 8) | (((c[3] >> sh) & 0xFu) << 12);
-                *reinterpret_cast<uint16_t *>(base + col * 16) = uint16_t(two);
-            }
+            pack_digits(v[j], alpha, lut, p.bimg + (size_t(kb) * p.ngroups + grp) * block + (kk >> 6) * kstep + ms * 256 + (half >> 4) * 128 + (half & 15));
         }
     }
 #ifdef INSG_PHASE_TIMES
@@ -181,31 +157,47 @@ __global__ void __launch_bounds__(kGThreads, 2) umma_digitize_kernel(const __gri
 
 // Causal convolution (kernel 4) + SiLU over `tokens` consecutive tokens of one sequence, in place: io[m][c] holds the raw
 // projection on entry and the activation on return; the three-value history per channel is read and left updated.
-// The filter is not recursive (out[m] needs raw[m-3..m] only), so a thread takes one channel and up to 32 tokens at a
-// time: all their loads are in flight together, then the outputs are stored.  (reference: src/qwen_kernels.cu:31, once per token)
-__global__ void conv_tokens_kernel(float *io, float *conv_state, const uint16_t *conv_w, int channels, int tokens)
+// (reference: src/qwen_kernels.cu:31, once per token)  The filter is not recursive (out[m] needs raw[m-3..m] only): a CTA
+// takes eight channels (one 32-byte sector per row) and 256 tokens at a time, a thread one channel and eight tokens; all
+// raw values are in registers before the first result is stored.  1024 CTAs at 8192 channels: 27 -> 6 us at 256 tokens
+// against one thread per channel walking the tokens.
+constexpr int kConvCh = 8, kConvTok = 8, kConvBlocks = 32;
+__global__ void __launch_bounds__(kConvCh * kConvBlocks) conv_tokens_kernel(float *io, float *conv_state, const uint16_t *conv_w, int channels, int tokens)
 {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= channels) return;
-    float *st = conv_state + size_t(c) * 3;
-    float h0 = st[0], h1 = st[1], h2 = st[2];
-    const uint2 wv = reinterpret_cast<const uint2 *>(conv_w)[c];
-    const float w0 = bf16_bits_to_float(wv.x & 0xffff), w1 = bf16_bits_to_float(wv.x >> 16);
-    const float w2 = bf16_bits_to_float(wv.y & 0xffff), w3 = bf16_bits_to_float(wv.y >> 16);
-    for (int m0 = 0; m0 < tokens; m0 += 32) {
-        float x[32];
-#pragma unroll
-        for (int j = 0; j < 32; j++) x[j] = m0 + j < tokens ? __ldcg(io + size_t(m0 + j) * channels + c) : 0.f;
-#pragma unroll
-        for (int j = 0; j < 32; j++) {
-            if (m0 + j < tokens) {
-                const float z = fmaf(h0, w0, fmaf(h1, w1, fmaf(h2, w2, x[j] * w3)));
-                h0 = h1; h1 = h2; h2 = x[j];
-                io[size_t(m0 + j) * channels + c] = fast_silu(z);
-            }
-        }
+    __shared__ float hist[2][3][kConvCh];
+    const int ch = threadIdx.x & (kConvCh - 1), blk = threadIdx.x / kConvCh, c = blockIdx.x * kConvCh + ch;
+    const bool on = c < channels;
+    pdl_launch_dependents();
+    float w0 = 0.f, w1 = 0.f, w2 = 0.f, w3 = 0.f;
+    if (on) {
+        const uint2 wv = reinterpret_cast<const uint2 *>(conv_w)[c];
+        w0 = bf16_bits_to_float(wv.x & 0xffff); w1 = bf16_bits_to_float(wv.x >> 16);
+        w2 = bf16_bits_to_float(wv.y & 0xffff); w3 = bf16_bits_to_float(wv.y >> 16);
     }
-    st[0] = h0; st[1] = h1; st[2] = h2;
+    pdl_wait();
+    if (blk < 3) hist[0][blk][ch] = on ? __ldcg(conv_state + size_t(c) * 3 + blk) : 0.f;
+    __syncthreads();
+    int cur = 0;
+    for (int m0 = 0; m0 < tokens; m0 += kConvTok * kConvBlocks, cur ^= 1) {
+        const int first = m0 + blk * kConvTok, end = min(tokens, m0 + kConvTok * kConvBlocks);
+        float x[kConvTok + 3]; // raw[first - 3 ..]
+#pragma unroll
+        for (int j = 0; j < kConvTok + 3; j++) {
+            const int m = first + j - 3;
+            x[j] = m < m0 ? hist[cur][m - m0 + 3][ch] : (on && m < end) ? __ldcg(io + size_t(m) * channels + c) : 0.f;
+        }
+        // the chunk's last three raw values (older ones when it is shorter than three) are the next history
+#pragma unroll
+        for (int j = 0; j < kConvTok + 3; j++) {
+            const int m = first + j - 3, i = m - (end - 3);
+            if (i >= 0 && i < 3 && (j >= 3 || blk == 0)) hist[cur ^ 1][i][ch] = x[j];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kConvTok; j++)
+            if (on && first + j < end) io[size_t(first + j) * channels + c] = fast_silu(fmaf(x[j], w0, fmaf(x[j + 1], w1, fmaf(x[j + 2], w2, x[j + 3] * w3))));
+    }
+    if (on && blk < 3) conv_state[size_t(c) * 3 + blk] = hist[cur][blk][ch];
 }
 
 __device__ __forceinline__ int gseg_of(const GParams &p, int tile)
@@ -413,6 +405,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
+    pdl_launch_dependents(); // this CTA holds its tensor memory: whatever follows may take an SM as it becomes free
     const uint32_t tmem = s_tmem;
     volatile int *abort_flag = &s_abort;
     if (tid == 0) GEMM_STAMP(1);
@@ -770,9 +763,9 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
             g_gemm_attr_done[dev] = true;
         }
     }
-    // the digitize kernel is in plain stream order (its input comes from whatever ran before); the GEMM is its programmatic
-    // dependent: it allocates tensor memory and requests its first weight records while the digits are being written
-    int rc = launch(umma_digitize_kernel, dim3(ngroups * tpg * d.parts), dim3(kGThreads), 0, st, false, d);
+    // the GEMM is the digitize kernel's programmatic dependent: it allocates tensor memory and requests its first weight
+    // records while the digits are being written
+    int rc = launch(umma_digitize_kernel, dim3(ngroups * tpg * d.parts), dim3(kGThreads), 0, st, op->pdl != 0, d);
     if (rc != INSG_OK) return rc;
     const int grid = std::max(1, std::min(std::min(sm_count(), kGMaxGrid), p.total_stages));
     p.share = p.total_stages / grid;
@@ -782,7 +775,7 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     for (int i = 0; i < op->n_segments; i++) {
         const insg_gemv_segment &s = op->seg[i];
         if (s.epilogue == INSG_EPI_CONV_SILU && s.conv_token_stride == 0) { // one sequence: the history runs through the tokens
-            rc = launch(conv_tokens_kernel, dim3((s.rows + 63) / 64), dim3(64), 0, st, false, s.out, s.conv_state, s.conv_w, s.rows, tokens);
+            rc = launch(conv_tokens_kernel, dim3((s.rows + kConvCh - 1) / kConvCh), dim3(kConvCh * kConvBlocks), 0, st, op->pdl != 0, s.out, s.conv_state, s.conv_w, s.rows, tokens);
             if (rc != INSG_OK) return rc;
         }
     }
