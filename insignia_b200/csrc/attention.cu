@@ -581,7 +581,7 @@ int insg_attention_chunk(const insg_attn_op *op, int tokens, float *q_scratch, i
         !op->out || !op->position || !op->scratch || !q_scratch)
         return fail(INSG_E_ARG, "attention_chunk: null pointer");
     if (tokens < 1 || tokens > 65535) return fail(INSG_E_SHAPE, "attention_chunk: 1 <= tokens <= 65535");
-    if (op->scratch_bytes < size_t(tokens) * attn_scratch_bytes()) return fail(INSG_E_SHAPE, "attention_chunk: scratch too small");
+    if (tokens <= kTileFromTokens && op->scratch_bytes < size_t(tokens) * attn_scratch_bytes()) return fail(INSG_E_SHAPE, "attention_chunk: scratch too small");
     if (op->max_context <= 0) return fail(INSG_E_SHAPE, "attention_chunk: max_context");
     AttnParams p = {};
     p.q = op->qraw; p.k_raw = op->k_raw; p.v_new = op->v; p.q_w = op->q_norm_w; p.k_w = op->k_norm_w;
