@@ -108,6 +108,9 @@ INSG_API int insg_mxfp4_repack(const uint32_t *weight, const uint8_t *scales, vo
  * K-major 4-bit operand, no swizzle) followed by the 512-byte scale block tcgen05.cp expects.  cols % 128 == 0.
  * Same 17 bytes per 32 weights.  No reference counterpart. */
 INSG_API size_t insg_mxfp4_packed_umma_bytes(int rows, int cols);
+/* Bytes of the digit image of `tokens` (1..8) activation vectors of `cols` elements: what a layout-1 launch leaves through
+ * insg_gemv_segment.prep and a later one takes as its INSG_PRO_PREPARED input.  0 when the shape has none. */
+INSG_API size_t insg_mxfp4_digit_image_bytes(int cols, int tokens);
 INSG_API int insg_mxfp4_repack_umma(const uint32_t *weight, const uint8_t *scales, void *packed, int rows, int cols,
                                     insg_stream_t stream);
 
@@ -176,7 +179,10 @@ typedef struct insg_gemv_segment {
      * prep: fp16 [2][rows] = the two half-precision pieces of out[row] * prep_w[row] / 16 (values beyond
      * +-1e6 saturate).  prep_w: bf16 [rows] multiplier, the weight of the RMSNorm that follows, or NULL for 1.
      * prep_partials (single-segment launches): fp32 [296], entry c = this launch's CTA c's sum of out[row]^2 over
-     * its rows (infinite if a value did not fit the image), unused entries zero. */
+     * its rows (infinite if a value did not fit the image), unused entries zero.
+     * Layout 1 (up to eight tokens, rows % 128 == 0): prep = the digit image of out * prep_w
+     * (insg_mxfp4_digit_image_bytes(rows, tokens), every value representable); prep_partials = fp32
+     * [tokens][rows / 32] sums of out^2 over groups of 32 rows. */
     void *prep;
     const uint16_t *prep_w;
     float *prep_partials;
@@ -189,7 +195,7 @@ typedef struct insg_gemv_segment {
 /* A fused launch: prologue on the shared input vector, up to 4 matrices that
  * all multiply it, an epilogue per matrix.  cols % 128 == 0, cols <= 12288. */
 typedef struct insg_gemv_op {
-    const float *in;          /* fp32 [cols] (INSG_PRO_PREPARED: the fp16 image [2][cols]) */
+    const float *in;          /* fp32 [cols] (INSG_PRO_PREPARED: the producer's image)     */
     const float *aux;         /* prologue operand (gate / z), or NULL                  */
     const uint16_t *norm_w;   /* bf16 norm weight for the RMSNorm prologues, or NULL   */
     float *x_out;             /* optional: the prologue's result fp32 [cols], or NULL  */

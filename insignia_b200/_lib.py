@@ -57,6 +57,7 @@ SIGNATURES = {
     "insg_mxfp4_packed_bytes": (sz, [i32, i32]),
     "insg_mxfp4_repack": (i32, [vp, vp, vp, i32, i32, vp]),
     "insg_mxfp4_packed_umma_bytes": (sz, [i32, i32]),
+    "insg_mxfp4_digit_image_bytes": (sz, [i32, i32]),
     "insg_mxfp4_repack_umma": (i32, [vp, vp, vp, i32, i32, vp]),
     "insg_mxfp4_gemv_packed": (i32, [vp, vp, vp, i32, i32, i32, vp]),
     "insg_umma_gemm_scratch_bytes": (sz, [i32, i32]),

@@ -54,6 +54,9 @@ struct DSeg {
     const float *A_log;
     const uint16_t *dt_bias;
     long long conv_stride; // 0: the tokens are one sequence (history carried through them in order), else token m's history at + m * stride
+    uint8_t *prep;         // optional: digit image of the output (times prep_w) for a later launch with a prepared input
+    const uint16_t *prep_w;
+    float *prep_partials;  // with it, [token][rows / 32] sums of squares of the output
     int tile_begin, epilogue, rows;
 };
 
@@ -61,6 +64,7 @@ struct DParams {
     const float *in, *aux;
     const uint16_t *norm_w;
     float *x_out;
+    const float *prep_partials; // prepared input: the producer's sums of squares, or null
     int cols, nkb, prologue, nseg, units, nmat, tokens, stages;
     DSeg seg[4];
     float2 *argmax_partial;
@@ -123,7 +127,7 @@ __device__ __forceinline__ int dseg_of(const DParams &p, int unit)
 // The digits of one 128-element k-block of one token (four elements per lane) into the B image, and their group scales.
 // Image of a k-block: [2 K-steps][T column groups][2 k cores][8 columns][16 B]; a token's eight digit columns are one group.
 template <int T>
-__device__ __forceinline__ void store_digits(float4 x, int m, uint8_t *bkb, uint8_t *sfkb, const uint8_t *lut, int lane)
+__device__ __forceinline__ void store_digits(float4 x, int m, uint8_t *bkb, const uint8_t *lut, int lane)
 {
     float mx = fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w)));
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1)); // a group of 32 elements = 8 lanes
@@ -134,7 +138,30 @@ __device__ __forceinline__ void store_digits(float4 x, int m, uint8_t *bkb, uint
     const float alpha = __uint_as_float(uint32_t(277 - eb) << 23); // largest element * alpha in [2^23, 2^24)
     pack_digits(x, alpha, lut, bkb + (lane >> 4) * (256 * T) + m * 256 + ((lane >> 3) & 1) * 128 + (lane & 7) * 2);
     const int n = 8 * m + (lane & 7); // scale block: row = column n of B (32 rows, then the next quarter), byte = group
-    sfkb[(n & 31) * 16 + (n >> 5) * 4 + (lane >> 3)] = uint8_t(eb - 23);
+    bkb[512 * T + (n & 31) * 16 + (n >> 5) * 4 + (lane >> 3)] = uint8_t(eb - 23);
+}
+
+// One output row per lane into the digit image a later launch takes as its prepared input (the layout of store_digits): the
+// warp's 32 rows are one 32-element group of that launch's K.  Costs the producer some 50 instructions per token; converting
+// in the consumer would be done by every cluster again (eight tokens: 6 us per launch at 4096 columns, 17 at 12288).
+template <int T> __device__ __forceinline__ void leave_digits(const DSeg &s, float v, float w, int row, int m, const uint8_t *lut, int lane)
+{
+    const float x = v * w;
+    int eb = int(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(x))) >> 23);
+    eb = min(max(eb, 24), 230);
+    const uint32_t c = digit_codes81(x, __uint_as_float(uint32_t(277 - eb) << 23), lut), o = __shfl_xor_sync(0xffffffffu, c, 1);
+    // a pair of lanes holds two neighbouring k = one byte per column: the even lane stores columns 0, 2, 4, 6, the odd one the others
+    const uint32_t b = (lane & 1) ? ((o >> 4) & 0x0F0F0F0Fu) | (c & 0xF0F0F0F0u) : (c & 0x0F0F0F0Fu) | ((o & 0x0F0F0F0Fu) << 4);
+    const int grp = row >> 5, g = grp & 3;
+    uint8_t *kb = s.prep + size_t(grp >> 2) * (512 * T + 512), *dst = kb + (g >> 1) * (256 * T) + m * 256 + (g & 1) * 128 + (lane & 1) * 16 + (lane >> 1);
+#pragma unroll
+    for (int j = 0; j < 4; j++) dst[32 * j] = uint8_t(b >> (8 * j));
+    const int n = 8 * m + (lane & 7);
+    if (lane < 8) kb[512 * T + (n & 31) * 16 + (n >> 5) * 4 + g] = uint8_t(eb - 23);
+    if (s.prep_partials) {
+        const float ss = warp_sum(v * v);
+        if (lane == 0) s.prep_partials[m * (s.rows >> 5) + grp] = ss;
+    }
 }
 
 // One accumulator: the eight digit columns of each token, digits combined (least significant first; 9^j is exact in fp32).
@@ -174,6 +201,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int kBKb = 512 * T;       // digit bytes per k-block
+    constexpr int kImg = kBKb + 512;    // a k-block of the image: digits, then their scale block
     constexpr int N = kDDigits * T;
     constexpr int kSlot = kDCl * 32 * T; // floats of one exchange slot: [source rank][32 rows][T]
     __shared__ __align__(8) uint64_t full[kDMaxStages], empty[kDMaxStages], dfull[2], dempty[2], xfull[8], xempty[8], ssfull, image[kDMaxKb / 8];
@@ -191,9 +219,9 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     const int nun = cl < p.units ? (p.units - cl + C - 1) / C : 0;             // units of this cluster: cl, cl + C, ...
     const int nruns = nun * nmat, nstages = nruns * spt;
     uint8_t *ring = smem;                                // S stages
-    uint8_t *bimg = ring + size_t(S) * kDStage;          // len x kBKb bytes of digits
-    uint8_t *sfb = bimg + size_t((nkb + 3) >> 2) * kBKb; // len x 512 bytes of their scales
-    float *xslot = reinterpret_cast<float *>(sfb + size_t((nkb + 3) >> 2) * 512); // 4 * nmat exchange slots
+    uint8_t *bimg = ring + size_t(S) * kDStage; // len x kImg bytes
+    float *xslot = reinterpret_cast<float *>(bimg + size_t((nkb + 3) >> 2) * kImg); // 4 * nmat exchange slots
+    const bool prepared = p.prologue == INSG_PRO_PREPARED;
 
     // ---- the weight stream starts first: it depends on nothing ----------------------------------------------------------
     auto run_src = [&](int run) -> const uint8_t * { // this CTA's records of the run (tile, matrix)
@@ -224,7 +252,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         for (int i = 0; i < 2; i++) { mbar_init(&dfull[i], 1); mbar_init(&dempty[i], 4); }
         for (int i = 0; i < 8; i++) { mbar_init(&xfull[i], 1); mbar_init(&xempty[i], kDCl); }
         mbar_init(&ssfull, 1);
-        for (int i = 0; i < kDMaxKb / 8; i++) mbar_init(&image[i], uint32_t(T * max(1, min(8, len - 8 * i)))); // one arrival per (token, k-block)
+        for (int i = 0; i < kDMaxKb / 8; i++) mbar_init(&image[i], prepared ? 1u : uint32_t(T * max(1, min(8, len - 8 * i)))); // one arrival per (token, k-block), or the copy's
         s_abort = 0;
         mbar_expect_tx(&ssfull, kDCl * T * 4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -243,7 +271,9 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     volatile int *abort_flag = &s_abort;
     bool arrived = false; // at the closing cluster barrier
 
-    if (warp < 8) {
+    if (prepared) {
+        if (warp >= 4 && warp < 8) pdl_wait(); // they read what earlier launches wrote
+    } else if (warp < 8) {
         // ---- activation prologue: this CTA's quarter of the columns ---------------------------------------------------------
         constexpr int kBatch = 3;
         const int items = len * T; // (token, k-block) pairs, dealt to the eight warps
@@ -324,7 +354,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 }
                 if (p.x_out && cl == 0 && !rms && m < p.tokens)
                     reinterpret_cast<float4 *>(p.x_out + size_t(m) * p.cols)[(kb0 + kb) * 32 + lane] = v;
-                store_digits<T>(v, m, bimg + size_t(kb) * kBKb, sfb + size_t(kb) * 512, s_lut, lane);
+                store_digits<T>(v, m, bimg + size_t(kb) * kImg, s_lut, lane);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // the tensor core reads the image through the async proxy
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&image[kb >> 3]);
@@ -344,6 +374,16 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         // ---- producer ----------------------------------------------------------------------------------------------------------
         {
             const bool one = elect_one();
+            if (prepared) { // the digits come ready: eight k-blocks per copy, so that the multiplies can start behind the first
+                pdl_wait();
+                asm volatile("fence.proxy.async;" ::: "memory"); // written by ordinary stores of the launch before
+                for (int kb = 0; kb < len; kb += 8)
+                    if (one) {
+                        const uint32_t bytes = uint32_t(min(8, len - kb)) * kImg;
+                        mbar_expect_tx(&image[kb >> 3], bytes);
+                        bulk_load(bimg + size_t(kb) * kImg, reinterpret_cast<const uint8_t *>(p.in) + size_t(kb0 + kb) * kImg, bytes, &image[kb >> 3]);
+                    }
+            }
             int i = 0, slot = 0;
             uint32_t phase = 1; // of the empty barriers: slot reuse n waits for the n-th release
             bool ok = true;
@@ -371,7 +411,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             constexpr uint32_t idesc0 = (1u << 7) | (1u << 10) | ((uint32_t(N) >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
             constexpr uint32_t idesc1 = idesc0 | (2u << 29) | (2u << 4);
             const uint64_t da0 = umma_desc(smem_u32(ring), 128, 256), dsf0 = umma_desc(smem_u32(ring) + 8192, 16, 128), db0 = umma_desc(smem_u32(bimg), 128, 256);
-            const uint64_t dsb0 = umma_desc(smem_u32(sfb), 16, 128);
+            const uint64_t dsb0 = umma_desc(smem_u32(bimg) + kBKb, 16, 128);
             bool ok = true;
             int st = 0, sfa = 0;
             uint32_t phase = 0;
@@ -397,20 +437,20 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                     if (one) {
                         const bool two = kb + 1 < len;
                         if (run == 0) { // the digits' scales stay in tensor memory for all tiles
-                            copy_scales(sb, dsb0 + uint64_t(kb * (512 >> 4)));
-                            if (two) copy_scales(sb + 4, dsb0 + uint64_t((kb + 1) * (512 >> 4)));
+                            copy_scales(sb, dsb0 + uint64_t(kb * (kImg >> 4)));
+                            if (two) copy_scales(sb + 4, dsb0 + uint64_t((kb + 1) * (kImg >> 4)));
                         }
                         copy_scales(sa, dsf);
                         if (two) copy_scales(sa + 4, dsf + (kURec >> 4));
                         mma_step(dcol, da, db, idesc0, kb > 0, sa, sb);
                         mma_step(dcol, da + 256, db + (kBKb >> 5), idesc1, true, sa, sb);
                         if (two) {
-                            mma_step(dcol, da + (kURec >> 4), db + (kBKb >> 4), idesc0, true, sa + 4, sb + 4);
-                            mma_step(dcol, da + (kURec >> 4) + 256, db + (kBKb >> 4) + (kBKb >> 5), idesc1, true, sa + 4, sb + 4);
+                            mma_step(dcol, da + (kURec >> 4), db + (kImg >> 4), idesc0, true, sa + 4, sb + 4);
+                            mma_step(dcol, da + (kURec >> 4) + 256, db + (kImg >> 4) + (kBKb >> 5), idesc1, true, sa + 4, sb + 4);
                         }
                         commit_to(&empty[cur]);
                     }
-                    db += 2 * (kBKb >> 4);
+                    db += 2 * (kImg >> 4);
                     sb += 8;
                     sfa = (sfa + 1) & 3;
                 }
@@ -454,8 +494,17 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         for (int t = 0; t < T; t++) scale[t] = 1.f;
         // The quarters' sums of squares arrive while the weights are still being multiplied.  Every CTA waits for all four
         // (also where they are not needed), so that nobody leaves while a peer still writes into its shared memory.
-        ok = __all_sync(0xffffffffu, mbar_wait_cluster(&ssfull, 0, abort_flag));
-        if (ok && p.prologue == INSG_PRO_RMSNORM) {
+        if (!prepared) ok = __all_sync(0xffffffffu, mbar_wait_cluster(&ssfull, 0, abort_flag));
+        if (prepared && p.prep_partials) {
+            const int groups = p.cols >> 5;
+#pragma unroll
+            for (int t = 0; t < T; t++) {
+                float ss = 0.f;
+                if (t < p.tokens)
+                    for (int i = lane; i < groups; i += 32) ss += __ldcg(p.prep_partials + t * groups + i);
+                scale[t] = rsqrtf(warp_sum(ss) / float(p.cols) + 1e-6f);
+            }
+        } else if (ok && p.prologue == INSG_PRO_RMSNORM) {
 #pragma unroll
             for (int t = 0; t < T; t++) scale[t] = rsqrtf((s_rss[t] + s_rss[T + t] + s_rss[2 * T + t] + s_rss[3 * T + t]) / float(p.cols) + 1e-6f);
             if (p.x_out && cl == 0) {
@@ -478,6 +527,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             // the epilogue's other operands are fetched before the wait for the sums
             float pre[T], h0 = 0.f, h1 = 0.f, h2 = 0.f;
             float cw0 = 0.f, cw1 = 0.f, cw2 = 0.f, cw3 = 0.f;
+            const float pw = s.prep_w ? bf16_bits_to_float(s.prep_w[row]) : 1.f; // rows % 128 == 0 where it is set
 #pragma unroll
             for (int t = 0; t < T; t++) pre[t] = 0.f;
             if (on && s.epilogue == INSG_EPI_RESIDUAL) {
@@ -530,7 +580,11 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             case INSG_EPI_RESIDUAL:
 #pragma unroll
                 for (int t = 0; t < T; t++)
-                    if (t < p.tokens) out[t * ld] = pre[t] + y[0][t];
+                    if (t < p.tokens) {
+                        const float v = pre[t] + y[0][t];
+                        out[t * ld] = v;
+                        if (s.prep) leave_digits<T>(s, v, pw, row, t, s_lut, lane);
+                    }
                 break;
             case INSG_EPI_CONV_SILU: {
                 float *hist = s.conv_state + size_t(row) * 3;
@@ -564,7 +618,11 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             case INSG_EPI_SWIGLU:
 #pragma unroll
                 for (int t = 0; t < T; t++)
-                    if (t < p.tokens) out[t * ld] = fast_silu(y[0][t]) * y[1][t];
+                    if (t < p.tokens) {
+                        const float v = fast_silu(y[0][t]) * y[1][t];
+                        out[t * ld] = v;
+                        if (s.prep) leave_digits<T>(s, v, pw, row, t, s_lut, lane);
+                    }
                 break;
             case INSG_EPI_LOGITS:
                 out[0] = y[0][0];
@@ -705,12 +763,16 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     if (tokens > 8) return fail(INSG_E_SHAPE, "gemv: 1..8 tokens");
     if (op->cols <= 0 || (op->cols & 127) || op->cols > kDMaxKb * kDCl * 128) return fail(INSG_E_SHAPE, "gemv: cols must be a multiple of 128, <= 12288");
     if (op->n_segments < 1 || op->n_segments > 4) return fail(INSG_E_SHAPE, "gemv: 1..4 segments");
-    if (op->prologue < 0 || op->prologue >= INSG_PRO_PREPARED) return fail(INSG_E_ARG, "gemv: a prepared input belongs to the mma.sync layout");
+    if (op->prologue < 0 || op->prologue > INSG_PRO_PREPARED) return fail(INSG_E_ARG, "gemv: unknown prologue");
     if ((op->prologue == INSG_PRO_RMSNORM || op->prologue == INSG_PRO_GATED_RMSNORM) && !op->norm_w) return fail(INSG_E_ARG, "gemv: norm weight missing");
-    if (op->prologue >= INSG_PRO_GATED_RMSNORM && !op->aux) return fail(INSG_E_ARG, "gemv: prologue operand missing");
+    if (op->prologue >= INSG_PRO_GATED_RMSNORM && op->prologue != INSG_PRO_PREPARED && !op->aux) return fail(INSG_E_ARG, "gemv: prologue operand missing");
     DParams p = {};
     p.in = op->in; p.aux = op->aux; p.norm_w = op->norm_w; p.x_out = op->x_out;
     p.cols = op->cols; p.prologue = op->prologue;
+    if (op->prologue == INSG_PRO_PREPARED) {
+        p.x_out = nullptr;
+        p.prep_partials = op->prep_rms ? op->prep_partials : nullptr;
+    }
     p.nkb = op->cols >> 7;
     p.nseg = op->n_segments;
     p.tokens = tokens;
@@ -718,7 +780,6 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     for (int i = 0; i < op->n_segments; i++) {
         const insg_gemv_segment &s = op->seg[i];
         if (!s.packed || !s.out || s.rows <= 0) return fail(INSG_E_SHAPE, "gemv: bad segment");
-        if (s.prep) return fail(INSG_E_SHAPE, "gemv: a prepared output belongs to the mma.sync layout");
         if (s.epilogue == INSG_EPI_SWIGLU && !s.packed2) return fail(INSG_E_ARG, "gemv: SwiGLU needs two matrices");
         if (s.epilogue == INSG_EPI_CONV_SILU && (!s.conv_state || !s.conv_w)) return fail(INSG_E_ARG, "gemv: conv operands missing");
         if (s.epilogue == INSG_EPI_DECAY && (!s.A_log || !s.dt_bias)) return fail(INSG_E_ARG, "gemv: decay operands missing");
@@ -727,6 +788,13 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
         d.packed2 = static_cast<const uint8_t *>(s.packed2);
         d.out = s.out; d.conv_state = s.conv_state; d.conv_w = s.conv_w; d.A_log = s.A_log; d.dt_bias = s.dt_bias;
         d.conv_stride = s.conv_token_stride;
+        if (s.prep) {
+            if (s.epilogue != INSG_EPI_RESIDUAL && s.epilogue != INSG_EPI_SWIGLU) return fail(INSG_E_ARG, "gemv: prepared output needs the residual or SwiGLU epilogue");
+            if (s.rows & 127) return fail(INSG_E_SHAPE, "gemv: a prepared output needs rows % 128 == 0");
+            d.prep = static_cast<uint8_t *>(s.prep);
+            d.prep_w = s.prep_w;
+            d.prep_partials = s.prep_partials;
+        }
         const int nmat = s.epilogue == INSG_EPI_SWIGLU ? 2 : 1;
         if (p.nmat && p.nmat != nmat) return fail(INSG_E_SHAPE, "gemv: SwiGLU segments cannot be mixed with others");
         p.nmat = nmat;
@@ -781,6 +849,13 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
 using namespace insg;
 
 extern "C" {
+
+size_t insg_mxfp4_digit_image_bytes(int cols, int tokens)
+{
+    if (cols <= 0 || (cols & 127) || tokens < 1 || tokens > 8) return 0;
+    const int T = tokens == 1 ? 1 : tokens == 2 ? 2 : tokens <= 4 ? 4 : 8;
+    return size_t(cols >> 7) * (512 * T + 512);
+}
 
 size_t insg_mxfp4_packed_umma_bytes(int rows, int cols)
 {

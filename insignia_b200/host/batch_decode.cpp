@@ -42,6 +42,8 @@ struct Qwen35BatchDecode::Impl {
     float *hidden{}, *qkv{}, *z{}, *a{}, *b{}, *core{}, *qg{}, *key{}, *value{}, *act{}, *logits{};
     float *delta_state{}, *conv_state{}; // [B][24][...]
     void *kv_keys{}, *kv_values{};       // [B][8][ctx][1024]
+    void *prep_hidden{}, *prep_act{};    // digit images of the residual stream and of the SwiGLU output for the next product
+    float *prep_sums{};                  // [8][128] sums of squares of the residual stream
     void *attn_scratch{};                // [B][insg_gqa_scratch_bytes]
     size_t attn_scratch_each = 0, kv_seq_bytes = 0;
     int *d_tokens{}, *d_next{}, *d_position{}, *d_error{}, *d_log{}; // log [ctx + 1][B]
@@ -86,6 +88,9 @@ Qwen35BatchDecode::Qwen35BatchDecode(Qwen35Weights &weights, int sequences, int 
     m.alloc(&m.kv_values, B * m.kv_seq_bytes, "cudaMalloc batch KV cache");
     m.attn_scratch_each = (insg_gqa_scratch_bytes(max_context) + 255) / 256 * 256;
     m.alloc(&m.attn_scratch, B * m.attn_scratch_each, "cudaMalloc batch attention scratch");
+    m.alloc(&m.prep_hidden, insg_mxfp4_digit_image_bytes(kHidden, m.B), "cudaMalloc batch digit image");
+    m.alloc(&m.prep_act, insg_mxfp4_digit_image_bytes(kInter, m.B), "cudaMalloc batch digit image");
+    m.alloc(&m.prep_sums, B * (kHidden / 32) * f, "cudaMalloc batch sums");
     m.alloc(&m.d_tokens, (3 * B + 8) * sizeof(int), "cudaMalloc batch scalars");
     m.d_next = m.d_tokens + B;
     m.d_position = m.d_next + B;
@@ -160,22 +165,40 @@ void Qwen35BatchDecode::enqueue_step()
         insg_check(insg_gemv_fused(&op, st));
         launches_++;
     };
-    auto mlp = [&](const DecodeBlock &blk) {
+    // a product that writes the residual stream leaves the digits of the RMSNorm'd input of the next one
+    auto normed_input = [&](insg_gemv_op &op, const uint16_t *norm_w, bool ready) {
+        op.cols = kHidden;
+        if (ready) {
+            op.in = static_cast<const float *>(m.prep_hidden);
+            op.prologue = INSG_PRO_PREPARED;
+            op.prep_partials = m.prep_sums;
+            op.prep_rms = 1;
+        } else {
+            op.in = m.hidden;
+            op.norm_w = norm_w;
+            op.prologue = INSG_PRO_RMSNORM;
+        }
+    };
+    auto residual_output = [&](insg_gemv_segment &sg, const uint16_t *following_norm_w) {
+        sg.prep = m.prep_hidden;
+        sg.prep_w = following_norm_w;
+        sg.prep_partials = m.prep_sums;
+    };
+    auto mlp = [&](const DecodeBlock &blk, const uint16_t *next_norm) {
         insg_gemv_op up = {};
-        up.in = m.hidden;
-        up.norm_w = blk.post_norm;
-        up.cols = kHidden;
-        up.prologue = INSG_PRO_RMSNORM;
+        normed_input(up, blk.post_norm, true);
         up.n_segments = 1;
         up.seg[0] = seg(blk.gate, m.act, INSG_EPI_SWIGLU);
         up.seg[0].packed2 = blk.up.data;
+        up.seg[0].prep = m.prep_act;
         gemv(up);
         insg_gemv_op dn = {};
-        dn.in = m.act;
+        dn.in = static_cast<const float *>(m.prep_act);
         dn.cols = kInter;
-        dn.prologue = INSG_PRO_PLAIN;
+        dn.prologue = INSG_PRO_PREPARED;
         dn.n_segments = 1;
         dn.seg[0] = seg(blk.down, m.hidden, INSG_EPI_RESIDUAL);
+        residual_output(dn.seg[0], next_norm);
         gemv(dn);
     };
     const uint32_t *ew = static_cast<const uint32_t *>(m.embed.weight.data);
@@ -189,10 +212,7 @@ void Qwen35BatchDecode::enqueue_step()
         if (!Qwen35Shape::full_attention(l)) {
             const int di = l - l / 4;
             insg_gemv_op in = {};
-            in.in = m.hidden;
-            in.norm_w = blk.in_norm;
-            in.cols = kHidden;
-            in.prologue = INSG_PRO_RMSNORM;
+            normed_input(in, blk.in_norm, l > 0);
             in.n_segments = 4;
             in.seg[0] = seg(blk.qkv, m.qkv, INSG_EPI_CONV_SILU);
             in.seg[0].conv_state = m.conv_state + size_t(di) * kConvLayer;
@@ -215,13 +235,11 @@ void Qwen35BatchDecode::enqueue_step()
             out.prologue = INSG_PRO_GATED_RMSNORM;
             out.n_segments = 1;
             out.seg[0] = seg(blk.out, m.hidden, INSG_EPI_RESIDUAL);
+            residual_output(out.seg[0], blk.post_norm);
             gemv(out);
         } else {
             insg_gemv_op in = {};
-            in.in = m.hidden;
-            in.norm_w = blk.in_norm;
-            in.cols = kHidden;
-            in.prologue = INSG_PRO_RMSNORM;
+            normed_input(in, blk.in_norm, l > 0);
             in.n_segments = 3;
             in.seg[0] = seg(blk.q, m.qg, INSG_EPI_STORE);
             in.seg[1] = seg(blk.k, m.key, INSG_EPI_STORE);
@@ -258,15 +276,13 @@ void Qwen35BatchDecode::enqueue_step()
             o.prologue = options_.gate_elementwise ? INSG_PRO_SIGMOID_GATE_QPROJ : INSG_PRO_SIGMOID_GATE_HEAD0;
             o.n_segments = 1;
             o.seg[0] = seg(blk.o, m.hidden, INSG_EPI_RESIDUAL);
+            residual_output(o.seg[0], blk.post_norm);
             gemv(o);
         }
-        mlp(blk);
+        mlp(blk, l + 1 < n ? m.layers[size_t(l) + 1].in_norm : m.final_norm);
     }
     insg_gemv_op head = {};
-    head.in = m.hidden;
-    head.norm_w = m.final_norm;
-    head.cols = kHidden;
-    head.prologue = INSG_PRO_RMSNORM;
+    normed_input(head, m.final_norm, n > 0);
     head.n_segments = 1;
     head.seg[0] = seg(m.lm_head, m.logits, INSG_EPI_STORE);
     head.seg[0].rows = options_.vocab;

@@ -23,8 +23,9 @@ namespace insignia {
 namespace {
 
 constexpr int kHidden = Qwen35Shape::hidden, kInter = Qwen35Shape::intermediate;
-// DecodeWorkspace::prep: fp16 image of the normalised-to-be hidden vector, fp16 image of the SwiGLU output, sums of squares
-constexpr size_t kPrepHidden = 0, kPrepAct = size_t(2) * kHidden * 2, kPrepSums = kPrepAct + size_t(2) * kInter * 2;
+// DecodeWorkspace::prep: images of the normalised-to-be hidden vectors and of the SwiGLU outputs, sums of squares.  Sized for
+// the digit images of eight tokens (insg_mxfp4_digit_image_bytes); the one-token fp16 images of the mma.sync kernel are smaller.
+constexpr size_t kPrepHidden = 0, kPrepAct = size_t(kHidden / 128) * (8 * 512 + 512), kPrepSums = kPrepAct + size_t(kInter / 128) * (8 * 512 + 512);
 constexpr int kMultiSteps = 8; // token steps per graph in Qwen35Decode::generate
 // DecodeWorkspace::multi: activations of up to kChunk consecutive tokens for Qwen35Decode::forward_tokens, [token][width] each
 constexpr int kChunk = 4;     // tokens per pass of the mma.sync kernel
@@ -37,7 +38,7 @@ constexpr size_t kMultiHidden = 0, kMultiQkv = kMultiHidden + size_t(kBigChunk) 
                  kMultiKey = kMultiQg + size_t(kBigChunk) * 8192, kMultiValue = kMultiKey + size_t(kBigChunk) * 1024,
                  kMultiAct = kMultiValue + size_t(kBigChunk) * 1024, kMultiQn = kMultiAct + size_t(kBigChunk) * 12288,
                  kMultiTokens = kMultiQn + size_t(kBigChunk) * 4096, kMultiFloats = kMultiTokens + kBigChunk;
-constexpr size_t kPrepBytes = kPrepSums + 2 * 296 * sizeof(float); // one row of sums per image
+constexpr size_t kPrepBytes = kPrepSums + 8 * (kHidden / 32) * sizeof(float); // [token][32-row group], or two rows of 296
 const char *const kLM = "language_model";
 
 void cuda_check(cudaError_t e, const char *what)
@@ -217,7 +218,7 @@ struct Ctx {
     void *prep_act() const { return static_cast<uint8_t *>(x.prep) + kPrepAct; }
     float *prep_sums() const { return reinterpret_cast<float *>(static_cast<uint8_t *>(x.prep) + kPrepSums); }
     bool tcgen05() const { return tcgen05_engine(x.options); }
-    bool prepared() const { return x.options.prepared_inputs && !tcgen05(); }
+    bool prepared() const { return x.options.prepared_inputs; }
 };
 
 // The block's first GEMV: RMSNorm of the residual stream, from the fp32 vector or from the image the previous block left.
@@ -295,7 +296,7 @@ static void enqueue_mlp_block(Ctx &c, const Qwen35Decode::Plan::Block &b)
     op.seg[0].packed2 = b.up.data;
     if (c.prepared()) {
         op.seg[0].prep = c.prep_act();
-        op.seg[0].prep_partials = c.prep_sums() + 296; // second row: sums of squares of the SwiGLU output
+        if (!c.tcgen05()) op.seg[0].prep_partials = c.prep_sums() + 296; // second row: sums of squares of the SwiGLU output (range check of the fp16 image)
     }
     run_gemv(c, op);
 
@@ -304,7 +305,7 @@ static void enqueue_mlp_block(Ctx &c, const Qwen35Decode::Plan::Block &b)
     dn.cols = kInter;
     dn.prologue = c.prepared() ? INSG_PRO_PREPARED : INSG_PRO_PLAIN;
     if (c.prepared()) {
-        dn.prep_partials = c.prep_sums() + 296;
+        if (!c.tcgen05()) dn.prep_partials = c.prep_sums() + 296;
         dn.aux = c.x.gate;
     }
     dn.n_segments = 1;
@@ -409,6 +410,9 @@ struct Multi {
     // dn_first and the state after the second to dn_second (bases of [24][32][128][128]); null = the workspace's state in place
     const float *dn_in = nullptr;
     float *dn_first = nullptr, *dn_second = nullptr;
+    // passes of up to eight tokens on the tcgen05 kernel: products hand their results on as digit images (as in a token step)
+    bool prep = false, hidden_prepared = false;
+    const uint16_t *next_norm = nullptr; // weight of the RMSNorm that reads the block's output next
     int rows_hint = 0; // eager passes: the rows the pass's last token attends (the host's position + T); 0 inside a replayed graph
     explicit Multi(DecodeWorkspace &x, int t)
         : hidden(x.multi + kMultiHidden), qkv(x.multi + kMultiQkv), z(x.multi + kMultiZ), a(x.multi + kMultiA), b(x.multi + kMultiB),
@@ -418,26 +422,48 @@ struct Multi {
     }
 };
 
+// The RMSNorm'd residual stream as a product's input, and the residual stream left prepared for the RMSNorm that follows.
+void multi_input(const Ctx &c, insg_gemv_op &op, const Multi &u, const uint16_t *norm_w, bool ready)
+{
+    op.cols = kHidden;
+    op.tokens = u.T;
+    if (ready) {
+        op.in = static_cast<const float *>(c.prep_hidden());
+        op.prologue = INSG_PRO_PREPARED;
+        op.prep_partials = c.prep_sums();
+        op.prep_rms = 1;
+    } else {
+        op.in = u.hidden;
+        op.norm_w = norm_w;
+        op.prologue = INSG_PRO_RMSNORM;
+    }
+}
+void multi_output(const Ctx &c, insg_gemv_segment &s, const Multi &u, const uint16_t *following_norm_w)
+{
+    if (!u.prep || !following_norm_w) return;
+    s.prep = c.prep_hidden();
+    s.prep_w = following_norm_w;
+    s.prep_partials = c.prep_sums();
+}
+
 void mlp_block_multi(Ctx &c, const Qwen35Decode::Plan::Block &b, const Multi &u)
 {
     insg_gemv_op op = {};
-    op.in = u.hidden;
-    op.norm_w = b.post_norm;
-    op.cols = kHidden;
-    op.prologue = INSG_PRO_RMSNORM;
-    op.tokens = u.T;
+    multi_input(c, op, u, b.post_norm, u.prep);
     op.n_segments = 1;
     op.seg[0] = seg(b.gate, u.act, INSG_EPI_SWIGLU);
     op.seg[0].packed2 = b.up.data;
+    if (u.prep) op.seg[0].prep = c.prep_act();
     run_gemv(c, op);
 
     insg_gemv_op dn = {};
-    dn.in = u.act;
+    dn.in = u.prep ? static_cast<const float *>(c.prep_act()) : u.act;
     dn.cols = kInter;
-    dn.prologue = INSG_PRO_PLAIN;
+    dn.prologue = u.prep ? INSG_PRO_PREPARED : INSG_PRO_PLAIN;
     dn.tokens = u.T;
     dn.n_segments = 1;
     dn.seg[0] = seg(b.down, u.hidden, INSG_EPI_RESIDUAL);
+    multi_output(c, dn.seg[0], u, u.next_norm);
     run_gemv(c, dn);
 }
 
@@ -445,11 +471,7 @@ void delta_block_multi(Ctx &c, const Qwen35Decode::Plan::Block &b, int di, const
 {
     DecodeWorkspace &x = c.x;
     insg_gemv_op in = {};
-    in.in = u.hidden;
-    in.norm_w = b.in_norm;
-    in.cols = kHidden;
-    in.prologue = INSG_PRO_RMSNORM;
-    in.tokens = u.T;
+    multi_input(c, in, u, b.in_norm, u.hidden_prepared);
     in.n_segments = 4;
     in.seg[0] = seg(b.qkv, u.qkv, INSG_EPI_CONV_SILU);
     in.seg[0].conv_state = x.conv_state + size_t(di) * 8192 * 3;
@@ -481,6 +503,7 @@ void delta_block_multi(Ctx &c, const Qwen35Decode::Plan::Block &b, int di, const
     out.tokens = u.T;
     out.n_segments = 1;
     out.seg[0] = seg(b.out, u.hidden, INSG_EPI_RESIDUAL);
+    multi_output(c, out.seg[0], u, b.post_norm);
     run_gemv(c, out);
 
     mlp_block_multi(c, b, u);
@@ -490,11 +513,7 @@ void attention_block_multi(Ctx &c, const Qwen35Decode::Plan::Block &b, void *kc,
 {
     DecodeWorkspace &x = c.x;
     insg_gemv_op in = {};
-    in.in = u.hidden;
-    in.norm_w = b.in_norm;
-    in.cols = kHidden;
-    in.prologue = INSG_PRO_RMSNORM;
-    in.tokens = u.T;
+    multi_input(c, in, u, b.in_norm, u.hidden_prepared);
     in.n_segments = 3;
     in.seg[0] = seg(b.q, u.qg, INSG_EPI_STORE);
     in.seg[1] = seg(b.k, u.key, INSG_EPI_STORE);
@@ -531,6 +550,7 @@ void attention_block_multi(Ctx &c, const Qwen35Decode::Plan::Block &b, void *kc,
     o.tokens = u.T;
     o.n_segments = 1;
     o.seg[0] = seg(b.o, u.hidden, INSG_EPI_RESIDUAL);
+    multi_output(c, o.seg[0], u, b.post_norm);
     run_gemv(c, o);
 
     mlp_block_multi(c, b, u);
@@ -857,6 +877,7 @@ void Qwen35Decode::forward_tokens(const int *tokens, int count)
         c.layout = use_umma ? 1 : -1;
         const std::vector<Plan::Block> &blocks = use_umma && !one_layout ? p.layers_umma : p.layers;
         Multi u(x_, T);
+        u.prep = one_layout && x_.options.prepared_inputs && T <= kSmallChunk;
         if (use_umma || one_layout) u.rows_hint = x_.position + T; // eager passes only: a replayed graph must not bake the context length in
         sync_scalars(-1); // the chunk's first position; token m of the chunk sits at position + m
         cuda_check(cudaMemcpyAsync(u.tokens, tokens + done, size_t(T) * sizeof(int), cudaMemcpyHostToDevice, p.stream), "copy tokens");
@@ -865,6 +886,8 @@ void Qwen35Decode::forward_tokens(const int *tokens, int count)
                                                u.hidden, u.tokens, T, p.embed.rows, kHidden, c.pdl ? 1 : 0, p.stream));
             launches_++;
             for (int l = 0; l < n; l++) {
+                u.hidden_prepared = u.prep && l > 0;
+                u.next_norm = l + 1 < n ? blocks[l + 1].in_norm : nullptr;
                 if (Qwen35Shape::full_attention(l)) {
                     const size_t esz = x_.options.kv_bf16 ? 2 : 4;
                     const size_t off = size_t(l / 4) * x_.max_context * 1024 * esz;
@@ -1230,6 +1253,7 @@ std::vector<int> Qwen35Decode::generate_speculative(int first_token, int count, 
         if (draft < 0 || draft >= Qwen35Shape::vocab) throw std::runtime_error("draft token out of range");
         // ---- verify: tokens [tok, draft] at positions P, P + 1 ----
         Multi u(x_, 2);
+        u.prep = c.tcgen05() && c.prepared();
         u.dn_in = cur;
         u.dn_first = cur;
         u.dn_second = alt;
@@ -1246,6 +1270,8 @@ std::vector<int> Qwen35Decode::generate_speculative(int first_token, int count, 
                 launches_++;
             }
             for (int l = 0; l < n; l++) {
+                u.hidden_prepared = u.prep && l > 0;
+                u.next_norm = l + 1 < n ? p.layers[l + 1].in_norm : p.final_norm;
                 if (Qwen35Shape::full_attention(l)) {
                     const size_t off = size_t(l / 4) * x_.max_context * 1024 * (x_.options.kv_bf16 ? 2 : 4);
                     attention_block_multi(c, p.layers[l], reinterpret_cast<uint8_t *>(x_.kv_keys) + off, reinterpret_cast<uint8_t *>(x_.kv_values) + off, u);
@@ -1254,11 +1280,7 @@ std::vector<int> Qwen35Decode::generate_speculative(int first_token, int count, 
                 }
             }
             insg_gemv_op head = {};
-            head.in = u.hidden;
-            head.norm_w = p.final_norm;
-            head.cols = kHidden;
-            head.prologue = INSG_PRO_RMSNORM;
-            head.tokens = 2;
+            multi_input(c, head, u, p.final_norm, u.prep && n > 0);
             head.n_segments = 1;
             head.seg[0] = seg(p.lm_head, p.spec_logits, INSG_EPI_STORE);
             head.seg[0].rows = x_.options.vocab;
