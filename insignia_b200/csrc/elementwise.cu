@@ -156,8 +156,9 @@ __global__ void conv_rollback_kernel(float *state, const float *snapshot, size_t
     state[c * 3 + 2] = y1;
 }
 
-// One CTA per row of [count][stride] logits: the arg-max of its first n entries (lowest index on ties).
-__global__ void __launch_bounds__(1024) argmax_rows_kernel(const float *x, long long stride, int n, int *out);
+// [count][stride] logits: the arg-max of the first n entries of every row (lowest index on ties).
+constexpr int kArgmaxCtas = 8;
+__global__ void argmax_rows_kernel(const float *x, long long stride, int n, int *out);
 
 // A decode batch's step end: the arg-max of every sequence becomes its next input token and is logged under the
 // current position, which then advances.
@@ -235,32 +236,41 @@ static int check_launch(const char *what)
     return e == cudaSuccess ? INSG_OK : cuda_fail(e, what);
 }
 
-__global__ void __launch_bounds__(1024) argmax_rows_kernel(const float *x, long long stride, int n, int *out)
+// A cluster of eight CTAs takes a row (a row of logits is a megabyte: one CTA read it in 37 us); the CTAs' winners meet in
+// the first one's shared memory.
+__global__ void __cluster_dims__(kArgmaxCtas, 1, 1) __launch_bounds__(512) argmax_rows_kernel(const float *x, long long stride, int n, int *out)
 {
-    __shared__ float sv[32];
-    __shared__ int si[32];
-    x += size_t(blockIdx.x) * stride;
+    __shared__ float sv[16], cv[kArgmaxCtas];
+    __shared__ int si[16], ci[kArgmaxCtas];
+    const int rank = blockIdx.x % kArgmaxCtas;
+    x += size_t(blockIdx.x / kArgmaxCtas) * stride;
     float best = -3.402823466e38f;
     int idx = 0x7fffffff;
-    for (int i = threadIdx.x; i < n; i += 1024) {
-        const float v = __ldcg(x + i);
+    auto take = [&](float v, int i) {
         if (v > best || (v == best && i < idx)) { best = v; idx = i; }
-    }
+    };
+    pdl_wait();
+    const int per = (n + kArgmaxCtas - 1) / kArgmaxCtas, i0 = rank * per, i1 = min(n, i0 + per);
+#pragma unroll 8
+    for (int i = i0 + int(threadIdx.x); i < i1; i += 512) take(__ldcg(x + i), i);
 #pragma unroll
-    for (int m = 16; m; m >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, best, m);
-        const int oi = __shfl_xor_sync(0xffffffffu, idx, m);
-        if (ov > best || (ov == best && oi < idx)) { best = ov; idx = oi; }
-    }
+    for (int m = 16; m; m >>= 1) take(__shfl_xor_sync(0xffffffffu, best, m), __shfl_xor_sync(0xffffffffu, idx, m));
     if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = best; si[threadIdx.x >> 5] = idx; }
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < 32; w++)
-            if (sv[w] > best || (sv[w] == best && si[w] < idx)) { best = sv[w]; idx = si[w]; }
-        out[blockIdx.x] = idx;
+        for (int w = 1; w < 16; w++) take(sv[w], si[w]);
+        uint32_t v, i;
+        asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(v) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(&cv[rank]))));
+        asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(i) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(&ci[rank]))));
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(v), "f"(best) : "memory");
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(i), "r"(idx) : "memory");
+    }
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+    if (rank == 0 && threadIdx.x == 0) {
+        for (int c = 1; c < kArgmaxCtas; c++) take(cv[c], ci[c]);
+        out[blockIdx.x / kArgmaxCtas] = idx;
     }
 }
-
 
 } // namespace insg
 
@@ -364,8 +374,7 @@ int insg_conv_rollback(float *state, const float *snapshot, long long channels, 
 int insg_argmax_rows(const float *logits, long long stride, int n, int count, int *device_tokens, insg_stream_t stream)
 {
     if (!logits || !device_tokens || n <= 0 || count <= 0 || stride < n) return fail(INSG_E_ARG, "argmax_rows: bad argument");
-    argmax_rows_kernel<<<count, 1024, 0, stream>>>(logits, stride, n, device_tokens);
-    return check_launch("argmax_rows");
+    return launch(argmax_rows_kernel, dim3(count * kArgmaxCtas), dim3(512), 0, stream, true, logits, stride, n, device_tokens);
 }
 int insg_commit_tokens(const int *next, int *tokens, int *log, int capacity, int *position, int n, insg_stream_t stream)
 {

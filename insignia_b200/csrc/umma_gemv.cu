@@ -196,6 +196,8 @@ template <int T> __device__ __forceinline__ void load_partial(uint32_t taddr, fl
     }
 }
 
+template <int T> constexpr int kUnitSlots = T == 1 ? 4 : 2; // units whose exchange slots exist at once
+
 template <int T>
 __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_constant__ DParams p)
 {
@@ -204,10 +206,12 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     constexpr int kImg = kBKb + 512;    // a k-block of the image: digits, then their scale block
     constexpr int N = kDDigits * T;
     constexpr int kSlot = kDCl * 32 * T; // floats of one exchange slot: [source rank][32 rows][T]
+    // The four owner warps: with several tokens they split the tokens of a unit among them (TN each), else they take units in turn.
+    constexpr int TW = T < 4 ? T : 4, TN = T / TW, kGroups = 4 / TW, XU = kUnitSlots<T>;
     __shared__ __align__(8) uint64_t full[kDMaxStages], empty[kDMaxStages], dfull[2], dempty[2], xfull[8], xempty[8], ssfull, image[kDMaxKb / 8];
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort, s_last;
-    __shared__ float s_ssq[T * kDMaxKb], s_rss[kDCl * T], s_best[4];
+    __shared__ float s_ssq[T * kDMaxKb], s_rss[kDCl * T], s_scale[T], s_best[4];
     __shared__ int s_bidx[4];
     __shared__ uint8_t s_lut[84];
 
@@ -220,7 +224,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     const int nruns = nun * nmat, nstages = nruns * spt;
     uint8_t *ring = smem;                                // S stages
     uint8_t *bimg = ring + size_t(S) * kDStage; // len x kImg bytes
-    float *xslot = reinterpret_cast<float *>(bimg + size_t((nkb + 3) >> 2) * kImg); // 4 * nmat exchange slots
+    float *xslot = reinterpret_cast<float *>(bimg + size_t((nkb + 3) >> 2) * kImg); // XU * nmat exchange slots
     const bool prepared = p.prologue == INSG_PRO_PREPARED;
 
     // ---- the weight stream starts first: it depends on nothing ----------------------------------------------------------
@@ -250,7 +254,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     } else if (tid == 0) {
         for (int i = 0; i < 2; i++) { mbar_init(&dfull[i], 1); mbar_init(&dempty[i], 4); }
-        for (int i = 0; i < 8; i++) { mbar_init(&xfull[i], 1); mbar_init(&xempty[i], kDCl); }
+        for (int i = 0; i < 8; i++) { mbar_init(&xfull[i], 1); mbar_init(&xempty[i], kDCl * TW); }
         mbar_init(&ssfull, 1);
         for (int i = 0; i < kDMaxKb / 8; i++) mbar_init(&image[i], prepared ? 1u : uint32_t(T * max(1, min(8, len - 8 * i)))); // one arrival per (token, k-block), or the copy's
         s_abort = 0;
@@ -461,7 +465,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         // ---- accumulators -> partial sums -> the CTA that owns these 32 rows (rank = warp) ------------------------------------
         const uint32_t dst = map_to_rank(smem_u32(xslot) + uint32_t((rank * 32 + lane) * T * 4), uint32_t(warp));
         const uint32_t dbar = map_to_rank(smem_u32(xfull), uint32_t(warp));
-        const int nslots = 4 * nmat;
+        const int nslots = XU * nmat;
         bool ok = true;
         for (int run = 0; run < nruns && ok; run++) {
             const int buf = run & 1;
@@ -486,38 +490,34 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         }
     } else if (warp < 8) {
         // ---- owner of 32 rows of every tile: add the four parts in rank order, fused epilogue ----------------------------------
-        const int fw = warp - 4;
-        float best = -3.402823466e38f, scale[T];
+        const int fw = warp - 4, group = fw / TW, t0 = (fw % TW) * TN;
+        float best = -3.402823466e38f;
         int best_idx = 0x7fffffff;
         bool ok = true;
-#pragma unroll
-        for (int t = 0; t < T; t++) scale[t] = 1.f;
         // The quarters' sums of squares arrive while the weights are still being multiplied.  Every CTA waits for all four
         // (also where they are not needed), so that nobody leaves while a peer still writes into its shared memory.
         if (!prepared) ok = __all_sync(0xffffffffu, mbar_wait_cluster(&ssfull, 0, abort_flag));
-        if (prepared && p.prep_partials) {
-            const int groups = p.cols >> 5;
 #pragma unroll
-            for (int t = 0; t < T; t++) {
+        for (int u = 0; u < TN; u++) {
+            const int t = t0 + u;
+            float sc = 1.f;
+            if (prepared && p.prep_partials) {
+                const int groups = p.cols >> 5;
                 float ss = 0.f;
                 if (t < p.tokens)
                     for (int i = lane; i < groups; i += 32) ss += __ldcg(p.prep_partials + t * groups + i);
-                scale[t] = rsqrtf(warp_sum(ss) / float(p.cols) + 1e-6f);
+                sc = rsqrtf(warp_sum(ss) / float(p.cols) + 1e-6f);
+            } else if (p.prologue == INSG_PRO_RMSNORM) {
+                sc = rsqrtf((s_rss[t] + s_rss[T + t] + s_rss[2 * T + t] + s_rss[3 * T + t]) / float(p.cols) + 1e-6f);
             }
-        } else if (ok && p.prologue == INSG_PRO_RMSNORM) {
-#pragma unroll
-            for (int t = 0; t < T; t++) scale[t] = rsqrtf((s_rss[t] + s_rss[T + t] + s_rss[2 * T + t] + s_rss[3 * T + t]) / float(p.cols) + 1e-6f);
-            if (p.x_out && cl == 0) {
-                for (int m = 0; m < p.tokens; m++) {
-                    float sc = scale[0];
-#pragma unroll
-                    for (int t = 1; t < T; t++) sc = t == m ? scale[t] : sc;
-                    for (int k = kb0 * 128 + fw * 32 + lane; k < (kb0 + len) * 128; k += 128)
-                        p.x_out[size_t(m) * p.cols + k] = __ldcg(p.in + size_t(m) * p.cols + k) * sc * bf16_bits_to_float(p.norm_w[k]);
-                }
-            }
+            if (lane == 0) s_scale[t] = sc;
         }
-        for (int i = fw; i < nun && ok; i += 4) {
+        asm volatile("bar.sync 3, 128;" ::: "memory");
+        if (ok && p.x_out && cl == 0 && p.prologue == INSG_PRO_RMSNORM)
+            for (int m = 0; m < p.tokens; m++)
+                for (int k = kb0 * 128 + fw * 32 + lane; k < (kb0 + len) * 128; k += 128)
+                    p.x_out[size_t(m) * p.cols + k] = __ldcg(p.in + size_t(m) * p.cols + k) * s_scale[m] * bf16_bits_to_float(p.norm_w[k]);
+        for (int i = group; i < nun && ok; i += kGroups) {
             const int unit = cl + i * C;
             const DSeg &s = p.seg[dseg_of(p, unit)];
             const int row = (unit - s.tile_begin) * 128 + rank * 32 + lane;
@@ -525,48 +525,63 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             const size_t ld = size_t(s.rows);
             float *out = s.out + row;
             // the epilogue's other operands are fetched before the wait for the sums
-            float pre[T], h0 = 0.f, h1 = 0.f, h2 = 0.f;
+            float pre[TN], h0 = 0.f, h1 = 0.f, h2 = 0.f;
             float cw0 = 0.f, cw1 = 0.f, cw2 = 0.f, cw3 = 0.f;
             const float pw = s.prep_w ? bf16_bits_to_float(s.prep_w[row]) : 1.f; // rows % 128 == 0 where it is set
 #pragma unroll
-            for (int t = 0; t < T; t++) pre[t] = 0.f;
+            for (int u = 0; u < TN; u++) pre[u] = 0.f;
+            const bool one_history = s.conv_stride == 0; // consecutive tokens of one sequence
             if (on && s.epilogue == INSG_EPI_RESIDUAL) {
 #pragma unroll
-                for (int t = 0; t < T; t++)
-                    if (t < p.tokens) pre[t] = __ldcg(out + t * ld);
+                for (int u = 0; u < TN; u++)
+                    if (t0 + u < p.tokens) pre[u] = __ldcg(out + (t0 + u) * ld);
             } else if (on && s.epilogue == INSG_EPI_CONV_SILU) {
                 const uint2 wv = reinterpret_cast<const uint2 *>(s.conv_w)[row];
                 cw0 = bf16_bits_to_float(wv.x & 0xffff); cw1 = bf16_bits_to_float(wv.x >> 16);
                 cw2 = bf16_bits_to_float(wv.y & 0xffff); cw3 = bf16_bits_to_float(wv.y >> 16);
-                const float *hist = s.conv_state + size_t(row) * 3;
-                h0 = __ldcg(hist); h1 = __ldcg(hist + 1); h2 = __ldcg(hist + 2);
+                if (t0 < p.tokens) {
+                    const float *hist = s.conv_state + t0 * s.conv_stride + size_t(row) * 3;
+                    h0 = __ldcg(hist); h1 = __ldcg(hist + 1); h2 = __ldcg(hist + 2);
+                }
             } else if (on && s.epilogue == INSG_EPI_DECAY) {
                 h0 = bf16_bits_to_float(s.dt_bias[row]);
                 h1 = -__expf(s.A_log[row]);
             }
-            float y[2][T];
+            float y[2][TN];
 #pragma unroll
             for (int mat = 0; mat < 2; mat++) {
                 if (mat >= nmat) break;
-                const int slot = fw * nmat + mat;
-                if (lane == 0) mbar_expect_tx(&xfull[slot], kSlot * 4);
-                ok = __all_sync(0xffffffffu, mbar_wait_cluster(&xfull[slot], (i >> 2) & 1, abort_flag));
+                const int slot = (i % XU) * nmat + mat;
+                if (lane == 0 && t0 == 0) mbar_expect_tx(&xfull[slot], kSlot * 4);
+                ok = __all_sync(0xffffffffu, mbar_wait_cluster(&xfull[slot], (i / XU) & 1, abort_flag));
                 if (!ok) break;
                 const float *src = xslot + size_t(slot) * kSlot + lane * T;
-#pragma unroll
-                for (int t = 0; t < T; t++) {
+                auto sum = [&](int t) { // the four parts in rank order
                     float z = src[t];
 #pragma unroll
                     for (int r = 1; r < kDCl; r++) z += src[r * 32 * T + t];
-                    y[mat][t] = z * scale[t];
+                    return z * s_scale[t];
+                };
+#pragma unroll
+                for (int u = 0; u < TN; u++) y[mat][u] = sum(t0 + u);
+                if (T > 1 && one_history && s.epilogue == INSG_EPI_CONV_SILU) { // the history runs through the tokens: one warp takes them in order
+                    if (t0 == 0 && on) {
+                        for (int t = 0; t < p.tokens; t++) {
+                            const float raw = sum(t);
+                            out[t * ld] = fast_silu(fmaf(h0, cw0, fmaf(h1, cw1, fmaf(h2, cw2, raw * cw3))));
+                            h0 = h1; h1 = h2; h2 = raw;
+                        }
+                        float *hist = s.conv_state + size_t(row) * 3;
+                        hist[0] = h0; hist[1] = h1; hist[2] = h2;
+                    }
                 }
-                if (i + 4 < nun) { // the slot will be used again: tell the four senders
+                if (i + XU < nun) { // the slot will be used again: tell the four senders
                     __syncwarp();
                     if (lane < kDCl) remote_arrive(map_to_rank(smem_u32(&xempty[slot]), uint32_t(lane)));
                 }
             }
             if (!ok) break;
-            if (i + 4 >= nun) { // nothing more comes in for this warp: the peers need not wait for its epilogue
+            if (i + kGroups >= nun) { // nothing more comes in for this warp: the peers need not wait for its epilogue
                 cluster_arrive();
                 arrived = true;
             }
@@ -574,54 +589,52 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             switch (s.epilogue) {
             case INSG_EPI_STORE:
 #pragma unroll
-                for (int t = 0; t < T; t++)
-                    if (t < p.tokens) out[t * ld] = y[0][t];
+                for (int u = 0; u < TN; u++)
+                    if (t0 + u < p.tokens) out[(t0 + u) * ld] = y[0][u];
                 break;
             case INSG_EPI_RESIDUAL:
 #pragma unroll
-                for (int t = 0; t < T; t++)
-                    if (t < p.tokens) {
-                        const float v = pre[t] + y[0][t];
-                        out[t * ld] = v;
-                        if (s.prep) leave_digits<T>(s, v, pw, row, t, s_lut, lane);
+                for (int u = 0; u < TN; u++)
+                    if (t0 + u < p.tokens) {
+                        const float v = pre[u] + y[0][u];
+                        out[(t0 + u) * ld] = v;
+                        if (s.prep) leave_digits<T>(s, v, pw, row, t0 + u, s_lut, lane);
                     }
                 break;
             case INSG_EPI_CONV_SILU: {
-                float *hist = s.conv_state + size_t(row) * 3;
+                if (T > 1 && one_history) break; // done above
 #pragma unroll
-                for (int t = 0; t < T; t++) {
+                for (int u = 0; u < TN; u++) {
+                    const int t = t0 + u;
                     if (t < p.tokens) {
-                        if (t > 0 && s.conv_stride != 0) { // independent sequences: each token has its own history
-                            hist += s.conv_stride;
-                            h0 = __ldcg(hist); h1 = __ldcg(hist + 1); h2 = __ldcg(hist + 2);
-                        }
-                        const float z = fmaf(h0, cw0, fmaf(h1, cw1, fmaf(h2, cw2, y[0][t] * cw3)));
-                        h0 = h1; h1 = h2; h2 = y[0][t];
+                        float *hist = s.conv_state + t * s.conv_stride + size_t(row) * 3; // independent sequences: each token has its own
+                        if (u > 0) { h0 = __ldcg(hist); h1 = __ldcg(hist + 1); h2 = __ldcg(hist + 2); }
+                        const float z = fmaf(h0, cw0, fmaf(h1, cw1, fmaf(h2, cw2, y[0][u] * cw3)));
                         out[t * ld] = fast_silu(z);
-                        if (s.conv_stride != 0 || t + 1 == p.tokens) { hist[0] = h0; hist[1] = h1; hist[2] = h2; }
+                        hist[0] = h1; hist[1] = h2; hist[2] = y[0][u];
                     }
                 }
                 break;
             }
             case INSG_EPI_BETA:
 #pragma unroll
-                for (int t = 0; t < T; t++)
-                    if (t < p.tokens) out[t * ld] = fast_sigmoid(y[0][t]);
+                for (int u = 0; u < TN; u++)
+                    if (t0 + u < p.tokens) out[(t0 + u) * ld] = fast_sigmoid(y[0][u]);
                 break;
             case INSG_EPI_DECAY:
 #pragma unroll
-                for (int t = 0; t < T; t++) {
-                    const float z = y[0][t] + h0;
-                    if (t < p.tokens) out[t * ld] = h1 * (z > 20.f ? z : log1pf(__expf(z)));
+                for (int u = 0; u < TN; u++) {
+                    const float z = y[0][u] + h0;
+                    if (t0 + u < p.tokens) out[(t0 + u) * ld] = h1 * (z > 20.f ? z : log1pf(__expf(z)));
                 }
                 break;
             case INSG_EPI_SWIGLU:
 #pragma unroll
-                for (int t = 0; t < T; t++)
-                    if (t < p.tokens) {
-                        const float v = fast_silu(y[0][t]) * y[1][t];
-                        out[t * ld] = v;
-                        if (s.prep) leave_digits<T>(s, v, pw, row, t, s_lut, lane);
+                for (int u = 0; u < TN; u++)
+                    if (t0 + u < p.tokens) {
+                        const float v = fast_silu(y[0][u]) * y[1][u];
+                        out[(t0 + u) * ld] = v;
+                        if (s.prep) leave_digits<T>(s, v, pw, row, t0 + u, s_lut, lane);
                     }
                 break;
             case INSG_EPI_LOGITS:
@@ -818,7 +831,7 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     const int clusters = std::min(p.units, max_clusters);
     const int T = tokens == 1 ? 1 : tokens == 2 ? 2 : tokens <= 4 ? 4 : 8;
     const int kbq = (p.nkb + 3) >> 2;
-    const size_t fixed = size_t(kbq) * (512 * T + 512) + size_t(4) * p.nmat * kDCl * 32 * T * sizeof(float);
+    const size_t fixed = size_t(kbq) * (512 * T + 512) + size_t(T == 1 ? 4 : 2) * p.nmat * kDCl * 32 * T * sizeof(float);
     // ring: no more stages than the launch has, within half an SM when that leaves at least four, else whatever fits
     const int need = ((p.units + clusters - 1) / clusters) * p.nmat * ((kbq + 1) / 2);
     int stages = fixed < size_t(kDHalfSm) ? int((kDHalfSm - fixed) / kDStage) : 0;

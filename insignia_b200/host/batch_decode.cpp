@@ -203,10 +203,8 @@ void Qwen35BatchDecode::enqueue_step()
     };
     const uint32_t *ew = static_cast<const uint32_t *>(m.embed.weight.data);
     const uint8_t *es = static_cast<const uint8_t *>(m.embed.scales.data);
-    for (int s = 0; s < B; s++) {
-        insg_check(insg_mxfp4_embed(ew, es, m.hidden + size_t(s) * kHidden, m.d_tokens + s, m.embed.rows, kHidden, 1, st));
-        launches_++;
-    }
+    insg_check(insg_mxfp4_embed_tokens(ew, es, m.hidden, m.d_tokens, B, m.embed.rows, kHidden, 1, st));
+    launches_++;
     for (int l = 0; l < n; l++) {
         const DecodeBlock &blk = m.layers[size_t(l)];
         if (!Qwen35Shape::full_attention(l)) {

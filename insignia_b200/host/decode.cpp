@@ -1264,11 +1264,9 @@ std::vector<int> Qwen35Decode::generate_speculative(int first_token, int count, 
         const int which = cur == x_.delta_state ? 0 : 1;
         run_graphed(x_.options.use_graph, p.stream, p.exec_verify[which], p.verify_runs[which], launches_, [&] {
             cuda_check(cudaMemcpyAsync(p.spec_conv, x_.conv_state, conv_floats * sizeof(float), cudaMemcpyDeviceToDevice, p.stream), "snapshot history");
-            for (int m = 0; m < 2; m++) {
-                insg_check(insg_mxfp4_embed(static_cast<const uint32_t *>(p.embed.weight.data), static_cast<const uint8_t *>(p.embed.scales.data),
-                                            u.hidden + size_t(m) * kHidden, u.tokens + m, p.embed.rows, kHidden, 0, p.stream));
-                launches_++;
-            }
+            insg_check(insg_mxfp4_embed_tokens(static_cast<const uint32_t *>(p.embed.weight.data), static_cast<const uint8_t *>(p.embed.scales.data),
+                                               u.hidden, u.tokens, 2, p.embed.rows, kHidden, 0, p.stream));
+            launches_++;
             for (int l = 0; l < n; l++) {
                 u.hidden_prepared = u.prep && l > 0;
                 u.next_norm = l + 1 < n ? p.layers[l + 1].in_norm : p.final_norm;
