@@ -229,6 +229,7 @@ typedef struct insg_gemv_op {
     void *umma_scratch;         /* layout 1 with tokens > 8: device scratch of insg_umma_gemm_scratch_bytes(cols, tokens) for
                                    the activations' digit image, rewritten by every call                                      */
     size_t umma_scratch_bytes;
+    int *host_result;           /* INSG_EPI_LOGITS, layout 1: {winning row, *error_flag} also go here (pinned host memory), or NULL */
 } insg_gemv_op;
 
 INSG_API size_t insg_gemv_argmax_scratch_bytes(void);
@@ -312,6 +313,12 @@ INSG_API int insg_deltanet_decode_batch(float *state, long long state_stride, co
 INSG_API int insg_deltanet_decode_verify(const float *state, float *state_first, float *state_second, const float *q16,
                                          const float *k16, const float *v32, const float *g32, const float *beta32, float *out32,
                                          int qkv_stride, int pdl, insg_stream_t stream);
+/* insg_deltanet_decode_batch for 1..8 sequences that also leaves the out projection's input, rmsnorm(out) * norm_w * silu(z)
+ * per head (INSG_PRO_GATED_RMSNORM), as the digit image of a layout-1 launch: z at + s * 4096, image of
+ * insg_mxfp4_digit_image_bytes(4096, sequences) bytes. */
+INSG_API int insg_deltanet_decode_gated(float *state, long long state_stride, const float *q16, const float *k16, const float *v32,
+                                        const float *g32, const float *beta32, float *out32, int sequences, int qkv_stride,
+                                        const float *z, const uint16_t *norm_w, void *image, int pdl, insg_stream_t stream);
 /* Convolution history [channels][3] after a rejected second token: from the history after two tokens (`state`, in
  * place) and the history before them (`snapshot`).  No reference counterpart. */
 INSG_API int insg_conv_rollback(float *state, const float *snapshot, long long channels, insg_stream_t stream);
@@ -376,6 +383,9 @@ typedef struct insg_attn_op {
     int pdl;
     int *error_flag;          /* device int set to 1 if a bounded wait inside the kernel ran out (bf16 cache, long contexts:
                                  rows are staged by bulk copies with mbarrier completion), or NULL */
+    void *image;              /* optional: besides out, the o projection's input out * sigmoid(gate) as the digit image of a
+                                 layout-1 launch (insg_mxfp4_digit_image_bytes(4096, tokens), up to eight tokens or sequences) */
+    int gate_elementwise;     /* with image: 1 = INSG_PRO_SIGMOID_GATE_QPROJ, 0 = INSG_PRO_SIGMOID_GATE_HEAD0 (aux = qraw)       */
 } insg_attn_op;
 INSG_API int insg_attention_step(const insg_attn_op *op /* host */, insg_stream_t stream);
 /* `tokens` consecutive tokens of one sequence in two launches (prompt processing): op describes token 0 (rotary position

@@ -134,7 +134,7 @@ private:
     void enqueue_delta(int layer, bool hidden_prepared = false, const uint16_t *next_norm = nullptr);
     void enqueue_attention(int layer, bool hidden_prepared = false, const uint16_t *next_norm = nullptr);
     void enqueue_head(bool hidden_prepared = false);
-    void enqueue_token_step();
+    void enqueue_token_step(int from_layer = 0, int to_layer = Qwen35Shape::layers + 1);
     void replay_token_step();
     Qwen35Weights &w_;
     DecodeWorkspace &x_;
@@ -149,6 +149,8 @@ private:
     insg_program *rec_{};         // non-null while a program is being recorded
     uint64_t *gemv_bytes_{};      // optional byte counter of the GEMVs enqueued
     bool fused_token_valid_{};
+    bool result_to_host_{};       // the head being enqueued also writes its result to pinned host memory
+    bool result_on_host_{};       // the last head did
 };
 
 } // namespace insignia

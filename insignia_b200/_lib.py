@@ -25,13 +25,14 @@ class GemvOp(C.Structure):
     _fields_ = [("in_", vp), ("aux", vp), ("norm_w", vp), ("x_out", vp), ("cols", i32), ("prologue", i32),
                 ("n_segments", i32), ("seg", GemvSegment * 4), ("argmax_scratch", vp), ("token_out", vp),
                 ("token_feedback", vp), ("token_log", vp), ("token_log_capacity", i32), ("position_inout", vp), ("layout", i32), ("error_flag", vp), ("pdl", i32),
-                ("prep_partials", vp), ("prep_rms", i32), ("tokens", i32), ("umma_scratch", vp), ("umma_scratch_bytes", sz)]
+                ("prep_partials", vp), ("prep_rms", i32), ("tokens", i32), ("umma_scratch", vp), ("umma_scratch_bytes", sz), ("host_result", vp)]
 
 
 class AttnOp(C.Structure):
     _fields_ = [("qraw", vp), ("k_raw", vp), ("v", vp), ("q_norm_w", vp), ("k_norm_w", vp), ("k_cache", vp),
                 ("v_cache", vp), ("out", vp), ("position", vp), ("position_offset", i32), ("max_context", i32),
-                ("kv_dtype", i32), ("fast_trig", i32), ("scratch", vp), ("scratch_bytes", sz), ("pdl", i32), ("error_flag", vp)]
+                ("kv_dtype", i32), ("fast_trig", i32), ("scratch", vp), ("scratch_bytes", sz), ("pdl", i32), ("error_flag", vp), ("image", vp),
+                ("gate_elementwise", i32)]
 
 
 class EngineOptions(C.Structure):
@@ -81,6 +82,7 @@ SIGNATURES = {
     "insg_deltanet_decode_tokens": (i32, [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, vp]),
     "insg_deltanet_decode_batch": (i32, [vp, C.c_longlong, vp, vp, vp, vp, vp, vp, i32, i32, i32, vp]),
     "insg_deltanet_decode_verify": (i32, [vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, vp]),
+    "insg_deltanet_decode_gated": (i32, [vp, C.c_longlong] + [vp] * 6 + [i32, i32, vp, vp, vp, i32, vp]),
     "insg_conv_rollback": (i32, [vp, vp, C.c_longlong, vp]),
     "insg_gqa_scratch_bytes": (sz, [i32]),
     "insg_gqa_decode": (i32, [vp, vp, vp, vp, i32, i32, vp, sz, vp]),

@@ -184,6 +184,8 @@ template <bool BF16, bool FUSED> __global__ void __launch_bounds__(kAtThreads) a
     int t0 = split * chunk, t1 = min(tokens, t0 + chunk);
     int fresh = tokens - 1; // the row the producer (or this kernel) is still writing
 
+    __shared__ uint8_t s_lut[84];
+    if (p.image && tid < 81) s_lut[tid] = digit_pair_code(tid); // read behind the barriers below
     bool use_mma = BF16 && tokens >= kMmaMinTokens; // long bf16 contexts: the tensor-core loop (reads every row from the cache)
     if (tid == 0) s_abort = 0;
     GroupRaw<BF16, kGroup> ga, gb; // this warp's next two token groups, in flight while it works on earlier ones
@@ -425,6 +427,12 @@ template <bool BF16, bool FUSED> __global__ void __launch_bounds__(kAtThreads) a
         __syncthreads();
         // a thread owns four output dims of one head; the loads of different splits are independent
         const int h = tid >> 6, c4 = tid & 63;
+        float4 gv = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (p.image) { // element 0 of the head's gate for all of it, or element by element
+            const float *gsrc = p.gate + size_t(blockIdx.y) * 8192 + (kvh * 4 + h) * 512 + 256;
+            if (p.gate_elementwise) gv = __ldcg(reinterpret_cast<const float4 *>(gsrc) + c4);
+            else gv.x = gv.y = gv.z = gv.w = __ldcg(gsrc);
+        }
         const float4 *src = reinterpret_cast<const float4 *>(pp + 8 + h * 256) + c4;
         float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
@@ -437,7 +445,13 @@ template <bool BF16, bool FUSED> __global__ void __launch_bounds__(kAtThreads) a
             a.w = fmaf(v.w, e, a.w);
         }
         const float inv = 1.0f / s_lg[h];
-        reinterpret_cast<float4 *>(out_base + size_t(kvh * 4 + h) * 256)[c4] = make_float4(a.x * inv, a.y * inv, a.z * inv, a.w * inv);
+        a = make_float4(a.x * inv, a.y * inv, a.z * inv, a.w * inv);
+        reinterpret_cast<float4 *>(out_base + size_t(kvh * 4 + h) * 256)[c4] = a;
+        if (p.image) { // a warp holds half a head = one k-block of the o projection's input
+            const float gx[4] = {fast_sigmoid(gv.x), fast_sigmoid(gv.y), fast_sigmoid(gv.z), fast_sigmoid(gv.w)};
+            store_digits(make_float4(a.x * gx[0], a.y * gx[1], a.z * gx[2], a.w * gx[3]), p.slots, int(blockIdx.y),
+                         p.image + size_t((kvh * 4 + h) * 2 + (warp & 1)) * (512 * p.slots + 512), s_lut, lane);
+        }
         if (tid == 0) counters[kvh] = 0u;
     }
     if (tid == 0 && s_abort && p.error_flag) *p.error_flag = 1;
@@ -500,6 +514,15 @@ template <bool BF16> __global__ void __launch_bounds__(kAtThreads) attn_chunk_pr
             for (int j = 0; j < 8; j++) Row::store(p.vc, row + j, __ldcg(p.v_new + size_t(m) * 1024 + h * 256 + lane * 8 + j));
         }
     }
+}
+
+// The optional digit image of the gated output (see insg_attn_op.image).
+static void set_image(AttnParams &p, const insg_attn_op *op, int tokens)
+{
+    p.image = static_cast<uint8_t *>(op->image);
+    p.gate = op->qraw;
+    p.gate_elementwise = op->gate_elementwise;
+    p.slots = op->image ? image_slots(tokens) : 0;
 }
 
 size_t attn_scratch_bytes() { return 64 + size_t(4) * kSplits * kPartFloats * sizeof(float); }
@@ -595,6 +618,8 @@ int insg_attention_chunk(const insg_attn_op *op, int tokens, float *q_scratch, i
     // More than 32 tokens: query tiles on the tensor cores.  Fewer: the token-by-token form below, whose results are those of
     // single steps bit for bit (at 33 tokens the tile kernel still has only twelve CTAs; the two take the same time near 24).
     if (tokens > kTileFromTokens) return attn_tile_launch(p, q_scratch, tokens, bf16, stream, false);
+    if (op->image && tokens > 8) return fail(INSG_E_SHAPE, "attention_chunk: a digit image holds up to 8 tokens");
+    set_image(p, op, tokens);
     // step two: every (kv head, split, token) CTA is the plain split-K decode of its token over the rows up to its own
     p.q = q_scratch; p.q_stride = 4096; p.out_stride = 4096; p.scratch_stride = attn_scratch_bytes();
     p.counters = static_cast<unsigned *>(op->scratch);
@@ -625,6 +650,8 @@ int insg_attention_batch(const insg_attn_op *op, int sequences, size_t cache_str
     p.counters = static_cast<unsigned *>(op->scratch);
     p.partials = reinterpret_cast<float *>(static_cast<uint8_t *>(op->scratch) + 64);
     p.q_stride = 8192; p.out_stride = 4096; p.kvin_stride = 1024; p.scratch_stride = attn_scratch_bytes(); p.cache_stride = cache_stride_bytes;
+    if (op->image && sequences > 8) return fail(INSG_E_SHAPE, "attention_batch: a digit image holds up to 8 sequences");
+    set_image(p, op, sequences);
     const bool pdl = op->pdl != 0;
     return op->kv_dtype == INSG_KV_BF16 ? launch_attn<true, true>(p, stream, pdl, sequences) : launch_attn<false, true>(p, stream, pdl, sequences);
 }
@@ -643,6 +670,7 @@ int insg_attention_step(const insg_attn_op *op, insg_stream_t stream)
     p.max_context = op->max_context; p.fast_trig = op->fast_trig; p.error_flag = op->error_flag;
     p.counters = static_cast<unsigned *>(op->scratch);
     p.partials = reinterpret_cast<float *>(static_cast<uint8_t *>(op->scratch) + 64);
+    set_image(p, op, 1);
     const bool pdl = op->pdl != 0;
     return op->kv_dtype == INSG_KV_BF16 ? launch_attn<true, true>(p, stream, pdl) : launch_attn<false, true>(p, stream, pdl);
 }

@@ -33,6 +33,10 @@ struct AttnParams {
     // also takes k_raw + s * kvin_stride, v_new + s * kvin_stride and the caches at + s * cache_stride bytes
     int kvin_stride;
     size_t cache_stride;
+    // optional: out, gated, as the digit image of the tcgen05 kernel (token slot = blockIdx.y); gate = interleaved q_proj output
+    const float *gate;
+    uint8_t *image;
+    int slots, gate_elementwise;
     int *error_flag;       // set to 1 when a bounded wait inside the kernel ran out (bf16 tensor-core path), or null
 };
 

@@ -19,6 +19,7 @@
 // the eight warps cross a CTA barrier.
 #include "common.cuh"
 #include "host_util.h"
+#include "umma_common.cuh"
 
 namespace insg {
 
@@ -294,6 +295,100 @@ __global__ void __launch_bounds__(kDnThreads) deltanet_steps_kernel(float *__res
     }
 }
 
+// One step of several sequences (a decode batch), which also leaves the out projection's input: the gated RMSNorm over the head
+// (src/qwen_kernels.cu:5) as the digit image of the tcgen05 kernel.  With three sequences or more there are enough heads to
+// fill the device without slicing them, and a CTA that holds a whole head normalises its output without asking anybody (four
+// slices exchanging their sums through a cluster took 16 us at eight sequences, this form 6; the out projection's own
+// conversion, done again by each of its clusters, 6 us more than taking the image).  A warp holds 16 rows of the state, a lane four columns: the
+// sums over k need no shuffles, only one pass over the eight warps' partials.
+struct DnGate {
+    const float *z;          // [sequences][4096]
+    const uint16_t *norm_w;  // bf16 [128]
+    uint8_t *image;
+    int slots;
+};
+__global__ void __launch_bounds__(kDnThreads, 2) deltanet_heads_kernel(float *__restrict__ state, long long state_stride, const float *__restrict__ q16,
+                                                                       const float *__restrict__ k16, const float *__restrict__ v32,
+                                                                       const float *__restrict__ g32, const float *__restrict__ beta32,
+                                                                       float *__restrict__ out32, int qkv_stride, const DnGate gate)
+{
+    __shared__ __align__(16) float s_qk[8][2][128];
+    __shared__ __align__(16) float4 s_part[2][8][32];
+    __shared__ float s_ss[4];
+    __shared__ uint8_t s_lut[84];
+    const int head = blockIdx.x, seq = blockIdx.y, kh = head >> 1;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+
+    pdl_launch_dependents();
+    float *S = state + size_t(seq) * state_stride + size_t(head) * 128 * 128 + lane * 4;
+    float4 cell[16]; // rows warp + 8 j
+#pragma unroll
+    for (int j = 0; j < 16; j++) cell[j] = __ldcg(reinterpret_cast<const float4 *>(S + size_t(warp + 8 * j) * 128));
+    if (tid < 81) s_lut[tid] = digit_pair_code(tid);
+    const float gw = tid < 128 ? bf16_bits_to_float(gate.norm_w[tid]) : 0.f;
+    pdl_wait();
+    const size_t in = size_t(seq) * qkv_stride;
+    const float4 q4 = __ldcg(reinterpret_cast<const float4 *>(q16 + in + kh * 128) + lane);
+    const float4 k4 = __ldcg(reinterpret_cast<const float4 *>(k16 + in + kh * 128) + lane);
+    const float4 v4 = __ldcg(reinterpret_cast<const float4 *>(v32 + in + head * 128) + lane);
+    const float g_in = __ldcg(g32 + seq * 32 + head), beta = __ldcg(beta32 + seq * 32 + head);
+    const float zv = tid < 128 ? __ldcg(gate.z + size_t(seq) * 4096 + head * 128 + tid) : 0.f;
+    const float qn = warp_sum(fmaf(q4.x, q4.x, fmaf(q4.y, q4.y, fmaf(q4.z, q4.z, q4.w * q4.w))));
+    const float kn = warp_sum(fmaf(k4.x, k4.x, fmaf(k4.y, k4.y, fmaf(k4.z, k4.z, k4.w * k4.w))));
+    const float qs = rsqrtf(qn + 1e-6f) * 0.08838834764831845f, ks = rsqrtf(kn + 1e-6f);
+    reinterpret_cast<float4 *>(s_qk[warp][0])[lane] = make_float4(q4.x * qs, q4.y * qs, q4.z * qs, q4.w * qs);
+    reinterpret_cast<float4 *>(s_qk[warp][1])[lane] = make_float4(k4.x * ks, k4.y * ks, k4.z * ks, k4.w * ks);
+    __syncwarp();
+    const float decay = expf(g_in);
+    float4 pm = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < 16; j++) { // mem_v = sum_i (S*d) * k
+        const float kk = s_qk[warp][1][warp + 8 * j];
+        cell[j].x *= decay; cell[j].y *= decay; cell[j].z *= decay; cell[j].w *= decay;
+        pm.x = fmaf(cell[j].x, kk, pm.x);
+        pm.y = fmaf(cell[j].y, kk, pm.y);
+        pm.z = fmaf(cell[j].z, kk, pm.z);
+        pm.w = fmaf(cell[j].w, kk, pm.w);
+    }
+    s_part[0][warp][lane] = pm;
+    __syncthreads();
+    float4 mem = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+        const float4 t = s_part[0][w][lane];
+        mem.x += t.x; mem.y += t.y; mem.z += t.z; mem.w += t.w;
+    }
+    const float4 dl = make_float4((v4.x - mem.x) * beta, (v4.y - mem.y) * beta, (v4.z - mem.z) * beta, (v4.w - mem.w) * beta);
+    float4 po = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < 16; j++) { // S = S*d + k*delta ; out_v = sum_i S * q
+        const float kk = s_qk[warp][1][warp + 8 * j], qq = s_qk[warp][0][warp + 8 * j];
+        cell[j].x = fmaf(kk, dl.x, cell[j].x);
+        cell[j].y = fmaf(kk, dl.y, cell[j].y);
+        cell[j].z = fmaf(kk, dl.z, cell[j].z);
+        cell[j].w = fmaf(kk, dl.w, cell[j].w);
+        po.x = fmaf(cell[j].x, qq, po.x);
+        po.y = fmaf(cell[j].y, qq, po.y);
+        po.z = fmaf(cell[j].z, qq, po.z);
+        po.w = fmaf(cell[j].w, qq, po.w);
+        *reinterpret_cast<float4 *>(S + size_t(warp + 8 * j) * 128) = cell[j];
+    }
+    s_part[1][warp][lane] = po;
+    __syncthreads();
+    float o = 0.f;
+    if (tid < 128) { // column tid of the head
+        const float *part = reinterpret_cast<const float *>(s_part[1]);
+#pragma unroll
+        for (int w = 0; w < 8; w++) o += part[w * 128 + tid];
+        out32[size_t(seq) * 4096 + head * 128 + tid] = o;
+        const float ss = warp_sum(o * o);
+        if (lane == 0) s_ss[warp] = ss;
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        const float inv = rsqrtf((s_ss[0] + s_ss[1] + s_ss[2] + s_ss[3]) / 128.f + 1e-6f);
+        group_digits(o * inv * gw * fast_silu(zv), gate.slots, seq, gate.image, head * 4 + warp, s_lut, lane);
+    }
+}
+
 } // namespace insg
 
 using namespace insg;
@@ -337,4 +432,14 @@ extern "C" int insg_deltanet_decode_batch(float *state, long long state_stride, 
     if (sequences < 1 || sequences > 64 || qkv_stride < 0 || state_stride < 32 * 128 * 128) return fail(INSG_E_SHAPE, "deltanet: 1..64 sequences");
     return launch(deltanet_step_kernel, dim3(32 * kSlices, sequences), dim3(kDnThreads), 0, stream, pdl != 0, state, q16, k16, v32, g32,
                   beta32, out32, 1, qkv_stride, state_stride, nullptr, nullptr);
+}
+
+extern "C" int insg_deltanet_decode_gated(float *state, long long state_stride, const float *q16, const float *k16, const float *v32, const float *g32,
+                                          const float *beta32, float *out32, int sequences, int qkv_stride, const float *z, const uint16_t *norm_w,
+                                          void *image, int pdl, insg_stream_t stream)
+{
+    if (!state || !q16 || !k16 || !v32 || !g32 || !beta32 || !out32 || !z || !norm_w || !image) return fail(INSG_E_ARG, "deltanet: null pointer");
+    if (sequences < 1 || sequences > 8 || qkv_stride < 0 || state_stride < 32 * 128 * 128) return fail(INSG_E_SHAPE, "deltanet: 1..8 sequences");
+    return launch(deltanet_heads_kernel, dim3(32, sequences), dim3(kDnThreads), 0, stream, pdl != 0, state, state_stride, q16, k16, v32, g32, beta32,
+                  out32, qkv_stride, DnGate{z, norm_w, static_cast<uint8_t *>(image), image_slots(sequences)});
 }

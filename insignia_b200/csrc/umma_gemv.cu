@@ -69,7 +69,7 @@ struct DParams {
     DSeg seg[4];
     float2 *argmax_partial;
     unsigned *argmax_ticket;
-    int *token_out, *token_feedback, *token_log, *position_inout;
+    int *token_out, *token_feedback, *token_log, *position_inout, *host_result;
     int *error_flag;
     int token_log_capacity;
 };
@@ -124,40 +124,13 @@ __device__ __forceinline__ int dseg_of(const DParams &p, int unit)
     return s;
 }
 
-// The digits of one 128-element k-block of one token (four elements per lane) into the B image, and their group scales.
-// Image of a k-block: [2 K-steps][T column groups][2 k cores][8 columns][16 B]; a token's eight digit columns are one group.
-template <int T>
-__device__ __forceinline__ void store_digits(float4 x, int m, uint8_t *bkb, const uint8_t *lut, int lane)
-{
-    float mx = fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w)));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1)); // a group of 32 elements = 8 lanes
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-    int eb = int((__float_as_uint(mx) >> 23) & 0xffu);
-    eb = min(max(eb, 24), 230);
-    const float alpha = __uint_as_float(uint32_t(277 - eb) << 23); // largest element * alpha in [2^23, 2^24)
-    pack_digits(x, alpha, lut, bkb + (lane >> 4) * (256 * T) + m * 256 + ((lane >> 3) & 1) * 128 + (lane & 7) * 2);
-    const int n = 8 * m + (lane & 7); // scale block: row = column n of B (32 rows, then the next quarter), byte = group
-    bkb[512 * T + (n & 31) * 16 + (n >> 5) * 4 + (lane >> 3)] = uint8_t(eb - 23);
-}
-
 // One output row per lane into the digit image a later launch takes as its prepared input (the layout of store_digits): the
 // warp's 32 rows are one 32-element group of that launch's K.  Costs the producer some 50 instructions per token; converting
 // in the consumer would be done by every cluster again (eight tokens: 6 us per launch at 4096 columns, 17 at 12288).
 template <int T> __device__ __forceinline__ void leave_digits(const DSeg &s, float v, float w, int row, int m, const uint8_t *lut, int lane)
 {
-    const float x = v * w;
-    int eb = int(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(x))) >> 23);
-    eb = min(max(eb, 24), 230);
-    const uint32_t c = digit_codes81(x, __uint_as_float(uint32_t(277 - eb) << 23), lut), o = __shfl_xor_sync(0xffffffffu, c, 1);
-    // a pair of lanes holds two neighbouring k = one byte per column: the even lane stores columns 0, 2, 4, 6, the odd one the others
-    const uint32_t b = (lane & 1) ? ((o >> 4) & 0x0F0F0F0Fu) | (c & 0xF0F0F0F0u) : (c & 0x0F0F0F0Fu) | ((o & 0x0F0F0F0Fu) << 4);
-    const int grp = row >> 5, g = grp & 3;
-    uint8_t *kb = s.prep + size_t(grp >> 2) * (512 * T + 512), *dst = kb + (g >> 1) * (256 * T) + m * 256 + (g & 1) * 128 + (lane & 1) * 16 + (lane >> 1);
-#pragma unroll
-    for (int j = 0; j < 4; j++) dst[32 * j] = uint8_t(b >> (8 * j));
-    const int n = 8 * m + (lane & 7);
-    if (lane < 8) kb[512 * T + (n & 31) * 16 + (n >> 5) * 4 + g] = uint8_t(eb - 23);
+    const int grp = row >> 5;
+    group_digits(v * w, T, m, s.prep, grp, lut, lane);
     if (s.prep_partials) {
         const float ss = warp_sum(v * v);
         if (lane == 0) s.prep_partials[m * (s.rows >> 5) + grp] = ss;
@@ -358,7 +331,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 }
                 if (p.x_out && cl == 0 && !rms && m < p.tokens)
                     reinterpret_cast<float4 *>(p.x_out + size_t(m) * p.cols)[(kb0 + kb) * 32 + lane] = v;
-                store_digits<T>(v, m, bimg + size_t(kb) * kImg, s_lut, lane);
+                store_digits(v, T, m, bimg + size_t(kb) * kImg, s_lut, lane);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // the tensor core reads the image through the async proxy
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&image[kb >> 3]);
@@ -680,6 +653,10 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                     if (lane == 0) {
                         *p.token_out = best_idx;
                         if (p.token_feedback) *p.token_feedback = best_idx;
+                        if (p.host_result) { // a host that waits for the stream needs no copy behind it
+                            p.host_result[0] = best_idx;
+                            p.host_result[1] = p.error_flag ? __ldcg(p.error_flag) | (s_abort != 0) : 0;
+                        }
                         if (p.position_inout) {
                             const int pos = __ldcg(p.position_inout);
                             if (p.token_log && pos >= 0 && pos < p.token_log_capacity) p.token_log[pos] = best_idx;
@@ -821,6 +798,7 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
         p.argmax_ticket = static_cast<unsigned *>(op->argmax_scratch);
         p.argmax_partial = reinterpret_cast<float2 *>(static_cast<uint8_t *>(op->argmax_scratch) + 64);
         p.token_out = op->token_out; p.token_feedback = op->token_feedback; p.token_log = op->token_log; p.position_inout = op->position_inout;
+        p.host_result = op->host_result;
         p.token_log_capacity = op->token_log_capacity;
         if (op->token_log && op->token_log_capacity <= 0) return fail(INSG_E_ARG, "gemv: token_log needs its capacity");
     }

@@ -13,6 +13,9 @@ namespace insignia {
 namespace {
 constexpr int kHidden = Qwen35Shape::hidden, kInter = Qwen35Shape::intermediate;
 constexpr size_t kStateLayer = size_t(32) * 128 * 128, kConvLayer = size_t(8192) * 3;
+// From this many sequences on the DeltaNet step runs a whole head per CTA and leaves the out projection's input itself; below,
+// its heads are cut into slices (more CTAs) and the out projection converts its few vectors in its prologue.
+constexpr int kGatedSequences = 3;
 const char *const kLM = "language_model";
 
 void cuda_check(cudaError_t e, const char *what)
@@ -42,7 +45,7 @@ struct Qwen35BatchDecode::Impl {
     float *hidden{}, *qkv{}, *z{}, *a{}, *b{}, *core{}, *qg{}, *key{}, *value{}, *act{}, *logits{};
     float *delta_state{}, *conv_state{}; // [B][24][...]
     void *kv_keys{}, *kv_values{};       // [B][8][ctx][1024]
-    void *prep_hidden{}, *prep_act{};    // digit images of the residual stream and of the SwiGLU output for the next product
+    void *prep_hidden{}, *prep_act{}, *prep_core{}; // digit images of the residual stream, the SwiGLU output and the gated core for the next product
     float *prep_sums{};                  // [8][128] sums of squares of the residual stream
     void *attn_scratch{};                // [B][insg_gqa_scratch_bytes]
     size_t attn_scratch_each = 0, kv_seq_bytes = 0;
@@ -89,6 +92,7 @@ Qwen35BatchDecode::Qwen35BatchDecode(Qwen35Weights &weights, int sequences, int 
     m.attn_scratch_each = (insg_gqa_scratch_bytes(max_context) + 255) / 256 * 256;
     m.alloc(&m.attn_scratch, B * m.attn_scratch_each, "cudaMalloc batch attention scratch");
     m.alloc(&m.prep_hidden, insg_mxfp4_digit_image_bytes(kHidden, m.B), "cudaMalloc batch digit image");
+    m.alloc(&m.prep_core, insg_mxfp4_digit_image_bytes(4096, m.B), "cudaMalloc batch digit image");
     m.alloc(&m.prep_act, insg_mxfp4_digit_image_bytes(kInter, m.B), "cudaMalloc batch digit image");
     m.alloc(&m.prep_sums, B * (kHidden / 32) * f, "cudaMalloc batch sums");
     m.alloc(&m.d_tokens, (3 * B + 8) * sizeof(int), "cudaMalloc batch scalars");
@@ -222,15 +226,19 @@ void Qwen35BatchDecode::enqueue_step()
             in.seg[2].dt_bias = blk.dt_bias;
             in.seg[3] = seg(blk.b, m.b, INSG_EPI_BETA);
             gemv(in);
-            insg_check(insg_deltanet_decode_batch(m.delta_state + size_t(di) * kStateLayer, (long long)(24 * kStateLayer), m.qkv, m.qkv + 2048,
-                                                  m.qkv + 4096, m.a, m.b, m.core, B, 8192, 1, st));
+            if (B >= kGatedSequences)
+                insg_check(insg_deltanet_decode_gated(m.delta_state + size_t(di) * kStateLayer, (long long)(24 * kStateLayer), m.qkv, m.qkv + 2048,
+                                                      m.qkv + 4096, m.a, m.b, m.core, B, 8192, m.z, blk.dn_norm, m.prep_core, 1, st));
+            else
+                insg_check(insg_deltanet_decode_batch(m.delta_state + size_t(di) * kStateLayer, (long long)(24 * kStateLayer), m.qkv, m.qkv + 2048,
+                                                      m.qkv + 4096, m.a, m.b, m.core, B, 8192, 1, st));
             launches_++;
             insg_gemv_op out = {};
-            out.in = m.core;
+            out.in = B >= kGatedSequences ? static_cast<const float *>(m.prep_core) : m.core;
             out.aux = m.z;
             out.norm_w = blk.dn_norm;
             out.cols = 4096;
-            out.prologue = INSG_PRO_GATED_RMSNORM;
+            out.prologue = B >= kGatedSequences ? INSG_PRO_PREPARED : INSG_PRO_GATED_RMSNORM;
             out.n_segments = 1;
             out.seg[0] = seg(blk.out, m.hidden, INSG_EPI_RESIDUAL);
             residual_output(out.seg[0], blk.post_norm);
@@ -264,14 +272,15 @@ void Qwen35BatchDecode::enqueue_step()
                 // safe with dependent-launch overlap: the cache rows the launch fetches before its dependency wait were
                 // written a whole step ago
                 at.pdl = 1;
+                at.image = m.prep_core;
+                at.gate_elementwise = options_.gate_elementwise ? 1 : 0;
                 insg_check(insg_attention_batch(&at, B, m.kv_seq_bytes, st));
                 launches_++;
             }
             insg_gemv_op o = {};
-            o.in = m.core;
-            o.aux = m.qg;
+            o.in = static_cast<const float *>(m.prep_core);
             o.cols = 4096;
-            o.prologue = options_.gate_elementwise ? INSG_PRO_SIGMOID_GATE_QPROJ : INSG_PRO_SIGMOID_GATE_HEAD0;
+            o.prologue = INSG_PRO_PREPARED;
             o.n_segments = 1;
             o.seg[0] = seg(blk.o, m.hidden, INSG_EPI_RESIDUAL);
             residual_output(o.seg[0], blk.post_norm);

@@ -23,9 +23,11 @@ namespace insignia {
 namespace {
 
 constexpr int kHidden = Qwen35Shape::hidden, kInter = Qwen35Shape::intermediate;
-// DecodeWorkspace::prep: images of the normalised-to-be hidden vectors and of the SwiGLU outputs, sums of squares.  Sized for
+// DecodeWorkspace::prep: images of the normalised-to-be hidden vectors, of the SwiGLU outputs and of the gated cores, sums of squares.  Sized for
 // the digit images of eight tokens (insg_mxfp4_digit_image_bytes); the one-token fp16 images of the mma.sync kernel are smaller.
-constexpr size_t kPrepHidden = 0, kPrepAct = size_t(kHidden / 128) * (8 * 512 + 512), kPrepSums = kPrepAct + size_t(kInter / 128) * (8 * 512 + 512);
+constexpr size_t kPrepHidden = 0, kPrepAct = size_t(kHidden / 128) * (8 * 512 + 512), kPrepCore = kPrepAct + size_t(kInter / 128) * (8 * 512 + 512),
+                 kPrepSums = kPrepCore + size_t(kHidden / 128) * (8 * 512 + 512);
+constexpr int kFrontLayers = 2; // layers of the short first graph of a host-fed step: some 70 us of work, what submitting the rest takes
 constexpr int kMultiSteps = 8; // token steps per graph in Qwen35Decode::generate
 // DecodeWorkspace::multi: activations of up to kChunk consecutive tokens for Qwen35Decode::forward_tokens, [token][width] each
 constexpr int kChunk = 4;     // tokens per pass of the mma.sync kernel
@@ -143,6 +145,12 @@ struct Qwen35Decode::Plan {
     cudaGraphExec_t exec{};
     uint64_t graph_nodes = 0, chunk_nodes = 0;
     bool capturing = false, chunk_warm = false;
+    // the step as decode_token runs it, {token, position} as arguments of its first node: a short front part (embedding and
+    // the first kFrontLayers layers) and the rest, so that the device is busy while the long graph is being submitted
+    cudaGraph_t graph_front{};
+    cudaGraphExec_t exec_front{}, exec_rest{};
+    cudaGraphNode_t scalars_node{};
+    cudaKernelNodeParams scalars_params{};
     cudaGraphExec_t exec_multi{}; // kMultiSteps token steps in one graph, for device-fed generation
     cudaGraphExec_t exec_chunk{}; // one pass of forward_tokens over kChunk prompt tokens
     int *host_result{}; // pinned: {next token, wait-expired flag}, so the per-token read-back is a true asynchronous copy
@@ -164,7 +172,9 @@ Qwen35Decode::~Qwen35Decode()
     Plan &p = *plan_;
     cudaStreamSynchronize(p.stream);
     if (p.exec) cudaGraphExecDestroy(p.exec);
-    if (p.exec_multi) cudaGraphExecDestroy(p.exec_multi);
+    for (cudaGraphExec_t e : {p.exec_multi, p.exec_front, p.exec_rest})
+        if (e) cudaGraphExecDestroy(e);
+    if (p.graph_front) cudaGraphDestroy(p.graph_front);
     if (p.exec_chunk) cudaGraphExecDestroy(p.exec_chunk);
     if (p.graph) cudaGraphDestroy(p.graph);
     if (p.prog) insg_program_destroy(p.prog);
@@ -216,6 +226,8 @@ struct Ctx {
     int layout = -1;                     // >= 0: weight layout of the GEMVs issued (else the engine's gemv_tcgen05 option)
     void *prep_hidden() const { return static_cast<uint8_t *>(x.prep) + kPrepHidden; }
     void *prep_act() const { return static_cast<uint8_t *>(x.prep) + kPrepAct; }
+    void *prep_core() const { return static_cast<uint8_t *>(x.prep) + kPrepCore; }
+    bool core_prepared() const { return tcgen05() && prepared() && !gemv_only; } // the attention step leaves the next product's digits
     float *prep_sums() const { return reinterpret_cast<float *>(static_cast<uint8_t *>(x.prep) + kPrepSums); }
     bool tcgen05() const { return tcgen05_engine(x.options); }
     bool prepared() const { return x.options.prepared_inputs; }
@@ -380,6 +392,10 @@ static void enqueue_attention_block(Ctx &c, const Qwen35Decode::Plan::Block &b, 
     at.scratch = x.attn_scratch;
     at.scratch_bytes = insg_gqa_scratch_bytes(x.max_context);
     at.pdl = c.pdl ? 1 : 0;
+    if (c.core_prepared()) {
+        at.image = c.prep_core();
+        at.gate_elementwise = x.options.gate_elementwise ? 1 : 0;
+    }
     if (!c.gemv_only) {
         if (c.rec) insg_check(insg_program_add_attention(c.rec, &at));
         else insg_check(insg_attention_step(&at, c.st));
@@ -387,10 +403,10 @@ static void enqueue_attention_block(Ctx &c, const Qwen35Decode::Plan::Block &b, 
     }
 
     insg_gemv_op o = {};
-    o.in = x.core;
+    o.in = c.core_prepared() ? static_cast<const float *>(c.prep_core()) : x.core;
     o.aux = x.gate;
     o.cols = 4096;
-    o.prologue = x.options.gate_elementwise ? INSG_PRO_SIGMOID_GATE_QPROJ : INSG_PRO_SIGMOID_GATE_HEAD0;
+    o.prologue = c.core_prepared() ? INSG_PRO_PREPARED : x.options.gate_elementwise ? INSG_PRO_SIGMOID_GATE_QPROJ : INSG_PRO_SIGMOID_GATE_HEAD0;
     o.n_segments = 1;
     o.seg[0] = seg(b.o, x.hidden, INSG_EPI_RESIDUAL);
     residual_output(c, o.seg[0], b.post_norm);
@@ -539,14 +555,18 @@ void attention_block_multi(Ctx &c, const Qwen35Decode::Plan::Block &b, void *kc,
     at.error_flag = x.d_token + 3;
     at.scratch = x.attn_scratch;
     at.scratch_bytes = size_t(kAttnRegions) * insg_gqa_scratch_bytes(x.max_context);
+    if (u.prep) {
+        at.image = c.prep_core();
+        at.gate_elementwise = x.options.gate_elementwise ? 1 : 0;
+    }
     insg_check(insg_attention_chunk(&at, u.T, u.qn, u.rows_hint, c.st));
     c.launches += 2;
 
     insg_gemv_op o = {};
-    o.in = u.core;
+    o.in = u.prep ? static_cast<const float *>(c.prep_core()) : u.core;
     o.aux = u.qg;
     o.cols = 4096;
-    o.prologue = x.options.gate_elementwise ? INSG_PRO_SIGMOID_GATE_QPROJ : INSG_PRO_SIGMOID_GATE_HEAD0;
+    o.prologue = u.prep ? INSG_PRO_PREPARED : x.options.gate_elementwise ? INSG_PRO_SIGMOID_GATE_QPROJ : INSG_PRO_SIGMOID_GATE_HEAD0;
     o.tokens = u.T;
     o.n_segments = 1;
     o.seg[0] = seg(b.o, u.hidden, INSG_EPI_RESIDUAL);
@@ -669,6 +689,7 @@ void Qwen35Decode::enqueue_head(bool hidden_prepared)
     op.token_log = x_.d_token + 4;
     op.token_log_capacity = x_.max_context + 1;
     op.position_inout = x_.d_position;
+    if (result_to_host_ && c.tcgen05()) op.host_result = p.host_result;
     run_gemv(c, op);
 }
 
@@ -697,21 +718,21 @@ void Qwen35Decode::layer(int l)
     else delta_layer(l);
 }
 
-// embed, all layers, head: what one graph replay does
-void Qwen35Decode::enqueue_token_step()
+// embed, all layers, head: what one graph replay does (the embedding belongs to layer 0, the head to the layer past the last)
+void Qwen35Decode::enqueue_token_step(int from, int to)
 {
     Plan &p = plan();
     const int n = x_.options.n_layers;
     for (int l = 0; l < n; l++) load_block(l); // every block's norm weight is needed by the block before it
     load_head();
-    enqueue_embed();
-    for (int l = 0; l < n; l++) {
+    if (from == 0) enqueue_embed();
+    for (int l = from; l < std::min(n, to); l++) {
         // inside the token step nobody touches hidden between two blocks: each block leaves the next one's input prepared
         const uint16_t *next_norm = l + 1 < n ? p.layers[l + 1].in_norm : p.final_norm;
         if (Qwen35Shape::full_attention(l)) enqueue_attention(l, l > 0, next_norm);
         else enqueue_delta(l, l > 0, next_norm);
     }
-    enqueue_head(n > 0);
+    if (to > n) enqueue_head(n > 0);
 }
 
 // Records the token step as a program (every weight is made resident first: uploads and repacks allocate and
@@ -829,6 +850,46 @@ void Qwen35Decode::replay_token_step()
         const cudaError_t e = cudaGraphInstantiate(&p.exec_multi, g, 0);
         cudaGraphDestroy(g);
         cuda_check(e, "instantiate graph");
+        if (tcgen05_engine(x_.options)) {
+            // the host-fed step in two graphs
+            const int cut = std::min(kFrontLayers, x_.options.n_layers);
+            auto record = [&](cudaGraph_t *out, auto &&body) {
+                *out = nullptr;
+                cuda_check(cudaStreamBeginCapture(p.stream, cudaStreamCaptureModeThreadLocal), "begin graph capture");
+                try {
+                    body();
+                } catch (...) {
+                    cudaStreamEndCapture(p.stream, out);
+                    if (*out) cudaGraphDestroy(*out);
+                    *out = nullptr;
+                    throw;
+                }
+                cuda_check(cudaStreamEndCapture(p.stream, out), "end graph capture");
+            };
+            record(&p.graph_front, [&] {
+                sync_scalars(0);
+                enqueue_token_step(0, cut);
+            });
+            cudaGraph_t rest = nullptr;
+            result_to_host_ = true;
+            try {
+                record(&rest, [&] { enqueue_token_step(cut); });
+            } catch (...) {
+                result_to_host_ = false;
+                throw;
+            }
+            result_to_host_ = false;
+            launches_ = before;
+            const cudaError_t er = cudaGraphInstantiate(&p.exec_rest, rest, 0);
+            cudaGraphDestroy(rest);
+            cuda_check(er, "instantiate graph");
+            cuda_check(cudaGraphInstantiate(&p.exec_front, p.graph_front, 0), "instantiate graph");
+            size_t roots = 1;
+            cuda_check(cudaGraphGetRootNodes(p.graph_front, &p.scalars_node, &roots), "graph root");
+            cuda_check(cudaGraphKernelNodeGetParams(p.scalars_node, &p.scalars_params), "graph root parameters");
+            cuda_check(cudaGraphUpload(p.exec_front, p.stream), "upload graph");
+            cuda_check(cudaGraphUpload(p.exec_rest, p.stream), "upload graph");
+        }
         // upload now: otherwise the first launch of each graph pays for it
         cuda_check(cudaGraphUpload(p.exec, p.stream), "upload graph");
         cuda_check(cudaGraphUpload(p.exec_multi, p.stream), "upload graph");
@@ -843,9 +904,23 @@ void Qwen35Decode::forward_token(int token)
     if (x_.position >= x_.max_context) throw std::runtime_error("KV cache full"); // also bounds the token log
     if (persistent()) {
         run_program(1, token);
+        result_on_host_ = false;
+    } else if (plan().exec_front) {
+        Plan &p = plan();
+        int position = x_.position, *dt = x_.d_token, *dp = x_.d_position;
+        void *args[] = {&dt, &token, &dp, &position};
+        cudaKernelNodeParams k = p.scalars_params;
+        k.kernelParams = args;
+        k.extra = nullptr;
+        cuda_check(cudaGraphExecKernelNodeSetParams(p.exec_front, p.scalars_node, &k), "set token");
+        cuda_check(cudaGraphLaunch(p.exec_front, p.stream), "launch graph");
+        cuda_check(cudaGraphLaunch(p.exec_rest, p.stream), "launch graph");
+        launches_ += p.graph_nodes + 1;
+        result_on_host_ = true;
     } else {
         sync_scalars(token);
         replay_token_step();
+        result_on_host_ = false;
     }
     x_.position++;
     fused_token_valid_ = true;
@@ -934,9 +1009,12 @@ void Qwen35Decode::forward_tokens(const int *tokens, int count)
     // arg-max, so logits_argmax() needs no further launch
     x_.position--;
     sync_scalars(tokens[count - 1]);
+    result_to_host_ = true;
     enqueue_head(false);
+    result_to_host_ = false;
     x_.position++;
     fused_token_valid_ = true;
+    result_on_host_ = one_layout;
     p.capturing = true; // every weight is resident now: the next forward_token may capture its graph
 }
 
@@ -959,10 +1037,12 @@ int Qwen35Decode::logits_argmax()
         insg_check(insg_argmax_logits(x_.logits, x_.options.vocab, x_.d_next, p.stream));
         launches_++;
     }
-    int *result = p.host_result; // next token, kernel wait-expired flag
-    result[0] = -1;
-    result[1] = 0;
-    cuda_check(cudaMemcpyAsync(result, x_.d_next, 2 * sizeof(int), cudaMemcpyDeviceToHost, p.stream), "read token");
+    int *result = p.host_result; // next token, kernel wait-expired flag: the head may have written them itself
+    if (!fused_token_valid_ || !result_on_host_) {
+        result[0] = -1;
+        result[1] = 0;
+        cuda_check(cudaMemcpyAsync(result, x_.d_next, 2 * sizeof(int), cudaMemcpyDeviceToHost, p.stream), "read token");
+    }
     cuda_check(cudaStreamSynchronize(p.stream), "synchronize");
     if (result[1]) {
         recover_after_timeout();
@@ -990,6 +1070,7 @@ std::vector<int> Qwen35Decode::generate(int first_token, int count)
         run_program(count, first_token);
         x_.position += count;
         fused_token_valid_ = true;
+        result_on_host_ = false;
         int *flag = p.host_result + 1;
         *flag = 0;
         cuda_check(cudaMemcpyAsync(out.data(), x_.d_token + 4 + start, size_t(count) * sizeof(int), cudaMemcpyDeviceToHost, p.stream),
@@ -1019,6 +1100,7 @@ std::vector<int> Qwen35Decode::generate(int first_token, int count)
         }
     }
     fused_token_valid_ = true;
+    result_on_host_ = false;
     cuda_check(cudaMemcpyAsync(out.data(), x_.d_token + 4 + start, size_t(count) * sizeof(int), cudaMemcpyDeviceToHost, p.stream),
                "read tokens");
     cuda_check(cudaStreamSynchronize(p.stream), "synchronize");
@@ -1185,6 +1267,7 @@ int Qwen35Decode::mtp_step(int token, bool draft)
         op.seg[0].rows = x_.options.vocab;
         op.argmax_scratch = x_.argmax_scratch;
         op.token_out = x_.d_next;
+        if (c.tcgen05()) op.host_result = p.host_result;
         run_gemv(c, op);
     });
     if (!draft) {
@@ -1192,6 +1275,7 @@ int Qwen35Decode::mtp_step(int token, bool draft)
         return -1;
     }
     fused_token_valid_ = true;
+    result_on_host_ = tcgen05_engine(x_.options);
     return logits_argmax();
 }
 
