@@ -7,16 +7,17 @@
 // (which fails past ~12K tokens) and re-reads each kv head's cache four times.
 // Here a CTA owns (kv head, token range): it streams its slab of K and V exactly
 // once for the four query heads that share the kv head, keeps an online softmax
-// per warp, and leaves (max, denominator, weighted V) partials in scratch; the
-// last CTA to finish for a kv head folds the partials in split order, so results
-// do not depend on scheduling.  The fused entry also does the per-head RMSNorm,
+// per warp, and hands (max, denominator, weighted V) to the CTAs of its cluster
+// (and, where one cluster is not enough, through scratch to the other clusters);
+// partials are folded in split order, so results do not depend on scheduling.  The fused entry also does the per-head RMSNorm,
 // partial RoPE and the cache write of the current token (src/ops.cu:9,
 // src/qwen_kernels.cu:15,31) so one launch replaces five.
 //
 // bf16 cache, long contexts: the scalar loop is bound by instruction issue (half the bytes, the same instructions),
 // so from kMmaMinTokens cached rows on the warps score and accumulate on the tensor cores instead (mma.sync
-// m16n8k16 bf16, fp32 accumulation): 16 cached rows per step per warp, fetched into the warp's own shared-memory tile
-// by one cp.async.bulk per lane (16 key rows + 16 value rows, mbarrier completion, bounded wait); the fp32 query goes in
+// m16n8k16 bf16, fp32 accumulation): 16 cached rows per step per warp, fetched into the warp's own shared-memory
+// tiles by one cp.async.bulk per row (keys and values on an mbarrier each, the next tile of one requested while the other is
+// worked on; bounded waits); the fp32 query goes in
 // as two bf16 pieces (hi + lo) in the eight N columns (4 heads x 2 pieces), the softmax weights likewise for P.V, so
 // products keep ~16 bits of the fp32 operands and the cache values are exact.
 #include "attention_body.cuh"
@@ -64,9 +65,27 @@ __device__ __forceinline__ void attn_mma_warp(const void *kc, const void *vc, in
     uint8_t *tile_k = tiles + size_t(warp) * 2 * kTileBytes, *tile_v = tile_k + kTileBytes;
     if (lane == 0) {
         mbar_init(bar, 1);
+        mbar_init(bar + 1, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
+    // Keys and values have a barrier each: a tile of keys is requested as soon as the one before has been scored, a tile of values
+    // as soon as the one before has been added, so that one of the two is on its way whatever the warp does.
+    auto request = [&](const void *cache, uint8_t *tile, uint64_t *b, int tb) {
+        __syncwarp();
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // the tile was read by ordinary loads; the copies below overwrite it
+        if (lane == 0) mbar_expect_tx(b, 16 * 512);
+        __syncwarp();
+        if (lane < 16) {
+            const int tok = min(tb + lane, t1 - 1); // rows past the split repeat its last row: masked below
+            bulk_load(tile + lane * kTileRow, static_cast<const uint8_t *>(cache) + (size_t(tok) * 4 + kvh) * 512, 512, b);
+        }
+    };
+    const int first = t0 + 16 * warp;
+    if (first < t1) {
+        request(kc, tile_k, bar, first);
+        request(vc, tile_v, bar + 1, first);
+    }
     // the query as the B operand: column g = (head g >> 1, piece g & 1), k rows 2t, 2t+1 and 2t+8, 2t+9 of every 16 dims
     uint32_t qb[16][2];
     {
@@ -87,17 +106,11 @@ __device__ __forceinline__ void attn_mma_warp(const void *kc, const void *vc, in
     const uint32_t k_addr = smem_u32(tile_k) + ((lm_id & 1) * 8 + lm_row) * kTileRow + (lm_id >> 1) * 16; // + 32 i: rows of K as m, dims as k
     const uint32_t v_addr = smem_u32(tile_v) + ((lm_id >> 1) * 8 + lm_row) * kTileRow + (lm_id & 1) * 16; // + 32 j: transposed: dims as m, rows as k
     for (int tb = t0 + 16 * warp; tb < t1; tb += 16 * kAtWarps) {
-        __syncwarp();
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // the tile was read by ordinary loads; the copies below overwrite it
-        if (lane == 0) mbar_expect_tx(bar, 32 * 512);
-        __syncwarp();
-        {
-            const int r = lane & 15, tok = min(tb + r, t1 - 1); // rows past the split repeat its last row: masked below
-            const uint8_t *src = static_cast<const uint8_t *>(lane < 16 ? kc : vc) + (size_t(tok) * 4 + kvh) * 512;
-            bulk_load((lane < 16 ? tile_k : tile_v) + r * kTileRow, src, 512, bar);
+        const int tn = tb + 16 * kAtWarps;
+        if (!mbar_wait(bar, phase, abort_flag)) {
+            mbar_wait(bar + 1, phase, abort_flag); // the values' copy, before the tile's memory is given up
+            break;
         }
-        if (!mbar_wait(bar, phase, abort_flag)) break;
-        phase ^= 1u;
         // ---- scores: S[16 rows][8 columns] = K tile . q pieces ----
         float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -106,6 +119,7 @@ __device__ __forceinline__ void attn_mma_warp(const void *kc, const void *vc, in
             asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(a0), "=r"(a1), "=r"(a2), "=r"(a3) : "r"(k_addr + 32 * i));
             mma_bf16(c, a0, a1, a2, a3, qb[i][0], qb[i][1]);
         }
+        if (tn < t1) request(kc, tile_k, bar, tn);
         const bool v0 = tb + g < t1, v1 = tb + g + 8 < t1;
         const float s0 = v0 ? c[0] + c[1] : -3.0e38f, s1 = v1 ? c[2] + c[3] : -3.0e38f; // rows tb + g and tb + g + 8, head t
         float mx = fmaxf(s0, s1);
@@ -123,12 +137,18 @@ __device__ __forceinline__ void attn_mma_warp(const void *kc, const void *vc, in
         const float x0 = __shfl_sync(0xffffffffu, p0, src_a), x1 = __shfl_sync(0xffffffffu, p0, src_b);
         const float y0 = __shfl_sync(0xffffffffu, p1, src_a), y1 = __shfl_sync(0xffffffffu, p1, src_b);
         const uint32_t pb0 = bf16_piece_pair(x0, x1, g & 1), pb1 = bf16_piece_pair(y0, y1, g & 1);
+        if (!mbar_wait(bar + 1, phase, abort_flag)) {
+            if (tn < t1) mbar_wait(bar, phase ^ 1u, abort_flag); // the next keys' copy
+            break;
+        }
+        phase ^= 1u;
 #pragma unroll
         for (int j = 0; j < 16; j++) {
             uint32_t a0, a1, a2, a3;
             asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(a0), "=r"(a1), "=r"(a2), "=r"(a3) : "r"(v_addr + 32 * j));
             mma_bf16(acc[j], a0, a1, a2, a3, pb0, pb1);
         }
+        if (tn < t1) request(vc, tile_v, bar + 1, tn);
     }
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 4);
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 8);
@@ -141,23 +161,49 @@ __device__ __forceinline__ void attn_mma_warp(const void *kc, const void *vc, in
     }
 }
 
-template <bool BF16, bool FUSED> __global__ void __launch_bounds__(kAtThreads) attn_splitk_kernel(const __grid_constant__ AttnParams p)
+// Clusters: a kv head's cache is cut over clusters of CL CTAs.  The CTAs of a cluster exchange their partial results through
+// distributed shared memory, each finishing its share of the output dims: a context that one cluster holds needs no global
+// scratch, fence or ticket.  Longer ones use up to `clusters` clusters per head; their results go to scratch and the last one
+// to arrive (a ticket per CTA rank) folds them in order.  The cut depends on the row count alone, so that a token gives the
+// same bits in a single step, a chunk or a batch whenever those launch the same clusters.
+// Measured (fp32 cache, one step): 40 rows 5.2 us (7.1 with one CTA per split and a ticket), 8 x 600 rows 13.5 (38.5),
+// 8 x 5000 rows 57 (119.5, 88 % of the copy peak); 1024 rows 9.9 (9.5).
+constexpr int kCtaRows = 48;    // rows per CTA from which another cluster is put to work (32, 48, 64, 96 tried: 48 is best or next to it)
+constexpr int kMaxClusters = 8; // per kv head
+
+struct AttnCut {
+    int active, chunk; // clusters at work, rows per CTA
+};
+template <int CL> __device__ __forceinline__ AttnCut attn_cut(int rows, int clusters)
+{
+    AttnCut c;
+    c.active = min(clusters, (rows + kCtaRows * CL - 1) / (kCtaRows * CL));
+    const int ctas = c.active * CL;
+    c.chunk = max(kMinChunk, (rows + ctas - 1) / ctas);
+    return c;
+}
+
+template <bool BF16, bool FUSED, int CL>
+__global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid_constant__ AttnParams p, int clusters)
 {
     using Row = KvRow<BF16>;
+    constexpr int kMine = 1024 / CL; // output dims this CTA finishes
     __shared__ __align__(16) float s_q[4][256];
     __shared__ __align__(16) float s_knew[256], s_vnew[256];
     __shared__ float s_m[kAtWarps][4], s_l[kAtWarps][4];
     __shared__ __align__(16) float s_acc[kAtWarps][4][256];
+    __shared__ __align__(16) float s_in[CL][kMine]; // the cluster's partial sums of this CTA's dims
+    __shared__ float s_min[CL], s_lin[CL];          // and their maxima and denominators
     __shared__ int s_last;
-    __shared__ float s_e[64][4], s_lg[4];
-    __shared__ __align__(8) uint64_t s_bar[kAtWarps];
+    __shared__ __align__(8) uint64_t s_bar[2 * kAtWarps];
     __shared__ int s_abort;
+    __shared__ uint8_t s_lut[84];
     extern __shared__ __align__(128) uint8_t s_tiles[]; // bf16 cache only: per warp a key tile and a value tile
 
-    const int ns = int(gridDim.x) >> 2; // splits launched per kv head (37, or fewer when the host knows the context is short)
-    const int kvh = blockIdx.x / ns, split = blockIdx.x % ns;
+    const int rank = int(blockIdx.x) % CL, cluster = int(blockIdx.x) / CL % clusters, kvh = int(blockIdx.x) / (CL * clusters);
+    const int split = cluster * CL + rank;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // token of a chunk (plain form only; a single launch has blockIdx.y == 0 and zero strides)
+    // token of a chunk (plain form) or sequence of a batch (fused form); a single launch has blockIdx.y == 0 and zero strides
     const int bt = blockIdx.y;
     const float *q_in = p.q + size_t(bt) * p.q_stride;
     float *out_base = p.out + size_t(bt) * p.out_stride;
@@ -167,6 +213,7 @@ template <bool BF16, bool FUSED> __global__ void __launch_bounds__(kAtThreads) a
     const float *k_raw = p.k_raw + size_t(bt) * p.kvin_stride, *v_new = p.v_new + size_t(bt) * p.kvin_stride;
 
     pdl_launch_dependents();
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory"); // the peers have started when this completes
 
     // Geometry from the position as it is visible now.  Cache rows of earlier tokens never change
     // again, so the first token group of every warp is fetched while the producer of q still runs;
@@ -179,20 +226,18 @@ template <bool BF16, bool FUSED> __global__ void __launch_bounds__(kAtThreads) a
         tokens = __ldcg(p.position) + p.position_offset + bt + 1;
     }
     tokens = max(1, min(tokens, p.max_context)); // host checks; never index past the cache
-    int chunk = max(kMinChunk, (tokens + kSplits - 1) / kSplits);
-    int nsplit = (tokens + chunk - 1) / chunk;
-    int t0 = split * chunk, t1 = min(tokens, t0 + chunk);
+    AttnCut cut = attn_cut<CL>(tokens, clusters);
+    int t0 = split * cut.chunk, t1 = min(tokens, t0 + cut.chunk);
     int fresh = tokens - 1; // the row the producer (or this kernel) is still writing
 
-    __shared__ uint8_t s_lut[84];
     if (p.image && tid < 81) s_lut[tid] = digit_pair_code(tid); // read behind the barriers below
     bool use_mma = BF16 && tokens >= kMmaMinTokens; // long bf16 contexts: the tensor-core loop (reads every row from the cache)
     if (tid == 0) s_abort = 0;
-    GroupRaw<BF16, kGroup> ga, gb; // this warp's next two token groups, in flight while it works on earlier ones
-    if (!use_mma) {
-        load_group<BF16, kGroup>(kc, vc, kvh, t0 + warp * kGroup, min(t1, fresh), lane, ga);
-        load_group<BF16, kGroup>(kc, vc, kvh, t0 + (warp + kAtWarps) * kGroup, min(t1, fresh), lane, gb);
-    }
+    // This warp's next token group: its keys are replaced by the following group's as soon as they are scored, its values as soon
+    // as they are added.  One group (two would take a CTA's registers past what fits beside the products' launches, and the
+    // launch could start only when its predecessor had left the SM).
+    GroupRaw<BF16, kGroup> ga;
+    if (!use_mma) load_group<BF16, kGroup>(kc, vc, kvh, t0 + warp * kGroup, min(t1, fresh), lane, ga);
     uint4 norm_wv = make_uint4(0u, 0u, 0u, 0u);
     float rope_c[8], rope_s[8];
     if constexpr (FUSED) {
@@ -209,21 +254,22 @@ template <bool BF16, bool FUSED> __global__ void __launch_bounds__(kAtThreads) a
         if (now != pos) {
             pos = now;
             tokens = max(1, min(pos + 1, p.max_context));
-            chunk = max(kMinChunk, (tokens + kSplits - 1) / kSplits);
-            nsplit = (tokens + chunk - 1) / chunk;
-            t0 = split * chunk;
-            t1 = min(tokens, t0 + chunk);
+            cut = attn_cut<CL>(tokens, clusters);
+            t0 = split * cut.chunk;
+            t1 = min(tokens, t0 + cut.chunk);
             fresh = tokens - 1;
             use_mma = BF16 && tokens >= kMmaMinTokens;
-            if (!use_mma) {
-                load_group<BF16, kGroup>(kc, vc, kvh, t0 + warp * kGroup, min(t1, fresh), lane, ga);
-                load_group<BF16, kGroup>(kc, vc, kvh, t0 + (warp + kAtWarps) * kGroup, min(t1, fresh), lane, gb);
-            }
+            if (!use_mma) load_group<BF16, kGroup>(kc, vc, kvh, t0 + warp * kGroup, min(t1, fresh), lane, ga);
             if (warp < 5 && lane < 8) rope_table(pos, lane, p.fast_trig != 0, rope_c, rope_s);
         }
     }
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    if (cluster >= cut.active) return; // the whole cluster
     const bool has_work = t0 < tokens;
-    if (nsplit > ns && tid == 0 && p.error_flag) *p.error_flag = 1; // the host's hint was too small: rows would be left out
+    // the gate of the output this CTA will finish (image only), fetched ahead
+    const int my_head = kvh * 4 + rank * kMine / 256, my_dim = rank * kMine % 256 + tid; // of thread tid < kMine
+    float gv = 0.f;
+    if (p.image && tid < kMine) gv = __ldcg(p.gate + size_t(bt) * 8192 + my_head * 512 + 256 + (p.gate_elementwise ? my_dim : 0));
 
     if (has_work) {
         // ---- query (and current key) preparation --------------------------------
@@ -268,196 +314,184 @@ template <bool BF16, bool FUSED> __global__ void __launch_bounds__(kAtThreads) a
     bool mma_done = false;
     if constexpr (BF16) {
         if (has_work && use_mma) {
-            attn_mma_warp(kc, vc, kvh, t0, t1, warp, lane, s_q, s_tiles, &s_bar[warp], &s_abort, s_m[warp], s_l[warp], s_acc[warp]);
+            attn_mma_warp(kc, vc, kvh, t0, t1, warp, lane, s_q, s_tiles, &s_bar[2 * warp], &s_abort, s_m[warp], s_l[warp], s_acc[warp]);
             mma_done = true;
         }
     }
-    if (has_work && !mma_done) {
-        float q[4][8];
+    if (!mma_done) {
+        // Of the sixteen scores of a group (four rows x four heads) lane L keeps number L >> 1: row L >> 3, head (L >> 1) & 3.
+        // The maximum is that head's, the denominator this lane's own share of it.
+        float m = -3.0e38f, l = 0.f, acc[4][8];
 #pragma unroll
         for (int h = 0; h < 4; h++)
 #pragma unroll
-            for (int j = 0; j < 8; j++) q[h][j] = s_q[h][lane * 8 + j] * 0.0625f;
-
-        float m[4], l[4], acc[4][8];
-#pragma unroll
-        for (int h = 0; h < 4; h++) {
-            m[h] = -3.0e38f;
-            l[h] = 0.f;
-#pragma unroll
             for (int j = 0; j < 8; j++) acc[h][j] = 0.f;
-        }
-        // one token group: scores of its (up to) four tokens for the four query heads, one online-softmax update
-        auto process = [&](const GroupRaw<BF16, kGroup> &grp, int tb) {
-            float kk[kGroup][8];
-#pragma unroll
-            for (int g = 0; g < kGroup; g++) Row::unpack(grp.k[g], kk[g]);
+        const int my_row = lane >> 3;
+        const int tend = min(t1, fresh);
+        for (int tb = has_work ? t0 + warp * kGroup : t1; tb < t1; tb += kAtWarps * kGroup) {
             const bool has_fresh = fresh >= tb && fresh < tb + kGroup && fresh < t1; // warp-uniform
-            typename Row::Raw vfresh = Row::zero();
             if (has_fresh) { // the newest row: from shared memory or, now that the wait is over, from the cache
 #pragma unroll
                 for (int g = 0; g < kGroup; g++) {
                     if (tb + g != fresh) continue;
                     if constexpr (FUSED) {
-#pragma unroll
-                        for (int j = 0; j < 8; j++) kk[g][j] = s_knew[lane * 8 + j];
+                        ga.k[g] = Row::pack(s_knew + lane * 8);
+                        ga.v[g] = Row::pack(s_vnew + lane * 8);
                     } else {
                         const size_t row = (size_t(fresh) * 4 + kvh) * 256;
-                        Row::unpack(Row::load_raw(kc, row, lane), kk[g]);
-                        vfresh = Row::load_raw(vc, row, lane);
+                        ga.k[g] = Row::load_raw(kc, row, lane);
+                        ga.v[g] = Row::load_raw(vc, row, lane);
                     }
                 }
             }
-            float s[kGroup][4];
-#pragma unroll
-            for (int g = 0; g < kGroup; g++)
-#pragma unroll
-                for (int h = 0; h < 4; h++) {
-                    float z = 0.f;
-#pragma unroll
-                    for (int j = 0; j < 8; j++) z = fmaf(q[h][j], kk[g][j], z);
-                    s[g][h] = z;
-                }
-#pragma unroll
-            for (int mk = 16; mk; mk >>= 1)
-#pragma unroll
-                for (int g = 0; g < kGroup; g++)
-#pragma unroll
-                    for (int h = 0; h < 4; h++) s[g][h] += __shfl_xor_sync(0xffffffffu, s[g][h], mk);
-            float pr[kGroup][4], corr[4];
+            float s[16];
 #pragma unroll
             for (int h = 0; h < 4; h++) {
-                float mn = m[h];
-#pragma unroll
-                for (int g = 0; g < kGroup; g++)
-                    if (tb + g < t1) mn = fmaxf(mn, s[g][h]);
-                corr[h] = __expf(m[h] - mn);
-                float psum = 0.f;
+                const float4 qa = *reinterpret_cast<const float4 *>(&s_q[h][lane * 8]), qb = *reinterpret_cast<const float4 *>(&s_q[h][lane * 8 + 4]);
 #pragma unroll
                 for (int g = 0; g < kGroup; g++) {
-                    pr[g][h] = tb + g < t1 ? __expf(s[g][h] - mn) : 0.f;
-                    psum += pr[g][h];
+                    float kk[8];
+                    Row::unpack(ga.k[g], kk);
+                    float z = qa.x * kk[0];
+                    z = fmaf(qa.y, kk[1], z); z = fmaf(qa.z, kk[2], z); z = fmaf(qa.w, kk[3], z);
+                    z = fmaf(qb.x, kk[4], z); z = fmaf(qb.y, kk[5], z); z = fmaf(qb.z, kk[6], z); z = fmaf(qb.w, kk[7], z);
+                    s[g * 4 + h] = z;
                 }
-                m[h] = mn;
-                l[h] = fmaf(l[h], corr[h], psum);
+            }
+            const int tn = tb + kAtWarps * kGroup; // the warp's next group
+            load_keys<BF16, kGroup>(kc, kvh, tn, tend, lane, ga);
+            // sums over the lanes, halving the values a lane carries at every step: 16 shuffles where summing each takes 80
 #pragma unroll
-                for (int j = 0; j < 8; j++) acc[h][j] *= corr[h];
+            for (int n = 8, mk = 16; n; n >>= 1, mk >>= 1) {
+                const bool up = (lane & mk) != 0;
+#pragma unroll
+                for (int i = 0; i < n; i++) {
+                    const float keep = up ? s[i + n] : s[i], send = up ? s[i] : s[i + n];
+                    s[i] = keep + __shfl_xor_sync(0xffffffffu, send, mk);
+                }
+            }
+            const float score = (s[0] + __shfl_xor_sync(0xffffffffu, s[0], 1)) * 0.0625f;
+            const bool on = tb + my_row < t1;
+            float mx = on ? score : -3.0e38f;
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+            const float mn = fmaxf(m, mx), corr = __expf(m - mn), pr = on ? __expf(score - mn) : 0.f;
+            m = mn;
+            l = fmaf(l, corr, pr);
+            if (__any_sync(0xffffffffu, corr != 1.f)) {
+#pragma unroll
+                for (int h = 0; h < 4; h++) {
+                    const float c = __shfl_sync(0xffffffffu, corr, 2 * h);
+#pragma unroll
+                    for (int j = 0; j < 8; j++) acc[h][j] *= c;
+                }
             }
 #pragma unroll
             for (int g = 0; g < kGroup; g++) {
                 float vv[8];
-                Row::unpack(grp.v[g], vv);
-                if (has_fresh && tb + g == fresh) {
-                    if constexpr (FUSED) {
+                Row::unpack(ga.v[g], vv);
 #pragma unroll
-                        for (int j = 0; j < 8; j++) vv[j] = s_vnew[lane * 8 + j];
-                    } else {
-                        Row::unpack(vfresh, vv);
-                    }
+                for (int h = 0; h < 4; h++) {
+                    const float w = __shfl_sync(0xffffffffu, pr, (g * 4 + h) * 2);
+#pragma unroll
+                    for (int j = 0; j < 8; j++) acc[h][j] = fmaf(w, vv[j], acc[h][j]);
                 }
-#pragma unroll
-                for (int h = 0; h < 4; h++)
-#pragma unroll
-                    for (int j = 0; j < 8; j++) acc[h][j] = fmaf(pr[g][h], vv[j], acc[h][j]);
             }
-        };
-        const int tend = min(t1, fresh);
-        for (int tb = t0 + warp * kGroup; tb < t1; tb += 2 * kAtWarps * kGroup) {
-            process(ga, tb);
-            load_group<BF16, kGroup>(kc, vc, kvh, tb + 2 * kAtWarps * kGroup, tend, lane, ga);
-            const int tb2 = tb + kAtWarps * kGroup;
-            if (tb2 < t1) {
-                process(gb, tb2);
-                load_group<BF16, kGroup>(kc, vc, kvh, tb2 + 2 * kAtWarps * kGroup, tend, lane, gb);
-            }
+            load_values<BF16, kGroup>(vc, kvh, tn, tend, lane, ga);
         }
-        // ---- fold the 8 warps --------------------------------------------------------
+        l += __shfl_xor_sync(0xffffffffu, l, 8);
+        l += __shfl_xor_sync(0xffffffffu, l, 16);
+        if (lane < 8 && !(lane & 1)) { s_m[warp][lane >> 1] = m; s_l[warp][lane >> 1] = l; }
 #pragma unroll
-        for (int h = 0; h < 4; h++) {
-            if (lane == 0) { s_m[warp][h] = m[h]; s_l[warp][h] = l[h]; }
+        for (int h = 0; h < 4; h++)
 #pragma unroll
-            for (int j = 0; j < 8; j++) s_acc[warp][h][lane * 8 + j] = acc[h][j];
-        }
+            for (int j = 0; j < 8; j += 4)
+                *reinterpret_cast<float4 *>(&s_acc[warp][h][lane * 8 + j]) = make_float4(acc[h][j], acc[h][j + 1], acc[h][j + 2], acc[h][j + 3]);
     }
     __syncthreads();
-    float *part = partials + size_t(kvh * kSplits + split) * kPartFloats;
-    if (has_work) {
-        const int d = tid;
+    // ---- fold the eight warps (thread = dim) and hand every CTA of the cluster the dims it finishes ----------------
 #pragma unroll
-        for (int h = 0; h < 4; h++) {
-            float mg = s_m[0][h];
+    for (int h = 0; h < 4; h++) {
+        float mg = s_m[0][h];
 #pragma unroll
-            for (int w = 1; w < kAtWarps; w++) mg = fmaxf(mg, s_m[w][h]);
-            float lg = 0.f, a = 0.f;
+        for (int w = 1; w < kAtWarps; w++) mg = fmaxf(mg, s_m[w][h]);
+        float lg = 0.f, a = 0.f;
 #pragma unroll
-            for (int w = 0; w < kAtWarps; w++) {
-                const float e = __expf(s_m[w][h] - mg); // warps without tokens carry m=-3e38, l=0, acc=0
-                lg = fmaf(s_l[w][h], e, lg);
-                a = fmaf(s_acc[w][h][d], e, a);
-            }
-            part[8 + h * 256 + d] = a;
-            if (d == 0) { part[h] = mg; part[4 + h] = lg; }
+        for (int w = 0; w < kAtWarps; w++) {
+            const float e = __expf(s_m[w][h] - mg); // warps without rows carry m = -3e38, l = 0, acc = 0
+            lg = fmaf(s_l[w][h], e, lg);
+            a = fmaf(s_acc[w][h][tid], e, a);
+        }
+        const int dim = h * 256 + tid, owner = dim / kMine;
+        uint32_t dst;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_u32(&s_in[rank][dim % kMine])), "r"(owner));
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(a) : "memory");
+        if (dim % kMine == 0) { // the head's maximum and denominator to the owner of these dims
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_u32(&s_min[rank])), "r"(owner));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(mg) : "memory");
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_u32(&s_lin[rank])), "r"(owner));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(lg) : "memory");
         }
     }
-    // ---- last CTA of this kv head folds the splits -----------------------------------
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) {
-        const unsigned ticket = atomicAdd(counters + kvh, 1u);
-        s_last = (ticket == unsigned(ns) - 1u);
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+    float mg = s_min[0];
+#pragma unroll
+    for (int c = 1; c < CL; c++) mg = fmaxf(mg, s_min[c]);
+    float lg = 0.f, a = 0.f;
+#pragma unroll
+    for (int c = 0; c < CL; c++) {
+        const float e = __expf(s_min[c] - mg);
+        lg = fmaf(s_lin[c], e, lg);
+        if (tid < kMine) a = fmaf(s_in[c][tid], e, a);
     }
-    __syncthreads();
-    if (s_last) {
+    if (cut.active > 1) { // several clusters: partial results to scratch, the last one folds them in order
+        float *part = partials + size_t(kvh * kSplits + cluster) * kPartFloats;
+        if (tid < kMine) part[8 + rank * kMine + tid] = a;
+        if (tid == 0) { // CTAs that share a head write the same values
+            part[my_head & 3] = mg;
+            part[4 + (my_head & 3)] = lg;
+        }
         __threadfence();
-        const float *pp = partials + size_t(kvh * kSplits) * kPartFloats;
-        // weights of the splits: warp h takes query head h, a lane takes splits lane and lane+32
-        if (warp < 4) {
-            const int h = warp, sa = lane, sb = lane + 32;
-            const float ma = sa < nsplit ? __ldcg(pp + size_t(sa) * kPartFloats + h) : -3.0e38f;
-            const float mb = sb < nsplit ? __ldcg(pp + size_t(sb) * kPartFloats + h) : -3.0e38f;
-            const float la = sa < nsplit ? __ldcg(pp + size_t(sa) * kPartFloats + 4 + h) : 0.f;
-            const float lb = sb < nsplit ? __ldcg(pp + size_t(sb) * kPartFloats + 4 + h) : 0.f;
-            const float mg = warp_max(fmaxf(ma, mb));
-            const float ea = sa < nsplit ? __expf(ma - mg) : 0.f, eb = sb < nsplit ? __expf(mb - mg) : 0.f;
-            const float lg = warp_sum(fmaf(la, ea, lb * eb));
-            s_e[sa][h] = ea;
-            if (sb < kSplits) s_e[sb][h] = eb;
-            if (lane == 0) s_lg[h] = lg;
+        __syncthreads();
+        const int ticket = kvh * CL + rank, shift = (ticket & 3) * 8; // four 8-bit counts per word
+        if (tid == 0) {
+            const unsigned old = atomicAdd(counters + (ticket >> 2), 1u << shift);
+            s_last = int((old >> shift) & 255u) == cut.active - 1;
         }
         __syncthreads();
-        // a thread owns four output dims of one head; the loads of different splits are independent
-        const int h = tid >> 6, c4 = tid & 63;
-        float4 gv = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (p.image) { // element 0 of the head's gate for all of it, or element by element
-            const float *gsrc = p.gate + size_t(blockIdx.y) * 8192 + (kvh * 4 + h) * 512 + 256;
-            if (p.gate_elementwise) gv = __ldcg(reinterpret_cast<const float4 *>(gsrc) + c4);
-            else gv.x = gv.y = gv.z = gv.w = __ldcg(gsrc);
+        if (!s_last) {
+            if (tid == 0 && s_abort && p.error_flag) *p.error_flag = 1;
+            return;
         }
-        const float4 *src = reinterpret_cast<const float4 *>(pp + 8 + h * 256) + c4;
-        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-        for (int s = 0; s < nsplit; s++) {
-            const float4 v = __ldcg(src + size_t(s) * (kPartFloats / 4));
-            const float e = s_e[s][h];
-            a.x = fmaf(v.x, e, a.x);
-            a.y = fmaf(v.y, e, a.y);
-            a.z = fmaf(v.z, e, a.z);
-            a.w = fmaf(v.w, e, a.w);
+        __threadfence();
+        const float *pp = partials + size_t(kvh * kSplits) * kPartFloats;
+        float ms[kMaxClusters];
+        mg = -3.0e38f;
+#pragma unroll
+        for (int c = 0; c < kMaxClusters; c++) {
+            ms[c] = c < cut.active ? __ldcg(pp + size_t(c) * kPartFloats + (my_head & 3)) : -3.0e38f;
+            mg = fmaxf(mg, ms[c]);
         }
-        const float inv = 1.0f / s_lg[h];
-        a = make_float4(a.x * inv, a.y * inv, a.z * inv, a.w * inv);
-        reinterpret_cast<float4 *>(out_base + size_t(kvh * 4 + h) * 256)[c4] = a;
-        if (p.image) { // a warp holds half a head = one k-block of the o projection's input
-            const float gx[4] = {fast_sigmoid(gv.x), fast_sigmoid(gv.y), fast_sigmoid(gv.z), fast_sigmoid(gv.w)};
-            store_digits(make_float4(a.x * gx[0], a.y * gx[1], a.z * gx[2], a.w * gx[3]), p.slots, int(blockIdx.y),
-                         p.image + size_t((kvh * 4 + h) * 2 + (warp & 1)) * (512 * p.slots + 512), s_lut, lane);
-        }
-        if (tid == 0) counters[kvh] = 0u;
+        lg = 0.f;
+        a = 0.f;
+#pragma unroll
+        for (int c = 0; c < kMaxClusters; c++)
+            if (c < cut.active) {
+                const float e = __expf(ms[c] - mg);
+                lg = fmaf(__ldcg(pp + size_t(c) * kPartFloats + 4 + (my_head & 3)), e, lg);
+                if (tid < kMine) a = fmaf(__ldcg(pp + size_t(c) * kPartFloats + 8 + rank * kMine + tid), e, a);
+            }
+        if (tid == 0) atomicSub(counters + (ticket >> 2), unsigned(cut.active) << shift);
+    }
+    if (tid < kMine) {
+        a *= 1.0f / lg;
+        out_base[size_t(my_head) * 256 + my_dim] = a;
+        if (p.image) group_digits(a * fast_sigmoid(gv), p.slots, bt, p.image, my_head * 8 + (my_dim >> 5), s_lut, lane);
     }
     if (tid == 0 && s_abort && p.error_flag) *p.error_flag = 1;
 }
 
-template <bool BF16, bool FUSED> int launch_attn(const AttnParams &p, cudaStream_t st, bool pdl, int chunk_tokens = 1, int splits = kSplits)
+template <bool BF16, bool FUSED, int CL> static int launch_clusters(const AttnParams &p, cudaStream_t st, bool pdl, int along, int rows, int clusters)
 {
     size_t smem = 0;
     if (BF16) { // the tensor-core loop's tiles: more than 48 KB of dynamic shared memory is a per-device opt-in
@@ -469,13 +503,44 @@ template <bool BF16, bool FUSED> int launch_attn(const AttnParams &p, cudaStream
         if (dev < 0 || dev >= 64) return fail(INSG_E_LIMIT, "attention: device ordinal beyond 63");
         std::lock_guard<std::mutex> lock(mu);
         if (!done[dev]) {
-            e = cudaFuncSetAttribute(attn_splitk_kernel<BF16, FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMmaSmem));
+            e = cudaFuncSetAttribute(attn_splitk_kernel<BF16, FUSED, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMmaSmem));
             if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(attention)");
             done[dev] = true;
         }
-        smem = kMmaSmem;
+        if (p.max_context >= kMmaMinTokens) smem = kMmaSmem; // else no launch of these operands gets to the tensor-core loop
     }
-    return launch(attn_splitk_kernel<BF16, FUSED>, dim3(4 * splits, chunk_tokens), dim3(kAtThreads), smem, st, pdl, p);
+    const int most = rows > 0 ? std::min(rows, p.max_context) : p.max_context;
+    clusters = std::max(1, std::min({clusters, kMaxClusters, (most + kCtaRows * CL - 1) / (kCtaRows * CL)}));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(4 * clusters * CL, along);
+    cfg.blockDim = dim3(kAtThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CL;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, attn_splitk_kernel<BF16, FUSED, CL>, p, clusters);
+    return e == cudaSuccess ? INSG_OK : cuda_fail(e, "attention launch");
+}
+
+// `along`: tokens of a chunk or sequences of a batch (grid rows); rows: an upper bound of the rows attended, when known.  As many
+// clusters as the device runs at once: 33 of eight CTAs at two per SM (fp32 cache), 71 of four CTAs at two per SM (bf16 cache)
+// or 33 at one (with the tensor-core loop's tiles), shared by the four heads of every grid row.  Where that leaves SMs idle (three
+// sequences or more, not a power of two) and the contexts can be long, the fp32 cache goes to clusters of four too.
+constexpr int kLongContext = 2048;
+template <bool BF16, bool FUSED> int launch_attn(const AttnParams &p, cudaStream_t st, bool pdl, int along = 1, int rows = 0)
+{
+    if constexpr (BF16) {
+        return launch_clusters<true, FUSED, 4>(p, st, pdl, along, rows, (p.max_context >= kMmaMinTokens ? kMaxClusters : 17) / along);
+    } else {
+        if (along > 2 && (along & (along - 1)) && p.max_context >= kLongContext) return launch_clusters<false, FUSED, 4>(p, st, pdl, along, rows, 17 / along);
+        return launch_clusters<false, FUSED, 8>(p, st, pdl, along, rows, kMaxClusters / along);
+    }
 }
 
 // A chunk of consecutive tokens, step one: per token m (one CTA each) the per-head RMSNorm + partial RoPE of the 16 query
@@ -624,13 +689,7 @@ int insg_attention_chunk(const insg_attn_op *op, int tokens, float *q_scratch, i
     p.q = q_scratch; p.q_stride = 4096; p.out_stride = 4096; p.scratch_stride = attn_scratch_bytes();
     p.counters = static_cast<unsigned *>(op->scratch);
     p.partials = reinterpret_cast<float *>(static_cast<uint8_t *>(op->scratch) + 64);
-    // the splits a context of rows_hint rows needs (the kernel's own geometry); fewer CTAs to start and to count in
-    int splits = kSplits;
-    if (rows_hint > 0) {
-        const int chunk = std::max(kMinChunk, (rows_hint + kSplits - 1) / kSplits);
-        splits = std::max(1, std::min(kSplits, (rows_hint + chunk - 1) / chunk));
-    }
-    return bf16 ? launch_attn<true, false>(p, stream, false, tokens, splits) : launch_attn<false, false>(p, stream, false, tokens, splits);
+    return bf16 ? launch_attn<true, false>(p, stream, false, tokens, rows_hint) : launch_attn<false, false>(p, stream, false, tokens, rows_hint);
 }
 
 int insg_attention_batch(const insg_attn_op *op, int sequences, size_t cache_stride_bytes, insg_stream_t stream)

@@ -54,6 +54,7 @@ template <> struct KvRow<false> {
     {
         o[0] = r.a.x; o[1] = r.a.y; o[2] = r.a.z; o[3] = r.a.w; o[4] = r.b.x; o[5] = r.b.y; o[6] = r.b.z; o[7] = r.b.w;
     }
+    static __device__ __forceinline__ Raw pack(const float *p) { return Raw{reinterpret_cast<const float4 *>(p)[0], reinterpret_cast<const float4 *>(p)[1]}; }
     static __device__ __forceinline__ float round(float v) { return v; }
     static __device__ __forceinline__ void store(void *base, size_t idx, float v) { static_cast<float *>(base)[idx] = v; }
 };
@@ -71,6 +72,15 @@ template <> struct KvRow<true> {
         o[2] = __uint_as_float(r.y << 16); o[3] = __uint_as_float(r.y & 0xffff0000u);
         o[4] = __uint_as_float(r.z << 16); o[5] = __uint_as_float(r.z & 0xffff0000u);
         o[6] = __uint_as_float(r.w << 16); o[7] = __uint_as_float(r.w & 0xffff0000u);
+    }
+    static __device__ __forceinline__ Raw pack(const float *p) // values already rounded to bf16
+    {
+        uint4 r;
+        r.x = (__float_as_uint(p[0]) >> 16) | (__float_as_uint(p[1]) & 0xffff0000u);
+        r.y = (__float_as_uint(p[2]) >> 16) | (__float_as_uint(p[3]) & 0xffff0000u);
+        r.z = (__float_as_uint(p[4]) >> 16) | (__float_as_uint(p[5]) & 0xffff0000u);
+        r.w = (__float_as_uint(p[6]) >> 16) | (__float_as_uint(p[7]) & 0xffff0000u);
+        return Raw{r};
     }
     static __device__ __forceinline__ float round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
     static __device__ __forceinline__ void store(void *base, size_t idx, float v)
@@ -99,6 +109,19 @@ __device__ __forceinline__ void load_group(const void *kc, const void *vc, int k
             g.v[i] = KvRow<BF16>::zero();
         }
     }
+}
+
+template <bool BF16, int KG>
+__device__ __forceinline__ void load_keys(const void *kc, int kvh, int tb, int tend, int lane, GroupRaw<BF16, KG> &g)
+{
+#pragma unroll
+    for (int i = 0; i < KG; i++) g.k[i] = tb + i < tend ? KvRow<BF16>::load_raw(kc, (size_t(tb + i) * 4 + kvh) * 256, lane) : KvRow<BF16>::zero();
+}
+template <bool BF16, int KG>
+__device__ __forceinline__ void load_values(const void *vc, int kvh, int tb, int tend, int lane, GroupRaw<BF16, KG> &g)
+{
+#pragma unroll
+    for (int i = 0; i < KG; i++) g.v[i] = tb + i < tend ? KvRow<BF16>::load_raw(vc, (size_t(tb + i) * 4 + kvh) * 256, lane) : KvRow<BF16>::zero();
 }
 
 // cos/sin of the rotate-half RoPE for the 8 dims a lane owns (only lanes 0..7 rotate: dims 0..63).
