@@ -8,290 +8,278 @@
 //   out_v  = sum_i S[i][v] * qh[i]
 // State layout fp32 [head][k=128][v=128], v contiguous.
 //
-// The reference reads the 64 KiB head state twice and writes it once from global
-// memory with 32 CTAs.  Columns v are independent, so here each head is cut into
-// 4 slices of 32 columns (128 CTAs); a CTA pulls its 16 KiB slice into registers
-// once (coalesced 128-byte row segments, issued before the dependent-launch wait
-// because the state was last written a whole token ago), does both reductions
-// over k on chip, and writes the slice back once: 2 x 2 MiB of traffic per layer.
-// The step is a latency chain, so it is kept short: all inputs are requested
-// together, every warp normalises q and k for itself, and only the two sums over
-// the eight warps cross a CTA barrier.
+// The reference reads the 64 KiB head state twice and writes it once from global memory with 32 CTAs.  Columns v are
+// independent, so here each head is cut into 4 slices of 32 columns (128 CTAs) and a slice over four warps; a warp pulls its
+// columns into registers once (issued before the dependent-launch wait because the state was last written a whole token
+// ago), does both reductions over k by shuffles, and writes them back once: 2 x 2 MiB of traffic per layer.  The step is a
+// latency chain, so it is kept short: all inputs are requested together, every warp normalises q and k for itself, and no
+// sum leaves the warp.
 #include "common.cuh"
 #include "host_util.h"
 #include "umma_common.cuh"
 
 namespace insg {
 
-constexpr int kDnThreads = 256;
+constexpr int kDnThreads = 128;
 constexpr int kSlices = 4; // 32 columns each
+
+// ---- the arithmetic of one step, shared by the kernels below (which are bit-identical for that reason) -----------------------
+// A warp owns eight columns: lane = (k part kq = lane & 7) x (column pair lane >> 3), 16 rows (32 j + 4 kq + 0..3) of two columns
+// per lane.  Rows go in pairs through the packed fp32 instructions of sm_100 (two lanes of arithmetic per issue), so that a
+// step of a warp is 16 packed multiply-adds three times over; a sum over k is three shuffles, and nothing crosses a warp.
+struct DnCells {
+    unsigned long long c[2][8]; // [column of the pair][row pair 2 j + h]
+};
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c)
+{
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b)
+{
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b)
+{
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+__device__ __forceinline__ void dn_load(DnCells &s, const float *S, int lane) // S: the warp's first column
+{
+    const float *base = S + size_t((lane & 7) * 4) * 128 + (lane >> 3) * 2;
+    float2 x[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) x[i] = __ldcg(reinterpret_cast<const float2 *>(base + size_t((i >> 2) * 32 + (i & 3)) * 128));
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        s.c[0][i] = pack2(x[2 * i].x, x[2 * i + 1].x);
+        s.c[1][i] = pack2(x[2 * i].y, x[2 * i + 1].y);
+    }
+}
+__device__ __forceinline__ void dn_store(const DnCells &s, float *S, int lane)
+{
+    float *base = S + size_t((lane & 7) * 4) * 128 + (lane >> 3) * 2;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const float2 a = unpack2(s.c[0][i]), b = unpack2(s.c[1][i]);
+        float *p = base + size_t((i >> 1) * 32 + (i & 1) * 2) * 128;
+        *reinterpret_cast<float2 *>(p) = make_float2(a.x, b.x);
+        *reinterpret_cast<float2 *>(p + 128) = make_float2(a.y, b.y);
+    }
+}
+// A lane's 16 values of a 128-vector in shared memory, as row pairs.
+__device__ __forceinline__ void dn_vector(unsigned long long (&v)[8], const float *s, int lane)
+{
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const ulonglong2 u = *reinterpret_cast<const ulonglong2 *>(s + 32 * j + (lane & 7) * 4);
+        v[2 * j] = u.x;
+        v[2 * j + 1] = u.y;
+    }
+}
+// This lane's part of sum_k cells * w for its two columns.
+__device__ __forceinline__ float2 dn_products(const DnCells &s, const unsigned long long (&w)[8])
+{
+    float r[2];
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+        unsigned long long a = mul2(s.c[c][0], w[0]), b = mul2(s.c[c][1], w[1]);
+#pragma unroll
+        for (int i = 2; i < 8; i += 2) {
+            a = fma2(s.c[c][i], w[i], a);
+            b = fma2(s.c[c][i + 1], w[i + 1], b);
+        }
+        const float2 t = unpack2(add2(a, b));
+        r[c] = t.x + t.y;
+    }
+    return make_float2(r[0], r[1]);
+}
+// The whole sum of this lane's own column (column lane & 1 of its pair).
+__device__ __forceinline__ float dn_fold(float2 p, int lane)
+{
+    const bool odd = lane & 1;
+    float x = (odd ? p.y : p.x) + __shfl_xor_sync(0xffffffffu, odd ? p.x : p.y, 1);
+    x += __shfl_xor_sync(0xffffffffu, x, 2);
+    x += __shfl_xor_sync(0xffffffffu, x, 4);
+    return x;
+}
+// S = S d + k (v - d S k) beta; v, and the result of dn_products(s, k) folded, are those of the lane's own column.
+__device__ __forceinline__ void dn_update(DnCells &s, const unsigned long long (&k)[8], float mem, float v, float decay, float beta, int lane)
+{
+    const float own = fmaf(-mem, decay, v) * beta, other = __shfl_xor_sync(0xffffffffu, own, 1);
+    const float d0 = (lane & 1) ? other : own, d1 = (lane & 1) ? own : other;
+    const unsigned long long dd = pack2(decay, decay), e0 = pack2(d0, d0), e1 = pack2(d1, d1);
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        s.c[0][i] = fma2(k[i], e0, mul2(s.c[0][i], dd));
+        s.c[1][i] = fma2(k[i], e1, mul2(s.c[1][i], dd));
+    }
+}
 
 // `tokens` consecutive steps of the sequence in one launch: the slice stays in registers from step to step and is
 // written back once; q/k/v of step m are at + m * qkv_stride, g/beta at + m * 32, the output at + m * 4096.
+// Every warp reads the whole q and k of its key head (four values per lane) and normalises them itself: no CTA barrier.
 __global__ void __launch_bounds__(kDnThreads) deltanet_step_kernel(float *__restrict__ state, const float *__restrict__ q16,
                                                                    const float *__restrict__ k16, const float *__restrict__ v32,
                                                                    const float *__restrict__ g32, const float *__restrict__ beta32,
                                                                    float *__restrict__ out32, int tokens, int qkv_stride, long long state_stride,
                                                                    float *__restrict__ state_first, float *__restrict__ state_last)
 {
-    __shared__ __align__(16) float s_qk[8][2][128]; // per warp: its own copy of the normalised q and k (no block barrier)
-    __shared__ __align__(16) float s_part[2][8][32]; // per-warp partial sums over k: [0] memory read-out, [1] output
-
+    __shared__ __align__(16) float s_qk[4][2][128];
     const int head = blockIdx.x / kSlices, slice = blockIdx.x % kSlices, kh = head >> 1;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int vq = tid & 7, kr = tid >> 3; // float4 column group, k row (rows kr, kr+32, kr+64, kr+96)
-    const int v0 = slice * 32 + vq * 4;
+    const int col = slice * 32 + warp * 8, mine = col + (lane >> 3) * 2 + (lane & 1); // the warp's first column, the lane's own
 
     pdl_launch_dependents();
 
     // blockIdx.y: independent sequence of a decode batch (its own state, its own inputs and outputs)
     const int seq = blockIdx.y;
-    q16 += size_t(seq) * qkv_stride; k16 += size_t(seq) * qkv_stride; v32 += size_t(seq) * qkv_stride;
-    g32 += seq * 32; beta32 += seq * 32; out32 += size_t(seq) * 4096;
-    float *S = state + size_t(seq) * state_stride + size_t(head) * 128 * 128;
-    float4 cell[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) cell[j] = __ldcg(reinterpret_cast<const float4 *>(S + size_t(kr + 32 * j) * 128 + v0));
+    q16 += size_t(seq) * qkv_stride + kh * 128; k16 += size_t(seq) * qkv_stride + kh * 128; v32 += size_t(seq) * qkv_stride + head * 128 + mine;
+    g32 += seq * 32 + head; beta32 += seq * 32 + head; out32 += size_t(seq) * 4096 + head * 128 + mine;
+    const size_t at = size_t(head) * 128 * 128 + col;
+    float *S = state + size_t(seq) * state_stride;
+    DnCells cells;
+    dn_load(cells, S + at, lane);
 
     pdl_wait();
 
     // Every dependent input of a step is requested at once; with several steps the next step's inputs are requested
     // before this step's arithmetic (they do not depend on it), so only the first step waits for a load.
-    // Each warp reads the whole q and k of the key head (four values per lane) and normalises them itself: L2 norms
-    // over 128 with eps added to the sum, as the reference.
-    float4 nq4 = __ldcg(reinterpret_cast<const float4 *>(q16 + kh * 128) + lane);
-    float4 nk4 = __ldcg(reinterpret_cast<const float4 *>(k16 + kh * 128) + lane);
-    float4 nv4 = __ldcg(reinterpret_cast<const float4 *>(v32 + head * 128 + slice * 32) + vq); // this thread's columns
-    float ng = __ldcg(g32 + head), nbeta = __ldcg(beta32 + head);
-    for (int step = 0; step < tokens; step++, q16 += qkv_stride, k16 += qkv_stride, v32 += qkv_stride, g32 += 32, beta32 += 32, out32 += 4096) {
-        __syncwarp(); // the previous step's reads of this warp's q/k copy are done
-        const float4 q4 = nq4, k4 = nk4, v4 = nv4;
-        const float g_in = ng, beta = nbeta;
+    float4 nq = __ldcg(reinterpret_cast<const float4 *>(q16) + lane), nk = __ldcg(reinterpret_cast<const float4 *>(k16) + lane);
+    float nv = __ldcg(v32), ng = __ldcg(g32), nb = __ldcg(beta32);
+    for (int step = 0; step < tokens; step++) {
+        const float4 q4 = nq, k4 = nk;
+        const float v = nv, g = ng, beta = nb;
         if (step + 1 < tokens) {
-            nq4 = __ldcg(reinterpret_cast<const float4 *>(q16 + qkv_stride + kh * 128) + lane);
-            nk4 = __ldcg(reinterpret_cast<const float4 *>(k16 + qkv_stride + kh * 128) + lane);
-            nv4 = __ldcg(reinterpret_cast<const float4 *>(v32 + qkv_stride + head * 128 + slice * 32) + vq);
-            ng = __ldcg(g32 + 32 + head);
-            nbeta = __ldcg(beta32 + 32 + head);
+            const size_t o = size_t(step + 1) * qkv_stride;
+            nq = __ldcg(reinterpret_cast<const float4 *>(q16 + o) + lane);
+            nk = __ldcg(reinterpret_cast<const float4 *>(k16 + o) + lane);
+            nv = __ldcg(v32 + o);
+            ng = __ldcg(g32 + size_t(step + 1) * 32);
+            nb = __ldcg(beta32 + size_t(step + 1) * 32);
         }
         const float qn = warp_sum(fmaf(q4.x, q4.x, fmaf(q4.y, q4.y, fmaf(q4.z, q4.z, q4.w * q4.w))));
         const float kn = warp_sum(fmaf(k4.x, k4.x, fmaf(k4.y, k4.y, fmaf(k4.z, k4.z, k4.w * k4.w))));
         const float qs = rsqrtf(qn + 1e-6f) * 0.08838834764831845f, ks = rsqrtf(kn + 1e-6f);
+        __syncwarp(); // the previous step's reads of this warp's copy are done
         reinterpret_cast<float4 *>(s_qk[warp][0])[lane] = make_float4(q4.x * qs, q4.y * qs, q4.z * qs, q4.w * qs);
         reinterpret_cast<float4 *>(s_qk[warp][1])[lane] = make_float4(k4.x * ks, k4.y * ks, k4.z * ks, k4.w * ks);
         __syncwarp();
-        float qq[4], kk[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            qq[j] = s_qk[warp][0][kr + 32 * j];
-            kk[j] = s_qk[warp][1][kr + 32 * j];
-        }
-        const float decay = expf(g_in);
-
-        // mem_v = sum_i (S*d) * k
-        float4 pm = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            pm.x = fmaf(cell[j].x * decay, kk[j], pm.x);
-            pm.y = fmaf(cell[j].y * decay, kk[j], pm.y);
-            pm.z = fmaf(cell[j].z * decay, kk[j], pm.z);
-            pm.w = fmaf(cell[j].w * decay, kk[j], pm.w);
-        }
-        // a warp holds 4 k-rows (lane>>3) x 8 column groups: fold the rows, then every thread folds the 8 warps itself
-#pragma unroll
-        for (int m = 8; m <= 16; m <<= 1) {
-            pm.x += __shfl_xor_sync(0xffffffffu, pm.x, m);
-            pm.y += __shfl_xor_sync(0xffffffffu, pm.y, m);
-            pm.z += __shfl_xor_sync(0xffffffffu, pm.z, m);
-            pm.w += __shfl_xor_sync(0xffffffffu, pm.w, m);
-        }
-        if (lane < 8) *reinterpret_cast<float4 *>(&s_part[0][warp][lane * 4]) = pm;
-        __syncthreads();
-        float4 mem = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int w = 0; w < 8; w++) {
-            const float4 t = *reinterpret_cast<const float4 *>(&s_part[0][w][vq * 4]);
-            mem.x += t.x; mem.y += t.y; mem.z += t.z; mem.w += t.w;
-        }
-        const float4 dl = make_float4((v4.x - mem.x) * beta, (v4.y - mem.y) * beta, (v4.z - mem.z) * beta, (v4.w - mem.w) * beta);
-
-        // S = S*d + k*delta ; out_v = sum_i S * q
-        float4 po = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            cell[j].x = fmaf(cell[j].x, decay, kk[j] * dl.x);
-            cell[j].y = fmaf(cell[j].y, decay, kk[j] * dl.y);
-            cell[j].z = fmaf(cell[j].z, decay, kk[j] * dl.z);
-            cell[j].w = fmaf(cell[j].w, decay, kk[j] * dl.w);
-            po.x = fmaf(cell[j].x, qq[j], po.x);
-            po.y = fmaf(cell[j].y, qq[j], po.y);
-            po.z = fmaf(cell[j].z, qq[j], po.z);
-            po.w = fmaf(cell[j].w, qq[j], po.w);
-            // the state after the last step goes to state_last (default: in place); a speculative verify pass also keeps the
-            // state after its first step (state_first), which is the one to continue from when the second token is rejected
-            if (step == tokens - 1) *reinterpret_cast<float4 *>((state_last ? state_last + size_t(head) * 128 * 128 : S) + size_t(kr + 32 * j) * 128 + v0) = cell[j];
-            else if (step == 0 && state_first) *reinterpret_cast<float4 *>(state_first + size_t(head) * 128 * 128 + size_t(kr + 32 * j) * 128 + v0) = cell[j];
-        }
-#pragma unroll
-        for (int m = 8; m <= 16; m <<= 1) {
-            po.x += __shfl_xor_sync(0xffffffffu, po.x, m);
-            po.y += __shfl_xor_sync(0xffffffffu, po.y, m);
-            po.z += __shfl_xor_sync(0xffffffffu, po.z, m);
-            po.w += __shfl_xor_sync(0xffffffffu, po.w, m);
-        }
-        if (lane < 8) *reinterpret_cast<float4 *>(&s_part[1][warp][lane * 4]) = po;
-        __syncthreads();
-        if (tid < 32) {
-            float o = 0.f;
-#pragma unroll
-            for (int w = 0; w < 8; w++) o += s_part[1][w][tid];
-            out32[head * 128 + slice * 32 + tid] = o;
-        }
+        unsigned long long q[8], k[8];
+        dn_vector(q, s_qk[warp][0], lane);
+        dn_vector(k, s_qk[warp][1], lane);
+        dn_update(cells, k, dn_fold(dn_products(cells, k), lane), v, expf(g), beta, lane);
+        const float o = dn_fold(dn_products(cells, q), lane);
+        if ((lane & 7) < 2) out32[size_t(step) * 4096] = o;
+        // the state after the last step goes to state_last (default: in place); a speculative verify pass also keeps the
+        // state after its first step (state_first), which is the one to continue from when the second token is rejected
+        if (step == tokens - 1) dn_store(cells, (state_last ? state_last : S) + at, lane);
+        else if (step == 0 && state_first) dn_store(cells, state_first + at, lane);
     }
 }
 
+// The recurrence over many consecutive steps (a prompt pass): the state stays in the registers of four warps, which find
+// everything that does not depend on it in shared memory: four more warps normalise q and k and fetch v, beta and exp(g) for
+// the next kDnBlock steps meanwhile.  A step is a latency chain (products, three shuffles, update) of some 200 cycles with no
+// barrier in it; the fold of step t's output runs beside step t + 1's.  (With the k sum cut over eight warps and a CTA barrier
+// in every step, and the inputs prepared between the blocks: 0.61 us a step.)
+constexpr int kDnBlock = 16;
+struct DnInputs {
+    float q[kDnBlock][128], k[kDnBlock][128], v[kDnBlock][32], decay[kDnBlock], beta[kDnBlock];
+};
 
-// The recurrence over many consecutive steps (a prompt pass): the same arithmetic in the same order as
-// deltanet_step_kernel, so the state and the outputs are bit-identical to single steps, with everything that does not
-// depend on the state taken off the serial chain.  Per block of 32 steps the eight warps normalise q and k (four steps
-// each, all loads in flight), fetch v, beta and exp(g) into shared memory; a step then is: products with the slice,
-// fold over k (shuffles + one CTA barrier), update, products with q.  The partial sums are double-buffered by step
-// parity, so one barrier per step is enough, and the output of step t is folded by warp 0 while step t+1 runs.
-constexpr int kDnBlock = 32;
-
-__global__ void __launch_bounds__(kDnThreads) deltanet_steps_kernel(float *__restrict__ state, const float *__restrict__ q16,
-                                                                    const float *__restrict__ k16, const float *__restrict__ v32,
-                                                                    const float *__restrict__ g32, const float *__restrict__ beta32,
-                                                                    float *__restrict__ out32, int tokens, int qkv_stride)
+__global__ void __launch_bounds__(2 * kDnThreads, 1) deltanet_steps_kernel(float *__restrict__ state, const float *__restrict__ q16,
+                                                                           const float *__restrict__ k16, const float *__restrict__ v32,
+                                                                           const float *__restrict__ g32, const float *__restrict__ beta32,
+                                                                           float *__restrict__ out32, int tokens, int qkv_stride)
 {
-    __shared__ __align__(16) float s_q[kDnBlock][128];
-    __shared__ __align__(16) float s_k[kDnBlock][128];
-    __shared__ __align__(16) float s_v[kDnBlock][32];
-    __shared__ float s_decay[kDnBlock], s_beta[kDnBlock];
-    __shared__ __align__(16) float s_mem[2][8][32];
-    __shared__ __align__(16) float s_out[2][8][32];
-
+    __shared__ __align__(16) DnInputs s_in[2];
     const int head = blockIdx.x / kSlices, slice = blockIdx.x % kSlices, kh = head >> 1;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int vq = tid & 7, kr = tid >> 3;
-    const int v0 = slice * 32 + vq * 4;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
 
     pdl_launch_dependents();
-    float *S = state + size_t(head) * 128 * 128;
-    float4 cell[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) cell[j] = __ldcg(reinterpret_cast<const float4 *>(S + size_t(kr + 32 * j) * 128 + v0));
+    const int col = slice * 32 + (warp & 3) * 8, in = (warp & 3) * 8 + (lane >> 3) * 2 + (lane & 1);
+    float *S = state + size_t(head) * 128 * 128 + col;
+    DnCells cells;
+    if (warp < 4) dn_load(cells, S, lane);
     pdl_wait();
 
-    for (int base = 0; base < tokens; base += kDnBlock) {
-        const int nb = min(kDnBlock, tokens - base);
-        // ---- inputs of the block's steps: warp w takes steps w, w+8, w+16, w+24 (every read of the previous block's rows
-        // lies before the barrier of its last step, which every warp has passed) ----
-        {
-            float4 q4[4], k4[4], x4[4];
-            float gs[4];
+    constexpr int kEach = kDnBlock / 4; // steps per preparing warp
+    auto prepare = [&](int base, DnInputs &d) {
+        float4 q4[kEach], k4[kEach], x4[kEach];
+        float gs[kEach];
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int s = warp + 8 * i;
-                q4[i] = k4[i] = x4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-                gs[i] = 0.f;
-                if (s < nb) {
-                    const size_t off = size_t(base + s) * qkv_stride;
-                    q4[i] = __ldcg(reinterpret_cast<const float4 *>(q16 + off + kh * 128) + lane);
-                    k4[i] = __ldcg(reinterpret_cast<const float4 *>(k16 + off + kh * 128) + lane);
-                    if (lane < 8) x4[i] = __ldcg(reinterpret_cast<const float4 *>(v32 + off + head * 128 + slice * 32) + lane);
-                    else if (lane == 8) gs[i] = __ldcg(g32 + size_t(base + s) * 32 + head);
-                    else if (lane == 9) gs[i] = __ldcg(beta32 + size_t(base + s) * 32 + head);
-                }
+        for (int i = 0; i < kEach; i++) {
+            const int s = (warp & 3) + 4 * i;
+            q4[i] = k4[i] = x4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            gs[i] = 0.f;
+            if (base + s < tokens) {
+                const size_t off = size_t(base + s) * qkv_stride;
+                q4[i] = __ldcg(reinterpret_cast<const float4 *>(q16 + off + kh * 128) + lane);
+                k4[i] = __ldcg(reinterpret_cast<const float4 *>(k16 + off + kh * 128) + lane);
+                if (lane < 8) x4[i] = __ldcg(reinterpret_cast<const float4 *>(v32 + off + head * 128 + slice * 32) + lane);
+                else if (lane == 8) gs[i] = __ldcg(g32 + size_t(base + s) * 32 + head);
+                else if (lane == 9) gs[i] = __ldcg(beta32 + size_t(base + s) * 32 + head);
             }
+        }
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int s = warp + 8 * i;
-                if (s < nb) { // warp-uniform
-                    const float qn = warp_sum(fmaf(q4[i].x, q4[i].x, fmaf(q4[i].y, q4[i].y, fmaf(q4[i].z, q4[i].z, q4[i].w * q4[i].w))));
-                    const float kn = warp_sum(fmaf(k4[i].x, k4[i].x, fmaf(k4[i].y, k4[i].y, fmaf(k4[i].z, k4[i].z, k4[i].w * k4[i].w))));
-                    const float qs = rsqrtf(qn + 1e-6f) * 0.08838834764831845f, ks = rsqrtf(kn + 1e-6f);
-                    reinterpret_cast<float4 *>(s_q[s])[lane] = make_float4(q4[i].x * qs, q4[i].y * qs, q4[i].z * qs, q4[i].w * qs);
-                    reinterpret_cast<float4 *>(s_k[s])[lane] = make_float4(k4[i].x * ks, k4[i].y * ks, k4[i].z * ks, k4[i].w * ks);
-                    if (lane < 8) reinterpret_cast<float4 *>(s_v[s])[lane] = x4[i];
-                    else if (lane == 8) s_decay[s] = expf(gs[i]);
-                    else if (lane == 9) s_beta[s] = gs[i];
-                }
+        for (int i = 0; i < kEach; i++) {
+            const int s = (warp & 3) + 4 * i;
+            const float qn = warp_sum(fmaf(q4[i].x, q4[i].x, fmaf(q4[i].y, q4[i].y, fmaf(q4[i].z, q4[i].z, q4[i].w * q4[i].w))));
+            const float kn = warp_sum(fmaf(k4[i].x, k4[i].x, fmaf(k4[i].y, k4[i].y, fmaf(k4[i].z, k4[i].z, k4[i].w * k4[i].w))));
+            const float qs = rsqrtf(qn + 1e-6f) * 0.08838834764831845f, ks = rsqrtf(kn + 1e-6f);
+            reinterpret_cast<float4 *>(d.q[s])[lane] = make_float4(q4[i].x * qs, q4[i].y * qs, q4[i].z * qs, q4[i].w * qs);
+            reinterpret_cast<float4 *>(d.k[s])[lane] = make_float4(k4[i].x * ks, k4[i].y * ks, k4[i].z * ks, k4[i].w * ks);
+            if (lane < 8) reinterpret_cast<float4 *>(d.v[s])[lane] = x4[i];
+            else if (lane == 8) d.decay[s] = expf(gs[i]);
+            else if (lane == 9) d.beta[s] = gs[i];
+        }
+    };
+    if (warp >= 4) prepare(0, s_in[0]);
+    __syncthreads();
+    float *out = out32 + head * 128 + slice * 32 + in;
+    float2 po = make_float2(0.f, 0.f);
+    for (int base = 0, b = 0; base < tokens; base += kDnBlock, b ^= 1) {
+        if (warp >= 4) {
+            if (base + kDnBlock < tokens) prepare(base + kDnBlock, s_in[b ^ 1]);
+        } else {
+            const DnInputs &d = s_in[b];
+            const int n = min(kDnBlock, tokens - base);
+            unsigned long long q[8], k[8];
+            dn_vector(k, d.k[0], lane);
+            for (int s = 0; s < n; s++) {
+                dn_vector(q, d.q[s], lane);
+                const float2 pm = dn_products(cells, k);
+                const float mem = dn_fold(pm, lane), o = dn_fold(po, lane); // po: the previous step's output
+                if (base + s > 0 && (lane & 7) < 2) out[size_t(base + s - 1) * 4096] = o;
+                dn_update(cells, k, mem, d.v[s][in], d.decay[s], d.beta[s], lane);
+                dn_vector(k, d.k[min(s + 1, kDnBlock - 1)], lane);
+                po = dn_products(cells, q);
             }
         }
         __syncthreads();
-
-        for (int s = 0; s < nb; s++) {
-            const int t = base + s, par = t & 1;
-            float qq[4], kk[4];
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                qq[j] = s_q[s][kr + 32 * j];
-                kk[j] = s_k[s][kr + 32 * j];
-            }
-            const float decay = s_decay[s], beta = s_beta[s];
-            const float4 v4 = *reinterpret_cast<const float4 *>(&s_v[s][vq * 4]);
-
-            float4 pm = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                pm.x = fmaf(cell[j].x * decay, kk[j], pm.x);
-                pm.y = fmaf(cell[j].y * decay, kk[j], pm.y);
-                pm.z = fmaf(cell[j].z * decay, kk[j], pm.z);
-                pm.w = fmaf(cell[j].w * decay, kk[j], pm.w);
-            }
-#pragma unroll
-            for (int m = 8; m <= 16; m <<= 1) {
-                pm.x += __shfl_xor_sync(0xffffffffu, pm.x, m);
-                pm.y += __shfl_xor_sync(0xffffffffu, pm.y, m);
-                pm.z += __shfl_xor_sync(0xffffffffu, pm.z, m);
-                pm.w += __shfl_xor_sync(0xffffffffu, pm.w, m);
-            }
-            if (lane < 8) *reinterpret_cast<float4 *>(&s_mem[par][warp][lane * 4]) = pm;
-            __syncthreads();
-            if (t > 0 && tid < 32) { // the previous step's output, off the chain
-                float o = 0.f;
-#pragma unroll
-                for (int w = 0; w < 8; w++) o += s_out[par ^ 1][w][tid];
-                out32[size_t(t - 1) * 4096 + head * 128 + slice * 32 + tid] = o;
-            }
-            float4 mem = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int w = 0; w < 8; w++) {
-                const float4 u = *reinterpret_cast<const float4 *>(&s_mem[par][w][vq * 4]);
-                mem.x += u.x; mem.y += u.y; mem.z += u.z; mem.w += u.w;
-            }
-            const float4 dl = make_float4((v4.x - mem.x) * beta, (v4.y - mem.y) * beta, (v4.z - mem.z) * beta, (v4.w - mem.w) * beta);
-            float4 po = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                cell[j].x = fmaf(cell[j].x, decay, kk[j] * dl.x);
-                cell[j].y = fmaf(cell[j].y, decay, kk[j] * dl.y);
-                cell[j].z = fmaf(cell[j].z, decay, kk[j] * dl.z);
-                cell[j].w = fmaf(cell[j].w, decay, kk[j] * dl.w);
-                po.x = fmaf(cell[j].x, qq[j], po.x);
-                po.y = fmaf(cell[j].y, qq[j], po.y);
-                po.z = fmaf(cell[j].z, qq[j], po.z);
-                po.w = fmaf(cell[j].w, qq[j], po.w);
-            }
-#pragma unroll
-            for (int m = 8; m <= 16; m <<= 1) {
-                po.x += __shfl_xor_sync(0xffffffffu, po.x, m);
-                po.y += __shfl_xor_sync(0xffffffffu, po.y, m);
-                po.z += __shfl_xor_sync(0xffffffffu, po.z, m);
-                po.w += __shfl_xor_sync(0xffffffffu, po.w, m);
-            }
-            if (lane < 8) *reinterpret_cast<float4 *>(&s_out[par][warp][lane * 4]) = po;
-        }
     }
-#pragma unroll
-    for (int j = 0; j < 4; j++) *reinterpret_cast<float4 *>(S + size_t(kr + 32 * j) * 128 + v0) = cell[j];
-    __syncthreads();
-    if (tid < 32) {
-        float o = 0.f;
-#pragma unroll
-        for (int w = 0; w < 8; w++) o += s_out[(tokens - 1) & 1][w][tid];
-        out32[size_t(tokens - 1) * 4096 + head * 128 + slice * 32 + tid] = o;
+    if (warp < 4) {
+        const float o = dn_fold(po, lane);
+        if ((lane & 7) < 2) out[size_t(tokens - 1) * 4096] = o;
+        dn_store(cells, S, lane);
     }
 }
 
@@ -301,13 +289,14 @@ __global__ void __launch_bounds__(kDnThreads) deltanet_steps_kernel(float *__res
 // slices exchanging their sums through a cluster took 16 us at eight sequences, this form 6; the out projection's own
 // conversion, done again by each of its clusters, 6 us more than taking the image).  A warp holds 16 rows of the state, a lane four columns: the
 // sums over k need no shuffles, only one pass over the eight warps' partials.
+constexpr int kHeadThreads = 256;
 struct DnGate {
     const float *z;          // [sequences][4096]
     const uint16_t *norm_w;  // bf16 [128]
     uint8_t *image;
     int slots;
 };
-__global__ void __launch_bounds__(kDnThreads, 2) deltanet_heads_kernel(float *__restrict__ state, long long state_stride, const float *__restrict__ q16,
+__global__ void __launch_bounds__(kHeadThreads, 2) deltanet_heads_kernel(float *__restrict__ state, long long state_stride, const float *__restrict__ q16,
                                                                        const float *__restrict__ k16, const float *__restrict__ v32,
                                                                        const float *__restrict__ g32, const float *__restrict__ beta32,
                                                                        float *__restrict__ out32, int qkv_stride, const DnGate gate)
@@ -410,7 +399,7 @@ extern "C" int insg_deltanet_decode_tokens(float *state, const float *q16, const
     if (tokens == 1)
         return launch(deltanet_step_kernel, dim3(32 * kSlices), dim3(kDnThreads), 0, stream, pdl != 0, state, q16, k16, v32, g32, beta32,
                       out32, 1, qkv_stride, 0ll, nullptr, nullptr);
-    return launch(deltanet_steps_kernel, dim3(32 * kSlices), dim3(kDnThreads), 0, stream, pdl != 0, state, q16, k16, v32, g32, beta32,
+    return launch(deltanet_steps_kernel, dim3(32 * kSlices), dim3(2 * kDnThreads), 0, stream, pdl != 0, state, q16, k16, v32, g32, beta32,
                   out32, tokens, qkv_stride);
 }
 
@@ -440,6 +429,6 @@ extern "C" int insg_deltanet_decode_gated(float *state, long long state_stride, 
 {
     if (!state || !q16 || !k16 || !v32 || !g32 || !beta32 || !out32 || !z || !norm_w || !image) return fail(INSG_E_ARG, "deltanet: null pointer");
     if (sequences < 1 || sequences > 8 || qkv_stride < 0 || state_stride < 32 * 128 * 128) return fail(INSG_E_SHAPE, "deltanet: 1..8 sequences");
-    return launch(deltanet_heads_kernel, dim3(32, sequences), dim3(kDnThreads), 0, stream, pdl != 0, state, state_stride, q16, k16, v32, g32, beta32,
+    return launch(deltanet_heads_kernel, dim3(32, sequences), dim3(kHeadThreads), 0, stream, pdl != 0, state, state_stride, q16, k16, v32, g32, beta32,
                   out32, qkv_stride, DnGate{z, norm_w, static_cast<uint8_t *>(image), image_slots(sequences)});
 }
