@@ -1,31 +1,34 @@
-// MXFP4 weights x several tokens on the 5th-generation tensor cores (tcgen05, sm_100a): the M >= 5 form of the GEMV.
+// MXFP4 weights x many tokens on the 5th-generation tensor cores (tcgen05, sm_100a): prompt passes of more than eight tokens.
 //
 // y[m][r] = sum_k e2m1(code(r,k)) * 2^(s(r,k/32)-127) * x[m][k]                 (reference: src/mxfp4.cu:41-66, M times)
 //
-// With several tokens the contraction is a real (if skinny) GEMM, and it runs where a GEMM belongs:
-// tcgen05.mma.kind::mxf4.block_scale, weights as the A operand in their native packed E2M1 + UE8M0 form (the tile
-// layout of insg_mxfp4_repack_umma, nothing dequantised), accumulators in tensor memory.  The activations are the
-// B operand.  kind::mxf4 wants E2M1 there too, so each fp32 activation is written as a 25-bit signed fixed-point
-// number (relative to its token's largest element) in balanced base 9: eight digits -4..4, every one exact in E2M1.
-// Column j of a token holds digit j of every element; the eight columns are combined as sum_j 9^j D_j in fp32 by the
-// epilogue, which gives the product to ~1e-7.  A token takes 8 columns of N: SIXTEEN tokens share one M128 x N128 x K64
-// instruction (eight tokens an N64 one), which costs the tensor pipe what the one-token instruction costs.
+// tcgen05.mma.kind::mxf4.block_scale, weights as the A operand in their native packed E2M1 + UE8M0 form (the tile layout of
+// insg_mxfp4_repack_umma, nothing dequantised), accumulators in tensor memory.  The activations are the B operand.
+// kind::mxf4 wants E2M1 there too, so each fp32 activation is written as a 25-bit signed fixed-point number (relative to its
+// token's largest element) in balanced base 9: eight digits -4..4, every one exact in E2M1.  Column j of a token holds digit
+// j of every element; the eight columns are combined as sum_j 9^j D_j in fp32 by the epilogue, which gives the product to
+// ~1e-7.  A token takes 8 columns of N.
+//
+// What bounds it: filling shared memory.  A stage multiplies two 128-row weight records (17.4 KB) with the digits of a group
+// of tokens; an SM takes in some 52 bytes a clock from L2, and sixteen tokens' digits (8.2 KB, N = 128) left the tensor pipe
+// half idle.  Twenty-four tokens (12.3 KB, N = 192) are half as much work again per stage for 16 % more bytes, and tensor
+// memory holds their two accumulators (384 of 512 columns) beside the scale factors; 24576 x 4096 at 512 tokens: 182 -> 153 us.
 //
 // Kernels:
 //   umma_digitize_kernel  one CTA per token: the fused activation prologue (RMSNorm, gates, ...), then the digit
 //                         image of the token in global memory, laid out as the shared-memory image the MMA reads
 //                         ([k-block][group of tokens][512 bytes x tokens per group], canonical K-major, no swizzle);
-//   umma_gemm_kernel      one CTA per SM.  The work is the sequence of all (tile of 128 rows, token group, matrix,
-//                         k-block) stages; every CTA takes an equal contiguous share of it (stream-K), so SMs are
-//                         busy whatever the number of tiles.  A ring of stages, each one weight record + the group's
-//                         digit block of the same k-block, both fetched by cp.async.bulk with mbarrier completion
-//                         (local, no multicast); one thread issues the scale copies and the MMAs; accumulators double
-//                         buffered so that four epilogue warps (tensor memory lane = output row) work on one run
-//                         while the next one multiplies.  A (tile, group) that lies inside one CTA's share goes
-//                         straight through the fused epilogue; one that is cut by a share boundary leaves per-CTA
-//                         partial sums in scratch, and the CTA that arrives last (a ticket per cut unit) adds them
-//                         in share order -- the result does not depend on which CTA that is -- and runs the
-//                         epilogue.  Every wait is bounded: on expiry an error flag is raised and all roles drain.
+//   umma_gemm_kernel      one CTA per SM.  The work is the sequence of all (pair of records, token group, k-block) stages;
+//                         every CTA takes an equal contiguous share of it (stream-K), so SMs are busy whatever the number
+//                         of tiles.  The pair is two row tiles, or the gate and the up tile of the same rows for SwiGLU
+//                         (whose epilogue then has both at hand).  A ring of stages, fetched by cp.async.bulk with mbarrier
+//                         completion (local, no multicast); one warp issues the scale copies and the MMAs; four epilogue
+//                         warps (tensor memory lane = output row) take a run's sums out before the next one multiplies,
+//                         while the ring refills.  A unit (pair, group) that lies inside one CTA's share goes straight
+//                         through the fused epilogue; one that is cut by a share boundary leaves per-CTA partial sums in
+//                         scratch, and the CTA that arrives last (a ticket per cut unit) adds them in share order -- the
+//                         result does not depend on which CTA that is -- and runs the epilogue.  Every wait is bounded:
+//                         on expiry an error flag is raised and all roles drain.
 //   conv_tokens_kernel    the causal convolution + SiLU over consecutive tokens of one sequence (the history runs
 //                         through the tokens in order, so it cannot live in a per-unit epilogue).
 #include "gemv_prologue.cuh"
@@ -41,25 +44,10 @@ constexpr int kGThreads = kProThreads;     // digitize kernel: the activation pr
 constexpr int kGemmThreads = 192;          // GEMM kernel: four epilogue warps, the MMA issuer, the producer
 constexpr int kDigits = 8;                 // balanced base-9 digits per activation = N columns per token
 constexpr int kGSfaBufs = 8;               // scale-factor column sets cycled by stage (a power of two)
-constexpr int kGTmemCols = 512;            // accumulators [0,256), weight scale factors [256,320), digit scale factors [320,324)
+constexpr int kGTmemCols = 512;            // two accumulators of up to 192 columns, weight scale factors [384,448), digit scale factors [448,456)
 constexpr int kGMaxStages = 16;
 constexpr int kGMaxGrid = 256;             // partial-sum slots and tickets are sized for this many CTAs
-constexpr int kSlotFloats = 128 * 16;      // one partial: 128 rows x up to 16 tokens
-
-// Development aid, compiled in only with -DINSG_PHASE_TIMES: clock stamps of the roles of every CTA of the last launch.
-#ifdef INSG_PHASE_TIMES
-__device__ unsigned long long g_gemm_stamps[kGMaxGrid * 16 + 4];
-#define GEMM_STAMP(slot)                                                                                   \
-    do {                                                                                                   \
-        unsigned long long t_;                                                                             \
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_));                                            \
-        g_gemm_stamps[blockIdx.x * 16 + (slot)] = t_;                                                      \
-    } while (0)
-#else
-#define GEMM_STAMP(slot) \
-    do {                 \
-    } while (0)
-#endif
+constexpr int kSlotFloats = 128 * 24;      // one partial: 128 rows x up to 24 tokens
 
 struct GSeg {
     const uint8_t *packed, *packed2;
@@ -69,15 +57,15 @@ struct GSeg {
     const float *A_log;
     const uint16_t *dt_bias;
     long long conv_stride; // 0: one sequence (the epilogue stores the raw product, conv_tokens_kernel follows); else token m's history at conv_state + m * stride
-    int tile_begin, ntiles, nmat, epilogue, rows;
+    int tile_begin, epilogue, rows;
 };
 
 struct GParams {
     const uint8_t *bimg;    // [nkb][ngroups][512 * tpg]
     const float *inv_alpha; // [ngroups * tpg]
-    float *partials;        // [grid][2 cut units][2 matrices][2 tiles][128 rows][tpg]
+    float *partials;        // [grid][2 cut units][2 records of the pair][128 rows][tpg]
     int *tickets;           // [grid], zero between launches
-    int nkb, nseg, total_tiles, stages, ngroups, tokens, tpg, nmat;
+    int nkb, nseg, total_tiles, stages, ngroups, tokens;
     int total_stages, share, share_rem; // CTA c owns stages [share * c + share_rem * c / G, ...): all products stay in 32 bits
     GSeg seg[4];
     int *error_flag;
@@ -100,13 +88,6 @@ __global__ void __launch_bounds__(kGThreads, 2) umma_digitize_kernel(const __gri
     __shared__ uint8_t lut[84];
     if (threadIdx.x < 81) lut[threadIdx.x] = digit_pair_code(threadIdx.x); // read after the prologue's barriers
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); // the GEMM may set itself up and fetch weights meanwhile
-#ifdef INSG_PHASE_TIMES
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        unsigned long long t_;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_));
-        g_gemm_stamps[kGMaxGrid * 16] = t_;
-    }
-#endif
     const int m = blockIdx.x / p.parts, part = blockIdx.x - m * p.parts, grp = m / p.tpg, ms = m - grp * p.tpg;
     const int tid = threadIdx.x;
     const bool live = m < p.tokens;
@@ -146,13 +127,6 @@ __global__ void __launch_bounds__(kGThreads, 2) umma_digitize_kernel(const __gri
             pack_digits(v[j], alpha, lut, p.bimg + (size_t(kb) * p.ngroups + grp) * block + (kk >> 6) * kstep + ms * 256 + (half >> 4) * 128 + (half & 15));
         }
     }
-#ifdef INSG_PHASE_TIMES
-    if (threadIdx.x == 0) {
-        unsigned long long t_;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_));
-        atomicMax(&g_gemm_stamps[kGMaxGrid * 16 + 1], t_);
-    }
-#endif
 }
 
 // Causal convolution (kernel 4) + SiLU over `tokens` consecutive tokens of one sequence, in place: io[m][c] holds the raw
@@ -210,9 +184,8 @@ __device__ __forceinline__ int gseg_of(const GParams &p, int tile)
 }
 
 // ---- the stream-K schedule ----------------------------------------------------------------------------------------------
-// Stage g of the launch: unit = g / L (L = nmat * nkb), unit = tile * ngroups + group; inside the unit matrix 0's k-blocks,
-// then matrix 1's.  CTA c owns stages [share_begin(c), share_begin(c + 1)).  A run = the part of one (unit, matrix) inside
-// one share; it has its own accumulator.
+// Stage g of the launch: unit = g / nkb = pair * ngroups + group, k-block = g % nkb.  CTA c owns stages [share_begin(c),
+// share_begin(c + 1)).  A run = the part of one unit inside one share.
 __device__ __forceinline__ int share_begin(const GParams &p, int c, int G) { return p.share * c + (p.share_rem * c) / G; }
 __device__ __forceinline__ int cta_of_stage(const GParams &p, int g, int G)
 {
@@ -223,20 +196,15 @@ __device__ __forceinline__ int cta_of_stage(const GParams &p, int g, int G)
 }
 
 struct GRun {
-    int g0;         // first stage
-    int len;        // stages
-    int unit, mat, kb0;
+    int len;       // stages
+    int unit, kb0;
 };
 __device__ __forceinline__ GRun run_at(const GParams &p, int g, int end)
 {
-    const int q = g / p.nkb;                 // (unit, matrix) index
-    const int qend = (q + 1) * p.nkb;
     GRun r;
-    r.g0 = g;
-    r.len = min(qend, end) - g;
-    r.unit = p.nmat == 2 ? q >> 1 : q;
-    r.mat = p.nmat == 2 ? q & 1 : 0;
-    r.kb0 = g - q * p.nkb;
+    r.unit = g / p.nkb;
+    r.len = min((r.unit + 1) * p.nkb, end) - g;
+    r.kb0 = g - r.unit * p.nkb;
     return r;
 }
 
@@ -342,55 +310,56 @@ __device__ __forceinline__ void load_sums(uint32_t taddr, float (&y)[TPG])
     }
 }
 
-// Where the weight records of one (tile pair, matrix) start, and whether the pair has its second tile.
+// Where the weight records of a pair start (two row tiles, the second one missing after an odd number; or gate and up).
 struct PairSrc {
     const uint8_t *a0, *a1;
     bool has1;
 };
-__device__ __forceinline__ PairSrc pair_src(const GParams &p, int pair, int mat, int kb)
+template <bool SWIGLU> __device__ __forceinline__ PairSrc pair_src(const GParams &p, int pair, int kb)
 {
     PairSrc q;
-    const int t0 = 2 * pair, t1 = t0 + 1;
+    const int t0 = SWIGLU ? pair : 2 * pair, t1 = t0 + 1;
     const GSeg &s0 = p.seg[gseg_of(p, t0)];
-    q.a0 = (mat ? s0.packed2 : s0.packed) + (size_t(t0 - s0.tile_begin) * p.nkb + kb) * kURec;
+    const size_t at = (size_t(t0 - s0.tile_begin) * p.nkb + kb) * kURec;
+    q.a0 = s0.packed + at;
+    if (SWIGLU) {
+        q.has1 = true;
+        q.a1 = s0.packed2 + at;
+        return q;
+    }
     q.has1 = t1 < p.total_tiles;
     q.a1 = q.a0;
     if (q.has1) {
         const GSeg &s1 = p.seg[gseg_of(p, t1)];
-        q.a1 = (mat ? s1.packed2 : s1.packed) + (size_t(t1 - s1.tile_begin) * p.nkb + kb) * kURec;
+        q.a1 = s1.packed + (size_t(t1 - s1.tile_begin) * p.nkb + kb) * kURec;
     }
     return q;
 }
 
-template <int TPG, int NMAT>
+template <int TPG, bool SWIGLU>
 __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid_constant__ GParams p)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int kBBlock = 512 * TPG;              // digits of the group's tokens for one k-block: 8 * TPG columns x 128 k x 4 bit
-    constexpr int kGStage = 2 * kURec + kBBlock;    // one ring stage: the weight records of a pair of row tiles + the digit block both multiply
+    constexpr int kGStage = 2 * kURec + kBBlock;    // one ring stage: the pair's weight records + the digit block both multiply
     constexpr int N = kDigits * TPG;
-    // Tensor memory: accumulator sets of 2 tiles x N columns from column 0 (two sets of 2 x 64, or one of 2 x 128), the
-    // weights' scale factors at [256, 320) (8 k-blocks x 2 tiles x 4 columns), the digits' (all 1) at [320, 324).
-    constexpr int NB = TPG == 8 ? 2 : 1;
-    constexpr uint32_t kSfaCol = 256, kSfbCol = 320;
+    constexpr uint32_t kSfaCol = 384, kSfbCol = 448;
+    static_assert(2 * N <= int(kSfaCol) && 8 * kGSfaBufs == int(kSfbCol - kSfaCol), "tensor memory");
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int nkb = p.nkb, S = p.stages;
     uint8_t *ring = smem;                          // S stages of kGStage bytes
     uint8_t *sfb = ring + size_t(S) * kGStage;     // 512 bytes
-    __shared__ __align__(8) uint64_t full[kGMaxStages], empty[kGMaxStages], dfull[2], dempty[2];
+    __shared__ __align__(8) uint64_t full[kGMaxStages], empty[kGMaxStages], dfull, dempty;
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort, s_last;
 
-    if (tid == 0) GEMM_STAMP(0);
     const int G = int(gridDim.x), c = int(blockIdx.x);
     const int begin = share_begin(p, c, G), end = share_begin(p, c + 1, G);
-    const int total_kb = int(end - begin);
-    constexpr int kNmat = NMAT;
-    const int L = kNmat * nkb;
 
     if (tid == 0) {
         for (int i = 0; i < S; i++) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-        for (int i = 0; i < 2; i++) { mbar_init(&dfull[i], 1); mbar_init(&dempty[i], 4); }
+        mbar_init(&dfull, 1);
+        mbar_init(&dempty, 4);
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -408,58 +377,53 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
     pdl_launch_dependents(); // this CTA holds its tensor memory: whatever follows may take an SM as it becomes free
     const uint32_t tmem = s_tmem;
     volatile int *abort_flag = &s_abort;
-    if (tid == 0) GEMM_STAMP(1);
 
     if (warp == 5) {
         // ---- producer: the pair's two weight records + the token group's digit block per stage -----------------------
         // The weights do not depend on the launch before this one (the digit image does): the first ring of weight
         // records is requested before the programmatic-dependency wait, the digit blocks of those stages after it.
         // The first ring is requested by one lane per stage (a bulk copy takes the issuing thread a few hundred cycles).
-        const int first = min(S, total_kb);
+        const int first = min(S, end - begin);
         const uint8_t *b0 = nullptr;
         uint8_t *dst0 = nullptr;
         if (lane < first) {
             const GRun r = run_at(p, begin + lane, end);
             const int pair = r.unit / p.ngroups, grp = r.unit - pair * p.ngroups;
-            const PairSrc q = pair_src(p, pair, r.mat, r.kb0);
+            const PairSrc q = pair_src<SWIGLU>(p, pair, r.kb0);
             b0 = p.bimg + (size_t(r.kb0) * p.ngroups + grp) * kBBlock;
             dst0 = ring + size_t(lane) * kGStage;
             mbar_expect_tx(&full[lane], (q.has1 ? 2 : 1) * kURec + kBBlock);
             bulk_load(dst0, q.a0, kURec, &full[lane]);
             if (q.has1) bulk_load(dst0 + kURec, q.a1, kURec, &full[lane]);
         }
-        if (tid == 160) GEMM_STAMP(2);
         asm volatile("griddepcontrol.wait;" ::: "memory");
-        if (tid == 160) GEMM_STAMP(3);
         if (lane < first) bulk_load(dst0 + 2 * kURec, b0, kBBlock, &full[lane]);
-        {   // from here on the whole warp walks the loop and one elected lane issues: warp-uniform operands issue twice as fast
-            const bool one = elect_one();
-            int g = begin + first, st = first == S ? 0 : first;
-            uint32_t phase = 0; // of the empty barriers
-            bool ok = true, room = g < end && mbar_test(&empty[st], phase);
-            while (g < end && ok) {
-                const GRun r = run_at(p, g, end);
-                const int pair = r.unit / p.ngroups, grp = r.unit - pair * p.ngroups;
-                const PairSrc q = pair_src(p, pair, r.mat, r.kb0);
-                const uint8_t *a0 = q.a0, *a1 = q.a1, *b = p.bimg + (size_t(r.kb0) * p.ngroups + grp) * kBBlock;
-                const size_t bstep = size_t(p.ngroups) * kBBlock;
-                const uint32_t bytes = (q.has1 ? 2 : 1) * kURec + kBBlock;
-                for (int k = 0; k < r.len; k++, a0 += kURec, a1 += kURec, b += bstep) {
-                    if (!room && !mbar_wait(&empty[st], phase, abort_flag)) { ok = false; break; }
-                    const int cur = st;
-                    if (++st == S) { st = 0; phase ^= 1; }
-                    room = mbar_test(&empty[st], phase);
-                    if (one) {
-                        uint8_t *dst = ring + size_t(cur) * kGStage;
-                        mbar_expect_tx(&full[cur], bytes);
-                        bulk_load(dst, a0, kURec, &full[cur]);
-                        if (q.has1) bulk_load(dst + kURec, a1, kURec, &full[cur]);
-                        bulk_load(dst + 2 * kURec, b, kBBlock, &full[cur]);
-                    }
+        // from here on the whole warp walks the loop and one elected lane issues: warp-uniform operands issue twice as fast
+        const bool one = elect_one();
+        int g = begin + first, st = first == S ? 0 : first;
+        uint32_t phase = 0; // of the empty barriers
+        bool ok = true, room = g < end && mbar_test(&empty[st], phase);
+        while (g < end && ok) {
+            const GRun r = run_at(p, g, end);
+            const int pair = r.unit / p.ngroups, grp = r.unit - pair * p.ngroups;
+            const PairSrc q = pair_src<SWIGLU>(p, pair, r.kb0);
+            const uint8_t *a0 = q.a0, *a1 = q.a1, *b = p.bimg + (size_t(r.kb0) * p.ngroups + grp) * kBBlock;
+            const size_t bstep = size_t(p.ngroups) * kBBlock;
+            const uint32_t bytes = (q.has1 ? 2 : 1) * kURec + kBBlock;
+            for (int k = 0; k < r.len; k++, a0 += kURec, a1 += kURec, b += bstep) {
+                if (!room && !mbar_wait(&empty[st], phase, abort_flag)) { ok = false; break; }
+                const int cur = st;
+                if (++st == S) { st = 0; phase ^= 1; }
+                room = mbar_test(&empty[st], phase);
+                if (one) {
+                    uint8_t *dst = ring + size_t(cur) * kGStage;
+                    mbar_expect_tx(&full[cur], bytes);
+                    bulk_load(dst, a0, kURec, &full[cur]);
+                    if (q.has1) bulk_load(dst + kURec, a1, kURec, &full[cur]);
+                    bulk_load(dst + 2 * kURec, b, kBBlock, &full[cur]);
                 }
-                g += r.len;
             }
-            GEMM_STAMP(4);
+            g += r.len;
         }
     } else if (warp == 4) {
         // ---- MMA issuer --------------------------------------------------------------------------------------------------
@@ -470,21 +434,22 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
         // E2M1 x E2M1, UE8M0 scales, N columns, M = 128; K-step s of a block uses the weight scale bytes 2s, 2s+1 and byte 0 of the digits' (all equal)
         constexpr uint32_t idesc0 = (1u << 7) | (1u << 10) | ((uint32_t(N) >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
         constexpr uint32_t idesc1 = idesc0 | (2u << 29);
-        if (one) copy_scales(tmem + kSfbCol, umma_desc(smem_u32(sfb), 16, 128));
+        if (one) { // 128 columns' scales per copy
+            copy_scales(tmem + kSfbCol, umma_desc(smem_u32(sfb), 16, 128));
+            if (N > 128) copy_scales(tmem + kSfbCol + 4, umma_desc(smem_u32(sfb), 16, 128));
+        }
         const uint64_t da0 = umma_desc(smem_u32(ring), 128, 256), dsf0 = umma_desc(smem_u32(ring) + 8192, 16, 128);
-        // (A missing second tile's copy and MMAs read ring bytes nobody wrote; their results are never looked at.)
+        const uint32_t d0 = tmem, d1 = tmem + uint32_t(N);
         int st = 0, sfa = 0;
         uint32_t phase = 0;
         bool ok = true, here = mbar_test(&full[0], 0);
         int g = begin;
         for (int run = 0; g < end && ok; run++) {
             const GRun r = run_at(p, g, end);
-            const bool has1 = 2 * (r.unit / p.ngroups) + 1 < p.total_tiles;
-            const int buf = run % NB;
-            ok = mbar_wait(&dempty[buf], ((run / NB) & 1) ^ 1, abort_flag); // first use of each set passes at once
+            const bool has1 = SWIGLU || 2 * (r.unit / p.ngroups) + 1 < p.total_tiles;
+            ok = mbar_wait(&dempty, (run & 1) ^ 1, abort_flag); // the first run passes at once
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t d0 = tmem + uint32_t(buf * 2 * N), d1 = d0 + uint32_t(N);
             for (int k = 0; k < r.len; k++) {
                 if (!here && !mbar_wait(&full[st], phase, abort_flag)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -505,34 +470,19 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
                 }
                 sfa = (sfa + 1) & (kGSfaBufs - 1);
             }
-            if (ok && one) commit_to(&dfull[buf]);
+            if (ok && one) commit_to(&dfull);
             g += r.len;
         }
-        GEMM_STAMP(6);
-    } else if (warp < 4) {
+    } else {
         // ---- epilogue: tensor-memory lane = row of the tile; token t of the group = columns 8t .. 8t+7 --------------------
-        float gate_val[NMAT == 2 ? 2 : 1][NMAT == 2 ? TPG : 1], zero[TPG];
-#pragma unroll
-        for (int t = 0; t < TPG; t++) zero[t] = 0.f;
-        if (NMAT == 2) {
-#pragma unroll
-            for (int t = 0; t < TPG; t++) gate_val[0][NMAT == 2 ? t : 0] = gate_val[NMAT == 2 ? 1 : 0][NMAT == 2 ? t : 0] = 0.f;
-        }
         asm volatile("griddepcontrol.wait;" ::: "memory"); // per-token scales, residual inputs and tickets come from earlier launches
         bool ok = true;
         int g = begin;
         for (int run = 0; g < end && ok; run++) {
             const GRun r = run_at(p, g, end);
             g += r.len;
-            const int buf = run % NB;
             const int pair = r.unit / p.ngroups, grp = r.unit - pair * p.ngroups;
-            float ia[TPG]; // the group's per-token scales: fetched while the run multiplies
-#pragma unroll
-            for (int t = 0; t < TPG; t += 4) {
-                const float4 q = __ldcg(reinterpret_cast<const float4 *>(p.inv_alpha + grp * TPG) + (t >> 2));
-                ia[t] = q.x; ia[t + 1] = q.y; ia[t + 2] = q.z; ia[t + 3] = q.w;
-            }
-            ok = mbar_wait(&dfull[buf], (run / NB) & 1, abort_flag);
+            ok = mbar_wait(&dfull, run & 1, abort_flag);
             {   // the 128 epilogue threads go on or give up together (they meet at named barriers below)
                 uint32_t all;
                 asm volatile("{\n.reg .pred q, r;\nsetp.ne.b32 q, %1, 0;\nbar.red.and.pred r, 1, 128, q;\nselp.u32 %0, 1, 0, r;\n}"
@@ -541,35 +491,31 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
             }
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (tid == 0 && g >= end) GEMM_STAMP(7); // the last run's accumulators are complete
-            const bool has1 = 2 * pair + 1 < p.total_tiles;
+            const bool has1 = SWIGLU || 2 * pair + 1 < p.total_tiles;
             float y[2][TPG];
-            load_sums<TPG>(tmem + uint32_t((buf * 2) * N) + (uint32_t(warp * 32) << 16), y[0]);
-            if (has1) load_sums<TPG>(tmem + uint32_t((buf * 2 + 1) * N) + (uint32_t(warp * 32) << 16), y[1]);
+            load_sums<TPG>(tmem + (uint32_t(warp * 32) << 16), y[0]);
+            if (has1) load_sums<TPG>(tmem + uint32_t(N) + (uint32_t(warp * 32) << 16), y[1]);
+            else {
+#pragma unroll
+                for (int t = 0; t < TPG; t++) y[1][t] = 0.f;
+            }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(&dempty[buf]);
-            if (tid == 0 && g >= end) GEMM_STAMP(10); // the last run's sums are in registers
+            if (lane == 0) mbar_arrive(&dempty);
 
-            const int ubegin = r.unit * L, uend = ubegin + L;
-            const bool whole = begin <= ubegin && uend <= end; // the whole unit lies in this CTA's share
-            bool last = false;
-            int c_first = 0, c_last = 0;
-            if (!whole) {
+            const int ubegin = r.unit * nkb, uend = ubegin + nkb;
+            if (begin > ubegin || uend > end) {
                 // ---- a unit cut by a share boundary: leave the partial sums; the CTA that arrives last adds them up ----
-                c_first = cta_of_stage(p, ubegin, G);
-                c_last = cta_of_stage(p, uend - 1, G);
+                const int c_first = cta_of_stage(p, ubegin, G), c_last = cta_of_stage(p, uend - 1, G);
                 const int which = (begin > ubegin) ? 0 : 1; // the unit that contains this share's first stage, or a later one
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     if (h == 1 && !has1) break;
-                    float *slot = p.partials + (((size_t(c) * 2 + which) * 2 + r.mat) * 2 + h) * kSlotFloats + size_t(tid) * TPG;
+                    float *slot = p.partials + ((size_t(c) * 2 + which) * 2 + h) * kSlotFloats + size_t(tid) * TPG;
 #pragma unroll
                     for (int t = 0; t < TPG; t += 4)
                         __stcg(reinterpret_cast<float4 *>(slot + t), make_float4(y[h][t], y[h][t + 1], y[h][t + 2], y[h][t + 3]));
                 }
-                const bool my_last_of_unit = g == end || g == uend;
-                if (!my_last_of_unit) continue;
                 // The barrier makes the 128 threads' partial stores visible to thread 0; its release at GPU scope is cumulative
                 // over them, and the last arriver's acquire + the next barrier hand the other CTAs' stores to its 128 readers.
                 asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -580,79 +526,65 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
                     if (s_last) p.tickets[c_first] = 0; // ready for the next launch
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");
-                last = s_last != 0;
+                const bool last = s_last != 0;
                 asm volatile("bar.sync 1, 128;" ::: "memory"); // s_last may be rewritten by the next cut unit
-                if (tid == 0 && g >= end) GEMM_STAMP(11);      // the last run's ticket is drawn
                 if (!last) continue;
-            } else if (NMAT == 2 && r.mat == 0) {
+                // the last arriver: add the parts in share order (the sum does not depend on who arrived last), both records
+                // of a part at once, so that a part costs one trip to L2
+                float acc[2][TPG];
 #pragma unroll
-                for (int t = 0; t < TPG; t++) { gate_val[0][NMAT == 2 ? t : 0] = y[0][t]; gate_val[NMAT == 2 ? 1 : 0][NMAT == 2 ? t : 0] = y[1][t]; }
-                continue;
+                for (int t = 0; t < TPG; t++) acc[0][t] = acc[1][t] = 0.f;
+                auto fetch = [&](int cc, float4 (&q)[2][TPG / 4]) {
+                    const float *slot = p.partials + (size_t(cc) * 2 + (share_begin(p, cc, G) > ubegin ? 0 : 1)) * 2 * kSlotFloats + size_t(tid) * TPG;
+#pragma unroll
+                    for (int h = 0; h < 2; h++)
+#pragma unroll
+                        for (int t = 0; t < TPG / 4; t++)
+                            q[h][t] = h == 0 || has1 ? __ldcg(reinterpret_cast<const float4 *>(slot + h * kSlotFloats) + t) : make_float4(0.f, 0.f, 0.f, 0.f);
+                };
+                float4 q[2][TPG / 4];
+                fetch(c_first, q);
+                for (int cc = c_first; cc <= c_last; cc++) {
+                    float4 nq[2][TPG / 4]; // the next part is on its way while this one is added
+                    fetch(min(cc + 1, c_last), nq);
+#pragma unroll
+                    for (int h = 0; h < 2; h++)
+#pragma unroll
+                        for (int t = 0; t < TPG / 4; t++) {
+                            acc[h][4 * t] += q[h][t].x; acc[h][4 * t + 1] += q[h][t].y; acc[h][4 * t + 2] += q[h][t].z; acc[h][4 * t + 3] += q[h][t].w;
+                            q[h][t] = nq[h][t];
+                        }
+                }
+#pragma unroll
+                for (int t = 0; t < TPG; t++) { y[0][t] = acc[0][t]; y[1][t] = acc[1][t]; }
             }
-            if (whole) {
+            float ia[TPG]; // the group's per-token scales
+#pragma unroll
+            for (int t = 0; t < TPG; t += 4) {
+                const float4 q = __ldcg(reinterpret_cast<const float4 *>(p.inv_alpha + grp * TPG) + (t >> 2));
+                ia[t] = q.x; ia[t + 1] = q.y; ia[t + 2] = q.z; ia[t + 3] = q.w;
+            }
+            if constexpr (SWIGLU) {
+                const GSeg &s = p.seg[gseg_of(p, pair)];
+                const int row = (pair - s.tile_begin) * 128 + tid;
+                if (row < s.rows) finish_row<TPG>(p, s, row, grp, y[1], y[0], ia);
+            } else {
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     if (h == 1 && !has1) break;
                     const int tile = 2 * pair + h;
                     const GSeg &s = p.seg[gseg_of(p, tile)];
                     const int row = (tile - s.tile_begin) * 128 + tid;
-                    if (row < s.rows) {
-                        if constexpr (NMAT == 2) finish_row<TPG>(p, s, row, grp, y[h], gate_val[h], ia);
-                        else finish_row<TPG>(p, s, row, grp, y[h], zero, ia);
-                    }
+                    if (row < s.rows) finish_row<TPG>(p, s, row, grp, y[h], y[h], ia);
                 }
-                continue;
-            }
-            // the last arriver: add the parts in share order (the sum does not depend on who arrived last)
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                if (h == 1 && !has1) break;
-                float acc[NMAT][TPG]; // [matrix][token]
-#pragma unroll
-                for (int t = 0; t < TPG; t++) acc[0][t] = acc[NMAT - 1][t] = 0.f;
-                int b = share_begin(p, c_first, G);
-                for (int cc = c_first; cc <= c_last; cc++) {
-                    const int e = share_begin(p, cc + 1, G);
-                    const int which = (b > ubegin) ? 0 : 1;
-#pragma unroll
-                    for (int mat = 0; mat < NMAT; mat++) {
-                        const int mb = ubegin + mat * nkb, me = mb + nkb;
-                        if (max(b, mb) >= min(e, me)) continue; // that share holds nothing of this matrix
-                        if (cc == c && mat == r.mat) { // this CTA's newest partial is still in registers
-#pragma unroll
-                            for (int t = 0; t < TPG; t++) acc[mat][t] += y[h][t];
-                            continue;
-                        }
-                        const float *slot = p.partials + (((size_t(cc) * 2 + which) * 2 + mat) * 2 + h) * kSlotFloats + size_t(tid) * TPG;
-                        float4 q[TPG / 4];
-#pragma unroll
-                        for (int t = 0; t < TPG / 4; t++) q[t] = __ldcg(reinterpret_cast<const float4 *>(slot) + t);
-#pragma unroll
-                        for (int t = 0; t < TPG / 4; t++) {
-                            acc[mat][4 * t] += q[t].x; acc[mat][4 * t + 1] += q[t].y; acc[mat][4 * t + 2] += q[t].z; acc[mat][4 * t + 3] += q[t].w;
-                        }
-                    }
-                    b = e;
-                }
-                if (tid == 0 && g >= end && h == 0) GEMM_STAMP(12); // first tile's parts added
-                const int tile = 2 * pair + h;
-                const GSeg &s = p.seg[gseg_of(p, tile)];
-                const int row = (tile - s.tile_begin) * 128 + tid;
-                if (row < s.rows) {
-                    if constexpr (NMAT == 2) finish_row<TPG>(p, s, row, grp, acc[1], acc[0], ia);
-                    else finish_row<TPG>(p, s, row, grp, acc[0], zero, ia);
-                }
-                if (tid == 0 && g >= end && h == 0) GEMM_STAMP(13); // first tile finished
             }
         }
     }
-    if (tid == 0) GEMM_STAMP(8); // epilogue role done
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kGTmemCols));
     if (tid == 0 && s_abort && p.error_flag) *p.error_flag = 1;
-    if (tid == 0) GEMM_STAMP(9);
 }
 
 // ---- host side --------------------------------------------------------------------------------------------------------
@@ -660,14 +592,19 @@ namespace {
 std::mutex g_gemm_attr_mutex;
 bool g_gemm_attr_done[64] = {false}; // the shared-memory opt-in is a per-device function attribute
 
-int tokens_per_group(int tokens) { return tokens <= 8 ? 8 : 16; }
+// Tokens per group: the one that takes fewer bytes into shared memory over all groups (the last one may be padded).
+int tokens_per_group(int tokens)
+{
+    const int g16 = (tokens + 15) / 16, g24 = (tokens + 23) / 24;
+    return g24 * (2 * kURec + 512 * 24) < g16 * (2 * kURec + 512 * 16) ? 24 : 16;
+}
 size_t image_bytes(int cols, int tokens)
 {
     const int tpg = tokens_per_group(tokens);
     const size_t groups = size_t(tokens + tpg - 1) / tpg;
     return size_t(cols >> 7) * groups * 512 * tpg;
 }
-constexpr size_t kPartialBytes = size_t(kGMaxGrid) * 2 * 2 * 2 * kSlotFloats * sizeof(float); // [CTA][cut unit][matrix][tile of the pair]
+constexpr size_t kPartialBytes = size_t(kGMaxGrid) * 2 * 2 * kSlotFloats * sizeof(float); // [CTA][cut unit][record of the pair]
 } // namespace
 
 
@@ -718,7 +655,6 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     p.nseg = op->n_segments;
     p.ngroups = ngroups;
     p.tokens = tokens;
-    p.tpg = tpg;
     int tiles = 0, nmat_all = 0;
     for (int i = 0; i < op->n_segments; i++) {
         const insg_gemv_segment &s = op->seg[i];
@@ -733,21 +669,21 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
         g.packed2 = static_cast<const uint8_t *>(s.packed2);
         g.out = s.out; g.conv_state = s.conv_state; g.conv_w = s.conv_w; g.A_log = s.A_log; g.dt_bias = s.dt_bias;
         g.conv_stride = s.conv_token_stride;
-        g.nmat = s.epilogue == INSG_EPI_SWIGLU ? 2 : 1;
-        if (nmat_all && nmat_all != g.nmat) return fail(INSG_E_SHAPE, "gemm: SwiGLU segments cannot be mixed with others");
-        nmat_all = g.nmat;
-        g.tile_begin = tiles; g.ntiles = (s.rows + 127) >> 7; tiles += g.ntiles; g.epilogue = s.epilogue; g.rows = s.rows;
+        const int nmat = s.epilogue == INSG_EPI_SWIGLU ? 2 : 1;
+        if (nmat_all && nmat_all != nmat) return fail(INSG_E_SHAPE, "gemm: SwiGLU segments cannot be mixed with others");
+        nmat_all = nmat;
+        g.tile_begin = tiles; tiles += (s.rows + 127) >> 7; g.epilogue = s.epilogue; g.rows = s.rows;
     }
     p.total_tiles = tiles;
-    p.nmat = nmat_all;
-    const long long total = (long long)((tiles + 1) / 2) * ngroups * nmat_all * nkb; // a unit = (pair of tiles, token group)
+    const long long total = (long long)(nmat_all == 2 ? tiles : (tiles + 1) / 2) * ngroups * nkb; // a unit = (pair of records, token group)
     if (total > (1ll << 30)) return fail(INSG_E_LIMIT, "gemm: more than 2^30 (tile, group, k-block) stages");
     p.total_stages = int(total);
     p.error_flag = op->error_flag;
     const int stage_bytes = 2 * kURec + 512 * tpg;
     p.stages = std::min(kGMaxStages, (224 * 1024 - 512) / stage_bytes);
     const size_t smem = size_t(p.stages) * stage_bytes + 512;
-    auto kernel = tpg == 8 ? (nmat_all == 2 ? umma_gemm_kernel<8, 2> : umma_gemm_kernel<8, 1>) : (nmat_all == 2 ? umma_gemm_kernel<16, 2> : umma_gemm_kernel<16, 1>);
+    auto kernel = tpg == 16 ? (nmat_all == 2 ? umma_gemm_kernel<16, true> : umma_gemm_kernel<16, false>)
+                            : (nmat_all == 2 ? umma_gemm_kernel<24, true> : umma_gemm_kernel<24, false>);
     {
         int dev = 0;
         cudaError_t e = cudaGetDevice(&dev);
@@ -755,10 +691,8 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
         if (dev < 0 || dev >= 64) return fail(INSG_E_LIMIT, "gemm: device ordinal beyond 63");
         std::lock_guard<std::mutex> lock(g_gemm_attr_mutex);
         if (!g_gemm_attr_done[dev]) {
-            e = cudaFuncSetAttribute(umma_gemm_kernel<8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(umma_gemm_kernel<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(umma_gemm_kernel<16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(umma_gemm_kernel<16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
+            for (auto k : {umma_gemm_kernel<16, false>, umma_gemm_kernel<16, true>, umma_gemm_kernel<24, false>, umma_gemm_kernel<24, true>})
+                if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
             if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(umma gemm)");
             g_gemm_attr_done[dev] = true;
         }
@@ -767,7 +701,11 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     // records while the digits are being written
     int rc = launch(umma_digitize_kernel, dim3(ngroups * tpg * d.parts), dim3(kGThreads), 0, st, op->pdl != 0, d);
     if (rc != INSG_OK) return rc;
-    const int grid = std::max(1, std::min(std::min(sm_count(), kGMaxGrid), p.total_stages));
+    // Every part of a cut unit costs the CTA that adds them a trip to L2, about what a stage takes: few stages go to fewer CTAs,
+    // so that a unit is cut into about sqrt(nkb) parts of sqrt(nkb) stages at most.
+    int least = 1;
+    while (least * least < nkb) least++;
+    const int grid = std::max(1, std::min({sm_count(), kGMaxGrid, p.total_stages, std::max(1, p.total_stages / least)}));
     p.share = p.total_stages / grid;
     p.share_rem = p.total_stages % grid;
     rc = launch(kernel, dim3(grid), dim3(kGemmThreads), smem, st, true, p); // may start while the digits are being written
@@ -788,18 +726,6 @@ using namespace insg;
 
 extern "C" {
 
-#ifdef INSG_PHASE_TIMES
-// development builds: the stamps of the last launch -> host array of 256 * 16 + 4 values
-__attribute__((visibility("default"))) int insg_debug_gemm_stamps(unsigned long long *host_out)
-{
-    return cudaMemcpyFromSymbol(host_out, g_gemm_stamps, sizeof(g_gemm_stamps)) == cudaSuccess ? 0 : 1;
-}
-__attribute__((visibility("default"))) int insg_debug_gemm_stamps_clear()
-{
-    static unsigned long long zeros[kGMaxGrid * 16 + 4];
-    return cudaMemcpyToSymbol(g_gemm_stamps, zeros, sizeof(zeros)) == cudaSuccess ? 0 : 1;
-}
-#endif
 
 size_t insg_umma_gemm_scratch_bytes(int cols, int tokens) { return umma_gemm_scratch(cols, tokens); }
 
