@@ -264,14 +264,22 @@ __global__ void __launch_bounds__(2 * kDnThreads, 1) deltanet_steps_kernel(float
             const int n = min(kDnBlock, tokens - base);
             unsigned long long q[8], k[8];
             dn_vector(k, d.k[0], lane);
+            float v = d.v[0][in], decay = d.decay[0], beta = d.beta[0];
+#pragma unroll 4
             for (int s = 0; s < n; s++) {
+                const int next = min(s + 1, kDnBlock - 1); // what the next step needs is requested a step ahead
+                unsigned long long nk[8];
+                dn_vector(nk, d.k[next], lane);
+                const float nv = d.v[next][in], ndecay = d.decay[next], nbeta = d.beta[next];
                 dn_vector(q, d.q[s], lane);
                 const float2 pm = dn_products(cells, k);
                 const float mem = dn_fold(pm, lane), o = dn_fold(po, lane); // po: the previous step's output
                 if (base + s > 0 && (lane & 7) < 2) out[size_t(base + s - 1) * 4096] = o;
-                dn_update(cells, k, mem, d.v[s][in], d.decay[s], d.beta[s], lane);
-                dn_vector(k, d.k[min(s + 1, kDnBlock - 1)], lane);
+                dn_update(cells, k, mem, v, decay, beta, lane);
                 po = dn_products(cells, q);
+#pragma unroll
+                for (int i = 0; i < 8; i++) k[i] = nk[i];
+                v = nv; decay = ndecay; beta = nbeta;
             }
         }
         __syncthreads();
