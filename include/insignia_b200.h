@@ -221,7 +221,7 @@ typedef struct insg_gemv_op {
     int prep_rms;               /* INSG_PRO_PREPARED: 1 = scale by the RMS factor computed from prep_partials            */
     int tokens;                 /* 0 or 1: one token.  More: consecutive tokens of one sequence in one call (the weights are
                                    streamed once per pass): in, aux and x_out are [tokens][cols], every out is
-                                   [tokens][rows]; the convolution history is advanced token by token.  layout 0: 2 or 4
+                                   [tokens][rows]; the convolution history is advanced token by token.  layout 0: 2 to 4
                                    tokens (one launch of the mma.sync kernel); layout 1: any count up to 4096, up to eight
                                    in one launch of the GEMV kernel, more through the GEMM kernel, sixteen tokens per
                                    tcgen05 instruction (needs umma_scratch).  Not with INSG_PRO_PREPARED, prepared

@@ -103,7 +103,7 @@ int gemv_build_params(const insg_gemv_op *op, int M, int max_grid, GemvParams *o
     if (op->cols <= 0 || (op->cols & 127) || op->cols > kMaxVec * kThreads * 4)
         return fail(INSG_E_SHAPE, "gemv: cols must be a multiple of 128, <= 12288");
     if (op->n_segments < 1 || op->n_segments > 4) return fail(INSG_E_SHAPE, "gemv: 1..4 segments");
-    if (M != 1 && M != 2 && M != 4) return fail(INSG_E_SHAPE, "gemv: 1, 2 or 4 tokens per launch");
+    if (M < 1 || M > 4) return fail(INSG_E_SHAPE, "gemv: 1..4 tokens per launch");
     if ((op->prologue == INSG_PRO_RMSNORM || op->prologue == INSG_PRO_GATED_RMSNORM) && !op->norm_w)
         return fail(INSG_E_ARG, "gemv: norm weight missing");
     if (op->prologue >= INSG_PRO_GATED_RMSNORM && op->prologue != INSG_PRO_PREPARED && !op->aux)
@@ -185,6 +185,7 @@ int gemv_fused_launch(const insg_gemv_op *op, int M, cudaStream_t st)
     switch (M) {
     case 1: return launch_variant<kUnr, 1>(p, grid, smem, st, pdl);
     case 2: return launch_variant<kUnr, 2>(p, grid, smem, st, pdl);
+    case 3: return launch_variant<2, 3>(p, grid, smem, st, pdl);
     default: return launch_variant<2, 4>(p, grid, smem, st, pdl); // four tokens: registers go to the accumulators
     }
 }
@@ -208,7 +209,7 @@ int insg_mxfp4_gemv_packed(const void *packed, const float *x, float *y, int row
     if (M < 1 || M > 4096) return fail(INSG_E_SHAPE, "gemv_packed: 1 <= M <= 4096");
     for (int m0 = 0; m0 < M;) {
         const int left = M - m0;
-        const int mm = left >= 4 ? 4 : (left >= 2 ? 2 : 1);
+        const int mm = std::min(left, 4);
         insg_gemv_op op = {};
         op.in = x + size_t(m0) * cols;
         op.cols = cols;

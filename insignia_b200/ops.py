@@ -18,8 +18,12 @@ EPI = {"store": 0, "residual": 1, "conv_silu": 2, "beta": 3, "decay": 4, "swiglu
 KV_F32, KV_BF16 = 0, 1
 
 
+# The handle of the current stream without a Stream object around it: on calls of a few microseconds that object is a tenth.
+_raw_stream, _current_device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+
+
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_current_device())
 
 
 def _p(t):
@@ -28,6 +32,12 @@ def _p(t):
     if not t.is_cuda or not t.is_contiguous():
         raise ValueError("expected a contiguous CUDA tensor")
     return t.data_ptr()
+
+
+def _tokens(x, cols):
+    if x.shape[-1] != cols:
+        raise ValueError(f"expected vectors of {cols} elements")
+    return x.numel() // cols
 
 
 def tune(key: str, value: int) -> None:
@@ -81,10 +91,10 @@ def repack_umma(weight, scales):
 def gemv_packed(packed, x, rows=None, cols=None):
     rows = rows or packed.rows
     cols = cols or packed.cols
-    x2 = x.reshape(-1, cols)
-    y = torch.empty((x2.shape[0], rows), dtype=torch.float32, device=x.device)
-    check(_lib.lib().insg_mxfp4_gemv_packed(_p(packed), _p(x2), _p(y), rows, cols, x2.shape[0], _stream()))
-    return y.reshape(*x.shape[:-1], rows)
+    M, x = _tokens(x, cols), x.contiguous()
+    y = x.new_empty((*x.shape[:-1], rows), dtype=torch.float32)
+    check(_lib.lib().insg_mxfp4_gemv_packed(_p(packed), _p(x), y.data_ptr(), rows, cols, M, _stream()))
+    return y
 
 
 def _gemv_op(inp, segments, prologue="plain", aux=None, norm_w=None, x_out=None, argmax=None, pdl=False, layout=0, error_flag=None,
@@ -122,12 +132,11 @@ def gemm_umma(packed_umma, x, rows=None, cols=None, scratch=None):
     """``y[m] = W x[m]`` for all rows of ``x`` on the tcgen05 tensor cores (weights from :func:`repack_umma`)."""
     rows = rows or packed_umma.rows
     cols = cols or packed_umma.cols
-    x2 = x.reshape(-1, cols)
-    M = x2.shape[0]
+    M, x = _tokens(x, cols), x.contiguous()
     scratch = scratch if scratch is not None else umma_gemm_scratch(cols, M, x.device)
-    y = torch.empty((M, rows), dtype=torch.float32, device=x.device)
-    check(_lib.lib().insg_mxfp4_gemm_umma(_p(packed_umma), _p(x2), _p(y), rows, cols, M, _p(scratch), scratch.numel(), _stream()))
-    return y.reshape(*x.shape[:-1], rows)
+    y = x.new_empty((*x.shape[:-1], rows), dtype=torch.float32)
+    check(_lib.lib().insg_mxfp4_gemm_umma(_p(packed_umma), _p(x), y.data_ptr(), rows, cols, M, _p(scratch), scratch.numel(), _stream()))
+    return y
 
 
 def gemv_fused(inp, segments, **kw):
