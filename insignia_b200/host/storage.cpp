@@ -149,7 +149,8 @@ struct TieredStorage::Impl {
     cudaStream_t consumer;
     std::unique_ptr<StorageBackend> be;
     mutable std::mutex mu;           // slots, lists, counters
-    std::condition_variable cv;      // a Loading slot became Resident (or Absent again)
+    std::condition_variable cv;      // a Loading slot became Resident (or Absent again), a prefetch ended
+    bool prefetching = false;        // the worker is loading a slot
     std::vector<Slot> slots;
     int lru_head = -1, lru_tail = -1; // head = least recently used
     int cache_head = -1, cache_tail = -1;
@@ -243,6 +244,18 @@ struct TieredStorage::Impl {
             used -= tensor(victim).bytes;
             st.evictions++;
         }
+    }
+
+    // A prefetch in flight holds its bytes without being evictable yet: whoever finds no room because of one waits for it.
+    // Caller holds mu; true when the wait changed something (the caller looks at its slot again).
+    bool wait_for_prefetch(uint64_t bytes, std::unique_lock<std::mutex> &lock)
+    {
+        if (!prefetching || bytes > budget) return false;
+        uint64_t evictable = 0;
+        for (int v = lru_head; v >= 0; v = slots[size_t(v)].next) evictable += tensor(v).bytes;
+        if (used - evictable + reserved + bytes <= budget) return false;
+        cv.wait(lock, [&] { return !prefetching; });
+        return true;
     }
 
     // The pinned-host cache keeps the most recently uploaded tensors within its own budget.  Caller holds mu.
@@ -354,12 +367,15 @@ struct TieredStorage::Impl {
             Slot &s = slots[size_t(i)];
             s.queued = false;
             if (s.state != Absent) continue;
+            prefetching = true;
             try {
                 load(i, lock, true);
                 if (s.pins == 0 && !s.in_lru) lru_push(i);
             } catch (...) {
                 // a prefetch that does not fit or fails is dropped; acquire() will report the error if it matters
             }
+            prefetching = false;
+            cv.notify_all();
         }
     }
 };
@@ -408,7 +424,8 @@ DeviceView TieredStorage::acquire(std::string_view name)
     std::unique_lock<std::mutex> lock(m.mu);
     ensure_backend(m.be);
     Impl::Slot &s = m.slots[size_t(i)];
-    m.cv.wait(lock, [&] { return s.state != Impl::Loading; }); // join an upload the prefetcher has in flight
+    do m.cv.wait(lock, [&] { return s.state != Impl::Loading; }); // join an upload the prefetcher has in flight
+    while (s.state == Impl::Absent && m.wait_for_prefetch(t.bytes, lock));
     if (s.state == Impl::Resident) m.st.hits++;
     else m.load(i, lock, false);
     m.lru_remove(i);
@@ -465,8 +482,9 @@ MemoryTier TieredStorage::tier(std::string_view name) const
 void TieredStorage::reserve(uint64_t bytes)
 {
     Impl &m = *impl_;
-    std::lock_guard<std::mutex> lock(m.mu);
+    std::unique_lock<std::mutex> lock(m.mu);
     ensure_backend(m.be);
+    while (m.wait_for_prefetch(bytes, lock));
     m.make_room(bytes, false);
     m.reserved += bytes;
 }
