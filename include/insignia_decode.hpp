@@ -139,7 +139,7 @@ private:
     Qwen35Weights &w_;
     DecodeWorkspace &x_;
     std::unique_ptr<Plan> plan_;
-    int mtp_step(int token, bool draft);
+    void mtp_step(int token, bool draft);
     void build_program();
     void run_program(int n_tokens, int token);
     void recover_after_timeout();

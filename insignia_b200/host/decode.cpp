@@ -153,7 +153,7 @@ struct Qwen35Decode::Plan {
     cudaKernelNodeParams scalars_params{};
     cudaGraphExec_t exec_multi{}; // kMultiSteps token steps in one graph, for device-fed generation
     cudaGraphExec_t exec_chunk{}; // one pass of forward_tokens over kChunk prompt tokens
-    int *host_result{}; // pinned: {next token, wait-expired flag}, so the per-token read-back is a true asynchronous copy
+    int *host_result{}; // pinned: {next token, wait-expired flag, the two results of a verify pass}, so the per-token read-back is a true asynchronous copy
     float *spec_state{}, *spec_conv{}, *spec_logits{}; // speculative decode: second DeltaNet state, convolution snapshot, [2][vocab] logits
     int *spec_pair{};                                  // device: the two arg-max results of a verify pass
     int *spec_host{};                                  // pinned: {token, draft} on the way in
@@ -202,7 +202,7 @@ Qwen35Decode::Plan &Qwen35Decode::plan()
             cuda_check(cudaStreamCreateWithFlags(&plan_->stream, cudaStreamDefault), "cudaStreamCreate");
             plan_->own_stream = true;
         }
-        cuda_check(cudaMallocHost(&plan_->host_result, 2 * sizeof(int)), "cudaMallocHost");
+        cuda_check(cudaMallocHost(&plan_->host_result, 4 * sizeof(int)), "cudaMallocHost");
     }
     return *plan_;
 }
@@ -1223,11 +1223,16 @@ template <class F> void run_graphed(bool use_graph, cudaStream_t st, cudaGraphEx
 }
 } // namespace
 
-int Qwen35Decode::mtp_draft(int token) { return mtp_step(token, true); }
+int Qwen35Decode::mtp_draft(int token)
+{
+    mtp_step(token, true);
+    return logits_argmax();
+}
 
 // The MTP block at the current position (reference: src/decode.cu:24-68).  draft = false stops before the head: the call
 // then only leaves the position's row in the MTP cache (a speculative decoder needs every row, the prompt's included).
-int Qwen35Decode::mtp_step(int token, bool draft)
+// Asynchronous: logits_argmax() waits for the draft.
+void Qwen35Decode::mtp_step(int token, bool draft)
 {
     if (token < 0 || token >= Qwen35Shape::vocab) throw std::runtime_error("token out of range");
     if (x_.position < 1) throw std::runtime_error("mtp_draft needs a forwarded token");
@@ -1270,13 +1275,8 @@ int Qwen35Decode::mtp_step(int token, bool draft)
         if (c.tcgen05()) op.host_result = p.host_result;
         run_gemv(c, op);
     });
-    if (!draft) {
-        fused_token_valid_ = false;
-        return -1;
-    }
-    fused_token_valid_ = true;
+    fused_token_valid_ = draft;
     result_on_host_ = tcgen05_engine(x_.options);
-    return logits_argmax();
 }
 
 // ---- speculative greedy decode: draft-1 / verify ---------------------------------------------------------------------
@@ -1333,7 +1333,10 @@ std::vector<int> Qwen35Decode::generate_speculative(int first_token, int count, 
             break;
         }
         const int P = x_.position;
-        const int draft = forced_drafts ? forced_drafts[out.size()] : mtp_draft(tok);
+        // A draft of the MTP head goes to the verify pass on the device: the host waits once per pass, behind both.
+        const bool ahead = !forced_drafts && tcgen05_engine(x_.options);
+        if (ahead) mtp_step(tok, true);
+        int draft = forced_drafts ? forced_drafts[out.size()] : ahead ? 0 : mtp_draft(tok);
         if (draft < 0 || draft >= Qwen35Shape::vocab) throw std::runtime_error("draft token out of range");
         // ---- verify: tokens [tok, draft] at positions P, P + 1 ----
         Multi u(x_, 2);
@@ -1344,7 +1347,8 @@ std::vector<int> Qwen35Decode::generate_speculative(int first_token, int count, 
         p.spec_host[0] = tok;
         p.spec_host[1] = draft;
         sync_scalars(-1);
-        cuda_check(cudaMemcpyAsync(u.tokens, p.spec_host, 2 * sizeof(int), cudaMemcpyHostToDevice, p.stream), "copy tokens");
+        cuda_check(cudaMemcpyAsync(u.tokens, p.spec_host, (ahead ? 1 : 2) * sizeof(int), cudaMemcpyHostToDevice, p.stream), "copy tokens");
+        if (ahead) cuda_check(cudaMemcpyAsync(u.tokens + 1, x_.d_next, sizeof(int), cudaMemcpyDeviceToDevice, p.stream), "copy draft");
         const int which = cur == x_.delta_state ? 0 : 1;
         run_graphed(x_.options.use_graph, p.stream, p.exec_verify[which], p.verify_runs[which], launches_, [&] {
             cuda_check(cudaMemcpyAsync(p.spec_conv, x_.conv_state, conv_floats * sizeof(float), cudaMemcpyDeviceToDevice, p.stream), "snapshot history");
@@ -1370,10 +1374,17 @@ std::vector<int> Qwen35Decode::generate_speculative(int first_token, int count, 
             insg_check(insg_argmax_rows(p.spec_logits, x_.options.vocab, x_.options.vocab, 2, p.spec_pair, p.stream));
             launches_++;
         });
-        int *res = p.host_result;
+        int *res = p.host_result + 2;
         cuda_check(cudaMemcpyAsync(res, p.spec_pair, 2 * sizeof(int), cudaMemcpyDeviceToHost, p.stream), "read tokens");
         cuda_check(cudaStreamSynchronize(p.stream), "synchronize");
         const int r1 = res[0], r2 = res[1];
+        if (ahead) { // the MTP head left its result in pinned memory
+            draft = p.host_result[0];
+            if (p.host_result[1]) {
+                recover_after_timeout();
+                throw std::runtime_error("a bounded wait inside a GPU kernel expired");
+            }
+        }
         out.push_back(r1);
         if (r1 == draft) { // accepted: both positions stand
             hits++;
