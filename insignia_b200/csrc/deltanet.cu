@@ -8,25 +8,161 @@
 //   out_v  = sum_i S[i][v] * qh[i]
 // State layout fp32 [head][k=128][v=128], v contiguous.
 //
-// The reference reads the 64 KiB head state twice and writes it once from global memory with 32 CTAs.  Columns v are
-// independent, so here each head is cut into 4 slices of 32 columns (128 CTAs) and a slice over four warps; a warp pulls its
-// columns into registers once (issued before the dependent-launch wait because the state was last written a whole token
-// ago), does both reductions over k by shuffles, and writes them back once: 2 x 2 MiB of traffic per layer.  The step is a
-// latency chain, so it is kept short: all inputs are requested together, every warp normalises q and k for itself, and no
-// sum leaves the warp.
+// The reference reads the 64 KiB head state twice and writes it once from global
+// memory with 32 CTAs.  Columns v are independent, so here each head is cut into
+// 4 slices of 32 columns (128 CTAs); a CTA pulls its 16 KiB slice into registers
+// once (coalesced 128-byte row segments, issued before the dependent-launch wait
+// because the state was last written a whole token ago), does both reductions
+// over k on chip, and writes the slice back once: 2 x 2 MiB of traffic per layer.
+// The step is a latency chain, so it is kept short: all inputs are requested
+// together, every warp normalises q and k for itself, and only the two sums over
+// the eight warps cross a CTA barrier.
 #include "common.cuh"
 #include "host_util.h"
 #include "umma_common.cuh"
 
 namespace insg {
 
-constexpr int kDnThreads = 128;
+constexpr int kDnThreads = 256;
 constexpr int kSlices = 4; // 32 columns each
 
-// ---- the arithmetic of one step, shared by the kernels below (which are bit-identical for that reason) -----------------------
+// `tokens` consecutive steps of the sequence in one launch: the slice stays in registers from step to step and is
+// written back once; q/k/v of step m are at + m * qkv_stride, g/beta at + m * 32, the output at + m * 4096.
+// For one step the chain from the inputs to the stored state counts, not the arithmetic: eight warps hold rows kr + 32 j of
+// 32 columns (whole 128-byte row segments), and the sums cross the warps through shared memory: 2.5 us against 2.9 with the
+// warp-local columns of the kernel below, whose 8-byte accesses to the state cost a decoded token 1316 us instead of 1214.
+// Sums are taken in that kernel's order: over j, the rows 4 kq + 0..3 as (0 + 2) + (1 + 3), then the eight kq (here the warps)
+// in a tree.
+__global__ void __launch_bounds__(kDnThreads) deltanet_step_kernel(float *__restrict__ state, const float *__restrict__ q16,
+                                                                   const float *__restrict__ k16, const float *__restrict__ v32,
+                                                                   const float *__restrict__ g32, const float *__restrict__ beta32,
+                                                                   float *__restrict__ out32, int tokens, int qkv_stride, long long state_stride,
+                                                                   float *__restrict__ state_first, float *__restrict__ state_last)
+{
+    __shared__ __align__(16) float s_qk[8][2][128]; // per warp: its own copy of the normalised q and k (no block barrier)
+    __shared__ __align__(16) float s_part[2][8][32]; // per-warp partial sums over k: [0] memory read-out, [1] output
+
+    const int head = blockIdx.x / kSlices, slice = blockIdx.x % kSlices, kh = head >> 1;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int vq = tid & 7, kr = tid >> 3; // float4 column group, k row (rows kr, kr+32, kr+64, kr+96)
+    const int v0 = slice * 32 + vq * 4;
+
+    pdl_launch_dependents();
+
+    // blockIdx.y: independent sequence of a decode batch (its own state, its own inputs and outputs)
+    const int seq = blockIdx.y;
+    q16 += size_t(seq) * qkv_stride; k16 += size_t(seq) * qkv_stride; v32 += size_t(seq) * qkv_stride;
+    g32 += seq * 32; beta32 += seq * 32; out32 += size_t(seq) * 4096;
+    float *S = state + size_t(seq) * state_stride + size_t(head) * 128 * 128;
+    float4 cell[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) cell[j] = __ldcg(reinterpret_cast<const float4 *>(S + size_t(kr + 32 * j) * 128 + v0));
+
+    pdl_wait();
+
+    // Every dependent input of a step is requested at once; with several steps the next step's inputs are requested
+    // before this step's arithmetic (they do not depend on it), so only the first step waits for a load.
+    // Each warp reads the whole q and k of the key head (four values per lane) and normalises them itself: L2 norms
+    // over 128 with eps added to the sum, as the reference.
+    float4 nq4 = __ldcg(reinterpret_cast<const float4 *>(q16 + kh * 128) + lane);
+    float4 nk4 = __ldcg(reinterpret_cast<const float4 *>(k16 + kh * 128) + lane);
+    float4 nv4 = __ldcg(reinterpret_cast<const float4 *>(v32 + head * 128 + slice * 32) + vq); // this thread's columns
+    float ng = __ldcg(g32 + head), nbeta = __ldcg(beta32 + head);
+    for (int step = 0; step < tokens; step++, q16 += qkv_stride, k16 += qkv_stride, v32 += qkv_stride, g32 += 32, beta32 += 32, out32 += 4096) {
+        __syncwarp(); // the previous step's reads of this warp's q/k copy are done
+        const float4 q4 = nq4, k4 = nk4, v4 = nv4;
+        const float g_in = ng, beta = nbeta;
+        if (step + 1 < tokens) {
+            nq4 = __ldcg(reinterpret_cast<const float4 *>(q16 + qkv_stride + kh * 128) + lane);
+            nk4 = __ldcg(reinterpret_cast<const float4 *>(k16 + qkv_stride + kh * 128) + lane);
+            nv4 = __ldcg(reinterpret_cast<const float4 *>(v32 + qkv_stride + head * 128 + slice * 32) + vq);
+            ng = __ldcg(g32 + 32 + head);
+            nbeta = __ldcg(beta32 + 32 + head);
+        }
+        const float qn = warp_sum(fmaf(q4.x, q4.x, fmaf(q4.y, q4.y, fmaf(q4.z, q4.z, q4.w * q4.w))));
+        const float kn = warp_sum(fmaf(k4.x, k4.x, fmaf(k4.y, k4.y, fmaf(k4.z, k4.z, k4.w * k4.w))));
+        const float qs = rsqrtf(qn + 1e-6f) * 0.08838834764831845f, ks = rsqrtf(kn + 1e-6f);
+        reinterpret_cast<float4 *>(s_qk[warp][0])[lane] = make_float4(q4.x * qs, q4.y * qs, q4.z * qs, q4.w * qs);
+        reinterpret_cast<float4 *>(s_qk[warp][1])[lane] = make_float4(k4.x * ks, k4.y * ks, k4.z * ks, k4.w * ks);
+        __syncwarp();
+        float qq[4], kk[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            qq[j] = s_qk[warp][0][kr + 32 * j];
+            kk[j] = s_qk[warp][1][kr + 32 * j];
+        }
+        const float decay = expf(g_in);
+
+        // mem_v = sum_i S * k (times d below)
+        float4 pm = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            pm.x = fmaf(cell[j].x, kk[j], pm.x);
+            pm.y = fmaf(cell[j].y, kk[j], pm.y);
+            pm.z = fmaf(cell[j].z, kk[j], pm.z);
+            pm.w = fmaf(cell[j].w, kk[j], pm.w);
+        }
+        // a warp holds 4 k-rows (lane>>3) x 8 column groups: fold the rows, then every thread folds the 8 warps itself
+#pragma unroll
+        for (int m = 16; m >= 8; m >>= 1) {
+            pm.x += __shfl_xor_sync(0xffffffffu, pm.x, m);
+            pm.y += __shfl_xor_sync(0xffffffffu, pm.y, m);
+            pm.z += __shfl_xor_sync(0xffffffffu, pm.z, m);
+            pm.w += __shfl_xor_sync(0xffffffffu, pm.w, m);
+        }
+        if (lane < 8) *reinterpret_cast<float4 *>(&s_part[0][warp][lane * 4]) = pm;
+        __syncthreads();
+        float4 t[8];
+#pragma unroll
+        for (int w = 0; w < 8; w++) t[w] = *reinterpret_cast<const float4 *>(&s_part[0][w][vq * 4]);
+#pragma unroll
+        for (int n = 1; n < 8; n <<= 1) // pairs of warps, then of pairs
+#pragma unroll
+            for (int w = 0; w < 8; w += 2 * n) { t[w].x += t[w + n].x; t[w].y += t[w + n].y; t[w].z += t[w + n].z; t[w].w += t[w + n].w; }
+        const float4 mem = t[0];
+        const float4 dl = make_float4(fmaf(-mem.x, decay, v4.x) * beta, fmaf(-mem.y, decay, v4.y) * beta, fmaf(-mem.z, decay, v4.z) * beta,
+                                      fmaf(-mem.w, decay, v4.w) * beta);
+
+        // S = S*d + k*delta ; out_v = sum_i S * q
+        float4 po = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            cell[j].x = fmaf(kk[j], dl.x, cell[j].x * decay);
+            cell[j].y = fmaf(kk[j], dl.y, cell[j].y * decay);
+            cell[j].z = fmaf(kk[j], dl.z, cell[j].z * decay);
+            cell[j].w = fmaf(kk[j], dl.w, cell[j].w * decay);
+            po.x = fmaf(cell[j].x, qq[j], po.x);
+            po.y = fmaf(cell[j].y, qq[j], po.y);
+            po.z = fmaf(cell[j].z, qq[j], po.z);
+            po.w = fmaf(cell[j].w, qq[j], po.w);
+            // the state after the last step goes to state_last (default: in place); a speculative verify pass also keeps the
+            // state after its first step (state_first), which is the one to continue from when the second token is rejected
+            if (step == tokens - 1) *reinterpret_cast<float4 *>((state_last ? state_last + size_t(head) * 128 * 128 : S) + size_t(kr + 32 * j) * 128 + v0) = cell[j];
+            else if (step == 0 && state_first) *reinterpret_cast<float4 *>(state_first + size_t(head) * 128 * 128 + size_t(kr + 32 * j) * 128 + v0) = cell[j];
+        }
+#pragma unroll
+        for (int m = 16; m >= 8; m >>= 1) {
+            po.x += __shfl_xor_sync(0xffffffffu, po.x, m);
+            po.y += __shfl_xor_sync(0xffffffffu, po.y, m);
+            po.z += __shfl_xor_sync(0xffffffffu, po.z, m);
+            po.w += __shfl_xor_sync(0xffffffffu, po.w, m);
+        }
+        if (lane < 8) *reinterpret_cast<float4 *>(&s_part[1][warp][lane * 4]) = po;
+        __syncthreads();
+        if (tid < 32) {
+            float o[8];
+#pragma unroll
+            for (int w = 0; w < 8; w++) o[w] = s_part[1][w][tid];
+            out32[head * 128 + slice * 32 + tid] = ((o[0] + o[1]) + (o[2] + o[3])) + ((o[4] + o[5]) + (o[6] + o[7]));
+        }
+    }
+}
+
+// ---- the same arithmetic inside a warp, for many steps ------------------------------------------------------------------------
 // A warp owns eight columns: lane = (k part kq = lane & 7) x (column pair lane >> 3), 16 rows (32 j + 4 kq + 0..3) of two columns
 // per lane.  Rows go in pairs through the packed fp32 instructions of sm_100 (two lanes of arithmetic per issue), so that a
 // step of a warp is 16 packed multiply-adds three times over; a sum over k is three shuffles, and nothing crosses a warp.
+// (Four columns and eight warps: 107 us for 512 steps against 97.)
 struct DnCells {
     unsigned long long c[2][8]; // [column of the pair][row pair 2 j + h]
 };
@@ -133,69 +269,7 @@ __device__ __forceinline__ void dn_update(DnCells &s, const unsigned long long (
     }
 }
 
-// `tokens` consecutive steps of the sequence in one launch: the slice stays in registers from step to step and is
-// written back once; q/k/v of step m are at + m * qkv_stride, g/beta at + m * 32, the output at + m * 4096.
-// Every warp reads the whole q and k of its key head (four values per lane) and normalises them itself: no CTA barrier.
-__global__ void __launch_bounds__(kDnThreads) deltanet_step_kernel(float *__restrict__ state, const float *__restrict__ q16,
-                                                                   const float *__restrict__ k16, const float *__restrict__ v32,
-                                                                   const float *__restrict__ g32, const float *__restrict__ beta32,
-                                                                   float *__restrict__ out32, int tokens, int qkv_stride, long long state_stride,
-                                                                   float *__restrict__ state_first, float *__restrict__ state_last)
-{
-    __shared__ __align__(16) float s_qk[4][2][128];
-    const int head = blockIdx.x / kSlices, slice = blockIdx.x % kSlices, kh = head >> 1;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int col = slice * 32 + warp * 8, mine = col + (lane >> 3) * 2 + (lane & 1); // the warp's first column, the lane's own
-
-    pdl_launch_dependents();
-
-    // blockIdx.y: independent sequence of a decode batch (its own state, its own inputs and outputs)
-    const int seq = blockIdx.y;
-    q16 += size_t(seq) * qkv_stride + kh * 128; k16 += size_t(seq) * qkv_stride + kh * 128; v32 += size_t(seq) * qkv_stride + head * 128 + mine;
-    g32 += seq * 32 + head; beta32 += seq * 32 + head; out32 += size_t(seq) * 4096 + head * 128 + mine;
-    const size_t at = size_t(head) * 128 * 128 + col;
-    float *S = state + size_t(seq) * state_stride;
-    DnCells cells;
-    dn_load(cells, S + at, lane);
-
-    pdl_wait();
-
-    // Every dependent input of a step is requested at once; with several steps the next step's inputs are requested
-    // before this step's arithmetic (they do not depend on it), so only the first step waits for a load.
-    float4 nq = __ldcg(reinterpret_cast<const float4 *>(q16) + lane), nk = __ldcg(reinterpret_cast<const float4 *>(k16) + lane);
-    float nv = __ldcg(v32), ng = __ldcg(g32), nb = __ldcg(beta32);
-    for (int step = 0; step < tokens; step++) {
-        const float4 q4 = nq, k4 = nk;
-        const float v = nv, g = ng, beta = nb;
-        if (step + 1 < tokens) {
-            const size_t o = size_t(step + 1) * qkv_stride;
-            nq = __ldcg(reinterpret_cast<const float4 *>(q16 + o) + lane);
-            nk = __ldcg(reinterpret_cast<const float4 *>(k16 + o) + lane);
-            nv = __ldcg(v32 + o);
-            ng = __ldcg(g32 + size_t(step + 1) * 32);
-            nb = __ldcg(beta32 + size_t(step + 1) * 32);
-        }
-        const float qn = warp_sum(fmaf(q4.x, q4.x, fmaf(q4.y, q4.y, fmaf(q4.z, q4.z, q4.w * q4.w))));
-        const float kn = warp_sum(fmaf(k4.x, k4.x, fmaf(k4.y, k4.y, fmaf(k4.z, k4.z, k4.w * k4.w))));
-        const float qs = rsqrtf(qn + 1e-6f) * 0.08838834764831845f, ks = rsqrtf(kn + 1e-6f);
-        __syncwarp(); // the previous step's reads of this warp's copy are done
-        reinterpret_cast<float4 *>(s_qk[warp][0])[lane] = make_float4(q4.x * qs, q4.y * qs, q4.z * qs, q4.w * qs);
-        reinterpret_cast<float4 *>(s_qk[warp][1])[lane] = make_float4(k4.x * ks, k4.y * ks, k4.z * ks, k4.w * ks);
-        __syncwarp();
-        unsigned long long q[8], k[8];
-        dn_vector(q, s_qk[warp][0], lane);
-        dn_vector(k, s_qk[warp][1], lane);
-        dn_update(cells, k, dn_fold(dn_products(cells, k), lane), v, expf(g), beta, lane);
-        const float o = dn_fold(dn_products(cells, q), lane);
-        if ((lane & 7) < 2) out32[size_t(step) * 4096] = o;
-        // the state after the last step goes to state_last (default: in place); a speculative verify pass also keeps the
-        // state after its first step (state_first), which is the one to continue from when the second token is rejected
-        if (step == tokens - 1) dn_store(cells, (state_last ? state_last : S) + at, lane);
-        else if (step == 0 && state_first) dn_store(cells, state_first + at, lane);
-    }
-}
-
-// The recurrence over many consecutive steps (a prompt pass): the state stays in the registers of four warps, which find
+// The recurrence over many consecutive steps (a prompt pass), bit-identical to single steps: the state stays in the registers of four warps, which find
 // everything that does not depend on it in shared memory: four more warps normalise q and k and fetch v, beta and exp(g) for
 // the next kDnBlock steps meanwhile.  A step is a latency chain (products, three shuffles, update) of some 200 cycles with no
 // barrier in it; the fold of step t's output runs beside step t + 1's.  (With the k sum cut over eight warps and a CTA barrier
@@ -205,7 +279,7 @@ struct DnInputs {
     float q[kDnBlock][128], k[kDnBlock][128], v[kDnBlock][32], decay[kDnBlock], beta[kDnBlock];
 };
 
-__global__ void __launch_bounds__(2 * kDnThreads, 1) deltanet_steps_kernel(float *__restrict__ state, const float *__restrict__ q16,
+__global__ void __launch_bounds__(kDnThreads, 1) deltanet_steps_kernel(float *__restrict__ state, const float *__restrict__ q16,
                                                                            const float *__restrict__ k16, const float *__restrict__ v32,
                                                                            const float *__restrict__ g32, const float *__restrict__ beta32,
                                                                            float *__restrict__ out32, int tokens, int qkv_stride)
@@ -297,14 +371,13 @@ __global__ void __launch_bounds__(2 * kDnThreads, 1) deltanet_steps_kernel(float
 // slices exchanging their sums through a cluster took 16 us at eight sequences, this form 6; the out projection's own
 // conversion, done again by each of its clusters, 6 us more than taking the image).  A warp holds 16 rows of the state, a lane four columns: the
 // sums over k need no shuffles, only one pass over the eight warps' partials.
-constexpr int kHeadThreads = 256;
 struct DnGate {
     const float *z;          // [sequences][4096]
     const uint16_t *norm_w;  // bf16 [128]
     uint8_t *image;
     int slots;
 };
-__global__ void __launch_bounds__(kHeadThreads, 2) deltanet_heads_kernel(float *__restrict__ state, long long state_stride, const float *__restrict__ q16,
+__global__ void __launch_bounds__(kDnThreads, 2) deltanet_heads_kernel(float *__restrict__ state, long long state_stride, const float *__restrict__ q16,
                                                                        const float *__restrict__ k16, const float *__restrict__ v32,
                                                                        const float *__restrict__ g32, const float *__restrict__ beta32,
                                                                        float *__restrict__ out32, int qkv_stride, const DnGate gate)
@@ -407,7 +480,7 @@ extern "C" int insg_deltanet_decode_tokens(float *state, const float *q16, const
     if (tokens == 1)
         return launch(deltanet_step_kernel, dim3(32 * kSlices), dim3(kDnThreads), 0, stream, pdl != 0, state, q16, k16, v32, g32, beta32,
                       out32, 1, qkv_stride, 0ll, nullptr, nullptr);
-    return launch(deltanet_steps_kernel, dim3(32 * kSlices), dim3(2 * kDnThreads), 0, stream, pdl != 0, state, q16, k16, v32, g32, beta32,
+    return launch(deltanet_steps_kernel, dim3(32 * kSlices), dim3(kDnThreads), 0, stream, pdl != 0, state, q16, k16, v32, g32, beta32,
                   out32, tokens, qkv_stride);
 }
 
@@ -437,6 +510,6 @@ extern "C" int insg_deltanet_decode_gated(float *state, long long state_stride, 
 {
     if (!state || !q16 || !k16 || !v32 || !g32 || !beta32 || !out32 || !z || !norm_w || !image) return fail(INSG_E_ARG, "deltanet: null pointer");
     if (sequences < 1 || sequences > 8 || qkv_stride < 0 || state_stride < 32 * 128 * 128) return fail(INSG_E_SHAPE, "deltanet: 1..8 sequences");
-    return launch(deltanet_heads_kernel, dim3(32, sequences), dim3(kHeadThreads), 0, stream, pdl != 0, state, state_stride, q16, k16, v32, g32, beta32,
+    return launch(deltanet_heads_kernel, dim3(32, sequences), dim3(kDnThreads), 0, stream, pdl != 0, state, state_stride, q16, k16, v32, g32, beta32,
                   out32, qkv_stride, DnGate{z, norm_w, static_cast<uint8_t *>(image), image_slots(sequences)});
 }
