@@ -174,19 +174,25 @@ constexpr int kMaxClusters = 8; // per kv head
 struct AttnCut {
     int active, chunk; // clusters at work, rows per CTA
 };
-template <int CL> __device__ __forceinline__ AttnCut attn_cut(int rows, int clusters)
+// HALVES: two clusters of four in place of one of eight, with the same bits: when both have rows, the last to arrive folds the
+// eight CTAs' results as the cluster of eight does.
+template <int CL, bool HALVES> __device__ __forceinline__ AttnCut attn_cut(int rows, int clusters)
 {
+    constexpr int kUnit = HALVES ? 2 * CL : CL; // CTAs
     AttnCut c;
-    c.active = min(clusters, (rows + kCtaRows * CL - 1) / (kCtaRows * CL));
-    const int ctas = c.active * CL;
+    c.active = min(HALVES ? clusters / 2 : clusters, (rows + kCtaRows * kUnit - 1) / (kCtaRows * kUnit));
+    const int ctas = c.active * kUnit;
     c.chunk = max(kMinChunk, (rows + ctas - 1) / ctas);
+    if (HALVES) c.active = (rows + c.chunk * CL - 1) / (c.chunk * CL); // a half without rows has nothing to do
     return c;
 }
 
-template <bool BF16, bool FUSED, int CL>
+template <bool BF16, bool FUSED, int CL, bool HALVES>
 __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid_constant__ AttnParams p, int clusters)
 {
     using Row = KvRow<BF16>;
+    constexpr bool kMma = BF16 && CL == 4 && !HALVES; // the bf16 launches of long contexts
+    constexpr int kParts = HALVES ? CL : 1; // partial results of a cluster in scratch
     constexpr int kMine = 1024 / CL; // output dims this CTA finishes
     __shared__ __align__(16) float s_q[4][256];
     __shared__ __align__(16) float s_knew[256], s_vnew[256];
@@ -226,12 +232,12 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
         tokens = __ldcg(p.position) + p.position_offset + bt + 1;
     }
     tokens = max(1, min(tokens, p.max_context)); // host checks; never index past the cache
-    AttnCut cut = attn_cut<CL>(tokens, clusters);
+    AttnCut cut = attn_cut<CL, HALVES>(tokens, clusters);
     int t0 = split * cut.chunk, t1 = min(tokens, t0 + cut.chunk);
     int fresh = tokens - 1; // the row the producer (or this kernel) is still writing
 
     if (p.image && tid < 81) s_lut[tid] = digit_pair_code(tid); // read behind the barriers below
-    bool use_mma = BF16 && tokens >= kMmaMinTokens; // long bf16 contexts: the tensor-core loop (reads every row from the cache)
+    bool use_mma = kMma && tokens >= kMmaMinTokens; // long bf16 contexts: the tensor-core loop (reads every row from the cache)
     if (tid == 0) s_abort = 0;
     // This warp's next token group: its keys are replaced by the following group's as soon as they are scored, its values as soon
     // as they are added.  One group (two would take a CTA's registers past what fits beside the products' launches, and the
@@ -254,11 +260,11 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
         if (now != pos) {
             pos = now;
             tokens = max(1, min(pos + 1, p.max_context));
-            cut = attn_cut<CL>(tokens, clusters);
+            cut = attn_cut<CL, HALVES>(tokens, clusters);
             t0 = split * cut.chunk;
             t1 = min(tokens, t0 + cut.chunk);
             fresh = tokens - 1;
-            use_mma = BF16 && tokens >= kMmaMinTokens;
+            use_mma = kMma && tokens >= kMmaMinTokens;
             if (!use_mma) load_group<BF16, kGroup>(kc, vc, kvh, t0 + warp * kGroup, min(t1, fresh), lane, ga);
             if (warp < 5 && lane < 8) rope_table(pos, lane, p.fast_trig != 0, rope_c, rope_s);
         }
@@ -312,7 +318,7 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
     __syncthreads();
 
     bool mma_done = false;
-    if constexpr (BF16) {
+    if constexpr (kMma) {
         if (has_work && use_mma) {
             attn_mma_warp(kc, vc, kvh, t0, t1, warp, lane, s_q, s_tiles, &s_bar[2 * warp], &s_abort, s_m[warp], s_l[warp], s_acc[warp]);
             mma_done = true;
@@ -445,11 +451,14 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
         if (tid < kMine) a = fmaf(s_in[c][tid], e, a);
     }
     if (cut.active > 1) { // several clusters: partial results to scratch, the last one folds them in order
-        float *part = partials + size_t(kvh * kSplits + cluster) * kPartFloats;
-        if (tid < kMine) part[8 + rank * kMine + tid] = a;
-        if (tid == 0) { // CTAs that share a head write the same values
-            part[my_head & 3] = mg;
-            part[4 + (my_head & 3)] = lg;
+        float *part = partials + size_t(kvh * kSplits + cluster * kParts) * kPartFloats;
+#pragma unroll
+        for (int c = 0; c < kParts; c++, part += kPartFloats) {
+            if (tid < kMine) part[8 + rank * kMine + tid] = HALVES ? s_in[c][tid] : a;
+            if (tid == 0) { // CTAs that share a head write the same values
+                part[my_head & 3] = HALVES ? s_min[c] : mg;
+                part[4 + (my_head & 3)] = HALVES ? s_lin[c] : lg;
+            }
         }
         __threadfence();
         __syncthreads();
@@ -465,18 +474,19 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
         }
         __threadfence();
         const float *pp = partials + size_t(kvh * kSplits) * kPartFloats;
+        const int nparts = cut.active * kParts;
         float ms[kMaxClusters];
         mg = -3.0e38f;
 #pragma unroll
         for (int c = 0; c < kMaxClusters; c++) {
-            ms[c] = c < cut.active ? __ldcg(pp + size_t(c) * kPartFloats + (my_head & 3)) : -3.0e38f;
+            ms[c] = c < nparts ? __ldcg(pp + size_t(c) * kPartFloats + (my_head & 3)) : -3.0e38f;
             mg = fmaxf(mg, ms[c]);
         }
         lg = 0.f;
         a = 0.f;
 #pragma unroll
         for (int c = 0; c < kMaxClusters; c++)
-            if (c < cut.active) {
+            if (c < nparts) {
                 const float e = __expf(ms[c] - mg);
                 lg = fmaf(__ldcg(pp + size_t(c) * kPartFloats + 4 + (my_head & 3)), e, lg);
                 if (tid < kMine) a = fmaf(__ldcg(pp + size_t(c) * kPartFloats + 8 + rank * kMine + tid), e, a);
@@ -491,10 +501,10 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
     if (tid == 0 && s_abort && p.error_flag) *p.error_flag = 1;
 }
 
-template <bool BF16, bool FUSED, int CL> static int launch_clusters(const AttnParams &p, cudaStream_t st, bool pdl, int along, int rows, int clusters)
+template <bool BF16, bool FUSED, int CL, bool HALVES = false> static int launch_clusters(const AttnParams &p, cudaStream_t st, bool pdl, int along, int rows, int clusters)
 {
     size_t smem = 0;
-    if (BF16) { // the tensor-core loop's tiles: more than 48 KB of dynamic shared memory is a per-device opt-in
+    if constexpr (BF16 && CL == 4 && !HALVES) { // the tensor-core loop's tiles: more than 48 KB of dynamic shared memory is a per-device opt-in
         static std::mutex mu;
         static bool done[64] = {false};
         int dev = 0;
@@ -503,14 +513,14 @@ template <bool BF16, bool FUSED, int CL> static int launch_clusters(const AttnPa
         if (dev < 0 || dev >= 64) return fail(INSG_E_LIMIT, "attention: device ordinal beyond 63");
         std::lock_guard<std::mutex> lock(mu);
         if (!done[dev]) {
-            e = cudaFuncSetAttribute(attn_splitk_kernel<BF16, FUSED, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMmaSmem));
+            e = cudaFuncSetAttribute(attn_splitk_kernel<BF16, FUSED, CL, HALVES>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMmaSmem));
             if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(attention)");
             done[dev] = true;
         }
         if (p.max_context >= kMmaMinTokens) smem = kMmaSmem; // else no launch of these operands gets to the tensor-core loop
     }
     const int most = rows > 0 ? std::min(rows, p.max_context) : p.max_context;
-    clusters = std::max(1, std::min({clusters, kMaxClusters, (most + kCtaRows * CL - 1) / (kCtaRows * CL)}));
+    if (!HALVES) clusters = std::max(1, std::min({clusters, kMaxClusters, (most + kCtaRows * CL - 1) / (kCtaRows * CL)}));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(4 * clusters * CL, along);
     cfg.blockDim = dim3(kAtThreads);
@@ -524,21 +534,30 @@ template <bool BF16, bool FUSED, int CL> static int launch_clusters(const AttnPa
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 2 : 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, attn_splitk_kernel<BF16, FUSED, CL>, p, clusters);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, attn_splitk_kernel<BF16, FUSED, CL, HALVES>, p, clusters);
     return e == cudaSuccess ? INSG_OK : cuda_fail(e, "attention launch");
 }
 
 // `along`: tokens of a chunk or sequences of a batch (grid rows); rows: an upper bound of the rows attended, when known.  As many
-// clusters as the device runs at once: 33 of eight CTAs at two per SM (fp32 cache), 71 of four CTAs at two per SM (bf16 cache)
-// or 33 at one (with the tensor-core loop's tiles), shared by the four heads of every grid row.  Where that leaves SMs idle (three
-// sequences or more, not a power of two) and the contexts can be long, the fp32 cache goes to clusters of four too.
+// clusters as the device runs at once: 33 of eight CTAs at two per SM, or 33 of four at one (with the tensor-core loop's tiles),
+// shared by the four heads of every grid row.  Where that leaves SMs idle (three sequences or more, not a power of two) and the
+// contexts can be long, the fp32 cache goes to clusters of four too.  Where contexts are short and the
+// CTAs more than one and a half per SM (seven sequences or more), a second CTA finds no registers beside the products' launches
+// before and after: clusters of four find a place sooner than those of eight, and up to 128 rows one of the two has nothing to
+// do.  A step of eight sequences 1803 -> 1755 us at 20 rows and 1885 -> 1818 at 450 (alone the launch is 1.5 us slower there);
+// five sequences win at 20 rows and lose 12 us from 130 on.
 constexpr int kLongContext = 2048;
+static_assert(kLongContext <= kMmaMinTokens, "short contexts never get to the tensor-core loop");
 template <bool BF16, bool FUSED> int launch_attn(const AttnParams &p, cudaStream_t st, bool pdl, int along = 1, int rows = 0)
 {
+    if (p.max_context < kLongContext) {
+        if (along > kMaxClusters / 2 && 2 * along * 4 * 8 > 3 * sm_count()) return launch_clusters<BF16, FUSED, 4, true>(p, st, pdl, along, rows, 2);
+        return launch_clusters<BF16, FUSED, 8>(p, st, pdl, along, rows, kMaxClusters / along);
+    }
     if constexpr (BF16) {
-        return launch_clusters<true, FUSED, 4>(p, st, pdl, along, rows, (p.max_context >= kMmaMinTokens ? kMaxClusters : 17) / along);
+        return launch_clusters<true, FUSED, 4>(p, st, pdl, along, rows, kMaxClusters / along);
     } else {
-        if (along > 2 && (along & (along - 1)) && p.max_context >= kLongContext) return launch_clusters<false, FUSED, 4>(p, st, pdl, along, rows, 17 / along);
+        if (along > 2 && (along & (along - 1))) return launch_clusters<false, FUSED, 4>(p, st, pdl, along, rows, 17 / along);
         return launch_clusters<false, FUSED, 8>(p, st, pdl, along, rows, kMaxClusters / along);
     }
 }
