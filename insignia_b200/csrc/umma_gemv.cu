@@ -43,7 +43,8 @@ constexpr int kDMaxKb = 24;                // k-blocks per CTA: 12288 / 128 / 4
 constexpr int kDDigits = 8;                // digits per activation = N columns per token
 constexpr uint32_t kDSfaCol = 128, kDSfbCol = 160, kDTmemCols = 256; // accumulators [0,128), weight scales [128,160), digit scales [160,256)
 // A CTA takes at most this much dynamic shared memory unless its operands need more: two of them (this launch and the next)
-// then fit an SM's 228 KB with their static part and the 1 KB the hardware keeps per CTA.
+// then fit an SM's 228 KB with their static part (at most 1 KB, which is why eight tokens' sums of squares are not in it) and
+// the 1 KB the hardware keeps per CTA.
 constexpr int kDHalfSm = 112 * 1024;
 
 struct DSeg {
@@ -83,9 +84,13 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t saddr, uint32_t rank)
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+// The arrivals below order no global store: a release at cluster scope waits until the epilogue's earlier stores have been
+// acknowledged, which a stream of weights makes slow (one token 1214 -> 1189 us, lm_head with four tokens 145 -> 87 us).  Slots are
+// handed back after they have been read, and the closing barrier only keeps CTAs from leaving early.
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
 __device__ __forceinline__ void remote_arrive(uint32_t bar)
 {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+    asm volatile("mbarrier.arrive.release.cta.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // T floats to another CTA's shared memory; their bytes complete on that CTA's barrier.
 template <int T> __device__ __forceinline__ void send_floats(uint32_t dst, const float (&v)[T], uint32_t bar)
@@ -169,7 +174,9 @@ template <int T> __device__ __forceinline__ void load_partial(uint32_t taddr, fl
     }
 }
 
-template <int T> constexpr int kUnitSlots = T == 1 ? 4 : 2; // units whose exchange slots exist at once
+// Units whose exchange slots exist at once.  Eight tokens: two matrices leave room for one unit's if the launch is to stay within
+// half an SM (24576 x 4096 as SwiGLU 14.3 -> 13.3 us in the chain); one matrix keeps two (one: 9.7 -> 10.7 us at 12352 x 4096).
+template <int T> __host__ __device__ constexpr int unit_slots(int nmat) { return T == 1 ? 4 : T == 8 ? 3 - nmat : 2; }
 
 template <int T>
 __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_constant__ DParams p)
@@ -180,17 +187,17 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     constexpr int N = kDDigits * T;
     constexpr int kSlot = kDCl * 32 * T; // floats of one exchange slot: [source rank][32 rows][T]
     // The four owner warps: with several tokens they split the tokens of a unit among them (TN each), else they take units in turn.
-    constexpr int TW = T < 4 ? T : 4, TN = T / TW, kGroups = 4 / TW, XU = kUnitSlots<T>;
+    constexpr int TW = T < 4 ? T : 4, TN = T / TW, kGroups = 4 / TW;
     __shared__ __align__(8) uint64_t full[kDMaxStages], empty[kDMaxStages], dfull[2], dempty[2], xfull[8], xempty[8], ssfull, image[kDMaxKb / 8];
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort, s_last;
-    __shared__ float s_ssq[T * kDMaxKb], s_rss[kDCl * T], s_scale[T], s_best[4];
+    __shared__ float s_ssq_static[T < 8 ? T * kDMaxKb : 1], s_rss[kDCl * T], s_scale[T], s_best[4];
     __shared__ int s_bidx[4];
     __shared__ uint8_t s_lut[84];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int rank = int(blockIdx.x) & (kDCl - 1), cl = int(blockIdx.x) / kDCl, C = int(gridDim.x) / kDCl;
-    const int nkb = p.nkb, S = p.stages, nmat = p.nmat;
+    const int nkb = p.nkb, S = p.stages, nmat = p.nmat, XU = unit_slots<T>(nmat);
     const int kb0 = (nkb * rank) >> 2, len = ((nkb * (rank + 1)) >> 2) - kb0; // this CTA's k-blocks
     const int spt = (len + 1) >> 1;                                            // ring stages per (tile, matrix)
     const int nun = cl < p.units ? (p.units - cl + C - 1) / C : 0;             // units of this cluster: cl, cl + C, ...
@@ -199,6 +206,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     uint8_t *bimg = ring + size_t(S) * kDStage; // len x kImg bytes
     float *xslot = reinterpret_cast<float *>(bimg + size_t((nkb + 3) >> 2) * kImg); // XU * nmat exchange slots
     const bool prepared = p.prologue == INSG_PRO_PREPARED;
+    float *s_ssq = T < 8 ? s_ssq_static : xslot + XU * nmat * kSlot; // [token][k-block], unless the input is prepared
 
     // ---- the weight stream starts first: it depends on nothing ----------------------------------------------------------
     auto run_src = [&](int run) -> const uint8_t * { // this CTA's records of the run (tile, matrix)
@@ -490,6 +498,36 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             for (int m = 0; m < p.tokens; m++)
                 for (int k = kb0 * 128 + fw * 32 + lane; k < (kb0 + len) * 128; k += 128)
                     p.x_out[size_t(m) * p.cols + k] = __ldcg(p.in + size_t(m) * p.cols + k) * s_scale[m] * bf16_bits_to_float(p.norm_w[k]);
+        // What the epilogue of a unit needs besides the sums: asked for before the wait for them; where one warp has two tokens of
+        // every unit, a unit ahead (eight sequences, in-projection: 10.5 -> 9.7 us; with fewer tokens it costs 0.2 us).
+        constexpr bool kAhead = TN > 1;
+        struct Fetched {
+            float h[TN][3]; // per token: the residual, or the convolution's history; decay: bias and rate
+            uint2 w;        // the convolution's weights
+        } next;
+        auto fetch = [&](int i) {
+            const int unit = cl + i * C;
+            const DSeg &s = p.seg[dseg_of(p, unit)];
+            const int row = (unit - s.tile_begin) * 128 + rank * 32 + lane;
+            if (row >= s.rows) return;
+            if (s.epilogue == INSG_EPI_CONV_SILU) next.w = reinterpret_cast<const uint2 *>(s.conv_w)[row];
+#pragma unroll
+            for (int u = 0; u < TN; u++) {
+                const int t = t0 + u;
+                if (t >= p.tokens) break;
+                if (s.epilogue == INSG_EPI_RESIDUAL) {
+                    next.h[u][0] = __ldcg(s.out + row + t * size_t(s.rows));
+                } else if (s.epilogue == INSG_EPI_CONV_SILU) {
+                    const float *hist = s.conv_state + t * s.conv_stride + size_t(row) * 3;
+#pragma unroll
+                    for (int j = 0; j < 3; j++) next.h[u][j] = __ldcg(hist + j);
+                } else if (s.epilogue == INSG_EPI_DECAY && u == 0) {
+                    next.h[0][0] = bf16_bits_to_float(s.dt_bias[row]);
+                    next.h[0][1] = -__expf(s.A_log[row]);
+                }
+            }
+        };
+        if (kAhead && ok && group < nun) fetch(group);
         for (int i = group; i < nun && ok; i += kGroups) {
             const int unit = cl + i * C;
             const DSeg &s = p.seg[dseg_of(p, unit)];
@@ -497,29 +535,13 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             const bool on = row < s.rows;
             const size_t ld = size_t(s.rows);
             float *out = s.out + row;
-            // the epilogue's other operands are fetched before the wait for the sums
-            float pre[TN], h0 = 0.f, h1 = 0.f, h2 = 0.f;
-            float cw0 = 0.f, cw1 = 0.f, cw2 = 0.f, cw3 = 0.f;
+            if (!kAhead) fetch(i);
+            const Fetched f = next;
+            if (kAhead && i + kGroups < nun) fetch(i + kGroups);
             const float pw = s.prep_w ? bf16_bits_to_float(s.prep_w[row]) : 1.f; // rows % 128 == 0 where it is set
-#pragma unroll
-            for (int u = 0; u < TN; u++) pre[u] = 0.f;
+            const float cw0 = bf16_bits_to_float(f.w.x & 0xffff), cw1 = bf16_bits_to_float(f.w.x >> 16);
+            const float cw2 = bf16_bits_to_float(f.w.y & 0xffff), cw3 = bf16_bits_to_float(f.w.y >> 16);
             const bool one_history = s.conv_stride == 0; // consecutive tokens of one sequence
-            if (on && s.epilogue == INSG_EPI_RESIDUAL) {
-#pragma unroll
-                for (int u = 0; u < TN; u++)
-                    if (t0 + u < p.tokens) pre[u] = __ldcg(out + (t0 + u) * ld);
-            } else if (on && s.epilogue == INSG_EPI_CONV_SILU) {
-                const uint2 wv = reinterpret_cast<const uint2 *>(s.conv_w)[row];
-                cw0 = bf16_bits_to_float(wv.x & 0xffff); cw1 = bf16_bits_to_float(wv.x >> 16);
-                cw2 = bf16_bits_to_float(wv.y & 0xffff); cw3 = bf16_bits_to_float(wv.y >> 16);
-                if (t0 < p.tokens) {
-                    const float *hist = s.conv_state + t0 * s.conv_stride + size_t(row) * 3;
-                    h0 = __ldcg(hist); h1 = __ldcg(hist + 1); h2 = __ldcg(hist + 2);
-                }
-            } else if (on && s.epilogue == INSG_EPI_DECAY) {
-                h0 = bf16_bits_to_float(s.dt_bias[row]);
-                h1 = -__expf(s.A_log[row]);
-            }
             float y[2][TN];
 #pragma unroll
             for (int mat = 0; mat < 2; mat++) {
@@ -539,6 +561,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 for (int u = 0; u < TN; u++) y[mat][u] = sum(t0 + u);
                 if (T > 1 && one_history && s.epilogue == INSG_EPI_CONV_SILU) { // the history runs through the tokens: one warp takes them in order
                     if (t0 == 0 && on) {
+                        float h0 = f.h[0][0], h1 = f.h[0][1], h2 = f.h[0][2];
                         for (int t = 0; t < p.tokens; t++) {
                             const float raw = sum(t);
                             out[t * ld] = fast_silu(fmaf(h0, cw0, fmaf(h1, cw1, fmaf(h2, cw2, raw * cw3))));
@@ -555,7 +578,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             }
             if (!ok) break;
             if (i + kGroups >= nun) { // nothing more comes in for this warp: the peers need not wait for its epilogue
-                cluster_arrive();
+                cluster_arrive_relaxed();
                 arrived = true;
             }
             if (!on) continue;
@@ -569,7 +592,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
 #pragma unroll
                 for (int u = 0; u < TN; u++)
                     if (t0 + u < p.tokens) {
-                        const float v = pre[u] + y[0][u];
+                        const float v = f.h[u][0] + y[0][u];
                         out[(t0 + u) * ld] = v;
                         if (s.prep) leave_digits<T>(s, v, pw, row, t0 + u, s_lut, lane);
                     }
@@ -581,10 +604,9 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                     const int t = t0 + u;
                     if (t < p.tokens) {
                         float *hist = s.conv_state + t * s.conv_stride + size_t(row) * 3; // independent sequences: each token has its own
-                        if (u > 0) { h0 = __ldcg(hist); h1 = __ldcg(hist + 1); h2 = __ldcg(hist + 2); }
-                        const float z = fmaf(h0, cw0, fmaf(h1, cw1, fmaf(h2, cw2, y[0][u] * cw3)));
+                        const float z = fmaf(f.h[u][0], cw0, fmaf(f.h[u][1], cw1, fmaf(f.h[u][2], cw2, y[0][u] * cw3)));
                         out[t * ld] = fast_silu(z);
-                        hist[0] = h1; hist[1] = h2; hist[2] = y[0][u];
+                        hist[0] = f.h[u][1]; hist[1] = f.h[u][2]; hist[2] = y[0][u];
                     }
                 }
                 break;
@@ -597,8 +619,8 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             case INSG_EPI_DECAY:
 #pragma unroll
                 for (int u = 0; u < TN; u++) {
-                    const float z = y[0][u] + h0;
-                    if (t0 + u < p.tokens) out[(t0 + u) * ld] = h1 * (z > 20.f ? z : log1pf(__expf(z)));
+                    const float z = y[0][u] + f.h[0][0];
+                    if (t0 + u < p.tokens) out[(t0 + u) * ld] = f.h[0][1] * (z > 20.f ? z : log1pf(__expf(z)));
                 }
                 break;
             case INSG_EPI_SWIGLU:
@@ -671,7 +693,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     // Nobody leaves while a peer may still write into its shared memory (after an expired wait too).
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    if (!arrived) cluster_arrive();
+    if (!arrived) cluster_arrive_relaxed();
     cluster_wait();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     __syncwarp();
@@ -809,11 +831,15 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     const int clusters = std::min(p.units, max_clusters);
     const int T = tokens == 1 ? 1 : tokens == 2 ? 2 : tokens <= 4 ? 4 : 8;
     const int kbq = (p.nkb + 3) >> 2;
-    const size_t fixed = size_t(kbq) * (512 * T + 512) + size_t(T == 1 ? 4 : 2) * p.nmat * kDCl * 32 * T * sizeof(float);
-    // ring: no more stages than the launch has, within half an SM when that leaves at least four, else whatever fits
+    const int slots = (T == 1 ? unit_slots<1>(p.nmat) : T == 8 ? unit_slots<8>(p.nmat) : unit_slots<2>(p.nmat)) * p.nmat;
+    const size_t fixed = size_t(kbq) * (512 * T + 512) + size_t(slots) * kDCl * 32 * T * sizeof(float) +
+                         (T == 8 && op->prologue != INSG_PRO_PREPARED ? size_t(8) * kDMaxKb * sizeof(float) : 0);
+    // ring: no more stages than the launch has, within half an SM when that leaves at least four, else whatever fits.  Four are too
+    // few to stream at full rate, so a launch of many units (the head: 55 per cluster, eight tokens 97 us against 91) takes the
+    // whole SM; one of a few gains more from starting beside its predecessor.
     const int need = ((p.units + clusters - 1) / clusters) * p.nmat * ((kbq + 1) / 2);
     int stages = fixed < size_t(kDHalfSm) ? int((kDHalfSm - fixed) / kDStage) : 0;
-    if (stages < 4) stages = int((size_t(222) * 1024 - fixed) / kDStage);
+    if (stages < 4 || (stages == 4 && need > 96)) stages = int((size_t(222) * 1024 - fixed) / kDStage);
     p.stages = std::max(1, std::min({stages, need, kDMaxStages}));
     const size_t smem = fixed + size_t(p.stages) * kDStage;
 
