@@ -297,8 +297,8 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
                 const size_t row = (size_t(pos) * 4 + kvh) * 256 + lane * 8;
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
-                    Row::store(kc, row + j, v[j]);
                     s_knew[lane * 8 + j] = Row::round(v[j]);
+                    if (use_mma) Row::store(kc, row + j, v[j]);
                 }
                 if (use_mma) asm volatile("fence.proxy.async;" ::: "memory"); // the tensor-core loop fetches this row by bulk copy
             } else if (warp == 5 && pos >= t0 && pos < t1) {
@@ -306,8 +306,8 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
                     const float v = __ldcg(v_new + kvh * 256 + lane * 8 + j);
-                    Row::store(vc, row + j, v);
                     s_vnew[lane * 8 + j] = Row::round(v);
+                    if (use_mma) Row::store(vc, row + j, v);
                 }
                 if (use_mma) asm volatile("fence.proxy.async;" ::: "memory");
             }
@@ -440,6 +440,13 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
         }
     }
     asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+    // the new row goes to the cache now: ahead of the barrier its release would wait for these stores
+    if constexpr (FUSED)
+        if (!use_mma && pos >= t0 && pos < t1) {
+            const size_t row = (size_t(pos) * 4 + kvh) * 256 + tid;
+            Row::store(kc, row, s_knew[tid]);
+            Row::store(vc, row, s_vnew[tid]);
+        }
     float mg = s_min[0];
 #pragma unroll
     for (int c = 1; c < CL; c++) mg = fmaxf(mg, s_min[c]);
