@@ -255,7 +255,13 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
 
     pdl_wait();
 
+    float raw[8]; // warps 0-3: a query head, 4: the new key, 5: the new value; asked for together with the position
     if constexpr (FUSED) {
+        if (warp < 6) {
+            const float *src = warp < 4 ? q_in + size_t(kvh * 4 + warp) * 512 : (warp == 4 ? k_raw : v_new) + kvh * 256;
+            const float4 a = __ldcg(reinterpret_cast<const float4 *>(src + lane * 8)), b = __ldcg(reinterpret_cast<const float4 *>(src + lane * 8 + 4));
+            raw[0] = a.x; raw[1] = a.y; raw[2] = a.z; raw[3] = a.w; raw[4] = b.x; raw[5] = b.y; raw[6] = b.z; raw[7] = b.w;
+        }
         const int now = __ldcg(p.position) + p.position_offset;
         if (now != pos) {
             pos = now;
@@ -281,35 +287,26 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
         // ---- query (and current key) preparation --------------------------------
         if constexpr (FUSED) {
             if (warp < 4) {
-                float v[8];
-                const float4 *src = reinterpret_cast<const float4 *>(q_in + size_t(kvh * 4 + warp) * 512 + lane * 8);
-                const float4 a = __ldcg(src), b = __ldcg(src + 1);
-                v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-                norm_rope_256(v, norm_wv, lane, pos, rope_c, rope_s);
+                norm_rope_256(raw, norm_wv, lane, pos, rope_c, rope_s);
 #pragma unroll
-                for (int j = 0; j < 8; j++) s_q[warp][lane * 8 + j] = v[j];
+                for (int j = 0; j < 8; j++) s_q[warp][lane * 8 + j] = raw[j];
             } else if (warp == 4 && pos >= t0 && pos < t1) {
-                float v[8];
-                const float4 *src = reinterpret_cast<const float4 *>(k_raw + kvh * 256 + lane * 8);
-                const float4 a = __ldcg(src), b = __ldcg(src + 1);
-                v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-                norm_rope_256(v, norm_wv, lane, pos, rope_c, rope_s);
+                norm_rope_256(raw, norm_wv, lane, pos, rope_c, rope_s);
                 const size_t row = (size_t(pos) * 4 + kvh) * 256 + lane * 8;
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
-                    s_knew[lane * 8 + j] = Row::round(v[j]);
-                    if (use_mma) Row::store(kc, row + j, v[j]);
+                    s_knew[lane * 8 + j] = Row::round(raw[j]);
+                    if (use_mma) Row::store(kc, row + j, raw[j]);
                 }
-                if (use_mma) asm volatile("fence.proxy.async;" ::: "memory"); // the tensor-core loop fetches this row by bulk copy
+                if (use_mma) asm volatile("fence.proxy.async.global;" ::: "memory"); // the tensor-core loop fetches this row by bulk copy
             } else if (warp == 5 && pos >= t0 && pos < t1) {
                 const size_t row = (size_t(pos) * 4 + kvh) * 256 + lane * 8;
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
-                    const float v = __ldcg(v_new + kvh * 256 + lane * 8 + j);
-                    s_vnew[lane * 8 + j] = Row::round(v);
-                    if (use_mma) Row::store(vc, row + j, v);
+                    s_vnew[lane * 8 + j] = Row::round(raw[j]);
+                    if (use_mma) Row::store(vc, row + j, raw[j]);
                 }
-                if (use_mma) asm volatile("fence.proxy.async;" ::: "memory");
+                if (use_mma) asm volatile("fence.proxy.async.global;" ::: "memory");
             }
         } else {
             for (int i = tid; i < 1024; i += kAtThreads) s_q[i >> 8][i & 255] = __ldcg(q_in + size_t(kvh) * 1024 + i);

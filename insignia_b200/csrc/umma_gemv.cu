@@ -32,6 +32,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 namespace insg {
 
@@ -361,7 +362,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             const bool one = elect_one();
             if (prepared) { // the digits come ready: eight k-blocks per copy, so that the multiplies can start behind the first
                 pdl_wait();
-                asm volatile("fence.proxy.async;" ::: "memory"); // written by ordinary stores of the launch before
+                asm volatile("fence.proxy.async.global;" ::: "memory"); // written by ordinary stores of the launch before
                 for (int kb = 0; kb < len; kb += 8)
                     if (one) {
                         const uint32_t bytes = uint32_t(min(8, len - kb)) * kImg;
@@ -409,9 +410,12 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 uint64_t db = db0;
                 uint32_t sb = tmem + kDSfbCol;
-                for (int kb = 0; kb < len; kb += 2) {
-                    if (!here && !mbar_wait(&full[st], phase, abort_flag)) { ok = false; break; }
-                    if (run == 0 && (kb & 7) == 0 && !mbar_wait(&image[kb >> 3], 0, abort_flag)) { ok = false; break; } // the digits of eight k-blocks
+                // Branches among the issued instructions cost more than the instructions: the first run, which also brings the
+                // digits' scales, and the single last block of an odd count have loops of their own.
+                auto stage = [&](int kb, auto is_first, auto has_two) -> bool {
+                    constexpr bool first = decltype(is_first)::value, two = decltype(has_two)::value;
+                    if (!here && !mbar_wait(&full[st], phase, abort_flag)) return false;
+                    if (first && (kb & 7) == 0 && !mbar_wait(&image[kb >> 3], 0, abort_flag)) return false; // the digits of eight k-blocks
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t da = da0 + uint64_t(uint32_t(st) * uint32_t(kDStage >> 4)), dsf = dsf0 + uint64_t(uint32_t(st) * uint32_t(kDStage >> 4));
                     const uint32_t sa = tmem + kDSfaCol + 8 * sfa;
@@ -420,8 +424,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                     here = mbar_test(&full[st], phase);
                     if (kb + 2 >= len) room = mbar_test(&dempty[buf ^ 1], (((run + 1) >> 1) & 1) ^ 1);
                     if (one) {
-                        const bool two = kb + 1 < len;
-                        if (run == 0) { // the digits' scales stay in tensor memory for all tiles
+                        if (first) { // the digits' scales stay in tensor memory for all tiles
                             copy_scales(sb, dsb0 + uint64_t(kb * (kImg >> 4)));
                             if (two) copy_scales(sb + 4, dsb0 + uint64_t((kb + 1) * (kImg >> 4)));
                         }
@@ -438,6 +441,17 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                     db += 2 * (kImg >> 4);
                     sb += 8;
                     sfa = (sfa + 1) & 3;
+                    return true;
+                };
+                constexpr std::true_type yes{};
+                constexpr std::false_type no{};
+                const int even = len & ~1;
+                if (run == 0) {
+                    for (int kb = 0; kb < even && ok; kb += 2) ok = stage(kb, yes, yes);
+                    if (ok && even < len) ok = stage(even, yes, no);
+                } else {
+                    for (int kb = 0; kb < even && ok; kb += 2) ok = stage(kb, no, yes);
+                    if (ok && even < len) ok = stage(even, no, no);
                 }
                 if (ok && one) commit_to(&dfull[buf]);
             }
