@@ -396,6 +396,9 @@ INSG_API int insg_attention_step(const insg_attn_op *op /* host */, insg_stream_
  * position_offset + tokens) when the host knows it: short contexts then start fewer CTAs (the results do not depend on it
  * while it holds).  op->pdl is ignored (plain stream order).  Same math per token as insg_attention_step. */
 INSG_API int insg_attention_chunk(const insg_attn_op *op /* host */, int tokens, float *q_scratch, int rows_hint, insg_stream_t stream);
+/* The cache rows of those tokens alone (keys normalised and rotated, values), for a block whose outputs nobody reads: k_raw, v,
+ * k_norm_w, the caches, position and the cache's description are used. */
+INSG_API int insg_attention_rows(const insg_attn_op *op /* host */, int tokens, insg_stream_t stream);
 /* One step for `sequences` independent sequences at the same position in ONE launch (a decode batch): op describes
  * sequence 0; sequence s takes qraw + s * 8192, k_raw + s * 1024, v + s * 1024, writes out + s * 4096, and has its
  * caches at k_cache / v_cache + s * cache_stride_bytes.  scratch: sequences * insg_gqa_scratch_bytes(.) bytes, the first
@@ -472,6 +475,12 @@ INSG_API int insg_commit_tokens(const int *next, int *tokens, int *log, int capa
 /* src/qwen_kernels.cu:26 : y[rows] = W_bf16[rows][cols] x (mtp.fc) */
 INSG_API int insg_bf16_gemv(const uint16_t *w, const float *x, float *y, int rows, int cols, int pdl,
                             insg_stream_t stream);
+/* The same for x[tokens][cols], y[tokens][rows], the weights read once per eight tokens. */
+INSG_API int insg_bf16_gemv_tokens(const uint16_t *w, const float *x, float *y, int rows, int cols, int tokens, insg_stream_t stream);
+/* The MTP block's input (src/decode.cu:24-40): out[m] = RMSNorm(embedding of device_tokens[m]) * norm_e | RMSNorm(hidden[m]) * norm_h,
+ * 2 * cols values; rows outside [0, rows) embed as zeros. */
+INSG_API int insg_mtp_input(const uint32_t *weight, const uint8_t *scales, const int *device_tokens, const float *hidden,
+                            const uint16_t *norm_e, const uint16_t *norm_h, float *out, int count, int rows, int cols, insg_stream_t stream);
 
 /* -------------------------------------------------------------- storage */
 /* Handle-based face of ModelFile + TieredStorage (include/insignia_model.hpp:20-40, include/insignia_storage.hpp:15-31 of

@@ -87,15 +87,14 @@ public:
     void layer(int layer);
     int decode_token(int token);
     void forward_token(int token);
-    // Additive: forward_token for `count` consecutive tokens (a prompt), the GEMVs taking four tokens per pass over the
-    // weights; leaves the same state as the loop would, and the logits and arg-max of the last token.
+    // Additive: forward_token for `count` consecutive tokens (a prompt), in passes of up to 512 over the weights; leaves the same state as the loop would, and the logits and arg-max of the last token.
     void forward_tokens(const int *tokens, int count);
     int logits_argmax();
     int mtp_draft(int input_token);
 
     // Additive: speculative greedy decode, draft-1 / verify (the reference has the draft half only).
-    // prime_speculative: the prompt token by token like forward_token, also leaving every position's row in the MTP
-    // head's cache; returns the greedy next token.  generate_speculative: `count` tokens, each step one MTP draft and
+    // prime_speculative: the prompt like forward_tokens, also leaving every position's row in the MTP head's cache; returns
+    // the greedy next token.  generate_speculative: `count` tokens, each step one MTP draft and
     // one two-token verify pass of the main model; a right draft yields two tokens per pass, a wrong one is rolled back
     // (DeltaNet state, convolution history).  Output identical to plain greedy decode.  *accepted receives the number of
     // drafts that were right.  forced_drafts (optional, `count` entries): drafts from the caller instead of the MTP head.
@@ -140,6 +139,8 @@ private:
     DecodeWorkspace &x_;
     std::unique_ptr<Plan> plan_;
     void mtp_step(int token, bool draft);
+    void load_mtp();
+    void run_prompt(const int *tokens, int count, bool mtp);
     void build_program();
     void run_program(int n_tokens, int token);
     void recover_after_timeout();

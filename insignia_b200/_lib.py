@@ -117,6 +117,9 @@ SIGNATURES = {
     "insg_argmax_rows": (i32, [vp, C.c_longlong, i32, i32, vp, vp]),
     "insg_commit_tokens": (i32, [vp, vp, vp, i32, vp, i32, vp]),
     "insg_bf16_gemv": (i32, [vp, vp, vp, i32, i32, i32, vp]),
+    "insg_bf16_gemv_tokens": (i32, [vp, vp, vp, i32, i32, i32, vp]),
+    "insg_mtp_input": (i32, [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, vp]),
+    "insg_attention_rows": (i32, [vp, i32, vp]),
     "insg_storage_open": (vp, [C.c_char_p, u64, i32]),
     "insg_storage_close": (None, [vp]),
     "insg_storage_acquire": (i32, [vp, C.c_char_p, C.POINTER(vp), C.POINTER(u64)]),

@@ -568,7 +568,7 @@ template <bool BF16, bool FUSED> int launch_attn(const AttnParams &p, cudaStream
 
 // A chunk of consecutive tokens, step one: per token m (one CTA each) the per-head RMSNorm + partial RoPE of the 16 query
 // heads (into qn[m][16][256]) and of the 4 key heads, and the token's key and value rows written to the cache at row
-// position + offset + m.  Warp tasks 0..15 = query heads, 16..19 = key heads, 20..23 = value heads.
+// position + offset + m.  Warp tasks 0..15 = query heads, 16..19 = key heads, 20..23 = value heads.  Without qn: the rows alone.
 // (reference: split_q_gate + qwen35_qk_norm_rope_gate + store_kv, src/qwen_kernels.cu:15,31 and src/ops.cu:9, once per token)
 template <bool BF16> __global__ void __launch_bounds__(kAtThreads) attn_chunk_prepare_kernel(const __grid_constant__ AttnParams p, float *qn)
 {
@@ -578,7 +578,7 @@ template <bool BF16> __global__ void __launch_bounds__(kAtThreads) attn_chunk_pr
     if (pos < 0 || pos >= p.max_context) return; // host checks; never index past the cache
     float rope_c[8], rope_s[8];
     if (lane < 8) rope_table(pos, lane, p.fast_trig != 0, rope_c, rope_s);
-    for (int task = warp; task < 24; task += kAtWarps) {
+    for (int task = qn ? warp : 16 + warp; task < 24; task += kAtWarps) {
         if (task < 20) {
             const bool is_q = task < 16;
             const int h = is_q ? task : task - 16;
@@ -684,6 +684,17 @@ int insg_gqa_decode(const float *q, const void *k_cache, const void *v_cache, fl
     if (kv_dtype != INSG_KV_F32 && kv_dtype != INSG_KV_BF16) return fail(INSG_E_ARG, "gqa_decode: bad kv dtype");
     if (scratch_bytes < attn_scratch_bytes()) return fail(INSG_E_SHAPE, "gqa_decode: scratch too small");
     return attn_plain_launch(q, k_cache, v_cache, out, tokens, kv_dtype, scratch, stream);
+}
+
+int insg_attention_rows(const insg_attn_op *op, int tokens, insg_stream_t stream)
+{
+    if (!op || !op->k_raw || !op->v || !op->k_norm_w || !op->k_cache || !op->v_cache || !op->position) return fail(INSG_E_ARG, "attention_rows: null pointer");
+    if (tokens < 1 || tokens > 65535 || op->max_context <= 0) return fail(INSG_E_SHAPE, "attention_rows: 1 <= tokens <= 65535, max_context > 0");
+    AttnParams p = {};
+    p.k_raw = op->k_raw; p.v_new = op->v; p.k_w = op->k_norm_w; p.kc = op->k_cache; p.vc = op->v_cache;
+    p.position = op->position; p.position_offset = op->position_offset; p.max_context = op->max_context; p.fast_trig = op->fast_trig;
+    auto kernel = op->kv_dtype == INSG_KV_BF16 ? attn_chunk_prepare_kernel<true> : attn_chunk_prepare_kernel<false>;
+    return launch(kernel, dim3(tokens), dim3(kAtThreads), 0, stream, false, p, static_cast<float *>(nullptr));
 }
 
 int insg_attention_chunk(const insg_attn_op *op, int tokens, float *q_scratch, int rows_hint, insg_stream_t stream)

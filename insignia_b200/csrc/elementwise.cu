@@ -206,28 +206,108 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const float *x, int n, int
     }
 }
 
-// y[rows] = W_bf16[rows][cols] x : one warp per row, 16-byte loads (src/qwen_kernels.cu:25; mtp.fc 4096x8192)
+// y[m][rows] = W_bf16[rows][cols] x[m] (src/qwen_kernels.cu:25; mtp.fc 4096 x 8192).  The weights bound it as long as nothing else
+// is waited for between them: x goes through shared memory (32 KB at a time, the two halves of an 8-column vector apart so that
+// a warp's reads meet no bank twice), a warp takes R rows of T tokens, and a vector's registers are refilled as soon as they have
+// been used, the first U ones before the producer of x is done.  4096 x 8192, one token: 31.8 us with a warp per row and x from
+// L2 -> 12.7 us (10.2 at copy rate); eight tokens 28 us, where the multiply-adds bound it.  Each row's sum has the same order in both.
+template <int T, int R, int U>
 __global__ void __launch_bounds__(256) bf16_gemv_kernel(const uint16_t *__restrict__ w, const float *__restrict__ x, float *__restrict__ y,
-                                                        int rows, int cols)
+                                                        int rows, int cols, int tokens)
 {
+    constexpr int KV = 1024 / T; // vectors of eight columns in shared memory, per token
+    static_assert(KV % (32 * U) == 0, "whole steps");
+    __shared__ __align__(16) float4 xs[2][T][KV];
     pdl_launch_dependents();
-    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (row >= rows) return;
-    const uint4 *wr = reinterpret_cast<const uint4 *>(w + size_t(row) * cols);
+    const int tid = threadIdx.x, lane = tid & 31, row0 = (blockIdx.x * 8 + (tid >> 5)) * R, t0 = blockIdx.y * T;
     const int nvec = cols >> 3;
+    const uint4 *wr[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) wr[r] = reinterpret_cast<const uint4 *>(w + size_t(min(row0 + r, rows - 1)) * cols);
+    uint4 q[R][U];
+    auto fetch = [&](int u, int i) {
+#pragma unroll
+        for (int r = 0; r < R; r++)
+            if (i < nvec) q[r][u] = ldg_stream(wr[r] + i);
+    };
+#pragma unroll
+    for (int u = 0; u < U; u++) fetch(u, lane + 32 * u);
+    float z[R][T];
+#pragma unroll
+    for (int r = 0; r < R; r++)
+#pragma unroll
+        for (int t = 0; t < T; t++) z[r][t] = 0.f;
     pdl_wait();
-    float z = 0.f;
-#pragma unroll 4
-    for (int i = lane; i < nvec; i += 32) {
-        const uint4 q = ldg_stream(wr + i);
-        const float4 x0 = __ldcg(reinterpret_cast<const float4 *>(x) + i * 2), x1 = __ldcg(reinterpret_cast<const float4 *>(x) + i * 2 + 1);
-        z = fmaf(__uint_as_float(q.x << 16), x0.x, z); z = fmaf(__uint_as_float(q.x & 0xffff0000u), x0.y, z);
-        z = fmaf(__uint_as_float(q.y << 16), x0.z, z); z = fmaf(__uint_as_float(q.y & 0xffff0000u), x0.w, z);
-        z = fmaf(__uint_as_float(q.z << 16), x1.x, z); z = fmaf(__uint_as_float(q.z & 0xffff0000u), x1.y, z);
-        z = fmaf(__uint_as_float(q.w << 16), x1.z, z); z = fmaf(__uint_as_float(q.w & 0xffff0000u), x1.w, z);
+    for (int c = 0; c < nvec; c += KV) {
+        if (c) __syncthreads();
+        const int here = min(KV, nvec - c); // vectors
+        for (int i = tid; i < T * KV * 2; i += 256) {
+            const int t = i / (2 * KV), j = i - t * 2 * KV;
+            if (j < 2 * here) xs[j & 1][t][j >> 1] = __ldcg(reinterpret_cast<const float4 *>(x + size_t(min(t0 + t, tokens - 1)) * cols + c * 8) + j);
+        }
+        __syncthreads();
+        for (int j0 = lane; j0 < here; j0 += 32 * U) {
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int j = j0 + 32 * u;
+                if (j >= here) break;
+#pragma unroll
+                for (int t = 0; t < T; t++) {
+                    const float4 x0 = xs[0][t][j], x1 = xs[1][t][j];
+#pragma unroll
+                    for (int r = 0; r < R; r++) {
+                        const uint4 v = q[r][u];
+                        float s = z[r][t];
+                        s = fmaf(__uint_as_float(v.x << 16), x0.x, s); s = fmaf(__uint_as_float(v.x & 0xffff0000u), x0.y, s);
+                        s = fmaf(__uint_as_float(v.y << 16), x0.z, s); s = fmaf(__uint_as_float(v.y & 0xffff0000u), x0.w, s);
+                        s = fmaf(__uint_as_float(v.z << 16), x1.x, s); s = fmaf(__uint_as_float(v.z & 0xffff0000u), x1.y, s);
+                        s = fmaf(__uint_as_float(v.w << 16), x1.z, s); s = fmaf(__uint_as_float(v.w & 0xffff0000u), x1.w, s);
+                        z[r][t] = s;
+                    }
+                }
+                fetch(u, c + j + 32 * U);
+            }
+        }
     }
-    z = warp_sum(z);
-    if (lane == 0) y[row] = z;
+#pragma unroll
+    for (int r = 0; r < R; r++)
+#pragma unroll
+        for (int t = 0; t < T; t++) {
+            const float s = warp_sum(z[r][t]);
+            if (lane == 0 && row0 + r < rows && t0 + t < tokens) y[size_t(t0 + t) * rows + row0 + r] = s;
+        }
+}
+
+// The MTP block's input rows [m][2 cols]: the embedding of tokens[m] and the hidden state hidden[m], each RMS-normalised
+// (reference: src/decode.cu:24-40, three launches).  CTA (half, m); the sums have rmsnorm_kernel's order.
+__global__ void __launch_bounds__(256) mtp_input_kernel(const uint32_t *__restrict__ w, const uint8_t *__restrict__ s, const int *__restrict__ tokens,
+                                                        const float *__restrict__ hidden, const uint16_t *__restrict__ norm_e,
+                                                        const uint16_t *__restrict__ norm_h, float *__restrict__ out, int rows, int cols)
+{
+    __shared__ float scratch[8];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int m = blockIdx.y;
+    const bool emb = blockIdx.x == 0;
+    const int row = emb ? __ldcg(tokens + m) : 0;
+    const bool known = row >= 0 && row < rows;
+    auto value = [&](int i) {
+        if (!emb) return __ldcg(hidden + size_t(m) * cols + i);
+        if (!known) return 0.f;
+        return e2m1_to_float(w[size_t(row) * (cols >> 3) + (i >> 3)] >> ((i & 7) * 4)) * e8m0_to_float(s[size_t(row) * (cols >> 5) + (i >> 5)]);
+    };
+    float ss = 0.f;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < cols; i += 256) {
+        const float v = value(i);
+        ss = fmaf(v, v, ss);
+    }
+    ss = block_sum<8>(ss, scratch);
+    const float inv = rsqrtf(ss / float(cols) + 1e-6f);
+    const uint16_t *nw = emb ? norm_e : norm_h;
+    float *y = out + size_t(m) * 2 * cols + (emb ? 0 : cols);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < cols; i += 256) y[i] = value(i) * inv * bf16_bits_to_float(nw[i]);
 }
 
 static int check_launch(const char *what)
@@ -385,7 +465,20 @@ int insg_commit_tokens(const int *next, int *tokens, int *log, int capacity, int
 int insg_bf16_gemv(const uint16_t *w, const float *x, float *y, int rows, int cols, int pdl, insg_stream_t stream)
 {
     if (!w || !x || !y || rows <= 0 || cols <= 0 || (cols & 7)) return fail(INSG_E_ARG, "bf16_gemv: bad argument");
-    return launch(bf16_gemv_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, pdl != 0, w, x, y, rows, cols);
+    return launch(bf16_gemv_kernel<1, 2, 8>, dim3((rows + 15) / 16), dim3(256), 0, stream, pdl != 0, w, x, y, rows, cols, 1);
+}
+int insg_bf16_gemv_tokens(const uint16_t *w, const float *x, float *y, int rows, int cols, int tokens, insg_stream_t stream)
+{
+    if (tokens == 1) return insg_bf16_gemv(w, x, y, rows, cols, 0, stream);
+    if (!w || !x || !y || rows <= 0 || cols <= 0 || (cols & 7) || tokens < 1 || tokens > 65535) return fail(INSG_E_ARG, "bf16_gemv_tokens: bad argument");
+    return launch(bf16_gemv_kernel<8, 4, 4>, dim3((rows + 31) / 32, (tokens + 7) / 8), dim3(256), 0, stream, false, w, x, y, rows, cols, tokens);
+}
+int insg_mtp_input(const uint32_t *weight, const uint8_t *scales, const int *device_tokens, const float *hidden, const uint16_t *norm_e,
+                   const uint16_t *norm_h, float *out, int count, int rows, int cols, insg_stream_t stream)
+{
+    if (!weight || !scales || !device_tokens || !hidden || !norm_e || !norm_h || !out) return fail(INSG_E_ARG, "mtp_input: null pointer");
+    if (rows <= 0 || cols <= 0 || (cols & 31) || count < 1 || count > 65535) return fail(INSG_E_SHAPE, "mtp_input: bad rows/cols/count");
+    return launch(mtp_input_kernel, dim3(2, count), dim3(256), 0, stream, false, weight, scales, device_tokens, hidden, norm_e, norm_h, out, rows, cols);
 }
 
 } // extern "C"

@@ -575,6 +575,35 @@ void attention_block_multi(Ctx &c, const Qwen35Decode::Plan::Block &b, void *kc,
 
     mlp_block_multi(c, b, u);
 }
+
+// The MTP block's key and value rows for `rows` consecutive tokens (input x: the block's residual stream), from the device
+// position + offset on.
+void mtp_rows(Ctx &c, const Qwen35Decode::Plan::Block &b, const float *x, float *key, float *value, int rows, int position_offset)
+{
+    insg_gemv_op in = {};
+    in.in = x;
+    in.norm_w = b.in_norm;
+    in.cols = kHidden;
+    in.prologue = INSG_PRO_RMSNORM;
+    in.tokens = rows;
+    in.n_segments = 2;
+    in.seg[0] = seg(b.k, key, INSG_EPI_STORE);
+    in.seg[1] = seg(b.v, value, INSG_EPI_STORE);
+    run_gemv(c, in);
+    insg_attn_op at = {};
+    at.k_raw = key;
+    at.v = value;
+    at.k_norm_w = b.k_norm;
+    at.k_cache = c.x.mtp_keys;
+    at.v_cache = c.x.mtp_values;
+    at.position = c.x.d_position;
+    at.position_offset = position_offset;
+    at.max_context = c.x.max_context;
+    at.kv_dtype = c.x.options.kv_bf16 ? INSG_KV_BF16 : INSG_KV_F32;
+    at.fast_trig = c.x.options.accurate_trig ? 0 : 1;
+    insg_check(insg_attention_rows(&at, rows, c.st));
+    c.launches++;
+}
 } // namespace
 
 // ------------------------------------------------------------------ public API
@@ -926,7 +955,10 @@ void Qwen35Decode::forward_token(int token)
     fused_token_valid_ = true;
 }
 
-void Qwen35Decode::forward_tokens(const int *tokens, int count)
+void Qwen35Decode::forward_tokens(const int *tokens, int count) { run_prompt(tokens, count, false); }
+
+// mtp: every pass also leaves the rows that the MTP head's cache gets from it: hidden state m with the embedding of token m + 1.
+void Qwen35Decode::run_prompt(const int *tokens, int count, bool mtp)
 {
     if (count <= 0) return;
     if (!tokens) throw std::runtime_error("forward_tokens: null token list");
@@ -998,6 +1030,17 @@ void Qwen35Decode::forward_tokens(const int *tokens, int count)
         } else {
             enqueue_chunk();
             p.chunk_warm |= !one_layout && !use_umma && T == kChunk;
+        }
+        if (mtp) {
+            const int rows = std::min(T, count - done - 1); // the prompt's last token has no successor yet
+            if (rows > 0) {
+                cuda_check(cudaMemcpyAsync(u.tokens, tokens + done + 1, size_t(rows) * sizeof(int), cudaMemcpyHostToDevice, p.stream), "copy tokens");
+                insg_check(insg_mtp_input(static_cast<const uint32_t *>(p.embed.weight.data), static_cast<const uint8_t *>(p.embed.scales.data), u.tokens,
+                                          u.hidden, p.mtp_norm_e, p.mtp_norm_h, u.qkv, rows, p.embed.rows, kHidden, p.stream));
+                insg_check(insg_bf16_gemv_tokens(p.mtp_fc, u.qkv, u.core, kHidden, 2 * kHidden, rows, p.stream));
+                launches_ += 2;
+                mtp_rows(c, p.mtp, u.core, u.key, u.value, rows, 0);
+            }
         }
         x_.position += T;
         done += T;
@@ -1229,38 +1272,45 @@ int Qwen35Decode::mtp_draft(int token)
     return logits_argmax();
 }
 
-// The MTP block at the current position (reference: src/decode.cu:24-68).  draft = false stops before the head: the call
-// then only leaves the position's row in the MTP cache (a speculative decoder needs every row, the prompt's included).
+void Qwen35Decode::load_mtp()
+{
+    Plan &p = plan();
+    if (p.mtp_ready) return;
+    const std::string m = std::string(kLM) + ".mtp";
+    Loader L{w_, p.pinned, tcgen05_engine(x_.options) ? 1 : 0};
+    p.mtp_fc = L.bf16(m + ".fc.weight", size_t(kHidden) * 2 * kHidden);
+    p.mtp_norm_e = L.bf16(m + ".pre_fc_norm_embedding.weight", kHidden);
+    p.mtp_norm_h = L.bf16(m + ".pre_fc_norm_hidden.weight", kHidden);
+    p.mtp_norm = L.bf16(m + ".norm.weight", kHidden);
+    load_attention(L, m + ".layers.0", p.mtp);
+    p.mtp_ready = true;
+}
+
+// The MTP block at the current position (reference: src/decode.cu:24-68).  draft = false only leaves the position's row
+// in the MTP cache (a speculative decoder needs every row, the prompt's included): the keys and values, and no more of the block.
 // Asynchronous: logits_argmax() waits for the draft.
 void Qwen35Decode::mtp_step(int token, bool draft)
 {
     if (token < 0 || token >= Qwen35Shape::vocab) throw std::runtime_error("token out of range");
     if (x_.position < 1) throw std::runtime_error("mtp_draft needs a forwarded token");
     Plan &p = plan();
-    const std::string m = std::string(kLM) + ".mtp";
-    if (!p.mtp_ready) {
-        Loader L{w_, p.pinned, tcgen05_engine(x_.options) ? 1 : 0};
-        p.mtp_fc = L.bf16(m + ".fc.weight", size_t(kHidden) * 2 * kHidden);
-        p.mtp_norm_e = L.bf16(m + ".pre_fc_norm_embedding.weight", kHidden);
-        p.mtp_norm_h = L.bf16(m + ".pre_fc_norm_hidden.weight", kHidden);
-        p.mtp_norm = L.bf16(m + ".norm.weight", kHidden);
-        load_attention(L, m + ".layers.0", p.mtp);
-        p.mtp_ready = true;
-    }
+    load_mtp();
     if (!p.head_ready || !p.embed_ready) throw std::runtime_error("mtp_draft needs a forwarded token");
     const bool pdl = x_.options.use_pdl;
     sync_scalars(token);
     run_graphed(x_.options.use_graph, p.stream, p.exec_mtp[draft ? 1 : 0], p.mtp_runs[draft ? 1 : 0], launches_, [&] {
         // embedding of the input token and the last hidden state, each normalised, side by side in qkv[8192]
-        insg_check(insg_mxfp4_embed(static_cast<const uint32_t *>(p.embed.weight.data), static_cast<const uint8_t *>(p.embed.scales.data),
-                                    x_.down, x_.d_token, p.embed.rows, kHidden, 0, p.stream));
-        insg_check(insg_rmsnorm_bf16(x_.down, p.mtp_norm_e, nullptr, x_.qkv, 1, kHidden, 0, p.stream));
-        insg_check(insg_rmsnorm_bf16(x_.hidden, p.mtp_norm_h, nullptr, x_.qkv + kHidden, 1, kHidden, 0, p.stream));
-        insg_check(insg_bf16_gemv(p.mtp_fc, x_.qkv, x_.hidden, kHidden, 2 * kHidden, 0, p.stream)); // overwrites the residual, as the reference
-        launches_ += 4;
+        insg_check(insg_mtp_input(static_cast<const uint32_t *>(p.embed.weight.data), static_cast<const uint8_t *>(p.embed.scales.data), x_.d_token,
+                                  x_.hidden, p.mtp_norm_e, p.mtp_norm_h, x_.qkv, 1, p.embed.rows, kHidden, p.stream));
+        float *fc_out = draft ? x_.hidden : x_.core; // a draft overwrites the residual, as the reference
+        insg_check(insg_bf16_gemv(p.mtp_fc, x_.qkv, fc_out, kHidden, 2 * kHidden, pdl ? 1 : 0, p.stream));
+        launches_ += 2;
         Ctx c{x_, p.stream, pdl, launches_, false, nullptr, nullptr};
+        if (!draft) {
+            mtp_rows(c, p.mtp, fc_out, x_.key, x_.value, 1, -1);
+            return;
+        }
         enqueue_attention_block(c, p.mtp, x_.mtp_keys, x_.mtp_values, -1); // rotary position / cache row position-1, position rows attended
-        if (!draft) return;
         insg_gemv_op op = {};
         op.in = x_.hidden;
         op.norm_w = p.mtp_norm;
@@ -1288,6 +1338,11 @@ void Qwen35Decode::mtp_step(int token, bool draft)
 int Qwen35Decode::prime_speculative(const int *prompt, int count)
 {
     if (!prompt || count < 1) throw std::runtime_error("prime_speculative: empty prompt");
+    if (tcgen05_engine(x_.options)) { // in passes, like any prompt
+        if (count > 1) load_mtp();
+        run_prompt(prompt, count, true);
+        return logits_argmax();
+    }
     for (int i = 0; i < count; i++) {
         forward_token(prompt[i]);
         if (i + 1 < count) mtp_step(prompt[i + 1], false); // row i of the MTP cache: hidden state i with the embedding of token i + 1

@@ -443,3 +443,18 @@ def bf16_gemv(w, x, pdl=False):
     y = torch.empty(w.shape[0], dtype=torch.float32, device=x.device)
     check(_lib.lib().insg_bf16_gemv(_p(w), _p(x), _p(y), w.shape[0], w.shape[1], int(pdl), _stream()))
     return y
+
+
+def bf16_gemv_tokens(w, x):
+    """``y[m] = w x[m]``, the weights read once per eight rows of ``x``."""
+    y = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device)
+    check(_lib.lib().insg_bf16_gemv_tokens(_p(w), _p(x), _p(y), w.shape[0], w.shape[1], x.shape[0], _stream()))
+    return y
+
+
+def mtp_input(weight, scales, tokens, hidden, norm_e, norm_h):
+    """The MTP block's input rows: the normalised embedding of each token beside its normalised hidden state."""
+    out = torch.empty((hidden.shape[0], 2 * hidden.shape[1]), dtype=torch.float32, device=hidden.device)
+    check(_lib.lib().insg_mtp_input(_p(weight), _p(scales), _p(tokens), _p(hidden), _p(norm_e), _p(norm_h), _p(out), hidden.shape[0],
+                                    weight.shape[0], hidden.shape[1], _stream()))
+    return out
