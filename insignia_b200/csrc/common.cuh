@@ -83,10 +83,10 @@ __device__ __forceinline__ uint4 ldg_stream(const void *p)
                  : "l"(p));
     return r;
 }
-__device__ __forceinline__ uint32_t ldg_stream_u16(const void *p)
+__device__ __forceinline__ uint2 ldg_stream_u64(const void *p)
 {
-    uint16_t r;
-    asm volatile("ld.global.nc.L1::no_allocate.u16 %0, [%1];" : "=h"(r) : "l"(p));
+    uint2 r;
+    asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p));
     return r;
 }
 

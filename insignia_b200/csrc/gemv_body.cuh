@@ -20,7 +20,9 @@ constexpr int kWarps = 16;  // warps per CTA, one CTA per SM
 constexpr int kThreads = kWarps * 32;
 constexpr float kLoScale = 1.0f / 2048.0f;
 constexpr int kMaxGrid = 296;
-constexpr int kUnr = 3;     // records per register prefetch chunk (2 / 3 / 4 measured 580 / 584 / 569 tokens/s in the engine)
+constexpr int kMaxSmem = 224 * 1024; // dynamic shared memory of a CTA, beside less than 1 KB of static
+constexpr int kUnr = 2;     // records per register chunk, two chunks in flight (three: 4096 x 4096 with one token 7.4 -> 8.1 us)
+constexpr int kXPad = 32;   // fp16 values between two pieces: neighbouring pieces start 16 banks apart (gemv_stream reads two at once)
 // Fixed pre-scale of a prepared activation image: the producer cannot know the vector's maximum, so instead of the
 // adaptive power of two of the in-kernel prologue the image holds x / 16.  fp16 then covers |x| from 1e-3 (below that
 // the low piece loses bits that are far under the fp32 rounding of a 4096-term dot product) to 1e6 (saturating).
@@ -85,9 +87,26 @@ __device__ __forceinline__ void dequant8(uint32_t q, uint32_t (&h)[4])
 __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                          uint32_t b1)
 {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// The first step of a sum: no accumulator to clear.
+__device__ __forceinline__ void mma16816_first(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
+{
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+
+// One word of a record.  Four such loads take a row's 64 bytes, the first of them brings the lines: they stay in L1 until the
+// others have been served, and leave it first.
+__device__ __forceinline__ uint32_t ldg_word(const void *p)
+{
+    uint32_t r;
+    asm volatile("ld.global.nc.L1::evict_first.b32 %0, [%1];" : "=r"(r) : "l"(p));
+    return r;
 }
 
 // Position in the linear record sequence.
@@ -137,26 +156,31 @@ __device__ __forceinline__ void it_next(const GemvParams &p, UnitIt &it, int nkb
 }
 
 template <int UNR> struct Chunk {
-    uint4 wa[UNR], wb[UNR];
-    uint32_t sc[UNR];
+    uint4 wa[UNR], wb[UNR]; // rows g and g+8: word t of each of the four scale groups
+    uint2 sc[UNR];          // their scale bytes: {g, g+8} of group 0, of group 1, ...
 };
 
-// Issues the loads of the next UNR records (those below `end`) and advances the iterator past them.
+// Issues the loads of the next record (if it is below `end`) and advances the iterator past it.
+template <int UNR>
+__device__ __forceinline__ void load_record(const GemvParams &p, Chunk<UNR> &b, int j, UnitIt &it, int end, int lane, int nkb, int total_units)
+{
+    if (it.u < end) {
+        const uint8_t *q = it.ptr + (lane >> 2) * 64 + (lane & 3) * 4;
+        b.wa[j] = make_uint4(ldg_word(q), ldg_word(q + 16), ldg_word(q + 32), ldg_word(q + 48));
+        b.wb[j] = make_uint4(ldg_word(q + 512), ldg_word(q + 528), ldg_word(q + 544), ldg_word(q + 560));
+        b.sc[j] = ldg_stream_u64(it.ptr + 1024 + (lane >> 2) * 8);
+        it_next(p, it, nkb, total_units);
+    }
+}
+
 template <int UNR>
 __device__ __forceinline__ void load_chunk(const GemvParams &p, Chunk<UNR> &b, UnitIt &it, int end, int lane, int nkb, int total_units)
 {
 #pragma unroll
     for (int j = 0; j < UNR; j++) {
-        if (it.u < end) {
-            b.wa[j] = ldg_stream(it.ptr + lane * 16);
-            b.wb[j] = ldg_stream(it.ptr + 512 + lane * 16);
-            b.sc[j] = ldg_stream_u16(it.ptr + 1024 + lane * 2);
-            it_next(p, it, nkb, total_units);
-        } else {
-            b.wa[j] = make_uint4(0, 0, 0, 0);
-            b.wb[j] = make_uint4(0, 0, 0, 0);
-            b.sc[j] = 0;
-        }
+        b.wa[j] = b.wb[j] = make_uint4(0, 0, 0, 0);
+        b.sc[j] = make_uint2(0, 0);
+        load_record<UNR>(p, b, j, it, end, lane, nkb, total_units);
     }
 }
 
@@ -198,13 +222,11 @@ __device__ __forceinline__ void gemv_publish_range(const GemvRange &r, GemvShare
     }
 }
 
-// ---- activation prologue: fp32 vector -> two fp16 pieces in shared memory ----
+// ---- activation prologue: fp32 vector (fetched by load_activation) -> two fp16 pieces in shared memory ----
 // Returns 1/alpha, which undoes the power-of-two pre-scale.
-__device__ __forceinline__ float prologue(const GemvParams &p, const ProIn &pin, int m, __half *xs, int xstride, const uint2 (&wpre)[kPreVec],
-                                          float *scratch)
+__device__ __forceinline__ float prologue(const GemvParams &p, const ProIn &pin, int m, float4 (&v)[kMaxVec], __half *xs, int xstride,
+                                          const uint2 (&wpre)[kPreVec], float *scratch)
 {
-    float4 v[kMaxVec];
-    load_activation(pin, m, v);
     const float tmax = transform_activation(pin, m, v, wpre, scratch);
     const int tid = threadIdx.x, nvec = p.cols >> 2;
     // alpha = 2^(12 - floor(log2(max))) puts the largest element in [2^12, 2^13): fp16 holds it with room to spare
@@ -228,6 +250,24 @@ __device__ __forceinline__ float prologue(const GemvParams &p, const ProIn &pin,
         }
     }
     return __uint_as_float(uint32_t(eb - 12) << 23);
+}
+
+// All tokens; the next one's first vectors (4096 columns) are asked for before this one's reductions.
+template <int M>
+__device__ __forceinline__ void prologue_tokens(const GemvParams &p, const ProIn &pin, __half *xs, int xstride, const uint2 (&wpre)[kPreVec],
+                                                float *scratch, float (&inv_alpha)[M])
+{
+    float4 next[kPreVec];
+    load_activation_part<0, kPreVec>(pin, 0, next);
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+        float4 v[kMaxVec];
+#pragma unroll
+        for (int j = 0; j < kPreVec; j++) v[j] = next[j];
+        load_activation_part<kPreVec, kMaxVec>(pin, m, v);
+        if (m + 1 < M) load_activation_part<0, kPreVec>(pin, m + 1, next);
+        inv_alpha[m] = prologue(p, pin, m, v, xs, xstride, wpre, scratch);
+    }
 }
 
 // The whole activation stage for M tokens; ends with a CTA barrier (the pieces are then visible to every warp).
@@ -269,16 +309,14 @@ __device__ __forceinline__ void gemv_activation(const GemvParams &p, __half *xs,
             const ProIn q{p.aux, nullptr, p.norm_w, p.x_out, p.cols, p.norm_w ? INSG_PRO_RMSNORM : INSG_PRO_PLAIN};
             preload_norm_weights(q, wpre);
             __syncthreads(); // every thread has read scratch[1]
-#pragma unroll
-            for (int m = 0; m < M; m++) inv_alpha[m] = prologue(p, q, m, xs, xstride, wpre, scratch);
+            prologue_tokens<M>(p, q, xs, xstride, wpre, scratch, inv_alpha);
         } else {
 #pragma unroll
             for (int m = 0; m < M; m++) inv_alpha[m] = scratch[0];
         }
     } else {
         const ProIn pin{p.in, p.aux, p.norm_w, p.x_out, p.cols, p.prologue};
-#pragma unroll
-        for (int m = 0; m < M; m++) inv_alpha[m] = prologue(p, pin, m, xs, xstride, wpre, scratch);
+        prologue_tokens<M>(p, pin, xs, xstride, wpre, scratch, inv_alpha);
     }
     __syncthreads();
 }
@@ -343,79 +381,96 @@ __device__ __forceinline__ void row_epilogue(const SegDev &s, int row, int m, fl
 
 // The record loop of one warp over [r.ua, r.ub).  A and B hold the first two chunks (gemv_issue_first); `lit` is the
 // load iterator past them.  `wrec` is this warp's slot array [slots][M][16].
+//
+// A quad holds one scale group at a time (word t of it in thread t), so the K of a multiply is 16 values of one group and its
+// eight columns are the pieces (hi, lo) of up to four tokens: eight multiplies a record whatever M, and the scales go on the
+// accumulators.  The loop is bound by the ALU pipe (conversions, byte extraction, scales: two cycles each), which is why
+// one token spreads its column pairs over the groups and scales one group per lane.  Reading a group per thread
+// (16-byte loads) leaves the groups to the columns, eight multiplies per token on three quarters of zeros; exchanging its
+// words within the quad instead costs sixteen selects a record on that same pipe.  Microseconds from 16-byte loads, tokens 1..4:
+// 12352 x 4096 11.7, 14.2, 28 (two launches; 20 in one), 26.8 -> 11.5, 13.3, 16.5, 19.7; 248320 x 4096 107, 129, 238, 241 -> 109,
+// 118, 125, 130 (4.1 TB/s and more).
 template <int UNR, int M>
 __device__ __forceinline__ void gemv_stream(const GemvParams &p, const GemvRange &r, Chunk<UNR> &A, Chunk<UNR> &B, UnitIt &lit,
                                             const __half *xs, int xstride, float *wrec, const float (&inv_alpha)[M], int lane)
 {
     const int g = lane >> 2, t = lane & 3;
-    const int nkb = p.nkb, total_units = p.total_units, ub = r.ub, tm_first = r.tm_first;
-    const bool bactive = (t == (g >> 1));
-    const int piece = g & 1;
-    float acc[M][4];
+    const int nkb = p.nkb, total_units = p.total_units, ub = r.ub;
+    // One token: column pair j of the multiplies belongs to group j, so that lane t scales group t only; several tokens:
+    // column pair m belongs to token m, and lane t scales all four groups of token t.
+    const int pair = g >> 1;
+    const __half *xcol = xs + size_t(M == 1 ? g & 1 : g % (2 * M)) * xstride + t * 8; // columns beyond the tokens repeat others, unread
+    float out_scale = inv_alpha[0];
 #pragma unroll
-    for (int m = 0; m < M; m++) acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
+    for (int m = 1; m < M; m++) out_scale = t == m ? inv_alpha[m] : out_scale;
+    constexpr int kAcc = M == 1 ? 1 : 4;
+    float acc[kAcc][4]; // [group: t alone, or all][rows g, g+8 x the two pieces]
+#pragma unroll
+    for (int i = 0; i < kAcc; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+    uint4 xv[4]; // one token: stays zero in the lanes of other column pairs
+#pragma unroll
+    for (int i = 0; i < 4; i++) xv[i] = make_uint4(0, 0, 0, 0);
+    auto add_scaled = [](float (&a)[4], const float (&c)[4], uint32_t sc) {
+        const float s0 = e8m0_to_float(sc & 0xffu), s1 = e8m0_to_float((sc >> 8) & 0xffu);
+        a[0] = fmaf(c[0], s0, a[0]);
+        a[1] = fmaf(c[1], s0, a[1]);
+        a[2] = fmaf(c[2], s1, a[2]);
+        a[3] = fmaf(c[3], s1, a[3]);
+    };
 
-    // consume one chunk: multiply its records, closing a (tile, matrix) run whenever one ends
-    UnitIt cit;
-    it_set(p, cit, r.ua);
-    auto compute = [&](const Chunk<UNR> &ch) {
+    // Consume one chunk: multiply its records, closing a (tile, matrix) run whenever one ends; a record's registers are asked
+    // for again at once.  Registers past the range are multiplied with whatever they hold and close nothing.
+    int u = r.ua, kb = u % nkb;
+    float *slot = wrec + (M > 1 && t < M ? t * 16 : 0) + (M > 1 ? g : 0);
+    auto compute = [&](Chunk<UNR> &ch) {
 #pragma unroll
         for (int j = 0; j < UNR; j++) {
-            if (cit.u >= ub) break; // warp-uniform
-            float cc[M][4];
+            const uint32_t wa[4] = {ch.wa[j].x, ch.wa[j].y, ch.wa[j].z, ch.wa[j].w}, wb[4] = {ch.wb[j].x, ch.wb[j].y, ch.wb[j].z, ch.wb[j].w};
+            const __half *xk = xcol + kb * 128;
+            float cc[4];
 #pragma unroll
-            for (int m = 0; m < M; m++) cc[m][0] = cc[m][1] = cc[m][2] = cc[m][3] = 0.f;
-            const uint32_t wa[4] = {ch.wa[j].x, ch.wa[j].y, ch.wa[j].z, ch.wa[j].w};
-            const uint32_t wb[4] = {ch.wb[j].x, ch.wb[j].y, ch.wb[j].z, ch.wb[j].w};
-            const int xoff = cit.kb * 128 + t * 32;
-#pragma unroll
-            for (int w = 0; w < 4; w++) {
+            for (int grp = 0; grp < 4; grp++) {
                 uint32_t ha[4], hb[4];
-                dequant8(wa[w], ha);
-                dequant8(wb[w], hb);
+                dequant8(wa[grp], ha);
+                dequant8(wb[grp], hb);
+                if (M > 1 || pair == grp) xv[grp] = *reinterpret_cast<const uint4 *>(xk + grp * 32);
+                if (M > 1 || grp == 0) mma16816_first(cc, ha[0], hb[0], ha[1], hb[1], xv[grp].x, xv[grp].y);
+                else mma16816(cc, ha[0], hb[0], ha[1], hb[1], xv[grp].x, xv[grp].y);
+                mma16816(cc, ha[2], hb[2], ha[3], hb[3], xv[grp].z, xv[grp].w);
+                if (M > 1) add_scaled(acc[grp % kAcc], cc, (grp & 2 ? ch.sc[j].y : ch.sc[j].x) >> (grp & 1 ? 16 : 0));
+            }
+            if (M == 1) add_scaled(acc[0], cc, (t & 2 ? ch.sc[j].y : ch.sc[j].x) >> (t & 1 ? 16 : 0));
+            const bool end = kb == nkb - 1;
+            if (u < ub && (end || u == ub - 1)) { // warp-uniform: fold hi/lo, add the groups (the same tree whatever M), park the run's sums
+                float v0[kAcc], v1[kAcc];
 #pragma unroll
-                for (int m = 0; m < M; m++) {
-                    uint4 xv = make_uint4(0, 0, 0, 0);
-                    if (bactive) xv = *reinterpret_cast<const uint4 *>(xs + size_t(m * 2 + piece) * xstride + xoff + w * 8);
-                    mma16816(cc[m], ha[0], hb[0], ha[1], hb[1], xv.x, xv.y);
-                    mma16816(cc[m], ha[2], hb[2], ha[3], hb[3], xv.z, xv.w);
+                for (int i = 0; i < kAcc; i++) {
+                    v0[i] = fmaf(acc[i][1], kLoScale, acc[i][0]);
+                    v1[i] = fmaf(acc[i][3], kLoScale, acc[i][2]);
+                    acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+                }
+                if constexpr (M == 1) {
+                    v0[0] += __shfl_xor_sync(0xffffffffu, v0[0], 1);
+                    v1[0] += __shfl_xor_sync(0xffffffffu, v1[0], 1);
+                    v0[0] += __shfl_xor_sync(0xffffffffu, v0[0], 2);
+                    v1[0] += __shfl_xor_sync(0xffffffffu, v1[0], 2);
+                    if (t < 2) slot[g + 8 * t] = (t ? v1[0] : v0[0]) * out_scale;
+                } else if (t < M) {
+                    slot[0] = ((v0[0] + v0[1]) + (v0[2] + v0[3])) * out_scale;
+                    slot[8] = ((v1[0] + v1[1]) + (v1[2] + v1[3])) * out_scale;
                 }
             }
-            const float s0 = e8m0_to_float(ch.sc[j] & 0xffu), s1 = e8m0_to_float(ch.sc[j] >> 8);
-#pragma unroll
-            for (int m = 0; m < M; m++) {
-                acc[m][0] = fmaf(cc[m][0], s0, acc[m][0]);
-                acc[m][1] = fmaf(cc[m][1], s0, acc[m][1]);
-                acc[m][2] = fmaf(cc[m][2], s1, acc[m][2]);
-                acc[m][3] = fmaf(cc[m][3], s1, acc[m][3]);
-            }
-            if (cit.kb == nkb - 1 || cit.u == ub - 1) {
-                // fold hi/lo, sum the quad (4 scale groups), gather rows 0..15 into lanes 0..15, park in this run's slot
-                float *slot = wrec + size_t(cit.tm - tm_first) * M * 16;
-#pragma unroll
-                for (int m = 0; m < M; m++) {
-                    float v0 = fmaf(acc[m][1], kLoScale, acc[m][0]);
-                    float v1 = fmaf(acc[m][3], kLoScale, acc[m][2]);
-                    v0 += __shfl_xor_sync(0xffffffffu, v0, 1);
-                    v1 += __shfl_xor_sync(0xffffffffu, v1, 1);
-                    v0 += __shfl_xor_sync(0xffffffffu, v0, 2);
-                    v1 += __shfl_xor_sync(0xffffffffu, v1, 2);
-                    const float r0 = __shfl_sync(0xffffffffu, v0, (lane & 7) * 4);
-                    const float r1 = __shfl_sync(0xffffffffu, v1, (lane & 7) * 4);
-                    if (lane < 16) slot[m * 16 + lane] = ((lane & 8) ? r1 : r0) * inv_alpha[m];
-                    acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
-                }
-            }
-            it_next(p, cit, nkb, total_units);
+            slot += end ? M * 16 : 0;
+            kb = end ? 0 : kb + 1;
+            u++;
+            load_record<UNR>(p, ch, j, lit, ub, lane, nkb, total_units);
         }
     };
 
-    while (cit.u < ub) {
+    while (u < ub) {
         compute(A);
-        load_chunk<UNR>(p, A, lit, ub, lane, nkb, total_units);
-        if (cit.u >= ub) break;
+        if (u >= ub) break;
         compute(B);
-        load_chunk<UNR>(p, B, lit, ub, lane, nkb, total_units);
     }
 }
 
@@ -544,7 +599,7 @@ __device__ __forceinline__ void gemv_finish(const GemvParams &p, const GemvRange
 // Dynamic shared memory of the body: the activation pieces, the per-warp slots, 64 floats of scratch.
 __host__ __device__ inline size_t gemv_smem_bytes(int M, int cols, int slots)
 {
-    return size_t(M) * 2 * (cols + 8) * sizeof(__half) + size_t(kWarps) * slots * M * 16 * 4 + 64 * 4;
+    return size_t(M) * 2 * (cols + kXPad) * sizeof(__half) + size_t(kWarps) * slots * M * 16 * 4 + 64 * 4;
 }
 
 } // namespace insg

@@ -5,9 +5,10 @@
 // The path is HBM-bound: 17 bytes arrive per 32 weights, so the kernel is built around the byte
 // stream, not around the arithmetic:
 //   * weights come from the tile-interleaved copy made by insg_mxfp4_repack: one (16 rows x 128 k)
-//     record is 1088 contiguous bytes, read by a warp with two coalesced 512-byte loads + 64 scale
-//     bytes (ld.global.nc, no L1 allocation); every warp keeps two chunks of UNR records in flight,
-//     both issued BEFORE the programmatic-dependent-launch wait so they overlap the previous kernel;
+//     record is 1088 contiguous bytes, read by a warp so that a quad of lanes shares a row's scale
+//     group (eight loads of a word per lane + 64 scale bytes); every warp keeps two chunks of UNR
+//     records in flight, both issued BEFORE the programmatic-dependent-launch wait so they overlap
+//     the previous kernel;
 //   * the launch's records form one linear sequence (segment, tile, matrix, k-block).  Output tiles
 //     are dealt evenly to the CTAs (one per SM, whole tiles only, so no CTA ever waits for another)
 //     and a CTA's records are then divided evenly over its 16 warps, so every warp of a CTA streams
@@ -19,9 +20,9 @@
 //   * E2M1 nibbles become fp16 pairs with cvt.rn.f16x2.e2m1x2 (exact); the multiply-adds run on
 //     mma.sync.m16n8k16 (fp16 in, fp32 accumulate) purely as a cheap FMA engine.  The fp32 activation
 //     is split into two fp16 pieces (hi + lo * 2^-11 after an exact power-of-two pre-scale) so the
-//     products keep ~22 bits of x; the 8 columns of the MMA's B operand hold (4 scale groups) x
-//     (hi, lo): thread t of a quad owns scale group t of the 128-wide k-block, so accumulator
-//     columns separate the groups and the E8M0 scale is applied once per (row, group) in fp32;
+//     products keep ~22 bits of x; the 8 columns of the MMA's B operand hold (hi, lo) of up to four
+//     tokens, or for one token (4 scale groups) x (hi, lo); every accumulator belongs to one group and
+//     the E8M0 scales are applied once per (row, group) in fp32;
 //   * the elementwise kernels around the GEMV are fused in: RMSNorm / gated RMSNorm / sigmoid-gate
 //     prologues on the activation, residual / conv+SiLU / decay / beta / SwiGLU / logits+arg-max
 //     epilogues on the rows.
@@ -41,7 +42,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_fused_kernel(const __grid_co
     extern __shared__ __align__(16) uint8_t smem_raw[];
     __shared__ GemvShared sh;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int xstride = p.cols + 8;
+    const int xstride = p.cols + kXPad;
     __half *xs = reinterpret_cast<__half *>(smem_raw);
     float *rec = reinterpret_cast<float *>(smem_raw + size_t(M) * 2 * xstride * sizeof(__half)); // [16 warps][slots][M][16]
     float *scratch = rec + size_t(kWarps) * p.slots * M * 16;                                    // 64 floats
@@ -82,7 +83,7 @@ template <int UNR, int M> int launch_variant(const GemvParams &p, int grid, size
     {
         std::lock_guard<std::mutex> lock(mu);
         if (!done[dev]) {
-            e = cudaFuncSetAttribute(gemv_fused_kernel<UNR, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+            e = cudaFuncSetAttribute(gemv_fused_kernel<UNR, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
             if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(gemv)");
             done[dev] = true;
         }
@@ -167,7 +168,7 @@ int gemv_build_params(const insg_gemv_op *op, int M, int max_grid, GemvParams *o
     p.prep_partials_in = op->prologue == INSG_PRO_PREPARED ? op->prep_partials : nullptr;
     p.prep_rms = op->prep_rms != 0;
     const size_t smem = gemv_smem_bytes(M, op->cols, p.slots);
-    if (smem > 220 * 1024) return fail(INSG_E_LIMIT, "gemv: shared memory beyond 220 KB");
+    if (smem > kMaxSmem) return fail(INSG_E_LIMIT, "gemv: shared memory beyond 224 KB");
     *out = p;
     *grid_out = grid;
     *smem_out = smem;
@@ -185,8 +186,8 @@ int gemv_fused_launch(const insg_gemv_op *op, int M, cudaStream_t st)
     switch (M) {
     case 1: return launch_variant<kUnr, 1>(p, grid, smem, st, pdl);
     case 2: return launch_variant<kUnr, 2>(p, grid, smem, st, pdl);
-    case 3: return launch_variant<2, 3>(p, grid, smem, st, pdl);
-    default: return launch_variant<2, 4>(p, grid, smem, st, pdl); // four tokens: registers go to the accumulators
+    case 3: return launch_variant<kUnr, 3>(p, grid, smem, st, pdl);
+    default: return launch_variant<kUnr, 4>(p, grid, smem, st, pdl);
     }
 }
 

@@ -47,17 +47,18 @@ __device__ __forceinline__ void preload_norm_weights(const ProIn &p, uint2 (&wv)
 
 // Requests elements 4*(tid + 512 j) .. +3 of token m's input vector.  Reads go through L2 (ld.global.cg): under
 // programmatic dependent launch this CTA may have been resident, and its L1 filled, before the producer wrote the inputs.
-__device__ __forceinline__ void load_activation(const ProIn &p, int m, float4 (&v)[kMaxVec])
+template <int J0, int J1> __device__ __forceinline__ void load_activation_part(const ProIn &p, int m, float4 *v) // vectors J0 .. J1-1 of it
 {
     const float *in = p.in + size_t(m) * p.cols;
     const int nvec = p.cols >> 2, tid = threadIdx.x;
 #pragma unroll
-    for (int j = 0; j < kMaxVec; j++) {
+    for (int j = J0; j < J1; j++) {
         const int i = tid + j * kProThreads;
         v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (i < nvec) v[j] = __ldcg(reinterpret_cast<const float4 *>(in) + i);
     }
 }
+__device__ __forceinline__ void load_activation(const ProIn &p, int m, float4 (&v)[kMaxVec]) { load_activation_part<0, kMaxVec>(p, m, v); }
 
 // Applies the fused transform to the vector load_activation fetched and returns max |x| over it.  `scratch` needs 32 floats.
 __device__ __forceinline__ float transform_activation(const ProIn &p, int m, float4 (&v)[kMaxVec], const uint2 (&wpre)[kPreVec], float *scratch)

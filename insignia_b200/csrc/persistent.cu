@@ -614,7 +614,7 @@ __global__ void __launch_bounds__(kThreads, 1) persistent_token_kernel(const __g
                 const int nph = ph + 1 < a.nphases ? ph + 1 : 0;
                 const bool more = step + 1 < total;
                 const bool chain = more && prog[nph].type == PH_GEMV;
-                const int xstride = p.cols + 8;
+                const int xstride = p.cols + kXPad;
                 __half *xs = reinterpret_cast<__half *>(work);
                 float *rec = reinterpret_cast<float *>(work + size_t(2) * xstride * sizeof(__half));
                 float *scratch = rec + size_t(kWarps) * p.slots * 16;
@@ -801,11 +801,11 @@ int insg_program_finalize(insg_program *g)
         g->phases[i].next_gemv = next;
         if (g->phases[i].type == PH_GEMV) next = i;
     }
-    cudaError_t e = cudaFuncSetAttribute(persistent_token_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(persistent_token_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(persistent)");
     g->smem = std::max<size_t>(g->smem, 1024);
     g->prog_bytes = (g->phases.size() * sizeof(Phase) + 127) / 128 * 128;
-    if (g->prog_bytes + g->smem > 220 * 1024)
+    if (g->prog_bytes + g->smem > size_t(kMaxSmem))
         return fail(INSG_E_LIMIT, "program: too many operations for the shared-memory copy of the program (about 180 with full-size GEMVs)");
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_token_kernel, kThreads, g->prog_bytes + g->smem);
