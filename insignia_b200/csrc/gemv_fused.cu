@@ -184,7 +184,9 @@ int gemv_fused_launch(const insg_gemv_op *op, int M, cudaStream_t st)
     if (rc != INSG_OK) return rc;
     const bool pdl = op->pdl != 0;
     switch (M) {
-    case 1: return launch_variant<kUnr, 1>(p, grid, smem, st, pdl);
+    case 1: // one token with many records a warp (the head: 209) has registers and time for deeper chunks, 108 -> 104 us; at 21 a warp they lose
+        if (p.total_units / (grid * kWarps) >= 64) return launch_variant<kUnr + 1, 1>(p, grid, smem, st, pdl);
+        return launch_variant<kUnr, 1>(p, grid, smem, st, pdl);
     case 2: return launch_variant<kUnr, 2>(p, grid, smem, st, pdl);
     case 3: return launch_variant<kUnr, 3>(p, grid, smem, st, pdl);
     default: return launch_variant<kUnr, 4>(p, grid, smem, st, pdl);
