@@ -252,21 +252,27 @@ __device__ __forceinline__ float prologue(const GemvParams &p, const ProIn &pin,
     return __uint_as_float(uint32_t(eb - 12) << 23);
 }
 
-// All tokens; the next one's first vectors (4096 columns) are asked for before this one's reductions.
+// All tokens; the next one's first vectors (4096 columns) are asked for before this one's reductions.  From three
+// tokens on a loop on purpose: unrolled, every token ran its own copy of the code for the first and only time, and waited
+// for it (4096 x 4096 with four tokens 15.6 -> 11.4 us).  The factors go through scratch[60 + m], read behind the caller's barrier.
 template <int M>
 __device__ __forceinline__ void prologue_tokens(const GemvParams &p, const ProIn &pin, __half *xs, int xstride, const uint2 (&wpre)[kPreVec],
-                                                float *scratch, float (&inv_alpha)[M])
+                                                float *scratch)
 {
+    constexpr bool kAhead = M < 4; // four tokens: the registers are the weights'
     float4 next[kPreVec];
-    load_activation_part<0, kPreVec>(pin, 0, next);
-#pragma unroll
+    if (kAhead) load_activation_part<0, kPreVec>(pin, 0, next);
+#pragma unroll (M > 2 ? 1 : M)
     for (int m = 0; m < M; m++) {
         float4 v[kMaxVec];
+        if (kAhead) {
 #pragma unroll
-        for (int j = 0; j < kPreVec; j++) v[j] = next[j];
-        load_activation_part<kPreVec, kMaxVec>(pin, m, v);
-        if (m + 1 < M) load_activation_part<0, kPreVec>(pin, m + 1, next);
-        inv_alpha[m] = prologue(p, pin, m, v, xs, xstride, wpre, scratch);
+            for (int j = 0; j < kPreVec; j++) v[j] = next[j];
+        }
+        load_activation_part<kAhead ? kPreVec : 0, kMaxVec>(pin, m, v);
+        if (kAhead && m + 1 < M) load_activation_part<0, kPreVec>(pin, m + 1, next);
+        const float inv = prologue(p, pin, m, v, xs, xstride, wpre, scratch);
+        if (threadIdx.x == 0) scratch[60 + m] = inv;
     }
 }
 
@@ -276,6 +282,7 @@ __device__ __forceinline__ void gemv_activation(const GemvParams &p, __half *xs,
                                                 float (&inv_alpha)[M])
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    bool fetched = false; // CTA-uniform: prologue_tokens ran
     if (p.prologue == INSG_PRO_PREPARED) {
         // The producer left both fp16 pieces ready: copy them (16-byte asynchronous copies through L2, no registers,
         // no reductions) and fold the RMS factor, when there is one, into the output scale.
@@ -309,16 +316,22 @@ __device__ __forceinline__ void gemv_activation(const GemvParams &p, __half *xs,
             const ProIn q{p.aux, nullptr, p.norm_w, p.x_out, p.cols, p.norm_w ? INSG_PRO_RMSNORM : INSG_PRO_PLAIN};
             preload_norm_weights(q, wpre);
             __syncthreads(); // every thread has read scratch[1]
-            prologue_tokens<M>(p, q, xs, xstride, wpre, scratch, inv_alpha);
+            prologue_tokens<M>(p, q, xs, xstride, wpre, scratch);
+            fetched = true;
         } else {
 #pragma unroll
             for (int m = 0; m < M; m++) inv_alpha[m] = scratch[0];
         }
     } else {
         const ProIn pin{p.in, p.aux, p.norm_w, p.x_out, p.cols, p.prologue};
-        prologue_tokens<M>(p, pin, xs, xstride, wpre, scratch, inv_alpha);
+        prologue_tokens<M>(p, pin, xs, xstride, wpre, scratch);
+        fetched = true;
     }
     __syncthreads();
+    if (fetched) {
+#pragma unroll
+        for (int m = 0; m < M; m++) inv_alpha[m] = scratch[60 + m];
+    }
 }
 
 // The two fp16 pieces of v * w / 16 (see kPrepScale) into a prepared image of `rows` elements.
@@ -388,8 +401,8 @@ __device__ __forceinline__ void row_epilogue(const SegDev &s, int row, int m, fl
 // one token spreads its column pairs over the groups and scales one group per lane.  Reading a group per thread
 // (16-byte loads) leaves the groups to the columns, eight multiplies per token on three quarters of zeros; exchanging its
 // words within the quad instead costs sixteen selects a record on that same pipe.  Microseconds from 16-byte loads, tokens 1..4:
-// 12352 x 4096 11.7, 14.2, 28 (two launches; 20 in one), 26.8 -> 11.5, 13.3, 16.5, 19.7; 248320 x 4096 107, 129, 238, 241 -> 109,
-// 118, 125, 130 (4.1 TB/s and more).
+// 12352 x 4096 11.7, 14.2, 28 (two launches; 20 in one), 26.8 -> 11.6, 13.5, 15.4, 15.8; 248320 x 4096 107, 129, 238, 241 -> 105,
+// 118, 123, 122 (4.4 TB/s).
 template <int UNR, int M>
 __device__ __forceinline__ void gemv_stream(const GemvParams &p, const GemvRange &r, Chunk<UNR> &A, Chunk<UNR> &B, UnitIt &lit,
                                             const __half *xs, int xstride, float *wrec, const float (&inv_alpha)[M], int lane)
