@@ -317,11 +317,12 @@ static int check_launch(const char *what)
 }
 
 // A cluster of eight CTAs takes a row (a row of logits is a megabyte: one CTA read it in 37 us); the CTAs' winners meet in
-// the first one's shared memory.
+// the first one's shared memory, which may be written once that CTA has started: the barrier all of them arrive at on entry.
 __global__ void __cluster_dims__(kArgmaxCtas, 1, 1) __launch_bounds__(512) argmax_rows_kernel(const float *x, long long stride, int n, int *out)
 {
     __shared__ float sv[16], cv[kArgmaxCtas];
     __shared__ int si[16], ci[kArgmaxCtas];
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     const int rank = blockIdx.x % kArgmaxCtas;
     x += size_t(blockIdx.x / kArgmaxCtas) * stride;
     float best = -3.402823466e38f;
@@ -337,6 +338,7 @@ __global__ void __cluster_dims__(kArgmaxCtas, 1, 1) __launch_bounds__(512) argma
     for (int m = 16; m; m >>= 1) take(__shfl_xor_sync(0xffffffffu, best, m), __shfl_xor_sync(0xffffffffu, idx, m));
     if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = best; si[threadIdx.x >> 5] = idx; }
     __syncthreads();
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
     if (threadIdx.x == 0) {
         for (int w = 1; w < 16; w++) take(sv[w], si[w]);
         uint32_t v, i;
