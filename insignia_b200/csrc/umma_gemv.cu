@@ -85,13 +85,15 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t saddr, uint32_t rank)
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
-// The arrivals below order no global store: a release at cluster scope waits until the epilogue's earlier stores have been
-// acknowledged, which a stream of weights makes slow (one token 1214 -> 1189 us, lm_head with four tokens 145 -> 87 us).  Slots are
-// handed back after they have been read, and the closing barrier only keeps CTAs from leaving early.
+// The closing barrier only keeps CTAs from leaving early.  A release there would wait until the epilogue's global stores have been
+// acknowledged, which a stream of weights makes slow (one token 1214 -> 1189 us, lm_head with four tokens 145 -> 87 us).
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+// Hands an exchange slot back to another CTA, whose next st.async must come after this CTA's reads of it: a release at cluster
+// scope, restricted to shared memory, so that it waits for none of those stores either.
 __device__ __forceinline__ void remote_arrive(uint32_t bar)
 {
-    asm volatile("mbarrier.arrive.release.cta.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+    asm volatile("fence.release.sync_restrict::shared::cta.cluster;\n"
+                 "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // T floats to another CTA's shared memory; their bytes complete on that CTA's barrier.
 template <int T> __device__ __forceinline__ void send_floats(uint32_t dst, const float (&v)[T], uint32_t bar)
