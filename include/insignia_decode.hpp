@@ -144,6 +144,7 @@ private:
     void build_program();
     void run_program(int n_tokens, int token);
     void recover_after_timeout();
+    void check_status(int flag);
     bool persistent() const;
     uint64_t launches_{};
     bool gemv_only_{};            // enqueue only the fused GEMVs (profile_gemv_chain)

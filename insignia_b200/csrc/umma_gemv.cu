@@ -674,6 +674,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                     for (int w = 1; w < 4; w++)
                         if (s_best[w] > best || (s_best[w] == best && s_bidx[w] < best_idx)) { best = s_best[w]; best_idx = s_bidx[w]; }
                     p.argmax_partial[blockIdx.x] = make_float2(best, __int_as_float(best_idx));
+                    if (*abort_flag && p.error_flag) *p.error_flag = 1; // ahead of the ticket: the last CTA reports for all of them
                     __threadfence();
                     s_last = atomicAdd(p.argmax_ticket, 1u) == gridDim.x - 1;
                 }
@@ -693,7 +694,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                         if (p.token_feedback) *p.token_feedback = best_idx;
                         if (p.host_result) { // a host that waits for the stream needs no copy behind it
                             p.host_result[0] = best_idx;
-                            p.host_result[1] = p.error_flag ? __ldcg(p.error_flag) | (s_abort != 0) : 0;
+                            p.host_result[1] = p.error_flag ? __ldcg(p.error_flag) : 0;
                         }
                         if (p.position_inout) {
                             const int pos = __ldcg(p.position_inout);

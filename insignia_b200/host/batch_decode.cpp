@@ -376,7 +376,9 @@ void Qwen35BatchDecode::generate(const int *first_tokens, int count, int *out)
     for (int i = 0; i < count; i++) run_step(); // each step's commit feeds the next
     std::vector<int> log(size_t(count) * m.B);
     cuda_check(cudaMemcpyAsync(log.data(), m.d_log + size_t(start) * m.B, log.size() * sizeof(int), cudaMemcpyDeviceToHost, m.stream), "read tokens");
+    cuda_check(cudaMemcpyAsync(m.host_tokens + m.B + 1, m.d_error, sizeof(int), cudaMemcpyDeviceToHost, m.stream), "read status");
     cuda_check(cudaStreamSynchronize(m.stream), "synchronize");
+    if (m.host_tokens[m.B + 1]) throw std::runtime_error("a bounded wait inside a GPU kernel expired");
     for (int i = 0; i < count; i++)
         for (int s = 0; s < sequences_; s++) out[size_t(i) * sequences_ + s] = log[size_t(i) * m.B + s];
 }

@@ -153,7 +153,7 @@ struct Qwen35Decode::Plan {
     cudaKernelNodeParams scalars_params{};
     cudaGraphExec_t exec_multi{}; // kMultiSteps token steps in one graph, for device-fed generation
     cudaGraphExec_t exec_chunk{}; // one pass of forward_tokens over kChunk prompt tokens
-    int *host_result{}; // pinned: {next token, wait-expired flag, the two results of a verify pass}, so the per-token read-back is a true asynchronous copy
+    int *host_result{}; // pinned: {next token, wait-expired flag, the two results of a verify pass, its flag}, so the per-token read-back is a true asynchronous copy
     float *spec_state{}, *spec_conv{}, *spec_logits{}; // speculative decode: second DeltaNet state, convolution snapshot, [2][vocab] logits
     int *spec_pair{};                                  // device: the two arg-max results of a verify pass
     int *spec_host{};                                  // pinned: {token, draft} on the way in
@@ -202,7 +202,7 @@ Qwen35Decode::Plan &Qwen35Decode::plan()
             cuda_check(cudaStreamCreateWithFlags(&plan_->stream, cudaStreamDefault), "cudaStreamCreate");
             plan_->own_stream = true;
         }
-        cuda_check(cudaMallocHost(&plan_->host_result, 4 * sizeof(int)), "cudaMallocHost");
+        cuda_check(cudaMallocHost(&plan_->host_result, 5 * sizeof(int)), "cudaMallocHost");
     }
     return *plan_;
 }
@@ -1073,6 +1073,13 @@ void Qwen35Decode::recover_after_timeout()
     fused_token_valid_ = false;
 }
 
+void Qwen35Decode::check_status(int flag)
+{
+    if (!flag) return;
+    recover_after_timeout();
+    throw std::runtime_error("a bounded wait inside a GPU kernel expired");
+}
+
 int Qwen35Decode::logits_argmax()
 {
     Plan &p = plan();
@@ -1087,10 +1094,7 @@ int Qwen35Decode::logits_argmax()
         cuda_check(cudaMemcpyAsync(result, x_.d_next, 2 * sizeof(int), cudaMemcpyDeviceToHost, p.stream), "read token");
     }
     cuda_check(cudaStreamSynchronize(p.stream), "synchronize");
-    if (result[1]) {
-        recover_after_timeout();
-        throw std::runtime_error("a bounded wait inside a GPU kernel expired");
-    }
+    check_status(result[1]);
     return result[0];
 }
 
@@ -1108,22 +1112,21 @@ std::vector<int> Qwen35Decode::generate(int first_token, int count)
     if (x_.position + count > x_.max_context) throw std::runtime_error("KV cache full");
     Plan &p = plan();
     const int start = x_.position;
+    auto read_log = [&] {
+        int *flag = p.host_result + 1;
+        cuda_check(cudaMemcpyAsync(out.data(), x_.d_token + 4 + start, size_t(count) * sizeof(int), cudaMemcpyDeviceToHost, p.stream),
+                   "read tokens");
+        cuda_check(cudaMemcpyAsync(flag, x_.d_token + 3, sizeof(int), cudaMemcpyDeviceToHost, p.stream), "read status");
+        cuda_check(cudaStreamSynchronize(p.stream), "synchronize");
+        check_status(*flag);
+    };
     if (persistent()) {
         // the kernel loops over the tokens itself: the head feeds its arg-max back and advances the position
         run_program(count, first_token);
         x_.position += count;
         fused_token_valid_ = true;
         result_on_host_ = false;
-        int *flag = p.host_result + 1;
-        *flag = 0;
-        cuda_check(cudaMemcpyAsync(out.data(), x_.d_token + 4 + start, size_t(count) * sizeof(int), cudaMemcpyDeviceToHost, p.stream),
-                   "read tokens");
-        cuda_check(cudaMemcpyAsync(flag, x_.d_token + 3, sizeof(int), cudaMemcpyDeviceToHost, p.stream), "read status");
-        cuda_check(cudaStreamSynchronize(p.stream), "synchronize");
-        if (*flag) {
-            recover_after_timeout();
-            throw std::runtime_error("a bounded wait inside a GPU kernel expired");
-        }
+        read_log();
         return out;
     }
     sync_scalars(first_token);
@@ -1144,9 +1147,7 @@ std::vector<int> Qwen35Decode::generate(int first_token, int count)
     }
     fused_token_valid_ = true;
     result_on_host_ = false;
-    cuda_check(cudaMemcpyAsync(out.data(), x_.d_token + 4 + start, size_t(count) * sizeof(int), cudaMemcpyDeviceToHost, p.stream),
-               "read tokens");
-    cuda_check(cudaStreamSynchronize(p.stream), "synchronize");
+    read_log();
     return out;
 }
 
@@ -1431,15 +1432,11 @@ std::vector<int> Qwen35Decode::generate_speculative(int first_token, int count, 
         });
         int *res = p.host_result + 2;
         cuda_check(cudaMemcpyAsync(res, p.spec_pair, 2 * sizeof(int), cudaMemcpyDeviceToHost, p.stream), "read tokens");
+        cuda_check(cudaMemcpyAsync(res + 2, x_.d_token + 3, sizeof(int), cudaMemcpyDeviceToHost, p.stream), "read status"); // the draft's and the pass's
         cuda_check(cudaStreamSynchronize(p.stream), "synchronize");
+        check_status(res[2]);
         const int r1 = res[0], r2 = res[1];
-        if (ahead) { // the MTP head left its result in pinned memory
-            draft = p.host_result[0];
-            if (p.host_result[1]) {
-                recover_after_timeout();
-                throw std::runtime_error("a bounded wait inside a GPU kernel expired");
-            }
-        }
+        if (ahead) draft = p.host_result[0]; // the MTP head left its result in pinned memory
         out.push_back(r1);
         if (r1 == draft) { // accepted: both positions stand
             hits++;
