@@ -164,8 +164,8 @@ __device__ __forceinline__ void attn_mma_warp(const void *kc, const void *vc, in
 // Clusters: a kv head's cache is cut over clusters of CL CTAs.  The CTAs of a cluster exchange their partial results through
 // distributed shared memory, each finishing its share of the output dims: a context that one cluster holds needs no global
 // scratch, fence or ticket.  Longer ones use up to `clusters` clusters per head; their results go to scratch and the last one
-// to arrive (a ticket per CTA rank) folds them in order.  The cut depends on the row count alone, so that a token gives the
-// same bits in a single step, a chunk or a batch whenever those launch the same clusters.
+// to arrive (a ticket per CTA rank) folds them in order.  For one launch's clusters the cut depends on the row count alone; the
+// clusters on the cache's type and capacity and, in a batch, on how many sequences share the device (launch_attn).
 // Measured (fp32 cache, one step): 40 rows 5.2 us (7.1 with one CTA per split and a ticket), 8 x 600 rows 13.5 (38.5),
 // 8 x 5000 rows 57 (119.5, 88 % of the copy peak); 1024 rows 9.9 (9.5).
 constexpr int kCtaRows = 48;    // rows per CTA from which another cluster is put to work (32, 48, 64, 96 tried: 48 is best or next to it)
@@ -542,27 +542,34 @@ template <bool BF16, bool FUSED, int CL, bool HALVES = false> static int launch_
     return e == cudaSuccess ? INSG_OK : cuda_fail(e, "attention launch");
 }
 
-// `along`: tokens of a chunk or sequences of a batch (grid rows); rows: an upper bound of the rows attended, when known.  As many
-// clusters as the device runs at once: 33 of eight CTAs at two per SM, or 33 of four at one (with the tensor-core loop's tiles),
-// shared by the four heads of every grid row.  Where that leaves SMs idle (three sequences or more, not a power of two) and the
+// `along`: tokens of a chunk or sequences of a batch (grid rows); rows: an upper bound of the rows attended, when known.
+//
+// The tokens of a chunk (the plain form) are cut as single steps are, whatever travels along, so that they have their bits: a
+// verify pass must not draw another token than plain decode.  CTAs beyond those that run at once take their turn; clusters without
+// rows cost a two-token verify pass on a 2560-row cache 13 us of 1690.
+//
+// The sequences of a batch share as many clusters as the device runs at once: 33 of eight CTAs at two per SM, or 33 of four at
+// one (with the tensor-core loop's tiles).  Where that leaves SMs idle (three sequences or more, not a power of two) and the
 // contexts can be long, the fp32 cache goes to clusters of four too.  Where contexts are short and the
 // CTAs more than one and a half per SM (seven sequences or more), a second CTA finds no registers beside the products' launches
 // before and after: clusters of four find a place sooner than those of eight, and up to 128 rows one of the two has nothing to
 // do.  A step of eight sequences 1803 -> 1755 us at 20 rows and 1885 -> 1818 at 450 (alone the launch is 1.5 us slower there);
-// five sequences win at 20 rows and lose 12 us from 130 on.
+// five sequences win at 20 rows and lose 12 us from 130 on.  A chunk takes the pairs while one cluster holds its rows.
 constexpr int kLongContext = 2048;
 static_assert(kLongContext <= kMmaMinTokens, "short contexts never get to the tensor-core loop");
 template <bool BF16, bool FUSED> int launch_attn(const AttnParams &p, cudaStream_t st, bool pdl, int along = 1, int rows = 0)
 {
+    const int clusters = FUSED ? kMaxClusters / along : kMaxClusters;
     if (p.max_context < kLongContext) {
-        if (along > kMaxClusters / 2 && 2 * along * 4 * 8 > 3 * sm_count()) return launch_clusters<BF16, FUSED, 4, true>(p, st, pdl, along, rows, 2);
-        return launch_clusters<BF16, FUSED, 8>(p, st, pdl, along, rows, kMaxClusters / along);
+        const bool one_cluster = rows > 0 && rows <= kCtaRows * 8;
+        if ((FUSED || one_cluster) && along > kMaxClusters / 2 && 2 * along * 4 * 8 > 3 * sm_count()) return launch_clusters<BF16, FUSED, 4, true>(p, st, pdl, along, rows, 2);
+        return launch_clusters<BF16, FUSED, 8>(p, st, pdl, along, rows, clusters);
     }
     if constexpr (BF16) {
-        return launch_clusters<true, FUSED, 4>(p, st, pdl, along, rows, kMaxClusters / along);
+        return launch_clusters<true, FUSED, 4>(p, st, pdl, along, rows, clusters);
     } else {
-        if (along > 2 && (along & (along - 1))) return launch_clusters<false, FUSED, 4>(p, st, pdl, along, rows, 17 / along);
-        return launch_clusters<false, FUSED, 8>(p, st, pdl, along, rows, kMaxClusters / along);
+        if (FUSED && along > 2 && (along & (along - 1))) return launch_clusters<false, FUSED, 4>(p, st, pdl, along, rows, 17 / along);
+        return launch_clusters<false, FUSED, 8>(p, st, pdl, along, rows, clusters);
     }
 }
 
