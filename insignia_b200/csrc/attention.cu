@@ -712,6 +712,7 @@ int insg_attention_chunk(const insg_attn_op *op, int tokens, float *q_scratch, i
     if (tokens < 1 || tokens > 65535) return fail(INSG_E_SHAPE, "attention_chunk: 1 <= tokens <= 65535");
     if (tokens <= kTileFromTokens && op->scratch_bytes < size_t(tokens) * attn_scratch_bytes()) return fail(INSG_E_SHAPE, "attention_chunk: scratch too small");
     if (op->max_context <= 0) return fail(INSG_E_SHAPE, "attention_chunk: max_context");
+    if (op->image && tokens > 8) return fail(INSG_E_SHAPE, "attention_chunk: a digit image holds up to 8 tokens");
     AttnParams p = {};
     p.q = op->qraw; p.k_raw = op->k_raw; p.v_new = op->v; p.q_w = op->q_norm_w; p.k_w = op->k_norm_w;
     p.kc = op->k_cache; p.vc = op->v_cache; p.out = op->out;
@@ -724,7 +725,6 @@ int insg_attention_chunk(const insg_attn_op *op, int tokens, float *q_scratch, i
     // More than 32 tokens: query tiles on the tensor cores.  Fewer: the token-by-token form below, whose results are those of
     // single steps bit for bit (at 33 tokens the tile kernel still has only twelve CTAs; the two take the same time near 24).
     if (tokens > kTileFromTokens) return attn_tile_launch(p, q_scratch, tokens, bf16, stream, false);
-    if (op->image && tokens > 8) return fail(INSG_E_SHAPE, "attention_chunk: a digit image holds up to 8 tokens");
     set_image(p, op, tokens);
     // step two: every (kv head, split, token) CTA is the plain split-K decode of its token over the rows up to its own
     p.q = q_scratch; p.q_stride = 4096; p.out_stride = 4096; p.scratch_stride = attn_scratch_bytes();

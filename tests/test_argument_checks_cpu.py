@@ -1,0 +1,32 @@
+"""Calls that a kernel could not serve are refused before anything is launched (checked without a GPU: a launch would fail
+with another status)."""
+import ctypes as C
+import os
+import sys
+
+import pytest
+
+sys.path.insert(0, os.path.join(os.path.dirname(__file__), ".."))
+
+E_SHAPE, E_ARG = -1, -3
+SOME = 1 << 20  # a pointer nobody follows
+
+
+def attn_op(**kw):
+    from insignia_b200 import _lib
+
+    op = _lib.AttnOp()
+    for f in ("qraw", "k_raw", "v", "q_norm_w", "k_norm_w", "k_cache", "v_cache", "out", "position", "scratch"):
+        setattr(op, f, SOME)
+    op.max_context, op.scratch_bytes = 4096, 1 << 40
+    for k, v in kw.items():
+        setattr(op, k, v)
+    return op
+
+
+@pytest.mark.parametrize("tokens", [9, 32, 33, 512])
+def test_a_chunk_of_more_than_eight_tokens_has_no_image(tokens):
+    from insignia_b200 import _lib
+
+    assert _lib.lib().insg_attention_chunk(C.byref(attn_op(image=SOME)), tokens, SOME, 0, None) == E_SHAPE
+    assert b"digit image" in _lib.lib().insg_last_error()
