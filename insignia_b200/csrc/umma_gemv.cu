@@ -799,6 +799,7 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     p.in = op->in; p.aux = op->aux; p.norm_w = op->norm_w; p.x_out = op->x_out;
     p.cols = op->cols; p.prologue = op->prologue;
     if (op->prologue == INSG_PRO_PREPARED) {
+        if (op->prep_rms && !op->prep_partials) return fail(INSG_E_ARG, "gemv: the RMS factor of a prepared input needs the producer's sums");
         p.x_out = nullptr;
         p.prep_partials = op->prep_rms ? op->prep_partials : nullptr;
     }

@@ -30,3 +30,22 @@ def test_a_chunk_of_more_than_eight_tokens_has_no_image(tokens):
 
     assert _lib.lib().insg_attention_chunk(C.byref(attn_op(image=SOME)), tokens, SOME, 0, None) == E_SHAPE
     assert b"digit image" in _lib.lib().insg_last_error()
+
+
+def gemv_op(tokens=1, rows=256, cols=4096, prologue="plain", **kw):
+    from insignia_b200 import _lib, ops
+
+    op = _lib.GemvOp()
+    op.in_, op.cols, op.prologue, op.n_segments, op.layout, op.tokens = SOME, cols, ops.PRO[prologue], 1, 1, tokens
+    op.seg[0].packed, op.seg[0].out, op.seg[0].rows = SOME, SOME, rows
+    for k, v in kw.items():
+        setattr(op, k, v)
+    return op
+
+
+@pytest.mark.parametrize("tokens", [1, 8])
+def test_the_rms_factor_of_a_prepared_input_needs_its_sums(tokens):
+    from insignia_b200 import _lib
+
+    assert _lib.lib().insg_gemv_fused(C.byref(gemv_op(tokens, prologue="prepared", prep_rms=1)), None) == E_ARG
+    assert b"sums" in _lib.lib().insg_last_error()
