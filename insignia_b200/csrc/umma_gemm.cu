@@ -748,6 +748,7 @@ int insg_mxfp4_gemm_umma(const void *packed_umma, const float *x, float *y, int 
     op.layout = 1;
     op.umma_scratch = scratch;
     op.umma_scratch_bytes = scratch_bytes;
+    if (M < 1) return fail(INSG_E_SHAPE, "gemm: 1 <= tokens <= 4096");
     return M <= 8 ? gemv_umma_launch(&op, stream) : gemm_umma_launch(&op, stream);
 }
 

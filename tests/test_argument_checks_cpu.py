@@ -49,3 +49,10 @@ def test_the_rms_factor_of_a_prepared_input_needs_its_sums(tokens):
 
     assert _lib.lib().insg_gemv_fused(C.byref(gemv_op(tokens, prologue="prepared", prep_rms=1)), None) == E_ARG
     assert b"sums" in _lib.lib().insg_last_error()
+
+
+@pytest.mark.parametrize("tokens", [0, -1, 4097])
+def test_a_product_takes_1_to_4096_tokens(tokens):
+    from insignia_b200 import _lib
+
+    assert _lib.lib().insg_mxfp4_gemm_umma(SOME, SOME, SOME, 256, 4096, tokens, SOME, 1 << 40, None) == E_SHAPE
