@@ -119,29 +119,38 @@ __device__ __forceinline__ void pack_digits(float4 x, float alpha, const uint8_t
     }
 }
 
+// ---- a group of 32 elements: its scale from its largest magnitude -------------------------------------------------------------
+// Infinities and NaN have no digits: the scale byte 255 is the format's NaN, and makes every product with the group NaN.
+__device__ __forceinline__ float fmax_nan(float a, float b) // NaN where either is
+{
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ int group_exponent(uint32_t max_bits) { return max(int(max_bits >> 23), 24); } // bits of |.|: 255 = not finite
+__device__ __forceinline__ float group_alpha(int eb) { return __uint_as_float(uint32_t(277 - eb) << 23); }  // largest element * alpha in [2^23, 2^24)
+__device__ __forceinline__ uint8_t group_scale(int eb) { return uint8_t(eb == 255 ? 255 : eb - 23); }
+
 // ---- digit image of activation vectors: [k-block of 128][digits of T token slots: 512 T bytes | scale block: 512 bytes] ----
 // The digits of one 128-element k-block of one token (four elements per lane) into the B image, and their group scales.
 // Image of a k-block: [2 K-steps][T column groups][2 k cores][8 columns][16 B]; a token's eight digit columns are one group.
 __device__ __forceinline__ void store_digits(float4 x, int T, int m, uint8_t *bkb, const uint8_t *lut, int lane)
 {
-    float mx = fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w)));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1)); // a group of 32 elements = 8 lanes
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-    int eb = int((__float_as_uint(mx) >> 23) & 0xffu);
-    eb = min(max(eb, 24), 230);
-    const float alpha = __uint_as_float(uint32_t(277 - eb) << 23); // largest element * alpha in [2^23, 2^24)
-    pack_digits(x, alpha, lut, bkb + (lane >> 4) * (256 * T) + m * 256 + ((lane >> 3) & 1) * 128 + (lane & 7) * 2);
+    float mx = fmax_nan(fmax_nan(fabsf(x.x), fabsf(x.y)), fmax_nan(fabsf(x.z), fabsf(x.w)));
+    mx = fmax_nan(mx, __shfl_xor_sync(0xffffffffu, mx, 1)); // a group of 32 elements = 8 lanes
+    mx = fmax_nan(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    mx = fmax_nan(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+    const int eb = group_exponent(__float_as_uint(mx));
+    pack_digits(x, group_alpha(eb), lut, bkb + (lane >> 4) * (256 * T) + m * 256 + ((lane >> 3) & 1) * 128 + (lane & 7) * 2);
     const int n = 8 * m + (lane & 7); // scale block: row = column n of B (32 rows, then the next quarter), byte = group
-    bkb[512 * T + (n & 31) * 16 + (n >> 5) * 4 + (lane >> 3)] = uint8_t(eb - 23);
+    bkb[512 * T + (n & 31) * 16 + (n >> 5) * 4 + (lane >> 3)] = group_scale(eb);
 }
 
 // One element per lane: the warp's 32 lanes are the 32-element group `grp` of token slot m's vector.
 __device__ __forceinline__ void group_digits(float x, int T, int m, uint8_t *image, int grp, const uint8_t *lut, int lane)
 {
-    int eb = int(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(x))) >> 23);
-    eb = min(max(eb, 24), 230);
-    const uint32_t c = digit_codes81(x, __uint_as_float(uint32_t(277 - eb) << 23), lut), o = __shfl_xor_sync(0xffffffffu, c, 1);
+    const int eb = group_exponent(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(x))));
+    const uint32_t c = digit_codes81(x, group_alpha(eb), lut), o = __shfl_xor_sync(0xffffffffu, c, 1);
     // a pair of lanes holds two neighbouring k = one byte per column: the even lane stores columns 0, 2, 4, 6, the odd one the others
     const uint32_t b = (lane & 1) ? ((o >> 4) & 0x0F0F0F0Fu) | (c & 0xF0F0F0F0u) : (c & 0x0F0F0F0Fu) | ((o & 0x0F0F0F0Fu) << 4);
     const int g = grp & 3;
@@ -149,7 +158,7 @@ __device__ __forceinline__ void group_digits(float x, int T, int m, uint8_t *ima
 #pragma unroll
     for (int j = 0; j < 4; j++) dst[32 * j] = uint8_t(b >> (8 * j));
     const int n = 8 * m + (lane & 7);
-    if (lane < 8) kb[512 * T + (n & 31) * 16 + (n >> 5) * 4 + g] = uint8_t(eb - 23);
+    if (lane < 8) kb[512 * T + (n & 31) * 16 + (n >> 5) * 4 + g] = group_scale(eb);
 }
 // Token slots of an image of `tokens` (1..8) vectors.
 __host__ __device__ inline int image_slots(int tokens) { return tokens == 1 ? 1 : tokens == 2 ? 2 : tokens <= 4 ? 4 : 8; }
