@@ -4,10 +4,10 @@
 //
 // tcgen05.mma.kind::mxf4.block_scale, weights as the A operand in their native packed E2M1 + UE8M0 form (the tile layout of
 // insg_mxfp4_repack_umma, nothing dequantised), accumulators in tensor memory.  The activations are the B operand.
-// kind::mxf4 wants E2M1 there too, so each fp32 activation is written as a 25-bit signed fixed-point number (relative to its
-// token's largest element) in balanced base 9: eight digits -4..4, every one exact in E2M1.  Column j of a token holds digit
-// j of every element; the eight columns are combined as sum_j 9^j D_j in fp32 by the epilogue, which gives the product to
-// ~1e-7.  A token takes 8 columns of N.
+// kind::mxf4 wants E2M1 there too, so each fp32 activation is written as a 25-bit signed fixed-point number (relative to the
+// largest element of its group of 32, whose power of two is the group's UE8M0 scale) in balanced base 9: eight digits -4..4,
+// every one exact in E2M1, as in umma_gemv.cu.  Column j of a token holds digit j of every element; the eight columns are
+// combined as sum_j 9^j D_j in fp32 by the epilogue, which gives the product to ~1e-7.  A token takes 8 columns of N.
 //
 // What bounds it: filling shared memory.  A stage multiplies two 128-row weight records (17.4 KB) with the digits of a group
 // of tokens; an SM takes in some 52 bytes a clock from L2, and sixteen tokens' digits (8.2 KB, N = 128) left the tensor pipe
@@ -17,7 +17,7 @@
 // Kernels:
 //   umma_digitize_kernel  one CTA per token: the fused activation prologue (RMSNorm, gates, ...), then the digit
 //                         image of the token in global memory, laid out as the shared-memory image the MMA reads
-//                         ([k-block][group of tokens][512 bytes x tokens per group], canonical K-major, no swizzle);
+//                         ([k-block][group of tokens][512 bytes x tokens per group, scale blocks], canonical K-major, no swizzle);
 //   umma_gemm_kernel      one CTA per SM.  The work is the sequence of all (pair of records, token group, k-block) stages;
 //                         every CTA takes an equal contiguous share of it (stream-K), so SMs are busy whatever the number
 //                         of tiles.  The pair is two row tiles, or the gate and the up tile of the same rows for SwiGLU
@@ -44,10 +44,12 @@ constexpr int kGThreads = kProThreads;     // digitize kernel: the activation pr
 constexpr int kGemmThreads = 192;          // GEMM kernel: four epilogue warps, the MMA issuer, the producer
 constexpr int kDigits = 8;                 // balanced base-9 digits per activation = N columns per token
 constexpr int kGSfaBufs = 8;               // scale-factor column sets cycled by stage (a power of two)
-constexpr int kGTmemCols = 512;            // two accumulators of up to 192 columns, weight scale factors [384,448), digit scale factors [448,456)
+constexpr int kGTmemCols = 512;            // two accumulators of up to 192 columns, weight scale factors [384,448), digit scale factors [448,512)
 constexpr int kGMaxStages = 16;
 constexpr int kGMaxGrid = 256;             // partial-sum slots and tickets are sized for this many CTAs
 constexpr int kSlotFloats = 128 * 24;      // one partial: 128 rows x up to 24 tokens
+// A k-block of a token group in the digit image: the digits (8 columns x 64 bytes per token), then a 512-byte scale block per 128 columns.
+__host__ __device__ constexpr int digit_block(int tpg) { return 512 * tpg + (tpg + 15) / 16 * 512; }
 
 struct GSeg {
     const uint8_t *packed, *packed2;
@@ -61,8 +63,7 @@ struct GSeg {
 };
 
 struct GParams {
-    const uint8_t *bimg;    // [nkb][ngroups][512 * tpg]
-    const float *inv_alpha; // [ngroups * tpg]
+    const uint8_t *bimg;    // [nkb][ngroups][digit_block(tpg)]
     float *partials;        // [grid][2 cut units][2 records of the pair][128 rows][tpg]
     int *tickets;           // [grid], zero between launches
     int nkb, nseg, total_tiles, stages, ngroups, tokens;
@@ -74,58 +75,42 @@ struct GParams {
 struct DigitizeParams {
     ProIn pro;
     uint8_t *bimg;
-    float *inv_alpha;
     int *tickets;
     int tokens, ngroups, tpg, parts; // a token's digits are written by `parts` CTAs, each a slice of the columns
 };
 
 // `parts` CTAs per token slot (slots beyond `tokens` are written as zeros so that their columns contribute nothing).  Every
-// CTA of a token runs the whole prologue (the norm and the token's largest element need all columns; that part is a few
-// loads and one reduction) and writes the digits of its slice of the columns only: the digit extraction is the long part.
+// CTA of a token runs the whole prologue (the norm needs all columns; that part is a few loads and one reduction) and writes
+// the digits of its slice of the k-blocks only: the digit extraction is the long part.
 __global__ void __launch_bounds__(kGThreads, 2) umma_digitize_kernel(const __grid_constant__ DigitizeParams p)
 {
     __shared__ float scratch[64];
     __shared__ uint8_t lut[84];
-    if (threadIdx.x < 81) lut[threadIdx.x] = digit_pair_code(threadIdx.x); // read after the prologue's barriers
+    if (threadIdx.x < 81) lut[threadIdx.x] = digit_pair_code(threadIdx.x);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); // the GEMM may set itself up and fetch weights meanwhile
     const int m = blockIdx.x / p.parts, part = blockIdx.x - m * p.parts, grp = m / p.tpg, ms = m - grp * p.tpg;
-    const int tid = threadIdx.x;
-    const bool live = m < p.tokens;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float4 v[kMaxVec];
-    float alpha = 0.f;
-    if (live) {
+    if (m < p.tokens) {
         ProIn pin = p.pro;
         pin.x_out = nullptr;
         uint2 wpre[kPreVec];
         preload_norm_weights(pin, wpre);
         pdl_wait();
         load_activation(pin, m, v);
-        const float tmax = transform_activation(pin, m, v, wpre, scratch);
-        int eb = int((__float_as_uint(tmax) >> 23) & 0xffu);
-        eb = min(max(eb, 24), 230);
-        alpha = __uint_as_float(uint32_t(127 + 23 - (eb - 127)) << 23); // max * alpha in [2^23, 2^24)
-        if (tid == 0 && part == 0) p.inv_alpha[m] = __uint_as_float(uint32_t(eb - 23) << 23);
+        transform_activation<false>(pin, m, v, wpre, scratch);
     } else {
         pdl_wait();
 #pragma unroll
         for (int j = 0; j < kMaxVec; j++) v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (tid == 0 && part == 0) p.inv_alpha[m] = 0.f;
-        __syncthreads(); // the table
     }
+    __syncthreads(); // the table
     if (blockIdx.x == 0 && tid < kGMaxGrid) p.tickets[tid] = 0;
-    const int nvec = p.pro.cols >> 2;
-    const int block = 512 * p.tpg, kstep = 256 * p.tpg;
-    const int per = (nvec + p.parts - 1) / p.parts, v0 = part * per, v1 = min(nvec, v0 + per);
+    const int nkb = p.pro.cols >> 7, per = (nkb + p.parts - 1) / p.parts, kb0 = part * per, kb1 = min(nkb, kb0 + per);
 #pragma unroll
-    for (int j = 0; j < kMaxVec; j++) {
-        const int i = tid + j * kGThreads;
-        if (i >= v0 && i < v1) {
-            // 4 consecutive k -> 2 bytes per column.  Block image: [2 K-steps][tpg column groups][2 k cores][8 columns][16 B];
-            // the token's eight digit columns are one column group.
-            const int k = i << 2, kb = k >> 7, kk = k & 127;
-            const int half = (kk & 63) >> 1; // byte index of these k inside the 32-byte row of a K-step
-            pack_digits(v[j], alpha, lut, p.bimg + (size_t(kb) * p.ngroups + grp) * block + (kk >> 6) * kstep + ms * 256 + (half >> 4) * 128 + (half & 15));
-        }
+    for (int j = 0; j < kMaxVec; j++) { // a warp holds a k-block per j
+        const int kb = warp + j * (kGThreads / 32);
+        if (kb >= kb0 && kb < kb1) store_digits<true>(v[j], p.tpg, ms, p.bimg + (size_t(kb) * p.ngroups + grp) * digit_block(p.tpg), lut, lane);
     }
 }
 
@@ -208,13 +193,12 @@ __device__ __forceinline__ GRun run_at(const GParams &p, int g, int end)
     return r;
 }
 
-// The fused epilogue of one row for the tokens of one group; y[] are finished sums (before the per-token scale).
+// The fused epilogue of one row for the tokens of one group; y[] are finished sums.
 // Everything stays in registers (fully unrolled, predicated): with nearly all of the SM's memory configured as shared
 // memory, the little L1 that is left cannot hold a stack frame per thread, and spilled arrays would go to L2 and back.
 // The switch sits outside the token loops so that a launch runs through one short straight-line piece only.
 template <int TPG>
-__device__ __forceinline__ void finish_row(const GParams &p, const GSeg &s, int row, int grp, const float (&y)[TPG], const float (&gate)[TPG],
-                                           const float (&ia)[TPG])
+__device__ __forceinline__ void finish_row(const GParams &p, const GSeg &s, int row, int grp, const float (&y)[TPG], const float (&gate)[TPG])
 {
     const int m0 = grp * TPG, live = min(TPG, p.tokens - m0);
     float *out = s.out + size_t(m0) * s.rows + row;
@@ -226,7 +210,7 @@ __device__ __forceinline__ void finish_row(const GParams &p, const GSeg &s, int 
         for (int t = 0; t < TPG; t++) r[t] = t < live ? __ldcg(out + t * ld) : 0.f;
 #pragma unroll
         for (int t = 0; t < TPG; t++)
-            if (t < live) out[t * ld] = r[t] + y[t] * ia[t];
+            if (t < live) out[t * ld] = r[t] + y[t];
         break;
     }
     case INSG_EPI_CONV_SILU:
@@ -238,7 +222,7 @@ __device__ __forceinline__ void finish_row(const GParams &p, const GSeg &s, int 
             for (int t = 0; t < TPG; t++) {
                 if (t < live) {
                     float *st = s.conv_state + size_t(m0 + t) * s.conv_stride + size_t(row) * 3;
-                    const float h0 = __ldcg(st), h1 = __ldcg(st + 1), h2 = __ldcg(st + 2), yv = y[t] * ia[t];
+                    const float h0 = __ldcg(st), h1 = __ldcg(st + 1), h2 = __ldcg(st + 2), yv = y[t];
                     st[0] = h1; st[1] = h2; st[2] = yv;
                     out[t * ld] = fast_silu(fmaf(h0, cw0, fmaf(h1, cw1, fmaf(h2, cw2, yv * cw3))));
                 }
@@ -250,18 +234,18 @@ __device__ __forceinline__ void finish_row(const GParams &p, const GSeg &s, int 
     case INSG_EPI_STORE:
 #pragma unroll
         for (int t = 0; t < TPG; t++)
-            if (t < live) out[t * ld] = y[t] * ia[t];
+            if (t < live) out[t * ld] = y[t];
         break;
     case INSG_EPI_BETA:
 #pragma unroll
         for (int t = 0; t < TPG; t++)
-            if (t < live) out[t * ld] = fast_sigmoid(y[t] * ia[t]);
+            if (t < live) out[t * ld] = fast_sigmoid(y[t]);
         break;
     case INSG_EPI_DECAY: {
         const float bias = bf16_bits_to_float(s.dt_bias[row]), a = -__expf(s.A_log[row]);
 #pragma unroll
         for (int t = 0; t < TPG; t++) {
-            const float z = y[t] * ia[t] + bias;
+            const float z = y[t] + bias;
             if (t < live) out[t * ld] = a * (z > 20.f ? z : log1pf(__expf(z)));
         }
         break;
@@ -269,7 +253,7 @@ __device__ __forceinline__ void finish_row(const GParams &p, const GSeg &s, int 
     case INSG_EPI_SWIGLU:
 #pragma unroll
         for (int t = 0; t < TPG; t++)
-            if (t < live) out[t * ld] = fast_silu(gate[t] * ia[t]) * (y[t] * ia[t]);
+            if (t < live) out[t * ld] = fast_silu(gate[t]) * y[t];
         break;
     default: break;
     }
@@ -340,15 +324,14 @@ template <int TPG, bool SWIGLU>
 __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid_constant__ GParams p)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
-    constexpr int kBBlock = 512 * TPG;              // digits of the group's tokens for one k-block: 8 * TPG columns x 128 k x 4 bit
+    constexpr int kBBlock = digit_block(TPG);       // digits of the group's tokens for one k-block: 8 * TPG columns x 128 k x 4 bit, and their scales
     constexpr int kGStage = 2 * kURec + kBBlock;    // one ring stage: the pair's weight records + the digit block both multiply
     constexpr int N = kDigits * TPG;
     constexpr uint32_t kSfaCol = 384, kSfbCol = 448;
-    static_assert(2 * N <= int(kSfaCol) && 8 * kGSfaBufs == int(kSfbCol - kSfaCol), "tensor memory");
+    static_assert(2 * N <= int(kSfaCol) && 8 * kGSfaBufs == int(kSfbCol - kSfaCol) && kSfbCol + 8 * kGSfaBufs == uint32_t(kGTmemCols), "tensor memory");
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int nkb = p.nkb, S = p.stages;
     uint8_t *ring = smem;                          // S stages of kGStage bytes
-    uint8_t *sfb = ring + size_t(S) * kGStage;     // 512 bytes
     __shared__ __align__(8) uint64_t full[kGMaxStages], empty[kGMaxStages], dfull, dempty;
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort, s_last;
@@ -367,9 +350,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(kGTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
-    // column block scales: all 1 (the digit weights 9^j are not powers of two; the epilogue applies them)
-    if (tid < 128) reinterpret_cast<uint32_t *>(sfb)[tid] = 0x7F7F7F7Fu;
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -431,13 +411,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
         // stage's barrier is polled before this stage's multiplies go out.
         const bool one = elect_one();
         asm volatile("griddepcontrol.wait;" ::: "memory");
-        // E2M1 x E2M1, UE8M0 scales, N columns, M = 128; K-step s of a block uses the weight scale bytes 2s, 2s+1 and byte 0 of the digits' (all equal)
+        // E2M1 x E2M1, UE8M0 scales, N columns, M = 128; K-step s of a block uses scale bytes 2s, 2s+1 of both operands
         constexpr uint32_t idesc0 = (1u << 7) | (1u << 10) | ((uint32_t(N) >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
-        constexpr uint32_t idesc1 = idesc0 | (2u << 29);
-        if (one) { // 128 columns' scales per copy
-            copy_scales(tmem + kSfbCol, umma_desc(smem_u32(sfb), 16, 128));
-            if (N > 128) copy_scales(tmem + kSfbCol + 4, umma_desc(smem_u32(sfb), 16, 128));
-        }
+        constexpr uint32_t idesc1 = idesc0 | (2u << 29) | (2u << 4);
         const uint64_t da0 = umma_desc(smem_u32(ring), 128, 256), dsf0 = umma_desc(smem_u32(ring) + 8192, 16, 128);
         const uint32_t d0 = tmem, d1 = tmem + uint32_t(N);
         int st = 0, sfa = 0;
@@ -455,17 +431,20 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t off = uint64_t(uint32_t(st) * uint32_t(kGStage >> 4));
                 const uint64_t da = da0 + off, dsf = dsf0 + off, db = da + uint64_t((2 * kURec) >> 4);
-                const uint32_t sa = tmem + kSfaCol + 8 * sfa;
+                const uint32_t sa = tmem + kSfaCol + 8 * sfa, sb = tmem + kSfbCol + 8 * sfa;
                 const int cur = st;
                 if (++st == S) { st = 0; phase ^= 1; }
                 here = mbar_test(&full[st], phase);
                 if (one) {
                     copy_scales(sa, dsf);
                     if (has1) copy_scales(sa + 4, dsf + (kURec >> 4));
-                    mma_step(d0, da, db, idesc0, k > 0, sa, tmem + kSfbCol); // the run's first MMA overwrites
-                    if (has1) mma_step(d1, da + (kURec >> 4), db, idesc0, k > 0, sa + 4, tmem + kSfbCol);
-                    mma_step(d0, da + 256, db + (kBBlock >> 5), idesc1, true, sa, tmem + kSfbCol);
-                    if (has1) mma_step(d1, da + (kURec >> 4) + 256, db + (kBBlock >> 5), idesc1, true, sa + 4, tmem + kSfbCol);
+                    const uint64_t dsb = dsf + uint64_t((2 * kURec - 8192 + 512 * TPG) >> 4); // 128 columns' scales per copy
+                    copy_scales(sb, dsb);
+                    if (N > 128) copy_scales(sb + 4, dsb + 32);
+                    mma_step(d0, da, db, idesc0, k > 0, sa, sb); // the run's first MMA overwrites
+                    if (has1) mma_step(d1, da + (kURec >> 4), db, idesc0, k > 0, sa + 4, sb);
+                    mma_step(d0, da + 256, db + 16 * TPG, idesc1, true, sa, sb);
+                    if (has1) mma_step(d1, da + (kURec >> 4) + 256, db + 16 * TPG, idesc1, true, sa + 4, sb);
                     commit_to(&empty[cur]);
                 }
                 sfa = (sfa + 1) & (kGSfaBufs - 1);
@@ -475,7 +454,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
         }
     } else {
         // ---- epilogue: tensor-memory lane = row of the tile; token t of the group = columns 8t .. 8t+7 --------------------
-        asm volatile("griddepcontrol.wait;" ::: "memory"); // per-token scales, residual inputs and tickets come from earlier launches
+        asm volatile("griddepcontrol.wait;" ::: "memory"); // residual inputs and tickets come from earlier launches
         bool ok = true;
         int g = begin;
         for (int run = 0; g < end && ok; run++) {
@@ -558,16 +537,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
 #pragma unroll
                 for (int t = 0; t < TPG; t++) { y[0][t] = acc[0][t]; y[1][t] = acc[1][t]; }
             }
-            float ia[TPG]; // the group's per-token scales
-#pragma unroll
-            for (int t = 0; t < TPG; t += 4) {
-                const float4 q = __ldcg(reinterpret_cast<const float4 *>(p.inv_alpha + grp * TPG) + (t >> 2));
-                ia[t] = q.x; ia[t + 1] = q.y; ia[t + 2] = q.z; ia[t + 3] = q.w;
-            }
             if constexpr (SWIGLU) {
                 const GSeg &s = p.seg[gseg_of(p, pair)];
                 const int row = (pair - s.tile_begin) * 128 + tid;
-                if (row < s.rows) finish_row<TPG>(p, s, row, grp, y[1], y[0], ia);
+                if (row < s.rows) finish_row<TPG>(p, s, row, grp, y[1], y[0]);
             } else {
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
@@ -575,7 +548,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
                     const int tile = 2 * pair + h;
                     const GSeg &s = p.seg[gseg_of(p, tile)];
                     const int row = (tile - s.tile_begin) * 128 + tid;
-                    if (row < s.rows) finish_row<TPG>(p, s, row, grp, y[h], y[h], ia);
+                    if (row < s.rows) finish_row<TPG>(p, s, row, grp, y[h], y[h]);
                 }
             }
         }
@@ -599,25 +572,23 @@ int tokens_per_group(int tokens)
 {
     if (tokens <= 48) return 16;
     const int g16 = (tokens + 15) / 16, g24 = (tokens + 23) / 24;
-    return g24 * (2 * kURec + 512 * 24) < g16 * (2 * kURec + 512 * 16) ? 24 : 16;
+    return g24 * (2 * kURec + digit_block(24)) < g16 * (2 * kURec + digit_block(16)) ? 24 : 16;
 }
 size_t image_bytes(int cols, int tokens)
 {
     const int tpg = tokens_per_group(tokens);
     const size_t groups = size_t(tokens + tpg - 1) / tpg;
-    return size_t(cols >> 7) * groups * 512 * tpg;
+    return size_t(cols >> 7) * groups * digit_block(tpg);
 }
 constexpr size_t kPartialBytes = size_t(kGMaxGrid) * 2 * 2 * kSlotFloats * sizeof(float); // [CTA][cut unit][record of the pair]
 } // namespace
 
 
-// digit image | per-token scales | partial sums of cut units | tickets
+// digit image | partial sums of cut units | tickets
 size_t umma_gemm_scratch(int cols, int tokens)
 {
     if (cols <= 0 || (cols & 127) || tokens <= 0) return 0;
-    const int tpg = tokens_per_group(tokens);
-    const size_t groups = size_t(tokens + tpg - 1) / tpg;
-    return image_bytes(cols, tokens) + ((groups * tpg * sizeof(float) + 255) & ~size_t(255)) + kPartialBytes + kGMaxGrid * sizeof(int);
+    return image_bytes(cols, tokens) + kPartialBytes + kGMaxGrid * sizeof(int);
 }
 
 int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st); // 1..8 tokens (umma_gemv.cu)
@@ -641,17 +612,15 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     DigitizeParams d = {};
     d.pro = ProIn{op->in, op->aux, op->norm_w, nullptr, op->cols, op->prologue};
     d.bimg = static_cast<uint8_t *>(op->umma_scratch);
-    d.inv_alpha = reinterpret_cast<float *>(d.bimg + image_bytes(op->cols, tokens));
     d.tokens = tokens;
     d.ngroups = ngroups;
     d.tpg = tpg;
-    // about one CTA per SM, a slice of at least 64 float4 columns each
-    d.parts = std::max(1, std::min((op->cols >> 2) / 64, sm_count() / (ngroups * tpg)));
+    // about one CTA per SM, a slice of at least two k-blocks each
+    d.parts = std::max(1, std::min(nkb / 2, sm_count() / (ngroups * tpg)));
 
     GParams p = {};
     p.bimg = d.bimg;
-    p.inv_alpha = d.inv_alpha;
-    p.partials = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(d.inv_alpha) + ((size_t(ngroups) * tpg * sizeof(float) + 255) & ~size_t(255)));
+    p.partials = reinterpret_cast<float *>(d.bimg + image_bytes(op->cols, tokens));
     p.tickets = reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(p.partials) + kPartialBytes);
     d.tickets = p.tickets;
     p.nkb = nkb;
@@ -682,9 +651,9 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     if (total > (1ll << 30)) return fail(INSG_E_LIMIT, "gemm: more than 2^30 (tile, group, k-block) stages");
     p.total_stages = int(total);
     p.error_flag = op->error_flag;
-    const int stage_bytes = 2 * kURec + 512 * tpg;
-    p.stages = std::min(kGMaxStages, (224 * 1024 - 512) / stage_bytes);
-    const size_t smem = size_t(p.stages) * stage_bytes + 512;
+    const int stage_bytes = 2 * kURec + digit_block(tpg);
+    p.stages = std::min(kGMaxStages, 224 * 1024 / stage_bytes);
+    const size_t smem = size_t(p.stages) * stage_bytes;
     auto kernel = tpg == 16 ? (nmat_all == 2 ? umma_gemm_kernel<16, true> : umma_gemm_kernel<16, false>)
                             : (nmat_all == 2 ? umma_gemm_kernel<24, true> : umma_gemm_kernel<24, false>);
     {

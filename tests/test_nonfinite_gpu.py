@@ -14,7 +14,8 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
-@pytest.mark.parametrize("tokens", [1, 2, 3, 8])
+# up to eight tokens: the GEMV; more: the GEMM with 16 (up to 48) or 24 tokens a group
+@pytest.mark.parametrize("tokens", [1, 2, 3, 8, 9, 16, 48, 49, 71])
 @pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
 def test_a_non_finite_activation_makes_its_token_nan(cuda, tokens, value):
     from insignia_b200 import ops
@@ -60,7 +61,7 @@ def test_a_prepared_image_carries_nan(cuda, tokens):
         assert np.isfinite(clean).all() and np.isnan(with_nan[-1]).all() and np.array_equal(clean[:-1], with_nan[:-1])
 
 
-@pytest.mark.parametrize("tokens", [1, 8])
+@pytest.mark.parametrize("tokens", [1, 8, 9, 49])
 @pytest.mark.parametrize("scale", [1e32, 1e-33])
 def test_groups_of_very_large_and_small_values(cuda, tokens, scale):
     from insignia_b200 import ops
