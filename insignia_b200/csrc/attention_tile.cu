@@ -7,14 +7,21 @@
 // in tiles of 32 and keeps an online softmax: every row fetched serves 64 query rows.
 //
 // Precision: the products run on mma.sync.m16n8k16 (fp16 in, fp32 accumulate).  Every fp32 operand is scaled by a power of two
-// that puts the largest element of its tile in [2^12, 2^13) and cut into two fp16 pieces hi + lo (22 bits and more of it);
-// the products hi*hi + hi*lo + lo*hi are accumulated, the missing lo*lo is below 2^-22 of the result.  A bf16 cache needs one
-// piece (8 significant bits fit fp16 exactly).  The value tiles share one running scale, so that the output accumulators are
-// rescaled (with the softmax correction, by a power of two) when a tile brings a larger element.
+// that puts the largest element of its tile in [2^12, 2^13) and cut into two fp16 pieces hi + lo, which together round it to
+// 23 bits or better; all four products of pieces are accumulated.  A bf16 cache needs one piece (8 significant bits fit fp16
+// exactly).  The value tiles share one running scale, so that the output accumulators are rescaled (with the softmax correction,
+// by a power of two) when a tile brings a larger element.
+// The instruction rounds its accumulator toward zero every time, and a sum kept in it through a whole row is off by some 1e-6.
+// So it only adds the products with a lo piece, 2^-11 of the rest, to a running sum; 16 products hi * hi start from zero and
+// are added outside, compensated, and so are the outputs.  Distance from float64 (2-norm, 512 tokens behind 512 rows):
+// 1.6e-7 (fp32 cache), 1.5e-7 (bf16), the split-K kernel's 1.8e-7; with everything left to the accumulator 2.4e-6 and 1.6e-6,
+// at 155 and 118 us instead of 226 and 163.
 //
-// Eight warps: warp & 3 = 16 of the query rows, warp >> 2 = which half of the 32 keys; the two halves are merged at the end.
-// Per tile of 32 keys a warp issues 96 + 96 MMAs (fp32 cache) and reads 48 KB of fragments from shared memory: the two are
-// about equal, which is what bounds it.  Rows of 528 bytes keep ldmatrix free of bank conflicts.
+// Eight warps: warp & 3 = 16 of the query rows, warp >> 2 = which half of the 32 keys a warp scores and which half of the 256
+// dims it sums; the two warps of a row exchange maxima and weights through shared memory.  Per tile of 32 keys a warp issues
+// 128 + 128 MMAs (fp32 cache) between the conversion of the tile and three barriers: the tensor pipe is busy a third of the time,
+// the issue slots half of it (two warps a scheduler; sixteen warps of half the keys and dims read the query twice as often and
+// take the same time).  Rows of 528 bytes keep ldmatrix free of bank conflicts.
 #include "attention_body.cuh"
 #include "host_util.h"
 
@@ -34,8 +41,6 @@ template <bool BF16> struct TileSmem {
     static constexpr int v = k + pieces * kTileKeys * kPitch;                  // [pieces][32] rows
     static constexpr int raw = v + pieces * kTileKeys * kPitch;                // [K, V][32] rows as cached
     static constexpr int bytes = raw + 2 * kTileKeys * raw_row;
-    // the merge of the two key halves reuses the front: four warps x 16 rows x 256 floats
-    static_assert(bytes >= 4 * 16 * 256 * 4, "merge buffer");
 };
 
 __device__ __forceinline__ uint32_t saddr32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -49,9 +54,22 @@ __device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], uint32_t addr)
 }
 __device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
 {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_f16_first(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) // no sum to add to
+{
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                 : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// sum + rest += x, rest being what the additions have rounded off.
+__device__ __forceinline__ void add_compensated(float &sum, float &rest, float x)
+{
+    const float y = x + rest, z = sum + y;
+    rest = y - (z - sum);
+    sum = z;
 }
 // hi and lo fp16 pieces of two scaled values
 __device__ __forceinline__ void split2(float a, float b, uint32_t &hi, uint32_t &lo)
@@ -73,7 +91,8 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
     using L = TileSmem<BF16>;
     extern __shared__ __align__(128) uint8_t sm[];
     __shared__ uint32_t s_max[3][2]; // largest magnitude bits of [tile buffer][K, V]; [2][0]: the query rows
-    __shared__ float s_ml[4][2][16];
+    __shared__ float s_mx[4][2][16], s_l[4][2][16]; // [16 query rows][key half][row]
+    __shared__ uint32_t s_p[4][2][8][32];            // the weights' pieces as the A operand: [16 query rows][key half][register][lane]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int kvh = blockIdx.x, q0 = (int(gridDim.y) - 1 - int(blockIdx.y)) * kTileTokens; // the longest rows first
     const int rg = warp & 3, kg = warp >> 2, g = lane >> 2, t = lane & 3;
@@ -128,15 +147,18 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
         }
     }
 
-    float o[32][4]; // [8 dims each][row g: dims 2t, 2t+1 | row g + 8: dims 2t, 2t+1]
+    float o[16][4], oc[16][4]; // [8 dims each][row g: dims 2t, 2t+1 | row g + 8: dims 2t, 2t+1]; the sum is o + oc
 #pragma unroll
-    for (int j = 0; j < 32; j++) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
-    float m_run[2] = {-3.0e38f, -3.0e38f}, l_run[2] = {0.f, 0.f}; // rows g and g + 8 (l as this thread's partial sum)
+    for (int j = 0; j < 16; j++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) o[j][c] = oc[j][c] = 0.f;
+    float m_run[2] = {-3.0e38f, -3.0e38f}, l_run[2] = {0.f, 0.f}, l_rest[2] = {0.f, 0.f}; // rows g and g + 8 (l: this thread's share of its keys)
     int ev = 24;                                                  // exponent of the running value scale
     const int limit0 = pos0 + q0 + ((rg * 16 + g) >> 2), limit1 = pos0 + q0 + ((rg * 16 + g + 8) >> 2); // last row each query row sees
     const uint32_t qaddr = saddr32(sm + L::q) + (rg * 16 + (lane & 15)) * kPitch + (lane >> 4) * 16;
     const uint32_t kaddr = saddr32(sm + L::k) + (kg * 16 + ((lane >> 4) & 1) * 8 + (lane & 7)) * kPitch + ((lane >> 3) & 1) * 16;
-    const uint32_t vaddr = saddr32(sm + L::v) + (kg * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * kPitch + ((lane >> 4) & 1) * 16;
+    const uint32_t vaddr = saddr32(sm + L::v) + (((lane >> 3) & 1) * 8 + (lane & 7)) * kPitch + ((lane >> 4) & 1) * 16 + kg * 256;
+    auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + rg) : "memory"); }; // the two warps of 16 query rows
 
     for (int tile = 0; tile < ntiles; tile++) {
         const int buf = tile & 1;
@@ -195,127 +217,142 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
             }
         }
         __syncthreads(); // the pieces are complete
-        const int key0 = tile * kTileKeys + kg * 16;
-        if (key0 < nkeys) { // warp-uniform; a half tile past the last row has nothing to add
-            // ---- scores of 16 rows x 16 keys ----
-            float s[2][4];
+        const int key0 = tile * kTileKeys + kg * 16 + 2 * t; // this thread's first key of four
+        // ---- scores of 16 rows x 16 keys ----
+        float s[2][4], comp[2][4], low[2][4]; // sums of hi*hi, what their additions rounded off, sums with a lo piece
 #pragma unroll
-            for (int n = 0; n < 2; n++) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
+        for (int n = 0; n < 2; n++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) s[n][c] = comp[n][c] = low[n][c] = 0.f;
 #pragma unroll 4
-            for (int i = 0; i < 16; i++) {
-                uint32_t qh[4], ql[4], kh[4];
-                ldsm4(qh, qaddr + 32 * i);
-                ldsm4(ql, qaddr + kTileRows * kPitch + 32 * i);
-                ldsm4(kh, kaddr + 32 * i);
-                mma_f16(s[0], qh, kh[0], kh[1]);
-                mma_f16(s[1], qh, kh[2], kh[3]);
-                mma_f16(s[0], ql, kh[0], kh[1]);
-                mma_f16(s[1], ql, kh[2], kh[3]);
-                if (!BF16) {
-                    uint32_t kl[4];
-                    ldsm4(kl, kaddr + kTileKeys * kPitch + 32 * i);
-                    mma_f16(s[0], qh, kl[0], kl[1]);
-                    mma_f16(s[1], qh, kl[2], kl[3]);
-                }
+        for (int i = 0; i < 16; i++) {
+            uint32_t qh[4], ql[4], kh[4], kl[4];
+            float part[2][4];
+            ldsm4(qh, qaddr + 32 * i);
+            ldsm4(ql, qaddr + kTileRows * kPitch + 32 * i);
+            ldsm4(kh, kaddr + 32 * i);
+            if (!BF16) ldsm4(kl, kaddr + kTileKeys * kPitch + 32 * i);
+#pragma unroll
+            for (int n = 0; n < 2; n++) {
+                mma_f16_first(part[n], qh, kh[2 * n], kh[2 * n + 1]);
+                if (!BF16) mma_f16(low[n], ql, kl[2 * n], kl[2 * n + 1]);
+                if (!BF16) mma_f16(low[n], qh, kl[2 * n], kl[2 * n + 1]);
+                mma_f16(low[n], ql, kh[2 * n], kh[2 * n + 1]);
             }
-            // ---- online softmax (rows g and g + 8; a row's 16 keys sit in the four lanes of a quad) ----
-            const float sc = invq * scale_down(ek);
-            float pr[2][4], corr[2];
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int limit = h ? limit1 : limit0;
-                float mx = -3.0e38f;
+            for (int n = 0; n < 2; n++)
 #pragma unroll
-                for (int n = 0; n < 2; n++)
+                for (int c = 0; c < 4; c++) add_compensated(s[n][c], comp[n][c], part[n][c]);
+        }
+        // ---- online softmax (rows g and g + 8; a row's 32 keys sit in the quads of two warps) ----
+        const float sc = invq * scale_down(ek);
+        bool on[2][4]; // the row sees the key
 #pragma unroll
-                    for (int c = 0; c < 2; c++) {
-                        const float x = s[n][2 * h + c] * sc;
-                        s[n][2 * h + c] = x;
-                        if (key0 + n * 8 + 2 * t + c <= limit) mx = fmaxf(mx, x);
-                    }
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-                const float m_new = fmaxf(m_run[h], mx);
-                corr[h] = __expf(m_run[h] - m_new);
-                m_run[h] = m_new;
-                float sum = 0.f;
+        for (int n = 0; n < 2; n++)
 #pragma unroll
-                for (int n = 0; n < 2; n++)
-#pragma unroll
-                    for (int c = 0; c < 2; c++) {
-                        const float e = key0 + n * 8 + 2 * t + c <= limit ? __expf(s[n][2 * h + c] - m_new) : 0.f;
-                        pr[n][2 * h + c] = e * 4096.f;
-                        sum += e;
-                    }
-                l_run[h] = fmaf(l_run[h], corr[h], sum);
+            for (int c = 0; c < 4; c++) {
+                s[n][c] = (s[n][c] + (low[n][c] + comp[n][c])) * sc;
+                on[n][c] = key0 + n * 8 + (c & 1) <= (c < 2 ? limit0 : limit1);
             }
-            uint32_t ph[4], pl[4]; // the weights as the A operand: keys as k
-            split2(pr[0][0], pr[0][1], ph[0], pl[0]);
-            split2(pr[0][2], pr[0][3], ph[1], pl[1]);
-            split2(pr[1][0], pr[1][1], ph[2], pl[2]);
-            split2(pr[1][2], pr[1][3], ph[3], pl[3]);
-            const float c0 = corr[0] * fv, c1 = corr[1] * fv;
-            // ---- values ----
-#pragma unroll
-            for (int j = 0; j < 16; j++) { // 16 dims each
-                uint32_t vh[4];
-                ldsm4t(vh, vaddr + 32 * j);
-#pragma unroll
-                for (int n = 0; n < 2; n++) {
-                    float (&a)[4] = o[2 * j + n];
-                    a[0] *= c0; a[1] *= c0; a[2] *= c1; a[3] *= c1;
-                    mma_f16(a, ph, vh[2 * n], vh[2 * n + 1]);
-                    mma_f16(a, pl, vh[2 * n], vh[2 * n + 1]);
-                }
-                if (!BF16) {
-                    uint32_t vl[4];
-                    ldsm4t(vl, vaddr + kTileKeys * kPitch + 32 * j);
-                    mma_f16(o[2 * j], ph, vl[0], vl[1]);
-                    mma_f16(o[2 * j + 1], ph, vl[2], vl[3]);
-                }
-            }
-        } else if (fv != 1.f) {
-#pragma unroll
-            for (int j = 0; j < 32; j++) { o[j][0] *= fv; o[j][1] *= fv; o[j][2] *= fv; o[j][3] *= fv; }
-        }
-    }
-    // ---- merge the two key halves and write the rows ----
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 1);
-        l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 2);
-    }
-    __syncthreads(); // the pieces are no longer needed
-    float2 *merge = reinterpret_cast<float2 *>(sm) + size_t(rg) * 32 * 64; // [j][2 rows][lane]
-    if (kg == 1) {
-#pragma unroll
-        for (int j = 0; j < 32; j++) {
-            merge[(2 * j) * 32 + lane] = make_float2(o[j][0], o[j][1]);
-            merge[(2 * j + 1) * 32 + lane] = make_float2(o[j][2], o[j][3]);
-        }
-        if (t == 0) {
-            s_ml[rg][0][g] = m_run[0]; s_ml[rg][0][g + 8] = m_run[1];
-            s_ml[rg][1][g] = l_run[0]; s_ml[rg][1][g + 8] = l_run[1];
-        }
-    }
-    __syncthreads();
-    if (kg == 0) {
-        const float inv_v = scale_down(ev) * (1.f / 4096.f);
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            const int r = rg * 16 + g + 8 * h, tok = q0 + (r >> 2);
-            const float mb = s_ml[rg][0][g + 8 * h], lb = s_ml[rg][1][g + 8 * h];
-            const float mg = fmaxf(m_run[h], mb), ea = __expf(m_run[h] - mg), eb = lb > 0.f ? __expf(mb - mg) : 0.f;
-            const float inv = inv_v / fmaf(l_run[h], ea, lb * eb);
-            if (tok < tokens) {
-                float *dst = p.out + (size_t(tok) * 16 + kvh * 4 + (r & 3)) * 256 + 2 * t;
+            float mx = -3.0e38f;
 #pragma unroll
-                for (int j = 0; j < 32; j++) {
-                    const float2 b = merge[(2 * j + h) * 32 + lane];
-                    *reinterpret_cast<float2 *>(dst + 8 * j) =
-                        make_float2(fmaf(o[j][2 * h], ea, b.x * eb) * inv, fmaf(o[j][2 * h + 1], ea, b.y * eb) * inv);
+            for (int n = 0; n < 2; n++)
+#pragma unroll
+                for (int c = 2 * h; c < 2 * h + 2; c++) mx = on[n][c] ? fmaxf(mx, s[n][c]) : mx;
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            if (t == 0) s_mx[rg][kg][g + 8 * h] = mx;
+        }
+        pair_sync();
+        float corr[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const float m_new = fmaxf(m_run[h], fmaxf(s_mx[rg][0][g + 8 * h], s_mx[rg][1][g + 8 * h]));
+            corr[h] = expf(m_run[h] - m_new);
+            m_run[h] = m_new;
+            float sum = 0.f;
+#pragma unroll
+            for (int n = 0; n < 2; n++) {
+#pragma unroll
+                for (int c = 2 * h; c < 2 * h + 2; c++) {
+                    s[n][c] = on[n][c] ? expf(s[n][c] - m_new) : 0.f;
+                    sum += s[n][c];
                 }
+                uint32_t hi, lo;
+                split2(s[n][2 * h] * 4096.f, s[n][2 * h + 1] * 4096.f, hi, lo);
+                s_p[rg][kg][2 * n + h][lane] = hi;
+                s_p[rg][kg][4 + 2 * n + h][lane] = lo;
             }
+            l_run[h] *= corr[h];
+            l_rest[h] *= corr[h];
+            add_compensated(l_run[h], l_rest[h], sum);
+        }
+        pair_sync();
+        uint32_t w[2][2][4]; // the weights as the A operand: [key half][hi, lo]
+#pragma unroll
+        for (int k = 0; k < 2; k++)
+#pragma unroll
+            for (int i = 0; i < 8; i++) w[k][i >> 2][i & 3] = s_p[rg][k][i][lane];
+        const float c0 = corr[0] * fv, c1 = corr[1] * fv;
+        if (__any_sync(0xffffffffu, c0 != 1.f || c1 != 1.f)) {
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                o[j][0] *= c0; o[j][1] *= c0; o[j][2] *= c1; o[j][3] *= c1;
+                oc[j][0] *= c0; oc[j][1] *= c0; oc[j][2] *= c1; oc[j][3] *= c1;
+            }
+        }
+        // ---- values: 128 of the 256 dims, 16 keys and 16 dims at a time; the small products first, one rounding of the large one ----
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                uint32_t vh[4], vl[4];
+                float part[2][4];
+                ldsm4t(vh, vaddr + k * 16 * kPitch + 32 * j);
+                if (!BF16) ldsm4t(vl, vaddr + (kTileKeys + k * 16) * kPitch + 32 * j);
+#pragma unroll
+                for (int n = 0; n < 2; n++) {
+                    if (BF16) {
+                        mma_f16_first(part[n], w[k][1], vh[2 * n], vh[2 * n + 1]);
+                    } else {
+                        mma_f16_first(part[n], w[k][1], vl[2 * n], vl[2 * n + 1]);
+                        mma_f16(part[n], w[k][1], vh[2 * n], vh[2 * n + 1]);
+                        mma_f16(part[n], w[k][0], vl[2 * n], vl[2 * n + 1]);
+                    }
+                    mma_f16(part[n], w[k][0], vh[2 * n], vh[2 * n + 1]);
+                }
+#pragma unroll
+                for (int n = 0; n < 2; n++)
+#pragma unroll
+                    for (int c = 0; c < 4; c++) add_compensated(o[2 * j + n][c], oc[2 * j + n][c], part[n][c]);
+            }
+        }
+    }
+    // ---- the denominator from both key halves; write the rows ----
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        l_run[h] += l_rest[h];
+        l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 1);
+        l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 2);
+        if (t == 0) s_l[rg][kg][g + 8 * h] = l_run[h];
+    }
+    pair_sync();
+    const float up_v = scale_down(ev) * (1.f / 4096.f); // undoes the values' and the weights' powers of two
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int r = rg * 16 + g + 8 * h, tok = q0 + (r >> 2);
+        const float l = s_l[rg][0][g + 8 * h] + s_l[rg][1][g + 8 * h], inv = 1.f / l, off = fmaf(-l, inv, 1.f);
+        auto quotient = [&](float a, float b) { // (a + b) / l with one rounding
+            const float q = a * inv;
+            return (q + fmaf(q, off, fmaf(a, inv, -q) + b * inv)) * up_v;
+        };
+        if (tok < tokens) {
+            float *dst = p.out + (size_t(tok) * 16 + kvh * 4 + (r & 3)) * 256 + kg * 128 + 2 * t;
+#pragma unroll
+            for (int j = 0; j < 16; j++)
+                *reinterpret_cast<float2 *>(dst + 8 * j) = make_float2(quotient(o[j][2 * h], oc[j][2 * h]), quotient(o[j][2 * h + 1], oc[j][2 * h + 1]));
         }
     }
 }
