@@ -81,9 +81,89 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t &hi, uint32_t 
     lo = *reinterpret_cast<const uint32_t *>(&l);
 }
 // Biased exponent of a tile's largest magnitude, kept where both 2^(12 - e) and its inverse are normal numbers.
-__device__ __forceinline__ int tile_exponent(uint32_t max_bits) { return min(max(int(max_bits >> 23), 24), 230); }
+constexpr int kMaxExponent = 230; // tiles beyond it are not multiplied
+__device__ __forceinline__ int tile_exponent(uint32_t max_bits) { return max(int(max_bits >> 23), 24); }
 __device__ __forceinline__ float scale_up(int e) { return __uint_as_float(uint32_t(127 + 12 + 127 - e) << 23); }   // 2^(12 - (e - 127))
 __device__ __forceinline__ float scale_down(int e) { return __uint_as_float(uint32_t(e - 12) << 23); }             // its inverse
+
+// One token's four query heads over its first `rows` cached rows in fp32, by a warp (the loop of attn_splitk_kernel): for what the
+// fp16 pieces cannot hold, infinities, NaN and values beyond 2^104, which must reach the tokens that see them and no others.
+// (For short contexts too it would be slower, 64 tokens from an empty cache 50 us against 30, and no closer to float64.)
+template <bool BF16> __device__ __noinline__ void attn_token(const AttnParams &p, const float *qn, int tok, int rows, int kvh)
+{
+    using Row = KvRow<BF16>;
+    const int lane = threadIdx.x & 31, my_row = lane >> 3;
+    float q[4][8], acc[4][8], m = -3.0e38f, l = 0.f;
+#pragma unroll
+    for (int h = 0; h < 4; h++) {
+        const float4 *src = reinterpret_cast<const float4 *>(qn + (size_t(tok) * 16 + kvh * 4 + h) * 256 + lane * 8);
+        const float4 a = __ldcg(src), b = __ldcg(src + 1);
+        q[h][0] = a.x; q[h][1] = a.y; q[h][2] = a.z; q[h][3] = a.w; q[h][4] = b.x; q[h][5] = b.y; q[h][6] = b.z; q[h][7] = b.w;
+#pragma unroll
+        for (int j = 0; j < 8; j++) acc[h][j] = 0.f;
+    }
+    GroupRaw<BF16, 4> kv;
+    load_group<BF16, 4>(p.kc, p.vc, kvh, 0, rows, lane, kv);
+    for (int tb = 0; tb < rows; tb += 4) {
+        float s[16]; // [row of the group][head]
+#pragma unroll
+        for (int g = 0; g < 4; g++) {
+            float k[8];
+            Row::unpack(kv.k[g], k);
+#pragma unroll
+            for (int h = 0; h < 4; h++) {
+                s[g * 4 + h] = q[h][0] * k[0];
+#pragma unroll
+                for (int j = 1; j < 8; j++) s[g * 4 + h] = fmaf(q[h][j], k[j], s[g * 4 + h]);
+            }
+        }
+        load_keys<BF16, 4>(p.kc, kvh, tb + 4, rows, lane, kv);
+#pragma unroll
+        for (int n = 8, mk = 16; n; n >>= 1, mk >>= 1) { // lane L is left with number L >> 1: row L >> 3, head (L >> 1) & 3
+            const bool up = (lane & mk) != 0;
+#pragma unroll
+            for (int i = 0; i < n; i++) {
+                const float keep = up ? s[i + n] : s[i], send = up ? s[i] : s[i + n];
+                s[i] = keep + __shfl_xor_sync(0xffffffffu, send, mk);
+            }
+        }
+        const float score = (s[0] + __shfl_xor_sync(0xffffffffu, s[0], 1)) * 0.0625f;
+        const bool on = tb + my_row < rows;
+        float mx = on ? score : -3.0e38f;
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+        const float mn = fmaxf(m, mx), corr = expf(m - mn), pr = on ? expf(score - mn) : 0.f;
+        m = mn;
+        l = fmaf(l, corr, pr);
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+            const float c = __shfl_sync(0xffffffffu, corr, 2 * h);
+#pragma unroll
+            for (int j = 0; j < 8; j++) acc[h][j] *= c;
+        }
+#pragma unroll
+        for (int g = 0; g < 4; g++) {
+            float v[8];
+            Row::unpack(kv.v[g], v);
+#pragma unroll
+            for (int h = 0; h < 4; h++) {
+                const float w = __shfl_sync(0xffffffffu, pr, (g * 4 + h) * 2);
+#pragma unroll
+                for (int j = 0; j < 8; j++) acc[h][j] = fmaf(w, v[j], acc[h][j]);
+            }
+        }
+        load_values<BF16, 4>(p.vc, kvh, tb + 4, rows, lane, kv);
+    }
+    l += __shfl_xor_sync(0xffffffffu, l, 8);
+    l += __shfl_xor_sync(0xffffffffu, l, 16);
+#pragma unroll
+    for (int h = 0; h < 4; h++) {
+        const float lh = __shfl_sync(0xffffffffu, l, 2 * h);
+        float4 *dst = reinterpret_cast<float4 *>(p.out + (size_t(tok) * 16 + kvh * 4 + h) * 256 + lane * 8);
+        dst[0] = make_float4(acc[h][0] / lh, acc[h][1] / lh, acc[h][2] / lh, acc[h][3] / lh);
+        dst[1] = make_float4(acc[h][4] / lh, acc[h][5] / lh, acc[h][6] / lh, acc[h][7] / lh);
+    }
+}
 
 template <bool BF16>
 __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_constant__ AttnParams p, const float *__restrict__ qn, int tokens)
@@ -116,6 +196,9 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    auto plain = [&] { // every token by a warp in fp32
+        for (int tok = q0 + warp; tok < min(q0 + kTileTokens, tokens); tok += kTThreads / 32) attn_token<BF16>(p, qn, tok, pos0 + tok + 1, kvh);
+    };
     fetch(0);
 
     // ---- query rows: scaled by 1/16 and the tile's power of two, two pieces ----
@@ -126,13 +209,18 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
             const int r = i >> 6, c = i & 63, tok = q0 + (r >> 2);
             if (tok < tokens) {
                 const float4 x = __ldcg(reinterpret_cast<const float4 *>(qn + (size_t(tok) * 16 + kvh * 4 + (r & 3)) * 256) + c);
-                mx = max(mx, __float_as_uint(fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w)))));
+                mx = max(max(mx, max(__float_as_uint(fabsf(x.x)), __float_as_uint(fabsf(x.y)))), max(__float_as_uint(fabsf(x.z)), __float_as_uint(fabsf(x.w))));
             }
         }
         mx = __reduce_max_sync(0xffffffffu, mx);
         if (lane == 0) atomicMax(&s_max[2][0], mx);
         __syncthreads();
         const int e = tile_exponent(s_max[2][0]);
+        if (e > kMaxExponent) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            plain();
+            return;
+        }
         const float up = scale_up(e);
         invq = scale_down(e) * 0.0625f;
         for (int i = tid; i < kTileRows * 64; i += kTThreads) {
@@ -186,8 +274,12 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
             if (lane == 0) atomicMax(&s_max[buf][kv], mx);
         }
         __syncthreads(); // maxima complete, the raw tile is in registers
-        if (tile + 1 < ntiles) fetch(tile + 1);
         const int ek = tile_exponent(s_max[buf][0]), ev_new = max(ev, tile_exponent(s_max[buf][1]));
+        if (max(ek, ev_new) > kMaxExponent) { // all threads; nothing is in flight
+            plain();
+            return;
+        }
+        if (tile + 1 < ntiles) fetch(tile + 1);
         const float fv = __uint_as_float(uint32_t(max(127 + ev - ev_new, 0)) << 23); // rescales what was accumulated so far
         ev = ev_new;
         {

@@ -74,3 +74,43 @@ def test_groups_of_very_large_and_small_values(cuda, tokens, scale):
     for m in range(tokens):
         want = orc.gemv_mlx_f64(w, s, x[m])
         assert np.max(np.abs(got[m] - want)) <= 4e-6 * np.abs(want).max()
+
+
+def _chunk(ops, case, tokens, start, ctx, k, v, step):
+    """The pass in calls of `step` tokens: `tokens` = the query tiles, 32 = the token-by-token form."""
+    kc, vc, pos = case["kc"].clone(), case["vc"].clone(), torch.zeros(1, dtype=torch.int32, device="cuda")
+    scratch, out = torch.zeros(32 * ops.gqa_scratch("cuda").numel(), dtype=torch.uint8, device="cuda"), []
+    if step > 32:
+        scratch = torch.zeros(step * ops.gqa_scratch("cuda").numel(), dtype=torch.uint8, device="cuda")
+    for first in range(0, tokens, step):
+        n = min(step, tokens - first)
+        pos.fill_(start + first)
+        out.append(host(ops.attention_chunk(case["q"][first:first + n].contiguous(), k[first:first + n].contiguous(), v[first:first + n].contiguous(), case["qw"],
+                                            case["kw"], kc, vc, pos, ctx, scratch, n)))
+    return np.concatenate(out).reshape(tokens, 16, 256)
+
+
+# the value sits in the pass (tokens before it must not see it) or in the rows behind it; start 0: the first rows of an empty cache
+@pytest.mark.parametrize("kv_bf16", [False, True])
+@pytest.mark.parametrize("start", [0, 200])
+@pytest.mark.parametrize("what,value", [("key", np.nan), ("value", np.nan), ("value", np.inf), ("value", 1e33), ("query", np.nan), ("none", 0.0)])
+def test_prompt_attention_keeps_a_bad_row_to_the_tokens_that_see_it(cuda, kv_bf16, start, what, value):
+    from insignia_b200 import ops
+
+    rng = np.random.default_rng(start)
+    tokens, at = 100, 41
+    ctx, dt = start + tokens, torch.bfloat16 if kv_bf16 else torch.float32
+    case = {n: torch.randn(ctx * 1024, device="cuda").to(dt) for n in ("kc", "vc")}
+    case.update(qw=dev(bf16(rng, 256)), kw=dev(bf16(rng, 256)), q=dev(rng.standard_normal((tokens, 8192)).astype(np.float32)))
+    k, v = (dev(rng.standard_normal((tokens, 1024)).astype(np.float32)) for _ in range(2))
+    clean = _chunk(ops, case, tokens, start, ctx, k, v, tokens)
+    if what == "query":
+        case["q"][at, 512 * 5 + 3] = value  # query head 5
+    else:
+        {"key": k, "value": v, "none": v}[what][at, 256 * 1 + 7] += value  # kv head 1: query heads 4..7
+    got, want = (_chunk(ops, case, tokens, start, ctx, k, v, step) for step in (tokens, 32))
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isinf(got), np.isinf(want))
+    ok = np.isfinite(want)
+    assert np.max(np.abs(got[ok] - want[ok]) / np.maximum(1, np.abs(want[ok]))) <= 1e-5  # two orders of fp32 sums
+    assert np.max(np.abs(got[:at] - clean[:at])) <= 1e-5 and np.array_equal(got[:32], clean[:32])
+    assert np.array_equal(np.delete(got, range(4, 8), 1), np.delete(clean, range(4, 8), 1))
