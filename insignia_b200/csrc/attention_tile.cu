@@ -182,8 +182,11 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
     pdl_wait();
     __syncthreads();
     const int pos0 = __ldcg(p.position) + p.position_offset;
-    if (pos0 < 0 || pos0 + tokens > p.max_context) return; // the prepare kernel refuses the same
-    const int nkeys = pos0 + min(q0 + kTileTokens, tokens); // rows the tile's last token attends
+    // only tokens with a place in the cache (the prepare kernel stores no others): first .. last - 1
+    const int first = max(q0, -pos0), last = min(min(q0 + kTileTokens, tokens), p.max_context - pos0); // of this tile
+    if (first >= last) return;
+    const int nkeys = pos0 + last; // rows the tile's last token attends
+    auto live = [&](int tok) { return tok >= first && tok < last; };
     const int ntiles = (nkeys + kTileKeys - 1) / kTileKeys;
 
     auto fetch = [&](int tile) { // both raw tiles of 32 cached rows by 16-byte asynchronous copies; rows past the end repeat the last
@@ -197,7 +200,7 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     auto plain = [&] { // every token by a warp in fp32
-        for (int tok = q0 + warp; tok < min(q0 + kTileTokens, tokens); tok += kTThreads / 32) attn_token<BF16>(p, qn, tok, pos0 + tok + 1, kvh);
+        for (int tok = first + warp; tok < last; tok += kTThreads / 32) attn_token<BF16>(p, qn, tok, pos0 + tok + 1, kvh);
     };
     fetch(0);
 
@@ -207,7 +210,7 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
         uint32_t mx = 0;
         for (int i = tid; i < kTileRows * 64; i += kTThreads) {
             const int r = i >> 6, c = i & 63, tok = q0 + (r >> 2);
-            if (tok < tokens) {
+            if (live(tok)) {
                 const float4 x = __ldcg(reinterpret_cast<const float4 *>(qn + (size_t(tok) * 16 + kvh * 4 + (r & 3)) * 256) + c);
                 mx = max(max(mx, max(__float_as_uint(fabsf(x.x)), __float_as_uint(fabsf(x.y)))), max(__float_as_uint(fabsf(x.z)), __float_as_uint(fabsf(x.w))));
             }
@@ -226,7 +229,7 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
         for (int i = tid; i < kTileRows * 64; i += kTThreads) {
             const int r = i >> 6, c = i & 63, tok = q0 + (r >> 2);
             float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (tok < tokens) x = __ldcg(reinterpret_cast<const float4 *>(qn + (size_t(tok) * 16 + kvh * 4 + (r & 3)) * 256) + c);
+            if (live(tok)) x = __ldcg(reinterpret_cast<const float4 *>(qn + (size_t(tok) * 16 + kvh * 4 + (r & 3)) * 256) + c);
             uint2 hi, lo;
             split2(x.x * up, x.y * up, hi.x, lo.x);
             split2(x.z * up, x.w * up, hi.y, lo.y);
@@ -440,7 +443,7 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
             const float q = a * inv;
             return (q + fmaf(q, off, fmaf(a, inv, -q) + b * inv)) * up_v;
         };
-        if (tok < tokens) {
+        if (live(tok)) {
             float *dst = p.out + (size_t(tok) * 16 + kvh * 4 + (r & 3)) * 256 + kg * 128 + 2 * t;
 #pragma unroll
             for (int j = 0; j < 16; j++)
