@@ -19,11 +19,16 @@ KV_F32, KV_BF16 = 0, 1
 
 
 # The handle of the current stream without a Stream object around it: on calls of a few microseconds that object is a tenth.
-_raw_stream, _current_device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+# A torch without CUDA has neither name; it can still import this module.
+try:
+    from torch._C import _cuda_getCurrentRawStream, _cuda_getDevice
 
+    def _stream():
+        return _cuda_getCurrentRawStream(_cuda_getDevice())
+except ImportError:
 
-def _stream():
-    return _raw_stream(_current_device())
+    def _stream():
+        return torch.cuda.current_stream().cuda_stream
 
 
 def _p(t):
