@@ -211,8 +211,7 @@ int insg_mxfp4_gemv_packed(const void *packed, const float *x, float *y, int row
 {
     if (M < 1 || M > 4096) return fail(INSG_E_SHAPE, "gemv_packed: 1 <= M <= 4096");
     for (int m0 = 0; m0 < M;) {
-        const int left = M - m0;
-        const int mm = std::min(left, 4);
+        int mm = std::min(M - m0, 4);
         insg_gemv_op op = {};
         op.in = x + size_t(m0) * cols;
         op.cols = cols;
@@ -222,7 +221,11 @@ int insg_mxfp4_gemv_packed(const void *packed, const float *x, float *y, int row
         op.seg[0].out = y + size_t(m0) * rows;
         op.seg[0].rows = rows;
         op.seg[0].epilogue = INSG_EPI_STORE;
-        const int rc = gemv_fused_launch(&op, mm, stream);
+        int rc = gemv_fused_launch(&op, mm, stream);
+        if (rc == INSG_E_LIMIT && mm == 3) { // the rows' sums of three tokens fit shared memory up to some 10^6 rows, of two half as many more
+            mm = 2;
+            rc = gemv_fused_launch(&op, mm, stream);
+        }
         if (rc) return rc;
         m0 += mm;
     }

@@ -56,3 +56,16 @@ def test_a_product_takes_1_to_4096_tokens(tokens):
     from insignia_b200 import _lib
 
     assert _lib.lib().insg_mxfp4_gemm_umma(SOME, SOME, SOME, 256, 4096, tokens, SOME, 1 << 40, None) == E_SHAPE
+
+
+@pytest.mark.parametrize("rows,cols", [(3_000_000, 128), (1_000_000, 12288)])
+def test_three_tokens_of_very_many_rows_are_not_refused(rows, cols):
+    """Their sums no longer fit one launch: they go as two and one.  Here the launch itself fails, for want of a device."""
+    import torch
+
+    from insignia_b200 import _lib
+
+    if torch.cuda.is_available():
+        pytest.skip("would launch")
+    L = _lib.lib()
+    assert [L.insg_mxfp4_gemv_packed(SOME, SOME, SOME, rows, cols, m, None) for m in (1, 2, 3)] == [-2] * 3  # INSG_E_CUDA
