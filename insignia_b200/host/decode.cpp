@@ -247,7 +247,7 @@ void rmsnorm_input(const Ctx &c, insg_gemv_op &op, const uint16_t *norm_w)
     } else {
         op.in = c.x.hidden;
         op.norm_w = norm_w;
-        op.x_out = c.hidden_prepared ? nullptr : c.x.norm; // inside a token step nobody reads the normalised vector
+        op.x_out = c.x.norm;
         op.prologue = INSG_PRO_RMSNORM;
     }
 }
