@@ -136,3 +136,21 @@ def test_reservations_share_the_budget(store):
     assert store.L.insg_storage_unreserve(store.h, 50 * MiB) == 0
     assert store.acquire(QKV)[0] == 0
     assert store.L.insg_storage_clear(store.h) == 0 and store.used() == 0 and store.tier(QKV) == 0
+
+
+def test_an_upload_waits_for_a_prefetch_that_holds_its_room(golden_ckpt):
+    """While a prefetch is being loaded its bytes can be neither used nor evicted: an acquire or a reservation that needs them
+    waits and then evicts them, whenever it comes."""
+    for trial in range(30):
+        s = Store(golden_ckpt[1], 60 * MiB)
+        try:
+            assert s.acquire(QKV)[0] == 0  # 16 of 60 MiB pinned: one of the two 24 MiB tensors fits beside it
+            assert s.L.insg_storage_prefetch(s.h, GATE.encode()) == 1
+            time.sleep(0.0005 * (trial % 10))  # before, while and after it is loaded
+            if trial & 1:
+                assert s.acquire(UP)[0] == 0, s.err()
+            else:
+                assert s.L.insg_storage_reserve(s.h, 24 * MiB) == 0, s.err()
+            assert s.tier(QKV) == 2 and s.used() + s.L.insg_storage_reserved_bytes(s.h) <= 60 * MiB
+        finally:
+            s.close()
