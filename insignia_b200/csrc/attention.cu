@@ -426,14 +426,10 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
             a = fmaf(s_acc[w][h][tid], e, a);
         }
         const int dim = h * 256 + tid, owner = dim / kMine;
-        uint32_t dst;
-        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_u32(&s_in[rank][dim % kMine])), "r"(owner));
-        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(a) : "memory");
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_to_rank(smem_u32(&s_in[rank][dim % kMine]), owner)), "f"(a) : "memory");
         if (dim % kMine == 0) { // the head's maximum and denominator to the owner of these dims
-            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_u32(&s_min[rank])), "r"(owner));
-            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(mg) : "memory");
-            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_u32(&s_lin[rank])), "r"(owner));
-            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(lg) : "memory");
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_to_rank(smem_u32(&s_min[rank]), owner)), "f"(mg) : "memory");
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_to_rank(smem_u32(&s_lin[rank]), owner)), "f"(lg) : "memory");
         }
     }
     asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");

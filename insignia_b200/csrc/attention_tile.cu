@@ -43,7 +43,6 @@ template <bool BF16> struct TileSmem {
     static constexpr int bytes = raw + 2 * kTileKeys * raw_row;
 };
 
-__device__ __forceinline__ uint32_t saddr32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr)
 {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
@@ -195,7 +194,7 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
             const int kv = i / (kTileKeys * per_row), r = (i / per_row) % kTileKeys, c = i % per_row;
             const int row = min(tile * kTileKeys + r, nkeys - 1);
             const uint8_t *src = static_cast<const uint8_t *>(kv ? p.vc : p.kc) + (size_t(row) * 4 + kvh) * L::raw_row + c * 16;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(saddr32(sm + L::raw + (kv * kTileKeys + r) * L::raw_row + c * 16)), "l"(src) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(sm + L::raw + (kv * kTileKeys + r) * L::raw_row + c * 16)), "l"(src) : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -246,9 +245,9 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
     float m_run[2] = {-3.0e38f, -3.0e38f}, l_run[2] = {0.f, 0.f}, l_rest[2] = {0.f, 0.f}; // rows g and g + 8 (l: this thread's share of its keys)
     int ev = 24;                                                  // exponent of the running value scale
     const int limit0 = pos0 + q0 + ((rg * 16 + g) >> 2), limit1 = pos0 + q0 + ((rg * 16 + g + 8) >> 2); // last row each query row sees
-    const uint32_t qaddr = saddr32(sm + L::q) + (rg * 16 + (lane & 15)) * kPitch + (lane >> 4) * 16;
-    const uint32_t kaddr = saddr32(sm + L::k) + (kg * 16 + ((lane >> 4) & 1) * 8 + (lane & 7)) * kPitch + ((lane >> 3) & 1) * 16;
-    const uint32_t vaddr = saddr32(sm + L::v) + (((lane >> 3) & 1) * 8 + (lane & 7)) * kPitch + ((lane >> 4) & 1) * 16 + kg * 256;
+    const uint32_t qaddr = smem_u32(sm + L::q) + (rg * 16 + (lane & 15)) * kPitch + (lane >> 4) * 16;
+    const uint32_t kaddr = smem_u32(sm + L::k) + (kg * 16 + ((lane >> 4) & 1) * 8 + (lane & 7)) * kPitch + ((lane >> 3) & 1) * 16;
+    const uint32_t vaddr = smem_u32(sm + L::v) + (((lane >> 3) & 1) * 8 + (lane & 7)) * kPitch + ((lane >> 4) & 1) * 16 + kg * 256;
     auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + rg) : "memory"); }; // the two warps of 16 query rows
 
     for (int tile = 0; tile < ntiles; tile++) {

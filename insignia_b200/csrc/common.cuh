@@ -75,6 +75,14 @@ __device__ __forceinline__ float fast_sigmoid(float v) { return 1.0f / (1.0f + _
 __device__ __forceinline__ float fast_silu(float v) { return v / (1.0f + __expf(-v)); }
 
 // 128-bit streaming load that does not allocate in L1 (weights are read once per token).
+__device__ __forceinline__ uint32_t smem_u32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+// The same shared-memory address in another CTA of the cluster.
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t saddr, uint32_t rank)
+{
+    uint32_t d;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(saddr), "r"(rank));
+    return d;
+}
 __device__ __forceinline__ uint4 ldg_stream(const void *p)
 {
     uint4 r;

@@ -341,11 +341,8 @@ __global__ void __cluster_dims__(kArgmaxCtas, 1, 1) __launch_bounds__(512) argma
     asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
     if (threadIdx.x == 0) {
         for (int w = 1; w < 16; w++) take(sv[w], si[w]);
-        uint32_t v, i;
-        asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(v) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(&cv[rank]))));
-        asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(i) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(&ci[rank]))));
-        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(v), "f"(best) : "memory");
-        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(i), "r"(idx) : "memory");
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_to_rank(smem_u32(&cv[rank]), 0)), "f"(best) : "memory");
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_to_rank(smem_u32(&ci[rank]), 0)), "r"(idx) : "memory");
     }
     asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
     if (rank == 0 && threadIdx.x == 0) {

@@ -67,7 +67,6 @@ struct GemvShared {
     int last;
 };
 
-__device__ __forceinline__ uint32_t smem_addr(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
 __device__ __forceinline__ void dequant8(uint32_t q, uint32_t (&h)[4])
 {
@@ -290,7 +289,7 @@ __device__ __forceinline__ void gemv_activation(const GemvParams &p, __half *xs,
         const uint4 *src = reinterpret_cast<const uint4 *>(p.in);
         for (int i = tid; i < 2 * n16; i += kThreads) {
             const int piece = i >= n16, k = i - piece * n16;
-            const uint32_t dst = smem_addr(xs + size_t(piece) * xstride + k * 8);
+            const uint32_t dst = smem_u32(xs + size_t(piece) * xstride + k * 8);
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src + i) : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");

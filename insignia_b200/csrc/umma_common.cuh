@@ -9,8 +9,6 @@ namespace insg {
 constexpr int kURec = 8704;          // bytes per (128-row tile, 128-k block) weight record: 8192 of codes + 512 of scales
 constexpr uint32_t kSpinLimit = 1u << 22;
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-
 // shared-memory matrix descriptor: no swizzle, version 1 (sm_100); offsets in bytes
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo)
 {
@@ -117,6 +115,19 @@ __device__ __forceinline__ void pack_digits(float4 x, float alpha, const uint8_t
         *reinterpret_cast<uint16_t *>(base + (2 * j) * 16) = uint16_t(__byte_perm(e01, e23, j | ((4 + j) << 4)));
         *reinterpret_cast<uint16_t *>(base + (2 * j + 1) * 16) = uint16_t(__byte_perm(o01, o23, j | ((4 + j) << 4)));
     }
+}
+
+// A token's eight digit columns of an accumulator: the sum they stand for (least significant first; 9^j is exact in fp32).
+__device__ __forceinline__ float combine_digits(const uint32_t *d)
+{
+    float y = __uint_as_float(d[0]);
+    y = fmaf(__uint_as_float(d[1]), 9.f, y);
+    y = fmaf(__uint_as_float(d[2]), 81.f, y);
+    y = fmaf(__uint_as_float(d[3]), 729.f, y);
+    y = fmaf(__uint_as_float(d[4]), 6561.f, y);
+    y = fmaf(__uint_as_float(d[5]), 59049.f, y);
+    y = fmaf(__uint_as_float(d[6]), 531441.f, y);
+    return fmaf(__uint_as_float(d[7]), 4782969.f, y);
 }
 
 // ---- a group of 32 elements: its scale from its largest magnitude -------------------------------------------------------------

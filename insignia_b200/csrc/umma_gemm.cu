@@ -278,19 +278,7 @@ __device__ __forceinline__ void load_sums(uint32_t taddr, float (&y)[TPG])
         }
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int t = 0; t < 8; t++) {
-            const uint32_t *q = &d[t >> 2][(t & 3) * 8];
-            // least significant digit first; 9^j is exact in fp32
-            float ya = __uint_as_float(q[0]);
-            ya = fmaf(__uint_as_float(q[1]), 9.f, ya);
-            ya = fmaf(__uint_as_float(q[2]), 81.f, ya);
-            ya = fmaf(__uint_as_float(q[3]), 729.f, ya);
-            ya = fmaf(__uint_as_float(q[4]), 6561.f, ya);
-            ya = fmaf(__uint_as_float(q[5]), 59049.f, ya);
-            ya = fmaf(__uint_as_float(q[6]), 531441.f, ya);
-            ya = fmaf(__uint_as_float(q[7]), 4782969.f, ya);
-            y[t0 + t] = ya;
-        }
+        for (int t = 0; t < 8; t++) y[t0 + t] = combine_digits(&d[t >> 2][(t & 3) * 8]);
     }
 }
 
@@ -565,15 +553,11 @@ namespace {
 std::mutex g_gemm_attr_mutex;
 bool g_gemm_attr_done[64] = {false}; // the shared-memory opt-in is a per-device function attribute
 
-// Tokens per group: the one that takes fewer bytes into shared memory over all groups (the last one may be padded).  With few
-// groups the weights bound the time and every CTA ends on a cut unit, whose parts 24 tokens make half as large again and whose
-// ring is shorter: a pass of 17..24 tokens 4.0 ms against 4.9 in one group of 24, 33..48 tokens 4.2 against 5.1, 64 equal.
-int tokens_per_group(int tokens)
-{
-    if (tokens <= 48) return 16;
-    const int g16 = (tokens + 15) / 16, g24 = (tokens + 23) / 24;
-    return g24 * (2 * kURec + digit_block(24)) < g16 * (2 * kURec + digit_block(16)) ? 24 : 16;
-}
+// Tokens per group.  24 take fewer bytes into shared memory than 16 for every count beyond 48, the last group's padding included
+// (24576 x 4096 at 512 tokens 153 us against 182).  Up to 48 the weights bound the time and every CTA ends on a cut unit, whose
+// parts 24 tokens make half as large again and whose ring is shorter: a pass of 17..24 tokens 4.0 ms against 4.9 in one group of
+// 24, 33..48 tokens 4.2 against 5.1.
+int tokens_per_group(int tokens) { return tokens <= 48 ? 16 : 24; }
 size_t image_bytes(int cols, int tokens)
 {
     const int tpg = tokens_per_group(tokens);

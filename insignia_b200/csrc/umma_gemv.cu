@@ -77,12 +77,6 @@ struct DParams {
 };
 
 // ---- cluster helpers -----------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t map_to_rank(uint32_t saddr, uint32_t rank)
-{
-    uint32_t d;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(saddr), "r"(rank));
-    return d;
-}
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 // The closing barrier only keeps CTAs from leaving early.  A release there would wait until the epilogue's global stores have been
@@ -145,7 +139,7 @@ template <int T> __device__ __forceinline__ void leave_digits(const DSeg &s, flo
     }
 }
 
-// One accumulator: the eight digit columns of each token, digits combined (least significant first; 9^j is exact in fp32).
+// One accumulator: the eight digit columns of each token, digits combined.
 template <int T> __device__ __forceinline__ void load_partial(uint32_t taddr, float (&y)[T])
 {
     uint32_t d[8 * T];
@@ -163,18 +157,7 @@ template <int T> __device__ __forceinline__ void load_partial(uint32_t taddr, fl
     }
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int t = 0; t < T; t++) {
-        const uint32_t *q = d + 8 * t;
-        float ya = __uint_as_float(q[0]);
-        ya = fmaf(__uint_as_float(q[1]), 9.f, ya);
-        ya = fmaf(__uint_as_float(q[2]), 81.f, ya);
-        ya = fmaf(__uint_as_float(q[3]), 729.f, ya);
-        ya = fmaf(__uint_as_float(q[4]), 6561.f, ya);
-        ya = fmaf(__uint_as_float(q[5]), 59049.f, ya);
-        ya = fmaf(__uint_as_float(q[6]), 531441.f, ya);
-        ya = fmaf(__uint_as_float(q[7]), 4782969.f, ya);
-        y[t] = ya;
-    }
+    for (int t = 0; t < T; t++) y[t] = combine_digits(d + 8 * t);
 }
 
 // Units whose exchange slots exist at once.  Eight tokens: two matrices leave room for one unit's if the launch is to stay within
