@@ -121,11 +121,12 @@ INSG_API int insg_mxfp4_repack_umma(const uint32_t *weight, const uint8_t *scale
 INSG_API int insg_mxfp4_gemv_packed(const void *packed, const float *x, float *y, int rows, int cols, int M,
                                     insg_stream_t stream);
 
-/* Y[m][rows] = W x[m] for M tokens on the tcgen05 tensor cores (kind::mxf4, weights in the insg_mxfp4_repack_umma
- * layout, sixteen tokens per instruction, fp32-exact activations as eight balanced base-9 digit columns each); x fp32
- * [M][cols], y fp32
- * [M][rows].  The M >= 8 counterpart of insg_mxfp4_gemv_packed (src/decode.cu:13 applied to M tokens; the reference
- * has no batched form).  scratch: insg_umma_gemm_scratch_bytes(cols, M) of device memory. */
+/* Y[m][rows] = W x[m] for M tokens (1 <= M <= 4096) on the tcgen05 tensor cores (kind::mxf4, weights in the
+ * insg_mxfp4_repack_umma layout, activations as eight balanced base-9 digit columns each, 25 bits relative to the largest
+ * element of their group of 32); x fp32 [M][cols], y fp32 [M][rows].  Up to eight tokens go through the GEMV kernel, more
+ * through the GEMM kernel, 16 tokens per instruction up to 48 and 24 beyond.  The counterpart of insg_mxfp4_gemv_packed for
+ * that layout (src/decode.cu:13 applied to M tokens; the reference has no batched form).  An infinity or NaN in x[m] makes
+ * Y[m] NaN.  scratch: insg_umma_gemm_scratch_bytes(cols, M) of device memory (not used up to eight tokens). */
 INSG_API size_t insg_umma_gemm_scratch_bytes(int cols, int tokens);
 INSG_API int insg_mxfp4_gemm_umma(const void *packed_umma, const float *x, float *y, int rows, int cols, int M, void *scratch,
                                   size_t scratch_bytes, insg_stream_t stream);
@@ -217,15 +218,17 @@ typedef struct insg_gemv_op {
     int layout;               /* weight layout of every segment: 0 = insg_mxfp4_repack records, 1 = insg_mxfp4_repack_umma   */
     int *error_flag;          /* set to 1 if a bounded wait inside the kernel ran out (device int), or NULL                 */
     int pdl;                  /* 1: launch with programmatic dependent launch          */
-    const float *prep_partials; /* INSG_PRO_PREPARED: the producer's prep_partials [296], or NULL                        */
-    int prep_rms;               /* INSG_PRO_PREPARED: 1 = scale by the RMS factor computed from prep_partials            */
+    const float *prep_partials; /* INSG_PRO_PREPARED: the producer's prep_partials (layout 0: [296], layout 1:
+                                   [tokens][cols / 32]), or NULL                                                         */
+    int prep_rms;               /* INSG_PRO_PREPARED: 1 = scale by the RMS factor computed from prep_partials (layout 1
+                                   refuses it without them)                                                              */
     int tokens;                 /* 0 or 1: one token.  More: consecutive tokens of one sequence in one call (the weights are
                                    streamed once per pass): in, aux and x_out are [tokens][cols], every out is
                                    [tokens][rows]; the convolution history is advanced token by token.  layout 0: 2 to 4
-                                   tokens (one launch of the mma.sync kernel); layout 1: any count up to 4096, up to eight
-                                   in one launch of the GEMV kernel, more through the GEMM kernel, sixteen tokens per
-                                   tcgen05 instruction (needs umma_scratch).  Not with INSG_PRO_PREPARED, prepared
-                                   outputs or INSG_EPI_LOGITS. */
+                                   tokens (one launch of the mma.sync kernel; no prepared inputs or outputs); layout 1: any
+                                   count up to 4096, up to eight in one launch of the GEMV kernel (prepared inputs and
+                                   outputs included), more through the GEMM kernel, 16 or 24 tokens per tcgen05 instruction
+                                   (needs umma_scratch; no prepared inputs or outputs).  Not with INSG_EPI_LOGITS. */
     void *umma_scratch;         /* layout 1 with tokens > 8: device scratch of insg_umma_gemm_scratch_bytes(cols, tokens) for
                                    the activations' digit image, rewritten by every call                                      */
     size_t umma_scratch_bytes;
@@ -390,11 +393,12 @@ typedef struct insg_attn_op {
 INSG_API int insg_attention_step(const insg_attn_op *op /* host */, insg_stream_t stream);
 /* `tokens` consecutive tokens of one sequence in two launches (prompt processing): op describes token 0 (rotary position
  * and cache row *position + position_offset); token m takes qraw + m * 8192, k_raw + m * 1024, v + m * 1024, writes
- * out + m * 4096 and cache row + m, and attends the rows up to its own.  scratch: tokens * insg_gqa_scratch_bytes(.)
- * bytes whose first 64 bytes per token are zero before the first use (the kernel leaves them zero); q_scratch: device,
- * tokens * 4096 floats.  rows_hint: 0, or an upper bound of the rows the LAST token of the chunk attends (*position +
+ * out + m * 4096 and cache row + m, and attends the rows up to its own; a token whose row lies outside the cache is left
+ * alone.  scratch: up to 32 tokens, tokens * insg_gqa_scratch_bytes(.) bytes whose first 64 bytes per token are zero before the
+ * first use (the kernel leaves them zero); more tokens use none.  q_scratch: device, tokens * 4096 floats.  rows_hint: 0, or an upper bound of the rows the LAST token of the chunk attends (*position +
  * position_offset + tokens) when the host knows it: short contexts then start fewer CTAs (the results do not depend on it
- * while it holds).  op->pdl is ignored (plain stream order).  Same math per token as insg_attention_step. */
+ * while it holds).  op->pdl is ignored (plain stream order).  Up to 32 tokens have the bits of insg_attention_step; more go
+ * through query tiles on the tensor cores, the same sums in another order.  op->image: up to 8 tokens. */
 INSG_API int insg_attention_chunk(const insg_attn_op *op /* host */, int tokens, float *q_scratch, int rows_hint, insg_stream_t stream);
 /* The cache rows of those tokens alone (keys normalised and rotated, values), for a block whose outputs nobody reads: k_raw, v,
  * k_norm_w, the caches, position and the cache's description are used. */

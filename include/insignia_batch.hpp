@@ -3,7 +3,8 @@
 // Additive: the reference decodes one sequence (include/insignia_decode.hpp:5-24, src/decode.cu:14-23).  A batch step
 // runs the same fused operations, with every weight matrix streamed once for all sequences: the GEMVs take the
 // sequences as the tokens of a several-token tcgen05 launch, the DeltaNet step runs one grid row per sequence, the
-// attention step all sequences in one launch, each on its own cache.  Every sequence has its own recurrent state, convolution history and KV cache; all
+// attention step all sequences in one launch, each on its own cache.  Every sequence has its own recurrent state,
+// convolution history and KV cache; all
 // advance by one position per step.
 #pragma once
 #include "insignia_qwen35.hpp"

@@ -71,7 +71,8 @@ public:
     float *multi{};      // device: activations of up to 512 consecutive tokens (forward_tokens)
     void *umma_scratch{}; // device: digit image of the activations for the tcgen05 kernel (forward_tokens)
     size_t umma_scratch_bytes{};
-    void *prep{};        // device: prepared GEMV inputs, fp16 [2][4096] + fp16 [2][12288] + fp32 [2][296] sums of squares
+    void *prep{};        // device: prepared inputs of products and sums of squares (digit images of up to eight tokens on tcgen05, the
+                         // fp16 pieces of one token on mma.sync)
     void reset(); // zero recurrent state and position, as a fresh workspace
 
 private:
@@ -87,7 +88,8 @@ public:
     void layer(int layer);
     int decode_token(int token);
     void forward_token(int token);
-    // Additive: forward_token for `count` consecutive tokens (a prompt), in passes of up to 512 over the weights; leaves the same state as the loop would, and the logits and arg-max of the last token.
+    // Additive: forward_token for `count` consecutive tokens (a prompt), in passes of up to 512 over the weights; leaves the
+    // state the loop would (to fp32 rounding), and the logits and arg-max of the last token.
     void forward_tokens(const int *tokens, int count);
     int logits_argmax();
     int mtp_draft(int input_token);

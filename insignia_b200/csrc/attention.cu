@@ -166,8 +166,8 @@ __device__ __forceinline__ void attn_mma_warp(const void *kc, const void *vc, in
 // scratch, fence or ticket.  Longer ones use up to `clusters` clusters per head; their results go to scratch and the last one
 // to arrive (a ticket per CTA rank) folds them in order.  For one launch's clusters the cut depends on the row count alone; the
 // clusters on the cache's type and capacity and, in a batch, on how many sequences share the device (launch_attn).
-// Measured (fp32 cache, one step): 40 rows 5.2 us (7.1 with one CTA per split and a ticket), 8 x 600 rows 13.5 (38.5),
-// 8 x 5000 rows 57 (119.5, 88 % of the copy peak); 1024 rows 9.9 (9.5).
+// Measured as graph replays (fp32 cache, one step; in brackets with one CTA per split and a ticket): 40 rows 6.0 us (7.1), 1024
+// rows 9.8 (10.3), 8 x 600 rows 16.2 (38.5), 8 x 5000 rows 60 (119.5), which is 5.4 TB/s, 84 % of the copy peak.
 constexpr int kCtaRows = 48;    // rows per CTA from which another cluster is put to work (32, 48, 64, 96 tried: 48 is best or next to it)
 constexpr int kMaxClusters = 8; // per kv head
 

@@ -14,8 +14,8 @@
 // The instruction rounds its accumulator toward zero every time, and a sum kept in it through a whole row is off by some 1e-6.
 // So it only adds the products with a lo piece, 2^-11 of the rest, to a running sum; 16 products hi * hi start from zero and
 // are added outside, compensated, and so are the outputs.  Distance from float64 (2-norm, 512 tokens behind 512 rows):
-// 1.6e-7 (fp32 cache), 1.5e-7 (bf16), the split-K kernel's 1.8e-7; with everything left to the accumulator 2.4e-6 and 1.6e-6,
-// at 155 and 118 us instead of 226 and 163.
+// 1.6e-7 (fp32 cache), 1.4e-7 (bf16), the split-K kernel's 1.8e-7; with everything left to the accumulator 2.4e-6 and 1.6e-6,
+// at 155 and 118 us instead of 220 and 156 (226 and 163 without the packed additions).
 //
 // Eight warps: warp & 3 = 16 of the query rows, warp >> 2 = which half of the 32 keys a warp scores and which half of the 256
 // dims it sums; the two warps of a row exchange maxima and weights through shared memory.  Per tile of 32 keys a warp issues
@@ -68,6 +68,13 @@ __device__ __forceinline__ void add_compensated(float &sum, float &rest, float x
 {
     const float y = x + rest, z = sum + y;
     rest = y - (z - sum);
+    sum = z;
+}
+// The same for two numbers in the packed fp32 instructions.
+__device__ __forceinline__ void add_compensated(unsigned long long &sum, unsigned long long &rest, float x0, float x1)
+{
+    const unsigned long long y = add2(pack2(x0, x1), rest), z = add2(sum, y), minus = pack2(-1.f, -1.f);
+    rest = fma2(fma2(sum, minus, z), minus, y);
     sum = z;
 }
 // hi and lo fp16 pieces of two scaled values
@@ -237,11 +244,9 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
         }
     }
 
-    float o[16][4], oc[16][4]; // [8 dims each][row g: dims 2t, 2t+1 | row g + 8: dims 2t, 2t+1]; the sum is o + oc
+    unsigned long long o[16][2], oc[16][2]; // [8 dims each][rows g, g + 8]: dims 2t, 2t+1; the sum is o + oc
 #pragma unroll
-    for (int j = 0; j < 16; j++)
-#pragma unroll
-        for (int c = 0; c < 4; c++) o[j][c] = oc[j][c] = 0.f;
+    for (int j = 0; j < 16; j++) o[j][0] = o[j][1] = oc[j][0] = oc[j][1] = 0ull;
     float m_run[2] = {-3.0e38f, -3.0e38f}, l_run[2] = {0.f, 0.f}, l_rest[2] = {0.f, 0.f}; // rows g and g + 8 (l: this thread's share of its keys)
     int ev = 24;                                                  // exponent of the running value scale
     const int limit0 = pos0 + q0 + ((rg * 16 + g) >> 2), limit1 = pos0 + q0 + ((rg * 16 + g + 8) >> 2); // last row each query row sees
@@ -313,11 +318,14 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
         __syncthreads(); // the pieces are complete
         const int key0 = tile * kTileKeys + kg * 16 + 2 * t; // this thread's first key of four
         // ---- scores of 16 rows x 16 keys ----
-        float s[2][4], comp[2][4], low[2][4]; // sums of hi*hi, what their additions rounded off, sums with a lo piece
+        float s[2][4], low[2][4]; // sums with a lo piece
+        unsigned long long high[2][2], rest[2][2]; // sums of hi*hi (rows g and g + 8), what their additions rounded off
 #pragma unroll
-        for (int n = 0; n < 2; n++)
+        for (int n = 0; n < 2; n++) {
+            high[n][0] = high[n][1] = rest[n][0] = rest[n][1] = 0ull;
 #pragma unroll
-            for (int c = 0; c < 4; c++) s[n][c] = comp[n][c] = low[n][c] = 0.f;
+            for (int c = 0; c < 4; c++) low[n][c] = 0.f;
+        }
 #pragma unroll 4
         for (int i = 0; i < 16; i++) {
             uint32_t qh[4], ql[4], kh[4], kl[4];
@@ -336,7 +344,7 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
 #pragma unroll
             for (int n = 0; n < 2; n++)
 #pragma unroll
-                for (int c = 0; c < 4; c++) add_compensated(s[n][c], comp[n][c], part[n][c]);
+                for (int h = 0; h < 2; h++) add_compensated(high[n][h], rest[n][h], part[n][2 * h], part[n][2 * h + 1]);
         }
         // ---- online softmax (rows g and g + 8; a row's 32 keys sit in the quads of two warps) ----
         const float sc = invq * scale_down(ek);
@@ -345,7 +353,8 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
         for (int n = 0; n < 2; n++)
 #pragma unroll
             for (int c = 0; c < 4; c++) {
-                s[n][c] = (s[n][c] + (low[n][c] + comp[n][c])) * sc;
+                const float2 a = unpack2(high[n][c >> 1]), b = unpack2(rest[n][c >> 1]);
+                s[n][c] = (c & 1) ? (a.y + (low[n][c] + b.y)) * sc : (a.x + (low[n][c] + b.x)) * sc;
                 on[n][c] = key0 + n * 8 + (c & 1) <= (c < 2 ? limit0 : limit1);
             }
 #pragma unroll
@@ -391,10 +400,11 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
             for (int i = 0; i < 8; i++) w[k][i >> 2][i & 3] = s_p[rg][k][i][lane];
         const float c0 = corr[0] * fv, c1 = corr[1] * fv;
         if (__any_sync(0xffffffffu, c0 != 1.f || c1 != 1.f)) {
+            const unsigned long long f0 = pack2(c0, c0), f1 = pack2(c1, c1);
 #pragma unroll
             for (int j = 0; j < 16; j++) {
-                o[j][0] *= c0; o[j][1] *= c0; o[j][2] *= c1; o[j][3] *= c1;
-                oc[j][0] *= c0; oc[j][1] *= c0; oc[j][2] *= c1; oc[j][3] *= c1;
+                o[j][0] = mul2(o[j][0], f0); o[j][1] = mul2(o[j][1], f1);
+                oc[j][0] = mul2(oc[j][0], f0); oc[j][1] = mul2(oc[j][1], f1);
             }
         }
         // ---- values: 128 of the 256 dims, 16 keys and 16 dims at a time; the small products first, one rounding of the large one ----
@@ -420,7 +430,7 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
 #pragma unroll
                 for (int n = 0; n < 2; n++)
 #pragma unroll
-                    for (int c = 0; c < 4; c++) add_compensated(o[2 * j + n][c], oc[2 * j + n][c], part[n][c]);
+                    for (int h = 0; h < 2; h++) add_compensated(o[2 * j + n][h], oc[2 * j + n][h], part[n][2 * h], part[n][2 * h + 1]);
             }
         }
     }
@@ -445,8 +455,10 @@ __global__ void __launch_bounds__(kTThreads, 1) attn_tile_kernel(const __grid_co
         if (live(tok)) {
             float *dst = p.out + (size_t(tok) * 16 + kvh * 4 + (r & 3)) * 256 + kg * 128 + 2 * t;
 #pragma unroll
-            for (int j = 0; j < 16; j++)
-                *reinterpret_cast<float2 *>(dst + 8 * j) = make_float2(quotient(o[j][2 * h], oc[j][2 * h]), quotient(o[j][2 * h + 1], oc[j][2 * h + 1]));
+            for (int j = 0; j < 16; j++) {
+                const float2 a = unpack2(o[j][h]), b = unpack2(oc[j][h]);
+                *reinterpret_cast<float2 *>(dst + 8 * j) = make_float2(quotient(a.x, b.x), quotient(a.y, b.y));
+            }
         }
     }
 }

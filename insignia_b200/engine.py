@@ -25,7 +25,8 @@ class Engine:
                  use_pdl: bool = True, n_layers: int = 32, vocab: int = 248320, device: int = 0,
                  gemv_tcgen05: bool = False, prepared_inputs: bool = True, persistent: bool = False, prefill_tcgen05: bool = True):
         """``persistent=False`` (default): one launch per fused operation, replayed from a CUDA graph when ``use_graph``;
-        ``True``: a token step is one persistent cooperative launch (``insg_program_*``)."""
+        ``True``: a token step is one persistent cooperative launch (``insg_program_*``).  The products run on tcgen05; with
+        ``prepared_inputs=False`` or ``persistent=True`` on mma.sync, unless ``gemv_tcgen05`` asks for tcgen05."""
         o = EngineOptions(budget_bytes, max_context, int(kv_bf16), int(gate_elementwise), int(accurate_trig),
                           int(use_graph), int(use_pdl), int(gemv_tcgen05), n_layers, vocab, device, int(persistent), int(not prefill_tcgen05),
                           int(not prepared_inputs))
@@ -59,7 +60,7 @@ class Engine:
         check(_lib.lib().insg_engine_forward_token(self._h, token))
 
     def forward_tokens(self, tokens):
-        """``forward_token`` over a list of consecutive tokens, four per pass over the weights (prompt processing)."""
+        """``forward_token`` over a list of consecutive tokens (a prompt), in passes of up to 512 over the weights."""
         arr = (C.c_int * len(tokens))(*[int(t) for t in tokens])
         check(_lib.lib().insg_engine_forward_tokens(self._h, arr, len(tokens)))
 

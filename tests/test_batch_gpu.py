@@ -23,7 +23,7 @@ def small_engine(idx, **kw):
 @pytest.mark.parametrize("sequences", [1, 2, 3, 4, 5, 8])
 def test_batch_equals_independent_engines(cuda, golden_ckpt, sequences):
     """Every sequence of a batch decodes the tokens the single-sequence engine decodes from the same prompt; states agree
-    to rounding (1..4 sequences ride the mma.sync kernel, 5..8 the tcgen05 kernel)."""
+    to rounding (the batch's products are tcgen05 launches, the engine's here mma.sync ones)."""
     from insignia_b200.engine import Batch
 
     rng = np.random.default_rng(sequences)
