@@ -84,7 +84,7 @@ def parse_args():
     ap.add_argument("--kv-bf16", action="store_true", help="bf16 KV cache (the default is the reference's fp32 cache)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-reference-check", action="store_true", help="skip comparing the generated tokens with the reference engine")
-    ap.add_argument("--gemv", default="mma", choices=["mma", "tcgen05"], help="GEMV kernel family of the engine")
+    ap.add_argument("--gemv", default="mma", choices=["mma", "tcgen05"], help="GEMV kernel family of the persistent kernel's engine (the graph of launches runs tcgen05)")
     ap.add_argument("--persistent", action="store_true", help="the persistent token kernel (one cooperative launch per token) instead of the graph of launches")
     ap.add_argument("--prefetch", type=int, default=-1, help="persistent kernel: weight records per warp kept prefetched into L2 (-1 = default)")
     ap.add_argument("--batch", type=int, default=1, help="config 4: sequences per GPU decoded in lock step (1..8)")

@@ -9,10 +9,11 @@
 // every one exact in E2M1, as in umma_gemv.cu.  Column j of a token holds digit j of every element; the eight columns are
 // combined as sum_j 9^j D_j in fp32 by the epilogue, which gives the product to ~1e-7.  A token takes 8 columns of N.
 //
-// What bounds it: filling shared memory.  A stage multiplies two 128-row weight records (17.4 KB) with the digits of a group
-// of tokens; an SM takes in some 52 bytes a clock from L2, and sixteen tokens' digits (8.2 KB, N = 128) left the tensor pipe
-// half idle.  Twenty-four tokens (12.3 KB, N = 192) are half as much work again per stage for 16 % more bytes, and tensor
-// memory holds their two accumulators (384 of 512 columns) beside the scale factors; 24576 x 4096 at 512 tokens: 182 -> 153 us.
+// What bounds it: filling shared memory and the tensor pipe together (77 % busy at 512 tokens).  A stage multiplies two 128-row
+// weight records (17.4 KB) with the digits of a group of tokens; an SM takes in some 52 bytes a clock from L2, and sixteen
+// tokens' digits and scales (8.7 KB, N = 128) left the tensor pipe half idle.  Twenty-four tokens (13.3 KB, N = 192) are half as
+// much work again per stage for 18 % more bytes, and tensor memory holds their two accumulators (384 of 512 columns) beside the
+// scale factors; 24576 x 4096 at 512 tokens: 182 -> 150 us.
 //
 // Kernels:
 //   umma_digitize_kernel  one CTA per token: the fused activation prologue (RMSNorm, gates, ...), then the digit

@@ -971,7 +971,8 @@ void Qwen35Decode::run_prompt(const int *tokens, int count, bool mtp)
     load_head();
     load_embed();
     Ctx c{x_, p.stream, x_.options.use_pdl, launches_, false, nullptr, nullptr};
-    // Long prompts go through the tcgen05 GEMM in passes of up to kBigChunk tokens; what is left, and short prompts, through the engine's own GEMV: up to eight tokens a pass on tcgen05, four on mma.sync.
+    // Long prompts go through the tcgen05 GEMM in passes of up to kBigChunk tokens; what is left, and short prompts, through
+    // the engine's own GEMV: up to eight tokens a pass on tcgen05, four on mma.sync.
     const bool one_layout = tcgen05_engine(x_.options);
     const bool big = x_.options.prefill_tcgen05 && count > (one_layout ? kSmallChunk : 15);
     if (big && !one_layout)
