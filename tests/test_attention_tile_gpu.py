@@ -47,6 +47,6 @@ def test_attention_tiles_vs_float64(cuda, kv_bf16, tokens, start, spread):
             x = K[:n, h >> 2] @ q[m, h] / 16
             p = np.exp(x - x.max())
             want = (p / p.sum()) @ V[:n, h >> 2]
-            # fp16 pieces keep 22 bits of every operand; scores of a few units turn their error into the same relative error
+            # fp16 pieces round every operand to 23 bits; scores of a few units turn their error into the same relative error
             # of a weight, and the fp32 rotation angle of position 1300 is good to 1300 * 2^-24: 5e-5 as for the split kernel
             assert np.max(np.abs(got[m, h] - want)) <= 5e-5 * np.abs(V[:n, h >> 2]).max(), (m, h)

@@ -1,4 +1,4 @@
-"""The several-token tcgen05 GEMM (eight or sixteen tokens per kind::mxf4 instruction, stream-K shares), through the C ABI, against the CPU oracle
+"""The several-token tcgen05 GEMM (16 or 24 tokens per kind::mxf4 instruction, stream-K shares), through the C ABI, against the CPU oracle
 and against the one-token kernels."""
 import os
 import sys
