@@ -63,6 +63,11 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t b
                  ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 
+__device__ __forceinline__ void bulk_prefetch(const void *src, uint32_t bytes) // to L2
+{
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+
 // ---- tcgen05 instructions as the kernels issue them ----
 __device__ __forceinline__ void copy_scales(uint32_t taddr, uint64_t desc)
 {

@@ -47,6 +47,13 @@ constexpr uint32_t kDSfaCol = 128, kDSfbCol = 160, kDTmemCols = 256; // accumula
 // then fit an SM's 228 KB with their static part (at most 1 KB, which is why eight tokens' sums of squares are not in it) and
 // the 1 KB the hardware keeps per CTA.
 constexpr int kDHalfSm = 112 * 1024;
+// The next launch may start when at most this many ring stages of a CTA are still to be requested, and asks L2 for a few beyond its
+// own ring.  Its requests share the SM's copy engine and the memory with this launch's: made while this launch still streams they delay
+// the stages it waits for.  The four products of a block with one token: 28.1 us with the next launch at once, 26.6 like this, 29.3 at
+// the very end, when its ring cannot fill in time; L2 asked for six stages 27.8, for all of them 28.0.  Eight tokens 35.3 -> 34.4 us,
+// where asking L2 gains nothing.  A token 1.16 -> 1.115 ms, a step of three or eight sequences 1 % less.
+template <int T> constexpr int kDTriggerStages = T <= 2 ? 6 : 4;
+template <int T> constexpr int kDAheadStages = T <= 2 ? 3 : 0;
 
 struct DSeg {
     const uint8_t *packed, *packed2;
@@ -233,9 +240,9 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    // The next launch may become resident now, not earlier: were it to take tensor memory before every CTA here has its own,
+    // The next launch may become resident from here on, not earlier: were it to take tensor memory before every CTA here has its own,
     // a CTA could wait for memory held by a CTA that waits for this grid.
-    pdl_launch_dependents();
+    if (warp == 9 && nstages - kDTriggerStages<T> <= S) pdl_launch_dependents();
     cluster_arrive();
     cluster_wait(); // the peers' barriers exist from here on
     const uint32_t tmem = s_tmem;
@@ -345,6 +352,11 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         // ---- producer ----------------------------------------------------------------------------------------------------------
         {
             const bool one = elect_one();
+            for (int i = S + lane; i < min(nstages, S + kDAheadStages<T>); i += 32) {
+                const int run = i / spt, st = i - run * spt;
+                bulk_prefetch(run_src(run) + size_t(st) * kDStage, uint32_t(min(2, len - 2 * st)) * kURec);
+            }
+            __syncwarp();
             if (prepared) { // the digits come ready: eight k-blocks per copy, so that the multiplies can start behind the first
                 pdl_wait();
                 asm volatile("fence.proxy.async.global;" ::: "memory"); // written by ordinary stores of the launch before
@@ -365,6 +377,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                         ok = mbar_wait(&empty[slot], phase, abort_flag);
                         if (!ok) break;
                         if (one) load_stage(slot, src, st);
+                        if (i == nstages - 1 - kDTriggerStages<T>) pdl_launch_dependents();
                     }
                     if (++slot == S) { slot = 0; phase ^= 1; }
                 }
