@@ -122,9 +122,9 @@ INSG_API int insg_mxfp4_gemv_packed(const void *packed, const float *x, float *y
                                     insg_stream_t stream);
 
 /* Y[m][rows] = W x[m] for M tokens (1 <= M <= 4096) on the tcgen05 tensor cores (kind::mxf4, weights in the
- * insg_mxfp4_repack_umma layout, activations as eight balanced base-9 digit columns each, 25 bits relative to the largest
- * element of their group of 32); x fp32 [M][cols], y fp32 [M][rows].  Up to eight tokens go through the GEMV kernel, more
- * through the GEMM kernel, 16 tokens per instruction up to 48 and 24 beyond.  The counterpart of insg_mxfp4_gemv_packed for
+ * insg_mxfp4_repack_umma layout, activations as seven base-13 digit columns each (eight balanced base-9 ones up to eight
+ * tokens), at least 25 bits relative to the largest element of their group of 32); x fp32 [M][cols], y fp32 [M][rows].  Up to eight tokens go through the GEMV kernel, more
+ * through the GEMM kernel, 16 tokens per instruction up to 48 and 32 beyond.  The counterpart of insg_mxfp4_gemv_packed for
  * that layout (src/decode.cu:13 applied to M tokens; the reference has no batched form).  An infinity or NaN in x[m] makes
  * Y[m] NaN.  scratch: insg_umma_gemm_scratch_bytes(cols, M) of device memory (not used up to eight tokens). */
 INSG_API size_t insg_umma_gemm_scratch_bytes(int cols, int tokens);
@@ -227,7 +227,7 @@ typedef struct insg_gemv_op {
                                    [tokens][rows]; the convolution history is advanced token by token.  layout 0: 2 to 4
                                    tokens (one launch of the mma.sync kernel; no prepared inputs or outputs); layout 1: any
                                    count up to 4096, up to eight in one launch of the GEMV kernel (prepared inputs and
-                                   outputs included), more through the GEMM kernel, 16 or 24 tokens per tcgen05 instruction
+                                   outputs included), more through the GEMM kernel, 16 or 32 tokens per tcgen05 instruction
                                    (needs umma_scratch; no prepared inputs or outputs).  Not with INSG_EPI_LOGITS. */
     void *umma_scratch;         /* layout 1 with tokens > 8: device scratch of insg_umma_gemm_scratch_bytes(cols, tokens) for
                                    the activations' digit image, rewritten by every call                                      */

@@ -38,7 +38,7 @@ struct DecodeOptions {
                                    // tile-layout copy for every pass size).  With `persistent` they stay on the mma.sync
                                    // kernel, whose producers leave the next product's input ready as fp16 pieces.
                                    // false: the mma.sync kernel, every product preparing its own input
-    bool prefill_tcgen05 = true;   // prompts: passes of up to 512 tokens through the tcgen05 GEMM (16 or 24 tokens per
+    bool prefill_tcgen05 = true;   // prompts: passes of up to 512 tokens through the tcgen05 GEMM (16 or 32 tokens per
                                    // instruction); false: passes of eight (tcgen05) or four (mma.sync) tokens
     int n_layers = Qwen35Shape::layers;
     int vocab = Qwen35Shape::vocab;

@@ -4,21 +4,21 @@
 //
 // tcgen05.mma.kind::mxf4.block_scale, weights as the A operand in their native packed E2M1 + UE8M0 form (the tile layout of
 // insg_mxfp4_repack_umma, nothing dequantised), accumulators in tensor memory.  The activations are the B operand.
-// kind::mxf4 wants E2M1 there too, so each fp32 activation is written as a 25-bit signed fixed-point number (relative to the
-// largest element of its group of 32, whose power of two is the group's UE8M0 scale) in balanced base 9: eight digits -4..4,
-// every one exact in E2M1, as in umma_gemv.cu.  Column j of a token holds digit j of every element; the eight columns are
-// combined as sum_j 9^j D_j in fp32 by the epilogue, which gives the product to ~1e-7.  A token takes 8 columns of N.
+// kind::mxf4 wants E2M1 there too, so each fp32 activation is written as a signed fixed-point number of at least 25 bits (relative to
+// the largest element of its group of 32, whose power of two is the group's UE8M0 scale) in base 13 with the digits 0, +-1..+-4, +-6 and
+// +-8, every one exact in E2M1: seven digits, where umma_gemv.cu's balanced base 9 takes eight.  Column j * tokens + t of a group holds
+// digit j of its token t; the epilogue combines the seven as sum_j 13^j D_j in fp32, which gives the product to ~7e-8 (4096 columns,
+// normal inputs; base 9: 8e-8).  A token takes 7 columns of N.
 //
-// What bounds it: filling shared memory and the tensor pipe together (77 % busy at 512 tokens).  A stage multiplies two 128-row
-// weight records (17.4 KB) with the digits of a group of tokens; an SM takes in some 52 bytes a clock from L2, and sixteen
-// tokens' digits and scales (8.7 KB, N = 128) left the tensor pipe half idle.  Twenty-four tokens (13.3 KB, N = 192) are half as
-// much work again per stage for 18 % more bytes, and tensor memory holds their two accumulators (384 of 512 columns) beside the
-// scale factors; 24576 x 4096 at 512 tokens: 182 -> 150 us.
+// What bounds it: filling shared memory and the tensor pipe together.  A stage multiplies two 128-row weight records (17.4 KB) with the
+// digits of a group of tokens; an SM takes in some 55 bytes a clock from L2.  Thirty-two tokens (15.4 KB, N = 224) fill tensor memory
+// (448 of 512 columns, beside the scale factors) and make the most of the weights' bytes; 24576 x 4096 at 512 tokens: 150 us with eight
+// digits and 24 tokens, 127 like this.
 //
 // Kernels:
 //   umma_digitize_kernel  one CTA per token: the fused activation prologue (RMSNorm, gates, ...), then the digit
 //                         image of the token in global memory, laid out as the shared-memory image the MMA reads
-//                         ([k-block][group of tokens][512 bytes x tokens per group, scale blocks], canonical K-major, no swizzle);
+//                         ([k-block][group of tokens][448 bytes x tokens per group, scale blocks], canonical K-major, no swizzle);
 //   umma_gemm_kernel      one CTA per SM.  The work is the sequence of all (pair of records, token group, k-block) stages;
 //                         every CTA takes an equal contiguous share of it (stream-K), so SMs are busy whatever the number
 //                         of tiles.  The pair is two row tiles, or the gate and the up tile of the same rows for SwiGLU
@@ -43,14 +43,85 @@ namespace insg {
 
 constexpr int kGThreads = kProThreads;     // digitize kernel: the activation prologue is written for this many threads
 constexpr int kGemmThreads = 192;          // GEMM kernel: four epilogue warps, the MMA issuer, the producer
-constexpr int kDigits = 8;                 // balanced base-9 digits per activation = N columns per token
-constexpr int kGSfaBufs = 8;               // scale-factor column sets cycled by stage (a power of two)
-constexpr int kGTmemCols = 512;            // two accumulators of up to 192 columns, weight scale factors [384,448), digit scale factors [448,512)
+constexpr int kDigits = 7;                 // base-13 digits per activation = N columns per token
+constexpr int kGSfaBufs = 4;               // scale-factor column sets cycled by stage (a power of two)
+constexpr int kGTmemCols = 512;            // two accumulators of up to 224 columns, weight scale factors [448,480), digit scale factors [480,512)
 constexpr int kGMaxStages = 16;
 constexpr int kGMaxGrid = 256;             // partial-sum slots and tickets are sized for this many CTAs
-constexpr int kSlotFloats = 128 * 24;      // one partial: 128 rows x up to 24 tokens
-// A k-block of a token group in the digit image: the digits (8 columns x 64 bytes per token), then a 512-byte scale block per 128 columns.
-__host__ __device__ constexpr int digit_block(int tpg) { return 512 * tpg + (tpg + 15) / 16 * 512; }
+constexpr int kSlotFloats = 128 * 32;      // one partial: 128 rows x up to 32 tokens
+// A k-block of a token group in the digit image: the digits (kDigits columns x 64 bytes per token; column = digit * tpg + token), then a
+// 512-byte scale block per 128 columns.
+__host__ __device__ constexpr int digit_bytes(int tpg) { return 64 * kDigits * tpg; }
+__host__ __device__ constexpr int digit_block(int tpg) { return digit_bytes(tpg) + (kDigits * tpg + 127) / 128 * 512; }
+
+// ---- seven digits of an activation -----------------------------------------------------------------------------------------------
+// E2M1 holds 0, 1, 2, 3, 4, 6, 8 and 12 halves of either sign.  Of these, {0, +-1, +-2, +-3, +-4, +-6, +-8} has every residue modulo 13
+// once (5 = -8, 7 = -6, 9..12 = -4..-1), so every integer has base-13 digits in it, and seven of them hold all |v| <= 4 1/3 * 13^6 =
+// 2^24.3: what is left for the seventh is -4..4.  Balanced base 9 takes eight digits for 2^24: an eighth more to multiply and to move.
+// Two digits at a time come from a table, with the carry that the negative ones leave to the next two; the halves go into the
+// group's scale.
+constexpr int kPair = 169, kSixDigits = kPair * kPair * kPair; // 13^2, 13^6
+__device__ __forceinline__ uint16_t digit_pair13(int n) // table entry: the codes of the two digits, least significant first, the carry in bit 8
+{
+    uint32_t r = 0;
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int m = n % 13;
+        const int d = m <= 4 || m == 6 || m == 8 ? m : m - 13, mag = d < 0 ? -d : d;
+        r |= uint32_t((mag <= 4 ? mag : mag == 6 ? 5 : 6) | (d < 0 ? 8 : 0)) << (4 * i);
+        n = (n - d) / 13;
+    }
+    return uint16_t(r | uint32_t(n) << 8);
+}
+// Seven codes of round(x * alpha) (|.| <= 4 1/3 * 13^6), digit j in nibble j.
+__device__ __forceinline__ uint32_t digit_codes13(float x, float alpha, const uint16_t *table)
+{
+    const int v = max(-20916000, min(__float2int_rn(x * alpha), 20916000));
+    const uint32_t u = uint32_t(v + 5 * kSixDigits); // a multiple of 13^6: only the seventh digit sees it
+    uint32_t q = u / uint32_t(kPair);
+    const uint32_t t0 = table[u - uint32_t(kPair) * q], u1 = q + (t0 >> 8);
+    q = u1 / uint32_t(kPair);
+    const uint32_t t1 = table[u1 - uint32_t(kPair) * q], u2 = q + (t1 >> 8);
+    q = u2 / uint32_t(kPair);
+    const uint32_t t2 = table[u2 - uint32_t(kPair) * q];
+    // what is left + 5 = 1..9 -> codes of -4..4
+    const uint32_t last = uint32_t(0x43210'9ABC0ull >> (4 * (q + (t2 >> 8)))) & 15u;
+    return (t0 & 0xFFu) | (t1 & 0xFFu) << 8 | (t2 & 0xFFu) << 16 | last << 24;
+}
+// A group's exponent (umma_common.cuh), one less where its largest magnitude leaves room for a bit more: 2^24 * 1.2422 fits.
+__device__ __forceinline__ int group_exponent13(uint32_t max_bits)
+{
+    const int eb = group_exponent(max_bits);
+    return eb - int(eb != 255 && int(max_bits >> 23) == eb && (max_bits & 0x7FFFFFu) < 0x1F0000u);
+}
+__device__ __forceinline__ uint8_t digit_scale(int eb) { return uint8_t(eb == 255 ? 255 : eb - 22); } // group_scale, times two for the halves
+
+// The digits of one 128-element k-block of token `t` of a group (four elements per lane) and their scales into the block at `blk`.
+template <int TPG> __device__ __forceinline__ void store_digits13(float4 x, int t, uint8_t *blk, const uint16_t *table, int lane)
+{
+    float mx = fmax_nan(fmax_nan(fabsf(x.x), fabsf(x.y)), fmax_nan(fabsf(x.z), fabsf(x.w)));
+    mx = fmax_nan(mx, __shfl_xor_sync(0xffffffffu, mx, 1)); // a group of 32 elements = 8 lanes
+    mx = fmax_nan(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    mx = fmax_nan(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+    const int eb = group_exponent13(__float_as_uint(mx));
+    const float alpha = group_alpha(eb);
+    const uint32_t c0 = digit_codes13(x.x, alpha, table), c1 = digit_codes13(x.y, alpha, table);
+    const uint32_t c2 = digit_codes13(x.z, alpha, table), c3 = digit_codes13(x.w, alpha, table);
+    // columns 0, 2, 4, 6 sit in the low nibbles of the four bytes, 1, 3, 5 in the high ones
+    const uint32_t e01 = (c0 & 0x0F0F0F0Fu) | ((c1 & 0x0F0F0F0Fu) << 4), e23 = (c2 & 0x0F0F0F0Fu) | ((c3 & 0x0F0F0F0Fu) << 4);
+    const uint32_t o01 = ((c0 >> 4) & 0x0F0F0F0Fu) | (c1 & 0xF0F0F0F0u), o23 = ((c2 >> 4) & 0x0F0F0F0Fu) | (c3 & 0xF0F0F0F0u);
+    uint8_t *dst = blk + (lane >> 4) * (digit_bytes(TPG) / 2) + (t >> 3) * 256 + ((lane >> 3) & 1) * 128 + (t & 7) * 16 + (lane & 7) * 2;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        *reinterpret_cast<uint16_t *>(dst + (2 * j) * (32 * TPG)) = uint16_t(__byte_perm(e01, e23, j | ((4 + j) << 4)));
+        if (j < 3) *reinterpret_cast<uint16_t *>(dst + (2 * j + 1) * (32 * TPG)) = uint16_t(__byte_perm(o01, o23, j | ((4 + j) << 4)));
+    }
+    // scale block: row = column mod 32, then the column quarter, byte = group; a token's columns share the four bytes
+    const uint32_t sc = digit_scale(eb);
+    const uint32_t w = __shfl_sync(0xffffffffu, sc, 0) | __shfl_sync(0xffffffffu, sc, 8) << 8 | __shfl_sync(0xffffffffu, sc, 16) << 16 | __shfl_sync(0xffffffffu, sc, 24) << 24;
+    if (lane < 2) // 16 tokens: columns of even and odd digits are rows t and 16 + t; 32: digits 0..3 and 4..6 are two blocks
+        *reinterpret_cast<uint4 *>(blk + digit_bytes(TPG) + (TPG == 16 ? (16 * lane + t) * 16 : 512 * lane + t * 16)) = make_uint4(w, w, w, w);
+}
 
 struct GSeg {
     const uint8_t *packed, *packed2;
@@ -77,19 +148,20 @@ struct DigitizeParams {
     ProIn pro;
     uint8_t *bimg;
     int *tickets;
-    int tokens, ngroups, tpg, parts; // a token's digits are written by `parts` CTAs, each a slice of the columns
+    int tokens, ngroups, parts; // a token's digits are written by `parts` CTAs, each a slice of the columns
 };
 
 // `parts` CTAs per token slot (slots beyond `tokens` are written as zeros so that their columns contribute nothing).  Every
 // CTA of a token runs the whole prologue (the norm needs all columns; that part is a few loads and one reduction) and writes
 // the digits of its slice of the k-blocks only: the digit extraction is the long part.
+template <int TPG>
 __global__ void __launch_bounds__(kGThreads, 2) umma_digitize_kernel(const __grid_constant__ DigitizeParams p)
 {
     __shared__ float scratch[64];
-    __shared__ uint8_t lut[84];
-    if (threadIdx.x < 81) lut[threadIdx.x] = digit_pair_code(threadIdx.x);
+    __shared__ uint16_t table[kPair];
+    if (threadIdx.x < kPair) table[threadIdx.x] = digit_pair13(int(threadIdx.x));
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); // the GEMM may set itself up and fetch weights meanwhile
-    const int m = blockIdx.x / p.parts, part = blockIdx.x - m * p.parts, grp = m / p.tpg, ms = m - grp * p.tpg;
+    const int m = blockIdx.x / p.parts, part = blockIdx.x - m * p.parts, grp = m / TPG, ms = m - grp * TPG;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float4 v[kMaxVec];
     if (m < p.tokens) {
@@ -111,7 +183,7 @@ __global__ void __launch_bounds__(kGThreads, 2) umma_digitize_kernel(const __gri
 #pragma unroll
     for (int j = 0; j < kMaxVec; j++) { // a warp holds a k-block per j
         const int kb = warp + j * (kGThreads / 32);
-        if (kb >= kb0 && kb < kb1) store_digits<true>(v[j], p.tpg, ms, p.bimg + (size_t(kb) * p.ngroups + grp) * digit_block(p.tpg), lut, lane);
+        if (kb >= kb0 && kb < kb1) store_digits13<TPG>(v[j], ms, p.bimg + (size_t(kb) * p.ngroups + grp) * digit_block(TPG), table, lane);
     }
 }
 
@@ -260,26 +332,41 @@ __device__ __forceinline__ void finish_row(const GParams &p, const GSeg &s, int 
     }
 }
 
-// The sums of the TPG tokens of one accumulator (TMEM lane = row, eight digit columns per token), digits combined.
-template <int TPG>
-__device__ __forceinline__ void load_sums(uint32_t taddr, float (&y)[TPG])
+// The sums of the TPG tokens of one accumulator (TMEM lane = row, column = digit * TPG + token), digits combined: least significant
+// first, 13^j is exact in fp32.
+template <int TPG> __device__ __forceinline__ void load_column_block(uint32_t taddr, uint32_t (&d)[TPG])
 {
+    static_assert(TPG == 16 || TPG == 32, "columns per load");
+    if constexpr (TPG == 32)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+                     "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+                     : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]),
+                       "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15]),
+                       "=r"(d[16]), "=r"(d[17]), "=r"(d[18]), "=r"(d[19]), "=r"(d[20]), "=r"(d[21]), "=r"(d[22]), "=r"(d[23]),
+                       "=r"(d[24]), "=r"(d[25]), "=r"(d[26]), "=r"(d[27]), "=r"(d[28]), "=r"(d[29]), "=r"(d[30]), "=r"(d[31])
+                     : "r"(taddr));
+    else
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                     : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]),
+                       "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15])
+                     : "r"(taddr));
+}
+template <int TPG> __device__ __forceinline__ void load_sums(uint32_t taddr, float (&y)[TPG])
+{
+    constexpr float kPower[kDigits] = {1.f, 13.f, 169.f, 2197.f, 28561.f, 371293.f, 4826809.f};
 #pragma unroll
-    for (int t0 = 0; t0 < TPG; t0 += 8) { // eight tokens (two loads of 32 columns) per wait
-        uint32_t d[2][32];
+    for (int t = 0; t < TPG; t++) y[t] = 0.f;
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-                         "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                         : "=r"(d[h][0]), "=r"(d[h][1]), "=r"(d[h][2]), "=r"(d[h][3]), "=r"(d[h][4]), "=r"(d[h][5]), "=r"(d[h][6]), "=r"(d[h][7]),
-                           "=r"(d[h][8]), "=r"(d[h][9]), "=r"(d[h][10]), "=r"(d[h][11]), "=r"(d[h][12]), "=r"(d[h][13]), "=r"(d[h][14]), "=r"(d[h][15]),
-                           "=r"(d[h][16]), "=r"(d[h][17]), "=r"(d[h][18]), "=r"(d[h][19]), "=r"(d[h][20]), "=r"(d[h][21]), "=r"(d[h][22]), "=r"(d[h][23]),
-                           "=r"(d[h][24]), "=r"(d[h][25]), "=r"(d[h][26]), "=r"(d[h][27]), "=r"(d[h][28]), "=r"(d[h][29]), "=r"(d[h][30]), "=r"(d[h][31])
-                         : "r"(taddr + kDigits * (t0 + 4 * h)));
-        }
+    for (int j = 0; j < kDigits; j += 2) { // two digits per wait
+        uint32_t d0[TPG], d1[TPG];
+        load_column_block<TPG>(taddr + j * TPG, d0);
+        if (j + 1 < kDigits) load_column_block<TPG>(taddr + (j + 1) * TPG, d1);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int t = 0; t < 8; t++) y[t0 + t] = combine_digits(&d[t >> 2][(t & 3) * 8]);
+        for (int t = 0; t < TPG; t++) {
+            y[t] = fmaf(__uint_as_float(d0[t]), kPower[j], y[t]);
+            if (j + 1 < kDigits) y[t] = fmaf(__uint_as_float(d1[t]), kPower[j + 1 < kDigits ? j + 1 : j], y[t]);
+        }
     }
 }
 
@@ -316,8 +403,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
     constexpr int kBBlock = digit_block(TPG);       // digits of the group's tokens for one k-block: 8 * TPG columns x 128 k x 4 bit, and their scales
     constexpr int kGStage = 2 * kURec + kBBlock;    // one ring stage: the pair's weight records + the digit block both multiply
     constexpr int N = kDigits * TPG;
-    constexpr uint32_t kSfaCol = 384, kSfbCol = 448;
-    static_assert(2 * N <= int(kSfaCol) && 8 * kGSfaBufs == int(kSfbCol - kSfaCol) && kSfbCol + 8 * kGSfaBufs == uint32_t(kGTmemCols), "tensor memory");
+    constexpr uint32_t kD1Col = TPG == 32 ? 224 : 128, kSfaCol = 448, kSfbCol = 480;
+    static_assert(N <= int(kD1Col) && kD1Col + N <= int(kSfaCol) && 8 * kGSfaBufs == int(kSfbCol - kSfaCol) && kSfbCol + 8 * kGSfaBufs == uint32_t(kGTmemCols), "tensor memory");
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int nkb = p.nkb, S = p.stages;
     uint8_t *ring = smem;                          // S stages of kGStage bytes
@@ -404,7 +491,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
         constexpr uint32_t idesc0 = (1u << 7) | (1u << 10) | ((uint32_t(N) >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
         constexpr uint32_t idesc1 = idesc0 | (2u << 29) | (2u << 4);
         const uint64_t da0 = umma_desc(smem_u32(ring), 128, 256), dsf0 = umma_desc(smem_u32(ring) + 8192, 16, 128);
-        const uint32_t d0 = tmem, d1 = tmem + uint32_t(N);
+        const uint32_t d0 = tmem, d1 = tmem + kD1Col;
         int st = 0, sfa = 0;
         uint32_t phase = 0;
         bool ok = true, here = mbar_test(&full[0], 0);
@@ -427,13 +514,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
                 if (one) {
                     copy_scales(sa, dsf);
                     if (has1) copy_scales(sa + 4, dsf + (kURec >> 4));
-                    const uint64_t dsb = dsf + uint64_t((2 * kURec - 8192 + 512 * TPG) >> 4); // 128 columns' scales per copy
+                    const uint64_t dsb = dsf + uint64_t((2 * kURec - 8192 + digit_bytes(TPG)) >> 4); // 128 columns' scales per copy
                     copy_scales(sb, dsb);
                     if (N > 128) copy_scales(sb + 4, dsb + 32);
                     mma_step(d0, da, db, idesc0, k > 0, sa, sb); // the run's first MMA overwrites
                     if (has1) mma_step(d1, da + (kURec >> 4), db, idesc0, k > 0, sa + 4, sb);
-                    mma_step(d0, da + 256, db + 16 * TPG, idesc1, true, sa, sb);
-                    if (has1) mma_step(d1, da + (kURec >> 4) + 256, db + 16 * TPG, idesc1, true, sa + 4, sb);
+                    mma_step(d0, da + 256, db + (digit_bytes(TPG) >> 5), idesc1, true, sa, sb);
+                    if (has1) mma_step(d1, da + (kURec >> 4) + 256, db + (digit_bytes(TPG) >> 5), idesc1, true, sa + 4, sb);
                     commit_to(&empty[cur]);
                 }
                 sfa = (sfa + 1) & (kGSfaBufs - 1);
@@ -462,7 +549,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
             const bool has1 = SWIGLU || 2 * pair + 1 < p.total_tiles;
             float y[2][TPG];
             load_sums<TPG>(tmem + (uint32_t(warp * 32) << 16), y[0]);
-            if (has1) load_sums<TPG>(tmem + uint32_t(N) + (uint32_t(warp * 32) << 16), y[1]);
+            if (has1) load_sums<TPG>(tmem + kD1Col + (uint32_t(warp * 32) << 16), y[1]);
             else {
 #pragma unroll
                 for (int t = 0; t < TPG; t++) y[1][t] = 0.f;
@@ -474,15 +561,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
             const int ubegin = r.unit * nkb, uend = ubegin + nkb;
             if (begin > ubegin || uend > end) {
                 // ---- a unit cut by a share boundary: leave the partial sums; the CTA that arrives last adds them up ----
+                // (A warp's rows lie side by side for each four tokens: with a row's tokens side by side instead every access touches
+                // 32 sectors, and 4096 x 4096 with 61 tokens took 35 us instead of 22.)
                 const int c_first = cta_of_stage(p, ubegin, G), c_last = cta_of_stage(p, uend - 1, G);
                 const int which = (begin > ubegin) ? 0 : 1; // the unit that contains this share's first stage, or a later one
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     if (h == 1 && !has1) break;
-                    float *slot = p.partials + ((size_t(c) * 2 + which) * 2 + h) * kSlotFloats + size_t(tid) * TPG;
+                    float4 *slot = reinterpret_cast<float4 *>(p.partials + ((size_t(c) * 2 + which) * 2 + h) * kSlotFloats) + tid; // [four tokens][row]
 #pragma unroll
-                    for (int t = 0; t < TPG; t += 4)
-                        __stcg(reinterpret_cast<float4 *>(slot + t), make_float4(y[h][t], y[h][t + 1], y[h][t + 2], y[h][t + 3]));
+                    for (int t = 0; t < TPG / 4; t++)
+                        __stcg(slot + t * 128, make_float4(y[h][4 * t], y[h][4 * t + 1], y[h][4 * t + 2], y[h][4 * t + 3]));
                 }
                 // The barrier makes the 128 threads' partial stores visible to thread 0; its release at GPU scope is cumulative
                 // over them, and the last arriver's acquire + the next barrier hand the other CTAs' stores to its 128 readers.
@@ -499,16 +588,15 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
                 if (!last) continue;
                 // the last arriver: add the parts in share order (the sum does not depend on who arrived last), both records
                 // of a part at once, so that a part costs one trip to L2
-                float acc[2][TPG];
 #pragma unroll
-                for (int t = 0; t < TPG; t++) acc[0][t] = acc[1][t] = 0.f;
+                for (int t = 0; t < TPG; t++) y[0][t] = y[1][t] = 0.f;
                 auto fetch = [&](int cc, float4 (&q)[2][TPG / 4]) {
-                    const float *slot = p.partials + (size_t(cc) * 2 + (share_begin(p, cc, G) > ubegin ? 0 : 1)) * 2 * kSlotFloats + size_t(tid) * TPG;
+                    const float4 *slot = reinterpret_cast<const float4 *>(p.partials + (size_t(cc) * 2 + (share_begin(p, cc, G) > ubegin ? 0 : 1)) * 2 * kSlotFloats) + tid;
 #pragma unroll
                     for (int h = 0; h < 2; h++)
 #pragma unroll
                         for (int t = 0; t < TPG / 4; t++)
-                            q[h][t] = h == 0 || has1 ? __ldcg(reinterpret_cast<const float4 *>(slot + h * kSlotFloats) + t) : make_float4(0.f, 0.f, 0.f, 0.f);
+                            q[h][t] = h == 0 || has1 ? __ldcg(slot + h * (kSlotFloats / 4) + t * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
                 };
                 float4 q[2][TPG / 4];
                 fetch(c_first, q);
@@ -519,12 +607,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
                     for (int h = 0; h < 2; h++)
 #pragma unroll
                         for (int t = 0; t < TPG / 4; t++) {
-                            acc[h][4 * t] += q[h][t].x; acc[h][4 * t + 1] += q[h][t].y; acc[h][4 * t + 2] += q[h][t].z; acc[h][4 * t + 3] += q[h][t].w;
+                            y[h][4 * t] += q[h][t].x; y[h][4 * t + 1] += q[h][t].y; y[h][4 * t + 2] += q[h][t].z; y[h][4 * t + 3] += q[h][t].w;
                             q[h][t] = nq[h][t];
                         }
                 }
-#pragma unroll
-                for (int t = 0; t < TPG; t++) { y[0][t] = acc[0][t]; y[1][t] = acc[1][t]; }
             }
             if constexpr (SWIGLU) {
                 const GSeg &s = p.seg[gseg_of(p, pair)];
@@ -554,11 +640,10 @@ namespace {
 std::mutex g_gemm_attr_mutex;
 bool g_gemm_attr_done[64] = {false}; // the shared-memory opt-in is a per-device function attribute
 
-// Tokens per group.  24 take fewer bytes into shared memory than 16 for every count beyond 48, the last group's padding included
-// (24576 x 4096 at 512 tokens 153 us against 182).  Up to 48 the weights bound the time and every CTA ends on a cut unit, whose
-// parts 24 tokens make half as large again and whose ring is shorter: a pass of 17..24 tokens 4.0 ms against 4.9 in one group of
-// 24, 33..48 tokens 4.2 against 5.1.
-int tokens_per_group(int tokens) { return tokens <= 48 ? 16 : 24; }
+// Tokens per group.  32 take fewer bytes into shared memory than 16 for every count beyond 48, the last group's padding included.  Up to
+// 48 the weights bound the time and every CTA ends on a cut unit, whose parts 32 tokens make twice as large and whose ring is shorter
+// (24576 x 4096: 40 tokens 28.2 us; 61 tokens in two groups 29.4).
+int tokens_per_group(int tokens) { return tokens <= 48 ? 16 : 32; }
 size_t image_bytes(int cols, int tokens)
 {
     const int tpg = tokens_per_group(tokens);
@@ -599,7 +684,6 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     d.bimg = static_cast<uint8_t *>(op->umma_scratch);
     d.tokens = tokens;
     d.ngroups = ngroups;
-    d.tpg = tpg;
     // about one CTA per SM, a slice of at least two k-blocks each
     d.parts = std::max(1, std::min(nkb / 2, sm_count() / (ngroups * tpg)));
 
@@ -640,7 +724,7 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     p.stages = std::min(kGMaxStages, 224 * 1024 / stage_bytes);
     const size_t smem = size_t(p.stages) * stage_bytes;
     auto kernel = tpg == 16 ? (nmat_all == 2 ? umma_gemm_kernel<16, true> : umma_gemm_kernel<16, false>)
-                            : (nmat_all == 2 ? umma_gemm_kernel<24, true> : umma_gemm_kernel<24, false>);
+                            : (nmat_all == 2 ? umma_gemm_kernel<32, true> : umma_gemm_kernel<32, false>);
     {
         int dev = 0;
         cudaError_t e = cudaGetDevice(&dev);
@@ -648,7 +732,7 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
         if (dev < 0 || dev >= 64) return fail(INSG_E_LIMIT, "gemm: device ordinal beyond 63");
         std::lock_guard<std::mutex> lock(g_gemm_attr_mutex);
         if (!g_gemm_attr_done[dev]) {
-            for (auto k : {umma_gemm_kernel<16, false>, umma_gemm_kernel<16, true>, umma_gemm_kernel<24, false>, umma_gemm_kernel<24, true>})
+            for (auto k : {umma_gemm_kernel<16, false>, umma_gemm_kernel<16, true>, umma_gemm_kernel<32, false>, umma_gemm_kernel<32, true>})
                 if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
             if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(umma gemm)");
             g_gemm_attr_done[dev] = true;
@@ -656,7 +740,7 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     }
     // the GEMM is the digitize kernel's programmatic dependent: it allocates tensor memory and requests its first weight
     // records while the digits are being written
-    int rc = launch(umma_digitize_kernel, dim3(ngroups * tpg * d.parts), dim3(kGThreads), 0, st, op->pdl != 0, d);
+    int rc = launch(tpg == 16 ? umma_digitize_kernel<16> : umma_digitize_kernel<32>, dim3(ngroups * tpg * d.parts), dim3(kGThreads), 0, st, op->pdl != 0, d);
     if (rc != INSG_OK) return rc;
     // Every part of a cut unit costs the CTA that adds them a trip to L2, about what a stage takes: few stages go to fewer CTAs,
     // so that a unit is cut into about sqrt(nkb) parts of sqrt(nkb) stages at most.
