@@ -221,6 +221,28 @@ __device__ __forceinline__ void gemv_publish_range(const GemvRange &r, GemvShare
     }
 }
 
+// alpha = 2^(12 - floor(log2(max))) puts the largest element in [2^12, 2^13): fp16 holds it with room to spare
+__device__ __forceinline__ float piece_scale(float largest, float &inv)
+{
+    int eb = int((__float_as_uint(largest) >> 23) & 0xffu);
+    eb = min(max(eb, 20), 240);
+    inv = __uint_as_float(uint32_t(eb - 12) << 23);
+    return __uint_as_float(uint32_t(266 - eb) << 23);
+}
+// Four elements as their two fp16 pieces, the low one `stride` values behind the high one.
+__device__ __forceinline__ void store_pieces(float4 v, float alpha, __half *hi, int stride)
+{
+    const float e[4] = {v.x * alpha, v.y * alpha, v.z * alpha, v.w * alpha};
+    __half h[4], l[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        h[q] = __float2half_rn(e[q]);
+        l[q] = __float2half_rn((e[q] - __half2float(h[q])) * 2048.0f);
+    }
+    *reinterpret_cast<uint2 *>(hi) = *reinterpret_cast<const uint2 *>(h);
+    *reinterpret_cast<uint2 *>(hi + stride) = *reinterpret_cast<const uint2 *>(l);
+}
+
 // ---- activation prologue: fp32 vector (fetched by load_activation) -> two fp16 pieces in shared memory ----
 // Returns 1/alpha, which undoes the power-of-two pre-scale.
 __device__ __forceinline__ float prologue(const GemvParams &p, const ProIn &pin, int m, float4 (&v)[kMaxVec], __half *xs, int xstride,
@@ -228,27 +250,58 @@ __device__ __forceinline__ float prologue(const GemvParams &p, const ProIn &pin,
 {
     const float tmax = transform_activation(pin, m, v, wpre, scratch);
     const int tid = threadIdx.x, nvec = p.cols >> 2;
-    // alpha = 2^(12 - floor(log2(max))) puts the largest element in [2^12, 2^13): fp16 holds it with room to spare
-    int eb = int((__float_as_uint(tmax) >> 23) & 0xffu);
-    eb = min(max(eb, 20), 240);
-    const float alpha = __uint_as_float(uint32_t(266 - eb) << 23);
-    __half *hi = xs + size_t(m * 2) * xstride, *lo = hi + xstride;
+    float inv;
+    const float alpha = piece_scale(tmax, inv);
+    __half *hi = xs + size_t(m * 2) * xstride;
 #pragma unroll
     for (int j = 0; j < kMaxVec; j++) {
         const int i = tid + j * kThreads;
-        if (i < nvec) {
-            const float e[4] = {v[j].x * alpha, v[j].y * alpha, v[j].z * alpha, v[j].w * alpha};
-            __half h[4], l[4];
+        if (i < nvec) store_pieces(v[j], alpha, hi + (i << 2), xstride);
+    }
+    return inv;
+}
+
+// Vectors that go in as they are, of up to 4096 columns: all tokens are loaded at once and their largest magnitudes found behind
+// one barrier, where token by token each costs a trip to L2 and two barriers (12352 x 4096 with three tokens PLAIN_X3, 4096 x 4096 with
+// one PLAIN_O1).  The same scale and pieces.
+template <int M>
+__device__ __forceinline__ void prologue_plain(const ProIn &pin, __half *xs, int xstride, float *scratch, float (&inv_alpha)[M])
+{
+    const int tid = threadIdx.x, lane = tid & 31, nvec = pin.cols >> 2;
+    float4 v[M][kPreVec];
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                h[q] = __float2half_rn(e[q]);
-                l[q] = __float2half_rn((e[q] - __half2float(h[q])) * 2048.0f);
-            }
-            *reinterpret_cast<uint2 *>(hi + (i << 2)) = *reinterpret_cast<const uint2 *>(h);
-            *reinterpret_cast<uint2 *>(lo + (i << 2)) = *reinterpret_cast<const uint2 *>(l);
+    for (int m = 0; m < M; m++) load_activation_part<0, kPreVec>(pin, m, v[m]);
+    float mx[M];
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+        mx[m] = 0.f;
+#pragma unroll
+        for (int j = 0; j < kPreVec; j++) mx[m] = fmaxf(mx[m], fmaxf(fmaxf(fabsf(v[m][j].x), fabsf(v[m][j].y)), fmaxf(fabsf(v[m][j].z), fabsf(v[m][j].w))));
+    }
+#pragma unroll
+    for (int mk = 16; mk; mk >>= 1)
+#pragma unroll
+        for (int m = 0; m < M; m++) mx[m] = fmaxf(mx[m], __shfl_xor_sync(0xffffffffu, mx[m], mk));
+    if (lane == 0) {
+#pragma unroll
+        for (int m = 0; m < M; m++) scratch[m * kWarps + (tid >> 5)] = mx[m];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < kWarps; w += 4) {
+            const float4 q = *reinterpret_cast<const float4 *>(scratch + m * kWarps + w);
+            t = fmaxf(t, fmaxf(fmaxf(q.x, q.y), fmaxf(q.z, q.w)));
+        }
+        const float alpha = piece_scale(t, inv_alpha[m]);
+#pragma unroll
+        for (int j = 0; j < kPreVec; j++) {
+            const int i = tid + j * kThreads;
+            if (i < nvec) store_pieces(v[m][j], alpha, xs + size_t(m * 2) * xstride + (i << 2), xstride);
         }
     }
-    return __uint_as_float(uint32_t(eb - 12) << 23);
 }
 
 // All tokens; the next one's first vectors (4096 columns) are asked for before this one's reductions.  From three
@@ -323,8 +376,12 @@ __device__ __forceinline__ void gemv_activation(const GemvParams &p, __half *xs,
         }
     } else {
         const ProIn pin{p.in, p.aux, p.norm_w, p.x_out, p.cols, p.prologue};
-        prologue_tokens<M>(p, pin, xs, xstride, wpre, scratch);
-        fetched = true;
+        if (p.prologue == INSG_PRO_PLAIN && !p.x_out && p.cols <= 4 * kPreVec * kThreads) {
+            prologue_plain<M>(pin, xs, xstride, scratch, inv_alpha);
+        } else {
+            prologue_tokens<M>(p, pin, xs, xstride, wpre, scratch);
+            fetched = true;
+        }
     }
     __syncthreads();
     if (fetched) {
