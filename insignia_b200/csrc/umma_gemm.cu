@@ -16,7 +16,7 @@
 // digits and 24 tokens, 127 like this.
 //
 // Kernels:
-//   umma_digitize_kernel  one CTA per token: the fused activation prologue (RMSNorm, gates, ...), then the digit
+//   umma_digitize_kernel  one CTA or more per token: the fused activation prologue (RMSNorm, gates, ...), then the digit
 //                         image of the token in global memory, laid out as the shared-memory image the MMA reads
 //                         ([k-block][group of tokens][448 bytes x tokens per group, scale blocks], canonical K-major, no swizzle);
 //   umma_gemm_kernel      one CTA per SM.  The work is the sequence of all (pair of records, token group, k-block) stages;
@@ -41,7 +41,7 @@
 
 namespace insg {
 
-constexpr int kGThreads = kProThreads;     // digitize kernel: the activation prologue is written for this many threads
+constexpr int kDigThreads = 256;           // digitize kernel
 constexpr int kGemmThreads = 192;          // GEMM kernel: four epilogue warps, the MMA issuer, the producer
 constexpr int kDigits = 7;                 // base-13 digits per activation = N columns per token
 constexpr int kGSfaBufs = 4;               // scale-factor column sets cycled by stage (a power of two)
@@ -151,39 +151,105 @@ struct DigitizeParams {
     int tokens, ngroups, parts; // a token's digits are written by `parts` CTAs, each a slice of the columns
 };
 
-// `parts` CTAs per token slot (slots beyond `tokens` are written as zeros so that their columns contribute nothing).  Every
-// CTA of a token runs the whole prologue (the norm needs all columns; that part is a few loads and one reduction) and writes
-// the digits of its slice of the k-blocks only: the digit extraction is the long part.
+// `parts` CTAs of eight warps per token slot, each a slice of the k-blocks (slots beyond `tokens` are written as zeros so that their columns
+// contribute nothing).  A warp takes a k-block at a time, four on their way at once; everything but the RMSNorm's sum stays inside the warp
+// (a head of the gated norm is one k-block), and that sum is the one barrier.  What bounds it: the latency of a CTA's chain, load to last
+// store, times the rounds of CTAs; so the CTAs are small enough for four an SM, 592 at once (4096 columns: 512 tokens 13.5 -> 9.9 us against one
+// CTA of sixteen warps per token, two an SM; 16 tokens 5.5 -> 3.7, 61 tokens 6.2 -> 4.4; 12288 columns 25 -> 23, bound by the ALU).
 template <int TPG>
-__global__ void __launch_bounds__(kGThreads, 2) umma_digitize_kernel(const __grid_constant__ DigitizeParams p)
+__global__ void __launch_bounds__(kDigThreads, 4) umma_digitize_kernel(const __grid_constant__ DigitizeParams p)
 {
-    __shared__ float scratch[64];
+    constexpr int kBatch = 4, kWarps = kDigThreads / 32;
+    __shared__ float scratch[kWarps];
     __shared__ uint16_t table[kPair];
-    if (threadIdx.x < kPair) table[threadIdx.x] = digit_pair13(int(threadIdx.x));
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid < kPair) table[tid] = digit_pair13(tid);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); // the GEMM may set itself up and fetch weights meanwhile
     const int m = blockIdx.x / p.parts, part = blockIdx.x - m * p.parts, grp = m / TPG, ms = m - grp * TPG;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    float4 v[kMaxVec];
-    if (m < p.tokens) {
-        ProIn pin = p.pro;
-        pin.x_out = nullptr;
-        uint2 wpre[kPreVec];
-        preload_norm_weights(pin, wpre);
-        pdl_wait();
-        load_activation(pin, m, v);
-        transform_activation<false>(pin, m, v, wpre, scratch);
+    const ProIn &o = p.pro;
+    const int nkb = o.cols >> 7, per = (nkb + p.parts - 1) / p.parts, kb0 = part * per, kb1 = min(nkb, kb0 + per);
+    const bool live = m < p.tokens, rms = o.prologue == INSG_PRO_RMSNORM;
+    const float *in = o.in + size_t(m) * o.cols + lane * 4;
+    pdl_wait();
+    if (blockIdx.x == 0)
+        for (int i = tid; i < kGMaxGrid; i += kDigThreads) p.tickets[i] = 0;
+    float4 x[kBatch];
+    auto load = [&](int b0) { // through L2 (see gemv_prologue.cuh)
+#pragma unroll
+        for (int j = 0; j < kBatch; j++) {
+            const int kb = b0 + j * kWarps;
+            x[j] = live && kb < kb1 ? __ldcg(reinterpret_cast<const float4 *>(in + size_t(kb) * 128)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    load(kb0 + warp);
+    float inv_rms = 1.f;
+    if (rms) {
+        float ss = 0.f;
+        if (p.parts == 1 && nkb <= kBatch * kWarps) { // the row is in the CTA's registers
+#pragma unroll
+            for (int j = 0; j < kBatch; j++) ss = fmaf(x[j].x, x[j].x, fmaf(x[j].y, x[j].y, fmaf(x[j].z, x[j].z, fmaf(x[j].w, x[j].w, ss))));
+        } else if (live) {
+#pragma unroll 4
+            for (int kb = warp; kb < nkb; kb += kWarps) {
+                const float4 v = __ldcg(reinterpret_cast<const float4 *>(in + size_t(kb) * 128));
+                ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss))));
+            }
+        }
+        ss = warp_sum(ss);
+        if (lane == 0) scratch[warp] = ss;
+        __syncthreads(); // and the table
+        float tot = 0.f;
+#pragma unroll
+        for (int w = 0; w < kWarps; w++) tot += scratch[w];
+        inv_rms = rsqrtf(tot / float(o.cols) + 1e-6f);
     } else {
-        pdl_wait();
-#pragma unroll
-        for (int j = 0; j < kMaxVec; j++) v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncthreads(); // the table
     }
-    __syncthreads(); // the table
-    if (blockIdx.x == 0 && tid < kGMaxGrid) p.tickets[tid] = 0;
-    const int nkb = p.pro.cols >> 7, per = (nkb + p.parts - 1) / p.parts, kb0 = part * per, kb1 = min(nkb, kb0 + per);
+    for (int b0 = kb0 + warp; b0 < kb1; b0 += kBatch * kWarps) {
+        if (b0 != kb0 + warp) load(b0);
 #pragma unroll
-    for (int j = 0; j < kMaxVec; j++) { // a warp holds a k-block per j
-        const int kb = warp + j * (kGThreads / 32);
-        if (kb >= kb0 && kb < kb1) store_digits13<TPG>(v[j], ms, p.bimg + (size_t(kb) * p.ngroups + grp) * digit_block(TPG), table, lane);
+        for (int j = 0; j < kBatch; j++) {
+            const int kb = b0 + j * kWarps;
+            if (kb >= kb1) break; // warp-uniform
+            float4 v = x[j];
+            const int k = kb * 128 + lane * 4;
+            if (live) {
+                auto weigh = [&](const uint16_t *w, float f) {
+                    const uint2 wv = *reinterpret_cast<const uint2 *>(w);
+                    v.x = v.x * f * bf16_bits_to_float(wv.x & 0xffff);
+                    v.y = v.y * f * bf16_bits_to_float(wv.x >> 16);
+                    v.z = v.z * f * bf16_bits_to_float(wv.y & 0xffff);
+                    v.w = v.w * f * bf16_bits_to_float(wv.y >> 16);
+                };
+                switch (o.prologue) {
+                case INSG_PRO_RMSNORM: weigh(o.norm_w + k, inv_rms); break;
+                case INSG_PRO_GATED_RMSNORM: { // a head is one k-block
+                    const float4 z = __ldcg(reinterpret_cast<const float4 *>(o.aux + size_t(m) * o.cols + k));
+                    const float hs = warp_sum(fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w))));
+                    weigh(o.norm_w + lane * 4, rsqrtf(hs / 128.f + 1e-6f));
+                    v.x *= fast_silu(z.x); v.y *= fast_silu(z.y); v.z *= fast_silu(z.z); v.w *= fast_silu(z.w);
+                    break;
+                }
+                case INSG_PRO_SIGMOID_GATE: {
+                    const float4 g = __ldcg(reinterpret_cast<const float4 *>(o.aux + size_t(m) * o.cols + k));
+                    v.x *= fast_sigmoid(g.x); v.y *= fast_sigmoid(g.y); v.z *= fast_sigmoid(g.z); v.w *= fast_sigmoid(g.w);
+                    break;
+                }
+                case INSG_PRO_SIGMOID_GATE_HEAD0: {
+                    const float g = fast_sigmoid(__ldcg(o.aux + size_t(m) * 2 * o.cols + (k >> 8) * 512 + 256));
+                    v.x *= g; v.y *= g; v.z *= g; v.w *= g;
+                    break;
+                }
+                case INSG_PRO_SIGMOID_GATE_QPROJ: {
+                    const float4 g = __ldcg(reinterpret_cast<const float4 *>(o.aux + size_t(m) * 2 * o.cols + (k >> 8) * 512 + 256 + (k & 255)));
+                    v.x *= fast_sigmoid(g.x); v.y *= fast_sigmoid(g.y); v.z *= fast_sigmoid(g.z); v.w *= fast_sigmoid(g.w);
+                    break;
+                }
+                default: break;
+                }
+            }
+            store_digits13<TPG>(v, ms, p.bimg + (size_t(kb) * p.ngroups + grp) * digit_block(TPG), table, lane);
+        }
     }
 }
 
@@ -668,7 +734,7 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     if (!op || !op->in) return fail(INSG_E_ARG, "gemm: null operand");
     const int tokens = op->tokens;
     if (tokens < 1 || tokens > 4096) return fail(INSG_E_SHAPE, "gemm: 1 <= tokens <= 4096");
-    if (op->cols <= 0 || (op->cols & 127) || op->cols > kMaxVec * kGThreads * 4) return fail(INSG_E_SHAPE, "gemm: cols must be a multiple of 128, <= 12288");
+    if (op->cols <= 0 || (op->cols & 127) || op->cols > kMaxVec * kProThreads * 4) return fail(INSG_E_SHAPE, "gemm: cols must be a multiple of 128, <= 12288");
     if (op->n_segments < 1 || op->n_segments > 4) return fail(INSG_E_SHAPE, "gemm: 1..4 segments");
     if (op->prologue < 0 || op->prologue >= INSG_PRO_PREPARED) return fail(INSG_E_ARG, "gemm: prologue not available for several tokens");
     if ((op->prologue == INSG_PRO_RMSNORM || op->prologue == INSG_PRO_GATED_RMSNORM) && !op->norm_w) return fail(INSG_E_ARG, "gemm: norm weight missing");
@@ -684,8 +750,8 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     d.bimg = static_cast<uint8_t *>(op->umma_scratch);
     d.tokens = tokens;
     d.ngroups = ngroups;
-    // about one CTA per SM, a slice of at least two k-blocks each
-    d.parts = std::max(1, std::min(nkb / 2, sm_count() / (ngroups * tpg)));
+    // up to four CTAs per SM, a k-block for every warp of theirs at least
+    d.parts = std::max(1, std::min(nkb / (kDigThreads / 32), 4 * sm_count() / (ngroups * tpg)));
 
     GParams p = {};
     p.bimg = d.bimg;
@@ -740,7 +806,7 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     }
     // the GEMM is the digitize kernel's programmatic dependent: it allocates tensor memory and requests its first weight
     // records while the digits are being written
-    int rc = launch(tpg == 16 ? umma_digitize_kernel<16> : umma_digitize_kernel<32>, dim3(ngroups * tpg * d.parts), dim3(kGThreads), 0, st, op->pdl != 0, d);
+    int rc = launch(tpg == 16 ? umma_digitize_kernel<16> : umma_digitize_kernel<32>, dim3(ngroups * tpg * d.parts), dim3(kDigThreads), 0, st, op->pdl != 0, d);
     if (rc != INSG_OK) return rc;
     // Every part of a cut unit costs the CTA that adds them a trip to L2, about what a stage takes: few stages go to fewer CTAs,
     // so that a unit is cut into about sqrt(nkb) parts of sqrt(nkb) stages at most.
