@@ -173,12 +173,22 @@ __global__ void __launch_bounds__(kDigThreads, 4) umma_digitize_kernel(const __g
     pdl_wait();
     if (blockIdx.x == 0)
         for (int i = tid; i < kGMaxGrid; i += kDigThreads) p.tickets[i] = 0;
-    float4 x[kBatch];
+    float4 x[kBatch], a[kBatch]; // values and what gates them
     auto load = [&](int b0) { // through L2 (see gemv_prologue.cuh)
 #pragma unroll
         for (int j = 0; j < kBatch; j++) {
-            const int kb = b0 + j * kWarps;
-            x[j] = live && kb < kb1 ? __ldcg(reinterpret_cast<const float4 *>(in + size_t(kb) * 128)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const int kb = b0 + j * kWarps, k = kb * 128 + lane * 4;
+            x[j] = a[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (!live || kb >= kb1) continue;
+            x[j] = __ldcg(reinterpret_cast<const float4 *>(in + size_t(kb) * 128));
+            const float *gate = o.aux + size_t(m) * 2 * o.cols + (k >> 8) * 512 + 256; // interleaved [head][query 256 | gate 256]
+            switch (o.prologue) {
+            case INSG_PRO_GATED_RMSNORM:
+            case INSG_PRO_SIGMOID_GATE: a[j] = __ldcg(reinterpret_cast<const float4 *>(o.aux + size_t(m) * o.cols + k)); break;
+            case INSG_PRO_SIGMOID_GATE_HEAD0: a[j].x = __ldcg(gate); break;
+            case INSG_PRO_SIGMOID_GATE_QPROJ: a[j] = __ldcg(reinterpret_cast<const float4 *>(gate + (k & 255))); break;
+            default: break;
+            }
         }
     };
     load(kb0 + warp);
@@ -224,25 +234,18 @@ __global__ void __launch_bounds__(kDigThreads, 4) umma_digitize_kernel(const __g
                 switch (o.prologue) {
                 case INSG_PRO_RMSNORM: weigh(o.norm_w + k, inv_rms); break;
                 case INSG_PRO_GATED_RMSNORM: { // a head is one k-block
-                    const float4 z = __ldcg(reinterpret_cast<const float4 *>(o.aux + size_t(m) * o.cols + k));
                     const float hs = warp_sum(fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w))));
                     weigh(o.norm_w + lane * 4, rsqrtf(hs / 128.f + 1e-6f));
-                    v.x *= fast_silu(z.x); v.y *= fast_silu(z.y); v.z *= fast_silu(z.z); v.w *= fast_silu(z.w);
+                    v.x *= fast_silu(a[j].x); v.y *= fast_silu(a[j].y); v.z *= fast_silu(a[j].z); v.w *= fast_silu(a[j].w);
                     break;
                 }
-                case INSG_PRO_SIGMOID_GATE: {
-                    const float4 g = __ldcg(reinterpret_cast<const float4 *>(o.aux + size_t(m) * o.cols + k));
-                    v.x *= fast_sigmoid(g.x); v.y *= fast_sigmoid(g.y); v.z *= fast_sigmoid(g.z); v.w *= fast_sigmoid(g.w);
+                case INSG_PRO_SIGMOID_GATE:
+                case INSG_PRO_SIGMOID_GATE_QPROJ:
+                    v.x *= fast_sigmoid(a[j].x); v.y *= fast_sigmoid(a[j].y); v.z *= fast_sigmoid(a[j].z); v.w *= fast_sigmoid(a[j].w);
                     break;
-                }
                 case INSG_PRO_SIGMOID_GATE_HEAD0: {
-                    const float g = fast_sigmoid(__ldcg(o.aux + size_t(m) * 2 * o.cols + (k >> 8) * 512 + 256));
+                    const float g = fast_sigmoid(a[j].x);
                     v.x *= g; v.y *= g; v.z *= g; v.w *= g;
-                    break;
-                }
-                case INSG_PRO_SIGMOID_GATE_QPROJ: {
-                    const float4 g = __ldcg(reinterpret_cast<const float4 *>(o.aux + size_t(m) * 2 * o.cols + (k >> 8) * 512 + 256 + (k & 255)));
-                    v.x *= fast_sigmoid(g.x); v.y *= fast_sigmoid(g.y); v.z *= fast_sigmoid(g.z); v.w *= fast_sigmoid(g.w);
                     break;
                 }
                 default: break;
@@ -476,7 +479,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
     uint8_t *ring = smem;                          // S stages of kGStage bytes
     __shared__ __align__(8) uint64_t full[kGMaxStages], empty[kGMaxStages], dfull, dempty;
     __shared__ uint32_t s_tmem;
-    __shared__ int s_abort, s_last;
+    __shared__ int s_abort, s_last, s_early[2];
 
     const int G = int(gridDim.x), c = int(blockIdx.x);
     const int begin = share_begin(p, c, G), end = share_begin(p, c + 1, G);
@@ -603,6 +606,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
             const GRun r = run_at(p, g, end);
             g += r.len;
             const int pair = r.unit / p.ngroups, grp = r.unit - pair * p.ngroups;
+            const int ubegin = r.unit * nkb, uend = ubegin + nkb;
+            const bool cut = begin > ubegin || uend > end;
+            const int c_first = cut ? cta_of_stage(p, ubegin, G) : c, c_last = cut ? cta_of_stage(p, uend - 1, G) : c;
+            // A unit of two parts whose other one is already there (the usual case of a share's last unit, with nothing behind it to hide
+            // the trips to L2): this CTA adds it to its own, which it need not store.
+            if (tid == 0) {
+                int seen = 0;
+                if (c_last == c_first + 1) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(p.tickets + c_first) : "memory");
+                s_early[run & 1] = seen;
+            }
             ok = mbar_wait(&dfull, run & 1, abort_flag);
             {   // the 128 epilogue threads go on or give up together (they meet at named barriers below)
                 uint32_t all;
@@ -624,12 +637,30 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
             __syncwarp();
             if (lane == 0) mbar_arrive(&dempty);
 
-            const int ubegin = r.unit * nkb, uend = ubegin + nkb;
-            if (begin > ubegin || uend > end) {
+            auto fetch = [&](int cc, float4 (&q)[2][TPG / 4]) { // a CTA's part of this unit
+                const float4 *slot = reinterpret_cast<const float4 *>(p.partials + (size_t(cc) * 2 + (share_begin(p, cc, G) > ubegin ? 0 : 1)) * 2 * kSlotFloats) + tid;
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+#pragma unroll
+                    for (int t = 0; t < TPG / 4; t++)
+                        q[h][t] = h == 0 || has1 ? __ldcg(slot + h * (kSlotFloats / 4) + t * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
+            };
+            if (cut && s_early[run & 1]) {
+                float4 q[2][TPG / 4];
+                fetch(c_first + c_last - c, q);
+                if (tid == 0) p.tickets[c_first] = 0; // ready for the next launch
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+#pragma unroll
+                    for (int t = 0; t < TPG / 4; t++) {
+                        const float part[4] = {q[h][t].x, q[h][t].y, q[h][t].z, q[h][t].w};
+#pragma unroll
+                        for (int i = 0; i < 4; i++) y[h][4 * t + i] = (y[h][4 * t + i] + 0.f) + part[i]; // from zero, as below (the sign of a zero)
+                    }
+            } else if (cut) {
                 // ---- a unit cut by a share boundary: leave the partial sums; the CTA that arrives last adds them up ----
                 // (A warp's rows lie side by side for each four tokens: with a row's tokens side by side instead every access touches
                 // 32 sectors, and 4096 x 4096 with 61 tokens took 35 us instead of 22.)
-                const int c_first = cta_of_stage(p, ubegin, G), c_last = cta_of_stage(p, uend - 1, G);
                 const int which = (begin > ubegin) ? 0 : 1; // the unit that contains this share's first stage, or a later one
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
@@ -656,14 +687,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
                 // of a part at once, so that a part costs one trip to L2
 #pragma unroll
                 for (int t = 0; t < TPG; t++) y[0][t] = y[1][t] = 0.f;
-                auto fetch = [&](int cc, float4 (&q)[2][TPG / 4]) {
-                    const float4 *slot = reinterpret_cast<const float4 *>(p.partials + (size_t(cc) * 2 + (share_begin(p, cc, G) > ubegin ? 0 : 1)) * 2 * kSlotFloats) + tid;
-#pragma unroll
-                    for (int h = 0; h < 2; h++)
-#pragma unroll
-                        for (int t = 0; t < TPG / 4; t++)
-                            q[h][t] = h == 0 || has1 ? __ldcg(slot + h * (kSlotFloats / 4) + t * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
-                };
                 float4 q[2][TPG / 4];
                 fetch(c_first, q);
                 for (int cc = c_first; cc <= c_last; cc++) {
