@@ -170,6 +170,16 @@ __global__ void __launch_bounds__(kDigThreads, 4) umma_digitize_kernel(const __g
     const int nkb = o.cols >> 7, per = (nkb + p.parts - 1) / p.parts, kb0 = part * per, kb1 = min(nkb, kb0 + per);
     const bool live = m < p.tokens, rms = o.prologue == INSG_PRO_RMSNORM;
     const float *in = o.in + size_t(m) * o.cols + lane * 4;
+    uint2 w[kBatch]; // the norm's weights are parameters: asked for before the wait
+    auto load_weights = [&](int b0) {
+#pragma unroll
+        for (int j = 0; j < kBatch; j++) {
+            const int kb = b0 + j * kWarps;
+            if (rms && kb < kb1) w[j] = *reinterpret_cast<const uint2 *>(o.norm_w + kb * 128 + lane * 4);
+            else if (o.prologue == INSG_PRO_GATED_RMSNORM) w[j] = *reinterpret_cast<const uint2 *>(o.norm_w + lane * 4);
+        }
+    };
+    load_weights(kb0 + warp);
     pdl_wait();
     if (blockIdx.x == 0)
         for (int i = tid; i < kGMaxGrid; i += kDigThreads) p.tickets[i] = 0;
@@ -216,26 +226,27 @@ __global__ void __launch_bounds__(kDigThreads, 4) umma_digitize_kernel(const __g
         __syncthreads(); // the table
     }
     for (int b0 = kb0 + warp; b0 < kb1; b0 += kBatch * kWarps) {
-        if (b0 != kb0 + warp) load(b0);
+        if (b0 != kb0 + warp) {
+            load_weights(b0);
+            load(b0);
+        }
 #pragma unroll
         for (int j = 0; j < kBatch; j++) {
             const int kb = b0 + j * kWarps;
             if (kb >= kb1) break; // warp-uniform
             float4 v = x[j];
-            const int k = kb * 128 + lane * 4;
             if (live) {
-                auto weigh = [&](const uint16_t *w, float f) {
-                    const uint2 wv = *reinterpret_cast<const uint2 *>(w);
-                    v.x = v.x * f * bf16_bits_to_float(wv.x & 0xffff);
-                    v.y = v.y * f * bf16_bits_to_float(wv.x >> 16);
-                    v.z = v.z * f * bf16_bits_to_float(wv.y & 0xffff);
-                    v.w = v.w * f * bf16_bits_to_float(wv.y >> 16);
+                auto weigh = [&](float f) {
+                    v.x = v.x * f * bf16_bits_to_float(w[j].x & 0xffff);
+                    v.y = v.y * f * bf16_bits_to_float(w[j].x >> 16);
+                    v.z = v.z * f * bf16_bits_to_float(w[j].y & 0xffff);
+                    v.w = v.w * f * bf16_bits_to_float(w[j].y >> 16);
                 };
                 switch (o.prologue) {
-                case INSG_PRO_RMSNORM: weigh(o.norm_w + k, inv_rms); break;
+                case INSG_PRO_RMSNORM: weigh(inv_rms); break;
                 case INSG_PRO_GATED_RMSNORM: { // a head is one k-block
                     const float hs = warp_sum(fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w))));
-                    weigh(o.norm_w + lane * 4, rsqrtf(hs / 128.f + 1e-6f));
+                    weigh(rsqrtf(hs / 128.f + 1e-6f));
                     v.x *= fast_silu(a[j].x); v.y *= fast_silu(a[j].y); v.z *= fast_silu(a[j].z); v.w *= fast_silu(a[j].w);
                     break;
                 }
