@@ -147,10 +147,9 @@ __device__ __forceinline__ int group_exponent(uint32_t max_bits) { return max(in
 __device__ __forceinline__ float group_alpha(int eb) { return __uint_as_float(uint32_t(277 - eb) << 23); }  // largest element * alpha in [2^23, 2^24)
 __device__ __forceinline__ uint8_t group_scale(int eb) { return uint8_t(eb == 255 ? 255 : eb - 23); }
 
-// ---- digit image of activation vectors: [k-block of 128][digits of T token slots: 512 T bytes | scale blocks: 512 bytes per 16 slots] ----
+// ---- digit image of activation vectors: [k-block of 128][digits of T token slots: 512 T bytes | scale block: 512 bytes] ----
 // The digits of one 128-element k-block of one token (four elements per lane) into the B image, and their group scales.
 // Image of a k-block: [2 K-steps][T column groups][2 k cores][8 columns][16 B]; a token's eight digit columns are one group.
-template <bool MANY = false> // more than sixteen slots: more than one scale block
 __device__ __forceinline__ void store_digits(float4 x, int T, int m, uint8_t *bkb, const uint8_t *lut, int lane)
 {
     float mx = fmax_nan(fmax_nan(fabsf(x.x), fabsf(x.y)), fmax_nan(fabsf(x.z), fabsf(x.w)));
@@ -160,8 +159,7 @@ __device__ __forceinline__ void store_digits(float4 x, int T, int m, uint8_t *bk
     const int eb = group_exponent(__float_as_uint(mx));
     pack_digits(x, group_alpha(eb), lut, bkb + (lane >> 4) * (256 * T) + m * 256 + ((lane >> 3) & 1) * 128 + (lane & 7) * 2);
     const int n = 8 * m + (lane & 7); // scale block: row = column n of B (32 rows, then the next quarter), byte = group
-    if (MANY) bkb += (n >> 7) * 512;
-    bkb[512 * T + (n & 31) * 16 + (MANY ? (n >> 5) & 3 : n >> 5) * 4 + (lane >> 3)] = group_scale(eb);
+    bkb[512 * T + (n & 31) * 16 + (n >> 5) * 4 + (lane >> 3)] = group_scale(eb);
 }
 
 // One element per lane: the warp's 32 lanes are the 32-element group `grp` of token slot m's vector.

@@ -609,7 +609,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
             g += r.len;
         }
     } else {
-        // ---- epilogue: tensor-memory lane = row of the tile; token t of the group = columns 8t .. 8t+7 --------------------
+        // ---- epilogue: tensor-memory lane = row of the tile; digit j of the group's token t = column j * TPG + t ------------
         asm volatile("griddepcontrol.wait;" ::: "memory"); // residual inputs and tickets come from earlier launches
         bool ok = true;
         int g = begin;
