@@ -533,6 +533,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
             if (q.has1) bulk_load(dst0 + kURec, q.a1, kURec, &full[lane]);
         }
         asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("fence.proxy.async.global;" ::: "memory"); // the digits were written by ordinary stores, the bulk copies read them through the async proxy
         if (lane < first) bulk_load(dst0 + 2 * kURec, b0, kBBlock, &full[lane]);
         // from here on the whole warp walks the loop and one elected lane issues: warp-uniform operands issue twice as fast
         const bool one = elect_one();
