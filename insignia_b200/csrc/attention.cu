@@ -68,6 +68,7 @@ __device__ __forceinline__ void attn_mma_warp(const void *kc, const void *vc, in
         mbar_init(bar + 1, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    asm volatile("fence.proxy.async.global;" ::: "memory"); // earlier launches wrote the rows by ordinary stores, the bulk copies read them through the async proxy
     __syncwarp();
     // Keys and values have a barrier each: a tile of keys is requested as soon as the one before has been scored, a tile of values
     // as soon as the one before has been added, so that one of the two is on its way whatever the warp does.
