@@ -51,7 +51,9 @@ constexpr int kDHalfSm = 112 * 1024;
 // own ring.  Its requests share the SM's copy engine and the memory with this launch's: made while this launch still streams they delay
 // the stages it waits for.  The four products of a block with one token: 28.1 us with the next launch at once, 26.6 like this, 29.3 at
 // the very end, when its ring cannot fill in time; L2 asked for six stages 27.8, for all of them 28.0.  Eight tokens 35.3 -> 34.4 us,
-// where asking L2 gains nothing.  A token 1.16 -> 1.115 ms, a step of three or eight sequences 1 % less.
+// where asking L2 gains nothing.  A token 1.16 -> 1.115 ms.  All threads execute the trigger where the CTA sets out: left to the
+// producer warp, with the L2 code in every variant, a launch that stands alone took 0.1-0.3 us more (4096 x 4096, one, two, eight tokens
+// 6.85, 8.11, 12.25 us; like this 6.78, 7.98, 12.10; with the trigger there for every size 6.77, 7.85, 12.07).
 template <int T> constexpr int kDTriggerStages = T <= 2 ? 6 : 4;
 template <int T> constexpr int kDAheadStages = T <= 2 ? 3 : 0;
 
@@ -75,6 +77,7 @@ struct DParams {
     float *x_out;
     const float *prep_partials; // prepared input: the producer's sums of squares, or null
     int cols, nkb, prologue, nseg, units, nmat, tokens, stages;
+    int ahead; // stages beyond the ring to ask L2 for
     DSeg seg[4];
     float2 *argmax_partial;
     unsigned *argmax_ticket;
@@ -242,7 +245,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // The next launch may become resident from here on, not earlier: were it to take tensor memory before every CTA here has its own,
     // a CTA could wait for memory held by a CTA that waits for this grid.
-    if (warp == 9 && nstages - kDTriggerStages<T> <= S) pdl_launch_dependents();
+    if (nstages - kDTriggerStages<T> <= S) pdl_launch_dependents();
     cluster_arrive();
     cluster_wait(); // the peers' barriers exist from here on
     const uint32_t tmem = s_tmem;
@@ -352,11 +355,13 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         // ---- producer ----------------------------------------------------------------------------------------------------------
         {
             const bool one = elect_one();
-            for (int i = S + lane; i < min(nstages, S + kDAheadStages<T>); i += 32) {
-                const int run = i / spt, st = i - run * spt;
-                bulk_prefetch(run_src(run) + size_t(st) * kDStage, uint32_t(min(2, len - 2 * st)) * kURec);
+            if constexpr (kDAheadStages<T> > 0) {
+                for (int i = S + lane; i < min(nstages, S + p.ahead); i += 32) {
+                    const int run = i / spt, st = i - run * spt;
+                    bulk_prefetch(run_src(run) + size_t(st) * kDStage, uint32_t(min(2, len - 2 * st)) * kURec);
+                }
+                __syncwarp();
             }
-            __syncwarp();
             if (prepared) { // the digits come ready: eight k-blocks per copy, so that the multiplies can start behind the first
                 pdl_wait();
                 asm volatile("fence.proxy.async.global;" ::: "memory"); // written by ordinary stores of the launch before
@@ -855,6 +860,7 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     int stages = fixed < size_t(kDHalfSm) ? int((kDHalfSm - fixed) / kDStage) : 0;
     if (stages < 4 || (stages == 4 && need > 96)) stages = int((size_t(222) * 1024 - fixed) / kDStage);
     p.stages = std::max(1, std::min({stages, need, kDMaxStages}));
+    p.ahead = !op->pdl ? 0 : T == 1 ? kDAheadStages<1> : T == 2 ? kDAheadStages<2> : 0; // a launch that waits for its predecessor anyway streams at once
     const size_t smem = fixed + size_t(p.stages) * kDStage;
 
     cudaLaunchConfig_t cfg = {};
