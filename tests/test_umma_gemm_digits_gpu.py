@@ -41,3 +41,58 @@ def test_digits_at_the_edges(cuda, tokens):
         # truncated) and the seven combinations add an ulp of the sum of magnitudes each at the very most
         bound = weights @ room[m] * 2.0**-24 + weights @ np.abs(x[m].astype(np.float64)) * 2.0**-23 * 8
         assert np.all(np.abs(y[m] - orc.gemv_mlx_f64(w, s, x[m])) <= bound), m
+
+
+BASE = 13
+
+
+def spread_values(rng, count, limit):
+    """`count` integers up to `limit` in magnitude: every residue of each of the three digit pairs, the carries between them (a pair of digits that
+    ends negative takes one from the next pair), every last digit."""
+    n = np.stack([rng.permutation(np.arange(count) % BASE**2) for _ in range(3)])
+    last = rng.permutation(np.arange(count) % 9) - 4
+    v = n[0] + BASE**2 * n[1] + BASE**4 * n[2] + BASE**6 * last.astype(np.int64)
+    return np.where(np.abs(v) <= limit, v, v % (2 * limit + 1) - limit)
+
+
+@pytest.mark.parametrize("tokens", [9, 16, 17, 48, 49, 64, 65])
+def test_every_digit_reaches_the_product(cuda, tokens):
+    """Rows with a single weight of one: each product is one activation as its digits hold it, the nearest multiple of its group's unit, and
+    nothing rounds on the way but the seventh digit's addition.  Bit for bit."""
+    from insignia_b200 import mxfp4, ops
+
+    cols = 384  # three k-blocks, three tiles of rows: an odd one
+    rng = np.random.default_rng(100 + tokens)
+    w, s = mxfp4.quantize_rows(np.eye(cols, dtype=np.float32))
+    assert np.array_equal(host(ops.dequant_mlx(dev(w), dev(s))), np.eye(cols, dtype=np.float32))
+    largest = np.array([1, np.nextafter(np.float32(EDGE), np.float32(0)), EDGE, np.nextafter(np.float32(2), np.float32(0)), 1.5], np.float64)
+    groups = tokens * cols // 32
+    mantissa, exponent = largest[np.arange(groups) % 5], rng.integers(-20, 20, groups)
+    unit = 2.0 ** (exponent - np.where(mantissa < EDGE, 24, 23))  # one bit more below the edge
+    limit = (mantissa * 2.0**exponent / unit).astype(np.int64)
+    v = np.stack([spread_values(rng, groups, 2**24 - 1) for _ in range(32)], axis=1)
+    v = np.clip(v, -limit[:, None], limit[:, None])
+    x = v * unit[:, None]
+    x[:, 16:24] += rng.uniform(-0.5, 0.5, (groups, 8)) * unit[:, None]  # between two multiples
+    x = np.clip(x, -(mantissa * 2.0**exponent)[:, None], (mantissa * 2.0**exponent)[:, None])
+    top = rng.integers(0, 32, groups)
+    x[np.arange(groups), top] = mantissa * 2.0**exponent * rng.choice([-1, 1], groups)
+    x = x.astype(np.float32)
+    want = (np.rint(x.astype(np.float64) / unit[:, None]) * unit[:, None]).astype(np.float32).reshape(tokens, cols)
+    got = host(ops.gemm_umma(ops.repack_umma(dev(w), dev(s)), dev(x.reshape(tokens, cols))))
+    assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("tokens", [16, 61])
+@pytest.mark.parametrize("cols", [640, 4096, 12288])
+def test_products_of_normal_vectors(cuda, tokens, cols):
+    """An activation is off by a uniform half unit, 2^-22 of sqrt(1/12) = 0.7e-7 for groups whose largest lies in [2, 4); signs are random,
+    so the product is off by as much of its root mean square, and its fp32 sums and combinations by about as much again."""
+    from insignia_b200 import ops
+
+    rng = np.random.default_rng(cols + tokens)
+    w, s = rand_matrix(rng, 256, cols)
+    x = rng.standard_normal((tokens, cols)).astype(np.float32)
+    y = host(ops.gemm_umma(ops.repack_umma(dev(w), dev(s)), dev(x)))
+    y64 = np.stack([orc.gemv_mlx_f64(w, s, x[m]) for m in range(tokens)])
+    assert np.sqrt(np.mean((y - y64) ** 2) / np.mean(y64**2)) <= 2e-7
