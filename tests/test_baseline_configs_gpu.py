@@ -104,7 +104,7 @@ def test_config1_matmul_shapes_and_token_counts(cuda, rows, cols):
         y1 = ops.gemv_packed(packed, dev(x[M - 1])).cpu().numpy()
         assert np.array_equal(y1, y[M - 1])
         if M >= 16:
-            # the tcgen05 kind::mxf4 kernel (16 or 24 tokens per instruction, stream-K shares): same bar on the sampled rows,
+            # the tcgen05 kind::mxf4 kernel (16 or 32 tokens per instruction, stream-K shares): same bar on the sampled rows,
             # and the whole matrix against the mma.sync kernel's result
             yt = ops.gemm_umma(tiles, dev(x)).cpu().numpy().reshape(M, rows)
             err_t = np.max(np.abs(yt[:, sample] - want)) / np.abs(want).max()

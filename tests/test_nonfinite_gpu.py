@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
-# up to eight tokens: the GEMV; more: the GEMM with 16 (up to 48) or 24 tokens a group
+# up to eight tokens: the GEMV; more: the GEMM with 16 (up to 48) or 32 tokens a group
 @pytest.mark.parametrize("tokens", [1, 2, 3, 8, 9, 16, 48, 49, 71])
 @pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
 def test_a_non_finite_activation_makes_its_token_nan(cuda, tokens, value):

@@ -1,4 +1,4 @@
-"""The several-token tcgen05 GEMM (16 or 24 tokens per kind::mxf4 instruction, stream-K shares), through the C ABI, against the CPU oracle
+"""The several-token tcgen05 GEMM (16 or 32 tokens per kind::mxf4 instruction, stream-K shares), through the C ABI, against the CPU oracle
 and against the one-token kernels."""
 import os
 import sys
@@ -50,6 +50,38 @@ def test_gemm_umma_is_deterministic_across_cut_units(cuda, rows, cols, M):
         assert np.array_equal(host(ops.gemm_umma(P, x, scratch=scratch)), first)
     y64 = orc.gemv_mlx_f64(w, s, host(x)[M - 1])
     assert np.max(np.abs(first[M - 1] - y64)) <= 4e-6 * np.abs(y64).max()
+
+
+# 37 tiles and two groups: 19 pairs, the last one of a single tile, every unit in two parts; five tiles: units in about ten parts; three groups:
+# units in two to five; the last one SwiGLU, where a pair is a gate and an up tile
+@pytest.mark.parametrize("rows,cols,M,swiglu", [(128 * 37, 512, 49, False), (640, 12288, 61, False), (4096, 4096, 65, False), (896, 4096, 61, True)])
+def test_cut_units_have_the_same_bits_whoever_arrives_last(cuda, rows, cols, M, swiglu):
+    """The CTA that finds the other part of a unit there adds it to its own; else the last one to arrive adds all parts.  Other work on the
+    GPU moves the arrivals."""
+    from insignia_b200 import ops
+
+    rng = np.random.default_rng(rows + M)
+    mats = [rand_matrix(rng, rows, cols) for _ in range(1 + swiglu)]
+    x = (rng.standard_normal((M, cols)) * 2).astype(np.float32)
+    packed = [ops.repack_umma(dev(w), dev(s)) for w, s in mats]
+    seg = dict(packed=packed[0], rows=rows, epilogue="store")
+    if swiglu:
+        seg.update(packed2=packed[1], epilogue="swiglu")
+    xd, scratch, calls = dev(x), ops.umma_gemm_scratch(cols, M), 60
+    outs = torch.zeros(calls, M, rows, device="cuda")
+    side, junk = torch.cuda.Stream(), torch.randn(1 << 22, device="cuda")
+    torch.cuda.synchronize()
+    for i in range(calls):
+        with torch.cuda.stream(side):
+            for _ in range(i % 4):
+                junk[: 1 << (12 + i % 11)].mul_(1.0)
+        ops.gemv_fused(xd, [dict(seg, out=outs[i])], layout=1, tokens=M, cols=cols, umma_scratch=scratch, pdl=i % 2 == 1)
+    torch.cuda.synchronize()
+    got = host(outs)
+    assert np.array_equal(got, np.broadcast_to(got[0], got.shape))
+    y64 = [np.stack([orc.gemv_mlx_f64(w, s, x[m]) for m in range(M)]) for w, s in mats]
+    want = y64[0] / (1 + np.exp(-y64[0])) * y64[1] if swiglu else y64[0]
+    assert np.max(np.abs(got[0] - want)) <= (2e-5 if swiglu else 4e-6) * np.abs(want).max()
 
 
 def test_gemm_umma_extreme_tokens(cuda):
