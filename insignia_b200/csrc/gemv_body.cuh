@@ -243,7 +243,7 @@ __device__ __forceinline__ void store_pieces(float4 v, float alpha, __half *hi, 
     *reinterpret_cast<uint2 *>(hi + stride) = *reinterpret_cast<const uint2 *>(l);
 }
 
-// ---- activation prologue: fp32 vector (fetched by load_activation) -> two fp16 pieces in shared memory ----
+// ---- activation prologue: fp32 vector (fetched by load_activation_part) -> two fp16 pieces in shared memory ----
 // Returns 1/alpha, which undoes the power-of-two pre-scale.
 __device__ __forceinline__ float prologue(const GemvParams &p, const ProIn &pin, int m, float4 (&v)[kMaxVec], __half *xs, int xstride,
                                           const uint2 (&wpre)[kPreVec], float *scratch)

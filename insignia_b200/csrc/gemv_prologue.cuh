@@ -58,11 +58,9 @@ template <int J0, int J1> __device__ __forceinline__ void load_activation_part(c
         if (i < nvec) v[j] = __ldcg(reinterpret_cast<const float4 *>(in) + i);
     }
 }
-__device__ __forceinline__ void load_activation(const ProIn &p, int m, float4 (&v)[kMaxVec]) { load_activation_part<0, kMaxVec>(p, m, v); }
 
-// Applies the fused transform to the vector load_activation fetched and returns max |x| over it (without MAX: 0).  `scratch`
-// needs 32 floats.
-template <bool MAX = true> __device__ __forceinline__ float transform_activation(const ProIn &p, int m, float4 (&v)[kMaxVec], const uint2 (&wpre)[kPreVec], float *scratch)
+// Applies the fused transform to the vector load_activation_part fetched and returns max |x| over it.  `scratch` needs 32 floats.
+__device__ __forceinline__ float transform_activation(const ProIn &p, int m, float4 (&v)[kMaxVec], const uint2 (&wpre)[kPreVec], float *scratch)
 {
     const int cols = p.cols, tid = threadIdx.x, lane = tid & 31;
     const int nvec = cols >> 2;
@@ -77,14 +75,14 @@ template <bool MAX = true> __device__ __forceinline__ float transform_activation
 #pragma unroll
         for (int j = 0; j < kMaxVec; j++) {
             const int i = tid + j * kProThreads;
-            if (MAX && i < nvec) {
+            if (i < nvec) {
                 const uint2 wv = j < kPreVec ? wpre[j < kPreVec ? j : 0] : reinterpret_cast<const uint2 *>(p.norm_w)[p.prologue == INSG_PRO_GATED_RMSNORM ? lane : i];
                 pre = fmaxf(pre, fmaxf(fmaxf(fabsf(v[j].x * bf16_bits_to_float(wv.x & 0xffff)), fabsf(v[j].y * bf16_bits_to_float(wv.x >> 16))),
                                        fmaxf(fabsf(v[j].z * bf16_bits_to_float(wv.y & 0xffff)), fabsf(v[j].w * bf16_bits_to_float(wv.y >> 16)))));
             }
         }
         ss = warp_sum(ss);
-        if (MAX) pre = warp_max(pre);
+        pre = warp_max(pre);
         __syncthreads();
         if (lane == 0) { scratch[tid >> 5] = ss; scratch[16 + (tid >> 5)] = pre; }
         __syncthreads();
@@ -144,7 +142,6 @@ template <bool MAX = true> __device__ __forceinline__ float transform_activation
             if (p.x_out && blockIdx.x == 0) reinterpret_cast<float4 *>(p.x_out + size_t(m) * cols)[i] = x;
         }
     }
-    if (!MAX) return 0.f;
     return p.prologue == INSG_PRO_RMSNORM ? amax : block_max16(amax, scratch);
 }
 
