@@ -152,14 +152,17 @@ struct DigitizeParams {
 };
 
 // `parts` CTAs of eight warps per token slot, each a slice of the k-blocks (slots beyond `tokens` are written as zeros so that their columns
-// contribute nothing).  A warp takes a k-block at a time, four on their way at once; everything but the RMSNorm's sum stays inside the warp
-// (a head of the gated norm is one k-block), and that sum is the one barrier.  What bounds it: the latency of a CTA's chain, load to last
-// store, times the rounds of CTAs; so the CTAs are small enough for four an SM, 592 at once (4096 columns: 512 tokens 13.5 -> 9.9 us against one
-// CTA of sixteen warps per token, two an SM; 16 tokens 5.5 -> 3.7, 61 tokens 6.2 -> 4.4; 12288 columns 25 -> 23, bound by the ALU).
+// contribute nothing).  A warp takes a k-block at a time, two on their way at once; everything but the RMSNorm's sum stays inside the warp
+// (a head of the gated norm is one k-block), and that sum is the one barrier.  With few tokens a CTA's chain, load to last store, is the
+// time, so the CTAs are small enough for four an SM, 592 at once.  With many it is short of no single thing: issue and ALU are some 60 %
+// busy, 512 tokens of 12288 columns take 13 % less without the stores and 32 % less without the digits' arithmetic.  Replayed
+// alone, sixteen-warp CTAs of a token with eight base-9 digits -> this with four k-blocks on their way -> with two (less code to run through):
+//   4096 columns, 16 tokens 2.63 -> 2.64 -> 2.43 us (gated norm 3.93 -> 2.92 -> 2.74), 128: 4.12 -> 4.46 -> 4.30, 512: 10.3 -> 9.7 -> 9.2
+//   12288 columns, 16 tokens 3.43 -> 3.20 -> 3.01 us, 128: 7.67 -> 7.96 -> 7.64, 512: 21.0 -> 23.8 -> 22.0
 template <int TPG>
 __global__ void __launch_bounds__(kDigThreads, 4) umma_digitize_kernel(const __grid_constant__ DigitizeParams p)
 {
-    constexpr int kBatch = 4, kWarps = kDigThreads / 32;
+    constexpr int kBatch = 2, kWarps = kDigThreads / 32;
     __shared__ float scratch[kWarps];
     __shared__ uint16_t table[kPair];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
