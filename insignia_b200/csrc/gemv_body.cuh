@@ -262,8 +262,9 @@ __device__ __forceinline__ float prologue(const GemvParams &p, const ProIn &pin,
 }
 
 // Vectors that go in as they are, of up to 4096 columns: all tokens are loaded at once and their largest magnitudes found behind
-// one barrier, where token by token each costs a trip to L2 and two barriers (12352 x 4096 with three tokens PLAIN_X3, 4096 x 4096 with
-// one PLAIN_O1).  The same scale and pieces.
+// one barrier, where token by token each costs a trip to L2 and two barriers (replayed from a graph, token by token -> like this:
+// 12352 x 4096 with three tokens 15.1 -> 12.6 us, 4096 x 4096 with one 7.2 -> 6.4, with four 11.2 -> 8.5).  The same scale and pieces.
+// Wider vectors stay token by token: three times the registers of the vectors that four tokens hold here.
 template <int M>
 __device__ __forceinline__ void prologue_plain(const ProIn &pin, __half *xs, int xstride, float *scratch, float (&inv_alpha)[M])
 {

@@ -11,9 +11,9 @@
 // normal inputs; base 9: 8e-8).  A token takes 7 columns of N.
 //
 // What bounds it: filling shared memory and the tensor pipe together.  A stage multiplies two 128-row weight records (17.4 KB) with the
-// digits of a group of tokens; an SM takes in some 55 bytes a clock from L2.  Thirty-two tokens (15.4 KB, N = 224) fill tensor memory
-// (448 of 512 columns, beside the scale factors) and make the most of the weights' bytes; 24576 x 4096 at 512 tokens: 150 us with eight
-// digits and 24 tokens, 127 like this.
+// digits of a group of tokens; at 512 tokens an SM takes in some 48 bytes a clock from L2 and its tensor pipe is busy 82 % of the time.
+// Thirty-two tokens (15.4 KB, N = 224) fill tensor memory (448 of 512 columns, beside the scale factors) and make the most of the weights'
+// bytes; 24576 x 4096 at 512 tokens: 148 us with eight digits and 24 tokens, 123 like this.
 //
 // Kernels:
 //   umma_digitize_kernel  one CTA or more per token: the fused activation prologue (RMSNorm, gates, ...), then the digit
@@ -136,7 +136,7 @@ struct GSeg {
 
 struct GParams {
     const uint8_t *bimg;    // [nkb][ngroups][digit_block(tpg)]
-    float *partials;        // [grid][2 cut units][2 records of the pair][128 rows][tpg]
+    float *partials;        // [grid][2 cut units][2 records of the pair][tpg / 4][128 rows][4 tokens], a record's part in kSlotFloats
     int *tickets;           // [grid], zero between launches
     int nkb, nseg, total_tiles, stages, ngroups, tokens;
     int total_stages, share, share_rem; // CTA c owns stages [share * c + share_rem * c / G, ...): all products stay in 32 bits
@@ -483,7 +483,7 @@ template <int TPG, bool SWIGLU>
 __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid_constant__ GParams p)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
-    constexpr int kBBlock = digit_block(TPG);       // digits of the group's tokens for one k-block: 8 * TPG columns x 128 k x 4 bit, and their scales
+    constexpr int kBBlock = digit_block(TPG);       // digits of the group's tokens for one k-block: 7 * TPG columns x 128 k x 4 bit, and their scales
     constexpr int kGStage = 2 * kURec + kBBlock;    // one ring stage: the pair's weight records + the digit block both multiply
     constexpr int N = kDigits * TPG;
     constexpr uint32_t kD1Col = TPG == 32 ? 224 : 128, kSfaCol = 448, kSfbCol = 480;
@@ -745,8 +745,12 @@ std::mutex g_gemm_attr_mutex;
 bool g_gemm_attr_done[64] = {false}; // the shared-memory opt-in is a per-device function attribute
 
 // Tokens per group.  32 take fewer bytes into shared memory than 16 for every count beyond 48, the last group's padding included.  Up to
-// 48 the weights bound the time and every CTA ends on a cut unit, whose parts 32 tokens make twice as large and whose ring is shorter
-// (24576 x 4096: 40 tokens 28.2 us; 61 tokens in two groups 29.4).
+// 48 the weights bound the time and every CTA ends on a cut unit, whose parts 32 tokens make twice as large and whose ring is shorter.
+// 16 / 32 a group, microseconds replayed:  24576 x 4096   4096 x 12288   12352 x 4096   4096 x 4096
+//   33..48 tokens                           26.2 / 25.9    22.0 / 27.3    19.1 / 22.3   15.6 / 23.0
+//   49..64                                  32.0 / 26.4    25.3 / 26.1    22.5 / 22.5   16.8 / 22.6    (a layer's four: even)
+//   65..72                                  37.1 / 31.4    28.1 / 27.4    25.7 / 22.7   18.2 / 18.8
+//   512                                      167 / 123      104 / 78        93 / 68       42 / 34
 int tokens_per_group(int tokens) { return tokens <= 48 ? 16 : 32; }
 size_t image_bytes(int cols, int tokens)
 {
