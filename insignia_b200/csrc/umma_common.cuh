@@ -30,9 +30,25 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *b, uint32_t bytes)
 // Bounded wait on a phase parity; false when the limit ran out or another role raised the abort flag.
 __device__ __forceinline__ bool mbar_wait(uint64_t *b, uint32_t parity, volatile int *abort_flag)
 {
+#pragma unroll 1
     for (uint32_t it = 0; it < kSpinLimit; it++) {
         uint32_t done;
         asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(done) : "r"(smem_u32(b)), "r"(parity) : "memory");
+        if (done) return true;
+        if ((it & 1023u) == 1023u && *abort_flag) return false;
+    }
+    *abort_flag = 1;
+    return false;
+}
+
+// A wait on data other CTAs of the cluster send (acquire at cluster scope).
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *b, uint32_t parity, volatile int *abort_flag)
+{
+#pragma unroll 1
+    for (uint32_t it = 0; it < kSpinLimit; it++) {
+        uint32_t done;
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
                      : "=r"(done) : "r"(smem_u32(b)), "r"(parity) : "memory");
         if (done) return true;
         if ((it & 1023u) == 1023u && *abort_flag) return false;

@@ -112,20 +112,6 @@ template <int T> __device__ __forceinline__ void send_floats(uint32_t dst, const
                          ::"r"(dst + 4 * t), "f"(v[t]), "f"(v[t + 1]), "f"(v[t + 2]), "f"(v[t + 3]), "r"(bar) : "memory");
     }
 }
-// A wait on data other CTAs of the cluster send (acquire at cluster scope).
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *b, uint32_t parity, volatile int *abort_flag)
-{
-    for (uint32_t it = 0; it < kSpinLimit; it++) {
-        uint32_t done;
-        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-                     : "=r"(done) : "r"(smem_u32(b)), "r"(parity) : "memory");
-        if (done) return true;
-        if ((it & 1023u) == 1023u && *abort_flag) return false;
-    }
-    *abort_flag = 1;
-    return false;
-}
-
 __device__ __forceinline__ int dseg_of(const DParams &p, int unit)
 {
     int s = 0;
@@ -173,12 +159,21 @@ template <int T> __device__ __forceinline__ void load_partial(uint32_t taddr, fl
 // half an SM (24576 x 4096 as SwiGLU 14.3 -> 13.3 us in the chain); one matrix keeps two (one: 9.7 -> 10.7 us at 12352 x 4096).
 template <int T> __host__ __device__ constexpr int unit_slots(int nmat) { return T == 1 ? 4 : T == 8 ? 3 - nmat : 2; }
 
-template <int T>
+// What a variant of the kernel has beside its tokens: a prepared input in place of the prologue, the logits' arg-max.
+// A token is 129 launches of some seven microseconds, and instructions that a launch runs through for the first time come
+// from L2 behind the stream of weights: as one kernel with everything in it (96 KB of code for one token, 125 for eight; prepared variants
+// 41 and 53) a token took 1084 us, three sequences 1308, eight 1503 and a speculative pass 1500; as variants, with the waits' loops
+// not unrolled and one store and one copy of the digits' code behind all epilogues, 1057, 1208, 1412 and 1428.  (20 KB more in the
+// issuer's loop, never run, cost a token 80 us.)
+constexpr int kDPrepared = 1, kDLogits = 2;
+
+template <int T, int F>
 __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_constant__ DParams p)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int kBKb = 512 * T;       // digit bytes per k-block
     constexpr int kImg = kBKb + 512;    // a k-block of the image: digits, then their scale block
+    constexpr bool prepared = (F & kDPrepared) != 0, logits = (F & kDLogits) != 0;
     constexpr int N = kDDigits * T;
     constexpr int kSlot = kDCl * 32 * T; // floats of one exchange slot: [source rank][32 rows][T]
     // The four owner warps: with several tokens they split the tokens of a unit among them (TN each), else they take units in turn.
@@ -200,7 +195,6 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     uint8_t *ring = smem;                                // S stages
     uint8_t *bimg = ring + size_t(S) * kDStage; // len x kImg bytes
     float *xslot = reinterpret_cast<float *>(bimg + size_t((nkb + 3) >> 2) * kImg); // XU * nmat exchange slots
-    const bool prepared = p.prologue == INSG_PRO_PREPARED;
     float *s_ssq = T < 8 ? s_ssq_static : xslot + XU * nmat * kSlot; // [token][k-block], unless the input is prepared
 
     // ---- the weight stream starts first: it depends on nothing ----------------------------------------------------------
@@ -215,26 +209,31 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         bulk_load(ring + size_t(slot) * kDStage, src + size_t(st) * kDStage, bytes, &full[slot]);
     };
     if (warp == 9) {
-        if (lane == 0) {
-            for (int i = 0; i < S; i++) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (lane < S) { // one lane per stage: its barriers and the first ring's copy into it
+            mbar_init(&full[lane], 1);
+            mbar_init(&empty[lane], 1);
         }
-        __syncwarp();
-        if (lane < S && lane < nstages) { // the first ring: one lane per stage
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (lane < S && lane < nstages) {
             const int run = lane / spt;
             load_stage(lane, run_src(run), lane - run * spt);
         }
     } else if (warp == 8) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(kDTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    } else if (tid == 0) {
-        for (int i = 0; i < 2; i++) { mbar_init(&dfull[i], 1); mbar_init(&dempty[i], 4); }
-        for (int i = 0; i < 8; i++) { mbar_init(&xfull[i], 1); mbar_init(&xempty[i], kDCl * TW); }
-        mbar_init(&ssfull, 1);
-        for (int i = 0; i < kDMaxKb / 8; i++) mbar_init(&image[i], prepared ? 1u : uint32_t(T * max(1, min(8, len - 8 * i)))); // one arrival per (token, k-block), or the copy's
-        s_abort = 0;
-        mbar_expect_tx(&ssfull, kDCl * T * 4);
+    } else if (warp == 0) { // the other barriers, one per lane
+        if (lane < 2) mbar_init(&dfull[lane], 1);
+        else if (lane < 4) mbar_init(&dempty[lane - 2], 4);
+        else if (lane < 12) mbar_init(&xfull[lane - 4], 1);
+        else if (lane < 20) mbar_init(&xempty[lane - 12], kDCl * TW);
+        else if (lane < 20 + kDMaxKb / 8) // one arrival per (token, k-block), or the copy's
+            mbar_init(&image[lane - 20], prepared ? 1u : uint32_t(T * max(1, min(8, len - 8 * (lane - 20)))));
+        else if (lane == 31) {
+            mbar_init(&ssfull, 1);
+            s_abort = 0;
+            mbar_expect_tx(&ssfull, kDCl * T * 4);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     } else if (tid >= 128 && tid < 128 + 81) {
         s_lut[tid - 128] = digit_pair_code(tid - 128);
@@ -254,7 +253,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     volatile int *abort_flag = &s_abort;
     bool arrived = false; // at the closing cluster barrier
 
-    if (prepared) {
+    if constexpr (prepared) {
         if (warp >= 4 && warp < 8) pdl_wait(); // they read what earlier launches wrote
     } else if (warp < 8) {
         // ---- activation prologue: this CTA's quarter of the columns ---------------------------------------------------------
@@ -348,6 +347,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             const int dst = lane / T, m = lane - dst * T;
             float ss[1] = {0.f};
             if (rms)
+#pragma unroll 4
                 for (int kb = 0; kb < len; kb++) ss[0] += s_ssq[m * kDMaxKb + kb];
             send_floats<1>(map_to_rank(smem_u32(&s_rss[rank * T + m]), uint32_t(dst)), ss, map_to_rank(smem_u32(&ssfull), uint32_t(dst)));
         }
@@ -364,9 +364,10 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 }
                 __syncwarp();
             }
-            if (prepared) { // the digits come ready: eight k-blocks per copy, so that the multiplies can start behind the first
+            if constexpr (prepared) { // the digits come ready: eight k-blocks per copy, so that the multiplies can start behind the first
                 pdl_wait();
                 asm volatile("fence.proxy.async.global;" ::: "memory"); // written by ordinary stores of the launch before
+#pragma unroll 1
                 for (int kb = 0; kb < len; kb += 8)
                     if (one) {
                         const uint32_t bytes = uint32_t(min(8, len - kb)) * kImg;
@@ -377,8 +378,10 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             int i = 0, slot = 0;
             uint32_t phase = 1; // of the empty barriers: slot reuse n waits for the n-th release
             bool ok = true;
+#pragma unroll 1
             for (int run = 0; run < nruns && ok; run++) {
                 const uint8_t *src = run_src(run);
+#pragma unroll 1
                 for (int st = 0; st < spt; st++, i++) {
                     if (i >= S) {
                         ok = mbar_wait(&empty[slot], phase, abort_flag);
@@ -407,6 +410,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             int st = 0, sfa = 0;
             uint32_t phase = 0;
             bool here = mbar_test(&full[0], 0), room = true;
+#pragma unroll 1
             for (int run = 0; run < nruns && ok; run++) {
                 const int buf = run & 1;
                 const uint32_t dcol = tmem + uint32_t(64 * buf);
@@ -422,7 +426,8 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                     if (!here && !mbar_wait(&full[st], phase, abort_flag)) return false;
                     if (first && (kb & 7) == 0 && !mbar_wait(&image[kb >> 3], 0, abort_flag)) return false; // the digits of eight k-blocks
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t da = da0 + uint64_t(uint32_t(st) * uint32_t(kDStage >> 4)), dsf = dsf0 + uint64_t(uint32_t(st) * uint32_t(kDStage >> 4));
+                    const uint64_t off = uint64_t(uint32_t(st) * uint32_t(kDStage >> 4)), da = da0 + off, dsf = dsf0 + off;
+                    const uint64_t dsb = dsb0 + uint64_t(kb * (kImg >> 4));
                     const uint32_t sa = tmem + kDSfaCol + 8 * sfa;
                     const int cur = st;
                     if (++st == S) { st = 0; phase ^= 1; }
@@ -430,8 +435,8 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                     if (kb + 2 >= len) room = mbar_test(&dempty[buf ^ 1], (((run + 1) >> 1) & 1) ^ 1);
                     if (one) {
                         if (first) { // the digits' scales stay in tensor memory for all tiles
-                            copy_scales(sb, dsb0 + uint64_t(kb * (kImg >> 4)));
-                            if (two) copy_scales(sb + 4, dsb0 + uint64_t((kb + 1) * (kImg >> 4)));
+                            copy_scales(sb, dsb);
+                            if (two) copy_scales(sb + 4, dsb + (kImg >> 4));
                         }
                         copy_scales(sa, dsf);
                         if (two) copy_scales(sa + 4, dsf + (kURec >> 4));
@@ -452,11 +457,13 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 constexpr std::false_type no{};
                 const int even = len & ~1;
                 if (run == 0) {
+#pragma unroll 1
                     for (int kb = 0; kb < even && ok; kb += 2) ok = stage(kb, yes, yes);
                     if (ok && even < len) ok = stage(even, yes, no);
                 } else {
+#pragma unroll 1
                     for (int kb = 0; kb < even && ok; kb += 2) ok = stage(kb, no, yes);
-                    if (ok && even < len) ok = stage(even, no, no);
+                    if (ok && even < len) ok = stage(even, yes, no); // the digits' scales once more: no copy of the code for a rare case
                 }
                 if (ok && one) commit_to(&dfull[buf]);
             }
@@ -467,6 +474,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         const uint32_t dbar = map_to_rank(smem_u32(xfull), uint32_t(warp));
         const int nslots = XU * nmat;
         bool ok = true;
+#pragma unroll 1
         for (int run = 0; run < nruns && ok; run++) {
             const int buf = run & 1;
             float y[T];
@@ -496,7 +504,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         bool ok = true;
         // The quarters' sums of squares arrive while the weights are still being multiplied.  Every CTA waits for all four
         // (also where they are not needed), so that nobody leaves while a peer still writes into its shared memory.
-        if (!prepared) ok = __all_sync(0xffffffffu, mbar_wait_cluster(&ssfull, 0, abort_flag));
+        if constexpr (!prepared) ok = __all_sync(0xffffffffu, mbar_wait_cluster(&ssfull, 0, abort_flag));
 #pragma unroll
         for (int u = 0; u < TN; u++) {
             const int t = t0 + u;
@@ -505,6 +513,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 const int groups = p.cols >> 5;
                 float ss = 0.f;
                 if (t < p.tokens)
+#pragma unroll 4
                     for (int i = lane; i < groups; i += 32) ss += __ldcg(p.prep_partials + t * groups + i);
                 sc = rsqrtf(warp_sum(ss) / float(p.cols) + 1e-6f);
             } else if (p.prologue == INSG_PRO_RMSNORM) {
@@ -513,8 +522,10 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             if (lane == 0) s_scale[t] = sc;
         }
         asm volatile("bar.sync 3, 128;" ::: "memory");
-        if (ok && p.x_out && cl == 0 && p.prologue == INSG_PRO_RMSNORM)
+        if (!prepared && ok && p.x_out && cl == 0 && p.prologue == INSG_PRO_RMSNORM)
+#pragma unroll 1
             for (int m = 0; m < p.tokens; m++)
+#pragma unroll 1
                 for (int k = kb0 * 128 + fw * 32 + lane; k < (kb0 + len) * 128; k += 128)
                     p.x_out[size_t(m) * p.cols + k] = __ldcg(p.in + size_t(m) * p.cols + k) * s_scale[m] * bf16_bits_to_float(p.norm_w[k]);
         // What the epilogue of a unit needs besides the sums: asked for before the wait for them; where one warp has two tokens of
@@ -547,6 +558,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             }
         };
         if (kAhead && ok && group < nun) fetch(group);
+#pragma unroll 1
         for (int i = group; i < nun && ok; i += kGroups) {
             const int unit = cl + i * C;
             const DSeg &s = p.seg[dseg_of(p, unit)];
@@ -581,6 +593,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 if (T > 1 && one_history && s.epilogue == INSG_EPI_CONV_SILU) { // the history runs through the tokens: one warp takes them in order
                     if (t0 == 0 && on) {
                         float h0 = f.h[0][0], h1 = f.h[0][1], h2 = f.h[0][2];
+#pragma unroll 1
                         for (int t = 0; t < p.tokens; t++) {
                             const float raw = sum(t);
                             out[t * ld] = fast_silu(fmaf(h0, cw0, fmaf(h1, cw1, fmaf(h2, cw2, raw * cw3))));
@@ -601,64 +614,56 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 arrived = true;
             }
             if (!on) continue;
-            switch (s.epilogue) {
-            case INSG_EPI_STORE:
-#pragma unroll
-                for (int u = 0; u < TN; u++)
-                    if (t0 + u < p.tokens) out[(t0 + u) * ld] = y[0][u];
-                break;
-            case INSG_EPI_RESIDUAL:
-#pragma unroll
-                for (int u = 0; u < TN; u++)
-                    if (t0 + u < p.tokens) {
-                        const float v = f.h[u][0] + y[0][u];
-                        out[(t0 + u) * ld] = v;
-                        if (s.prep) leave_digits<T>(s, v, pw, row, t0 + u, s_lut, lane);
-                    }
-                break;
-            case INSG_EPI_CONV_SILU: {
-                if (T > 1 && one_history) break; // done above
-#pragma unroll
-                for (int u = 0; u < TN; u++) {
-                    const int t = t0 + u;
-                    if (t < p.tokens) {
-                        float *hist = s.conv_state + t * s.conv_stride + size_t(row) * 3; // independent sequences: each token has its own
-                        const float z = fmaf(f.h[u][0], cw0, fmaf(f.h[u][1], cw1, fmaf(f.h[u][2], cw2, y[0][u] * cw3)));
-                        out[t * ld] = fast_silu(z);
-                        hist[0] = f.h[u][1]; hist[1] = f.h[u][2]; hist[2] = y[0][u];
-                    }
-                }
-                break;
-            }
-            case INSG_EPI_BETA:
-#pragma unroll
-                for (int u = 0; u < TN; u++)
-                    if (t0 + u < p.tokens) out[(t0 + u) * ld] = fast_sigmoid(y[0][u]);
-                break;
-            case INSG_EPI_DECAY:
-#pragma unroll
-                for (int u = 0; u < TN; u++) {
-                    const float z = y[0][u] + f.h[0][0];
-                    if (t0 + u < p.tokens) out[(t0 + u) * ld] = f.h[0][1] * (z > 20.f ? z : log1pf(__expf(z)));
-                }
-                break;
-            case INSG_EPI_SWIGLU:
-#pragma unroll
-                for (int u = 0; u < TN; u++)
-                    if (t0 + u < p.tokens) {
-                        const float v = fast_silu(y[0][u]) * y[1][u];
-                        out[(t0 + u) * ld] = v;
-                        if (s.prep) leave_digits<T>(s, v, pw, row, t0 + u, s_lut, lane);
-                    }
-                break;
-            case INSG_EPI_LOGITS:
+            if constexpr (logits) {
                 out[0] = y[0][0];
                 if (y[0][0] > best || (y[0][0] == best && row < best_idx)) { best = y[0][0]; best_idx = row; }
-                break;
-            default: break;
+            } else {
+                // Each epilogue leaves its value in v; one store and one copy of the digits' code serve them all.
+                float v[TN];
+                if (T > 1 && one_history && s.epilogue == INSG_EPI_CONV_SILU) continue; // done above
+#pragma unroll
+                for (int u = 0; u < TN; u++) v[u] = y[0][u];
+                switch (s.epilogue) {
+                case INSG_EPI_RESIDUAL:
+#pragma unroll
+                    for (int u = 0; u < TN; u++) v[u] = f.h[u][0] + y[0][u];
+                    break;
+                case INSG_EPI_CONV_SILU:
+#pragma unroll
+                    for (int u = 0; u < TN; u++) {
+                        if (t0 + u < p.tokens) {
+                            float *hist = s.conv_state + (t0 + u) * s.conv_stride + size_t(row) * 3; // independent sequences: each token has its own
+                            v[u] = fast_silu(fmaf(f.h[u][0], cw0, fmaf(f.h[u][1], cw1, fmaf(f.h[u][2], cw2, y[0][u] * cw3))));
+                            hist[0] = f.h[u][1]; hist[1] = f.h[u][2]; hist[2] = y[0][u];
+                        }
+                    }
+                    break;
+                case INSG_EPI_BETA:
+#pragma unroll
+                    for (int u = 0; u < TN; u++) v[u] = fast_sigmoid(y[0][u]);
+                    break;
+                case INSG_EPI_DECAY:
+#pragma unroll
+                    for (int u = 0; u < TN; u++) {
+                        const float z = y[0][u] + f.h[0][0];
+                        v[u] = f.h[0][1] * (z > 20.f ? z : log1pf(__expf(z)));
+                    }
+                    break;
+                case INSG_EPI_SWIGLU:
+#pragma unroll
+                    for (int u = 0; u < TN; u++) v[u] = fast_silu(y[0][u]) * y[1][u];
+                    break;
+                default: break;
+                }
+#pragma unroll
+                for (int u = 0; u < TN; u++) {
+                    if (t0 + u >= p.tokens) break;
+                    out[(t0 + u) * ld] = v[u];
+                    if (s.prep) leave_digits<T>(s, v[u], pw, row, t0 + u, s_lut, lane);
+                }
             }
         }
-        if (p.argmax_partial) {
+        if constexpr (logits) {
             // per-CTA arg-max, then the last CTA of the grid folds the CTAs' (lowest index on ties)
             auto fold = [&] {
 #pragma unroll
@@ -674,6 +679,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             asm volatile("bar.sync 2, 128;" ::: "memory");
             if (fw == 0) {
                 if (lane == 0) {
+#pragma unroll 1
                     for (int w = 1; w < 4; w++)
                         if (s_best[w] > best || (s_best[w] == best && s_bidx[w] < best_idx)) { best = s_best[w]; best_idx = s_bidx[w]; }
                     p.argmax_partial[blockIdx.x] = make_float2(best, __int_as_float(best_idx));
@@ -686,6 +692,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                     __threadfence();
                     best = -3.402823466e38f;
                     best_idx = 0x7fffffff;
+#pragma unroll 1
                     for (int i = lane; i < int(gridDim.x); i += 32) {
                         const float2 e = __ldcg(p.argmax_partial + i);
                         const int idx = __float_as_int(e.y);
@@ -764,7 +771,8 @@ int device_clusters(int *out)
     if (dev < 0 || dev >= 64) return fail(INSG_E_LIMIT, "gemv: device ordinal beyond 63");
     std::lock_guard<std::mutex> lock(g_attr_mutex);
     if (!g_max_clusters[dev]) {
-        for (auto k : {umma_gemv_kernel<1>, umma_gemv_kernel<2>, umma_gemv_kernel<4>, umma_gemv_kernel<8>}) {
+        for (auto k : {umma_gemv_kernel<1, 0>, umma_gemv_kernel<1, 1>, umma_gemv_kernel<1, 2>, umma_gemv_kernel<1, 3>, umma_gemv_kernel<2, 0>, umma_gemv_kernel<2, 1>,
+                       umma_gemv_kernel<4, 0>, umma_gemv_kernel<4, 1>, umma_gemv_kernel<8, 0>, umma_gemv_kernel<8, 1>}) {
             e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
             if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(umma gemv)");
         }
@@ -779,7 +787,7 @@ int device_clusters(int *out)
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int n = 0;
-        e = cudaOccupancyMaxActiveClusters(&n, umma_gemv_kernel<1>, &cfg);
+        e = cudaOccupancyMaxActiveClusters(&n, umma_gemv_kernel<1, 0>, &cfg);
         if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveClusters");
         g_max_clusters[dev] = std::max(1, std::min(n, 128)); // 128 clusters: the arg-max partials are sized for 512 CTAs
     }
@@ -853,8 +861,8 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     const int T = tokens == 1 ? 1 : tokens == 2 ? 2 : tokens <= 4 ? 4 : 8;
     const int kbq = (p.nkb + 3) >> 2;
     const int slots = (T == 1 ? unit_slots<1>(p.nmat) : T == 8 ? unit_slots<8>(p.nmat) : unit_slots<2>(p.nmat)) * p.nmat;
-    const size_t fixed = size_t(kbq) * (512 * T + 512) + size_t(slots) * kDCl * 32 * T * sizeof(float) +
-                         (T == 8 && op->prologue != INSG_PRO_PREPARED ? size_t(8) * kDMaxKb * sizeof(float) : 0);
+    const bool prep = op->prologue == INSG_PRO_PREPARED;
+    const size_t fixed = size_t(kbq) * (512 * T + 512) + size_t(slots) * kDCl * 32 * T * sizeof(float) + (T == 8 && !prep ? size_t(8) * kDMaxKb * sizeof(float) : 0);
     // ring: no more stages than the launch has, within half an SM when that leaves at least four, else whatever fits.  Four are too
     // few to stream at full rate, so a launch of many units (the head: 55 per cluster, eight tokens 97 us against 91) takes the
     // whole SM; one of a few gains more from starting beside its predecessor.
@@ -878,7 +886,10 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = op->pdl ? 2 : 1;
-    auto kernel = T == 1 ? umma_gemv_kernel<1> : T == 2 ? umma_gemv_kernel<2> : T == 4 ? umma_gemv_kernel<4> : umma_gemv_kernel<8>;
+    auto kernel = T == 1 ? (logits ? (prep ? umma_gemv_kernel<1, 3> : umma_gemv_kernel<1, 2>) : (prep ? umma_gemv_kernel<1, 1> : umma_gemv_kernel<1, 0>))
+                : T == 2 ? (prep ? umma_gemv_kernel<2, 1> : umma_gemv_kernel<2, 0>)
+                : T == 4 ? (prep ? umma_gemv_kernel<4, 1> : umma_gemv_kernel<4, 0>)
+                         : (prep ? umma_gemv_kernel<8, 1> : umma_gemv_kernel<8, 0>);
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
     return e == cudaSuccess ? INSG_OK : cuda_fail(e, "umma gemv launch");
 }
