@@ -159,13 +159,13 @@ template <int T> __device__ __forceinline__ void load_partial(uint32_t taddr, fl
 // half an SM (24576 x 4096 as SwiGLU 14.3 -> 13.3 us in the chain); one matrix keeps two (one: 9.7 -> 10.7 us at 12352 x 4096).
 template <int T> __host__ __device__ constexpr int unit_slots(int nmat) { return T == 1 ? 4 : T == 8 ? 3 - nmat : 2; }
 
-// What a variant of the kernel has beside its tokens: a prepared input in place of the prologue, the logits' arg-max.
-// A token is 129 launches of some seven microseconds, and instructions that a launch runs through for the first time come
+// What a variant of the kernel has beside its tokens: a prepared input in place of the prologue, the logits' arg-max, digits that come with
+// the weights.  A token is 129 launches of some seven microseconds, and instructions that a launch runs through for the first time come
 // from L2 behind the stream of weights: as one kernel with everything in it (96 KB of code for one token, 125 for eight; prepared variants
 // 41 and 53) a token took 1084 us, three sequences 1308, eight 1503 and a speculative pass 1500; as variants, with the waits' loops
 // not unrolled and one store and one copy of the digits' code behind all epilogues, 1057, 1208, 1412 and 1428.  (20 KB more in the
 // issuer's loop, never run, cost a token 80 us.)
-constexpr int kDPrepared = 1, kDLogits = 2;
+constexpr int kDPrepared = 1, kDLogits = 2, kDStreamed = 4;
 
 template <int T, int F>
 __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_constant__ DParams p)
@@ -173,7 +173,9 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int kBKb = 512 * T;       // digit bytes per k-block
     constexpr int kImg = kBKb + 512;    // a k-block of the image: digits, then their scale block
-    constexpr bool prepared = (F & kDPrepared) != 0, logits = (F & kDLogits) != 0;
+    constexpr bool prepared = (F & kDPrepared) != 0, logits = (F & kDLogits) != 0, streamed = (F & kDStreamed) != 0;
+    constexpr int kStage = kDStage + (streamed ? 2 * kImg : 0); // streamed: one unit a cluster, so that its digits come with the weights they multiply
+    static_assert(!streamed || prepared, "a streamed image is a prepared one");
     constexpr int N = kDDigits * T;
     constexpr int kSlot = kDCl * 32 * T; // floats of one exchange slot: [source rank][32 rows][T]
     // The four owner warps: with several tokens they split the tokens of a unit among them (TN each), else they take units in turn.
@@ -193,8 +195,8 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     const int nun = cl < p.units ? (p.units - cl + C - 1) / C : 0;             // units of this cluster: cl, cl + C, ...
     const int nruns = nun * nmat, nstages = nruns * spt;
     uint8_t *ring = smem;                                // S stages
-    uint8_t *bimg = ring + size_t(S) * kDStage; // len x kImg bytes
-    float *xslot = reinterpret_cast<float *>(bimg + size_t((nkb + 3) >> 2) * kImg); // XU * nmat exchange slots
+    uint8_t *bimg = ring + size_t(S) * kStage; // len x kImg bytes, unless streamed
+    float *xslot = reinterpret_cast<float *>(bimg + (streamed ? 0 : size_t((nkb + 3) >> 2) * kImg)); // XU * nmat exchange slots
     float *s_ssq = T < 8 ? s_ssq_static : xslot + XU * nmat * kSlot; // [token][k-block], unless the input is prepared
 
     // ---- the weight stream starts first: it depends on nothing ----------------------------------------------------------
@@ -204,9 +206,12 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         return (nmat == 2 && (run & 1) ? s.packed2 : s.packed) + (size_t(unit - s.tile_begin) * nkb + kb0) * kURec;
     };
     auto load_stage = [&](int slot, const uint8_t *src, int st) { // stage st of a run: two records, or the last one of an odd count
-        const uint32_t bytes = uint32_t(min(2, len - 2 * st)) * kURec;
-        mbar_expect_tx(&full[slot], bytes);
-        bulk_load(ring + size_t(slot) * kDStage, src + size_t(st) * kDStage, bytes, &full[slot]);
+        const uint32_t records = uint32_t(min(2, len - 2 * st));
+        mbar_expect_tx(&full[slot], records * (kURec + (streamed ? kImg : 0)));
+        bulk_load(ring + size_t(slot) * kStage, src + size_t(st) * kDStage, records * kURec, &full[slot]);
+    };
+    auto load_digits = [&](int slot, int st) { // streamed: behind the weights of the only run's stage st
+        bulk_load(ring + size_t(slot) * kStage + kDStage, reinterpret_cast<const uint8_t *>(p.in) + size_t(kb0 + 2 * st) * kImg, uint32_t(min(2, len - 2 * st)) * kImg, &full[slot]);
     };
     if (warp == 9) {
         if (lane < S) { // one lane per stage: its barriers and the first ring's copy into it
@@ -367,6 +372,10 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             if constexpr (prepared) { // the digits come ready: eight k-blocks per copy, so that the multiplies can start behind the first
                 pdl_wait();
                 asm volatile("fence.proxy.async.global;" ::: "memory"); // written by ordinary stores of the launch before
+                if constexpr (streamed) {
+                    if (lane < S && lane < nstages) load_digits(lane, lane);
+                    __syncwarp();
+                } else
 #pragma unroll 1
                 for (int kb = 0; kb < len; kb += 8)
                     if (one) {
@@ -386,7 +395,10 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                     if (i >= S) {
                         ok = mbar_wait(&empty[slot], phase, abort_flag);
                         if (!ok) break;
-                        if (one) load_stage(slot, src, st);
+                        if (one) {
+                            load_stage(slot, src, st);
+                            if (streamed) load_digits(slot, st);
+                        }
                         if (i == nstages - 1 - kDTriggerStages<T>) pdl_launch_dependents();
                     }
                     if (++slot == S) { slot = 0; phase ^= 1; }
@@ -404,8 +416,8 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             // E2M1 x E2M1, UE8M0 scales, N columns, M = 128; K-step s of a block uses scale bytes 2s, 2s+1 of both operands
             constexpr uint32_t idesc0 = (1u << 7) | (1u << 10) | ((uint32_t(N) >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
             constexpr uint32_t idesc1 = idesc0 | (2u << 29) | (2u << 4);
-            const uint64_t da0 = umma_desc(smem_u32(ring), 128, 256), dsf0 = umma_desc(smem_u32(ring) + 8192, 16, 128), db0 = umma_desc(smem_u32(bimg), 128, 256);
-            const uint64_t dsb0 = umma_desc(smem_u32(bimg) + kBKb, 16, 128);
+            const uint64_t da0 = umma_desc(smem_u32(ring), 128, 256), dsf0 = umma_desc(smem_u32(ring) + 8192, 16, 128), db0 = umma_desc(smem_u32(streamed ? ring + kDStage : bimg), 128, 256);
+            const uint64_t dsb0 = umma_desc(smem_u32(streamed ? ring + kDStage : bimg) + kBKb, 16, 128);
             bool ok = true;
             int st = 0, sfa = 0;
             uint32_t phase = 0;
@@ -424,10 +436,11 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 auto stage = [&](int kb, auto is_first, auto has_two) -> bool {
                     constexpr bool first = decltype(is_first)::value, two = decltype(has_two)::value;
                     if (!here && !mbar_wait(&full[st], phase, abort_flag)) return false;
-                    if (first && (kb & 7) == 0 && !mbar_wait(&image[kb >> 3], 0, abort_flag)) return false; // the digits of eight k-blocks
+                    if (!streamed && first && (kb & 7) == 0 && !mbar_wait(&image[kb >> 3], 0, abort_flag)) return false; // the digits of eight k-blocks
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t off = uint64_t(uint32_t(st) * uint32_t(kDStage >> 4)), da = da0 + off, dsf = dsf0 + off;
-                    const uint64_t dsb = dsb0 + uint64_t(kb * (kImg >> 4));
+                    const uint64_t off = uint64_t(uint32_t(st) * uint32_t(kStage >> 4)), da = da0 + off, dsf = dsf0 + off;
+                    if (streamed) db = db0 + off;
+                    const uint64_t dsb = streamed ? dsb0 + off : dsb0 + uint64_t(kb * (kImg >> 4));
                     const uint32_t sa = tmem + kDSfaCol + 8 * sfa;
                     const int cur = st;
                     if (++st == S) { st = 0; phase ^= 1; }
@@ -448,7 +461,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                         }
                         commit_to(&empty[cur]);
                     }
-                    db += 2 * (kImg >> 4);
+                    if (!streamed) db += 2 * (kImg >> 4);
                     sb += 8;
                     sfa = (sfa + 1) & 3;
                     return true;
@@ -772,7 +785,7 @@ int device_clusters(int *out)
     std::lock_guard<std::mutex> lock(g_attr_mutex);
     if (!g_max_clusters[dev]) {
         for (auto k : {umma_gemv_kernel<1, 0>, umma_gemv_kernel<1, 1>, umma_gemv_kernel<1, 2>, umma_gemv_kernel<1, 3>, umma_gemv_kernel<2, 0>, umma_gemv_kernel<2, 1>,
-                       umma_gemv_kernel<4, 0>, umma_gemv_kernel<4, 1>, umma_gemv_kernel<8, 0>, umma_gemv_kernel<8, 1>}) {
+                       umma_gemv_kernel<4, 0>, umma_gemv_kernel<4, 1>, umma_gemv_kernel<4, 5>, umma_gemv_kernel<8, 0>, umma_gemv_kernel<8, 1>, umma_gemv_kernel<8, 5>}) {
             e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
             if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(umma gemv)");
         }
@@ -861,17 +874,23 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     const int T = tokens == 1 ? 1 : tokens == 2 ? 2 : tokens <= 4 ? 4 : 8;
     const int kbq = (p.nkb + 3) >> 2;
     const int slots = (T == 1 ? unit_slots<1>(p.nmat) : T == 8 ? unit_slots<8>(p.nmat) : unit_slots<2>(p.nmat)) * p.nmat;
+    const size_t exchange = size_t(slots) * kDCl * 32 * T * sizeof(float), kblock = 512 * T + 512;
+    // Digits that only one unit per cluster reads need not lie in shared memory as a whole: with the weights they multiply, two k-blocks a
+    // stage, they leave the launch within half an SM where the image (61 KB for three tokens of 12288 columns, 111 for eight) would not,
+    // so that it starts beside its predecessor and the next launch beside it: a step of three sequences 1208 -> 1204 us, of eight 1412 -> 1402.
     const bool prep = op->prologue == INSG_PRO_PREPARED;
-    const size_t fixed = size_t(kbq) * (512 * T + 512) + size_t(slots) * kDCl * 32 * T * sizeof(float) + (T == 8 && !prep ? size_t(8) * kDMaxKb * sizeof(float) : 0);
+    const bool streamed = prep && T >= 4 && p.nmat == 1 && p.units <= clusters && kbq * kblock + exchange + 4 * kDStage > size_t(kDHalfSm);
+    const size_t stage_bytes = kDStage + (streamed ? 2 * kblock : 0);
+    const size_t fixed = exchange + (streamed ? 0 : kbq * kblock) + (T == 8 && !prep ? size_t(8) * kDMaxKb * sizeof(float) : 0);
     // ring: no more stages than the launch has, within half an SM when that leaves at least four, else whatever fits.  Four are too
     // few to stream at full rate, so a launch of many units (the head: 55 per cluster, eight tokens 97 us against 91) takes the
     // whole SM; one of a few gains more from starting beside its predecessor.
     const int need = ((p.units + clusters - 1) / clusters) * p.nmat * ((kbq + 1) / 2);
-    int stages = fixed < size_t(kDHalfSm) ? int((kDHalfSm - fixed) / kDStage) : 0;
-    if (stages < 4 || (stages == 4 && need > 96)) stages = int((size_t(222) * 1024 - fixed) / kDStage);
+    int stages = fixed < size_t(kDHalfSm) ? int((kDHalfSm - fixed) / stage_bytes) : 0;
+    if (stages < 4 || (stages == 4 && need > 96)) stages = int((size_t(222) * 1024 - fixed) / stage_bytes);
     p.stages = std::max(1, std::min({stages, need, kDMaxStages}));
     p.ahead = !op->pdl ? 0 : T == 1 ? kDAheadStages<1> : T == 2 ? kDAheadStages<2> : 0; // a launch that waits for its predecessor anyway streams at once
-    const size_t smem = fixed + size_t(p.stages) * kDStage;
+    const size_t smem = fixed + size_t(p.stages) * stage_bytes;
 
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(clusters * kDCl));
@@ -888,8 +907,8 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     cfg.numAttrs = op->pdl ? 2 : 1;
     auto kernel = T == 1 ? (logits ? (prep ? umma_gemv_kernel<1, 3> : umma_gemv_kernel<1, 2>) : (prep ? umma_gemv_kernel<1, 1> : umma_gemv_kernel<1, 0>))
                 : T == 2 ? (prep ? umma_gemv_kernel<2, 1> : umma_gemv_kernel<2, 0>)
-                : T == 4 ? (prep ? umma_gemv_kernel<4, 1> : umma_gemv_kernel<4, 0>)
-                         : (prep ? umma_gemv_kernel<8, 1> : umma_gemv_kernel<8, 0>);
+                : T == 4 ? (streamed ? umma_gemv_kernel<4, 5> : prep ? umma_gemv_kernel<4, 1> : umma_gemv_kernel<4, 0>)
+                         : (streamed ? umma_gemv_kernel<8, 5> : prep ? umma_gemv_kernel<8, 1> : umma_gemv_kernel<8, 0>);
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
     return e == cudaSuccess ? INSG_OK : cuda_fail(e, "umma gemv launch");
 }
