@@ -10,19 +10,21 @@
 // digit j of its token t; the epilogue combines the seven as sum_j 13^j D_j in fp32, which gives the product to ~7e-8 (4096 columns,
 // normal inputs; base 9: 8e-8).  A token takes 7 columns of N.
 //
-// What bounds it: filling shared memory and the tensor pipe together.  A stage multiplies two 128-row weight records (17.4 KB) with the
-// digits of a group of tokens; at 512 tokens an SM takes in some 48 bytes a clock from L2 and its tensor pipe is busy 82 % of the time.
-// Thirty-two tokens (15.4 KB, N = 224) fill tensor memory (448 of 512 columns, beside the scale factors) and make the most of the weights'
-// bytes; 24576 x 4096 at 512 tokens: 148 us with eight digits and 24 tokens, 123 like this.
+// What bounds it: the tensor pipe, and filling shared memory beside it.  A stage multiplies two 128-row weight records (17.4 KB) a CTA with
+// the digits of a group of tokens.  Thirty-two tokens (N = 224) fill tensor memory (448 of 512 columns, beside the scale factors) and
+// make the most of the weights' bytes; two CTAs then work on four records with one set of digits, of which each fetches and holds half
+// (cta_group::2).  24576 x 4096 at 512 tokens, digitize launch included: one CTA a unit 126 us; pairs 121; without the multiplies 83,
+// without the copies 106 (332 stages of 448 cycles on the tensor pipe are 78).
 //
 // Kernels:
 //   umma_digitize_kernel  one CTA or more per token: the fused activation prologue (RMSNorm, gates, ...), then the digit
 //                         image of the token in global memory, laid out as the shared-memory image the MMA reads
 //                         ([k-block][group of tokens][448 bytes x tokens per group, scale blocks], canonical K-major, no swizzle);
-//   umma_gemm_kernel      one CTA per SM.  The work is the sequence of all (pair of records, token group, k-block) stages;
+//   umma_gemm_kernel      one CTA per SM, from 49 tokens on two that work together.  The work is the sequence of all (pair of records, token group, k-block) stages;
 //                         every CTA takes an equal contiguous share of it (stream-K), so SMs are busy whatever the number
 //                         of tiles.  The pair is two row tiles, or the gate and the up tile of the same rows for SwiGLU
-//                         (whose epilogue then has both at hand).  A ring of stages, fetched by cp.async.bulk with mbarrier
+//                         (whose epilogue then has both at hand); two CTAs take twice as many tiles, each with its own
+//                         rows' sums and epilogue, and the first one issues for both.  A ring of stages, fetched by cp.async.bulk with mbarrier
 //                         completion (local, no multicast); one warp issues the scale copies and the MMAs; four epilogue
 //                         warps (tensor memory lane = output row) take a run's sums out before the next one multiplies,
 //                         while the ring refills.  A unit (pair, group) that lies inside one CTA's share goes straight
@@ -42,7 +44,7 @@
 namespace insg {
 
 constexpr int kDigThreads = 256;           // digitize kernel
-constexpr int kGemmThreads = 192;          // GEMM kernel: four epilogue warps, the MMA issuer, the producer
+constexpr int kGemmThreads = 224;          // GEMM kernel: four epilogue warps, the MMA issuer, the producers of weights and of digits
 constexpr int kDigits = 7;                 // base-13 digits per activation = N columns per token
 constexpr int kGSfaBufs = 4;               // scale-factor column sets cycled by stage (a power of two)
 constexpr int kGTmemCols = 512;            // two accumulators of up to 224 columns, weight scale factors [448,480), digit scale factors [480,512)
@@ -53,6 +55,9 @@ constexpr int kSlotFloats = 128 * 32;      // one partial: 128 rows x up to 32 t
 // 512-byte scale block per 128 columns.
 __host__ __device__ constexpr int digit_bytes(int tpg) { return 64 * kDigits * tpg; }
 __host__ __device__ constexpr int digit_block(int tpg) { return digit_bytes(tpg) + (kDigits * tpg + 127) / 128 * 512; }
+// CTAs that work on a unit together.  Groups of 32 tokens: two, whose tensor cores each multiply their own rows with all columns and
+// read half of the digits each from either one's shared memory; the digits then lie [half of the columns][K-step].
+__host__ __device__ constexpr int group_ctas(int tpg) { return tpg == 32 ? 2 : 1; }
 
 // ---- seven digits of an activation -----------------------------------------------------------------------------------------------
 // E2M1 holds 0, 1, 2, 3, 4, 6, 8 and 12 halves of either sign.  Of these, {0, +-1, +-2, +-3, +-4, +-6, +-8} has every residue modulo 13
@@ -110,11 +115,17 @@ template <int TPG> __device__ __forceinline__ void store_digits13(float4 x, int 
     // columns 0, 2, 4, 6 sit in the low nibbles of the four bytes, 1, 3, 5 in the high ones
     const uint32_t e01 = (c0 & 0x0F0F0F0Fu) | ((c1 & 0x0F0F0F0Fu) << 4), e23 = (c2 & 0x0F0F0F0Fu) | ((c3 & 0x0F0F0F0Fu) << 4);
     const uint32_t o01 = ((c0 >> 4) & 0x0F0F0F0Fu) | (c1 & 0xF0F0F0F0u), o23 = ((c2 >> 4) & 0x0F0F0F0Fu) | (c3 & 0xF0F0F0F0u);
-    uint8_t *dst = blk + (lane >> 4) * (digit_bytes(TPG) / 2) + (t >> 3) * 256 + ((lane >> 3) & 1) * 128 + (t & 7) * 16 + (lane & 7) * 2;
+    // columns in groups of eight: [half of the groups][K-step][group][k core][column][16 bytes]
+    constexpr int kHalves = group_ctas(TPG), kGroups = kDigits * TPG / 8 / kHalves;
+    uint8_t *dst = blk + (lane >> 4) * (kGroups * 256) + ((lane >> 3) & 1) * 128 + (t & 7) * 16 + (lane & 7) * 2;
+    auto column = [&](int j) { // of digit j
+        const int g = j * (TPG / 8) + (t >> 3);
+        return dst + g * 256 + (g >= kGroups ? kGroups * 256 : 0);
+    };
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-        *reinterpret_cast<uint16_t *>(dst + (2 * j) * (32 * TPG)) = uint16_t(__byte_perm(e01, e23, j | ((4 + j) << 4)));
-        if (j < 3) *reinterpret_cast<uint16_t *>(dst + (2 * j + 1) * (32 * TPG)) = uint16_t(__byte_perm(o01, o23, j | ((4 + j) << 4)));
+        *reinterpret_cast<uint16_t *>(column(2 * j)) = uint16_t(__byte_perm(e01, e23, j | ((4 + j) << 4)));
+        if (j < 3) *reinterpret_cast<uint16_t *>(column(2 * j + 1)) = uint16_t(__byte_perm(o01, o23, j | ((4 + j) << 4)));
     }
     // scale block: row = column mod 32, then the column quarter, byte = group; a token's columns share the four bytes
     const uint32_t sc = digit_scale(eb);
@@ -353,12 +364,18 @@ __device__ __forceinline__ GRun run_at(const GParams &p, int g, int end)
 // Everything stays in registers (fully unrolled, predicated): with nearly all of the SM's memory configured as shared
 // memory, the little L1 that is left cannot hold a stack frame per thread, and spilled arrays would go to L2 and back.
 // The switch sits outside the token loops so that a launch runs through one short straight-line piece only.
-template <int TPG>
+template <int TPG, bool SWIGLU>
 __device__ __forceinline__ void finish_row(const GParams &p, const GSeg &s, int row, int grp, const float (&y)[TPG], const float (&gate)[TPG])
 {
     const int m0 = grp * TPG, live = min(TPG, p.tokens - m0);
     float *out = s.out + size_t(m0) * s.rows + row;
     const size_t ld = size_t(s.rows);
+    if constexpr (SWIGLU) {
+#pragma unroll
+        for (int t = 0; t < TPG; t++)
+            if (t < live) out[t * ld] = fast_silu(gate[t]) * y[t];
+        return;
+    }
     switch (s.epilogue) {
     case INSG_EPI_RESIDUAL: {
         float r[TPG];
@@ -406,11 +423,6 @@ __device__ __forceinline__ void finish_row(const GParams &p, const GSeg &s, int 
         }
         break;
     }
-    case INSG_EPI_SWIGLU:
-#pragma unroll
-        for (int t = 0; t < TPG; t++)
-            if (t < live) out[t * ld] = fast_silu(gate[t]) * y[t];
-        break;
     default: break;
     }
 }
@@ -453,38 +465,65 @@ template <int TPG> __device__ __forceinline__ void load_sums(uint32_t taddr, flo
     }
 }
 
-// Where the weight records of a pair start (two row tiles, the second one missing after an odd number; or gate and up).
+// The two weight records CTA `rank` of CL multiplies for a unit: row tiles 2 CL u + h CL + rank (h = 0, 1), or the gate and the up tile of
+// rows CL u + rank.  Beyond the last tile a CTA of a pair multiplies that one again and leaves no result.
 struct PairSrc {
-    const uint8_t *a0, *a1;
-    bool has1;
+    const uint8_t *a[2];
+    int tile[2];
+    bool live[2]; // has results
+    bool two;     // the unit has a second record (for all of its CTAs)
 };
-template <bool SWIGLU> __device__ __forceinline__ PairSrc pair_src(const GParams &p, int pair, int kb)
+template <int CL, bool SWIGLU> __device__ __forceinline__ PairSrc pair_src(const GParams &p, int u, int rank, int kb)
 {
     PairSrc q;
-    const int t0 = SWIGLU ? pair : 2 * pair, t1 = t0 + 1;
-    const GSeg &s0 = p.seg[gseg_of(p, t0)];
-    const size_t at = (size_t(t0 - s0.tile_begin) * p.nkb + kb) * kURec;
-    q.a0 = s0.packed + at;
-    if (SWIGLU) {
-        q.has1 = true;
-        q.a1 = s0.packed2 + at;
-        return q;
-    }
-    q.has1 = t1 < p.total_tiles;
-    q.a1 = q.a0;
-    if (q.has1) {
-        const GSeg &s1 = p.seg[gseg_of(p, t1)];
-        q.a1 = s1.packed + (size_t(t1 - s1.tile_begin) * p.nkb + kb) * kURec;
+    q.two = SWIGLU || 2 * CL * u + CL < p.total_tiles;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int want = SWIGLU ? CL * u + rank : 2 * CL * u + h * CL + rank;
+        q.live[h] = want < p.total_tiles;
+        q.tile[h] = min(want, p.total_tiles - 1);
+        const GSeg &s = p.seg[gseg_of(p, q.tile[h])];
+        q.a[h] = (SWIGLU && h == 1 ? s.packed2 : s.packed) + (size_t(q.tile[h] - s.tile_begin) * p.nkb + kb) * kURec;
     }
     return q;
+}
+
+// ---- tcgen05 instructions of one CTA or of a pair (issued by its first CTA) ------------------------------------------------------
+template <int CL> __device__ __forceinline__ void g_copy_scales(uint32_t taddr, uint64_t desc) // CL == 2: in both CTAs, each from its own shared memory
+{
+    if constexpr (CL == 1) copy_scales(taddr, desc);
+    else asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(desc) : "memory");
+}
+template <int CL> __device__ __forceinline__ void g_mma(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, bool accumulate, uint32_t sa, uint32_t sb)
+{
+    if constexpr (CL == 1) mma_step(d, da, db, idesc, accumulate, sa, sb);
+    else
+        asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %4, 0;\n"
+                     "tcgen05.mma.cta_group::2.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%5], [%6], q;\n}"
+                     ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"(uint32_t(accumulate)), "r"(sa), "r"(sb) : "memory");
+}
+template <int CL> __device__ __forceinline__ void g_commit(uint64_t *bar) // CL == 2: arrives at both CTAs' barrier
+{
+    if constexpr (CL == 1) commit_to(bar);
+    else
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                     ::"r"(smem_u32(bar)), "h"(uint16_t(3)) : "memory");
+}
+// Arrival at a barrier of the pair's first CTA.  Nothing is handed over that the arriving thread wrote, so no release: one at cluster scope
+// waits for what the thread's memory operations left behind, some 800 cycles a stage.
+__device__ __forceinline__ void first_arrive(uint64_t *bar)
+{
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(map_to_rank(smem_u32(bar), 0)) : "memory");
 }
 
 template <int TPG, bool SWIGLU>
 __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid_constant__ GParams p)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
-    constexpr int kBBlock = digit_block(TPG);       // digits of the group's tokens for one k-block: 7 * TPG columns x 128 k x 4 bit, and their scales
-    constexpr int kGStage = 2 * kURec + kBBlock;    // one ring stage: the pair's weight records + the digit block both multiply
+    constexpr int CL = group_ctas(TPG);
+    constexpr int kBBlock = digit_block(TPG);                 // the group's digits of one k-block, 7 * TPG columns x 128 k x 4 bit, and their scales
+    constexpr int kBDig = digit_bytes(TPG) / CL, kBScales = kBBlock - digit_bytes(TPG); // this CTA's columns; every CTA has all scales
+    constexpr int kGStage = 2 * kURec + kBDig + kBScales;     // one ring stage: the CTA's two weight records + the digits both multiply
     constexpr int N = kDigits * TPG;
     constexpr uint32_t kD1Col = TPG == 32 ? 224 : 128, kSfaCol = 448, kSfbCol = 480;
     static_assert(N <= int(kD1Col) && kD1Col + N <= int(kSfaCol) && 8 * kGSfaBufs == int(kSfbCol - kSfaCol) && kSfbCol + 8 * kGSfaBufs == uint32_t(kGTmemCols), "tensor memory");
@@ -495,22 +534,34 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort, s_last, s_early[2];
 
-    const int G = int(gridDim.x), c = int(blockIdx.x);
+    const int G = int(gridDim.x) / CL, c = int(blockIdx.x) / CL, rank = int(blockIdx.x) % CL;
     const int begin = share_begin(p, c, G), end = share_begin(p, c + 1, G);
 
     if (tid == 0) {
-        for (int i = 0; i < S; i++) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+        for (int i = 0; i < S; i++) {
+            mbar_init(&full[i], CL == 2 && rank == 0 ? 3 : 2); // the two producers; in the first CTA of a pair the second one's word for its part, too
+            mbar_init(&empty[i], 1);
+        }
         mbar_init(&dfull, 1);
-        mbar_init(&dempty, 4);
+        mbar_init(&dempty, 4 * CL);
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(kGTmemCols));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+        if constexpr (CL == 2) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(kGTmemCols));
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(kGTmemCols));
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if constexpr (CL == 2) { // the other CTA's barriers and tensor memory
+        asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
     pdl_launch_dependents(); // this CTA holds its tensor memory: whatever follows may take an SM as it becomes free
@@ -518,26 +569,19 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
     volatile int *abort_flag = &s_abort;
 
     if (warp == 5) {
-        // ---- producer: the pair's two weight records + the token group's digit block per stage -----------------------
-        // The weights do not depend on the launch before this one (the digit image does): the first ring of weight
-        // records is requested before the programmatic-dependency wait, the digit blocks of those stages after it.
-        // The first ring is requested by one lane per stage (a bulk copy takes the issuing thread a few hundred cycles).
+        // ---- producer of the weights: two records per stage ----------------------------------------------------------
+        // They do not depend on the launch before this one (the digits do): the first ring is requested at once, by one lane per
+        // stage (a bulk copy takes the issuing thread a few hundred cycles).
         const int first = min(S, end - begin);
-        const uint8_t *b0 = nullptr;
-        uint8_t *dst0 = nullptr;
         if (lane < first) {
             const GRun r = run_at(p, begin + lane, end);
-            const int pair = r.unit / p.ngroups, grp = r.unit - pair * p.ngroups;
-            const PairSrc q = pair_src<SWIGLU>(p, pair, r.kb0);
-            b0 = p.bimg + (size_t(r.kb0) * p.ngroups + grp) * kBBlock;
-            dst0 = ring + size_t(lane) * kGStage;
-            mbar_expect_tx(&full[lane], (q.has1 ? 2 : 1) * kURec + kBBlock);
-            bulk_load(dst0, q.a0, kURec, &full[lane]);
-            if (q.has1) bulk_load(dst0 + kURec, q.a1, kURec, &full[lane]);
+            const PairSrc q = pair_src<CL, SWIGLU>(p, r.unit / p.ngroups, rank, r.kb0);
+            uint8_t *dst = ring + size_t(lane) * kGStage;
+            mbar_expect_tx(&full[lane], (q.two ? 2 : 1) * kURec);
+            bulk_load(dst, q.a[0], kURec, &full[lane]);
+            if (q.two) bulk_load(dst + kURec, q.a[1], kURec, &full[lane]);
         }
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        asm volatile("fence.proxy.async.global;" ::: "memory"); // the digits were written by ordinary stores, the bulk copies read them through the async proxy
-        if (lane < first) bulk_load(dst0 + 2 * kURec, b0, kBBlock, &full[lane]);
+        __syncwarp();
         // from here on the whole warp walks the loop and one elected lane issues: warp-uniform operands issue twice as fast
         const bool one = elect_one();
         int g = begin + first, st = first == S ? 0 : first;
@@ -545,74 +589,115 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
         bool ok = true, room = g < end && mbar_test(&empty[st], phase);
         while (g < end && ok) {
             const GRun r = run_at(p, g, end);
-            const int pair = r.unit / p.ngroups, grp = r.unit - pair * p.ngroups;
-            const PairSrc q = pair_src<SWIGLU>(p, pair, r.kb0);
-            const uint8_t *a0 = q.a0, *a1 = q.a1, *b = p.bimg + (size_t(r.kb0) * p.ngroups + grp) * kBBlock;
-            const size_t bstep = size_t(p.ngroups) * kBBlock;
-            const uint32_t bytes = (q.has1 ? 2 : 1) * kURec + kBBlock;
-            for (int k = 0; k < r.len; k++, a0 += kURec, a1 += kURec, b += bstep) {
+            const PairSrc q = pair_src<CL, SWIGLU>(p, r.unit / p.ngroups, rank, r.kb0);
+            const uint8_t *a0 = q.a[0], *a1 = q.a[1];
+            for (int k = 0; k < r.len; k++, a0 += kURec, a1 += kURec) {
                 if (!room && !mbar_wait(&empty[st], phase, abort_flag)) { ok = false; break; }
                 const int cur = st;
                 if (++st == S) { st = 0; phase ^= 1; }
                 room = mbar_test(&empty[st], phase);
                 if (one) {
                     uint8_t *dst = ring + size_t(cur) * kGStage;
-                    mbar_expect_tx(&full[cur], bytes);
+                    mbar_expect_tx(&full[cur], (q.two ? 2 : 1) * kURec);
                     bulk_load(dst, a0, kURec, &full[cur]);
-                    if (q.has1) bulk_load(dst + kURec, a1, kURec, &full[cur]);
-                    bulk_load(dst + 2 * kURec, b, kBBlock, &full[cur]);
+                    if (q.two) bulk_load(dst + kURec, a1, kURec, &full[cur]);
                 }
             }
             g += r.len;
         }
+    } else if (warp == 6) {
+        // ---- producer of the digits: this CTA's columns and all scales -----------------------------------------------
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("fence.proxy.async.global;" ::: "memory"); // the digits were written by ordinary stores, the bulk copies read them through the async proxy
+        auto load = [&](uint8_t *dst, const uint8_t *b, uint64_t *bar) {
+            mbar_expect_tx(bar, kBDig + kBScales);
+            if constexpr (CL == 1) bulk_load(dst, b, kBBlock, bar);
+            else {
+                bulk_load(dst, b + rank * kBDig, kBDig, bar);
+                bulk_load(dst + kBDig, b + digit_bytes(TPG), kBScales, bar);
+            }
+        };
+        const int first = min(S, end - begin);
+        if (lane < first) {
+            const GRun r = run_at(p, begin + lane, end);
+            const int grp = r.unit % p.ngroups;
+            load(ring + size_t(lane) * kGStage + 2 * kURec, p.bimg + (size_t(r.kb0) * p.ngroups + grp) * kBBlock, &full[lane]);
+        }
+        __syncwarp();
+        const bool one = elect_one();
+        int g = begin + first, st = first == S ? 0 : first;
+        uint32_t phase = 0;
+        bool ok = true, room = g < end && mbar_test(&empty[st], phase);
+        while (g < end && ok) {
+            const GRun r = run_at(p, g, end);
+            const uint8_t *b = p.bimg + (size_t(r.kb0) * p.ngroups + r.unit % p.ngroups) * kBBlock;
+            const size_t bstep = size_t(p.ngroups) * kBBlock;
+            for (int k = 0; k < r.len; k++, b += bstep) {
+                if (!room && !mbar_wait(&empty[st], phase, abort_flag)) { ok = false; break; }
+                const int cur = st;
+                if (++st == S) { st = 0; phase ^= 1; }
+                room = mbar_test(&empty[st], phase);
+                if (one) load(ring + size_t(cur) * kGStage + 2 * kURec, b, &full[cur]);
+            }
+            g += r.len;
+        }
+    } else if (warp == 4 && rank == 1) {
+        // ---- the second CTA of a pair tells the first one which of its stages are there ------------------------------
+        int st = 0;
+        uint32_t phase = 0;
+        for (int g = begin; g < end; g++) {
+            if (!mbar_wait(&full[st], phase, abort_flag)) break;
+            if (lane == 0) first_arrive(&full[st]);
+            __syncwarp();
+            if (++st == S) { st = 0; phase ^= 1; }
+        }
     } else if (warp == 4) {
         // ---- MMA issuer --------------------------------------------------------------------------------------------------
         // The whole warp walks the loop and one elected lane issues (see umma_gemv.cu: operands in uniform registers); the next
-        // stage's barrier is polled before this stage's multiplies go out.
+        // stage's barriers are polled before this stage's multiplies go out.
         const bool one = elect_one();
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        // E2M1 x E2M1, UE8M0 scales, N columns, M = 128; K-step s of a block uses scale bytes 2s, 2s+1 of both operands
-        constexpr uint32_t idesc0 = (1u << 7) | (1u << 10) | ((uint32_t(N) >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
+        // E2M1 x E2M1, UE8M0 scales, N columns, M = 128 rows a CTA; K-step s of a block uses scale bytes 2s, 2s+1 of both operands
+        constexpr uint32_t idesc0 = (1u << 7) | (1u << 10) | ((uint32_t(N) >> 3) << 17) | (1u << 23) | (uint32_t(128 * CL >> 4) << 24);
         constexpr uint32_t idesc1 = idesc0 | (2u << 29) | (2u << 4);
         const uint64_t da0 = umma_desc(smem_u32(ring), 128, 256), dsf0 = umma_desc(smem_u32(ring) + 8192, 16, 128);
         const uint32_t d0 = tmem, d1 = tmem + kD1Col;
         int st = 0, sfa = 0;
         uint32_t phase = 0;
-        bool ok = true, here = mbar_test(&full[0], 0);
+        bool ok = true;
         int g = begin;
         for (int run = 0; g < end && ok; run++) {
             const GRun r = run_at(p, g, end);
-            const bool has1 = SWIGLU || 2 * (r.unit / p.ngroups) + 1 < p.total_tiles;
+            const bool two = SWIGLU || 2 * CL * (r.unit / p.ngroups) + CL < p.total_tiles;
             ok = mbar_wait(&dempty, (run & 1) ^ 1, abort_flag); // the first run passes at once
             if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
             for (int k = 0; k < r.len; k++) {
-                if (!here && !mbar_wait(&full[st], phase, abort_flag)) { ok = false; break; }
+                // (Two or four stages behind one look at their barriers, in straight-line code: no faster.)
+                if (!__all_sync(0xffffffffu, mbar_test(&full[st], phase)) && !mbar_wait(&full[st], phase, abort_flag)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t off = uint64_t(uint32_t(st) * uint32_t(kGStage >> 4));
                 const uint64_t da = da0 + off, dsf = dsf0 + off, db = da + uint64_t((2 * kURec) >> 4);
                 const uint32_t sa = tmem + kSfaCol + 8 * sfa, sb = tmem + kSfbCol + 8 * sfa;
-                const int cur = st;
+                uint64_t *back = &empty[st];
                 if (++st == S) { st = 0; phase ^= 1; }
-                here = mbar_test(&full[st], phase);
                 if (one) {
-                    copy_scales(sa, dsf);
-                    if (has1) copy_scales(sa + 4, dsf + (kURec >> 4));
-                    const uint64_t dsb = dsf + uint64_t((2 * kURec - 8192 + digit_bytes(TPG)) >> 4); // 128 columns' scales per copy
-                    copy_scales(sb, dsb);
-                    if (N > 128) copy_scales(sb + 4, dsb + 32);
-                    mma_step(d0, da, db, idesc0, k > 0, sa, sb); // the run's first MMA overwrites
-                    if (has1) mma_step(d1, da + (kURec >> 4), db, idesc0, k > 0, sa + 4, sb);
-                    mma_step(d0, da + 256, db + (digit_bytes(TPG) >> 5), idesc1, true, sa, sb);
-                    if (has1) mma_step(d1, da + (kURec >> 4) + 256, db + (digit_bytes(TPG) >> 5), idesc1, true, sa + 4, sb);
-                    commit_to(&empty[cur]);
+                    g_copy_scales<CL>(sa, dsf);
+                    if (two) g_copy_scales<CL>(sa + 4, dsf + (kURec >> 4));
+                    const uint64_t dsb = dsf + uint64_t((2 * kURec - 8192 + kBDig) >> 4); // 128 columns' scales per copy
+                    g_copy_scales<CL>(sb, dsb);
+                    if (N > 128) g_copy_scales<CL>(sb + 4, dsb + 32);
+                    g_mma<CL>(d0, da, db, idesc0, k > 0, sa, sb); // the run's first MMA overwrites
+                    if (two) g_mma<CL>(d1, da + (kURec >> 4), db, idesc0, k > 0, sa + 4, sb);
+                    g_mma<CL>(d0, da + 256, db + (kBDig >> 5), idesc1, true, sa, sb);
+                    if (two) g_mma<CL>(d1, da + (kURec >> 4) + 256, db + (kBDig >> 5), idesc1, true, sa + 4, sb);
+                    g_commit<CL>(back);
                 }
                 sfa = (sfa + 1) & (kGSfaBufs - 1);
             }
-            if (ok && one) commit_to(&dfull);
+            if (ok && one) g_commit<CL>(&dfull);
             g += r.len;
         }
-    } else {
+    } else if (warp < 4) {
         // ---- epilogue: tensor-memory lane = row of the tile; digit j of the group's token t = column j * TPG + t ------------
         asm volatile("griddepcontrol.wait;" ::: "memory"); // residual inputs and tickets come from earlier launches
         bool ok = true;
@@ -620,7 +705,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
         for (int run = 0; g < end && ok; run++) {
             const GRun r = run_at(p, g, end);
             g += r.len;
-            const int pair = r.unit / p.ngroups, grp = r.unit - pair * p.ngroups;
+            const int u = r.unit / p.ngroups, grp = r.unit - u * p.ngroups;
             const int ubegin = r.unit * nkb, uend = ubegin + nkb;
             const bool cut = begin > ubegin || uend > end;
             const int c_first = cut ? cta_of_stage(p, ubegin, G) : c, c_last = cut ? cta_of_stage(p, uend - 1, G) : c;
@@ -628,7 +713,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
             // the trips to L2): this CTA adds it to its own, which it need not store.
             if (tid == 0) {
                 int seen = 0;
-                if (c_last == c_first + 1) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(p.tickets + c_first) : "memory");
+                if (c_last == c_first + 1) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(p.tickets + CL * c_first + rank) : "memory");
                 s_early[run & 1] = seen;
             }
             ok = mbar_wait(&dfull, run & 1, abort_flag);
@@ -640,7 +725,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
             }
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const bool has1 = SWIGLU || 2 * pair + 1 < p.total_tiles;
+            const PairSrc q0 = pair_src<CL, SWIGLU>(p, u, rank, 0);
+            const bool has1 = q0.two;
             float y[2][TPG];
             load_sums<TPG>(tmem + (uint32_t(warp * 32) << 16), y[0]);
             if (has1) load_sums<TPG>(tmem + kD1Col + (uint32_t(warp * 32) << 16), y[1]);
@@ -650,10 +736,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(&dempty);
+            if (lane == 0) { // the issuer sits in the first CTA
+                if constexpr (CL == 2) first_arrive(&dempty);
+                else mbar_arrive(&dempty);
+            }
 
             auto fetch = [&](int cc, float4 (&q)[2][TPG / 4]) { // a CTA's part of this unit
-                const float4 *slot = reinterpret_cast<const float4 *>(p.partials + (size_t(cc) * 2 + (share_begin(p, cc, G) > ubegin ? 0 : 1)) * 2 * kSlotFloats) + tid;
+                const float4 *slot = reinterpret_cast<const float4 *>(p.partials + (size_t(CL * cc + rank) * 2 + (share_begin(p, cc, G) > ubegin ? 0 : 1)) * 2 * kSlotFloats) + tid;
 #pragma unroll
                 for (int h = 0; h < 2; h++)
 #pragma unroll
@@ -663,7 +752,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
             if (cut && s_early[run & 1]) {
                 float4 q[2][TPG / 4];
                 fetch(c_first + c_last - c, q);
-                if (tid == 0) p.tickets[c_first] = 0; // ready for the next launch
+                if (tid == 0) p.tickets[CL * c_first + rank] = 0; // ready for the next launch
 #pragma unroll
                 for (int h = 0; h < 2; h++)
 #pragma unroll
@@ -680,7 +769,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     if (h == 1 && !has1) break;
-                    float4 *slot = reinterpret_cast<float4 *>(p.partials + ((size_t(c) * 2 + which) * 2 + h) * kSlotFloats) + tid; // [four tokens][row]
+                    float4 *slot = reinterpret_cast<float4 *>(p.partials + ((size_t(CL * c + rank) * 2 + which) * 2 + h) * kSlotFloats) + tid; // [four tokens][row]
 #pragma unroll
                     for (int t = 0; t < TPG / 4; t++)
                         __stcg(slot + t * 128, make_float4(y[h][4 * t], y[h][4 * t + 1], y[h][4 * t + 2], y[h][4 * t + 3]));
@@ -690,9 +779,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 if (tid == 0) {
                     int seen;
-                    asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(seen) : "l"(p.tickets + c_first) : "memory");
+                    asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(seen) : "l"(p.tickets + CL * c_first + rank) : "memory");
                     s_last = seen == c_last - c_first;
-                    if (s_last) p.tickets[c_first] = 0; // ready for the next launch
+                    if (s_last) p.tickets[CL * c_first + rank] = 0; // ready for the next launch
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 const bool last = s_last != 0;
@@ -717,25 +806,34 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
                 }
             }
             if constexpr (SWIGLU) {
-                const GSeg &s = p.seg[gseg_of(p, pair)];
-                const int row = (pair - s.tile_begin) * 128 + tid;
-                if (row < s.rows) finish_row<TPG>(p, s, row, grp, y[1], y[0]);
+                const GSeg &s = p.seg[gseg_of(p, q0.tile[0])];
+                const int row = (q0.tile[0] - s.tile_begin) * 128 + tid;
+                if (q0.live[0] && row < s.rows) finish_row<TPG, SWIGLU>(p, s, row, grp, y[1], y[0]);
             } else {
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    if (h == 1 && !has1) break;
-                    const int tile = 2 * pair + h;
+#pragma unroll 1
+                for (int h = 0; h < 2; h++) { // one copy of the code for both records
+                    const int tile = h ? q0.tile[1] : q0.tile[0];
                     const GSeg &s = p.seg[gseg_of(p, tile)];
                     const int row = (tile - s.tile_begin) * 128 + tid;
-                    if (row < s.rows) finish_row<TPG>(p, s, row, grp, y[h], y[h]);
+                    if ((h ? q0.live[1] : q0.live[0]) && row < s.rows) finish_row<TPG, SWIGLU>(p, s, row, grp, y[0], y[0]);
+#pragma unroll
+                    for (int t = 0; t < TPG; t++) y[0][t] = y[1][t];
                 }
             }
         }
     }
+    __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if constexpr (CL == 2) { // nobody leaves while the other CTA may still read its shared memory or arrive at its barriers
+        asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kGTmemCols));
+    if (warp == 0) {
+        if constexpr (CL == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kGTmemCols));
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kGTmemCols));
+    }
     if (tid == 0 && s_abort && p.error_flag) *p.error_flag = 1;
 }
 
@@ -744,13 +842,14 @@ namespace {
 std::mutex g_gemm_attr_mutex;
 bool g_gemm_attr_done[64] = {false}; // the shared-memory opt-in is a per-device function attribute
 
-// Tokens per group.  32 take fewer bytes into shared memory than 16 for every count beyond 48, the last group's padding included.  Up to
-// 48 the weights bound the time and every CTA ends on a cut unit, whose parts 32 tokens make twice as large and whose ring is shorter.
-// 16 / 32 a group, microseconds replayed:  24576 x 4096   4096 x 12288   12352 x 4096   4096 x 4096
-//   33..48 tokens                           26.2 / 25.9    22.0 / 27.3    19.1 / 22.3   15.6 / 23.0
-//   49..64                                  32.0 / 26.4    25.3 / 26.1    22.5 / 22.5   16.8 / 22.6    (a layer's four: even)
-//   65..72                                  37.1 / 31.4    28.1 / 27.4    25.7 / 22.7   18.2 / 18.8
-//   512                                      167 / 123      104 / 78        93 / 68       42 / 34
+// Tokens per group, with 32 on pairs of CTAs.  32 take fewer bytes into shared memory than 16 for every count beyond 48, the last group's
+// padding included.  Up to 48 the weights bound the time and every CTA ends on a cut unit, whose parts 32 tokens make twice as large and
+// whose ring is shorter.  16 / 32 a group, microseconds replayed (in brackets 32 with one CTA a unit):
+//                  24576 x 4096         4096 x 12288        12352 x 4096        4096 x 4096
+//   33..48 tokens  26.2 / 26.5          22.0 / 24.8         19.1 / 23.0         15.6 / 18.5
+//   49..64         32.0 / 26.5 (26.4)   25.3 / 24.8 (26.1)  22.5 / 23.0 (22.5)  16.8 / 18.5 (22.6)    (a layer's four: even)
+//   65..96         37.1 / 31.5 (31.7)   28.1 / 26.7 (27.4)  25.7 / 21.8 (22.9)  18.2 / 18.2 (18.7)
+//   512             167 / 121 (126)      104 / 74 (77.5)      93 / 67 (69)        42 / 33 (34.3)
 int tokens_per_group(int tokens) { return tokens <= 48 ? 16 : 32; }
 size_t image_bytes(int cols, int tokens)
 {
@@ -824,11 +923,12 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
         g.tile_begin = tiles; tiles += (s.rows + 127) >> 7; g.epilogue = s.epilogue; g.rows = s.rows;
     }
     p.total_tiles = tiles;
-    const long long total = (long long)(nmat_all == 2 ? tiles : (tiles + 1) / 2) * ngroups * nkb; // a unit = (pair of records, token group)
+    const int cl = group_ctas(tpg), per_unit = (nmat_all == 2 ? 1 : 2) * cl; // a unit = (row tiles of cl CTAs, token group)
+    const long long total = (long long)((tiles + per_unit - 1) / per_unit) * ngroups * nkb;
     if (total > (1ll << 30)) return fail(INSG_E_LIMIT, "gemm: more than 2^30 (tile, group, k-block) stages");
     p.total_stages = int(total);
     p.error_flag = op->error_flag;
-    const int stage_bytes = 2 * kURec + digit_block(tpg);
+    const int stage_bytes = 2 * kURec + digit_block(tpg) - digit_bytes(tpg) + digit_bytes(tpg) / cl;
     p.stages = std::min(kGMaxStages, 224 * 1024 / stage_bytes);
     const size_t smem = size_t(p.stages) * stage_bytes;
     auto kernel = tpg == 16 ? (nmat_all == 2 ? umma_gemm_kernel<16, true> : umma_gemm_kernel<16, false>)
@@ -854,11 +954,26 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     // so that a unit is cut into about sqrt(nkb) parts of sqrt(nkb) stages at most.
     int least = 1;
     while (least * least < nkb) least++;
-    const int grid = std::max(1, std::min({sm_count(), kGMaxGrid, p.total_stages, std::max(1, p.total_stages / least)}));
+    const int grid = std::max(1, std::min({sm_count() / cl, kGMaxGrid / cl, p.total_stages, std::max(1, p.total_stages / least)})); // of cl CTAs
     p.share = p.total_stages / grid;
     p.share_rem = p.total_stages % grid;
-    rc = launch(kernel, dim3(grid), dim3(kGemmThreads), smem, st, true, p); // may start while the digits are being written
-    if (rc != INSG_OK) return rc;
+    {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(unsigned(grid * cl));
+        cfg.blockDim = dim3(kGemmThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; // may start while the digits are being written
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = unsigned(cl);
+        attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = cl > 1 ? 2 : 1;
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
+        if (e != cudaSuccess) return cuda_fail(e, "umma gemm launch");
+    }
     for (int i = 0; i < op->n_segments; i++) {
         const insg_gemv_segment &s = op->seg[i];
         if (s.epilogue == INSG_EPI_CONV_SILU && s.conv_token_stride == 0) { // one sequence: the history runs through the tokens
