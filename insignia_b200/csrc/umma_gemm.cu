@@ -170,7 +170,7 @@ struct DigitizeParams {
 // alone, sixteen-warp CTAs of a token with eight base-9 digits -> this with four k-blocks on their way -> with two (less code to run through):
 //   4096 columns, 16 tokens 2.63 -> 2.64 -> 2.43 us (gated norm 3.93 -> 2.92 -> 2.74), 128: 4.12 -> 4.46 -> 4.30, 512: 10.3 -> 9.7 -> 9.2
 //   12288 columns, 16 tokens 3.43 -> 3.20 -> 3.01 us, 128: 7.67 -> 7.96 -> 7.64, 512: 21.0 -> 23.8 -> 22.0
-template <int TPG>
+template <int TPG, int PRO>
 __global__ void __launch_bounds__(kDigThreads, 4) umma_digitize_kernel(const __grid_constant__ DigitizeParams p)
 {
     constexpr int kBatch = 2, kWarps = kDigThreads / 32;
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kDigThreads, 4) umma_digitize_kernel(const __g
     const int m = blockIdx.x / p.parts, part = blockIdx.x - m * p.parts, grp = m / TPG, ms = m - grp * TPG;
     const ProIn &o = p.pro;
     const int nkb = o.cols >> 7, per = (nkb + p.parts - 1) / p.parts, kb0 = part * per, kb1 = min(nkb, kb0 + per);
-    const bool live = m < p.tokens, rms = o.prologue == INSG_PRO_RMSNORM;
+    const bool live = m < p.tokens, rms = PRO == INSG_PRO_RMSNORM;
     const float *in = o.in + size_t(m) * o.cols + lane * 4;
     uint2 w[kBatch]; // the norm's weights are parameters: asked for before the wait
     auto load_weights = [&](int b0) {
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(kDigThreads, 4) umma_digitize_kernel(const __g
         for (int j = 0; j < kBatch; j++) {
             const int kb = b0 + j * kWarps;
             if (rms && kb < kb1) w[j] = *reinterpret_cast<const uint2 *>(o.norm_w + kb * 128 + lane * 4);
-            else if (o.prologue == INSG_PRO_GATED_RMSNORM) w[j] = *reinterpret_cast<const uint2 *>(o.norm_w + lane * 4);
+            else if (PRO == INSG_PRO_GATED_RMSNORM) w[j] = *reinterpret_cast<const uint2 *>(o.norm_w + lane * 4);
         }
     };
     load_weights(kb0 + warp);
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kDigThreads, 4) umma_digitize_kernel(const __g
             if (!live || kb >= kb1) continue;
             x[j] = __ldcg(reinterpret_cast<const float4 *>(in + size_t(kb) * 128));
             const float *gate = o.aux + size_t(m) * 2 * o.cols + (k >> 8) * 512 + 256; // interleaved [head][query 256 | gate 256]
-            switch (o.prologue) {
+            switch (PRO) {
             case INSG_PRO_GATED_RMSNORM:
             case INSG_PRO_SIGMOID_GATE: a[j] = __ldcg(reinterpret_cast<const float4 *>(o.aux + size_t(m) * o.cols + k)); break;
             case INSG_PRO_SIGMOID_GATE_HEAD0: a[j].x = __ldcg(gate); break;
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(kDigThreads, 4) umma_digitize_kernel(const __g
                     v.z = v.z * f * bf16_bits_to_float(w[j].y & 0xffff);
                     v.w = v.w * f * bf16_bits_to_float(w[j].y >> 16);
                 };
-                switch (o.prologue) {
+                switch (PRO) {
                 case INSG_PRO_RMSNORM: weigh(inv_rms); break;
                 case INSG_PRO_GATED_RMSNORM: { // a head is one k-block
                     const float hs = warp_sum(fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w))));
@@ -857,6 +857,18 @@ size_t image_bytes(int cols, int tokens)
     const size_t groups = size_t(tokens + tpg - 1) / tpg;
     return size_t(cols >> 7) * groups * digit_block(tpg);
 }
+// One kernel per prologue: a launch of some ten microseconds runs through little code.
+template <int TPG> auto digitize_kernel(int prologue)
+{
+    switch (prologue) {
+    case INSG_PRO_RMSNORM: return umma_digitize_kernel<TPG, INSG_PRO_RMSNORM>;
+    case INSG_PRO_GATED_RMSNORM: return umma_digitize_kernel<TPG, INSG_PRO_GATED_RMSNORM>;
+    case INSG_PRO_SIGMOID_GATE: return umma_digitize_kernel<TPG, INSG_PRO_SIGMOID_GATE>;
+    case INSG_PRO_SIGMOID_GATE_HEAD0: return umma_digitize_kernel<TPG, INSG_PRO_SIGMOID_GATE_HEAD0>;
+    case INSG_PRO_SIGMOID_GATE_QPROJ: return umma_digitize_kernel<TPG, INSG_PRO_SIGMOID_GATE_QPROJ>;
+    default: return umma_digitize_kernel<TPG, INSG_PRO_PLAIN>;
+    }
+}
 constexpr size_t kPartialBytes = size_t(kGMaxGrid) * 2 * 2 * kSlotFloats * sizeof(float); // [CTA][cut unit][record of the pair]
 } // namespace
 
@@ -948,7 +960,7 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     }
     // the GEMM is the digitize kernel's programmatic dependent: it allocates tensor memory and requests its first weight
     // records while the digits are being written
-    int rc = launch(tpg == 16 ? umma_digitize_kernel<16> : umma_digitize_kernel<32>, dim3(ngroups * tpg * d.parts), dim3(kDigThreads), 0, st, op->pdl != 0, d);
+    int rc = launch(tpg == 16 ? digitize_kernel<16>(op->prologue) : digitize_kernel<32>(op->prologue), dim3(ngroups * tpg * d.parts), dim3(kDigThreads), 0, st, op->pdl != 0, d);
     if (rc != INSG_OK) return rc;
     // Every part of a cut unit costs the CTA that adds them a trip to L2, about what a stage takes: few stages go to fewer CTAs,
     // so that a unit is cut into about sqrt(nkb) parts of sqrt(nkb) stages at most.
