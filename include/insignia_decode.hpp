@@ -38,7 +38,7 @@ struct DecodeOptions {
                                    // tile-layout copy for every pass size).  With `persistent` they stay on the mma.sync
                                    // kernel, whose producers leave the next product's input ready as fp16 pieces.
                                    // false: the mma.sync kernel, every product preparing its own input
-    bool prefill_tcgen05 = true;   // prompts: passes of up to 512 tokens through the tcgen05 GEMM (16 or 32 tokens per
+    bool prefill_tcgen05 = true;   // prompts: passes of up to 1024 tokens through the tcgen05 GEMM (16 or 32 tokens per
                                    // instruction); false: passes of eight (tcgen05) or four (mma.sync) tokens
     int n_layers = Qwen35Shape::layers;
     int vocab = Qwen35Shape::vocab;
@@ -68,7 +68,7 @@ public:
     int *d_next{};       // device: arg-max of the last logits
     void *attn_scratch{};
     void *argmax_scratch{};
-    float *multi{};      // device: activations of up to 512 consecutive tokens (forward_tokens)
+    float *multi{};      // device: activations of up to 1024 consecutive tokens (forward_tokens)
     void *umma_scratch{}; // device: digit image of the activations for the tcgen05 kernel (forward_tokens)
     size_t umma_scratch_bytes{};
     void *prep{};        // device: prepared inputs of products and sums of squares (digit images of up to eight tokens on tcgen05, the
@@ -88,7 +88,7 @@ public:
     void layer(int layer);
     int decode_token(int token);
     void forward_token(int token);
-    // Additive: forward_token for `count` consecutive tokens (a prompt), in passes of up to 512 over the weights; leaves the
+    // Additive: forward_token for `count` consecutive tokens (a prompt), in passes of up to 1024 over the weights; leaves the
     // state the loop would (to fp32 rounding), and the logits and arg-max of the last token.
     void forward_tokens(const int *tokens, int count);
     int logits_argmax();

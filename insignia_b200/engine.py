@@ -60,7 +60,7 @@ class Engine:
         check(_lib.lib().insg_engine_forward_token(self._h, token))
 
     def forward_tokens(self, tokens):
-        """``forward_token`` over a list of consecutive tokens (a prompt), in passes of up to 512 over the weights."""
+        """``forward_token`` over a list of consecutive tokens (a prompt), in passes of up to 1024 over the weights."""
         arr = (C.c_int * len(tokens))(*[int(t) for t in tokens])
         check(_lib.lib().insg_engine_forward_tokens(self._h, arr, len(tokens)))
 
