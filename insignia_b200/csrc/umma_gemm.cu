@@ -842,21 +842,25 @@ namespace {
 std::mutex g_gemm_attr_mutex;
 bool g_gemm_attr_done[64] = {false}; // the shared-memory opt-in is a per-device function attribute
 
-// Tokens per group, with 32 on pairs of CTAs.  32 take fewer bytes into shared memory than 16 for every count beyond 48, the last group's
-// padding included.  Up to 48 the weights bound the time and every CTA ends on a cut unit, whose parts 32 tokens make twice as large and
-// whose ring is shorter.  16 / 32 a group, microseconds replayed (in brackets 32 with one CTA a unit):
-//                  24576 x 4096         4096 x 12288        12352 x 4096        4096 x 4096
-//   33..48 tokens  26.2 / 26.5          22.0 / 24.8         19.1 / 23.0         15.6 / 18.5
-//   49..64         32.0 / 26.5 (26.4)   25.3 / 24.8 (26.1)  22.5 / 23.0 (22.5)  16.8 / 18.5 (22.6)    (a layer's four: even)
-//   65..96         37.1 / 31.5 (31.7)   28.1 / 26.7 (27.4)  25.7 / 21.8 (22.9)  18.2 / 18.2 (18.7)
-//   512             167 / 121 (126)      104 / 74 (77.5)      93 / 67 (69)        42 / 33 (34.3)
-int tokens_per_group(int tokens) { return tokens <= 48 ? 16 : 32; }
-size_t image_bytes(int cols, int tokens)
+// Tokens per group, 32 of them on pairs of CTAs.  32 take fewer bytes into shared memory for every count beyond 48, the last group's padding
+// included.  Where an SM has few stages, every CTA works on parts of cut units and what these cost is the time: 16 tokens make them half as
+// large, and up to 48 tokens the weights bound it.  Microseconds replayed with 16 / 32 a group, in brackets the stages an SM has with 16:
+//                  24576 x 4096      4096 x 12288      12352 x 4096      10240 x 4096      8192 x 4096       4096 x 4096
+//   49..64 tokens  32.7 / 26.4 (83)  24.6 / 24.8 (42)  22.4 / 22.6 (42)  19.1 / 20.7 (35)  18.7 / 19.4 (28)  15.9 / 19.9 (14)
+//   65..80         38.1 / 31.3 (104) 27.7 / 26.5 (52)  25.1 / 21.6 (53)  21.3 / 23.1 (43)  19.1 / 20.8 (35)  16.6 / 17.6 (17)
+//   96                                                                   24.1 / 23.1 (52)  21.0 / 21.1 (42)  17.5 / 18.4 (21)
+//   128                                                                  28.5 / 23.7 (69)  24.7 / 23.2 (55)  19.8 / 19.8 (28)
+//   192                                                                                                      22.0 / 22.2 (42)
+//   256                                                                                                      25.7 / 24.2 (55)
+constexpr int kFewStages = 44;
+int tokens_per_group(int tokens, long long stages16) { return tokens <= 48 || stages16 <= (long long)kFewStages * sm_count() ? 16 : 32; }
+size_t image_bytes(int cols, int tokens) // room for either: groups of 32 take as many bytes as groups of 16 or more
 {
-    const int tpg = tokens_per_group(tokens);
+    const int tpg = tokens <= 48 ? 16 : 32;
     const size_t groups = size_t(tokens + tpg - 1) / tpg;
     return size_t(cols >> 7) * groups * digit_block(tpg);
 }
+static_assert(2 * digit_block(16) <= digit_block(32), "a group of 32 has room for two of 16");
 // One kernel per prologue: a launch of some ten microseconds runs through little code.
 template <int TPG> auto digitize_kernel(int prologue)
 {
@@ -895,26 +899,7 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     const size_t need = umma_gemm_scratch(op->cols, tokens);
     if (!op->umma_scratch || op->umma_scratch_bytes < need) return fail(INSG_E_ARG, "gemm: scratch missing or too small (insg_umma_gemm_scratch_bytes)");
     if (reinterpret_cast<uintptr_t>(op->umma_scratch) & 255) return fail(INSG_E_ARG, "gemm: scratch must be 256-byte aligned");
-    const int tpg = tokens_per_group(tokens);
-    const int ngroups = (tokens + tpg - 1) / tpg, nkb = op->cols >> 7;
-
-    DigitizeParams d = {};
-    d.pro = ProIn{op->in, op->aux, op->norm_w, nullptr, op->cols, op->prologue};
-    d.bimg = static_cast<uint8_t *>(op->umma_scratch);
-    d.tokens = tokens;
-    d.ngroups = ngroups;
-    // up to four CTAs per SM, a k-block for every warp of theirs at least
-    d.parts = std::max(1, std::min(nkb / (kDigThreads / 32), 4 * sm_count() / (ngroups * tpg)));
-
     GParams p = {};
-    p.bimg = d.bimg;
-    p.partials = reinterpret_cast<float *>(d.bimg + image_bytes(op->cols, tokens));
-    p.tickets = reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(p.partials) + kPartialBytes);
-    d.tickets = p.tickets;
-    p.nkb = nkb;
-    p.nseg = op->n_segments;
-    p.ngroups = ngroups;
-    p.tokens = tokens;
     int tiles = 0, nmat_all = 0;
     for (int i = 0; i < op->n_segments; i++) {
         const insg_gemv_segment &s = op->seg[i];
@@ -934,6 +919,26 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
         nmat_all = nmat;
         g.tile_begin = tiles; tiles += (s.rows + 127) >> 7; g.epilogue = s.epilogue; g.rows = s.rows;
     }
+    const int nkb = op->cols >> 7;
+    const int tpg = tokens_per_group(tokens, (long long)(nmat_all == 2 ? tiles : (tiles + 1) / 2) * ((tokens + 15) / 16) * nkb);
+    const int ngroups = (tokens + tpg - 1) / tpg;
+
+    DigitizeParams d = {};
+    d.pro = ProIn{op->in, op->aux, op->norm_w, nullptr, op->cols, op->prologue};
+    d.bimg = static_cast<uint8_t *>(op->umma_scratch);
+    d.tokens = tokens;
+    d.ngroups = ngroups;
+    // up to four CTAs per SM, a k-block for every warp of theirs at least
+    d.parts = std::max(1, std::min(nkb / (kDigThreads / 32), 4 * sm_count() / (ngroups * tpg)));
+
+    p.bimg = d.bimg;
+    p.partials = reinterpret_cast<float *>(d.bimg + image_bytes(op->cols, tokens));
+    p.tickets = reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(p.partials) + kPartialBytes);
+    d.tickets = p.tickets;
+    p.nkb = nkb;
+    p.nseg = op->n_segments;
+    p.ngroups = ngroups;
+    p.tokens = tokens;
     p.total_tiles = tiles;
     const int cl = group_ctas(tpg), per_unit = (nmat_all == 2 ? 1 : 2) * cl; // a unit = (row tiles of cl CTAs, token group)
     const long long total = (long long)((tiles + per_unit - 1) / per_unit) * ngroups * nkb;

@@ -1,4 +1,4 @@
-"""Products of more than 48 tokens run on pairs of CTAs that multiply four row tiles with one set of digits."""
+"""Products with many stages run on pairs of CTAs that multiply four row tiles with one set of digits, those with few in groups of 16 tokens."""
 import os
 import sys
 
@@ -13,10 +13,12 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
-# rows: one to nine tiles (the last four of a pair of CTAs: one, two, three or all there), a ragged last tile; cols: one k-block, an odd
-# number of them; tokens: the first count of the form, a full and a just begun group, sixteen groups
-@pytest.mark.parametrize("rows,cols,M", [(100, 128, 49), (256, 384, 64), (384, 1152, 65), (500, 512, 96), (640, 4096, 49), (768, 256, 97), (1152, 12288, 64),
-                                         (4096, 128, 512), (19008, 512, 100)])
+# From 44 stages of 16 tokens an SM on (148 SMs: 6512 pairs of tiles x groups of 16 x k-blocks) two CTAs share a group of 32.  One, two, three
+# and five tiles with long sums and many groups; 101 to 104 tiles (the last four one to all there, the very last ragged), odd k-blocks, a full and
+# a just begun last group; then below the line: 16 tokens a group beyond 48 tokens
+@pytest.mark.parametrize("rows,cols,M", [(100, 12288, 1200), (256, 12288, 1090), (384, 12288, 600), (640, 12288, 400), (128 * 101, 4224, 49), (128 * 102, 4096, 64),
+                                         (128 * 103 - 28, 4224, 65), (128 * 104, 4096, 96), (128 * 150, 2176, 100),
+                                         (100, 128, 49), (640, 4096, 61), (1152, 1152, 97), (4096, 128, 512)])
 def test_pairs_vs_oracle(cuda, rows, cols, M):
     from insignia_b200 import ops
 
@@ -32,17 +34,17 @@ def test_pairs_vs_oracle(cuda, rows, cols, M):
 
 
 # SwiGLU: a unit is the gate and up tiles of two times 128 rows; an odd number of row tiles leaves the second CTA without
-@pytest.mark.parametrize("rows,M", [(128, 49), (300, 64), (640, 70)])
-def test_pairs_swiglu(cuda, rows, M):
+@pytest.mark.parametrize("rows,cols,M", [(128, 12288, 1100), (300, 4096, 1100), (640, 4096, 700), (640, 1024, 70)])
+def test_pairs_swiglu(cuda, rows, cols, M):
     from insignia_b200 import ops
 
     rng = np.random.default_rng(rows + M)
-    mats = [rand_matrix(rng, rows, 1024) for _ in range(2)]
-    x = rng.standard_normal((M, 1024)).astype(np.float32)
+    mats = [rand_matrix(rng, rows, cols) for _ in range(2)]
+    x = rng.standard_normal((M, cols)).astype(np.float32)
     g, u = (ops.repack_umma(dev(w), dev(s)) for w, s in mats)
     out = torch.zeros(M, rows, device="cuda")
-    ops.gemv_fused(dev(x), [dict(packed=g, packed2=u, out=out, rows=rows, epilogue="swiglu")], layout=1, tokens=M, cols=1024,
-                   umma_scratch=ops.umma_gemm_scratch(1024, M))
+    ops.gemv_fused(dev(x), [dict(packed=g, packed2=u, out=out, rows=rows, epilogue="swiglu")], layout=1, tokens=M, cols=cols,
+                   umma_scratch=ops.umma_gemm_scratch(cols, M))
     for m in (0, 31, 32, M - 1):
         a, b = (orc.gemv_mlx_f64(w, s, x[m]) for w, s in mats)
         want = a / (1 + np.exp(-a)) * b
