@@ -159,13 +159,16 @@ template <int T> __device__ __forceinline__ void load_partial(uint32_t taddr, fl
 // half an SM (24576 x 4096 as SwiGLU 14.3 -> 13.3 us in the chain); one matrix keeps two (one: 9.7 -> 10.7 us at 12352 x 4096).
 template <int T> __host__ __device__ constexpr int unit_slots(int nmat) { return T == 1 ? 4 : T == 8 ? 3 - nmat : 2; }
 
-// What a variant of the kernel has beside its tokens: a prepared input in place of the prologue, the logits' arg-max, digits that come with
-// the weights.  A token is 129 launches of some seven microseconds, and instructions that a launch runs through for the first time come
-// from L2 behind the stream of weights: as one kernel with everything in it (96 KB of code for one token, 125 for eight; prepared variants
-// 41 and 53) a token took 1084 us, three sequences 1308, eight 1503 and a speculative pass 1500; as variants, with the waits' loops
-// not unrolled and one store and one copy of the digits' code behind all epilogues, 1057, 1208, 1412 and 1428.  (20 KB more in the
-// issuer's loop, never run, cost a token 80 us.)
-constexpr int kDPrepared = 1, kDLogits = 2, kDStreamed = 4;
+// What a variant of the kernel has beside its tokens: a prepared input in place of the prologue, the logits' arg-max, two matrices (SwiGLU), one
+// segment that adds into the residual stream; that with digits that come with the weights, or behind the gated norm.  A token is 129 launches of some
+// seven microseconds, and instructions that a launch runs through for the first time come from L2 behind the stream of weights.  Microseconds of a
+// token, a step of three sequences, of eight, and a speculative pass (a process is now and then 2 % off all of its life):
+//   one kernel with everything in it (96 KB of code for one token, 125 for eight)              1084 1308 1503 1500
+//   variants with a prepared input and with the arg-max, the waits' loops not unrolled,
+//   one store and one copy of the digits' code behind all epilogues (41 and 53 KB)             1057 1208 1412 1428
+//   and with two matrices, the gated norm, one segment where digits come with the weights      1040 1187 1380 1407
+// (20 KB more in the issuer's loop, never run, cost a token 80 us.)
+constexpr int kDPrepared = 1, kDLogits = 2, kDStreamed = 4, kDGated = 8, kDTwo = 16, kDResidual = 32;
 
 template <int T, int F>
 __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_constant__ DParams p)
@@ -174,6 +177,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     constexpr int kBKb = 512 * T;       // digit bytes per k-block
     constexpr int kImg = kBKb + 512;    // a k-block of the image: digits, then their scale block
     constexpr bool prepared = (F & kDPrepared) != 0, logits = (F & kDLogits) != 0, streamed = (F & kDStreamed) != 0;
+    const int pro = (F & kDGated) != 0 ? int(INSG_PRO_GATED_RMSNORM) : p.prologue;
     constexpr int kStage = kDStage + (streamed ? 2 * kImg : 0); // streamed: one unit a cluster, so that its digits come with the weights they multiply
     static_assert(!streamed || prepared, "a streamed image is a prepared one");
     constexpr int N = kDDigits * T;
@@ -189,7 +193,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
 
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int rank = int(blockIdx.x) & (kDCl - 1), cl = int(blockIdx.x) / kDCl, C = int(gridDim.x) / kDCl;
-    const int nkb = p.nkb, S = p.stages, nmat = p.nmat, XU = unit_slots<T>(nmat);
+    const int nkb = p.nkb, S = p.stages, nmat = (F & kDTwo) != 0 ? 2 : prepared || (F & kDGated) != 0 ? 1 : p.nmat, XU = unit_slots<T>(nmat);
     const int kb0 = (nkb * rank) >> 2, len = ((nkb * (rank + 1)) >> 2) - kb0; // this CTA's k-blocks
     const int spt = (len + 1) >> 1;                                            // ring stages per (tile, matrix)
     const int nun = cl < p.units ? (p.units - cl + C - 1) / C : 0;             // units of this cluster: cl, cl + C, ...
@@ -199,10 +203,12 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     float *xslot = reinterpret_cast<float *>(bimg + (streamed ? 0 : size_t((nkb + 3) >> 2) * kImg)); // XU * nmat exchange slots
     float *s_ssq = T < 8 ? s_ssq_static : xslot + XU * nmat * kSlot; // [token][k-block], unless the input is prepared
 
+    constexpr bool residual = (F & (kDResidual | kDStreamed | kDGated)) != 0, single = residual; // one segment, added into the residual stream
+    auto seg_of = [&](int unit) -> const DSeg & { return p.seg[single ? 0 : dseg_of(p, unit)]; };
     // ---- the weight stream starts first: it depends on nothing ----------------------------------------------------------
     auto run_src = [&](int run) -> const uint8_t * { // this CTA's records of the run (tile, matrix)
         const int unit = cl + (nmat == 2 ? run >> 1 : run) * C;
-        const DSeg &s = p.seg[dseg_of(p, unit)];
+        const DSeg &s = seg_of(unit);
         return (nmat == 2 && (run & 1) ? s.packed2 : s.packed) + (size_t(unit - s.tile_begin) * nkb + kb0) * kURec;
     };
     auto load_stage = [&](int slot, const uint8_t *src, int st) { // stage st of a run: two records, or the last one of an odd count
@@ -262,9 +268,9 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         if (warp >= 4 && warp < 8) pdl_wait(); // they read what earlier launches wrote
     } else if (warp < 8) {
         // ---- activation prologue: this CTA's quarter of the columns ---------------------------------------------------------
-        constexpr int kBatch = 3;
+        constexpr int kBatch = (F & kDGated) != 0 ? 1 : 3;
         const int items = len * T; // (token, k-block) pairs, dealt to the eight warps
-        const bool rms = p.prologue == INSG_PRO_RMSNORM;
+        const bool rms = pro == INSG_PRO_RMSNORM;
         float4 x[kBatch], a[kBatch];
         uint2 w[kBatch];
         auto place = [&](int it, int &m, int &kb) { m = T == 1 ? 0 : it / len; kb = T == 1 ? it : it - m * len; };
@@ -276,7 +282,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 w[j] = make_uint2(0u, 0u);
                 if (b0 + 8 * j < items) {
                     if (rms) w[j] = reinterpret_cast<const uint2 *>(p.norm_w)[(kb0 + kb) * 32 + lane];
-                    else if (p.prologue == INSG_PRO_GATED_RMSNORM) w[j] = reinterpret_cast<const uint2 *>(p.norm_w)[lane];
+                    else if (pro == INSG_PRO_GATED_RMSNORM) w[j] = reinterpret_cast<const uint2 *>(p.norm_w)[lane];
                 }
             }
         };
@@ -292,7 +298,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 if (b0 + 8 * j < items && m < p.tokens) {
                     const int k = (kb0 + kb) * 128 + lane * 4;
                     x[j] = __ldcg(reinterpret_cast<const float4 *>(p.in + size_t(m) * p.cols + k));
-                    switch (p.prologue) {
+                    switch (pro) {
                     case INSG_PRO_GATED_RMSNORM:
                     case INSG_PRO_SIGMOID_GATE: a[j] = __ldcg(reinterpret_cast<const float4 *>(p.aux + size_t(m) * p.cols + k)); break;
                     case INSG_PRO_SIGMOID_GATE_HEAD0: a[j].x = __ldcg(p.aux + size_t(m) * 2 * p.cols + (k >> 8) * 512 + 256); break;
@@ -309,7 +315,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 int m, kb;
                 place(b0 + 8 * j, m, kb);
                 float4 v = x[j];
-                switch (p.prologue) {
+                switch (pro) {
                 case INSG_PRO_RMSNORM: { // the factor 1/rms is one number per token: the epilogue applies it
                     const float ss = warp_sum(fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w))));
                     if (lane == 0) s_ssq[m * kDMaxKb + kb] = ss;
@@ -339,7 +345,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 }
                 default: break;
                 }
-                if (p.x_out && cl == 0 && !rms && m < p.tokens)
+                if (!(F & kDGated) && p.x_out && cl == 0 && !rms && m < p.tokens)
                     reinterpret_cast<float4 *>(p.x_out + size_t(m) * p.cols)[(kb0 + kb) * 32 + lane] = v;
                 store_digits(v, T, m, bimg + size_t(kb) * kImg, s_lut, lane);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // the tensor core reads the image through the async proxy
@@ -529,13 +535,13 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
 #pragma unroll 4
                     for (int i = lane; i < groups; i += 32) ss += __ldcg(p.prep_partials + t * groups + i);
                 sc = rsqrtf(warp_sum(ss) / float(p.cols) + 1e-6f);
-            } else if (p.prologue == INSG_PRO_RMSNORM) {
+            } else if (pro == INSG_PRO_RMSNORM) {
                 sc = rsqrtf((s_rss[t] + s_rss[T + t] + s_rss[2 * T + t] + s_rss[3 * T + t]) / float(p.cols) + 1e-6f);
             }
             if (lane == 0) s_scale[t] = sc;
         }
         asm volatile("bar.sync 3, 128;" ::: "memory");
-        if (!prepared && ok && p.x_out && cl == 0 && p.prologue == INSG_PRO_RMSNORM)
+        if (!prepared && ok && p.x_out && cl == 0 && pro == INSG_PRO_RMSNORM)
 #pragma unroll 1
             for (int m = 0; m < p.tokens; m++)
 #pragma unroll 1
@@ -550,15 +556,15 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         } next;
         auto fetch = [&](int i) {
             const int unit = cl + i * C;
-            const DSeg &s = p.seg[dseg_of(p, unit)];
+            const DSeg &s = seg_of(unit);
             const int row = (unit - s.tile_begin) * 128 + rank * 32 + lane;
-            if (row >= s.rows) return;
-            if (s.epilogue == INSG_EPI_CONV_SILU) next.w = reinterpret_cast<const uint2 *>(s.conv_w)[row];
+            if ((F & kDTwo) != 0 || row >= s.rows) return;
+            if (!residual && s.epilogue == INSG_EPI_CONV_SILU) next.w = reinterpret_cast<const uint2 *>(s.conv_w)[row];
 #pragma unroll
             for (int u = 0; u < TN; u++) {
                 const int t = t0 + u;
                 if (t >= p.tokens) break;
-                if (s.epilogue == INSG_EPI_RESIDUAL) {
+                if (residual || s.epilogue == INSG_EPI_RESIDUAL) {
                     next.h[u][0] = __ldcg(s.out + row + t * size_t(s.rows));
                 } else if (s.epilogue == INSG_EPI_CONV_SILU) {
                     const float *hist = s.conv_state + t * s.conv_stride + size_t(row) * 3;
@@ -574,7 +580,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
 #pragma unroll 1
         for (int i = group; i < nun && ok; i += kGroups) {
             const int unit = cl + i * C;
-            const DSeg &s = p.seg[dseg_of(p, unit)];
+            const DSeg &s = seg_of(unit);
             const int row = (unit - s.tile_begin) * 128 + rank * 32 + lane;
             const bool on = row < s.rows;
             const size_t ld = size_t(s.rows);
@@ -603,7 +609,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 };
 #pragma unroll
                 for (int u = 0; u < TN; u++) y[mat][u] = sum(t0 + u);
-                if (T > 1 && one_history && s.epilogue == INSG_EPI_CONV_SILU) { // the history runs through the tokens: one warp takes them in order
+                if (T > 1 && !(F & kDTwo) && !residual && one_history && s.epilogue == INSG_EPI_CONV_SILU) { // the history runs through the tokens: one warp takes them in order
                     if (t0 == 0 && on) {
                         float h0 = f.h[0][0], h1 = f.h[0][1], h2 = f.h[0][2];
 #pragma unroll 1
@@ -633,9 +639,16 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             } else {
                 // Each epilogue leaves its value in v; one store and one copy of the digits' code serve them all.
                 float v[TN];
-                if (T > 1 && one_history && s.epilogue == INSG_EPI_CONV_SILU) continue; // done above
+                if (T > 1 && !(F & kDTwo) && !residual && one_history && s.epilogue == INSG_EPI_CONV_SILU) continue; // done above
 #pragma unroll
                 for (int u = 0; u < TN; u++) v[u] = y[0][u];
+                if constexpr ((F & kDTwo) != 0) {
+#pragma unroll
+                    for (int u = 0; u < TN; u++) v[u] = fast_silu(y[0][u]) * y[1][u];
+                } else if constexpr (residual) {
+#pragma unroll
+                    for (int u = 0; u < TN; u++) v[u] = f.h[u][0] + y[0][u];
+                } else {
                 switch (s.epilogue) {
                 case INSG_EPI_RESIDUAL:
 #pragma unroll
@@ -663,10 +676,13 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                     }
                     break;
                 case INSG_EPI_SWIGLU:
+                    if constexpr (!prepared) {
 #pragma unroll
-                    for (int u = 0; u < TN; u++) v[u] = fast_silu(y[0][u]) * y[1][u];
+                        for (int u = 0; u < TN; u++) v[u] = fast_silu(y[0][u]) * y[1][u];
+                    }
                     break;
                 default: break;
+                }
                 }
 #pragma unroll
                 for (int u = 0; u < TN; u++) {
@@ -784,8 +800,8 @@ int device_clusters(int *out)
     if (dev < 0 || dev >= 64) return fail(INSG_E_LIMIT, "gemv: device ordinal beyond 63");
     std::lock_guard<std::mutex> lock(g_attr_mutex);
     if (!g_max_clusters[dev]) {
-        for (auto k : {umma_gemv_kernel<1, 0>, umma_gemv_kernel<1, 1>, umma_gemv_kernel<1, 2>, umma_gemv_kernel<1, 3>, umma_gemv_kernel<2, 0>, umma_gemv_kernel<2, 1>,
-                       umma_gemv_kernel<4, 0>, umma_gemv_kernel<4, 1>, umma_gemv_kernel<4, 5>, umma_gemv_kernel<8, 0>, umma_gemv_kernel<8, 1>, umma_gemv_kernel<8, 5>}) {
+        for (auto k : {umma_gemv_kernel<1, 0>, umma_gemv_kernel<1, 1>, umma_gemv_kernel<1, 17>, umma_gemv_kernel<1, 33>, umma_gemv_kernel<1, 2>, umma_gemv_kernel<1, 3>, umma_gemv_kernel<1, 8>, umma_gemv_kernel<2, 0>, umma_gemv_kernel<2, 1>, umma_gemv_kernel<2, 17>, umma_gemv_kernel<2, 33>, umma_gemv_kernel<2, 8>,
+                       umma_gemv_kernel<4, 0>, umma_gemv_kernel<4, 1>, umma_gemv_kernel<4, 17>, umma_gemv_kernel<4, 33>, umma_gemv_kernel<4, 5>, umma_gemv_kernel<8, 0>, umma_gemv_kernel<8, 1>, umma_gemv_kernel<8, 17>, umma_gemv_kernel<8, 33>, umma_gemv_kernel<8, 5>}) {
             e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
             if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(umma gemv)");
         }
@@ -879,7 +895,8 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     // stage, they leave the launch within half an SM where the image (61 KB for three tokens of 12288 columns, 111 for eight) would not,
     // so that it starts beside its predecessor and the next launch beside it: a step of three sequences 1208 -> 1204 us, of eight 1412 -> 1402.
     const bool prep = op->prologue == INSG_PRO_PREPARED;
-    const bool streamed = prep && T >= 4 && p.nmat == 1 && p.units <= clusters && kbq * kblock + exchange + 4 * kDStage > size_t(kDHalfSm);
+    const bool resid = p.nseg == 1 && p.seg[0].epilogue == INSG_EPI_RESIDUAL;
+    const bool streamed = prep && T >= 4 && resid && p.units <= clusters && kbq * kblock + exchange + 4 * kDStage > size_t(kDHalfSm);
     const size_t stage_bytes = kDStage + (streamed ? 2 * kblock : 0);
     const size_t fixed = exchange + (streamed ? 0 : kbq * kblock) + (T == 8 && !prep ? size_t(8) * kDMaxKb * sizeof(float) : 0);
     // ring: no more stages than the launch has, within half an SM when that leaves at least four, else whatever fits.  Four are too
@@ -905,10 +922,11 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = op->pdl ? 2 : 1;
-    auto kernel = T == 1 ? (logits ? (prep ? umma_gemv_kernel<1, 3> : umma_gemv_kernel<1, 2>) : (prep ? umma_gemv_kernel<1, 1> : umma_gemv_kernel<1, 0>))
-                : T == 2 ? (prep ? umma_gemv_kernel<2, 1> : umma_gemv_kernel<2, 0>)
-                : T == 4 ? (streamed ? umma_gemv_kernel<4, 5> : prep ? umma_gemv_kernel<4, 1> : umma_gemv_kernel<4, 0>)
-                         : (streamed ? umma_gemv_kernel<8, 5> : prep ? umma_gemv_kernel<8, 1> : umma_gemv_kernel<8, 0>);
+    const bool gated = op->prologue == INSG_PRO_GATED_RMSNORM && !op->x_out && resid, two = p.nmat == 2;
+    auto kernel = T == 1 ? (logits ? (prep ? umma_gemv_kernel<1, 3> : umma_gemv_kernel<1, 2>) : (prep ? (two ? umma_gemv_kernel<1, 17> : resid ? umma_gemv_kernel<1, 33> : umma_gemv_kernel<1, 1>) : gated ? umma_gemv_kernel<1, 8> : umma_gemv_kernel<1, 0>))
+                : T == 2 ? (prep ? (two ? umma_gemv_kernel<2, 17> : resid ? umma_gemv_kernel<2, 33> : umma_gemv_kernel<2, 1>) : gated ? umma_gemv_kernel<2, 8> : umma_gemv_kernel<2, 0>)
+                : T == 4 ? (streamed ? umma_gemv_kernel<4, 5> : prep ? (two ? umma_gemv_kernel<4, 17> : resid ? umma_gemv_kernel<4, 33> : umma_gemv_kernel<4, 1>) : umma_gemv_kernel<4, 0>)
+                         : (streamed ? umma_gemv_kernel<8, 5> : prep ? (two ? umma_gemv_kernel<8, 17> : resid ? umma_gemv_kernel<8, 33> : umma_gemv_kernel<8, 1>) : umma_gemv_kernel<8, 0>);
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
     return e == cudaSuccess ? INSG_OK : cuda_fail(e, "umma gemv launch");
 }
