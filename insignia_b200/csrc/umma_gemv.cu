@@ -168,7 +168,7 @@ template <int T> __host__ __device__ constexpr int unit_slots(int nmat) { return
 //   one store and one copy of the digits' code behind all epilogues (41 and 53 KB)             1057 1208 1412 1428
 //   and with two matrices, the gated norm, one segment where digits come with the weights      1040 1187 1380 1407
 // (20 KB more in the issuer's loop, never run, cost a token 80 us.)
-constexpr int kDPrepared = 1, kDLogits = 2, kDStreamed = 4, kDGated = 8, kDTwo = 16, kDResidual = 32;
+constexpr int kDPrepared = 1, kDLogits = 2, kDStreamed = 4, kDGated = 8, kDTwo = 16, kDResidual = 32, kDPlain = 64;
 
 template <int T, int F>
 __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_constant__ DParams p)
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
 
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int rank = int(blockIdx.x) & (kDCl - 1), cl = int(blockIdx.x) / kDCl, C = int(gridDim.x) / kDCl;
-    const int nkb = p.nkb, S = p.stages, nmat = (F & kDTwo) != 0 ? 2 : prepared || (F & kDGated) != 0 ? 1 : p.nmat, XU = unit_slots<T>(nmat);
+    const int nkb = p.nkb, S = p.stages, nmat = (F & kDTwo) != 0 ? 2 : (F & (kDResidual | kDStreamed | kDGated | kDPlain)) != 0 ? 1 : p.nmat, XU = unit_slots<T>(nmat);
     const int kb0 = (nkb * rank) >> 2, len = ((nkb * (rank + 1)) >> 2) - kb0; // this CTA's k-blocks
     const int spt = (len + 1) >> 1;                                            // ring stages per (tile, matrix)
     const int nun = cl < p.units ? (p.units - cl + C - 1) / C : 0;             // units of this cluster: cl, cl + C, ...
@@ -203,7 +203,9 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     float *xslot = reinterpret_cast<float *>(bimg + (streamed ? 0 : size_t((nkb + 3) >> 2) * kImg)); // XU * nmat exchange slots
     float *s_ssq = T < 8 ? s_ssq_static : xslot + XU * nmat * kSlot; // [token][k-block], unless the input is prepared
 
-    constexpr bool residual = (F & (kDResidual | kDStreamed | kDGated)) != 0, single = residual; // one segment, added into the residual stream
+    constexpr bool residual = (F & (kDResidual | kDStreamed | kDGated)) != 0, single = residual; // one segment, added into the residual stream, one unit per cluster
+    constexpr bool plain = (F & kDPlain) != 0;                       // nothing is left prepared
+    constexpr bool even = residual || plain || (F & kDTwo) != 0;     // every CTA has an even number of k-blocks
     auto seg_of = [&](int unit) -> const DSeg & { return p.seg[single ? 0 : dseg_of(p, unit)]; };
     // ---- the weight stream starts first: it depends on nothing ----------------------------------------------------------
     auto run_src = [&](int run) -> const uint8_t * { // this CTA's records of the run (tile, matrix)
@@ -474,16 +476,16 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 };
                 constexpr std::true_type yes{};
                 constexpr std::false_type no{};
-                const int even = len & ~1;
-                if (run == 0) {
+                const int evens = len & ~1;
+                if (residual || run == 0) {
 #pragma unroll 1
-                    for (int kb = 0; kb < even && ok; kb += 2) ok = stage(kb, yes, yes);
-                    if (ok && even < len) ok = stage(even, yes, no);
+                    for (int kb = 0; kb < evens && ok; kb += 2) ok = stage(kb, yes, yes);
                 } else {
 #pragma unroll 1
-                    for (int kb = 0; kb < even && ok; kb += 2) ok = stage(kb, no, yes);
-                    if (ok && even < len) ok = stage(even, yes, no); // the digits' scales once more: no copy of the code for a rare case
+                    for (int kb = 0; kb < evens && ok; kb += 2) ok = stage(kb, no, yes);
                 }
+                if constexpr (!even)
+                    if (ok && evens < len) ok = stage(evens, yes, no); // the digits' scales once more: no copy of the code for a rare case
                 if (ok && one) commit_to(&dfull[buf]);
             }
         }
@@ -509,7 +511,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 if (lane == 0) mbar_arrive(&dempty[buf]);
             }
             const int slot = run % nslots;
-            if (run >= nslots) { // the slot's previous content must have been added up by its owner
+            if (!residual && run >= nslots) { // the slot's previous content must have been added up by its owner
                 ok = __all_sync(0xffffffffu, mbar_wait_cluster(&xempty[slot], ((run / nslots) - 1) & 1, abort_flag));
                 if (!ok) break;
             }
@@ -564,7 +566,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             for (int u = 0; u < TN; u++) {
                 const int t = t0 + u;
                 if (t >= p.tokens) break;
-                if (residual || s.epilogue == INSG_EPI_RESIDUAL) {
+                if (residual || (!plain && s.epilogue == INSG_EPI_RESIDUAL)) {
                     next.h[u][0] = __ldcg(s.out + row + t * size_t(s.rows));
                 } else if (s.epilogue == INSG_EPI_CONV_SILU) {
                     const float *hist = s.conv_state + t * s.conv_stride + size_t(row) * 3;
@@ -588,7 +590,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             if (!kAhead) fetch(i);
             const Fetched f = next;
             if (kAhead && i + kGroups < nun) fetch(i + kGroups);
-            const float pw = s.prep_w ? bf16_bits_to_float(s.prep_w[row]) : 1.f; // rows % 128 == 0 where it is set
+            const float pw = !plain && s.prep_w ? bf16_bits_to_float(s.prep_w[row]) : 1.f; // rows % 128 == 0 where it is set
             const float cw0 = bf16_bits_to_float(f.w.x & 0xffff), cw1 = bf16_bits_to_float(f.w.x >> 16);
             const float cw2 = bf16_bits_to_float(f.w.y & 0xffff), cw3 = bf16_bits_to_float(f.w.y >> 16);
             const bool one_history = s.conv_stride == 0; // consecutive tokens of one sequence
@@ -622,7 +624,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                         hist[0] = h0; hist[1] = h1; hist[2] = h2;
                     }
                 }
-                if (i + XU < nun) { // the slot will be used again: tell the four senders
+                if (!residual && i + XU < nun) { // the slot will be used again: tell the four senders
                     __syncwarp();
                     if (lane < kDCl) remote_arrive(map_to_rank(smem_u32(&xempty[slot]), uint32_t(lane)));
                 }
@@ -651,6 +653,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 } else {
                 switch (s.epilogue) {
                 case INSG_EPI_RESIDUAL:
+                    if (plain) break;
 #pragma unroll
                     for (int u = 0; u < TN; u++) v[u] = f.h[u][0] + y[0][u];
                     break;
@@ -676,10 +679,9 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                     }
                     break;
                 case INSG_EPI_SWIGLU:
-                    if constexpr (!prepared) {
+                    if (plain) break;
 #pragma unroll
-                        for (int u = 0; u < TN; u++) v[u] = fast_silu(y[0][u]) * y[1][u];
-                    }
+                    for (int u = 0; u < TN; u++) v[u] = fast_silu(y[0][u]) * y[1][u];
                     break;
                 default: break;
                 }
@@ -688,7 +690,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 for (int u = 0; u < TN; u++) {
                     if (t0 + u >= p.tokens) break;
                     out[(t0 + u) * ld] = v[u];
-                    if (s.prep) leave_digits<T>(s, v[u], pw, row, t0 + u, s_lut, lane);
+                    if (!plain && s.prep) leave_digits<T>(s, v[u], pw, row, t0 + u, s_lut, lane);
                 }
             }
         }
@@ -800,8 +802,8 @@ int device_clusters(int *out)
     if (dev < 0 || dev >= 64) return fail(INSG_E_LIMIT, "gemv: device ordinal beyond 63");
     std::lock_guard<std::mutex> lock(g_attr_mutex);
     if (!g_max_clusters[dev]) {
-        for (auto k : {umma_gemv_kernel<1, 0>, umma_gemv_kernel<1, 1>, umma_gemv_kernel<1, 17>, umma_gemv_kernel<1, 33>, umma_gemv_kernel<1, 2>, umma_gemv_kernel<1, 3>, umma_gemv_kernel<1, 8>, umma_gemv_kernel<2, 0>, umma_gemv_kernel<2, 1>, umma_gemv_kernel<2, 17>, umma_gemv_kernel<2, 33>, umma_gemv_kernel<2, 8>,
-                       umma_gemv_kernel<4, 0>, umma_gemv_kernel<4, 1>, umma_gemv_kernel<4, 17>, umma_gemv_kernel<4, 33>, umma_gemv_kernel<4, 5>, umma_gemv_kernel<8, 0>, umma_gemv_kernel<8, 1>, umma_gemv_kernel<8, 17>, umma_gemv_kernel<8, 33>, umma_gemv_kernel<8, 5>}) {
+        for (auto k : {umma_gemv_kernel<1, 0>, umma_gemv_kernel<1, 1>, umma_gemv_kernel<1, 17>, umma_gemv_kernel<1, 33>, umma_gemv_kernel<1, 65>, umma_gemv_kernel<1, 2>, umma_gemv_kernel<1, 3>, umma_gemv_kernel<1, 8>, umma_gemv_kernel<2, 0>, umma_gemv_kernel<2, 1>, umma_gemv_kernel<2, 17>, umma_gemv_kernel<2, 33>, umma_gemv_kernel<2, 65>, umma_gemv_kernel<2, 8>,
+                       umma_gemv_kernel<4, 0>, umma_gemv_kernel<4, 1>, umma_gemv_kernel<4, 17>, umma_gemv_kernel<4, 33>, umma_gemv_kernel<4, 65>, umma_gemv_kernel<4, 5>, umma_gemv_kernel<8, 0>, umma_gemv_kernel<8, 1>, umma_gemv_kernel<8, 17>, umma_gemv_kernel<8, 33>, umma_gemv_kernel<8, 65>, umma_gemv_kernel<8, 5>}) {
             e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
             if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(umma gemv)");
         }
@@ -895,8 +897,10 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     // stage, they leave the launch within half an SM where the image (61 KB for three tokens of 12288 columns, 111 for eight) would not,
     // so that it starts beside its predecessor and the next launch beside it: a step of three sequences 1208 -> 1204 us, of eight 1412 -> 1402.
     const bool prep = op->prologue == INSG_PRO_PREPARED;
-    const bool resid = p.nseg == 1 && p.seg[0].epilogue == INSG_EPI_RESIDUAL;
-    const bool streamed = prep && T >= 4 && resid && p.units <= clusters && kbq * kblock + exchange + 4 * kDStage > size_t(kDHalfSm);
+    const bool whole = (p.nkb & 7) == 0, resid = whole && p.nseg == 1 && p.seg[0].epilogue == INSG_EPI_RESIDUAL && p.units <= clusters;
+    bool plain = whole; // epilogues that add nothing and leave nothing prepared
+    for (int i = 0; i < p.nseg; i++) plain &= p.seg[i].epilogue != INSG_EPI_RESIDUAL && p.seg[i].epilogue != INSG_EPI_SWIGLU && p.seg[i].epilogue != INSG_EPI_LOGITS;
+    const bool streamed = prep && T >= 4 && resid && kbq * kblock + exchange + 4 * kDStage > size_t(kDHalfSm);
     const size_t stage_bytes = kDStage + (streamed ? 2 * kblock : 0);
     const size_t fixed = exchange + (streamed ? 0 : kbq * kblock) + (T == 8 && !prep ? size_t(8) * kDMaxKb * sizeof(float) : 0);
     // ring: no more stages than the launch has, within half an SM when that leaves at least four, else whatever fits.  Four are too
@@ -922,11 +926,11 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = op->pdl ? 2 : 1;
-    const bool gated = op->prologue == INSG_PRO_GATED_RMSNORM && !op->x_out && resid, two = p.nmat == 2;
-    auto kernel = T == 1 ? (logits ? (prep ? umma_gemv_kernel<1, 3> : umma_gemv_kernel<1, 2>) : (prep ? (two ? umma_gemv_kernel<1, 17> : resid ? umma_gemv_kernel<1, 33> : umma_gemv_kernel<1, 1>) : gated ? umma_gemv_kernel<1, 8> : umma_gemv_kernel<1, 0>))
-                : T == 2 ? (prep ? (two ? umma_gemv_kernel<2, 17> : resid ? umma_gemv_kernel<2, 33> : umma_gemv_kernel<2, 1>) : gated ? umma_gemv_kernel<2, 8> : umma_gemv_kernel<2, 0>)
-                : T == 4 ? (streamed ? umma_gemv_kernel<4, 5> : prep ? (two ? umma_gemv_kernel<4, 17> : resid ? umma_gemv_kernel<4, 33> : umma_gemv_kernel<4, 1>) : umma_gemv_kernel<4, 0>)
-                         : (streamed ? umma_gemv_kernel<8, 5> : prep ? (two ? umma_gemv_kernel<8, 17> : resid ? umma_gemv_kernel<8, 33> : umma_gemv_kernel<8, 1>) : umma_gemv_kernel<8, 0>);
+    const bool gated = op->prologue == INSG_PRO_GATED_RMSNORM && !op->x_out && resid, two = whole && p.nmat == 2;
+    auto kernel = T == 1 ? (logits ? (prep ? umma_gemv_kernel<1, 3> : umma_gemv_kernel<1, 2>) : (prep ? (two ? umma_gemv_kernel<1, 17> : resid ? umma_gemv_kernel<1, 33> : plain ? umma_gemv_kernel<1, 65> : umma_gemv_kernel<1, 1>) : gated ? umma_gemv_kernel<1, 8> : umma_gemv_kernel<1, 0>))
+                : T == 2 ? (prep ? (two ? umma_gemv_kernel<2, 17> : resid ? umma_gemv_kernel<2, 33> : plain ? umma_gemv_kernel<2, 65> : umma_gemv_kernel<2, 1>) : gated ? umma_gemv_kernel<2, 8> : umma_gemv_kernel<2, 0>)
+                : T == 4 ? (streamed ? umma_gemv_kernel<4, 5> : prep ? (two ? umma_gemv_kernel<4, 17> : resid ? umma_gemv_kernel<4, 33> : plain ? umma_gemv_kernel<4, 65> : umma_gemv_kernel<4, 1>) : umma_gemv_kernel<4, 0>)
+                         : (streamed ? umma_gemv_kernel<8, 5> : prep ? (two ? umma_gemv_kernel<8, 17> : resid ? umma_gemv_kernel<8, 33> : plain ? umma_gemv_kernel<8, 65> : umma_gemv_kernel<8, 1>) : umma_gemv_kernel<8, 0>);
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
     return e == cudaSuccess ? INSG_OK : cuda_fail(e, "umma gemv launch");
 }
