@@ -192,20 +192,20 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     __shared__ uint8_t s_lut[84];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    constexpr bool residual = (F & (kDResidual | kDStreamed | kDGated)) != 0, single = residual; // one segment, added into the residual stream, one unit per cluster
+    constexpr bool plain = (F & kDPlain) != 0;                       // nothing is left prepared
+    constexpr bool even = residual || plain || (F & kDTwo) != 0;     // every CTA has an even number of k-blocks
     const int rank = int(blockIdx.x) & (kDCl - 1), cl = int(blockIdx.x) / kDCl, C = int(gridDim.x) / kDCl;
     const int nkb = p.nkb, S = p.stages, nmat = (F & kDTwo) != 0 ? 2 : (F & (kDResidual | kDStreamed | kDGated | kDPlain)) != 0 ? 1 : p.nmat, XU = unit_slots<T>(nmat);
     const int kb0 = (nkb * rank) >> 2, len = ((nkb * (rank + 1)) >> 2) - kb0; // this CTA's k-blocks
     const int spt = (len + 1) >> 1;                                            // ring stages per (tile, matrix)
-    const int nun = cl < p.units ? (p.units - cl + C - 1) / C : 0;             // units of this cluster: cl, cl + C, ...
+    const int nun = residual ? 1 : cl < p.units ? (p.units - cl + C - 1) / C : 0;             // units of this cluster: cl, cl + C, ...
     const int nruns = nun * nmat, nstages = nruns * spt;
     uint8_t *ring = smem;                                // S stages
     uint8_t *bimg = ring + size_t(S) * kStage; // len x kImg bytes, unless streamed
     float *xslot = reinterpret_cast<float *>(bimg + (streamed ? 0 : size_t((nkb + 3) >> 2) * kImg)); // XU * nmat exchange slots
     float *s_ssq = T < 8 ? s_ssq_static : xslot + XU * nmat * kSlot; // [token][k-block], unless the input is prepared
 
-    constexpr bool residual = (F & (kDResidual | kDStreamed | kDGated)) != 0, single = residual; // one segment, added into the residual stream, one unit per cluster
-    constexpr bool plain = (F & kDPlain) != 0;                       // nothing is left prepared
-    constexpr bool even = residual || plain || (F & kDTwo) != 0;     // every CTA has an even number of k-blocks
     auto seg_of = [&](int unit) -> const DSeg & { return p.seg[single ? 0 : dseg_of(p, unit)]; };
     // ---- the weight stream starts first: it depends on nothing ----------------------------------------------------------
     auto run_src = [&](int run) -> const uint8_t * { // this CTA's records of the run (tile, matrix)
@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         if (lane < S && lane < nstages) {
-            const int run = lane / spt;
+            const int run = residual ? 0 : lane / spt;
             load_stage(lane, run_src(run), lane - run * spt);
         }
     } else if (warp == 8) {
@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             const bool one = elect_one();
             if constexpr (kDAheadStages<T> > 0) {
                 for (int i = S + lane; i < min(nstages, S + p.ahead); i += 32) {
-                    const int run = i / spt, st = i - run * spt;
+                    const int run = residual ? 0 : i / spt, st = i - run * spt;
                     bulk_prefetch(run_src(run) + size_t(st) * kDStage, uint32_t(min(2, len - 2 * st)) * kURec);
                 }
                 __syncwarp();
