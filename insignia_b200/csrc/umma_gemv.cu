@@ -159,14 +159,17 @@ template <int T> __device__ __forceinline__ void load_partial(uint32_t taddr, fl
 // half an SM (24576 x 4096 as SwiGLU 14.3 -> 13.3 us in the chain); one matrix keeps two (one: 9.7 -> 10.7 us at 12352 x 4096).
 template <int T> __host__ __device__ constexpr int unit_slots(int nmat) { return T == 1 ? 4 : T == 8 ? 3 - nmat : 2; }
 
-// What a variant of the kernel has beside its tokens: a prepared input in place of the prologue, the logits' arg-max, two matrices (SwiGLU), one
-// segment that adds into the residual stream; that with digits that come with the weights, or behind the gated norm.  A token is 129 launches of some
-// seven microseconds, and instructions that a launch runs through for the first time come from L2 behind the stream of weights.  Microseconds of a
-// token, a step of three sequences, of eight, and a speculative pass (a process is now and then 2 % off all of its life):
-//   one kernel with everything in it (96 KB of code for one token, 125 for eight)              1084 1308 1503 1500
-//   variants with a prepared input and with the arg-max, the waits' loops not unrolled,
-//   one store and one copy of the digits' code behind all epilogues (41 and 53 KB)             1057 1208 1412 1428
-//   and with two matrices, the gated norm, one segment where digits come with the weights      1040 1187 1380 1407
+// What a variant of the kernel has beside its tokens: a prepared input in place of the prologue; the logits' arg-max; two matrices (SwiGLU); one
+// segment that adds into the residual stream, one unit per cluster (kDResidual; with digits that come with the weights kDStreamed, behind the
+// gated norm kDGated); epilogues that add nothing and leave nothing prepared (kDPlain).  A launch that fits none takes the general ones.
+// A token is 129 launches of some seven microseconds, and instructions that a launch runs through for the first time come from L2 behind the
+// stream of weights.  Microseconds of a token, a step of three sequences, of eight, and a speculative pass (a process is now and then 2 % off for
+// all of its life), and the code of a launch:
+//   one kernel with everything in it                                                  1084 1308 1503 1500   96-125 KB
+//   variants prepared and arg-max, the waits' loops not unrolled, one store and one
+//   copy of the digits' code behind all epilogues                                     1057 1208 1412 1428   41-66
+//   and two matrices, the gated norm, residual                                        1057 1170 1348 1387   28-48
+//   and plain; no later runs, last odd block or slot reuse where there are none       1031 1156 1330 1365   20-37
 // (20 KB more in the issuer's loop, never run, cost a token 80 us.)
 constexpr int kDPrepared = 1, kDLogits = 2, kDStreamed = 4, kDGated = 8, kDTwo = 16, kDResidual = 32, kDPlain = 64;
 
@@ -653,9 +656,10 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 } else {
                 switch (s.epilogue) {
                 case INSG_EPI_RESIDUAL:
-                    if (plain) break;
+                    if constexpr (!plain) {
 #pragma unroll
-                    for (int u = 0; u < TN; u++) v[u] = f.h[u][0] + y[0][u];
+                        for (int u = 0; u < TN; u++) v[u] = f.h[u][0] + y[0][u];
+                    }
                     break;
                 case INSG_EPI_CONV_SILU:
 #pragma unroll
@@ -679,9 +683,10 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                     }
                     break;
                 case INSG_EPI_SWIGLU:
-                    if (plain) break;
+                    if constexpr (!plain) {
 #pragma unroll
-                    for (int u = 0; u < TN; u++) v[u] = fast_silu(y[0][u]) * y[1][u];
+                        for (int u = 0; u < TN; u++) v[u] = fast_silu(y[0][u]) * y[1][u];
+                    }
                     break;
                 default: break;
                 }
