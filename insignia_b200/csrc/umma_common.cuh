@@ -57,11 +57,26 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t *b, uint32_t parity, 
     return false;
 }
 
+// An arrival at another CTA's barrier that hands over what this thread did or saw in its own shared memory: a release at cluster scope,
+// restricted to shared memory, so that it waits for no store to global memory.
+__device__ __forceinline__ void remote_arrive(uint32_t bar)
+{
+    asm volatile("fence.release.sync_restrict::shared::cta.cluster;\n"
+                 "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
 // A poll that never suspends the thread.
 __device__ __forceinline__ bool mbar_test(uint64_t *b, uint32_t parity)
 {
     uint32_t done;
     asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(done) : "r"(smem_u32(b)), "r"(parity) : "memory");
+    return done != 0;
+}
+__device__ __forceinline__ bool mbar_test_cluster(uint64_t *b, uint32_t parity) // of what other CTAs of the cluster arrive at
+{
+    uint32_t done;
+    asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
                  : "=r"(done) : "r"(smem_u32(b)), "r"(parity) : "memory");
     return done != 0;
 }

@@ -509,11 +509,15 @@ template <int CL> __device__ __forceinline__ void g_commit(uint64_t *bar) // CL 
         asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                      ::"r"(smem_u32(bar)), "h"(uint16_t(3)) : "memory");
 }
-// Arrival at a barrier of the pair's first CTA.  Nothing is handed over that the arriving thread wrote, so no release: one at cluster scope
-// waits for what the thread's memory operations left behind, some 800 cycles a stage.
-__device__ __forceinline__ void first_arrive(uint64_t *bar)
+// Arrival at a barrier of the pair's first CTA: what this CTA's copies brought, or that its sums have been taken out of tensor memory.  A
+// release of everything, global memory included, waited some 800 cycles a stage; restricted to shared memory, with the issuer's waits acquiring
+// at cluster scope, a product takes as long as without any order (24576 x 4096, 512 tokens: 119.4 us either way).
+__device__ __forceinline__ void first_arrive(uint64_t *bar) { remote_arrive(map_to_rank(smem_u32(bar), 0)); }
+// The issuer's looks at its barriers; with CL == 2 the other CTA arrives there, too.
+template <int CL> __device__ __forceinline__ bool g_test(uint64_t *bar, uint32_t parity) { return CL == 1 ? mbar_test(bar, parity) : mbar_test_cluster(bar, parity); }
+template <int CL> __device__ __forceinline__ bool g_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag)
 {
-    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(map_to_rank(smem_u32(bar), 0)) : "memory");
+    return CL == 1 ? mbar_wait(bar, parity, abort_flag) : mbar_wait_cluster(bar, parity, abort_flag);
 }
 
 template <int TPG, bool SWIGLU>
@@ -668,12 +672,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
         for (int run = 0; g < end && ok; run++) {
             const GRun r = run_at(p, g, end);
             const bool two = SWIGLU || 2 * CL * (r.unit / p.ngroups) + CL < p.total_tiles;
-            ok = mbar_wait(&dempty, (run & 1) ^ 1, abort_flag); // the first run passes at once
+            ok = g_wait<CL>(&dempty, (run & 1) ^ 1, abort_flag); // the first run passes at once
             if (!ok) break;
 #pragma unroll 1
             for (int k = 0; k < r.len; k++) {
                 // (Two or four stages behind one look at their barriers, in straight-line code: no faster.)
-                if (!__all_sync(0xffffffffu, mbar_test(&full[st], phase)) && !mbar_wait(&full[st], phase, abort_flag)) { ok = false; break; }
+                if (!__all_sync(0xffffffffu, g_test<CL>(&full[st], phase)) && !g_wait<CL>(&full[st], phase, abort_flag)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t off = uint64_t(uint32_t(st) * uint32_t(kGStage >> 4));
                 const uint64_t da = da0 + off, dsf = dsf0 + off, db = da + uint64_t((2 * kURec) >> 4);

@@ -91,13 +91,6 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // The closing barrier only keeps CTAs from leaving early.  A release there would wait until the epilogue's global stores have been
 // acknowledged, which a stream of weights makes slow (one token 1214 -> 1189 us, lm_head with four tokens 145 -> 87 us).
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
-// Hands an exchange slot back to another CTA, whose next st.async must come after this CTA's reads of it: a release at cluster
-// scope, restricted to shared memory, so that it waits for none of those stores either.
-__device__ __forceinline__ void remote_arrive(uint32_t bar)
-{
-    asm volatile("fence.release.sync_restrict::shared::cta.cluster;\n"
-                 "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 // T floats to another CTA's shared memory; their bytes complete on that CTA's barrier.
 template <int T> __device__ __forceinline__ void send_floats(uint32_t dst, const float (&v)[T], uint32_t bar)
 {
@@ -627,7 +620,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                         hist[0] = h0; hist[1] = h1; hist[2] = h2;
                     }
                 }
-                if (!residual && i + XU < nun) { // the slot will be used again: tell the four senders
+                if (!residual && i + XU < nun) { // the slot will be used again: tell the four senders, whose next st.async must come after these reads
                     __syncwarp();
                     if (lane < kDCl) remote_arrive(map_to_rank(smem_u32(&xempty[slot]), uint32_t(lane)));
                 }

@@ -13,6 +13,14 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
+def pair_tokens(rows, cols, swiglu=False):
+    """The fewest tokens with which a product of these sizes runs on pairs of CTAs on this GPU: its stages in groups of 16 tokens (pairs of row
+    tiles, or gate and up tiles, x groups x k-blocks) are then more than 44 an SM."""
+    tiles = (rows + 127) // 128
+    per_group = (tiles if swiglu else (tiles + 1) // 2) * (cols // 128)
+    return max(49, 16 * (44 * torch.cuda.get_device_properties(0).multi_processor_count // per_group) + 1)
+
+
 # From 44 stages of 16 tokens an SM on (148 SMs: 6512 pairs of tiles x groups of 16 x k-blocks) two CTAs share a group of 32.  One, two, three
 # and five tiles with long sums and many groups; 101 to 104 tiles (the last four one to all there, the very last ragged), odd k-blocks, a full and
 # a just begun last group; then below the line: 16 tokens a group beyond 48 tokens
@@ -49,3 +57,35 @@ def test_pairs_swiglu(cuda, rows, cols, M):
         a, b = (orc.gemv_mlx_f64(w, s, x[m]) for w, s in mats)
         want = a / (1 + np.exp(-a)) * b
         assert np.max(np.abs(host(out)[m] - want)) <= 1e-5 * np.abs(want).max(), m
+
+
+# Five tiles: the last unit is a single one, multiplied by both CTAs; seven of SwiGLU: the last unit leaves the second CTA without a result
+@pytest.mark.parametrize("rows,cols,swiglu", [(640, 12288, False), (4096, 4096, False), (256, 4096, False), (896, 4096, True)])
+def test_pairs_have_the_same_bits_whoever_arrives_last(cuda, rows, cols, swiglu):
+    """What one CTA of a pair hands the other (copied stages, emptied accumulators), and whichever pair finds or adds the other parts of a unit,
+    shows in no bit.  Other work on the GPU moves the arrivals."""
+    from insignia_b200 import ops
+
+    M = pair_tokens(rows, cols, swiglu)
+    rng = np.random.default_rng(rows + M)
+    mats = [rand_matrix(rng, rows, cols) for _ in range(1 + swiglu)]
+    x = (rng.standard_normal((M, cols)) * 2).astype(np.float32)
+    packed = [ops.repack_umma(dev(w), dev(s)) for w, s in mats]
+    seg = dict(packed=packed[0], rows=rows, epilogue="store")
+    if swiglu:
+        seg.update(packed2=packed[1], epilogue="swiglu")
+    xd, scratch, calls = dev(x), ops.umma_gemm_scratch(cols, M), 60
+    outs = torch.zeros(calls, M, rows, device="cuda")
+    side, junk = torch.cuda.Stream(), torch.randn(1 << 22, device="cuda")
+    torch.cuda.synchronize()
+    for i in range(calls):
+        with torch.cuda.stream(side):
+            for _ in range(i % 4):
+                junk[: 1 << (12 + i % 11)].mul_(1.0)
+        ops.gemv_fused(xd, [dict(seg, out=outs[i])], layout=1, tokens=M, cols=cols, umma_scratch=scratch, pdl=i % 2 == 1)
+    torch.cuda.synchronize()
+    assert bool((outs == outs[0]).all())
+    for m in (0, 15, 16, M // 2, M - 1):
+        y64 = [orc.gemv_mlx_f64(w, s, x[m]) for w, s in mats]
+        want = y64[0] / (1 + np.exp(-y64[0])) * y64[1] if swiglu else y64[0]
+        assert np.max(np.abs(host(outs[0, m]) - want)) <= (2e-5 if swiglu else 4e-6) * np.abs(want).max(), m
