@@ -650,7 +650,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
         int st = 0;
         uint32_t phase = 0;
         for (int g = begin; g < end; g++) {
-            if (!mbar_wait(&full[st], phase, abort_flag)) break;
+            if (!__all_sync(0xffffffffu, mbar_wait(&full[st], phase, abort_flag))) break; // together: the lanes meet again below
             if (lane == 0) first_arrive(&full[st]);
             __syncwarp();
             if (++st == S) { st = 0; phase ^= 1; }
@@ -672,12 +672,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
         for (int run = 0; g < end && ok; run++) {
             const GRun r = run_at(p, g, end);
             const bool two = SWIGLU || 2 * CL * (r.unit / p.ngroups) + CL < p.total_tiles;
-            ok = g_wait<CL>(&dempty, (run & 1) ^ 1, abort_flag); // the first run passes at once
+            // a wait that runs out ends the loop for all lanes: they vote again at the next stage
+            ok = __all_sync(0xffffffffu, g_wait<CL>(&dempty, (run & 1) ^ 1, abort_flag)); // the first run passes at once
             if (!ok) break;
 #pragma unroll 1
             for (int k = 0; k < r.len; k++) {
                 // (Two or four stages behind one look at their barriers, in straight-line code: no faster.)
-                if (!__all_sync(0xffffffffu, g_test<CL>(&full[st], phase)) && !g_wait<CL>(&full[st], phase, abort_flag)) { ok = false; break; }
+                if (!__all_sync(0xffffffffu, g_test<CL>(&full[st], phase)) && !__all_sync(0xffffffffu, g_wait<CL>(&full[st], phase, abort_flag))) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t off = uint64_t(uint32_t(st) * uint32_t(kGStage >> 4));
                 const uint64_t da = da0 + off, dsf = dsf0 + off, db = da + uint64_t((2 * kURec) >> 4);
