@@ -648,6 +648,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                     for (int u = 0; u < TN; u++) v[u] = f.h[u][0] + y[0][u];
                 } else {
                 switch (s.epilogue) {
+                case INSG_EPI_STORE: break;
                 case INSG_EPI_RESIDUAL:
                     if constexpr (!plain) {
 #pragma unroll
@@ -681,7 +682,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                         for (int u = 0; u < TN; u++) v[u] = fast_silu(y[0][u]) * y[1][u];
                     }
                     break;
-                default: break;
+                default: continue; // no such epilogue: nothing is stored
                 }
                 }
 #pragma unroll
