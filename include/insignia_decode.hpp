@@ -68,7 +68,8 @@ public:
     int *d_next{};       // device: arg-max of the last logits
     void *attn_scratch{};
     void *argmax_scratch{};
-    float *multi{};      // device: activations of up to 1024 consecutive tokens (forward_tokens)
+    int pass_tokens{};   // longest pass of forward_tokens: 1024 tokens, fewer where max_context is (a multiple of eight)
+    float *multi{};      // device: activations of pass_tokens consecutive tokens
     void *umma_scratch{}; // device: digit image of the activations for the tcgen05 kernel (forward_tokens)
     size_t umma_scratch_bytes{};
     void *prep{};        // device: prepared inputs of products and sums of squares (digit images of up to eight tokens on tcgen05, the

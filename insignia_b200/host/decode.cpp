@@ -29,17 +29,15 @@ constexpr size_t kPrepHidden = 0, kPrepAct = size_t(kHidden / 128) * (8 * 512 + 
                  kPrepSums = kPrepCore + size_t(kHidden / 128) * (8 * 512 + 512);
 constexpr int kFrontLayers = 2; // layers of the short first graph of a host-fed step: some 70 us of work, what submitting the rest takes
 constexpr int kMultiSteps = 8; // token steps per graph in Qwen35Decode::generate
-// DecodeWorkspace::multi: activations of up to kChunk consecutive tokens for Qwen35Decode::forward_tokens, [token][width] each
+// Qwen35Decode::forward_tokens: tokens per pass
 constexpr int kChunk = 4;     // tokens per pass of the mma.sync kernel
 constexpr int kSmallChunk = 8; // tokens per pass of the tcgen05 GEMV
 constexpr int kBigChunk = 1024; // tokens per pass of the tcgen05 GEMM: a 2048-token prompt takes 59.3 ms in passes of 512 and 53.3 of 1024; of 2048 another 2 % less for 240 MB more
 constexpr int kAttnRegions = 32; // attention scratch regions: passes of more tokens run in query tiles, which need none
-constexpr size_t kMultiHidden = 0, kMultiQkv = kMultiHidden + size_t(kBigChunk) * 4096, kMultiZ = kMultiQkv + size_t(kBigChunk) * 8192,
-                 kMultiA = kMultiZ + size_t(kBigChunk) * 4096, kMultiB = kMultiA + size_t(kBigChunk) * 32,
-                 kMultiCore = kMultiB + size_t(kBigChunk) * 32, kMultiQg = kMultiCore + size_t(kBigChunk) * 4096,
-                 kMultiKey = kMultiQg + size_t(kBigChunk) * 8192, kMultiValue = kMultiKey + size_t(kBigChunk) * 1024,
-                 kMultiAct = kMultiValue + size_t(kBigChunk) * 1024, kMultiQn = kMultiAct + size_t(kBigChunk) * 12288,
-                 kMultiTokens = kMultiQn + size_t(kBigChunk) * 4096, kMultiFloats = kMultiTokens + kBigChunk;
+// offsets in DecodeWorkspace::multi, floats for each of its pass_tokens tokens
+constexpr size_t kMultiHidden = 0, kMultiQkv = kMultiHidden + 4096, kMultiZ = kMultiQkv + 8192, kMultiA = kMultiZ + 4096, kMultiB = kMultiA + 32,
+                 kMultiCore = kMultiB + 32, kMultiQg = kMultiCore + 4096, kMultiKey = kMultiQg + 8192, kMultiValue = kMultiKey + 1024,
+                 kMultiAct = kMultiValue + 1024, kMultiQn = kMultiAct + 12288, kMultiTokens = kMultiQn + 4096, kMultiFloats = kMultiTokens + 1;
 constexpr size_t kPrepBytes = kPrepSums + 8 * (kHidden / 32) * sizeof(float); // [token][32-row group], or two rows of 296
 const char *const kLM = "language_model";
 
@@ -99,8 +97,9 @@ void DecodeWorkspace::allocate()
     cuda_check(cudaMalloc(&attn_scratch, size_t(kAttnRegions) * insg_gqa_scratch_bytes(max_context)), "cudaMalloc attention scratch");
     cuda_check(cudaMalloc(&argmax_scratch, insg_gemv_argmax_scratch_bytes()), "cudaMalloc arg-max scratch");
     cuda_check(cudaMalloc(&prep, kPrepBytes), "cudaMalloc prepared inputs");
-    cuda_check(cudaMalloc(&multi, kMultiFloats * sizeof(float)), "cudaMalloc multi-token buffers");
-    umma_scratch_bytes = insg_umma_gemm_scratch_bytes(kInter, kBigChunk);
+    pass_tokens = (std::min(max_context, kBigChunk) + kSmallChunk - 1) / kSmallChunk * kSmallChunk; // no pass is longer than the context
+    cuda_check(cudaMalloc(&multi, kMultiFloats * pass_tokens * sizeof(float)), "cudaMalloc multi-token buffers");
+    umma_scratch_bytes = insg_umma_gemm_scratch_bytes(kInter, pass_tokens);
     cuda_check(cudaMalloc(&umma_scratch, umma_scratch_bytes), "cudaMalloc tcgen05 activation image");
     cuda_check(cudaMemsetAsync(prep, 0, kPrepBytes, stream), "memset");
     cuda_check(cudaMemsetAsync(attn_scratch, 0, size_t(kAttnRegions) * insg_gqa_scratch_bytes(max_context), stream), "memset");
@@ -431,11 +430,12 @@ struct Multi {
     const uint16_t *next_norm = nullptr; // weight of the RMSNorm that reads the block's output next
     int rows_hint = 0; // eager passes: the rows the pass's last token attends (the host's position + T); 0 inside a replayed graph
     explicit Multi(DecodeWorkspace &x, int t)
-        : hidden(x.multi + kMultiHidden), qkv(x.multi + kMultiQkv), z(x.multi + kMultiZ), a(x.multi + kMultiA), b(x.multi + kMultiB),
-          core(x.multi + kMultiCore), qg(x.multi + kMultiQg), key(x.multi + kMultiKey), value(x.multi + kMultiValue),
-          act(x.multi + kMultiAct), qn(x.multi + kMultiQn), tokens(reinterpret_cast<int *>(x.multi + kMultiTokens)), T(t)
+        : hidden(at(x, kMultiHidden)), qkv(at(x, kMultiQkv)), z(at(x, kMultiZ)), a(at(x, kMultiA)), b(at(x, kMultiB)), core(at(x, kMultiCore)),
+          qg(at(x, kMultiQg)), key(at(x, kMultiKey)), value(at(x, kMultiValue)), act(at(x, kMultiAct)), qn(at(x, kMultiQn)),
+          tokens(reinterpret_cast<int *>(at(x, kMultiTokens))), T(t)
     {
     }
+    static float *at(const DecodeWorkspace &x, size_t offset) { return x.multi + offset * size_t(x.pass_tokens); }
 };
 
 // The RMSNorm'd residual stream as a product's input, and the residual stream left prepared for the RMSNorm that follows.
@@ -971,7 +971,7 @@ void Qwen35Decode::run_prompt(const int *tokens, int count, bool mtp)
     load_head();
     load_embed();
     Ctx c{x_, p.stream, x_.options.use_pdl, launches_, false, nullptr, nullptr};
-    // Long prompts go through the tcgen05 GEMM in passes of up to kBigChunk tokens; what is left, and short prompts, through
+    // Long prompts go through the tcgen05 GEMM in passes of up to pass_tokens tokens; what is left, and short prompts, through
     // the engine's own GEMV: up to eight tokens a pass on tcgen05, four on mma.sync.
     const bool one_layout = tcgen05_engine(x_.options);
     const bool big = x_.options.prefill_tcgen05 && count > (one_layout ? kSmallChunk : 15);
@@ -980,7 +980,7 @@ void Qwen35Decode::run_prompt(const int *tokens, int count, bool mtp)
     for (int done = 0; done < count;) {
         const int left = count - done;
         const bool use_umma = big && left > (one_layout ? kSmallChunk : 7);
-        const int T = use_umma ? std::min(left, kBigChunk) : one_layout ? std::min(left, kSmallChunk) : (left >= 4 ? 4 : (left >= 2 ? 2 : 1));
+        const int T = use_umma ? std::min(left, x_.pass_tokens) : one_layout ? std::min(left, kSmallChunk) : (left >= 4 ? 4 : (left >= 2 ? 2 : 1));
         c.layout = use_umma ? 1 : -1;
         const std::vector<Plan::Block> &blocks = use_umma && !one_layout ? p.layers_umma : p.layers;
         Multi u(x_, T);
