@@ -294,6 +294,7 @@ INSG_API uint64_t insg_program_weight_bytes(const insg_program *prog);
 INSG_API int insg_deltanet_decode(float *state, const float *q16, const float *k16, const float *v32,
                                   const float *g32, const float *beta32, float *out32, int pdl,
                                   insg_stream_t stream);
+#define INSG_DELTANET_MAX_TOKENS 1024 /* steps of a launch */
 /* The same step for `tokens` (1..1024) consecutive positions of the sequence in one launch: the state is read once,
  * kept on chip from step to step and written once (two or more tokens run a kernel that prepares the inputs of 32
  * steps at a time; bit-identical results).  q16/k16/v32 of step m are at + m * qkv_stride floats, g32/beta32 at

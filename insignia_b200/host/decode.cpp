@@ -32,7 +32,8 @@ constexpr int kMultiSteps = 8; // token steps per graph in Qwen35Decode::generat
 // Qwen35Decode::forward_tokens: tokens per pass
 constexpr int kChunk = 4;     // tokens per pass of the mma.sync kernel
 constexpr int kSmallChunk = 8; // tokens per pass of the tcgen05 GEMV
-constexpr int kBigChunk = 1024; // tokens per pass of the tcgen05 GEMM: a 2048-token prompt takes 59.3 ms in passes of 512 and 53.3 of 1024; of 2048 another 2 % less for 240 MB more
+constexpr int kBigChunk = 1024; // tokens per pass of the tcgen05 GEMM at most: a 2048-token prompt (fp32 cache) takes 59.4 ms in passes of 512, 53.1 in these
+static_assert(kBigChunk <= INSG_DELTANET_MAX_TOKENS, "a pass's steps go out in one launch");
 constexpr int kAttnRegions = 32; // attention scratch regions: passes of more tokens run in query tiles, which need none
 // offsets in DecodeWorkspace::multi, floats for each of its pass_tokens tokens
 constexpr size_t kMultiHidden = 0, kMultiQkv = kMultiHidden + 4096, kMultiZ = kMultiQkv + 8192, kMultiA = kMultiZ + 4096, kMultiB = kMultiA + 32,
