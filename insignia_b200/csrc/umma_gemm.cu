@@ -857,8 +857,14 @@ bool g_gemm_attr_done[64] = {false}; // the shared-memory opt-in is a per-device
 //   128                                                                  28.5 / 23.7 (69)  24.7 / 23.2 (55)  19.8 / 19.8 (28)
 //   192                                                                                                      22.0 / 22.2 (42)
 //   256                                                                                                      25.7 / 24.2 (55)
+// With few k-blocks that many stages are whole units, of which only the first and the last are cut: then 32 again, from 2.5 units an SM on
+// (16 / 32, in brackets the units): 4096 x 1024, 256 tokens 14.4 / 15.0 (1.7), 12352 x 2048, 100 tokens 19.2 / 18.8 (2.3), 8192 x 2048, 192 tokens
+// 21.1 / 19.2 (2.6), 8192 x 1024, 256 tokens 18.2 / 17.4 (3.5), 12352 x 1024, 256 tokens 22.4 / 20.2 (5.3), 24576 x 256, 512 tokens 40.7 / 36.0 (21).
 constexpr int kFewStages = 44;
-int tokens_per_group(int tokens, long long stages16) { return tokens <= 48 || stages16 <= (long long)kFewStages * sm_count() ? 16 : 32; }
+int tokens_per_group(int tokens, long long stages16, int nkb)
+{
+    return tokens <= 48 || (stages16 <= (long long)kFewStages * sm_count() && 2 * stages16 <= 5ll * nkb * sm_count()) ? 16 : 32;
+}
 size_t image_bytes(int cols, int tokens) // room for either: groups of 32 take as many bytes as groups of 16 or more
 {
     const int tpg = tokens <= 48 ? 16 : 32;
@@ -925,7 +931,7 @@ int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
         g.tile_begin = tiles; tiles += (s.rows + 127) >> 7; g.epilogue = s.epilogue; g.rows = s.rows;
     }
     const int nkb = op->cols >> 7;
-    const int tpg = tokens_per_group(tokens, (long long)(nmat_all == 2 ? tiles : (tiles + 1) / 2) * ((tokens + 15) / 16) * nkb);
+    const int tpg = tokens_per_group(tokens, (long long)(nmat_all == 2 ? tiles : (tiles + 1) / 2) * ((tokens + 15) / 16) * nkb, nkb);
     const int ngroups = (tokens + tpg - 1) / tpg;
 
     DigitizeParams d = {};

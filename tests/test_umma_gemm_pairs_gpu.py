@@ -1,4 +1,4 @@
-"""Products with many stages run on pairs of CTAs that multiply four row tiles with one set of digits, those with few in groups of 16 tokens."""
+"""Products with many stages or units run on pairs of CTAs that multiply four row tiles with one set of digits, those with few in groups of 16 tokens."""
 import os
 import sys
 
@@ -14,11 +14,11 @@ torch = pytest.importorskip("torch")
 
 
 def pair_tokens(rows, cols, swiglu=False):
-    """The fewest tokens with which a product of these sizes runs on pairs of CTAs on this GPU: its stages in groups of 16 tokens (pairs of row
-    tiles, or gate and up tiles, x groups x k-blocks) are then more than 44 an SM."""
-    tiles = (rows + 127) // 128
-    per_group = (tiles if swiglu else (tiles + 1) // 2) * (cols // 128)
-    return max(49, 16 * (44 * torch.cuda.get_device_properties(0).multi_processor_count // per_group) + 1)
+    """The fewest tokens with which a product of these sizes runs on pairs of CTAs on this GPU: in groups of 16 tokens it has more than 44 stages
+    (pairs of row tiles, or gate and up tiles, x groups x k-blocks) or more than 2.5 units (without the k-blocks) an SM."""
+    tiles, sms = (rows + 127) // 128, torch.cuda.get_device_properties(0).multi_processor_count
+    units = tiles if swiglu else (tiles + 1) // 2
+    return max(49, 16 * (min(44 * sms // (cols // 128), 5 * sms // 2) // units) + 1)
 
 
 # From 44 stages of 16 tokens an SM on (148 SMs: 6512 pairs of tiles x groups of 16 x k-blocks) two CTAs share a group of 32.  One, two, three
@@ -59,8 +59,24 @@ def test_pairs_swiglu(cuda, rows, cols, M):
         assert np.max(np.abs(host(out)[m] - want)) <= 1e-5 * np.abs(want).max(), m
 
 
+# On both sides of the line, where the stages draw it and where the units do (few k-blocks)
+@pytest.mark.parametrize("rows,cols", [(2048, 4096), (1152, 2304), (4096, 1024), (12352, 256), (640, 128)])
+def test_either_side_of_the_line(cuda, rows, cols):
+    from insignia_b200 import ops
+
+    rng = np.random.default_rng(rows + cols)
+    w, s = rand_matrix(rng, rows, cols)
+    P, line = ops.repack_umma(dev(w), dev(s)), pair_tokens(rows, cols)
+    x = (rng.standard_normal((line, cols)) * rng.uniform(0.01, 30, (line, 1))).astype(np.float32)
+    for M in (line - 1, line):
+        y = host(ops.gemm_umma(P, dev(x[:M])))
+        for m in (0, 17, M - 1):
+            y64 = orc.gemv_mlx_f64(w, s, x[m])
+            assert np.max(np.abs(y[m] - y64)) <= 4e-6 * np.abs(y64).max() + 1e-7, (M, m)
+
+
 # Five tiles: the last unit is a single one, multiplied by both CTAs; seven of SwiGLU: the last unit leaves the second CTA without a result
-@pytest.mark.parametrize("rows,cols,swiglu", [(640, 12288, False), (4096, 4096, False), (256, 4096, False), (896, 4096, True)])
+@pytest.mark.parametrize("rows,cols,swiglu", [(640, 12288, False), (4096, 4096, False), (256, 4096, False), (128 * 37, 512, False), (896, 4096, True)])
 def test_pairs_have_the_same_bits_whoever_arrives_last(cuda, rows, cols, swiglu):
     """What one CTA of a pair hands the other (copied stages, emptied accumulators), and whichever pair finds or adds the other parts of a unit,
     shows in no bit.  Other work on the GPU moves the arrivals."""
