@@ -121,3 +121,15 @@ def rmsnorm(R=3, C=4096):
 
 def max_rel(actual, expected, eps):
     return float(np.max(np.abs(actual - expected) / (np.abs(expected) + eps)))
+
+
+def pair_tokens(rows, cols, swiglu=False, last=None):
+    """The fewest tokens with which a product of these sizes runs in groups of 32 tokens on pairs of CTAs on this GPU: in groups of 16 it has more
+    than 44 stages (pairs of row tiles, or gate and up tiles, x groups x k-blocks) or more than 2.5 units (without the k-blocks) an SM.  `last`:
+    so many tokens in the last group."""
+    import torch
+
+    tiles, sms = (rows + 127) // 128, torch.cuda.get_device_properties(0).multi_processor_count
+    units = tiles if swiglu else (tiles + 1) // 2
+    fewest = max(49, 16 * (min(44 * sms // (cols // 128), 5 * sms // 2) // units) + 1)
+    return fewest if last is None else fewest + (last - fewest) % 32

@@ -7,19 +7,23 @@ import numpy as np
 import pytest
 
 sys.path.insert(0, os.path.join(os.path.dirname(__file__), ".."))
+from tests.fixtures import pair_tokens  # noqa: E402
 from tests.test_kernels_gpu import bf16, dev, host, rand_matrix  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
-@pytest.mark.parametrize("tokens", [9, 49, 300])
+@pytest.mark.parametrize("tokens", [9, 49, 300, "pairs"])
 @pytest.mark.parametrize("pdl", [False, True])
 def test_queued_products_read_their_own_digits(cuda, tokens, pdl):
     from insignia_b200 import ops
 
-    rng = np.random.default_rng(tokens)
     rows, cols, calls = 384, 1152, 24
+    if tokens == "pairs":  # the GEMM on pairs of CTAs, whose digits have a producer warp of their own
+        rows = 2432
+        tokens = pair_tokens(rows, cols)
+    rng = np.random.default_rng(tokens)
     packed = ops.repack_umma(*(dev(a) for a in rand_matrix(rng, rows, cols)))
     xs = [torch.randn(tokens, cols, device="cuda") for _ in range(calls)]
 

@@ -8,20 +8,24 @@ import pytest
 
 sys.path.insert(0, os.path.join(os.path.dirname(__file__), ".."))
 from oracle import oracle as orc  # noqa: E402
+from tests.fixtures import pair_tokens  # noqa: E402
 from tests.test_kernels_gpu import bf16, dev, host, rand_matrix  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
-# up to eight tokens: the GEMV; more: the GEMM with 16 (up to 48) or 32 tokens a group
-@pytest.mark.parametrize("tokens", [1, 2, 3, 8, 9, 16, 48, 49, 71])
+# up to eight tokens: the GEMV; more: the GEMM with 16 tokens a group, or with 32 on pairs of CTAs (with 17 in the last one)
+@pytest.mark.parametrize("tokens", [1, 2, 3, 8, 9, 16, 48, 49, 71, "pairs"])
 @pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
 def test_a_non_finite_activation_makes_its_token_nan(cuda, tokens, value):
     from insignia_b200 import ops
 
-    rng = np.random.default_rng(tokens)
     rows, cols = 384, 1152
+    if tokens == "pairs":
+        rows = 2432  # 19 tiles
+        tokens = pair_tokens(rows, cols, last=17)
+    rng = np.random.default_rng(tokens)
     P = ops.repack_umma(*(dev(a) for a in rand_matrix(rng, rows, cols)))
     x = rng.standard_normal((tokens, cols)).astype(np.float32)
     clean = host(ops.gemm_umma(P, dev(x)))
@@ -61,13 +65,17 @@ def test_a_prepared_image_carries_nan(cuda, tokens):
         assert np.isfinite(clean).all() and np.isnan(with_nan[-1]).all() and np.array_equal(clean[:-1], with_nan[:-1])
 
 
-@pytest.mark.parametrize("tokens", [1, 8, 9, 49])
+@pytest.mark.parametrize("tokens", [1, 8, 9, 49, "pairs"])
 @pytest.mark.parametrize("scale", [1e32, 1e-33])
 def test_groups_of_very_large_and_small_values(cuda, tokens, scale):
     from insignia_b200 import ops
 
+    rows = 256
+    if tokens == "pairs":
+        rows = 2432
+        tokens = pair_tokens(rows, 1152)
     rng = np.random.default_rng(tokens)
-    w, s = rand_matrix(rng, 256, 1152)
+    w, s = rand_matrix(rng, rows, 1152)
     x = (rng.standard_normal((tokens, 1152)) * scale).astype(np.float32)
     x[:, 64:96] *= 1e3  # one group far above the others
     got = host(ops.gemm_umma(ops.repack_umma(dev(w), dev(s)), dev(x))).astype(np.float64)

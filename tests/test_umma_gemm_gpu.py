@@ -52,8 +52,8 @@ def test_gemm_umma_is_deterministic_across_cut_units(cuda, rows, cols, M):
     assert np.max(np.abs(first[M - 1] - y64)) <= 4e-6 * np.abs(y64).max()
 
 
-# 37 tiles and two groups: 19 pairs, the last one of a single tile, every unit in two parts; five tiles: units in about ten parts; three groups:
-# units in two to five; the last one SwiGLU, where a pair is a gate and an up tile
+# Groups of 16 tokens: 37 tiles, four groups: 19 pairs of tiles, the last one of a single tile; five tiles: units in about ten parts; 32 tiles, five
+# groups; the last one SwiGLU, where a pair is a gate and an up tile.  (Groups of 32 tokens on pairs of CTAs: test_umma_gemm_pairs_gpu.py.)
 @pytest.mark.parametrize("rows,cols,M,swiglu", [(128 * 37, 512, 49, False), (640, 12288, 61, False), (4096, 4096, 65, False), (896, 4096, 61, True)])
 def test_cut_units_have_the_same_bits_whoever_arrives_last(cuda, rows, cols, M, swiglu):
     """The CTA that finds the other part of a unit there adds it to its own; else the last one to arrive adds all parts.  Other work on the

@@ -7,21 +7,14 @@ import pytest
 
 sys.path.insert(0, os.path.join(os.path.dirname(__file__), ".."))
 from oracle import oracle as orc  # noqa: E402
-from tests.test_kernels_gpu import dev, host, rand_matrix  # noqa: E402
+from tests.fixtures import pair_tokens  # noqa: E402
+from tests.test_kernels_gpu import bf16, dev, host, rand_matrix  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
-def pair_tokens(rows, cols, swiglu=False):
-    """The fewest tokens with which a product of these sizes runs on pairs of CTAs on this GPU: in groups of 16 tokens it has more than 44 stages
-    (pairs of row tiles, or gate and up tiles, x groups x k-blocks) or more than 2.5 units (without the k-blocks) an SM."""
-    tiles, sms = (rows + 127) // 128, torch.cuda.get_device_properties(0).multi_processor_count
-    units = tiles if swiglu else (tiles + 1) // 2
-    return max(49, 16 * (min(44 * sms // (cols // 128), 5 * sms // 2) // units) + 1)
-
-
-# From 44 stages of 16 tokens an SM on (148 SMs: 6512 pairs of tiles x groups of 16 x k-blocks) two CTAs share a group of 32.  One, two, three
+# Beyond 44 stages of 16 tokens an SM (148 SMs: 6512 pairs of tiles x groups of 16 x k-blocks), or 2.5 units, two CTAs share a group of 32.  One, two, three
 # and five tiles with long sums and many groups; 101 to 104 tiles (the last four one to all there, the very last ragged), odd k-blocks, a full and
 # a just begun last group; then below the line: 16 tokens a group beyond 48 tokens
 @pytest.mark.parametrize("rows,cols,M", [(100, 12288, 1200), (256, 12288, 1090), (384, 12288, 600), (640, 12288, 400), (128 * 101, 4224, 49), (128 * 102, 4096, 64),
@@ -105,3 +98,67 @@ def test_pairs_have_the_same_bits_whoever_arrives_last(cuda, rows, cols, swiglu)
         y64 = [orc.gemv_mlx_f64(w, s, x[m]) for w, s in mats]
         want = y64[0] / (1 + np.exp(-y64[0])) * y64[1] if swiglu else y64[0]
         assert np.max(np.abs(host(outs[0, m]) - want)) <= (2e-5 if swiglu else 4e-6) * np.abs(want).max(), m
+
+
+def test_pairs_fused_inproj(cuda):
+    """in_proj(qkv|z|a|b) of a long pass on pairs: RMSNorm per token, conv + SiLU with the history carried through the tokens, store, decay, beta; segments
+    of three, two, one and one tiles (the last two of 32 rows) in units of four."""
+    from insignia_b200 import mxfp4, ops
+
+    rng = np.random.default_rng(41)
+    nq, nz, cols = 384, 256, 4096
+    T = pair_tokens(nq + nz + 128 + 128, cols, last=9)
+    (wq, sq), (wz, sz) = rand_matrix(rng, nq, cols), rand_matrix(rng, nz, cols)
+    (wa, sa), (wb, sb) = rand_matrix(rng, 32, cols, std=0.05), rand_matrix(rng, 32, cols, std=0.05)
+    conv_w = mxfp4.f32_to_bf16_bits((0.5 * rng.standard_normal((nq, 4))).astype(np.float32))
+    A_log, dt = rng.uniform(-1, 1, 32).astype(np.float32), mxfp4.f32_to_bf16_bits((0.5 * rng.standard_normal(32)).astype(np.float32))
+    nw = bf16(rng, cols)
+    P = [ops.repack_umma(dev(w), dev(s)) for w, s in ((wq, sq), (wz, sz), (wa, sa), (wb, sb))]
+    state0 = (rng.standard_normal(nq * 3) * 0.3).astype(np.float32)
+    conv_state, err = dev(state0.copy()), torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = [torch.zeros(T, r, device="cuda") for r in (nq, nz, 32, 32)]
+    hidden = (rng.standard_normal((T, cols)) * 3).astype(np.float32)
+    ops.gemv_fused(dev(hidden), [
+        dict(packed=P[0], out=out[0], rows=nq, epilogue="conv_silu", conv_state=conv_state, conv_w=dev(conv_w)),
+        dict(packed=P[1], out=out[1], rows=nz, epilogue="store"),
+        dict(packed=P[2], out=out[2], rows=32, epilogue="decay", A_log=dev(A_log), dt_bias=dev(dt)),
+        dict(packed=P[3], out=out[3], rows=32, epilogue="beta")], prologue="rmsnorm", norm_w=dev(nw), layout=1, error_flag=err, tokens=T, cols=cols,
+        umma_scratch=ops.umma_gemm_scratch(cols, T))
+    gq, gz, ga, gb = (host(o) for o in out)
+    ref_state = state0.copy()
+    for m in range(T):
+        n = orc.rmsnorm_bf16(hidden[m], nw)
+        q = orc.gemv_mlx(wq, sq, n)
+        orc.causal_conv4_silu(q, ref_state, conv_w)
+        assert np.max(np.abs(gq[m] - q)) <= 2e-5 * max(1.0, np.abs(q).max()), m
+        if m % 16 in (0, 15) or m == T - 1:
+            a, b = orc.gemv_mlx(wa, sa, n), orc.gemv_mlx(wb, sb, n)
+            orc.deltanet_parameters(a, b, A_log, dt)
+            assert np.max(np.abs(gz[m] - orc.gemv_mlx(wz, sz, n))) <= 2e-5, m
+            assert np.max(np.abs(ga[m] - a)) <= 2e-5 * max(1.0, np.abs(a).max()) and np.max(np.abs(gb[m] - b)) <= 2e-6, m
+    assert np.max(np.abs(host(conv_state) - ref_state)) <= 2e-5 * np.abs(ref_state).max()
+    assert int(err.item()) == 0
+
+
+@pytest.mark.parametrize("prologue", ["gated_rmsnorm", "sigmoid_gate", "sigmoid_gate_head0", "sigmoid_gate_qproj"])
+def test_pairs_residual_behind_each_gate(cuda, prologue):
+    """The out and o projections of a long pass on pairs against the same tokens in calls of 16 (the other form, which the oracle tests): two orders of
+    fp32 sums, each within 4e-7 of the largest."""
+    from insignia_b200 import ops
+
+    rng = np.random.default_rng(len(prologue))
+    rows, cols = 1000, 4096
+    T = pair_tokens(rows, cols, last=1)
+    P = ops.repack_umma(*(dev(a) for a in rand_matrix(rng, rows, cols)))
+    x = dev(rng.standard_normal((T, cols)).astype(np.float32))
+    aux = dev(rng.standard_normal((T, cols if prologue in ("gated_rmsnorm", "sigmoid_gate") else 2 * cols)).astype(np.float32))
+    res, nw = rng.standard_normal((T, rows)).astype(np.float32), dev(bf16(rng, 128))
+    kw = dict(prologue=prologue, layout=1, cols=cols, umma_scratch=ops.umma_gemm_scratch(cols, T), **(dict(norm_w=nw) if prologue == "gated_rmsnorm" else {}))
+    got, want = dev(res.copy()), dev(res.copy())
+    ops.gemv_fused(x, [dict(packed=P, out=got, rows=rows, epilogue="residual")], aux=aux, tokens=T, **kw)
+    for m in range(0, T, 16):
+        n = min(16, T - m)
+        ops.gemv_fused(x[m:m + n], [dict(packed=P, out=want[m:m + n], rows=rows, epilogue="residual")], aux=aux[m:m + n], tokens=n, **kw)
+    got, want = host(got), host(want)
+    assert np.max(np.abs(got - want)) <= 8e-7 * np.abs(want).max()
+    assert np.max(np.abs(want - res)) > 0.1
