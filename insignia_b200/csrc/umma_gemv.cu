@@ -789,6 +789,25 @@ __global__ void repack_umma_kernel(const uint32_t *__restrict__ w, const uint8_t
 }
 
 namespace {
+// The variants there are, for T token slots: the launch chooses among them and the attributes are set for them by the same list.
+using DKernel = void (*)(DParams);
+template <int T, int... F> DKernel variant_of(int f)
+{
+    DKernel k = nullptr;
+    ((f == F ? void(k = umma_gemv_kernel<T, F>) : void()), ...);
+    return k;
+}
+DKernel gemv_kernel(int slots, int f)
+{
+    constexpr int kP = kDPrepared;
+    switch (slots) {
+    case 1: return variant_of<1, 0, kP, kP | kDTwo, kP | kDResidual, kP | kDPlain, kDLogits, kP | kDLogits, kDGated>(f);
+    case 2: return variant_of<2, 0, kP, kP | kDTwo, kP | kDResidual, kP | kDPlain, kDGated>(f);
+    case 4: return variant_of<4, 0, kP, kP | kDTwo, kP | kDResidual, kP | kDPlain, kP | kDStreamed>(f);
+    default: return variant_of<8, 0, kP, kP | kDTwo, kP | kDResidual, kP | kDPlain, kP | kDStreamed>(f);
+    }
+}
+
 std::mutex g_attr_mutex;
 int g_max_clusters[64] = {0}; // per device: clusters that run at once with one CTA per SM (0 = not asked yet)
 
@@ -801,11 +820,12 @@ int device_clusters(int *out)
     if (dev < 0 || dev >= 64) return fail(INSG_E_LIMIT, "gemv: device ordinal beyond 63");
     std::lock_guard<std::mutex> lock(g_attr_mutex);
     if (!g_max_clusters[dev]) {
-        for (auto k : {umma_gemv_kernel<1, 0>, umma_gemv_kernel<1, 1>, umma_gemv_kernel<1, 17>, umma_gemv_kernel<1, 33>, umma_gemv_kernel<1, 65>, umma_gemv_kernel<1, 2>, umma_gemv_kernel<1, 3>, umma_gemv_kernel<1, 8>, umma_gemv_kernel<2, 0>, umma_gemv_kernel<2, 1>, umma_gemv_kernel<2, 17>, umma_gemv_kernel<2, 33>, umma_gemv_kernel<2, 65>, umma_gemv_kernel<2, 8>,
-                       umma_gemv_kernel<4, 0>, umma_gemv_kernel<4, 1>, umma_gemv_kernel<4, 17>, umma_gemv_kernel<4, 33>, umma_gemv_kernel<4, 65>, umma_gemv_kernel<4, 5>, umma_gemv_kernel<8, 0>, umma_gemv_kernel<8, 1>, umma_gemv_kernel<8, 17>, umma_gemv_kernel<8, 33>, umma_gemv_kernel<8, 65>, umma_gemv_kernel<8, 5>}) {
-            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
-            if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(umma gemv)");
-        }
+        for (int slots : {1, 2, 4, 8})
+            for (int f = 0; f < 2 * kDPlain; f++)
+                if (const DKernel k = gemv_kernel(slots, f)) {
+                    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
+                    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(umma gemv)");
+                }
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(kDCl);
         cfg.blockDim = dim3(kDThreads);
@@ -925,11 +945,10 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = op->pdl ? 2 : 1;
-    const bool gated = op->prologue == INSG_PRO_GATED_RMSNORM && !op->x_out && resid, two = whole && p.nmat == 2;
-    auto kernel = T == 1 ? (logits ? (prep ? umma_gemv_kernel<1, 3> : umma_gemv_kernel<1, 2>) : (prep ? (two ? umma_gemv_kernel<1, 17> : resid ? umma_gemv_kernel<1, 33> : plain ? umma_gemv_kernel<1, 65> : umma_gemv_kernel<1, 1>) : gated ? umma_gemv_kernel<1, 8> : umma_gemv_kernel<1, 0>))
-                : T == 2 ? (prep ? (two ? umma_gemv_kernel<2, 17> : resid ? umma_gemv_kernel<2, 33> : plain ? umma_gemv_kernel<2, 65> : umma_gemv_kernel<2, 1>) : gated ? umma_gemv_kernel<2, 8> : umma_gemv_kernel<2, 0>)
-                : T == 4 ? (streamed ? umma_gemv_kernel<4, 5> : prep ? (two ? umma_gemv_kernel<4, 17> : resid ? umma_gemv_kernel<4, 33> : plain ? umma_gemv_kernel<4, 65> : umma_gemv_kernel<4, 1>) : umma_gemv_kernel<4, 0>)
-                         : (streamed ? umma_gemv_kernel<8, 5> : prep ? (two ? umma_gemv_kernel<8, 17> : resid ? umma_gemv_kernel<8, 33> : plain ? umma_gemv_kernel<8, 65> : umma_gemv_kernel<8, 1>) : umma_gemv_kernel<8, 0>);
+    const bool gated = op->prologue == INSG_PRO_GATED_RMSNORM && !op->x_out && resid && T <= 2;
+    const int special = logits ? kDLogits : streamed ? kDStreamed : prep && whole && p.nmat == 2 ? kDTwo : prep && resid ? kDResidual : prep && plain ? kDPlain : gated ? kDGated : 0;
+    const DKernel kernel = gemv_kernel(T, special | (prep ? kDPrepared : 0));
+    if (!kernel) return fail(INSG_E_ARG, "gemv: no such variant");
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
     return e == cudaSuccess ? INSG_OK : cuda_fail(e, "umma gemv launch");
 }
