@@ -535,9 +535,10 @@ typedef struct insg_engine_options {
     int device;                   /* CUDA device ordinal                                        */
     int persistent;               /* 0: one launch per fused operation (162 per token), replayed from a CUDA graph when
                                      use_graph is set; 1: a token step is ONE persistent cooperative launch (insg_program_*) */
-    int prefill_mma_sync;         /* 0: insg_engine_forward_tokens sends 16 or more tokens through the tcgen05 kernel in passes
-                                     of up to 256 (second copy of the weights in its tile layout); 1: always passes of four
-                                     through the mma.sync kernel */
+    int prefill_mma_sync;         /* 0: insg_engine_forward_tokens sends more than eight tokens through the tcgen05 GEMM in
+                                     passes of up to 1024 (an engine on the mma.sync kernel 16 or more, with a second copy
+                                     of the weights); 1: always passes of eight through the tcgen05 GEMV, of four through
+                                     the mma.sync kernel */
     int gemv_unprepared;          /* 0: a GEMV that writes the residual stream or the SwiGLU output leaves the next
                                      GEMV's input prepared (insg_gemv_segment.prep); 1: every GEMV converts its own */
 } insg_engine_options;
@@ -551,9 +552,9 @@ INSG_API int insg_engine_layer(insg_engine *e, int layer);
 /* Qwen35Decode::forward_token (src/decode.cu:21): asynchronous */
 INSG_API int insg_engine_forward_token(insg_engine *e, int token);
 /* Qwen35Decode::logits_argmax (src/decode.cu:22): synchronises, returns the token id (>=0) */
-/* Additive: insg_engine_forward_token for `count` consecutive tokens (host array), four tokens per pass over the
- * weights; same resulting state, logits and arg-max of the last token.  No reference counterpart (its prompt loop is
- * src/generate_ids.cu:4). */
+/* Additive: insg_engine_forward_token for `count` consecutive tokens (host array), in passes of up to 1024 tokens over the
+ * weights (prefill_mma_sync); same resulting state, logits and arg-max of the last token.  No reference counterpart (its
+ * prompt loop is src/generate_ids.cu:4). */
 INSG_API int insg_engine_forward_tokens(insg_engine *e, const int *tokens /* host */, int count);
 INSG_API int insg_engine_logits_argmax(insg_engine *e);
 /* Qwen35Decode::decode_token (src/decode.cu:23): synchronises, returns the token id (>=0) */

@@ -20,7 +20,7 @@
 //   umma_digitize_kernel  one CTA or more per token: the fused activation prologue (RMSNorm, gates, ...), then the digit
 //                         image of the token in global memory, laid out as the shared-memory image the MMA reads
 //                         ([k-block][group of tokens][448 bytes x tokens per group, scale blocks], canonical K-major, no swizzle);
-//   umma_gemm_kernel      one CTA per SM, from 49 tokens on two that work together.  The work is the sequence of all (pair of records, token group, k-block) stages;
+//   umma_gemm_kernel      one CTA per SM; with groups of 32 tokens (tokens_per_group) two work together.  The work is the sequence of all (pair of records, token group, k-block) stages;
 //                         every CTA takes an equal contiguous share of it (stream-K), so SMs are busy whatever the number
 //                         of tiles.  The pair is two row tiles, or the gate and the up tile of the same rows for SwiGLU
 //                         (whose epilogue then has both at hand); two CTAs take twice as many tiles, each with its own

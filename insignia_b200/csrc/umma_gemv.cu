@@ -156,8 +156,9 @@ template <int T> __host__ __device__ constexpr int unit_slots(int nmat) { return
 // segment that adds into the residual stream, one unit per cluster (kDResidual; with digits that come with the weights kDStreamed, behind the
 // gated norm kDGated); epilogues that add nothing and leave nothing prepared (kDPlain).  A launch that fits none takes the general ones.
 // A token is 129 launches of some seven microseconds, and instructions that a launch runs through for the first time come from L2 behind the
-// stream of weights.  Microseconds of a token, a step of three sequences, of eight, and a speculative pass (a process is now and then 2 % off for
-// all of its life), and the code of a launch:
+// stream of weights.  Microseconds of a device-fed token (a host-fed decode_token gained half of it), a step of three sequences, of eight, and a
+// speculative pass (a process is now and then 2 % off for all of its life), and the code of a launch (the last line: of the special variants; what
+// takes a general one runs up to 82 KB):
 //   one kernel with everything in it                                                  1084 1308 1503 1500   96-125 KB
 //   variants prepared and arg-max, the waits' loops not unrolled, one store and one
 //   copy of the digits' code behind all epilogues                                     1057 1208 1412 1428   41-66

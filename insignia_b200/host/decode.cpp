@@ -27,7 +27,7 @@ constexpr int kHidden = Qwen35Shape::hidden, kInter = Qwen35Shape::intermediate;
 // the digit images of eight tokens (insg_mxfp4_digit_image_bytes); the one-token fp16 images of the mma.sync kernel are smaller.
 constexpr size_t kPrepHidden = 0, kPrepAct = size_t(kHidden / 128) * (8 * 512 + 512), kPrepCore = kPrepAct + size_t(kInter / 128) * (8 * 512 + 512),
                  kPrepSums = kPrepCore + size_t(kHidden / 128) * (8 * 512 + 512);
-constexpr int kFrontLayers = 2; // layers of the short first graph of a host-fed step: some 70 us of work, what submitting the rest takes
+constexpr int kFrontLayers = 2; // layers of the short first graph of a host-fed step: some 60 us of work (70 when it was chosen, what submitting the rest took)
 constexpr int kMultiSteps = 8; // token steps per graph in Qwen35Decode::generate
 // Qwen35Decode::forward_tokens: tokens per pass
 constexpr int kChunk = 4;     // tokens per pass of the mma.sync kernel
