@@ -162,8 +162,7 @@ def test_speculative_decode_identical_to_reference(cuda, full_ckpt, cfg3_referen
 
 
 def test_prompt_in_passes_of_four_then_greedy_tokens_identical_to_reference(cuda, full_ckpt):
-    """The prompt through forward_tokens (four tokens per pass over the weights), then greedy decode: same ids as the
-    reference fed token by token."""
+    """The prompt through forward_tokens, then greedy decode: same ids as the reference fed token by token."""
     from insignia_b200.engine import Engine
 
     n_prompt, n_gen = 61, 48  # all 61 in one pass through the tcgen05 kernel

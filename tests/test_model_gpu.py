@@ -176,9 +176,8 @@ def test_forward_tokens_equals_token_loop(cuda, golden_ckpt, count):
 
 @pytest.mark.parametrize("count", [16, 37, 50, 300])
 def test_forward_tokens_through_tcgen05_passes(cuda, golden_ckpt, count):
-    """Prompts of 16 tokens or more go through the tcgen05 kernel in passes of up to 256 tokens (the rest in passes of
-    four; 300 tokens = a full pass, a second one of 44): the same state as the token loop to rounding, the same arg-max,
-    and decoding continues with the same tokens."""
+    """Prompts of more than eight tokens go through the tcgen05 GEMM, here in one pass each: the same state as the token loop
+    to rounding, the same arg-max, and decoding continues with the same tokens.  (Several passes: test_prompt_passes_gpu.py.)"""
     rng = np.random.default_rng(count)
     prompt = [int(t) for t in rng.integers(0, 64, count)]
     ctx = max(64, count + 8)
