@@ -489,25 +489,25 @@ template <int CL, bool SWIGLU> __device__ __forceinline__ PairSrc pair_src(const
 }
 
 // ---- tcgen05 instructions of one CTA or of a pair (issued by its first CTA) ------------------------------------------------------
-template <int CL> __device__ __forceinline__ void g_copy_scales(uint32_t taddr, uint64_t desc) // CL == 2: in both CTAs, each from its own shared memory
+template <int CL> __device__ __forceinline__ void g_copy_scales(uint32_t on, uint32_t taddr, uint64_t desc) // CL == 2: in both CTAs, each from its own shared memory
 {
-    if constexpr (CL == 1) copy_scales(taddr, desc);
-    else asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(desc) : "memory");
+    if constexpr (CL == 1) copy_scales_if(on, taddr, desc);
+    else asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %2, 0;\n@q tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;\n}" ::"r"(taddr), "l"(desc), "r"(on) : "memory");
 }
-template <int CL> __device__ __forceinline__ void g_mma(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, bool accumulate, uint32_t sa, uint32_t sb)
+template <int CL> __device__ __forceinline__ void g_mma(uint32_t on, uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, bool accumulate, uint32_t sa, uint32_t sb)
 {
-    if constexpr (CL == 1) mma_step(d, da, db, idesc, accumulate, sa, sb);
+    if constexpr (CL == 1) mma_step_if(on, d, da, db, idesc, accumulate, sa, sb);
     else
-        asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %4, 0;\n"
-                     "tcgen05.mma.cta_group::2.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%5], [%6], q;\n}"
-                     ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"(uint32_t(accumulate)), "r"(sa), "r"(sb) : "memory");
+        asm volatile("{\n.reg .pred q, r;\nsetp.ne.b32 q, %4, 0;\nsetp.ne.b32 r, %7, 0;\n"
+                     "@r tcgen05.mma.cta_group::2.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%5], [%6], q;\n}"
+                     ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"(uint32_t(accumulate)), "r"(sa), "r"(sb), "r"(on) : "memory");
 }
-template <int CL> __device__ __forceinline__ void g_commit(uint64_t *bar) // CL == 2: arrives at both CTAs' barrier
+template <int CL> __device__ __forceinline__ void g_commit(uint32_t on, uint64_t *bar) // CL == 2: arrives at both CTAs' barrier
 {
-    if constexpr (CL == 1) commit_to(bar);
+    if constexpr (CL == 1) commit_if(on, bar);
     else
-        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                     ::"r"(smem_u32(bar)), "h"(uint16_t(3)) : "memory");
+        asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %2, 0;\n@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n}"
+                     ::"r"(smem_u32(bar)), "h"(uint16_t(3)), "r"(on) : "memory");
 }
 // Arrival at a barrier of the pair's first CTA: what this CTA's copies brought, or that its sums have been taken out of tensor memory.  A
 // release of everything, global memory included, waited some 800 cycles a stage; restricted to shared memory, with the issuer's waits acquiring
@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
         // ---- MMA issuer --------------------------------------------------------------------------------------------------
         // The whole warp walks the loop and one elected lane issues (see umma_gemv.cu: operands in uniform registers); the next
         // stage's barriers are polled before this stage's multiplies go out.
-        const bool one = elect_one();
+        const uint32_t one = elect_one();
         // E2M1 x E2M1, UE8M0 scales, N columns, M = 128 rows a CTA; K-step s of a block uses scale bytes 2s, 2s+1 of both operands
         constexpr uint32_t idesc0 = (1u << 7) | (1u << 10) | ((uint32_t(N) >> 3) << 17) | (1u << 23) | (uint32_t(128 * CL >> 4) << 24);
         constexpr uint32_t idesc1 = idesc0 | (2u << 29) | (2u << 4);
@@ -667,7 +667,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
         const uint32_t d0 = tmem, d1 = tmem + kD1Col;
         int st = 0, sfa = 0;
         uint32_t phase = 0;
-        bool ok = true;
+        bool ok = true, here = g_test<CL>(&full[0], 0);
         int g = begin;
         for (int run = 0; g < end && ok; run++) {
             const GRun r = run_at(p, g, end);
@@ -677,29 +677,30 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
             if (!ok) break;
 #pragma unroll 1
             for (int k = 0; k < r.len; k++) {
-                // (Two or four stages behind one look at their barriers, in straight-line code: no faster.)
-                if (!__all_sync(0xffffffffu, g_test<CL>(&full[st], phase)) && !__all_sync(0xffffffffu, g_wait<CL>(&full[st], phase, abort_flag))) { ok = false; break; }
+                // (Two or four stages behind one look at their barriers, in straight-line code: no faster.  Without the early look at the next stage's
+                // 40 tokens of 24576 x 4096 take 24.3 us instead of 23.5, 61 of 12352 x 4096 20.9 instead of 20.1; large products the same.)
+                if (!__all_sync(0xffffffffu, here) && !__all_sync(0xffffffffu, g_wait<CL>(&full[st], phase, abort_flag))) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t off = uint64_t(uint32_t(st) * uint32_t(kGStage >> 4));
                 const uint64_t da = da0 + off, dsf = dsf0 + off, db = da + uint64_t((2 * kURec) >> 4);
                 const uint32_t sa = tmem + kSfaCol + 8 * sfa, sb = tmem + kSfbCol + 8 * sfa;
                 uint64_t *back = &empty[st];
                 if (++st == S) { st = 0; phase ^= 1; }
-                if (one) {
-                    g_copy_scales<CL>(sa, dsf);
-                    if (two) g_copy_scales<CL>(sa + 4, dsf + (kURec >> 4));
-                    const uint64_t dsb = dsf + uint64_t((2 * kURec - 8192 + kBDig) >> 4); // 128 columns' scales per copy
-                    g_copy_scales<CL>(sb, dsb);
-                    if (N > 128) g_copy_scales<CL>(sb + 4, dsb + 32);
-                    g_mma<CL>(d0, da, db, idesc0, k > 0, sa, sb); // the run's first MMA overwrites
-                    if (two) g_mma<CL>(d1, da + (kURec >> 4), db, idesc0, k > 0, sa + 4, sb);
-                    g_mma<CL>(d0, da + 256, db + (kBDig >> 5), idesc1, true, sa, sb);
-                    if (two) g_mma<CL>(d1, da + (kURec >> 4) + 256, db + (kBDig >> 5), idesc1, true, sa + 4, sb);
-                    g_commit<CL>(back);
-                }
+                here = g_test<CL>(&full[st], phase);
+                const uint32_t second = two ? one : 0u;
+                g_copy_scales<CL>(one, sa, dsf);
+                g_copy_scales<CL>(second, sa + 4, dsf + (kURec >> 4));
+                const uint64_t dsb = dsf + uint64_t((2 * kURec - 8192 + kBDig) >> 4); // 128 columns' scales per copy
+                g_copy_scales<CL>(one, sb, dsb);
+                if (N > 128) g_copy_scales<CL>(one, sb + 4, dsb + 32);
+                g_mma<CL>(one, d0, da, db, idesc0, k > 0, sa, sb); // the run's first MMA overwrites
+                g_mma<CL>(second, d1, da + (kURec >> 4), db, idesc0, k > 0, sa + 4, sb);
+                g_mma<CL>(one, d0, da + 256, db + (kBDig >> 5), idesc1, true, sa, sb);
+                g_mma<CL>(second, d1, da + (kURec >> 4) + 256, db + (kBDig >> 5), idesc1, true, sa + 4, sb);
+                g_commit<CL>(one, back);
                 sfa = (sfa + 1) & (kGSfaBufs - 1);
             }
-            if (ok && one) g_commit<CL>(&dfull);
+            if (ok) g_commit<CL>(one, &dfull);
             g += r.len;
         }
     } else if (warp < 4) {

@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         // which is more than a stage of weights takes to arrive.  Descriptors advance by adding to their address field, and
         // the next stage's barrier is polled before this stage's multiplies are issued.
         if (len > 0 && nruns > 0) {
-            const bool one = elect_one();
+            const uint32_t one = elect_one();
             // E2M1 x E2M1, UE8M0 scales, N columns, M = 128; K-step s of a block uses scale bytes 2s, 2s+1 of both operands
             constexpr uint32_t idesc0 = (1u << 7) | (1u << 10) | ((uint32_t(N) >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
             constexpr uint32_t idesc1 = idesc0 | (2u << 29) | (2u << 4);
@@ -451,21 +451,19 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                     if (++st == S) { st = 0; phase ^= 1; }
                     here = mbar_test(&full[st], phase);
                     if (kb + 2 >= len) room = mbar_test(&dempty[buf ^ 1], (((run + 1) >> 1) & 1) ^ 1);
-                    if (one) {
-                        if (first) { // the digits' scales stay in tensor memory for all tiles
-                            copy_scales(sb, dsb);
-                            if (two) copy_scales(sb + 4, dsb + (kImg >> 4));
-                        }
-                        copy_scales(sa, dsf);
-                        if (two) copy_scales(sa + 4, dsf + (kURec >> 4));
-                        mma_step(dcol, da, db, idesc0, kb > 0, sa, sb);
-                        mma_step(dcol, da + 256, db + (kBKb >> 5), idesc1, true, sa, sb);
-                        if (two) {
-                            mma_step(dcol, da + (kURec >> 4), db + (kImg >> 4), idesc0, true, sa + 4, sb + 4);
-                            mma_step(dcol, da + (kURec >> 4) + 256, db + (kImg >> 4) + (kBKb >> 5), idesc1, true, sa + 4, sb + 4);
-                        }
-                        commit_to(&empty[cur]);
+                    if (first) { // the digits' scales stay in tensor memory for all tiles
+                        copy_scales_if(one, sb, dsb);
+                        if (two) copy_scales_if(one, sb + 4, dsb + (kImg >> 4));
                     }
+                    copy_scales_if(one, sa, dsf);
+                    if (two) copy_scales_if(one, sa + 4, dsf + (kURec >> 4));
+                    mma_step_if(one, dcol, da, db, idesc0, kb > 0, sa, sb);
+                    mma_step_if(one, dcol, da + 256, db + (kBKb >> 5), idesc1, true, sa, sb);
+                    if (two) {
+                        mma_step_if(one, dcol, da + (kURec >> 4), db + (kImg >> 4), idesc0, true, sa + 4, sb + 4);
+                        mma_step_if(one, dcol, da + (kURec >> 4) + 256, db + (kImg >> 4) + (kBKb >> 5), idesc1, true, sa + 4, sb + 4);
+                    }
+                    commit_if(one, &empty[cur]);
                     if (!streamed) db += 2 * (kImg >> 4);
                     sb += 8;
                     sfa = (sfa + 1) & 3;
@@ -483,7 +481,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 }
                 if constexpr (!even)
                     if (ok && evens < len) ok = stage(evens, yes, no); // the digits' scales once more: no copy of the code for a rare case
-                if (ok && one) commit_to(&dfull[buf]);
+                if (ok) commit_if(one, &dfull[buf]);
             }
         }
     } else if (warp < 4) {
