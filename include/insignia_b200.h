@@ -217,7 +217,8 @@ typedef struct insg_gemv_op {
     int *position_inout;
     int layout;               /* weight layout of every segment: 0 = insg_mxfp4_repack records, 1 = insg_mxfp4_repack_umma   */
     int *error_flag;          /* set to 1 if a bounded wait inside the kernel ran out (device int), or NULL                 */
-    int pdl;                  /* 1: launch with programmatic dependent launch          */
+    int pdl;                  /* 1: launch with programmatic dependent launch; 2: and the launch after this one is
+                                 insg_deltanet_gated_step (layout 1, INSG_PRO_PREPARED, up to eight tokens)          */
     const float *prep_partials; /* INSG_PRO_PREPARED: the producer's prep_partials (layout 0: [296], layout 1:
                                    [tokens][cols / 32]), or NULL                                                         */
     int prep_rms;               /* INSG_PRO_PREPARED: 1 = scale by the RMS factor computed from prep_partials (layout 1
@@ -323,6 +324,20 @@ INSG_API int insg_deltanet_decode_verify(const float *state, float *state_first,
 INSG_API int insg_deltanet_decode_gated(float *state, long long state_stride, const float *q16, const float *k16, const float *v32,
                                         const float *g32, const float *beta32, float *out32, int sequences, int qkv_stride,
                                         const float *z, const uint16_t *norm_w, void *image, int pdl, insg_stream_t stream);
+/* One step together with the product its output is gated with, in one launch: z = gate's product (layout 1,
+ * INSG_PRO_PREPARED, one token, one INSG_EPI_STORE segment of 4096 rows, cols % 1024 == 0), the step as insg_deltanet_decode,
+ * then image as insg_deltanet_decode_gated leaves it for one sequence, all with the bits of insg_gemv_fused, insg_deltanet_decode
+ * and the INSG_PRO_GATED_RMSNORM prologue.  With gate->pdl the product is made ahead of the wait for the launch before this
+ * one: that launch must be an insg_gemv_fused with pdl = 2 (it makes q, k, v, g and beta), and must not write gate's input.
+ * Where the GPU cannot hold the 32 clusters of four CTAs at once the product and insg_deltanet_decode_gated run one after the other. */
+typedef struct insg_delta_op {
+    float *state;             /* fp32 [32][128][128], in place */
+    const float *q16, *k16, *v32, *g32, *beta32;
+    float *out32;             /* fp32 [4096] */
+    const uint16_t *norm_w;   /* bf16 [128] */
+    void *image;              /* insg_mxfp4_digit_image_bytes(4096, 1) bytes */
+} insg_delta_op;
+INSG_API int insg_deltanet_gated_step(const insg_gemv_op *gate /* host */, const insg_delta_op *step /* host */, insg_stream_t stream);
 /* Convolution history [channels][3] after a rejected second token: from the history after two tokens (`state`, in
  * place) and the history before them (`snapshot`).  No reference counterpart. */
 INSG_API int insg_conv_rollback(float *state, const float *snapshot, long long channels, insg_stream_t stream);

@@ -28,6 +28,10 @@ class GemvOp(C.Structure):
                 ("prep_partials", vp), ("prep_rms", i32), ("tokens", i32), ("umma_scratch", vp), ("umma_scratch_bytes", sz), ("host_result", vp)]
 
 
+class DeltaOp(C.Structure):
+    _fields_ = [(n, vp) for n in ("state", "q16", "k16", "v32", "g32", "beta32", "out32", "norm_w", "image")]
+
+
 class AttnOp(C.Structure):
     _fields_ = [("qraw", vp), ("k_raw", vp), ("v", vp), ("q_norm_w", vp), ("k_norm_w", vp), ("k_cache", vp),
                 ("v_cache", vp), ("out", vp), ("position", vp), ("position_offset", i32), ("max_context", i32),
@@ -83,6 +87,7 @@ SIGNATURES = {
     "insg_deltanet_decode_batch": (i32, [vp, C.c_longlong, vp, vp, vp, vp, vp, vp, i32, i32, i32, vp]),
     "insg_deltanet_decode_verify": (i32, [vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, vp]),
     "insg_deltanet_decode_gated": (i32, [vp, C.c_longlong] + [vp] * 6 + [i32, i32, vp, vp, vp, i32, vp]),
+    "insg_deltanet_gated_step": (i32, [C.POINTER(GemvOp), C.POINTER(DeltaOp), vp]),
     "insg_conv_rollback": (i32, [vp, vp, C.c_longlong, vp]),
     "insg_gqa_scratch_bytes": (sz, [i32]),
     "insg_gqa_decode": (i32, [vp, vp, vp, vp, i32, i32, vp, sz, vp]),

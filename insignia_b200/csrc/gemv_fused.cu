@@ -93,7 +93,7 @@ template <int UNR, int M> int launch_variant(const GemvParams &p, int grid, size
 
 } // namespace
 
-int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st);
+int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st, const insg_delta_op *step);
 int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st);
 
 // Validates a fused-GEMV description and turns it into the kernel's parameter block for a grid of at most `max_grid`
@@ -203,7 +203,7 @@ size_t insg_gemv_argmax_scratch_bytes(void) { return 64 + size_t(8) * 512; }
 
 int insg_gemv_fused(const insg_gemv_op *op, insg_stream_t stream)
 {
-    if (op && op->layout == 1) return op->tokens > 8 ? gemm_umma_launch(op, stream) : gemv_umma_launch(op, stream);
+    if (op && op->layout == 1) return op->tokens > 8 ? gemm_umma_launch(op, stream) : gemv_umma_launch(op, stream, nullptr);
     return gemv_fused_launch(op, op && op->tokens > 1 ? op->tokens : 1, stream);
 }
 

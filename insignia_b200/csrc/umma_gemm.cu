@@ -896,7 +896,7 @@ size_t umma_gemm_scratch(int cols, int tokens)
     return image_bytes(cols, tokens) + kPartialBytes + kGMaxGrid * sizeof(int);
 }
 
-int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st); // 1..8 tokens (umma_gemv.cu)
+int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st, const insg_delta_op *step); // 1..8 tokens (umma_gemv.cu)
 
 int gemm_umma_launch(const insg_gemv_op *op, cudaStream_t st)
 {
@@ -1039,7 +1039,7 @@ int insg_mxfp4_gemm_umma(const void *packed_umma, const float *x, float *y, int 
     op.umma_scratch = scratch;
     op.umma_scratch_bytes = scratch_bytes;
     if (M < 1) return fail(INSG_E_SHAPE, "gemm: 1 <= tokens <= 4096");
-    return M <= 8 ? gemv_umma_launch(&op, stream) : gemm_umma_launch(&op, stream);
+    return M <= 8 ? gemv_umma_launch(&op, stream, nullptr) : gemm_umma_launch(&op, stream);
 }
 
 } // extern "C"

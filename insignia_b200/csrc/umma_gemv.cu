@@ -71,6 +71,15 @@ struct DSeg {
     int tile_begin, epilogue, rows;
 };
 
+// The DeltaNet step a launch makes beside the product its output is gated with (kDDelta).
+struct DDelta {
+    float *state;
+    const float *q, *k, *v, *g, *beta;
+    float *out;
+    const uint16_t *norm_w;
+    uint8_t *image;
+};
+
 struct DParams {
     const float *in, *aux;
     const uint16_t *norm_w;
@@ -78,6 +87,8 @@ struct DParams {
     const float *prep_partials; // prepared input: the producer's sums of squares, or null
     int cols, nkb, prologue, nseg, units, nmat, tokens, stages;
     int ahead; // stages beyond the ring to ask L2 for
+    int late;  // the next launch reads what was there before this one: it may start when this launch's own wait is over
+    DDelta delta;
     DSeg seg[4];
     float2 *argmax_partial;
     unsigned *argmax_ticket;
@@ -154,7 +165,8 @@ template <int T> __host__ __device__ constexpr int unit_slots(int nmat) { return
 
 // What a variant of the kernel has beside its tokens: a prepared input in place of the prologue; the logits' arg-max; two matrices (SwiGLU); one
 // segment that adds into the residual stream, one unit per cluster (kDResidual; with digits that come with the weights kDStreamed, behind the
-// gated norm kDGated); epilogues that add nothing and leave nothing prepared (kDPlain).  A launch that fits none takes the general ones.
+// gated norm kDGated); epilogues that add nothing and leave nothing prepared (kDPlain); a DeltaNet step beside the product that gates its output
+// (kDDelta).  A launch that fits none takes the general ones.
 // A token is 129 launches of some seven microseconds, and instructions that a launch runs through for the first time come from L2 behind the
 // stream of weights.  Microseconds of a device-fed token (a host-fed decode_token gained half of it), a step of three sequences, of eight, and a
 // speculative pass (a process is now and then 2 % off for all of its life), and the code of a launch (the last line: of the special variants; what
@@ -165,7 +177,110 @@ template <int T> __host__ __device__ constexpr int unit_slots(int nmat) { return
 //   and two matrices, the gated norm, residual                                        1057 1170 1348 1387   28-48
 //   and plain; no later runs, last odd block or slot reuse where there are none       1031 1156 1330 1365   20-37
 // (20 KB more in the issuer's loop, never run, cost a token 80 us.)
-constexpr int kDPrepared = 1, kDLogits = 2, kDStreamed = 4, kDGated = 8, kDTwo = 16, kDResidual = 32, kDPlain = 64;
+constexpr int kDPrepared = 1, kDLogits = 2, kDStreamed = 4, kDGated = 8, kDTwo = 16, kDResidual = 32, kDPlain = 64, kDDelta = 128;
+
+// One DeltaNet step of 32 columns of a head by the first eight warps of a CTA, whose cluster has the head: the arithmetic, and the order of every
+// sum, of deltanet_step_kernel and of the gated prologue, so that their bits are the same.  cell: rows kr + 32 j of the state, four columns.
+// The step waits for the in-projection, a chain of latencies that leaves the memory and the tensor cores idle, and its gate z is not wanted before
+// its end: z's rows of the in-projection (a tile a head, so that a cluster's four CTAs have their columns' gates at hand) are multiplied here,
+// from the input that the launch before the in-projection left.  The in-projection then has two units a cluster and not three, and the out
+// projection takes digits and not the gated norm: a device-fed token 1010 -> 994 us.
+struct DeltaShared {
+    float qk[8][2][128]; // per warp: its own copy of the normalised q and k
+    float part[2][8][32];
+    float squares[32];   // of the head's output, four columns each
+    float z[32];         // what gates this CTA's columns
+};
+__device__ __forceinline__ void delta_step(const DDelta &d, float4 (&cell)[4], DeltaShared &sh, int head, int slice, uint64_t *bar, volatile int *abort_flag, const uint8_t *lut,
+                                           int tid)
+{
+    const int lane = tid & 31, warp = tid >> 5, kh = head >> 1, vq = tid & 7, kr = tid >> 3, v0 = slice * 32 + vq * 4;
+    const float gw = warp == 0 ? bf16_bits_to_float(d.norm_w[slice * 32 + lane]) : 0.f;
+    pdl_wait();
+    const float4 q4 = __ldcg(reinterpret_cast<const float4 *>(d.q + kh * 128) + lane);
+    const float4 k4 = __ldcg(reinterpret_cast<const float4 *>(d.k + kh * 128) + lane);
+    const float4 v4 = __ldcg(reinterpret_cast<const float4 *>(d.v + head * 128 + slice * 32) + vq);
+    const float g_in = __ldcg(d.g + head), beta = __ldcg(d.beta + head);
+    const float qn = warp_sum(fmaf(q4.x, q4.x, fmaf(q4.y, q4.y, fmaf(q4.z, q4.z, q4.w * q4.w))));
+    const float kn = warp_sum(fmaf(k4.x, k4.x, fmaf(k4.y, k4.y, fmaf(k4.z, k4.z, k4.w * k4.w))));
+    const float qs = rsqrtf(qn + 1e-6f) * 0.08838834764831845f, ks = rsqrtf(kn + 1e-6f);
+    reinterpret_cast<float4 *>(sh.qk[warp][0])[lane] = make_float4(q4.x * qs, q4.y * qs, q4.z * qs, q4.w * qs);
+    reinterpret_cast<float4 *>(sh.qk[warp][1])[lane] = make_float4(k4.x * ks, k4.y * ks, k4.z * ks, k4.w * ks);
+    __syncwarp();
+    float qq[4], kk[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        qq[j] = sh.qk[warp][0][kr + 32 * j];
+        kk[j] = sh.qk[warp][1][kr + 32 * j];
+    }
+    const float decay = expf(g_in);
+    float4 pm = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        pm.x = fmaf(cell[j].x, kk[j], pm.x);
+        pm.y = fmaf(cell[j].y, kk[j], pm.y);
+        pm.z = fmaf(cell[j].z, kk[j], pm.z);
+        pm.w = fmaf(cell[j].w, kk[j], pm.w);
+    }
+#pragma unroll
+    for (int m = 16; m >= 8; m >>= 1) {
+        pm.x += __shfl_xor_sync(0xffffffffu, pm.x, m);
+        pm.y += __shfl_xor_sync(0xffffffffu, pm.y, m);
+        pm.z += __shfl_xor_sync(0xffffffffu, pm.z, m);
+        pm.w += __shfl_xor_sync(0xffffffffu, pm.w, m);
+    }
+    if (lane < 8) *reinterpret_cast<float4 *>(&sh.part[0][warp][lane * 4]) = pm;
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    float4 t[8];
+#pragma unroll
+    for (int w = 0; w < 8; w++) t[w] = *reinterpret_cast<const float4 *>(&sh.part[0][w][vq * 4]);
+#pragma unroll
+    for (int n = 1; n < 8; n <<= 1) // pairs of warps, then of pairs
+#pragma unroll
+        for (int w = 0; w < 8; w += 2 * n) { t[w].x += t[w + n].x; t[w].y += t[w + n].y; t[w].z += t[w + n].z; t[w].w += t[w + n].w; }
+    const float4 dl = make_float4(fmaf(-t[0].x, decay, v4.x) * beta, fmaf(-t[0].y, decay, v4.y) * beta, fmaf(-t[0].z, decay, v4.z) * beta,
+                                  fmaf(-t[0].w, decay, v4.w) * beta);
+    float *S = d.state + size_t(head) * 128 * 128;
+    float4 po = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        cell[j].x = fmaf(kk[j], dl.x, cell[j].x * decay);
+        cell[j].y = fmaf(kk[j], dl.y, cell[j].y * decay);
+        cell[j].z = fmaf(kk[j], dl.z, cell[j].z * decay);
+        cell[j].w = fmaf(kk[j], dl.w, cell[j].w * decay);
+        po.x = fmaf(cell[j].x, qq[j], po.x);
+        po.y = fmaf(cell[j].y, qq[j], po.y);
+        po.z = fmaf(cell[j].z, qq[j], po.z);
+        po.w = fmaf(cell[j].w, qq[j], po.w);
+        *reinterpret_cast<float4 *>(S + size_t(kr + 32 * j) * 128 + v0) = cell[j];
+    }
+#pragma unroll
+    for (int m = 16; m >= 8; m >>= 1) {
+        po.x += __shfl_xor_sync(0xffffffffu, po.x, m);
+        po.y += __shfl_xor_sync(0xffffffffu, po.y, m);
+        po.z += __shfl_xor_sync(0xffffffffu, po.z, m);
+        po.w += __shfl_xor_sync(0xffffffffu, po.w, m);
+    }
+    if (lane < 8) *reinterpret_cast<float4 *>(&sh.part[1][warp][lane * 4]) = po;
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    if (warp != 0) return;
+    float w8[8];
+#pragma unroll
+    for (int w = 0; w < 8; w++) w8[w] = sh.part[1][w][lane];
+    const float o = ((w8[0] + w8[1]) + (w8[2] + w8[3])) + ((w8[4] + w8[5]) + (w8[6] + w8[7]));
+    // The head's sum of squares: four columns a term, the terms of the four slices exchanged, then the sum over the 32 lanes that the prologue takes.
+    float ss[1];
+    {
+        const float x = __shfl_sync(0xffffffffu, o, (lane & 7) * 4), y = __shfl_sync(0xffffffffu, o, (lane & 7) * 4 + 1);
+        const float u = __shfl_sync(0xffffffffu, o, (lane & 7) * 4 + 2), v = __shfl_sync(0xffffffffu, o, (lane & 7) * 4 + 3);
+        ss[0] = fmaf(x, x, fmaf(y, y, fmaf(u, u, v * v)));
+    }
+    send_floats<1>(map_to_rank(smem_u32(&sh.squares[slice * 8 + (lane & 7)]), uint32_t(lane >> 3)), ss, map_to_rank(smem_u32(bar), uint32_t(lane >> 3)));
+    d.out[head * 128 + slice * 32 + lane] = o;
+    __all_sync(0xffffffffu, mbar_wait_cluster(bar, 0, abort_flag));
+    const float inv = rsqrtf(warp_sum(sh.squares[lane]) / 128.f + 1e-6f);
+    group_digits(o * inv * gw * fast_silu(sh.z[lane]), 1, 0, d.image, head * 4 + slice, lut, lane);
+}
 
 template <int T, int F>
 __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_constant__ DParams p)
@@ -189,19 +304,23 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     __shared__ uint8_t s_lut[84];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    constexpr bool residual = (F & (kDResidual | kDStreamed | kDGated)) != 0, single = residual; // one segment, added into the residual stream, one unit per cluster
+    constexpr bool residual = (F & (kDResidual | kDStreamed | kDGated)) != 0; // one segment, added into the residual stream, one unit per cluster
+    constexpr bool delta = (F & kDDelta) != 0, single = residual || delta;   // one segment, one unit per cluster
+    static_assert(!delta || (prepared && T == 1), "the step's product takes one token's prepared input");
     constexpr bool plain = (F & kDPlain) != 0;                       // nothing is left prepared
-    constexpr bool even = residual || plain || (F & kDTwo) != 0;     // every CTA has an even number of k-blocks
+    constexpr bool even = single || plain || (F & kDTwo) != 0;     // every CTA has an even number of k-blocks
     const int rank = int(blockIdx.x) & (kDCl - 1), cl = int(blockIdx.x) / kDCl, C = int(gridDim.x) / kDCl;
-    const int nkb = p.nkb, S = p.stages, nmat = (F & kDTwo) != 0 ? 2 : (F & (kDResidual | kDStreamed | kDGated | kDPlain)) != 0 ? 1 : p.nmat, XU = unit_slots<T>(nmat);
+    const int nkb = p.nkb, S = p.stages, nmat = (F & kDTwo) != 0 ? 2 : (F & (kDResidual | kDStreamed | kDGated | kDPlain | kDDelta)) != 0 ? 1 : p.nmat, XU = unit_slots<T>(nmat);
     const int kb0 = (nkb * rank) >> 2, len = ((nkb * (rank + 1)) >> 2) - kb0; // this CTA's k-blocks
     const int spt = (len + 1) >> 1;                                            // ring stages per (tile, matrix)
-    const int nun = residual ? 1 : cl < p.units ? (p.units - cl + C - 1) / C : 0;             // units of this cluster: cl, cl + C, ...
+    const int nun = single ? 1 : cl < p.units ? (p.units - cl + C - 1) / C : 0;             // units of this cluster: cl, cl + C, ...
     const int nruns = nun * nmat, nstages = nruns * spt;
     uint8_t *ring = smem;                                // S stages
     uint8_t *bimg = ring + size_t(S) * kStage; // len x kImg bytes, unless streamed
     float *xslot = reinterpret_cast<float *>(bimg + (streamed ? 0 : size_t((nkb + 3) >> 2) * kImg)); // XU * nmat exchange slots
     float *s_ssq = T < 8 ? s_ssq_static : xslot + XU * nmat * kSlot; // [token][k-block], unless the input is prepared
+
+    DeltaShared &s_delta = *reinterpret_cast<DeltaShared *>(xslot + XU * nmat * kSlot); // of a launch with a step
 
     auto seg_of = [&](int unit) -> const DSeg & { return p.seg[single ? 0 : dseg_of(p, unit)]; };
     // ---- the weight stream starts first: it depends on nothing ----------------------------------------------------------
@@ -226,7 +345,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         if (lane < S && lane < nstages) {
-            const int run = residual ? 0 : lane / spt;
+            const int run = single ? 0 : lane / spt;
             load_stage(lane, run_src(run), lane - run * spt);
         }
     } else if (warp == 8) {
@@ -242,7 +361,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         else if (lane == 31) {
             mbar_init(&ssfull, 1);
             s_abort = 0;
-            mbar_expect_tx(&ssfull, kDCl * T * 4);
+            mbar_expect_tx(&ssfull, delta ? kDCl * 8 * 4 : kDCl * T * 4);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     } else if (tid >= 128 && tid < 128 + 81) {
@@ -251,9 +370,11 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // (late: the next launch reads the input of this one ahead of its own wait.  It may start when this launch has seen that input, in the producer.)
     // The next launch may become resident from here on, not earlier: were it to take tensor memory before every CTA here has its own,
     // a CTA could wait for memory held by a CTA that waits for this grid.
-    if (nstages - kDTriggerStages<T> <= S) pdl_launch_dependents();
+    const bool at_once = nstages - kDTriggerStages<T> <= S;
+    if (at_once && !(prepared && p.late)) pdl_launch_dependents();
     // The peers' barriers exist when this completes.  Their initialisation is published by the fences above; a release here waited for
     // whatever the SM still had under way, up to 2 us in a launch that could not start beside its predecessor (eight tokens 1540 -> 1503 us
     // a step, one token 1098 -> 1084).
@@ -263,8 +384,16 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     volatile int *abort_flag = &s_abort;
     bool arrived = false; // at the closing cluster barrier
 
+    float4 cell[delta ? 4 : 1]; // this thread's part of the state, last written a token ago
+    if constexpr (delta) {
+        if (warp < 8) {
+            const float *S = p.delta.state + size_t(cl) * 128 * 128 + size_t(tid >> 3) * 128 + rank * 32 + (tid & 7) * 4;
+#pragma unroll
+            for (int j = 0; j < 4; j++) cell[j] = __ldcg(reinterpret_cast<const float4 *>(S + size_t(32 * j) * 128));
+        }
+    }
     if constexpr (prepared) {
-        if (warp >= 4 && warp < 8) pdl_wait(); // they read what earlier launches wrote
+        if (!delta && warp >= 4 && warp < 8) pdl_wait(); // they read what earlier launches wrote
     } else if (warp < 8) {
         // ---- activation prologue: this CTA's quarter of the columns ---------------------------------------------------------
         constexpr int kBatch = (F & kDGated) != 0 ? 1 : 3;
@@ -369,14 +498,15 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             const bool one = elect_one();
             if constexpr (kDAheadStages<T> > 0) {
                 for (int i = S + lane; i < min(nstages, S + p.ahead); i += 32) {
-                    const int run = residual ? 0 : i / spt, st = i - run * spt;
+                    const int run = single ? 0 : i / spt, st = i - run * spt;
                     bulk_prefetch(run_src(run) + size_t(st) * kDStage, uint32_t(min(2, len - 2 * st)) * kURec);
                 }
                 __syncwarp();
             }
             if constexpr (prepared) { // the digits come ready: eight k-blocks per copy, so that the multiplies can start behind the first
-                pdl_wait();
-                asm volatile("fence.proxy.async.global;" ::: "memory"); // written by ordinary stores of the launch before
+                if (!delta) pdl_wait(); // (delta: they were there when the launch before this one let it start)
+                if (at_once && p.late) pdl_launch_dependents();
+                asm volatile("fence.proxy.async.global;" ::: "memory"); // written by ordinary stores of an earlier launch
                 if constexpr (streamed) {
                     if (lane < S && lane < nstages) load_digits(lane, lane);
                     __syncwarp();
@@ -472,7 +602,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 constexpr std::true_type yes{};
                 constexpr std::false_type no{};
                 const int evens = len & ~1;
-                if (residual || run == 0) {
+                if (single || run == 0) {
 #pragma unroll 1
                     for (int kb = 0; kb < evens && ok; kb += 2) ok = stage(kb, yes, yes);
                 } else {
@@ -506,7 +636,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                 if (lane == 0) mbar_arrive(&dempty[buf]);
             }
             const int slot = run % nslots;
-            if (!residual && run >= nslots) { // the slot's previous content must have been added up by its owner
+            if (!single && run >= nslots) { // the slot's previous content must have been added up by its owner
                 ok = __all_sync(0xffffffffu, mbar_wait_cluster(&xempty[slot], ((run / nslots) - 1) & 1, abort_flag));
                 if (!ok) break;
             }
@@ -555,7 +685,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             const int unit = cl + i * C;
             const DSeg &s = seg_of(unit);
             const int row = (unit - s.tile_begin) * 128 + rank * 32 + lane;
-            if ((F & kDTwo) != 0 || row >= s.rows) return;
+            if ((F & kDTwo) != 0 || delta || row >= s.rows) return;
             if (!residual && s.epilogue == INSG_EPI_CONV_SILU) next.w = reinterpret_cast<const uint2 *>(s.conv_w)[row];
 #pragma unroll
             for (int u = 0; u < TN; u++) {
@@ -619,18 +749,21 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                         hist[0] = h0; hist[1] = h1; hist[2] = h2;
                     }
                 }
-                if (!residual && i + XU < nun) { // the slot will be used again: tell the four senders, whose next st.async must come after these reads
+                if (!single && i + XU < nun) { // the slot will be used again: tell the four senders, whose next st.async must come after these reads
                     __syncwarp();
                     if (lane < kDCl) remote_arrive(map_to_rank(smem_u32(&xempty[slot]), uint32_t(lane)));
                 }
             }
             if (!ok) break;
-            if (i + kGroups >= nun) { // nothing more comes in for this warp: the peers need not wait for its epilogue
+            if (!delta && i + kGroups >= nun) { // nothing more comes in for this warp: the peers need not wait for its epilogue
                 cluster_arrive_relaxed();
                 arrived = true;
             }
             if (!on) continue;
-            if constexpr (logits) {
+            if constexpr (delta) {
+                out[0] = y[0][0];
+                s_delta.z[lane] = y[0][0];
+            } else if constexpr (logits) {
                 out[0] = y[0][0];
                 if (y[0][0] > best || (y[0][0] == best && row < best_idx)) { best = y[0][0]; best_idx = row; }
             } else {
@@ -746,6 +879,8 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             }
         }
     }
+    if constexpr (delta)
+        if (warp < 8) delta_step(p.delta, cell, s_delta, cl, rank, &ssfull, abort_flag, s_lut, tid);
     // Nobody leaves while a peer may still write into its shared memory (after an expired wait too).
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -800,7 +935,7 @@ DKernel gemv_kernel(int slots, int f)
 {
     constexpr int kP = kDPrepared;
     switch (slots) {
-    case 1: return variant_of<1, 0, kP, kP | kDTwo, kP | kDResidual, kP | kDPlain, kDLogits, kP | kDLogits, kDGated>(f);
+    case 1: return variant_of<1, 0, kP, kP | kDTwo, kP | kDResidual, kP | kDPlain, kDLogits, kP | kDLogits, kDGated, kP | kDDelta>(f);
     case 2: return variant_of<2, 0, kP, kP | kDTwo, kP | kDResidual, kP | kDPlain, kDGated>(f);
     case 4: return variant_of<4, 0, kP, kP | kDTwo, kP | kDResidual, kP | kDPlain, kP | kDStreamed>(f);
     default: return variant_of<8, 0, kP, kP | kDTwo, kP | kDResidual, kP | kDPlain, kP | kDStreamed>(f);
@@ -820,7 +955,7 @@ int device_clusters(int *out)
     std::lock_guard<std::mutex> lock(g_attr_mutex);
     if (!g_max_clusters[dev]) {
         for (int slots : {1, 2, 4, 8})
-            for (int f = 0; f < 2 * kDPlain; f++)
+            for (int f = 0; f < 2 * kDDelta; f++)
                 if (const DKernel k = gemv_kernel(slots, f)) {
                     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
                     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(umma gemv)");
@@ -845,7 +980,7 @@ int device_clusters(int *out)
 }
 } // namespace
 
-int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
+int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st, const insg_delta_op *step)
 {
     if (!op || !op->in) return fail(INSG_E_ARG, "gemv: null operand");
     const int tokens = op->tokens > 1 ? op->tokens : 1;
@@ -903,6 +1038,7 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
         if (op->token_log && op->token_log_capacity <= 0) return fail(INSG_E_ARG, "gemv: token_log needs its capacity");
     }
     p.error_flag = static_cast<int *>(op->error_flag);
+    p.late = op->pdl == 2;
     int max_clusters = 0;
     const int rc = device_clusters(&max_clusters);
     if (rc != INSG_OK) return rc;
@@ -920,7 +1056,7 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     for (int i = 0; i < p.nseg; i++) plain &= p.seg[i].epilogue != INSG_EPI_RESIDUAL && p.seg[i].epilogue != INSG_EPI_SWIGLU && p.seg[i].epilogue != INSG_EPI_LOGITS;
     const bool streamed = prep && T >= 4 && resid && kbq * kblock + exchange + 4 * kDStage > size_t(kDHalfSm);
     const size_t stage_bytes = kDStage + (streamed ? 2 * kblock : 0);
-    const size_t fixed = exchange + (streamed ? 0 : kbq * kblock) + (T == 8 && !prep ? size_t(8) * kDMaxKb * sizeof(float) : 0);
+    const size_t fixed = exchange + (step ? sizeof(DeltaShared) : 0) + (streamed ? 0 : kbq * kblock) + (T == 8 && !prep ? size_t(8) * kDMaxKb * sizeof(float) : 0);
     // ring: no more stages than the launch has, within half an SM when that leaves at least four, else whatever fits.  Four are too
     // few to stream at full rate, so a launch of many units (the head: 55 per cluster, eight tokens 97 us against 91) takes the
     // whole SM; one of a few gains more from starting beside its predecessor.
@@ -944,8 +1080,12 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = op->pdl ? 2 : 1;
+    if (step) {
+        if (!prep || tokens != 1 || !whole || p.nseg != 1 || p.seg[0].epilogue != INSG_EPI_STORE || p.seg[0].rows != 4096) return fail(INSG_E_SHAPE, "deltanet: the gate's product takes one token, a prepared input and 4096 rows");
+        p.delta = DDelta{step->state, step->q16, step->k16, step->v32, step->g32, step->beta32, step->out32, step->norm_w, static_cast<uint8_t *>(step->image)};
+    }
     const bool gated = op->prologue == INSG_PRO_GATED_RMSNORM && !op->x_out && resid && T <= 2;
-    const int special = logits ? kDLogits : streamed ? kDStreamed : prep && whole && p.nmat == 2 ? kDTwo : prep && resid ? kDResidual : prep && plain ? kDPlain : gated ? kDGated : 0;
+    const int special = step ? kDDelta : logits ? kDLogits : streamed ? kDStreamed : prep && whole && p.nmat == 2 ? kDTwo : prep && resid ? kDResidual : prep && plain ? kDPlain : gated ? kDGated : 0;
     const DKernel kernel = gemv_kernel(T, special | (prep ? kDPrepared : 0));
     if (!kernel) return fail(INSG_E_ARG, "gemv: no such variant");
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
@@ -957,6 +1097,20 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st)
 using namespace insg;
 
 extern "C" {
+
+int insg_deltanet_gated_step(const insg_gemv_op *gate, const insg_delta_op *step, insg_stream_t stream)
+{
+    if (!gate || !step || !step->state || !step->q16 || !step->k16 || !step->v32 || !step->g32 || !step->beta32 || !step->out32 || !step->norm_w || !step->image)
+        return fail(INSG_E_ARG, "deltanet: null pointer");
+    if (gate->layout != 1) return fail(INSG_E_SHAPE, "deltanet: the gate's product takes the tcgen05 layout");
+    int clusters = 0;
+    int rc = device_clusters(&clusters);
+    if (rc == INSG_OK && clusters >= 32) return gemv_umma_launch(gate, stream, step);
+    if (rc == INSG_OK) rc = gemv_umma_launch(gate, stream, nullptr);
+    if (rc != INSG_OK) return rc;
+    return insg_deltanet_decode_gated(step->state, 32 * 128 * 128, step->q16, step->k16, step->v32, step->g32, step->beta32, step->out32, 1, 0, gate->seg[0].out, step->norm_w,
+                                      step->image, gate->pdl, stream);
+}
 
 size_t insg_mxfp4_digit_image_bytes(int cols, int tokens)
 {

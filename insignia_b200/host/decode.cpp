@@ -3,7 +3,7 @@
 //
 // Kernel sequence per token (reference: 18 launches per layer, ~580 per token):
 //   embed                                                       1
-//   DeltaNet layer : in_proj(qkv|z|a|b) + conv/SiLU/gates, delta step, out_proj+residual,
+//   DeltaNet layer : in_proj(qkv|a|b) + conv/SiLU/gates, z product + delta step + gated norm, out_proj+residual,
 //                    gate/up + SwiGLU, down + residual           5
 //   attention layer: q|k|v proj, norm/RoPE/KV store/split-K attention, o_proj(gated)+residual,
 //                    gate/up + SwiGLU, down + residual           5
@@ -269,9 +269,9 @@ uint64_t gemv_weight_bytes(const insg_gemv_op &op)
     return b;
 }
 
-void run_gemv(Ctx &c, insg_gemv_op &op)
+void run_gemv(Ctx &c, insg_gemv_op &op, const insg_delta_op *step = nullptr) // step: made in the same launch, its output gated with the product's
 {
-    op.pdl = c.pdl ? 1 : 0;
+    op.pdl = !c.pdl ? 0 : op.pdl ? op.pdl : 1;
     op.layout = c.layout >= 0 ? c.layout : (c.tcgen05() ? 1 : 0);
     op.error_flag = c.x.d_token + 3;
     if (op.layout == 1 && op.tokens > kSmallChunk) {
@@ -280,7 +280,7 @@ void run_gemv(Ctx &c, insg_gemv_op &op)
     }
     if (c.gemv_bytes) *c.gemv_bytes += gemv_weight_bytes(op);
     if (c.rec) insg_check(insg_program_add_gemv(c.rec, &op));
-    else insg_check(insg_gemv_fused(&op, c.st));
+    else insg_check(step ? insg_deltanet_gated_step(&op, step, c.st) : insg_gemv_fused(&op, c.st));
     c.launches++;
 }
 
@@ -331,30 +331,47 @@ static void enqueue_delta_block(Ctx &c, const Qwen35Decode::Plan::Block &b, int 
     DecodeWorkspace &x = c.x;
     insg_gemv_op in = {};
     rmsnorm_input(c, in, b.in_norm);
-    in.n_segments = 4;
-    in.seg[0] = seg(b.qkv, x.qkv, INSG_EPI_CONV_SILU);
-    in.seg[0].conv_state = x.conv_state + size_t(di) * 8192 * 3;
-    in.seg[0].conv_w = b.conv_w;
-    in.seg[1] = seg(b.z, x.z, INSG_EPI_STORE);
-    in.seg[2] = seg(b.a, x.a, INSG_EPI_DECAY);
-    in.seg[2].A_log = b.A_log;
-    in.seg[2].dt_bias = b.dt_bias;
-    in.seg[3] = seg(b.b, x.b, INSG_EPI_BETA);
+    // What gates the step's output is needed last: its product is made in the step's launch, where the step waits for the rest (994 us a token;
+    // 1010 with the gate's rows in the in-projection).  Not where the input comes as fp32 (the first block) or operations are recorded.
+    const bool beside = c.core_prepared() && !c.rec && in.prologue == INSG_PRO_PREPARED;
+    insg_gemv_op zp = in;
+    int n = 0;
+    in.seg[n] = seg(b.qkv, x.qkv, INSG_EPI_CONV_SILU);
+    in.seg[n].conv_state = x.conv_state + size_t(di) * 8192 * 3;
+    in.seg[n++].conv_w = b.conv_w;
+    if (!beside) in.seg[n++] = seg(b.z, x.z, INSG_EPI_STORE);
+    in.seg[n] = seg(b.a, x.a, INSG_EPI_DECAY);
+    in.seg[n].A_log = b.A_log;
+    in.seg[n++].dt_bias = b.dt_bias;
+    in.seg[n++] = seg(b.b, x.b, INSG_EPI_BETA);
+    in.n_segments = n;
+    if (beside) in.pdl = 2;
     run_gemv(c, in);
 
-    if (!c.gemv_only) {
-        float *state = x.delta_state + size_t(di) * 32 * 128 * 128;
+    float *state = x.delta_state + size_t(di) * 32 * 128 * 128;
+    if (beside) {
+        zp.n_segments = 1;
+        zp.seg[0] = seg(b.z, x.z, INSG_EPI_STORE);
+        insg_delta_op step = {};
+        step.state = state;
+        step.q16 = x.qkv; step.k16 = x.qkv + 2048; step.v32 = x.qkv + 4096;
+        step.g32 = x.a; step.beta32 = x.b;
+        step.out32 = x.core;
+        step.norm_w = b.dn_norm;
+        step.image = c.prep_core();
+        run_gemv(c, zp, &step);
+    } else if (!c.gemv_only) {
         if (c.rec) insg_check(insg_program_add_deltanet(c.rec, state, x.qkv, x.qkv + 2048, x.qkv + 4096, x.a, x.b, x.core));
         else insg_check(insg_deltanet_decode(state, x.qkv, x.qkv + 2048, x.qkv + 4096, x.a, x.b, x.core, c.pdl ? 1 : 0, c.st));
         c.launches++;
     }
 
     insg_gemv_op out = {};
-    out.in = x.core;
+    out.in = beside ? static_cast<const float *>(c.prep_core()) : x.core;
     out.aux = x.z;
     out.norm_w = b.dn_norm;
     out.cols = 4096;
-    out.prologue = INSG_PRO_GATED_RMSNORM;
+    out.prologue = beside ? INSG_PRO_PREPARED : INSG_PRO_GATED_RMSNORM;
     out.n_segments = 1;
     out.seg[0] = seg(b.out, x.hidden, INSG_EPI_RESIDUAL);
     residual_output(c, out.seg[0], b.post_norm);
