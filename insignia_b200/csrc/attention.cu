@@ -32,12 +32,19 @@ namespace insg {
 constexpr int kAtThreads = 256;
 constexpr int kAtWarps = 8;
 constexpr int kGroup = 4;                    // tokens a warp scores at once
-constexpr int kMinChunk = kAtWarps * kGroup; // tokens per split at least: one group per warp
+constexpr int kBlock = kAtWarps * kGroup;    // rows the warps of a CTA score at once
+constexpr int kMinChunk = kBlock;            // tokens per split at least
 constexpr int kMmaMinTokens = 2048;          // bf16 cache: cached rows from which the tensor-core loop is used
 constexpr int kTileRow = 528;                // a staged row: 512 bytes of bf16 + 16 of padding (conflict-free ldmatrix)
 constexpr int kTileBytes = 16 * kTileRow;    // 16 rows
 constexpr size_t kMmaSmem = size_t(kAtWarps) * 2 * kTileBytes; // per warp: a key tile and a value tile
 
+__device__ __forceinline__ float warp_max_redux(float v) // maximum over the warp, as fmaxf takes it
+{
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
 __device__ __forceinline__ uint32_t bf16_piece_pair(float a, float b, int piece)
 {
     // piece 0: the bf16 roundings of a and b; piece 1: the bf16 roundings of what those left over
@@ -167,21 +174,37 @@ __device__ __forceinline__ void attn_mma_warp(const void *kc, const void *vc, in
 // scratch, fence or ticket.  Longer ones use up to `clusters` clusters per head; their results go to scratch and the last one
 // to arrive (a ticket per CTA rank) folds them in order.  For one launch's clusters the cut depends on the row count alone; the
 // clusters on the cache's type and capacity and, in a batch, on how many sequences share the device (launch_attn).
-// Measured as graph replays (fp32 cache, one step; in brackets with one CTA per split and a ticket): 40 rows 6.0 us (7.1), 1024
-// rows 9.8 (10.3), 8 x 600 rows 16.2 (38.5), 8 x 5000 rows 60 (119.5), which is 5.4 TB/s, 84 % of the copy peak.
-constexpr int kCtaRows = 48;    // rows per CTA from which another cluster is put to work (32, 48, 64, 96 tried: 48 is best or next to it)
+// Measured as graph replays (fp32 cache, one step; in brackets with one CTA per split and a ticket): 40 rows 4.9 us (7.1), 1024
+// rows 8.8 (10.3), 8 x 600 rows 14.2 (38.5), 8 x 5000 rows 58.6 (119.5), which is 5.6 TB/s, 86 % of the copy peak.
+//
+// A block more costs a CTA 1.5 us (bf16 1.1), the exchange between clusters 2.4 us: one cluster up to two blocks a CTA (three in a batch, whose
+// sequences share the device, and with the bf16 cache); then, with the fp32 cache, clusters of one block a CTA up to four blocks a CTA of one
+// cluster; beyond that clusters of two.  fp32 cache, one cluster / one block a CTA / two: 400 rows 6.8 / 7.4 / -, 600 rows 8.3 / 7.7 / 8.5, 800 rows
+// 9.9 / 8.4 / 8.8, 1500 rows 13.4 / 10.2 / 9.4 us; two sequences of 600 rows 8.4 / 9.2 / 10.4; bf16 cache, 600 rows 7.3 / 7.8 / 8.6.
 constexpr int kMaxClusters = 8; // per kv head
+struct AttnRule {
+    int one, some; // rows up to which one cluster takes them, up to which several take a block a CTA
+};
+__host__ __device__ inline AttnRule attn_rule(bool bf16, bool batch, int unit) // unit: CTAs of a cluster
+{
+    return AttnRule{(bf16 || batch ? 3 : 2) * kBlock * unit, bf16 ? 0 : 4 * kBlock * unit};
+}
+__host__ __device__ inline int attn_clusters(const AttnRule &r, int rows, int unit)
+{
+    const int per = (rows <= r.some ? kBlock : 2 * kBlock) * unit;
+    return rows <= r.one ? 1 : (rows + per - 1) / per;
+}
 
 struct AttnCut {
     int active, chunk; // clusters at work, rows per CTA
 };
 // HALVES: two clusters of four in place of one of eight, with the same bits: when both have rows, the last to arrive folds the
 // eight CTAs' results as the cluster of eight does.
-template <int CL, bool HALVES> __device__ __forceinline__ AttnCut attn_cut(int rows, int clusters)
+template <int CL, bool HALVES> __device__ __forceinline__ AttnCut attn_cut(int rows, int clusters, const AttnRule &rule)
 {
     constexpr int kUnit = HALVES ? 2 * CL : CL; // CTAs
     AttnCut c;
-    c.active = min(HALVES ? clusters / 2 : clusters, (rows + kCtaRows * kUnit - 1) / (kCtaRows * kUnit));
+    c.active = min(HALVES ? clusters / 2 : clusters, attn_clusters(rule, rows, kUnit));
     const int ctas = c.active * kUnit;
     c.chunk = max(kMinChunk, (rows + ctas - 1) / ctas);
     if (HALVES) c.active = (rows + c.chunk * CL - 1) / (c.chunk * CL); // a half without rows has nothing to do
@@ -193,14 +216,18 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
 {
     using Row = KvRow<BF16>;
     constexpr bool kMma = BF16 && CL == 4 && !HALVES; // the bf16 launches of long contexts
+    constexpr bool kQuarters = !BF16 || kMma; // the loop over blocks of rows (below)
     constexpr int kParts = HALVES ? CL : 1; // partial results of a cluster in scratch
     constexpr int kMine = 1024 / CL; // output dims this CTA finishes
     __shared__ __align__(16) float s_q[4][256];
     __shared__ __align__(16) float s_knew[256], s_vnew[256];
     __shared__ float s_m[kAtWarps][4], s_l[kAtWarps][4];
-    __shared__ __align__(16) float s_acc[kAtWarps][4][256];
+    __shared__ __align__(16) float s_acc[kQuarters && !kMma ? 4 : kAtWarps][4][256]; // the quarters' or the warps' sums
+    __shared__ __align__(16) float4 s_score[2][kQuarters ? kBlock : 1];     // [row] scores of the four heads
+    __shared__ __align__(16) float4 s_p[kAtWarps][kQuarters ? kBlock : 1];  // a warp's copy of the weights
     __shared__ __align__(16) float s_in[CL][kMine]; // the cluster's partial sums of this CTA's dims
-    __shared__ float s_min[CL], s_lin[CL];          // and their maxima and denominators
+    __shared__ __align__(8) float2 s_ml[CL];        // and their maxima and denominators
+    __shared__ __align__(8) uint64_t s_there;       // all of them have come
     __shared__ int s_last;
     __shared__ __align__(8) uint64_t s_bar[2 * kAtWarps];
     __shared__ int s_abort;
@@ -220,7 +247,12 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
     const float *k_raw = p.k_raw + size_t(bt) * p.kvin_stride, *v_new = p.v_new + size_t(bt) * p.kvin_stride;
 
     pdl_launch_dependents();
-    asm volatile("barrier.cluster.arrive.release;" ::: "memory"); // the peers have started when this completes
+    if (tid == 0) {
+        s_abort = 0;
+        mbar_init(&s_there, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory"); // the peers have started, with their barriers, when this completes
 
     // Geometry from the position as it is visible now.  Cache rows of earlier tokens never change
     // again, so the first token group of every warp is fetched while the producer of q still runs;
@@ -233,18 +265,42 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
         tokens = __ldcg(p.position) + p.position_offset + bt + 1;
     }
     tokens = max(1, min(tokens, p.max_context)); // host checks; never index past the cache
-    AttnCut cut = attn_cut<CL, HALVES>(tokens, clusters);
+    const AttnRule rule = attn_rule(BF16, p.batch != 0, HALVES ? 2 * CL : CL);
+    AttnCut cut = attn_cut<CL, HALVES>(tokens, clusters, rule);
     int t0 = split * cut.chunk, t1 = min(tokens, t0 + cut.chunk);
     int fresh = tokens - 1; // the row the producer (or this kernel) is still writing
 
     if (p.image && tid < 81) s_lut[tid] = digit_pair_code(tid); // read behind the barriers below
     bool use_mma = kMma && tokens >= kMmaMinTokens; // long bf16 contexts: the tensor-core loop (reads every row from the cache)
-    if (tid == 0) s_abort = 0;
-    // This warp's next token group: its keys are replaced by the following group's as soon as they are scored, its values as soon
-    // as they are added.  One group (two would take a CTA's registers past what fits beside the products' launches, and the
-    // launch could start only when its predecessor had left the SM).
+    // The rows that come next: a warp's four rows of keys are replaced by the following ones as soon as they are scored, its values (of the same rows, or
+    // half of the dims of a quarter of the block's rows) as soon as they are added.  (Two groups or blocks would take a CTA's registers past
+    // what fits beside the products' launches, and the launch could start only when its predecessor had left the SM.)
     GroupRaw<BF16, kGroup> ga;
-    if (!use_mma) load_group<BF16, kGroup>(kc, vc, kvh, t0 + warp * kGroup, min(t1, fresh), lane, ga);
+    const int quarter = warp >> 1, dim0 = (warp & 1) * 128 + lane * 4;
+    typename Row::Quad vr[kQuarters ? kBlock / 4 : 1];
+    auto load_quad = [&](const void *cache, int t) { return Row::load_quad(cache, (size_t(t) * 4 + kvh) * 256 + dim0); };
+    auto fetch_keys = [&](int tb, int tend) {
+#pragma unroll
+        for (int g = 0; g < kGroup; g++) {
+            const int t = tb + warp * kGroup + g;
+            ga.k[g] = t < tend ? Row::load_raw(kc, (size_t(t) * 4 + kvh) * 256, lane) : Row::zero();
+        }
+    };
+    auto fetch_values = [&](int tb, int tend) {
+#pragma unroll
+        for (int g = 0; g < kBlock / 4; g++) {
+            const int t = tb + quarter * (kBlock / 4) + g;
+            vr[g] = t < tend ? load_quad(vc, t) : Row::zero_quad();
+        }
+    };
+    auto fetch = [&] {
+        if constexpr (kQuarters) {
+            if (use_mma) return;
+            fetch_keys(t0, min(t1, fresh));
+            fetch_values(t0, min(t1, fresh));
+        } else if (!use_mma) load_group<BF16, kGroup>(kc, vc, kvh, t0 + warp * kGroup, min(t1, fresh), lane, ga);
+    };
+    fetch();
     uint4 norm_wv = make_uint4(0u, 0u, 0u, 0u);
     float rope_c[8], rope_s[8];
     if constexpr (FUSED) {
@@ -267,12 +323,12 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
         if (now != pos) {
             pos = now;
             tokens = max(1, min(pos + 1, p.max_context));
-            cut = attn_cut<CL, HALVES>(tokens, clusters);
+            cut = attn_cut<CL, HALVES>(tokens, clusters, rule);
             t0 = split * cut.chunk;
             t1 = min(tokens, t0 + cut.chunk);
             fresh = tokens - 1;
             use_mma = kMma && tokens >= kMmaMinTokens;
-            if (!use_mma) load_group<BF16, kGroup>(kc, vc, kvh, t0 + warp * kGroup, min(t1, fresh), lane, ga);
+            fetch();
             if (warp < 5 && lane < 8) rope_table(pos, lane, p.fast_trig != 0, rope_c, rope_s);
         }
     }
@@ -289,8 +345,8 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
         if constexpr (FUSED) {
             if (warp < 4) {
                 norm_rope_256(raw, norm_wv, lane, pos, rope_c, rope_s);
-#pragma unroll
-                for (int j = 0; j < 8; j++) s_q[warp][lane * 8 + j] = raw[j];
+                reinterpret_cast<float4 *>(s_q[warp])[lane * 2] = make_float4(raw[0], raw[1], raw[2], raw[3]);
+                reinterpret_cast<float4 *>(s_q[warp])[lane * 2 + 1] = make_float4(raw[4], raw[5], raw[6], raw[7]);
             } else if (warp == 4 && pos >= t0 && pos < t1) {
                 norm_rope_256(raw, norm_wv, lane, pos, rope_c, rope_s);
                 const size_t row = (size_t(pos) * 4 + kvh) * 256 + lane * 8;
@@ -322,7 +378,110 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
             mma_done = true;
         }
     }
+    float m0 = -3.0e38f, l0 = 0.f; // of head warp >> 1: the CTA's maximum and denominator
+    if constexpr (kQuarters) {
     if (!mma_done) {
+        // ---- fp32 cache (and the few rows of a long bf16 cache): blocks of 32 rows.  The CTA's warps score four rows each, then every warp has the weights of all rows and adds its part of the
+        // values, so that the warps share their maxima and nothing is left to be rescaled between them.  With a loop as below 40 rows took 5.3 us
+        // instead of 4.9, 8192 rows 19.7 instead of 18.1, 8 x 5000 rows the same 58.7; the bf16 cache, with half the bytes to wait for, is better off without
+        // the barrier (8 x 2000 rows 24.1 like this, 21.1 as below).
+        float m[4], l[4], acc[4][4]; // per head; l: this lane's rows
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+            m[h] = -3.0e38f;
+            l[h] = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc[h][j] = 0.f;
+        }
+        const int tend = min(t1, fresh);
+        int buf = 0;
+#pragma unroll 1
+        for (int tb = t0; tb < t1; tb += kBlock, buf ^= 1) {
+            const int gk = fresh < t1 ? fresh - tb - warp * kGroup : -1, gv_row = fresh < t1 ? fresh - tb - quarter * (kBlock / 4) : -1; // the newest row's place
+            if (gk >= 0 && gk < kGroup) { // from shared memory or, now that the wait is over, from the cache
+                const typename Row::Raw x = FUSED ? Row::pack(s_knew + lane * 8) : Row::load_raw(kc, (size_t(fresh) * 4 + kvh) * 256, lane);
+#pragma unroll
+                for (int g = 0; g < kGroup; g++)
+                    if (g == gk) ga.k[g] = x;
+            }
+            if (gv_row >= 0 && gv_row < kBlock / 4) {
+                const typename Row::Quad x = FUSED ? Row::pack_quad(s_vnew + dim0) : load_quad(vc, fresh);
+#pragma unroll
+                for (int g = 0; g < kBlock / 4; g++)
+                    if (g == gv_row) vr[g] = x;
+            }
+            float s[16];
+#pragma unroll
+            for (int h = 0; h < 4; h++) {
+                const float4 qa = *reinterpret_cast<const float4 *>(&s_q[h][lane * 8]), qb = *reinterpret_cast<const float4 *>(&s_q[h][lane * 8 + 4]);
+#pragma unroll
+                for (int g = 0; g < kGroup; g++) {
+                    float kk[8];
+                    Row::unpack(ga.k[g], kk);
+                    float z = qa.x * kk[0];
+                    z = fmaf(qa.y, kk[1], z); z = fmaf(qa.z, kk[2], z); z = fmaf(qa.w, kk[3], z);
+                    z = fmaf(qb.x, kk[4], z); z = fmaf(qb.y, kk[5], z); z = fmaf(qb.z, kk[6], z); z = fmaf(qb.w, kk[7], z);
+                    s[g * 4 + h] = z;
+                }
+            }
+            if (tb + kBlock < t1) fetch_keys(tb + kBlock, tend);
+            // sums over the lanes, halving the values a lane carries at every step: 16 shuffles where summing each takes 80
+#pragma unroll
+            for (int n = 8, mk = 16; n; n >>= 1, mk >>= 1) {
+                const bool up = (lane & mk) != 0;
+#pragma unroll
+                for (int i = 0; i < n; i++) {
+                    const float keep = up ? s[i + n] : s[i], send = up ? s[i] : s[i + n];
+                    s[i] = keep + __shfl_xor_sync(0xffffffffu, send, mk);
+                }
+            }
+            const float score = (s[0] + __shfl_xor_sync(0xffffffffu, s[0], 1)) * 0.0625f; // row lane >> 3, head (lane >> 1) & 3
+            if (!(lane & 1)) reinterpret_cast<float *>(&s_score[buf][warp * kGroup + (lane >> 3)])[(lane >> 1) & 3] = score;
+            __syncthreads();
+            const float4 own = s_score[buf][lane]; // row `lane` of the block
+            const float sc[4] = {own.x, own.y, own.z, own.w};
+            const bool on = tb + lane < t1;
+            float pr[4], corr[4];
+#pragma unroll
+            for (int h = 0; h < 4; h++) {
+                const float mn = fmaxf(m[h], warp_max_redux(on ? sc[h] : -3.0e38f));
+                corr[h] = __expf(m[h] - mn);
+                pr[h] = on ? __expf(sc[h] - mn) : 0.f;
+                m[h] = mn;
+                l[h] = fmaf(l[h], corr[h], pr[h]);
+            }
+            s_p[warp][lane] = make_float4(pr[0], pr[1], pr[2], pr[3]);
+            __syncwarp();
+            float part[4][4]; // of this block
+#pragma unroll
+            for (int g = 0; g < kBlock / 4; g++) {
+                const float4 w = s_p[warp][quarter * (kBlock / 4) + g];
+                float vv[4];
+                Row::unpack_quad(vr[g], vv);
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    part[0][j] = g ? fmaf(w.x, vv[j], part[0][j]) : w.x * vv[j];
+                    part[1][j] = g ? fmaf(w.y, vv[j], part[1][j]) : w.y * vv[j];
+                    part[2][j] = g ? fmaf(w.z, vv[j], part[2][j]) : w.z * vv[j];
+                    part[3][j] = g ? fmaf(w.w, vv[j], part[3][j]) : w.w * vv[j];
+                }
+            }
+            if (tb + kBlock < t1) fetch_values(tb + kBlock, tend);
+#pragma unroll
+            for (int h = 0; h < 4; h++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[h][j] = fmaf(acc[h][j], corr[h], part[h][j]);
+            __syncwarp(); // the weights have been read
+        }
+        if (has_work) {
+#pragma unroll
+            for (int h = 0; h < 4; h++) *reinterpret_cast<float4 *>(&s_acc[quarter][h][dim0]) = make_float4(acc[h][0], acc[h][1], acc[h][2], acc[h][3]);
+            const int h = warp >> 1; // the head this thread hands on below
+            m0 = h == 0 ? m[0] : h == 1 ? m[1] : h == 2 ? m[2] : m[3];
+            l0 = warp_sum(h == 0 ? l[0] : h == 1 ? l[1] : h == 2 ? l[2] : l[3]);
+        }
+    }
+    } else if (!mma_done) {
         // Of the sixteen scores of a group (four rows x four heads) lane L keeps number L >> 1: row L >> 3, head (L >> 1) & 3.
         // The maximum is that head's, the denominator this lane's own share of it.
         float m = -3.0e38f, l = 0.f, acc[4][8];
@@ -413,52 +572,65 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
                 *reinterpret_cast<float4 *>(&s_acc[warp][h][lane * 8 + j]) = make_float4(acc[h][j], acc[h][j + 1], acc[h][j + 2], acc[h][j + 3]);
     }
     __syncthreads();
-    // ---- fold the eight warps (thread = dim) and hand every CTA of the cluster the dims it finishes ----------------
+    // ---- add up the CTA's sums, four dims of a head a thread, and hand them to the CTA of the cluster that finishes them ----------------
+    const int working = max(0, min(CL, (tokens - t0 + rank * cut.chunk + cut.chunk - 1) / cut.chunk)); // CTAs of the cluster with rows: the first ones
+    if (tid == 0) mbar_expect_tx(&s_there, uint32_t(working) * (kMine * 4 + 8));
+    if (has_work) {
+        const int h = warp >> 1, dim = (tid & 63) * 4, at = h * 256 + dim, owner = at / kMine;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (kQuarters && !mma_done) {
+            float4 x[4];
 #pragma unroll
-    for (int h = 0; h < 4; h++) {
-        float mg = s_m[0][h];
+            for (int i = 0; i < 4; i++) x[i] = *reinterpret_cast<const float4 *>(&s_acc[i][h][dim]);
+            a = make_float4((x[0].x + x[1].x) + (x[2].x + x[3].x), (x[0].y + x[1].y) + (x[2].y + x[3].y), (x[0].z + x[1].z) + (x[2].z + x[3].z),
+                            (x[0].w + x[1].w) + (x[2].w + x[3].w));
+        } else {
+            m0 = s_m[0][h];
 #pragma unroll
-        for (int w = 1; w < kAtWarps; w++) mg = fmaxf(mg, s_m[w][h]);
-        float lg = 0.f, a = 0.f;
+            for (int w = 1; w < kAtWarps; w++) m0 = fmaxf(m0, s_m[w][h]);
 #pragma unroll
-        for (int w = 0; w < kAtWarps; w++) {
-            const float e = __expf(s_m[w][h] - mg); // warps without rows carry m = -3e38, l = 0, acc = 0
-            lg = fmaf(s_l[w][h], e, lg);
-            a = fmaf(s_acc[w][h][tid], e, a);
+            for (int w = 0; w < kAtWarps; w++) {
+                const float e = __expf(s_m[w][h] - m0); // warps without rows carry m = -3e38, l = 0, acc = 0
+                const float4 x = *reinterpret_cast<const float4 *>(&s_acc[w][h][dim]);
+                l0 = fmaf(s_l[w][h], e, l0);
+                a.x = fmaf(x.x, e, a.x); a.y = fmaf(x.y, e, a.y); a.z = fmaf(x.z, e, a.z); a.w = fmaf(x.w, e, a.w);
+            }
         }
-        const int dim = h * 256 + tid, owner = dim / kMine;
-        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_to_rank(smem_u32(&s_in[rank][dim % kMine]), owner)), "f"(a) : "memory");
-        if (dim % kMine == 0) { // the head's maximum and denominator to the owner of these dims
-            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_to_rank(smem_u32(&s_min[rank]), owner)), "f"(mg) : "memory");
-            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_to_rank(smem_u32(&s_lin[rank]), owner)), "f"(lg) : "memory");
-        }
+        const uint32_t bar = map_to_rank(smem_u32(&s_there), owner);
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
+                     ::"r"(map_to_rank(smem_u32(&s_in[rank][at % kMine]), owner)), "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w), "r"(bar) : "memory");
+        if (at % kMine == 0) // the head's maximum and denominator to the owner of these dims
+            asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];"
+                         ::"r"(map_to_rank(smem_u32(&s_ml[rank]), owner)), "f"(m0), "f"(l0), "r"(bar) : "memory");
     }
-    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
-    // the new row goes to the cache now: ahead of the barrier its release would wait for these stores
+    // the new row goes to the cache while the others' parts come in
     if constexpr (FUSED)
         if (!use_mma && pos >= t0 && pos < t1) {
             const size_t row = (size_t(pos) * 4 + kvh) * 256 + tid;
             Row::store(kc, row, s_knew[tid]);
             Row::store(vc, row, s_vnew[tid]);
         }
-    float mg = s_min[0];
+    mbar_wait_cluster(&s_there, 0, &s_abort);
+    float mg = -3.0e38f, lg = 0.f, a = 0.f;
 #pragma unroll
-    for (int c = 1; c < CL; c++) mg = fmaxf(mg, s_min[c]);
-    float lg = 0.f, a = 0.f;
+    for (int c = 0; c < CL; c++)
+        if (c < working) mg = fmaxf(mg, s_ml[c].x);
 #pragma unroll
-    for (int c = 0; c < CL; c++) {
-        const float e = __expf(s_min[c] - mg);
-        lg = fmaf(s_lin[c], e, lg);
-        if (tid < kMine) a = fmaf(s_in[c][tid], e, a);
-    }
+    for (int c = 0; c < CL; c++)
+        if (c < working) {
+            const float2 ml = s_ml[c];
+            const float e = __expf(ml.x - mg);
+            lg = fmaf(ml.y, e, lg);
+            if (tid < kMine) a = fmaf(s_in[c][tid], e, a);
+        }
     if (cut.active > 1) { // several clusters: partial results to scratch, the last one folds them in order
         float *part = partials + size_t(kvh * kSplits + cluster * kParts) * kPartFloats;
 #pragma unroll
         for (int c = 0; c < kParts; c++, part += kPartFloats) {
-            if (tid < kMine) part[8 + rank * kMine + tid] = HALVES ? s_in[c][tid] : a;
+            if (tid < kMine) part[8 + rank * kMine + tid] = !HALVES ? a : c < working ? s_in[c][tid] : 0.f;
             if (tid == 0) { // CTAs that share a head write the same values
-                part[my_head & 3] = HALVES ? s_min[c] : mg;
-                part[4 + (my_head & 3)] = HALVES ? s_lin[c] : lg;
+                part[my_head & 3] = !HALVES ? mg : c < working ? s_ml[c].x : -3.0e38f;
+                part[4 + (my_head & 3)] = !HALVES ? lg : c < working ? s_ml[c].y : 0.f;
             }
         }
         __threadfence();
@@ -521,7 +693,11 @@ template <bool BF16, bool FUSED, int CL, bool HALVES = false> static int launch_
         if (p.max_context >= kMmaMinTokens) smem = kMmaSmem; // else no launch of these operands gets to the tensor-core loop
     }
     const int most = rows > 0 ? std::min(rows, p.max_context) : p.max_context;
-    if (!HALVES) clusters = std::max(1, std::min({clusters, kMaxClusters, (most + kCtaRows * CL - 1) / (kCtaRows * CL)}));
+    if (!HALVES) { // as many as some row count up to `most` has at work: clusters without rows cost a launch of two sequences 3 us of 11
+        const AttnRule rule = attn_rule(BF16, p.batch != 0, CL);
+        const int at_work = std::max(attn_clusters(rule, most, CL), attn_clusters(rule, std::min(most, rule.some), CL));
+        clusters = std::max(1, std::min({clusters, kMaxClusters, at_work}));
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(4 * clusters * CL, along);
     cfg.blockDim = dim3(kAtThreads);
@@ -554,11 +730,12 @@ template <bool BF16, bool FUSED, int CL, bool HALVES = false> static int launch_
 // five sequences win at 20 rows and lose 12 us from 130 on.  A chunk takes the pairs while one cluster holds its rows.
 constexpr int kLongContext = 2048;
 static_assert(kLongContext <= kMmaMinTokens, "short contexts never get to the tensor-core loop");
-template <bool BF16, bool FUSED> int launch_attn(const AttnParams &p, cudaStream_t st, bool pdl, int along = 1, int rows = 0)
+template <bool BF16, bool FUSED> int launch_attn(AttnParams p, cudaStream_t st, bool pdl, int along = 1, int rows = 0)
 {
+    p.batch = FUSED && along > 1;
     const int clusters = FUSED ? kMaxClusters / along : kMaxClusters;
     if (p.max_context < kLongContext) {
-        const bool one_cluster = rows > 0 && rows <= kCtaRows * 8;
+        const bool one_cluster = rows > 0 && rows <= attn_rule(BF16, false, 8).one;
         if ((FUSED || one_cluster) && along > kMaxClusters / 2 && 2 * along * 4 * 8 > 3 * sm_count()) return launch_clusters<BF16, FUSED, 4, true>(p, st, pdl, along, rows, 2);
         return launch_clusters<BF16, FUSED, 8>(p, st, pdl, along, rows, clusters);
     }

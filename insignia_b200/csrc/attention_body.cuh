@@ -37,6 +37,7 @@ struct AttnParams {
     const float *gate;
     uint8_t *image;
     int slots, gate_elementwise;
+    int batch;             // several sequences share the launch
     int *error_flag;       // set to 1 when a bounded wait inside the kernel ran out (bf16 tensor-core path), or null
 };
 
@@ -57,6 +58,12 @@ template <> struct KvRow<false> {
     static __device__ __forceinline__ Raw pack(const float *p) { return Raw{reinterpret_cast<const float4 *>(p)[0], reinterpret_cast<const float4 *>(p)[1]}; }
     static __device__ __forceinline__ float round(float v) { return v; }
     static __device__ __forceinline__ void store(void *base, size_t idx, float v) { static_cast<float *>(base)[idx] = v; }
+    // four dims of a row
+    using Quad = float4;
+    static __device__ __forceinline__ Quad load_quad(const void *base, size_t idx) { return __ldcg(reinterpret_cast<const float4 *>(static_cast<const float *>(base) + idx)); }
+    static __device__ __forceinline__ Quad zero_quad() { return make_float4(0.f, 0.f, 0.f, 0.f); }
+    static __device__ __forceinline__ Quad pack_quad(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+    static __device__ __forceinline__ void unpack_quad(const Quad &r, float (&o)[4]) { o[0] = r.x; o[1] = r.y; o[2] = r.z; o[3] = r.w; }
 };
 template <> struct KvRow<true> {
     struct Raw { uint4 r; };
@@ -86,6 +93,18 @@ template <> struct KvRow<true> {
     static __device__ __forceinline__ void store(void *base, size_t idx, float v)
     {
         static_cast<__nv_bfloat16 *>(base)[idx] = __float2bfloat16_rn(v);
+    }
+    using Quad = uint2;
+    static __device__ __forceinline__ Quad load_quad(const void *base, size_t idx) { return __ldcg(reinterpret_cast<const uint2 *>(static_cast<const uint16_t *>(base) + idx)); }
+    static __device__ __forceinline__ Quad zero_quad() { return make_uint2(0u, 0u); }
+    static __device__ __forceinline__ Quad pack_quad(const float *p)
+    {
+        return make_uint2((__float_as_uint(p[0]) >> 16) | (__float_as_uint(p[1]) & 0xffff0000u), (__float_as_uint(p[2]) >> 16) | (__float_as_uint(p[3]) & 0xffff0000u));
+    }
+    static __device__ __forceinline__ void unpack_quad(const Quad &r, float (&o)[4])
+    {
+        o[0] = __uint_as_float(r.x << 16); o[1] = __uint_as_float(r.x & 0xffff0000u);
+        o[2] = __uint_as_float(r.y << 16); o[3] = __uint_as_float(r.y & 0xffff0000u);
     }
 };
 
