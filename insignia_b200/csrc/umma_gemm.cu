@@ -576,14 +576,22 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
         // ---- producer of the weights: two records per stage ----------------------------------------------------------
         // They do not depend on the launch before this one (the digits do): the first ring is requested at once, by one lane per
         // stage (a bulk copy takes the issuing thread a few hundred cycles).
+        // One group of tokens reads a record once.  (Several read it one after the other: with the hint for the last of them 24576 x 4096 with 23
+        // tokens takes 21.9 us instead of 20.0.)
+        const bool once = TPG == 16 && p.ngroups == 1;
+        const uint64_t policy = once_policy();
+        auto load_record = [&](uint8_t *dst, const uint8_t *src, uint64_t *bar) {
+            if (once) bulk_load_hint(dst, src, kURec, bar, policy);
+            else bulk_load(dst, src, kURec, bar);
+        };
         const int first = min(S, end - begin);
         if (lane < first) {
             const GRun r = run_at(p, begin + lane, end);
             const PairSrc q = pair_src<CL, SWIGLU>(p, r.unit / p.ngroups, rank, r.kb0);
             uint8_t *dst = ring + size_t(lane) * kGStage;
             mbar_expect_tx(&full[lane], (q.two ? 2 : 1) * kURec);
-            bulk_load(dst, q.a[0], kURec, &full[lane]);
-            if (q.two) bulk_load(dst + kURec, q.a[1], kURec, &full[lane]);
+            load_record(dst, q.a[0], &full[lane]);
+            if (q.two) load_record(dst + kURec, q.a[1], &full[lane]);
         }
         __syncwarp();
         // from here on the whole warp walks the loop and one elected lane issues: warp-uniform operands issue twice as fast
@@ -603,8 +611,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) umma_gemm_kernel(const __grid
                 if (one) {
                     uint8_t *dst = ring + size_t(cur) * kGStage;
                     mbar_expect_tx(&full[cur], (q.two ? 2 : 1) * kURec);
-                    bulk_load(dst, a0, kURec, &full[cur]);
-                    if (q.two) bulk_load(dst + kURec, a1, kURec, &full[cur]);
+                    load_record(dst, a0, &full[cur]);
+                    if (q.two) load_record(dst + kURec, a1, &full[cur]);
                 }
             }
             g += r.len;

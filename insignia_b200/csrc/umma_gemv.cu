@@ -329,10 +329,11 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         const DSeg &s = seg_of(unit);
         return (nmat == 2 && (run & 1) ? s.packed2 : s.packed) + (size_t(unit - s.tile_begin) * nkb + kb0) * kURec;
     };
+    const uint64_t once = once_policy();
     auto load_stage = [&](int slot, const uint8_t *src, int st) { // stage st of a run: two records, or the last one of an odd count
         const uint32_t records = uint32_t(min(2, len - 2 * st));
         mbar_expect_tx(&full[slot], records * (kURec + (streamed ? kImg : 0)));
-        bulk_load(ring + size_t(slot) * kStage, src + size_t(st) * kDStage, records * kURec, &full[slot]);
+        bulk_load_hint(ring + size_t(slot) * kStage, src + size_t(st) * kDStage, records * kURec, &full[slot], once);
     };
     auto load_digits = [&](int slot, int st) { // streamed: behind the weights of the only run's stage st
         bulk_load(ring + size_t(slot) * kStage + kDStage, reinterpret_cast<const uint8_t *>(p.in) + size_t(kb0 + 2 * st) * kImg, uint32_t(min(2, len - 2 * st)) * kImg, &full[slot]);
@@ -499,7 +500,7 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             if constexpr (kDAheadStages<T> > 0) {
                 for (int i = S + lane; i < min(nstages, S + p.ahead); i += 32) {
                     const int run = single ? 0 : i / spt, st = i - run * spt;
-                    bulk_prefetch(run_src(run) + size_t(st) * kDStage, uint32_t(min(2, len - 2 * st)) * kURec);
+                    bulk_prefetch_hint(run_src(run) + size_t(st) * kDStage, uint32_t(min(2, len - 2 * st)) * kURec, once);
                 }
                 __syncwarp();
             }
