@@ -49,13 +49,16 @@ constexpr uint32_t kDSfaCol = 128, kDSfbCol = 160, kDTmemCols = 256; // accumula
 constexpr int kDHalfSm = 112 * 1024;
 // The next launch may start when at most this many ring stages of a CTA are still to be requested, and asks L2 for a few beyond its
 // own ring.  Its requests share the SM's copy engine and the memory with this launch's: made while this launch still streams they delay
-// the stages it waits for.  The four products of a block with one token: 28.1 us with the next launch at once, 26.6 like this, 29.3 at
-// the very end, when its ring cannot fill in time; L2 asked for six stages 27.8, for all of them 28.0.  Eight tokens 35.3 -> 34.4 us,
-// where asking L2 gains nothing.  A token 1.16 -> 1.115 ms.  All threads execute the trigger where the CTA sets out: left to the
-// producer warp, with the L2 code in every variant, a launch that stands alone took 0.1-0.3 us more (4096 x 4096, one, two, eight tokens
-// 6.85, 8.11, 12.25 us; like this 6.78, 7.98, 12.10; with the trigger there for every size 6.77, 7.85, 12.07).
-template <int T> constexpr int kDTriggerStages = T <= 2 ? 6 : 4;
-template <int T> constexpr int kDAheadStages = T <= 2 ? 3 : 0;
+// the stages it waits for, made at the very end its ring cannot fill in time.  Microseconds a step by (stages left, stages asked of L2), with weights
+// that leave L2 first (where they stay, asking for more than three or, from three tokens on, any gains nothing):
+//   one token (4, 3) 969, (6, 2) 973, (6, 3) 959, (6, 4) 965, (6, 10) 968, (8, 3) 1025; a speculative pass (5, 4) 1306, (5, 5) 1302,
+//   (5, 6) 1301, (6, 3) 1311, (7, 3) 1331, two sequences 1063, 1063, 1070, 1065, -
+//   three sequences (3, 6) 1100, (4, 0) 1096, (4, 3) 1074, (4, 6) 1063, (4, 8) 1085, (5, 6) 1074, (6, 0) 1113
+//   eight sequences (2, 6) 1250, (2, 8) 1287, (3, 4) 1254, (3, 6) 1246, (3, 10) 1268, (4, 0) 1265, (4, 6) 1250, (6, 3) 1291
+// All threads execute the trigger where the CTA sets out: left to the producer warp, with the L2 code in every variant, a launch that stands
+// alone took 0.1-0.3 us more (4096 x 4096, one, two, eight tokens 6.85, 8.11, 12.25 us; like this 6.78, 7.98, 12.10).
+template <int T> constexpr int kDTriggerStages = T == 1 ? 6 : T == 2 ? 5 : T == 4 ? 4 : 3;
+template <int T> constexpr int kDAheadStages = T == 1 ? 3 : T == 2 ? 5 : 6;
 
 struct DSeg {
     const uint8_t *packed, *packed2;
@@ -497,13 +500,11 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         // ---- producer ----------------------------------------------------------------------------------------------------------
         {
             const bool one = elect_one();
-            if constexpr (kDAheadStages<T> > 0) {
-                for (int i = S + lane; i < min(nstages, S + p.ahead); i += 32) {
-                    const int run = single ? 0 : i / spt, st = i - run * spt;
-                    bulk_prefetch_hint(run_src(run) + size_t(st) * kDStage, uint32_t(min(2, len - 2 * st)) * kURec, once);
-                }
-                __syncwarp();
+            for (int i = S + lane; i < min(nstages, S + p.ahead); i += 32) {
+                const int run = single ? 0 : i / spt, st = i - run * spt;
+                bulk_prefetch_hint(run_src(run) + size_t(st) * kDStage, uint32_t(min(2, len - 2 * st)) * kURec, once);
             }
+            __syncwarp();
             if constexpr (prepared) { // the digits come ready: eight k-blocks per copy, so that the multiplies can start behind the first
                 if (!delta) pdl_wait(); // (delta: they were there when the launch before this one let it start)
                 if (at_once && p.late) pdl_launch_dependents();
@@ -1065,7 +1066,7 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st, const insg_delta_o
     int stages = fixed < size_t(kDHalfSm) ? int((kDHalfSm - fixed) / stage_bytes) : 0;
     if (stages < 4 || (stages == 4 && need > 96)) stages = int((size_t(222) * 1024 - fixed) / stage_bytes);
     p.stages = std::max(1, std::min({stages, need, kDMaxStages}));
-    p.ahead = !op->pdl ? 0 : T == 1 ? kDAheadStages<1> : T == 2 ? kDAheadStages<2> : 0; // a launch that waits for its predecessor anyway streams at once
+    p.ahead = !op->pdl ? 0 : T == 1 ? kDAheadStages<1> : T == 2 ? kDAheadStages<2> : kDAheadStages<4>; // a launch that waits for its predecessor anyway streams at once
     const size_t smem = fixed + size_t(p.stages) * stage_bytes;
 
     cudaLaunchConfig_t cfg = {};
