@@ -210,6 +210,11 @@ int insg_gemv_fused(const insg_gemv_op *op, insg_stream_t stream)
 int insg_mxfp4_gemv_packed(const void *packed, const float *x, float *y, int rows, int cols, int M, insg_stream_t stream)
 {
     if (M < 1 || M > 4096) return fail(INSG_E_SHAPE, "gemv_packed: 1 <= M <= 4096");
+    // On tcgen05 (umma_gemv.cu) from 12 million weights on, whatever the tokens, so that a token's bits do not depend on the others.  Smaller matrices
+    // are bound by the host's side of the call, which a launch of clusters makes half a microsecond longer (a call for 8192 x 1024 7.8 us here, 8.1 there;
+    // 4096 x 4096, one to four tokens 8.2, 9.9, 10.3, 10.3 here, 8.1, 8.0, 8.4, 9.1 there).
+    const bool on_tensor_cores = packed && x && y && rows > 0 && (rows & 15) == 0 && cols > 0 && (cols & 127) == 0 && cols <= 12288 &&
+                                 (long long)rows * cols >= 12ll << 20 && ((reinterpret_cast<uintptr_t>(packed) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
     for (int m0 = 0; m0 < M;) {
         int mm = std::min(M - m0, 4);
         insg_gemv_op op = {};
@@ -221,8 +226,9 @@ int insg_mxfp4_gemv_packed(const void *packed, const float *x, float *y, int row
         op.seg[0].out = y + size_t(m0) * rows;
         op.seg[0].rows = rows;
         op.seg[0].epilogue = INSG_EPI_STORE;
-        int rc = gemv_fused_launch(&op, mm, stream);
-        if (rc == INSG_E_LIMIT && mm == 3) { // the rows' sums of three tokens fit shared memory up to some 10^6 rows, of two half as many more
+        op.tokens = mm;
+        int rc = on_tensor_cores ? gemv_umma_launch(&op, stream, nullptr) : gemv_fused_launch(&op, mm, stream);
+        if (rc == INSG_E_LIMIT && mm == 3 && !on_tensor_cores) { // the rows' sums of three tokens fit shared memory up to some 10^6 rows, of two half as many more
             mm = 2;
             rc = gemv_fused_launch(&op, mm, stream);
         }

@@ -38,6 +38,7 @@ namespace insg {
 
 constexpr int kDCl = 4;                    // CTAs per cluster = parts K is cut into = 32-row blocks of a tile
 constexpr int kDThreads = 320;
+constexpr int kDLoaders = 4;               // warps that fetch packed records (kDRecords), two row tiles each
 constexpr int kDStage = 2 * kURec;         // one ring stage: two consecutive k-blocks of a tile
 constexpr int kDMaxStages = 8;
 constexpr int kDMaxKb = 24;                // k-blocks per CTA: 12288 / 128 / 4
@@ -169,7 +170,7 @@ template <int T> __host__ __device__ constexpr int unit_slots(int nmat) { return
 // What a variant of the kernel has beside its tokens: a prepared input in place of the prologue; the logits' arg-max; two matrices (SwiGLU); one
 // segment that adds into the residual stream, one unit per cluster (kDResidual; with digits that come with the weights kDStreamed, behind the
 // gated norm kDGated); epilogues that add nothing and leave nothing prepared (kDPlain); a DeltaNet step beside the product that gates its output
-// (kDDelta).  A launch that fits none takes the general ones.
+// (kDDelta); weights that come as the packed records of insg_mxfp4_repack (kDRecords).  A launch that fits none takes the general ones.
 // A token is 129 launches of some seven microseconds, and instructions that a launch runs through for the first time come from L2 behind the
 // stream of weights.  Microseconds of a device-fed token (a host-fed decode_token gained half of it), a step of three sequences, of eight, and a
 // speculative pass (a process is now and then 2 % off for all of its life), and the code of a launch (the last line: of the special variants; what
@@ -180,7 +181,18 @@ template <int T> __host__ __device__ constexpr int unit_slots(int nmat) { return
 //   and two matrices, the gated norm, residual                                        1057 1170 1348 1387   28-48
 //   and plain; no later runs, last odd block or slot reuse where there are none       1031 1156 1330 1365   20-37
 // (20 KB more in the issuer's loop, never run, cost a token 80 us.)
-constexpr int kDPrepared = 1, kDLogits = 2, kDStreamed = 4, kDGated = 8, kDTwo = 16, kDResidual = 32, kDPlain = 64, kDDelta = 128;
+constexpr int kDPrepared = 1, kDLogits = 2, kDStreamed = 4, kDGated = 8, kDTwo = 16, kDResidual = 32, kDPlain = 64, kDDelta = 128, kDRecords = 256;
+constexpr int kRec = 1088;                 // a packed record: 16 rows x 128 k (insg_mxfp4_repack)
+constexpr int kDLoadAhead = 5;             // stages a loading thread has on their way; fewer than the ring has, or all there are (4 to 6 the same, 7 a third slower)
+
+__device__ __forceinline__ void copy16(void *dst, const void *src) // to shared memory, past L1
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy8(void *dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
 
 // One DeltaNet step of 32 columns of a head by the first eight warps of a CTA, whose cluster has the head: the arithmetic, and the order of every
 // sum, of deltanet_step_kernel and of the gated prologue, so that their bits are the same.  cell: rows kr + 32 j of the state, four columns.
@@ -286,14 +298,15 @@ __device__ __forceinline__ void delta_step(const DDelta &d, float4 (&cell)[4], D
 }
 
 template <int T, int F>
-__global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_constant__ DParams p)
+__global__ void __cluster_dims__(kDCl, 1, 1) __launch_bounds__(kDThreads + ((F & kDRecords) != 0 ? 32 * kDLoaders : 0), (F & kDRecords) != 0 ? 1 : 2) umma_gemv_kernel(const __grid_constant__ DParams p)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int kBKb = 512 * T;       // digit bytes per k-block
     constexpr int kImg = kBKb + 512;    // a k-block of the image: digits, then their scale block
     constexpr bool prepared = (F & kDPrepared) != 0, logits = (F & kDLogits) != 0, streamed = (F & kDStreamed) != 0;
-    const int pro = (F & kDGated) != 0 ? int(INSG_PRO_GATED_RMSNORM) : p.prologue;
-    constexpr int kStage = kDStage + (streamed ? 2 * kImg : 0); // streamed: one unit a cluster, so that its digits come with the weights they multiply
+    constexpr bool records = (F & kDRecords) != 0; // the weights come as packed records; a plain vector, one segment that is stored
+    const int pro = (F & kDGated) != 0 ? int(INSG_PRO_GATED_RMSNORM) : records ? int(INSG_PRO_PLAIN) : p.prologue;
+    constexpr int kStage = kDStage + (streamed ? 2 * kImg : 0) + (records ? 1024 : 0); // streamed: one unit a cluster, so that its digits come with the weights they multiply
     static_assert(!streamed || prepared, "a streamed image is a prepared one");
     constexpr int N = kDDigits * T;
     constexpr int kSlot = kDCl * 32 * T; // floats of one exchange slot: [source rank][32 rows][T]
@@ -310,10 +323,10 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     constexpr bool residual = (F & (kDResidual | kDStreamed | kDGated)) != 0; // one segment, added into the residual stream, one unit per cluster
     constexpr bool delta = (F & kDDelta) != 0, single = residual || delta;   // one segment, one unit per cluster
     static_assert(!delta || (prepared && T == 1), "the step's product takes one token's prepared input");
-    constexpr bool plain = (F & kDPlain) != 0;                       // nothing is left prepared
-    constexpr bool even = single || plain || (F & kDTwo) != 0;     // every CTA has an even number of k-blocks
+    constexpr bool plain = (F & (kDPlain | kDRecords)) != 0;                       // nothing is left prepared
+    constexpr bool even = single || (F & kDPlain) != 0 || (F & kDTwo) != 0;     // every CTA has an even number of k-blocks
     const int rank = int(blockIdx.x) & (kDCl - 1), cl = int(blockIdx.x) / kDCl, C = int(gridDim.x) / kDCl;
-    const int nkb = p.nkb, S = p.stages, nmat = (F & kDTwo) != 0 ? 2 : (F & (kDResidual | kDStreamed | kDGated | kDPlain | kDDelta)) != 0 ? 1 : p.nmat, XU = unit_slots<T>(nmat);
+    const int nkb = p.nkb, S = p.stages, nmat = (F & kDTwo) != 0 ? 2 : (F & (kDResidual | kDStreamed | kDGated | kDPlain | kDDelta | kDRecords)) != 0 ? 1 : p.nmat, XU = unit_slots<T>(nmat);
     const int kb0 = (nkb * rank) >> 2, len = ((nkb * (rank + 1)) >> 2) - kb0; // this CTA's k-blocks
     const int spt = (len + 1) >> 1;                                            // ring stages per (tile, matrix)
     const int nun = single ? 1 : cl < p.units ? (p.units - cl + C - 1) / C : 0;             // units of this cluster: cl, cl + C, ...
@@ -343,12 +356,12 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
     };
     if (warp == 9) {
         if (lane < S) { // one lane per stage: its barriers and the first ring's copy into it
-            mbar_init(&full[lane], 1);
+            mbar_init(&full[lane], records ? kDLoaders : 1);
             mbar_init(&empty[lane], 1);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        if (lane < S && lane < nstages) {
+        if (!records && lane < S && lane < nstages) {
             const int run = single ? 0 : lane / spt;
             load_stage(lane, run_src(run), lane - run * spt);
         }
@@ -496,7 +509,69 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
         }
     }
 
-    if (warp == 9) {
+    if constexpr (records) {
+        if (warp >= 10) {
+            // ---- loaders: packed records into what the tensor core reads -------------------------------------------------
+            // For plain products on packed records the kernel of gemv_fused.cu dequantises in registers, which bounds it by its ALU pipe; here nothing is
+            // computed on a weight.  Replayed, that kernel -> this one (weights beyond L2): 4096 x 4096, one to four tokens 6.9, 7.6, 8.5, 8.8 -> 5.7, 6.1, 7.3,
+            // 7.8 us; 12352 x 4096 11.3, 12.4, 13.1, 13.4 -> 9.0, 9.4, 10.2, 10.5; 4096 x 12288 12.5, 15.0, 17.3, 19.0 -> 9.4, 10.8, 13.6, 13.6; 248320 x 4096 103,
+            // 118, 117, 118 -> 94, 95, 99, 100 (5.7 TB/s).  With the unswizzled image, whose cells of a row lie 128 and 4096 bytes apart, 191.
+            // A record holds its rows' 64 bytes one after the other: K-major rows as the tensor core takes them with the 64-byte swizzle, which
+            // moves 16-byte cells about within a row.  So every cell goes straight to its place, 512 consecutive bytes of either side a warp.
+            // The scale bytes of rows g and g + 8 lie side by side: they come as they are, and the lane that asked for them sorts them when they are there.
+            const int w = warp - 10, g = lane & 7, t = lane >> 3;
+            const uint8_t *cells = p.seg[0].packed + lane * 16, *scales = p.seg[0].packed + 1024 + g * 8;
+            const int cell = (lane >> 2) * 64 + (((lane & 3) ^ ((lane >> 3) & 3)) << 4);
+            constexpr int kTiles = 8 / kDLoaders;
+            const int mine = kTiles * w + (t >> 1), raw = w * (128 * kTiles) + lane * 8, tiles = p.seg[0].rows >> 4; // the record whose scales this lane sorts
+            const bool sorts = lane < 16 * kTiles;
+            bool ok = true;
+            int slot = 0, done = 0, st = 0, unit = cl;
+            uint32_t phase = 1;
+#pragma unroll 1
+            for (int i = 0; i < nstages + kDLoadAhead && ok; i++) {
+                if (i < nstages) {
+                    if (i >= S) ok = mbar_wait(&empty[slot], phase, abort_flag);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    uint8_t *dst = ring + size_t(slot) * kStage;
+                    const int blocks = min(2, len - 2 * st);
+#pragma unroll
+                    for (int h = 0; h < kTiles; h++) { // this warp's tiles of the eight
+                        const int tile = unit * 8 + kTiles * w + h;
+                        const size_t rec = (size_t(tile) * nkb + kb0 + 2 * st) * kRec;
+#pragma unroll
+                        for (int b = 0; b < 2; b++)
+                            if (tile < tiles && b < blocks) {
+                                copy16(dst + b * kURec + cell + (2 * (kTiles * w + h)) * 512, cells + rec + b * kRec);
+                                copy16(dst + b * kURec + cell + (2 * (kTiles * w + h) + 1) * 512, cells + rec + b * kRec + 512);
+                            }
+                    }
+                    const int tile = unit * 8 + mine;
+                    if (sorts && tile < tiles && (t & 1) < blocks) copy8(dst + kDStage + raw, scales + (size_t(tile) * nkb + kb0 + 2 * st + (t & 1)) * kRec);
+                    if (++slot == S) { slot = 0; phase ^= 1; }
+                    if (++st == spt) { st = 0; unit += C; }
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");
+                if (i < kDLoadAhead) continue;
+                asm volatile("cp.async.wait_group %0;" ::"n"(kDLoadAhead) : "memory");
+                uint8_t *dst = ring + size_t(done) * kStage;
+                if (sorts) {
+                    const uint2 sc = *reinterpret_cast<const uint2 *>(dst + kDStage + raw); // row g: bytes 0, 2, 4, 6; row g + 8: 1, 3, 5, 7
+                    const int r = mine * 16 + g;
+                    uint8_t *block = dst + (t & 1) * kURec + 8192;
+                    *reinterpret_cast<uint32_t *>(block + (r & 31) * 16 + (r >> 5) * 4) = __byte_perm(sc.x, sc.y, 0x6420);
+                    *reinterpret_cast<uint32_t *>(block + ((r + 8) & 31) * 16 + (r >> 5) * 4) = __byte_perm(sc.x, sc.y, 0x7531);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full[done]);
+                if (++done == S) done = 0;
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+        }
+    }
+    if (warp == 9 && !records) {
         // ---- producer ----------------------------------------------------------------------------------------------------------
         {
             const bool one = elect_one();
@@ -553,7 +628,8 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
             // E2M1 x E2M1, UE8M0 scales, N columns, M = 128; K-step s of a block uses scale bytes 2s, 2s+1 of both operands
             constexpr uint32_t idesc0 = (1u << 7) | (1u << 10) | ((uint32_t(N) >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
             constexpr uint32_t idesc1 = idesc0 | (2u << 29) | (2u << 4);
-            const uint64_t da0 = umma_desc(smem_u32(ring), 128, 256), dsf0 = umma_desc(smem_u32(ring) + 8192, 16, 128), db0 = umma_desc(smem_u32(streamed ? ring + kDStage : bimg), 128, 256);
+            constexpr int kHalf = records ? 2 : 256; // from K-step to K-step of a block: 32 bytes of a row, or half of the image
+            const uint64_t da0 = records ? umma_desc(smem_u32(ring), 16, 512) | (uint64_t(4) << 61) : umma_desc(smem_u32(ring), 128, 256), dsf0 = umma_desc(smem_u32(ring) + 8192, 16, 128), db0 = umma_desc(smem_u32(streamed ? ring + kDStage : bimg), 128, 256);
             const uint64_t dsb0 = umma_desc(smem_u32(streamed ? ring + kDStage : bimg) + kBKb, 16, 128);
             bool ok = true;
             int st = 0, sfa = 0;
@@ -590,10 +666,10 @@ __global__ void __launch_bounds__(kDThreads, 2) umma_gemv_kernel(const __grid_co
                     copy_scales_if(one, sa, dsf);
                     if (two) copy_scales_if(one, sa + 4, dsf + (kURec >> 4));
                     mma_step_if(one, dcol, da, db, idesc0, kb > 0, sa, sb);
-                    mma_step_if(one, dcol, da + 256, db + (kBKb >> 5), idesc1, true, sa, sb);
+                    mma_step_if(one, dcol, da + kHalf, db + (kBKb >> 5), idesc1, true, sa, sb);
                     if (two) {
                         mma_step_if(one, dcol, da + (kURec >> 4), db + (kImg >> 4), idesc0, true, sa + 4, sb + 4);
-                        mma_step_if(one, dcol, da + (kURec >> 4) + 256, db + (kImg >> 4) + (kBKb >> 5), idesc1, true, sa + 4, sb + 4);
+                        mma_step_if(one, dcol, da + (kURec >> 4) + kHalf, db + (kImg >> 4) + (kBKb >> 5), idesc1, true, sa + 4, sb + 4);
                     }
                     commit_if(one, &empty[cur]);
                     if (!streamed) db += 2 * (kImg >> 4);
@@ -937,9 +1013,9 @@ DKernel gemv_kernel(int slots, int f)
 {
     constexpr int kP = kDPrepared;
     switch (slots) {
-    case 1: return variant_of<1, 0, kP, kP | kDTwo, kP | kDResidual, kP | kDPlain, kDLogits, kP | kDLogits, kDGated, kP | kDDelta>(f);
-    case 2: return variant_of<2, 0, kP, kP | kDTwo, kP | kDResidual, kP | kDPlain, kDGated>(f);
-    case 4: return variant_of<4, 0, kP, kP | kDTwo, kP | kDResidual, kP | kDPlain, kP | kDStreamed>(f);
+    case 1: return variant_of<1, 0, kP, kP | kDTwo, kP | kDResidual, kP | kDPlain, kDLogits, kP | kDLogits, kDGated, kP | kDDelta, kDRecords>(f);
+    case 2: return variant_of<2, 0, kP, kP | kDTwo, kP | kDResidual, kP | kDPlain, kDGated, kDRecords>(f);
+    case 4: return variant_of<4, 0, kP, kP | kDTwo, kP | kDResidual, kP | kDPlain, kP | kDStreamed, kDRecords>(f);
     default: return variant_of<8, 0, kP, kP | kDTwo, kP | kDResidual, kP | kDPlain, kP | kDStreamed>(f);
     }
 }
@@ -957,7 +1033,7 @@ int device_clusters(int *out)
     std::lock_guard<std::mutex> lock(g_attr_mutex);
     if (!g_max_clusters[dev]) {
         for (int slots : {1, 2, 4, 8})
-            for (int f = 0; f < 2 * kDDelta; f++)
+            for (int f = 0; f < 2 * kDRecords; f++)
                 if (const DKernel k = gemv_kernel(slots, f)) {
                     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
                     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(umma gemv)");
@@ -984,6 +1060,7 @@ int device_clusters(int *out)
 
 int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st, const insg_delta_op *step)
 {
+    const bool records = op && op->layout == 0; // one plain product of up to four tokens (insg_mxfp4_gemv_packed)
     if (!op || !op->in) return fail(INSG_E_ARG, "gemv: null operand");
     const int tokens = op->tokens > 1 ? op->tokens : 1;
     if (tokens > 8) return fail(INSG_E_SHAPE, "gemv: 1..8 tokens");
@@ -1057,38 +1134,35 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st, const insg_delta_o
     bool plain = whole; // epilogues that add nothing and leave nothing prepared
     for (int i = 0; i < p.nseg; i++) plain &= p.seg[i].epilogue != INSG_EPI_RESIDUAL && p.seg[i].epilogue != INSG_EPI_SWIGLU && p.seg[i].epilogue != INSG_EPI_LOGITS;
     const bool streamed = prep && T >= 4 && resid && kbq * kblock + exchange + 4 * kDStage > size_t(kDHalfSm);
-    const size_t stage_bytes = kDStage + (streamed ? 2 * kblock : 0);
+    const size_t stage_bytes = kDStage + (streamed ? 2 * kblock : 0) + (records ? 1024 : 0);
     const size_t fixed = exchange + (step ? sizeof(DeltaShared) : 0) + (streamed ? 0 : kbq * kblock) + (T == 8 && !prep ? size_t(8) * kDMaxKb * sizeof(float) : 0);
     // ring: no more stages than the launch has, within half an SM when that leaves at least four, else whatever fits.  Four are too
     // few to stream at full rate, so a launch of many units (the head: 55 per cluster, eight tokens 97 us against 91) takes the
     // whole SM; one of a few gains more from starting beside its predecessor.
     const int need = ((p.units + clusters - 1) / clusters) * p.nmat * ((kbq + 1) / 2);
     int stages = fixed < size_t(kDHalfSm) ? int((kDHalfSm - fixed) / stage_bytes) : 0;
-    if (stages < 4 || (stages == 4 && need > 96)) stages = int((size_t(222) * 1024 - fixed) / stage_bytes);
+    if (records || stages < 4 || (stages == 4 && need > 96)) stages = int((size_t(222) * 1024 - fixed) / stage_bytes);
     p.stages = std::max(1, std::min({stages, need, kDMaxStages}));
     p.ahead = !op->pdl ? 0 : T == 1 ? kDAheadStages<1> : T == 2 ? kDAheadStages<2> : kDAheadStages<4>; // a launch that waits for its predecessor anyway streams at once
     const size_t smem = fixed + size_t(p.stages) * stage_bytes;
 
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(clusters * kDCl));
-    cfg.blockDim = dim3(kDThreads);
+    cfg.blockDim = dim3(kDThreads + (records ? 32 * kDLoaders : 0));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = kDCl;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[1]; // the cluster's shape is part of the kernel
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = op->pdl ? 2 : 1;
+    cfg.numAttrs = op->pdl ? 1 : 0;
     if (step) {
         if (!prep || tokens != 1 || !whole || p.nseg != 1 || p.seg[0].epilogue != INSG_EPI_STORE || p.seg[0].rows != 4096) return fail(INSG_E_SHAPE, "deltanet: the gate's product takes one token, a prepared input and 4096 rows");
         p.delta = DDelta{step->state, step->q16, step->k16, step->v32, step->g32, step->beta32, step->out32, step->norm_w, static_cast<uint8_t *>(step->image)};
     }
     const bool gated = op->prologue == INSG_PRO_GATED_RMSNORM && !op->x_out && resid && T <= 2;
     const int special = step ? kDDelta : logits ? kDLogits : streamed ? kDStreamed : prep && whole && p.nmat == 2 ? kDTwo : prep && resid ? kDResidual : prep && plain ? kDPlain : gated ? kDGated : 0;
-    const DKernel kernel = gemv_kernel(T, special | (prep ? kDPrepared : 0));
+    const DKernel kernel = records ? gemv_kernel(T, kDRecords) : gemv_kernel(T, special | (prep ? kDPrepared : 0));
     if (!kernel) return fail(INSG_E_ARG, "gemv: no such variant");
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
     return e == cudaSuccess ? INSG_OK : cuda_fail(e, "umma gemv launch");
