@@ -29,7 +29,7 @@ divided by the slowest rank's time (weak scaling).
 If that library is absent it falls back to the CPU oracle port.
 
 ``--config 1`` times the MXFP4 matrix products alone (the model's three largest shapes at 1, 2, 4, 16 and 64
-tokens; 1-4 tokens on the mma.sync kernel, 16 and 64 on the tcgen05 kernel) and ``--config 2`` the attention
+tokens; 1-4 tokens on packed records, 16 and 64 through the tcgen05 GEMM) and ``--config 2`` the attention
 decode kernel over cached contexts of 1024, 8192 and 32768 tokens; both print one JSON line with a ``legs`` list and run on
 one GPU.
 
@@ -483,7 +483,7 @@ def run_kernel_configs(args):
                             ops.gemm_umma(packs[it[0] % copies], x, scratch=scratch)
                     else:
                         packs = [ops.repack(dw, ds) for _ in range(copies)]
-                        kernel = "gemv_fused_kernel (mma.sync)"
+                        kernel = "umma_gemv_kernel on packed records (tcgen05 kind::mxf4)"
 
                         def fn():
                             it[0] += 1
