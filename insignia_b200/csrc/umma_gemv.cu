@@ -91,6 +91,7 @@ struct DParams {
     const float *prep_partials; // prepared input: the producer's sums of squares, or null
     int cols, nkb, prologue, nseg, units, nmat, tokens, stages;
     int ahead; // stages beyond the ring to ask L2 for
+    int wait_first; // nothing may be read before the launch before this one has ended
     int late;  // the next launch reads what was there before this one: it may start when this launch's own wait is over
     DDelta delta;
     DSeg seg[4];
@@ -354,6 +355,10 @@ __global__ void __cluster_dims__(kDCl, 1, 1) __launch_bounds__(kDThreads + ((F &
     auto load_digits = [&](int slot, int st) { // streamed: behind the weights of the only run's stage st
         bulk_load(ring + size_t(slot) * kStage + kDStage, reinterpret_cast<const uint8_t *>(p.in) + size_t(kb0 + 2 * st) * kImg, uint32_t(min(2, len - 2 * st)) * kImg, &full[slot]);
     };
+    // Launches that may not read ahead (no pdl) start as early as the others and wait here, ahead of taking tensor memory that the launch before may still
+    // want; what follows them may start when they have waited, as if they had been launched then.  Calls one behind the other gain what a launch takes:
+    // 12352 x 4096 on packed records, three tokens 11.3 -> 9.2 us, 4096 x 4096, one 8.2 -> 7.5.
+    if (p.wait_first) pdl_wait();
     if (warp == 9) {
         if (lane < S) { // one lane per stage: its barriers and the first ring's copy into it
             mbar_init(&full[lane], records ? kDLoaders : 1);
@@ -391,7 +396,7 @@ __global__ void __cluster_dims__(kDCl, 1, 1) __launch_bounds__(kDThreads + ((F &
     // The next launch may become resident from here on, not earlier: were it to take tensor memory before every CTA here has its own,
     // a CTA could wait for memory held by a CTA that waits for this grid.
     const bool at_once = nstages - kDTriggerStages<T> <= S;
-    if (at_once && !(prepared && p.late)) pdl_launch_dependents();
+    if (records || (at_once && !(prepared && p.late))) pdl_launch_dependents();
     // The peers' barriers exist when this completes.  Their initialisation is published by the fences above; a release here waited for
     // whatever the SM still had under way, up to 2 us in a launch that could not start beside its predecessor (eight tokens 1540 -> 1503 us
     // a step, one token 1098 -> 1084).
@@ -1118,6 +1123,7 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st, const insg_delta_o
     }
     p.error_flag = static_cast<int *>(op->error_flag);
     p.late = op->pdl == 2;
+    p.wait_first = !op->pdl;
     int max_clusters = 0;
     const int rc = device_clusters(&max_clusters);
     if (rc != INSG_OK) return rc;
@@ -1155,7 +1161,7 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st, const insg_delta_o
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = op->pdl ? 1 : 0;
+    cfg.numAttrs = 1; // without pdl the launch starts as early, and waits before it reads
     if (step) {
         if (!prep || tokens != 1 || !whole || p.nseg != 1 || p.seg[0].epilogue != INSG_EPI_STORE || p.seg[0].rows != 4096) return fail(INSG_E_SHAPE, "deltanet: the gate's product takes one token, a prepared input and 4096 rows");
         p.delta = DDelta{step->state, step->q16, step->k16, step->v32, step->g32, step->beta32, step->out32, step->norm_w, static_cast<uint8_t *>(step->image)};
