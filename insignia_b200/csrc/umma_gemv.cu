@@ -19,7 +19,8 @@
 //
 // CTA roles (320 threads): warps 0-7 run the activation prologue (fused RMSNorm / gates, digits); then warps 0-3 read the
 // accumulators (tcgen05.ld, tensor-memory lane = row) and send the partial sums to the rows' owners, warps 4-7 add the
-// four parts and run the fused epilogue; warp 8 issues tcgen05.cp / tcgen05.mma, warp 9 the bulk copies.  Every wait is
+// four parts and run the fused epilogue; warp 8 issues tcgen05.cp / tcgen05.mma, warp 9 the bulk copies
+// (for packed records four more warps copy cells in its place).  In a launch with a DeltaNet step warps 0-7 make it at the end.  Every wait is
 // bounded: on expiry a flag is raised in global memory and all roles drain.
 //
 // Layout of the weights (insg_mxfp4_repack_umma): rows in tiles of 128, K in blocks of 128; one (tile, block) record is 8704
