@@ -358,7 +358,8 @@ INSG_API size_t insg_gqa_scratch_bytes(int tokens);
  * layout [token][4][256] of fp32 or bf16.  q fp32 [16][256] already normalised
  * and rotated.  `scratch` holds the per-split partials (see
  * insg_gqa_scratch_bytes); its first 64 bytes must be zero before the first call
- * and are left zero by every call.  Replaces gqa_decode
+ * and are left zero by every call.  Should a bounded wait inside the kernel run out,
+ * what it concerned is left as NaN.  Replaces gqa_decode
  * (include/insignia_attention.cuh:4, src/attention.cu:4-5), without its ~12K-token
  * shared-memory limit. */
 INSG_API int insg_gqa_decode(const float *q, const void *k_cache, const void *v_cache, float *out, int tokens,
@@ -403,8 +404,9 @@ typedef struct insg_attn_op {
     void *scratch;
     size_t scratch_bytes;
     int pdl;
-    int *error_flag;          /* device int set to 1 if a bounded wait inside the kernel ran out (bf16 cache, long contexts:
-                                 rows are staged by bulk copies with mbarrier completion), or NULL */
+    int *error_flag;          /* device int set to 1 if a bounded wait inside the kernel ran out, or NULL: on the parts of a
+                                 result that CTAs send one another, and (bf16 cache, long contexts) on rows staged by
+                                 bulk copies.  Flag or not, what such a wait concerned is left as NaN */
     void *image;              /* optional: besides out, the o projection's input out * sigmoid(gate) as the digit image of a
                                  layout-1 launch (insg_mxfp4_digit_image_bytes(4096, tokens), up to eight tokens or sequences) */
     int gate_elementwise;     /* with image: 1 = INSG_PRO_SIGMOID_GATE_QPROJ, 0 = INSG_PRO_SIGMOID_GATE_HEAD0 (aux = qraw)       */

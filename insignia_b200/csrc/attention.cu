@@ -39,6 +39,7 @@ constexpr int kTileRow = 528;                // a staged row: 512 bytes of bf16 
 constexpr int kTileBytes = 16 * kTileRow;    // 16 rows
 constexpr size_t kMmaSmem = size_t(kAtWarps) * 2 * kTileBytes; // per warp: a key tile and a value tile
 
+constexpr float kNan = __builtin_nanf("");
 __device__ __forceinline__ float warp_max_redux(float v) // maximum over the warp, as fmaxf takes it
 {
     float r;
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
     __shared__ __align__(8) uint64_t s_there;       // all of them have come
     __shared__ int s_last;
     __shared__ __align__(8) uint64_t s_bar[2 * kAtWarps];
-    __shared__ int s_abort;
+    __shared__ int s_abort, s_lost; // a wait of the tensor-core loop, or of the exchange, ran out
     __shared__ uint8_t s_lut[84];
     extern __shared__ __align__(128) uint8_t s_tiles[]; // bf16 cache only: per warp a key tile and a value tile
 
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
     const float *k_raw = p.k_raw + size_t(bt) * p.kvin_stride, *v_new = p.v_new + size_t(bt) * p.kvin_stride;
 
     if (tid == 0) {
-        s_abort = 0;
+        s_abort = s_lost = 0;
         mbar_init(&s_there, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -598,6 +599,7 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
                 l0 = fmaf(s_l[w][h], e, l0);
                 a.x = fmaf(x.x, e, a.x); a.y = fmaf(x.y, e, a.y); a.z = fmaf(x.z, e, a.z); a.w = fmaf(x.w, e, a.w);
             }
+            if (kMma && s_abort) l0 = kNan; // rows are missing
         }
         const uint32_t bar = map_to_rank(smem_u32(&s_there), owner);
         asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
@@ -613,7 +615,14 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
             Row::store(kc, row, s_knew[tid]);
             Row::store(vc, row, s_vnew[tid]);
         }
-    mbar_wait_cluster(&s_there, 0, &s_abort);
+    // (s_lost: a wait of the tensor-core loop that ran out does not cut this one short)
+    if (!mbar_wait_cluster(&s_there, 0, &s_lost)) { // what has not come counts as NaN, with an error flag or without
+#pragma unroll 1
+        for (int c = 0; c < CL; c++) {
+            if (tid < kMine) s_in[c][tid] = kNan;
+            s_ml[c] = make_float2(-3.0e38f, kNan);
+        }
+    }
     float mg = -3.0e38f, lg = 0.f, a = 0.f;
 #pragma unroll
     for (int c = 0; c < CL; c++)
@@ -626,6 +635,16 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
             lg = fmaf(ml.y, e, lg);
             if (tid < kMine) a = fmaf(s_in[c][tid], e, a);
         }
+    auto leave = [&] {
+        const bool lost = *static_cast<volatile int *>(&s_lost) != 0;
+        if ((lost || (tid == 0 && s_abort)) && p.error_flag) *p.error_flag = 1;
+        // Nobody leaves while a peer may still write into its shared memory.  Ordinarily all of it has come.  After a wait that ran out the peers
+        // have sent when they have left or stand here too, and what they sent gets the time of another wait to come in.
+        if (lost) {
+            asm volatile("barrier.cluster.arrive.relaxed;\nbarrier.cluster.wait;" ::: "memory");
+            mbar_wait_cluster(&s_there, 0, &s_lost);
+        }
+    };
     if (cut.active > 1) { // several clusters: partial results to scratch, the last one folds them in order
         float *part = partials + size_t(kvh * kSplits + cluster * kParts) * kPartFloats;
 #pragma unroll
@@ -645,7 +664,7 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
         }
         __syncthreads();
         if (!s_last) {
-            if (tid == 0 && s_abort && p.error_flag) *p.error_flag = 1;
+            leave();
             return;
         }
         __threadfence();
@@ -674,7 +693,7 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
         out_base[size_t(my_head) * 256 + my_dim] = a;
         if (p.image) group_digits(a * fast_sigmoid(gv), p.slots, bt, p.image, my_head * 8 + (my_dim >> 5), s_lut, lane);
     }
-    if (tid == 0 && s_abort && p.error_flag) *p.error_flag = 1;
+    leave();
 }
 
 template <bool BF16, bool FUSED, int CL, bool HALVES = false> static int launch_clusters(const AttnParams &p, cudaStream_t st, int along, int rows, int clusters)

@@ -39,7 +39,7 @@ struct AttnParams {
     int slots, gate_elementwise;
     int batch;             // several sequences share the launch
     int wait_first;        // nothing may be read before the launch before this one has ended
-    int *error_flag;       // set to 1 when a bounded wait inside the kernel ran out (bf16 tensor-core path), or null
+    int *error_flag;       // set to 1 when a bounded wait inside the kernel ran out (its results are NaN then), or null
 };
 
 // A lane's 8 dims of one cache row, as loaded (converted only when used, so that two token groups can be in flight).
