@@ -640,10 +640,8 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
         if ((lost || (tid == 0 && s_abort)) && p.error_flag) *p.error_flag = 1;
         // Nobody leaves while a peer may still write into its shared memory.  Ordinarily all of it has come.  After a wait that ran out the peers
         // have sent when they have left or stand here too, and what they sent gets the time of another wait to come in.
-        if (lost) {
-            asm volatile("barrier.cluster.arrive.relaxed;\nbarrier.cluster.wait;" ::: "memory");
-            mbar_wait_cluster(&s_there, 0, &s_lost);
-        }
+        if (p.leave_together || lost) asm volatile("barrier.cluster.arrive.relaxed;\nbarrier.cluster.wait;" ::: "memory");
+        if (lost) mbar_wait_cluster(&s_there, 0, &s_lost);
     };
     if (cut.active > 1) { // several clusters: partial results to scratch, the last one folds them in order
         float *part = partials + size_t(kvh * kSplits + cluster * kParts) * kPartFloats;
@@ -696,7 +694,7 @@ __global__ void __launch_bounds__(kAtThreads, 2) attn_splitk_kernel(const __grid
     leave();
 }
 
-template <bool BF16, bool FUSED, int CL, bool HALVES = false> static int launch_clusters(const AttnParams &p, cudaStream_t st, int along, int rows, int clusters)
+template <bool BF16, bool FUSED, int CL, bool HALVES = false> static int launch_clusters(AttnParams p, cudaStream_t st, int along, int rows, int clusters)
 {
     size_t smem = 0;
     if constexpr (BF16 && CL == 4 && !HALVES) { // the tensor-core loop's tiles: more than 48 KB of dynamic shared memory is a per-device opt-in
@@ -715,11 +713,20 @@ template <bool BF16, bool FUSED, int CL, bool HALVES = false> static int launch_
         if (p.max_context >= kMmaMinTokens) smem = kMmaSmem; // else no launch of these operands gets to the tensor-core loop
     }
     const int most = rows > 0 ? std::min(rows, p.max_context) : p.max_context;
-    if (!HALVES) { // as many as some row count up to `most` has at work: clusters without rows cost a launch of two sequences 3 us of 11
+    if (!HALVES) { // as many as some row count up to `most` has at work: clusters without rows cost a launch of two sequences 3 us of 11.  A plain launch's
+                   // count is known (1500 rows, called again and again, with three clusters 8.5 us, with a fourth that has no rows 10.7)
         const AttnRule rule = attn_rule(BF16, p.batch != 0, CL);
-        const int at_work = std::max(attn_clusters(rule, most, CL), attn_clusters(rule, std::min(most, rule.some), CL));
+        const bool known = !FUSED && !p.position;
+        const int at_work = std::max(attn_clusters(rule, known ? p.tokens : most, CL), known ? 1 : attn_clusters(rule, std::min(most, rule.some), CL));
         clusters = std::max(1, std::min({clusters, kMaxClusters, at_work}));
     }
+    // A launch that started beside this one takes its places as they come free, a cluster of eight at a time.  Where several clusters share a head, those of a
+    // cluster's CTAs that arrive last fold and end later than the others: the next launch's clusters then found places for 28 to 31 of 32 and the rest
+    // began when the first had ended (8545 rows, called again and again: a call in two took 30 us instead of 20).  Ending as one costs them nothing.
+    // Replayed, CTAs ending one by one / as one / launches that start when the one before has ended: 3600 rows 14.6 / 11.9 / 12.6 us, 6000 rows 18.0 / 14.5 /
+    // 15.4, 2 x 6000 26.4 / 22.4 / 22.8, 4 x 2047 18.7 / 16.8 / 16.9.  Not where the grid is more than the device holds, whose own later CTAs take the places
+    // (eight tokens at 4096 rows 83.7 / 84.9), and not with clusters of four, which find places (three sequences of 4096 rows 24.7 / 24.8).
+    if (CL == 8 && p.wait_first && clusters > 1 && 4 * clusters * CL * along <= 2 * sm_count()) p.leave_together = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(4 * clusters * CL, along);
     cfg.blockDim = dim3(kAtThreads);

@@ -38,6 +38,7 @@ struct AttnParams {
     uint8_t *image;
     int slots, gate_elementwise;
     int batch;             // several sequences share the launch
+    int leave_together;    // a cluster's CTAs end as one (launch_clusters)
     int wait_first;        // nothing may be read before the launch before this one has ended
     int *error_flag;       // set to 1 when a bounded wait inside the kernel ran out (its results are NaN then), or null
 };
