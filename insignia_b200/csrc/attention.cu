@@ -786,7 +786,8 @@ template <bool BF16> __global__ void __launch_bounds__(kAtThreads) attn_chunk_pr
     using Row = KvRow<BF16>;
     const int m = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     pdl_wait();
-    pdl_launch_dependents();
+    // What follows a chunk's rows waits before it reads them.  What follows the rows alone may be a step that fetches them ahead of its wait.
+    if (qn) pdl_launch_dependents();
     const int pos = __ldcg(p.position) + p.position_offset + m;
     if (pos < 0 || pos >= p.max_context) return; // host checks; never index past the cache
     float rope_c[8], rope_s[8];

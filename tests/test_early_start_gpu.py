@@ -62,3 +62,42 @@ def test_calls_one_behind_the_other_see_what_was_written_before(cuda):
         for _ in range(3):
             for a, b in zip(_calls(ops, make(), lambda: None), apart):
                 assert np.array_equal(a, b)
+
+
+def _rows_then_step(ops, gen, between, tokens, alone):
+    """The rows of `tokens` tokens, alone or with their attention, and the next token's step, which fetches rows ahead of its wait."""
+    import ctypes as C
+
+    from insignia_b200 import _lib
+
+    L, ctx = _lib.lib(), tokens + 1
+    randn = lambda *s: torch.randn(*s, generator=gen, device="cuda")  # noqa: E731
+    kc, vc, raw, last = randn(ctx * 1024), randn(ctx * 1024), (randn(tokens, 8192), randn(tokens, 1024), randn(tokens, 1024)), (randn(1, 8192), randn(1, 1024), randn(1, 1024))
+    norm = torch.ones(256, device="cuda").to(torch.bfloat16).view(torch.int16)
+    first, next_ = (torch.full((1,), at, dtype=torch.int32, device="cuda") for at in (0, tokens))
+    scratch = torch.zeros(max(1, min(tokens, 32)) * ops.gqa_scratch("cuda").numel(), dtype=torch.uint8, device="cuda")
+    between()
+    if alone:
+        op = _lib.AttnOp()
+        op.k_raw, op.v, op.k_norm_w, op.k_cache, op.v_cache, op.position = (t.data_ptr() for t in (raw[1], raw[2], norm, kc, vc, first))
+        op.max_context, op.kv_dtype, op.fast_trig = ctx, ops.KV_F32, 1
+        _lib.check(L.insg_attention_rows(C.byref(op), tokens, torch.cuda.current_stream().cuda_stream))
+        got = []
+    else:
+        got = [ops.attention_chunk(*raw, norm, norm, kc, vc, first, ctx, scratch, tokens)]
+    between()
+    got += [ops.attention_step(*last, norm, norm, kc, vc, next_, ctx, scratch, pdl=True), kc, vc]
+    torch.cuda.synchronize()
+    return [host(t) for t in got]
+
+
+@pytest.mark.parametrize("tokens,alone", [(3, True), (1500, True), (3, False), (20, False), (300, False)])
+def test_a_step_that_reads_ahead_sees_the_rows_of_the_call_before(cuda, tokens, alone):
+    from insignia_b200 import ops
+
+    for seed in range(4):
+        make = lambda: torch.Generator(device="cuda").manual_seed(seed)  # noqa: E731
+        apart = _rows_then_step(ops, make(), torch.cuda.synchronize, tokens, alone)
+        for _ in range(4):
+            for a, b in zip(_rows_then_step(ops, make(), lambda: None, tokens, alone), apart):
+                assert np.array_equal(a, b)
