@@ -332,7 +332,8 @@ INSG_API int insg_deltanet_decode_gated(float *state, long long state_stride, co
  * then image as insg_deltanet_decode_gated leaves it for one sequence, all with the bits of insg_gemv_fused, insg_deltanet_decode
  * and the INSG_PRO_GATED_RMSNORM prologue.  With gate->pdl the product is made ahead of the wait for the launch before this
  * one: that launch must be an insg_gemv_fused with pdl = 2 (it makes q, k, v, g and beta), and must not write gate's input.
- * Where the GPU cannot hold the 32 clusters of four CTAs at once the product and insg_deltanet_decode_gated run one after the other. */
+ * Where the GPU cannot hold the 32 clusters of four CTAs at once it runs insg_deltanet_gated_step_apart: the product, the step and the digits as three
+ * launches, with the same requirements and the same bits. */
 typedef struct insg_delta_op {
     float *state;             /* fp32 [32][128][128], in place */
     const float *q16, *k16, *v32, *g32, *beta32;
@@ -341,6 +342,7 @@ typedef struct insg_delta_op {
     void *image;              /* insg_mxfp4_digit_image_bytes(4096, 1) bytes */
 } insg_delta_op;
 INSG_API int insg_deltanet_gated_step(const insg_gemv_op *gate /* host */, const insg_delta_op *step /* host */, insg_stream_t stream);
+INSG_API int insg_deltanet_gated_step_apart(const insg_gemv_op *gate /* host */, const insg_delta_op *step /* host */, insg_stream_t stream);
 /* Convolution history [channels][3] after a rejected second token: from the history after two tokens (`state`, in
  * place) and the history before them (`snapshot`).  No reference counterpart. */
 INSG_API int insg_conv_rollback(float *state, const float *snapshot, long long channels, insg_stream_t stream);

@@ -88,6 +88,7 @@ SIGNATURES = {
     "insg_deltanet_decode_verify": (i32, [vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, vp]),
     "insg_deltanet_decode_gated": (i32, [vp, C.c_longlong] + [vp] * 6 + [i32, i32, vp, vp, vp, i32, vp]),
     "insg_deltanet_gated_step": (i32, [C.POINTER(GemvOp), C.POINTER(DeltaOp), vp]),
+    "insg_deltanet_gated_step_apart": (i32, [C.POINTER(GemvOp), C.POINTER(DeltaOp), vp]),
     "insg_conv_rollback": (i32, [vp, vp, C.c_longlong, vp]),
     "insg_gqa_scratch_bytes": (sz, [i32]),
     "insg_gqa_decode": (i32, [vp, vp, vp, vp, i32, i32, vp, sz, vp]),

@@ -1064,6 +1064,37 @@ int device_clusters(int *out)
 }
 } // namespace
 
+// What the gated-norm prologue makes of a step's output, as a launch of its own: the digits of one token, a warp per head, with its order of every sum.
+constexpr int kDigitHeads = 4;
+__global__ void __launch_bounds__(32 * kDigitHeads) gated_digits_kernel(const float *core, const float *z, const uint16_t *norm_w, uint8_t *image)
+{
+    __shared__ uint8_t s_lut[84];
+    const int tid = threadIdx.x, lane = tid & 31, head = blockIdx.x * kDigitHeads + (tid >> 5);
+    if (tid < 81) s_lut[tid] = digit_pair_code(tid);
+    __syncthreads();
+    const uint2 w = reinterpret_cast<const uint2 *>(norm_w)[lane];
+    pdl_wait();
+    float4 v = __ldcg(reinterpret_cast<const float4 *>(core) + head * 32 + lane);
+    const float4 g = __ldcg(reinterpret_cast<const float4 *>(z) + head * 32 + lane);
+    const float inv = rsqrtf(warp_sum(fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w)))) / 128.f + 1e-6f);
+    v.x = v.x * inv * bf16_bits_to_float(w.x & 0xffff) * fast_silu(g.x);
+    v.y = v.y * inv * bf16_bits_to_float(w.x >> 16) * fast_silu(g.y);
+    v.z = v.z * inv * bf16_bits_to_float(w.y & 0xffff) * fast_silu(g.z);
+    v.w = v.w * inv * bf16_bits_to_float(w.y >> 16) * fast_silu(g.w);
+    store_digits(v, 1, 0, image + size_t(head) * 1024, s_lut, lane);
+}
+
+static int check_gated_step(const insg_gemv_op *gate, const insg_delta_op *step)
+{
+    if (!gate || !step || !step->state || !step->q16 || !step->k16 || !step->v32 || !step->g32 || !step->beta32 || !step->out32 || !step->norm_w || !step->image)
+        return fail(INSG_E_ARG, "deltanet: null pointer");
+    if (gate->layout != 1) return fail(INSG_E_SHAPE, "deltanet: the gate's product takes the tcgen05 layout");
+    if (gate->prologue != INSG_PRO_PREPARED || gate->tokens > 1 || gate->n_segments != 1 || gate->seg[0].epilogue != INSG_EPI_STORE || gate->seg[0].rows != 4096 ||
+        gate->cols <= 0 || gate->cols % 1024)
+        return fail(INSG_E_SHAPE, "deltanet: the gate's product takes one token, a prepared input of a multiple of 1024 columns and one stored segment of 4096 rows");
+    return INSG_OK;
+}
+
 int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st, const insg_delta_op *step)
 {
     const bool records = op && op->layout == 0; // one plain product of up to four tokens (insg_mxfp4_gemv_packed)
@@ -1164,7 +1195,6 @@ int gemv_umma_launch(const insg_gemv_op *op, cudaStream_t st, const insg_delta_o
     cfg.attrs = attr;
     cfg.numAttrs = 1; // without pdl the launch starts as early, and waits before it reads
     if (step) {
-        if (!prep || tokens != 1 || !whole || p.nseg != 1 || p.seg[0].epilogue != INSG_EPI_STORE || p.seg[0].rows != 4096) return fail(INSG_E_SHAPE, "deltanet: the gate's product takes one token, a prepared input and 4096 rows");
         p.delta = DDelta{step->state, step->q16, step->k16, step->v32, step->g32, step->beta32, step->out32, step->norm_w, static_cast<uint8_t *>(step->image)};
     }
     const bool gated = op->prologue == INSG_PRO_GATED_RMSNORM && !op->x_out && resid && T <= 2;
@@ -1183,16 +1213,19 @@ extern "C" {
 
 int insg_deltanet_gated_step(const insg_gemv_op *gate, const insg_delta_op *step, insg_stream_t stream)
 {
-    if (!gate || !step || !step->state || !step->q16 || !step->k16 || !step->v32 || !step->g32 || !step->beta32 || !step->out32 || !step->norm_w || !step->image)
-        return fail(INSG_E_ARG, "deltanet: null pointer");
-    if (gate->layout != 1) return fail(INSG_E_SHAPE, "deltanet: the gate's product takes the tcgen05 layout");
-    int clusters = 0;
-    int rc = device_clusters(&clusters);
-    if (rc == INSG_OK && clusters >= 32) return gemv_umma_launch(gate, stream, step);
-    if (rc == INSG_OK) rc = gemv_umma_launch(gate, stream, nullptr);
+    int clusters = 0, rc = check_gated_step(gate, step);
+    if (rc == INSG_OK) rc = device_clusters(&clusters);
     if (rc != INSG_OK) return rc;
-    return insg_deltanet_decode_gated(step->state, 32 * 128 * 128, step->q16, step->k16, step->v32, step->g32, step->beta32, step->out32, 1, 0, gate->seg[0].out, step->norm_w,
-                                      step->image, gate->pdl, stream);
+    return clusters >= 32 ? gemv_umma_launch(gate, stream, step) : insg_deltanet_gated_step_apart(gate, step, stream);
+}
+
+int insg_deltanet_gated_step_apart(const insg_gemv_op *gate, const insg_delta_op *step, insg_stream_t stream)
+{
+    int rc = check_gated_step(gate, step);
+    if (rc == INSG_OK) rc = gemv_umma_launch(gate, stream, nullptr);
+    if (rc == INSG_OK) rc = insg_deltanet_decode(step->state, step->q16, step->k16, step->v32, step->g32, step->beta32, step->out32, gate->pdl, stream);
+    if (rc == INSG_OK) rc = launch(gated_digits_kernel, dim3(32 / kDigitHeads), dim3(32 * kDigitHeads), 0, stream, true, step->out32, gate->seg[0].out, step->norm_w, static_cast<uint8_t *>(step->image));
+    return rc;
 }
 
 size_t insg_mxfp4_digit_image_bytes(int cols, int tokens)

@@ -69,3 +69,21 @@ def test_three_tokens_of_very_many_rows_are_not_refused(rows, cols):
         pytest.skip("would launch")
     L = _lib.lib()
     assert [L.insg_mxfp4_gemv_packed(SOME, SOME, SOME, rows, cols, m, None) for m in (1, 2, 3)] == [-2] * 3  # INSG_E_CUDA
+
+
+@pytest.mark.parametrize("entry", ["insg_deltanet_gated_step", "insg_deltanet_gated_step_apart"])
+@pytest.mark.parametrize("change", [dict(layout=0), dict(tokens=2), dict(prologue="plain"), dict(cols=896), dict(cols=0), dict(rows=2048), dict(epilogue="residual"), dict(n_segments=2)])
+def test_a_gated_step_takes_one_kind_of_product_on_every_route(entry, change):
+    """The step reads 4096 gates of the product whichever way it goes: what does not make them is refused before the way is chosen."""
+    from insignia_b200 import _lib, ops
+
+    kw = dict(rows=4096, cols=1024, prologue="prepared")
+    kw.update(change)
+    epilogue = kw.pop("epilogue", "store")
+    op, step = gemv_op(**kw), _lib.DeltaOp()
+    op.seg[0].epilogue = ops.EPI[epilogue]
+    for name, _ in step._fields_:
+        setattr(step, name, SOME)
+    assert getattr(_lib.lib(), entry)(C.byref(op), C.byref(step), None) == E_SHAPE
+    step.norm_w = None
+    assert getattr(_lib.lib(), entry)(C.byref(op), C.byref(step), None) == E_ARG
