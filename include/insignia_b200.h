@@ -221,7 +221,7 @@ typedef struct insg_gemv_op {
     int *error_flag;          /* set to 1 if a bounded wait inside the kernel ran out (device int), or NULL                 */
     int pdl;                  /* 1: launch with programmatic dependent launch, weights and states read ahead of the wait
                                  (0: layout 1 launches start as early and wait before they read anything); 2: and the launch after this one is
-                                 insg_deltanet_gated_step (layout 1, INSG_PRO_PREPARED, up to eight tokens)          */
+                                 insg_deltanet_gated_step (refused but for layout 1, INSG_PRO_PREPARED, up to eight tokens) */
     const float *prep_partials; /* INSG_PRO_PREPARED: the producer's prep_partials (layout 0: [296], layout 1:
                                    [tokens][cols / 32]), or NULL                                                         */
     int prep_rms;               /* INSG_PRO_PREPARED: 1 = scale by the RMS factor computed from prep_partials (layout 1

@@ -203,6 +203,9 @@ size_t insg_gemv_argmax_scratch_bytes(void) { return 64 + size_t(8) * 512; }
 
 int insg_gemv_fused(const insg_gemv_op *op, insg_stream_t stream)
 {
+    // The launch behind one with pdl = 2 reads ahead of its wait what the launch before this one wrote: only these launches let it start no earlier than that
+    if (op && op->pdl == 2 && (op->layout != 1 || op->prologue != INSG_PRO_PREPARED || op->tokens > 8))
+        return fail(INSG_E_ARG, "gemv: pdl = 2 takes layout 1, a prepared input and up to eight tokens");
     if (op && op->layout == 1) return op->tokens > 8 ? gemm_umma_launch(op, stream) : gemv_umma_launch(op, stream, nullptr);
     return gemv_fused_launch(op, op && op->tokens > 1 ? op->tokens : 1, stream);
 }

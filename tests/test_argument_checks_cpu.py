@@ -87,3 +87,13 @@ def test_a_gated_step_takes_one_kind_of_product_on_every_route(entry, change):
     assert getattr(_lib.lib(), entry)(C.byref(op), C.byref(step), None) == E_SHAPE
     step.norm_w = None
     assert getattr(_lib.lib(), entry)(C.byref(op), C.byref(step), None) == E_ARG
+
+
+@pytest.mark.parametrize("change", [dict(layout=0), dict(prologue="plain"), dict(prologue="rmsnorm", norm_w=SOME), dict(tokens=9)])
+def test_a_launch_that_does_not_hold_back_the_gated_step_is_refused(change):
+    """pdl = 2 promises that the launch behind starts when this launch's own input is complete; other launches let it start at once."""
+    from insignia_b200 import _lib
+
+    op = gemv_op(**{**dict(prologue="prepared", pdl=2, umma_scratch=SOME, umma_scratch_bytes=1 << 40), **change})
+    assert _lib.lib().insg_gemv_fused(C.byref(op), None) == E_ARG
+    assert b"pdl = 2" in _lib.lib().insg_last_error()
