@@ -299,6 +299,62 @@ __device__ __forceinline__ void delta_step(const DDelta &d, float4 (&cell)[4], D
     group_digits(o * inv * gw * fast_silu(sh.z[lane]), 1, 0, d.image, head * 4 + slice, lut, lane);
 }
 
+// Plain products on packed records take any activation and any scale byte, as on mma.sync.  Digits alone do not: below 2^-103 a group's largest element has
+// fewer than 24 bits, and with scale bytes below 24 the digit columns are subnormal in tensor memory.  So the digits are those of 2^64 x (kDLift), and
+// the sums are taken back by 2^-64: the same bits, and zeros stay exact.  What leaves the range at its other end (elements from 2^64 on, sums that overflow),
+// the scale byte 255 (infinity, in digits NaN) and sums of groups with the scale byte 0 (nothing, in digits 2^-127: at most 2^-110 of the token's largest
+// element, 12288 of them) are told by a sum that is not finite or below kDFewBits of that element, and its row is added up once more in fp32, each group's
+// factor, weights' and token's, applied to its finished sum.  A warp takes four rows of its 32 (in `mask`) at a time, a lane a group of 32 columns; 32 rows of
+// 4096 columns take it 80 us.  Ordinary products: 4096 x 4096 with one to four tokens, replayed, 4.9, 5.5, 6.5, 6.6 us without all this, 4.6, 5.2, 6.2, 6.3 like this.
+constexpr float kDLift = 18446744073709551616.f;        // 2^64
+constexpr float kDFewBits = 5.16987882845642297e-26f;   // 2^-84
+__device__ __noinline__ float rows_again(const uint8_t *packed, const float *x, int nkb, int row0, uint32_t mask, uint32_t top, float y, int lane)
+{
+    const int eb = min(max(int(top >> 23), 1), 253);
+    const float alpha = __uint_as_float(uint32_t(254 - eb) << 23); // the largest element to [1, 4), a subnormal one to 2^-23 at least
+#pragma unroll 1
+    while (mask) {
+        int r[4];
+        const uint8_t *cells[4];
+        float acc[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            r[i] = mask ? __ffs(mask) - 1 : r[0];
+            mask &= mask - 1u;
+            const int row = row0 + r[i];
+            cells[i] = packed + size_t(row >> 4) * nkb * kRec;
+            acc[i] = 0.f;
+        }
+#pragma unroll 1
+        for (int g = lane; g < nkb * 4; g += 32) {
+            const size_t rec = size_t(g >> 2) * kRec;
+            float part[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+            for (int j = 0; j < 4; j++) { // eight columns
+                const float4 a = __ldcg(reinterpret_cast<const float4 *>(x + g * 32 + j * 8)), b = __ldcg(reinterpret_cast<const float4 *>(x + g * 32 + j * 8 + 4));
+                const float v[8] = {a.x * alpha, a.y * alpha, a.z * alpha, a.w * alpha, b.x * alpha, b.y * alpha, b.z * alpha, b.w * alpha};
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const uint32_t q = *reinterpret_cast<const uint32_t *>(cells[i] + rec + ((row0 + r[i]) & 15) * 64 + (g & 3) * 16 + j * 4);
+#pragma unroll
+                    for (int k = 0; k < 8; k++) part[i] = fmaf(e2m1_to_float(q >> (4 * k)), v[k], part[i]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int tile_row = (row0 + r[i]) & 15, sc = cells[i][rec + 1024 + (tile_row & 7) * 8 + (g & 3) * 2 + (tile_row >> 3)];
+                if (sc) acc[i] += sc == 255 ? part[i] * __int_as_float(0x7f800000) : ldexpf(part[i], sc + eb - 254);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float sum = warp_sum(acc[i]);
+            if (lane == r[i]) y = sum;
+        }
+    }
+    return y;
+}
+
 template <int T, int F>
 __global__ void __cluster_dims__(kDCl, 1, 1) __launch_bounds__(kDThreads + ((F & kDRecords) != 0 ? 32 * kDLoaders : 0), (F & kDRecords) != 0 ? 1 : 2) umma_gemv_kernel(const __grid_constant__ DParams p)
 {
@@ -498,6 +554,12 @@ __global__ void __cluster_dims__(kDCl, 1, 1) __launch_bounds__(kDThreads + ((F &
                 }
                 if (!(F & kDGated) && p.x_out && cl == 0 && !rms && m < p.tokens)
                     reinterpret_cast<float4 *>(p.x_out + size_t(m) * p.cols)[(kb0 + kb) * 32 + lane] = v;
+                if constexpr (records) { // the k-block's largest magnitude (rows_again)
+                    const uint32_t bx = __float_as_uint(fabsf(v.x)), by = __float_as_uint(fabsf(v.y)), bz = __float_as_uint(fabsf(v.z)), bw = __float_as_uint(fabsf(v.w));
+                    const uint32_t top = __reduce_max_sync(0xffffffffu, max(max(bx, by), max(bz, bw)));
+                    if (lane == 0) s_ssq[m * kDMaxKb + kb] = __uint_as_float(top);
+                }
+                if constexpr (records) { v.x *= kDLift; v.y *= kDLift; v.z *= kDLift; v.w *= kDLift; }
                 store_digits(v, T, m, bimg + size_t(kb) * kImg, s_lut, lane);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // the tensor core reads the image through the async proxy
                 __syncwarp();
@@ -511,6 +573,9 @@ __global__ void __cluster_dims__(kDCl, 1, 1) __launch_bounds__(kDThreads + ((F &
             if (rms)
 #pragma unroll 4
                 for (int kb = 0; kb < len; kb++) ss[0] += s_ssq[m * kDMaxKb + kb];
+            if (records) // (and its largest magnitude, as bits)
+#pragma unroll 4
+                for (int kb = 0; kb < len; kb++) ss[0] = __uint_as_float(max(__float_as_uint(ss[0]), __float_as_uint(s_ssq[m * kDMaxKb + kb])));
             send_floats<1>(map_to_rank(smem_u32(&s_rss[rank * T + m]), uint32_t(dst)), ss, map_to_rank(smem_u32(&ssfull), uint32_t(dst)));
         }
     }
@@ -738,7 +803,7 @@ __global__ void __cluster_dims__(kDCl, 1, 1) __launch_bounds__(kDThreads + ((F &
 #pragma unroll
         for (int u = 0; u < TN; u++) {
             const int t = t0 + u;
-            float sc = 1.f;
+            float sc = records ? 1.f / kDLift : 1.f;
             if (prepared && p.prep_partials) {
                 const int groups = p.cols >> 5;
                 float ss = 0.f;
@@ -842,6 +907,17 @@ __global__ void __cluster_dims__(kDCl, 1, 1) __launch_bounds__(kDThreads + ((F &
             if (!delta && i + kGroups >= nun) { // nothing more comes in for this warp: the peers need not wait for its epilogue
                 cluster_arrive_relaxed();
                 arrived = true;
+            }
+            if constexpr (records) {
+#pragma unroll
+                for (int u = 0; u < TN; u++) {
+                    const int t = t0 + u;
+                    const uint32_t top = max(max(__float_as_uint(s_rss[t]), __float_as_uint(s_rss[T + t])), max(__float_as_uint(s_rss[2 * T + t]), __float_as_uint(s_rss[3 * T + t])));
+                    const float a = fabsf(y[0][u]);
+                    const uint32_t again = __ballot_sync(0xffffffffu, on && t < p.tokens && (!(a <= 3.402823466e38f) || (a > 0.f && a < kDFewBits * __uint_as_float(top))));
+                    if (again && top < 0x7f800000u) // (a token with an infinity or NaN is NaN)
+                        y[0][u] = rows_again(s.packed, p.in + size_t(t) * p.cols, nkb, row - lane, again, top, y[0][u], lane);
+                }
             }
             if (!on) continue;
             if constexpr (delta) {
