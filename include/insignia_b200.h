@@ -119,7 +119,8 @@ INSG_API int insg_mxfp4_repack_umma(const uint32_t *weight, const uint8_t *scale
  * the kernel the engine runs; replaces Qwen35Decode::linear (src/decode.cu:13).
  * Tokens go through in passes of four (the weights are streamed once per pass).  Matrices of 12 * 2^20 weights and more run on
  * tcgen05, smaller ones on mma.sync; either way a token's result does not depend on the tokens beside it, an infinity or NaN in x[m] makes
- * y[m] NaN, a scale byte of 255 counts as infinity (its row is infinite or NaN) and one of 0 as nothing. */
+ * y[m] NaN, a scale byte of 255 counts as infinity (its row is infinite or NaN) and one of 0 as nothing.  Should a bounded
+ * wait inside the tcgen05 kernel run out, the rows it concerned are left as NaN. */
 INSG_API int insg_mxfp4_gemv_packed(const void *packed, const float *x, float *y, int rows, int cols, int M,
                                     insg_stream_t stream);
 

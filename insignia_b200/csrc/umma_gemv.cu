@@ -853,8 +853,9 @@ __global__ void __cluster_dims__(kDCl, 1, 1) __launch_bounds__(kDThreads + ((F &
             }
         };
         if (kAhead && ok && group < nun) fetch(group);
+        int i = group;
 #pragma unroll 1
-        for (int i = group; i < nun && ok; i += kGroups) {
+        for (; i < nun && ok; i += kGroups) {
             const int unit = cl + i * C;
             const DSeg &s = seg_of(unit);
             const int row = (unit - s.tile_begin) * 128 + rank * 32 + lane;
@@ -985,6 +986,14 @@ __global__ void __cluster_dims__(kDCl, 1, 1) __launch_bounds__(kDThreads + ((F &
                 }
             }
         }
+        if constexpr (records) // after a wait that ran out: a plain product has no error flag, so what it leaves out must not pass for a result
+            if (!ok)
+#pragma unroll 1
+                for (; i < nun; i += kGroups) {
+                    const int row = (cl + i * C) * 128 + rank * 32 + lane;
+                    for (int t = t0; t < min(t0 + TN, p.tokens); t++)
+                        if (row < p.seg[0].rows) p.seg[0].out[t * size_t(p.seg[0].rows) + row] = __int_as_float(0x7fc00000);
+                }
         if constexpr (logits) {
             // per-CTA arg-max, then the last CTA of the grid folds the CTAs' (lowest index on ties)
             auto fold = [&] {
