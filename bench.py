@@ -14,7 +14,7 @@ the same ModelFile -> TieredStorage path a real checkpoint takes.
   the same context length) until about two seconds have been timed; the median block counts.
 * ``e2e``    tok/s through the reference-facing call Qwen35Decode::decode_token(int) -> int: the token id goes
   host -> device and the result device -> host every step; same repetition rule.
-* ``roofline``  the fused GEMV kernel: algorithmic weight bytes of its 129 launches per token / the time of those
+* ``roofline``  the fused GEMV kernel: algorithmic weight bytes of its 152 launches per token / the time of those
   launches replayed alone (CUDA events), against the measured HBM copy bandwidth of MEASURED_PEAKS.json.
 * ``cpu_baseline``  the CPU oracle port (oracle/, C + OpenMP) decoding a few tokens of the same model on the host cores;
   ``cpu_baseline_legs`` adds the DeltaNet-layer workload of configs[0] on the port and with pre-dequantised weights.

@@ -597,7 +597,7 @@ INSG_API int insg_engine_generate(insg_engine *e, int first_token, int count, in
 INSG_API int insg_engine_prime_speculative(insg_engine *e, const int *prompt /* host */, int count);
 INSG_API int insg_engine_generate_speculative(insg_engine *e, int first_token, int count, int *out_tokens /* host */,
                                               int *accepted /* host */, const int *forced_drafts /* host */);
-/* The fused-GEMV operations of one token step alone, run `replays` (1..64) times between two CUDA events (one
+/* The fused-GEMV operations of one token step alone, a gate's product without the DeltaNet step beside it, run `replays` (1..64) times between two CUDA events (one
  * CUDA graph of launches with dependent-launch overlap per replay, or with `persistent` one persistent launch):
  * *ms_per_token = time of one replay, *bytes = the algorithmic weight bytes of those operations, *launches = their
  * count.  Needs one forwarded token first.  The sequence state is meaningless afterwards (call insg_engine_reset).

@@ -109,7 +109,7 @@ public:
     uint64_t launch_count() const noexcept { return launches_; }
     cudaStream_t execution_stream();
     // Additive: the fused-GEMV operations of one token step alone (no DeltaNet, attention or embedding work between
-    // them), run `replays` times between two events: as a graph of launches with dependent-launch overlap, or with
+    // them or, for a gate's product, beside it), run `replays` times between two events: as a graph of launches with dependent-launch overlap, or with
     // `persistent` as one persistent launch each.  Gives the weight-streaming time of a token.  The sequence state
     // (hidden, convolution history) is meaningless afterwards: reset the workspace before decoding again.
     void profile_gemv_chain(int replays, float *ms_per_token, uint64_t *bytes, int *launches);

@@ -173,7 +173,7 @@ template <int T> __host__ __device__ constexpr int unit_slots(int nmat) { return
 // segment that adds into the residual stream, one unit per cluster (kDResidual; with digits that come with the weights kDStreamed, behind the
 // gated norm kDGated); epilogues that add nothing and leave nothing prepared (kDPlain); a DeltaNet step beside the product that gates its output
 // (kDDelta); weights that come as the packed records of insg_mxfp4_repack (kDRecords).  A launch that fits none takes the general ones.
-// A token is 129 launches of some seven microseconds, and instructions that a launch runs through for the first time come from L2 behind the
+// A token is 152 of these launches, five to six microseconds each (129 when these figures were taken, the gates' products in the in-projections), and instructions that a launch runs through for the first time come from L2 behind the
 // stream of weights.  Microseconds of a device-fed token (a host-fed decode_token gained half of it), a step of three sequences, of eight, and a
 // speculative pass (a process is now and then 2 % off for all of its life), and the code of a launch (the last line: of the special variants; what
 // takes a general one runs up to 82 KB):

@@ -227,7 +227,7 @@ struct Ctx {
     void *prep_hidden() const { return static_cast<uint8_t *>(x.prep) + kPrepHidden; }
     void *prep_act() const { return static_cast<uint8_t *>(x.prep) + kPrepAct; }
     void *prep_core() const { return static_cast<uint8_t *>(x.prep) + kPrepCore; }
-    bool core_prepared() const { return tcgen05() && prepared() && !gemv_only; } // the attention step leaves the next product's digits
+    bool core_prepared() const { return tcgen05() && prepared(); } // the step leaves the next product's digits (gemv_only: those of some token before)
     float *prep_sums() const { return reinterpret_cast<float *>(static_cast<uint8_t *>(x.prep) + kPrepSums); }
     bool tcgen05() const { return tcgen05_engine(x.options); }
     bool prepared() const { return x.options.prepared_inputs; }
@@ -359,7 +359,7 @@ static void enqueue_delta_block(Ctx &c, const Qwen35Decode::Plan::Block &b, int 
         step.out32 = x.core;
         step.norm_w = b.dn_norm;
         step.image = c.prep_core();
-        run_gemv(c, zp, &step);
+        run_gemv(c, zp, c.gemv_only ? nullptr : &step);
     } else if (!c.gemv_only) {
         if (c.rec) insg_check(insg_program_add_deltanet(c.rec, state, x.qkv, x.qkv + 2048, x.qkv + 4096, x.a, x.b, x.core));
         else insg_check(insg_deltanet_decode(state, x.qkv, x.qkv + 2048, x.qkv + 4096, x.a, x.b, x.core, c.pdl ? 1 : 0, c.st));
