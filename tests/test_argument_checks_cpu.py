@@ -97,3 +97,15 @@ def test_a_launch_that_does_not_hold_back_the_gated_step_is_refused(change):
     op = gemv_op(**{**dict(prologue="prepared", pdl=2, umma_scratch=SOME, umma_scratch_bytes=1 << 40), **change})
     assert _lib.lib().insg_gemv_fused(C.byref(op), None) == E_ARG
     assert b"pdl = 2" in _lib.lib().insg_last_error()
+
+
+@pytest.mark.parametrize("rows,cols", [(3_000_000, 128), (1_000_000, 12288)])
+def test_nor_where_the_records_do_not_start_on_sixteen_bytes(rows, cols):
+    """Such records stay on mma.sync whatever their number, whose sums of three tokens are the ones that go as two and one."""
+    import torch
+
+    from insignia_b200 import _lib
+
+    if torch.cuda.is_available():
+        pytest.skip("would launch")
+    assert [_lib.lib().insg_mxfp4_gemv_packed(SOME + 8, SOME, SOME, rows, cols, m, None) for m in (1, 2, 3)] == [-2] * 3  # INSG_E_CUDA
