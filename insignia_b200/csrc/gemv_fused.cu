@@ -213,9 +213,12 @@ int insg_gemv_fused(const insg_gemv_op *op, insg_stream_t stream)
 int insg_mxfp4_gemv_packed(const void *packed, const float *x, float *y, int rows, int cols, int M, insg_stream_t stream)
 {
     if (M < 1 || M > 4096) return fail(INSG_E_SHAPE, "gemv_packed: 1 <= M <= 4096");
-    // On tcgen05 (umma_gemv.cu) from 12 million weights on, whatever the tokens, so that a token's bits do not depend on the others.  Smaller matrices
-    // are bound by the host's side of the call, which a launch of clusters makes half a microsecond longer (a call for 8192 x 1024 7.8 us here, 8.1 there;
-    // 4096 x 4096, one to four tokens 8.2, 9.9, 10.3, 10.3 here, 8.1, 8.0, 8.4, 9.1 there).
+    // On tcgen05 (umma_gemv.cu) from 12 million weights on, whatever the tokens, so that a token's bits do not depend on the others.  The line stands where
+    // it was drawn when a launch of clusters took the host half a microsecond more and could not start beside the call ahead.  Since it can, nothing speaks for
+    // mma.sync below it but the bits of these matrices: one to four tokens, calls one behind the other (the host's side bounds the smaller ones) / replayed,
+    //   1024 x 1024 8 to 9 / 4.2, 5.0, 5.8, 6.0 us here, 8 to 10 / 3.0, 3.4, 3.7, 3.7 there; 8192 x 1024 7.8, 8.0, 8.3, 8.5 / 5.3, 5.8, 6.8, 6.9, there 7.8, 7.7, 7.7, 7.9 / 4.2,
+    //   4.3, 4.7, 4.8; 3056 x 4096 8.3, 9.8, 10.3, 10.3 / 6.8, 7.6, 8.4, 8.7, there 7.8, 7.8, 7.7, 7.8 / 4.5, 5.1, 6.1, 6.3; 4096 x 4096, above it, 8.3, 10.2, 10.3, 10.3 / 7.0, 7.7,
+    //   8.5, 8.9, there 7.4, 7.4, 7.3, 7.5 / 4.6, 5.2, 6.2, 6.3.
     const bool on_tensor_cores = packed && x && y && rows > 0 && (rows & 15) == 0 && cols > 0 && (cols & 127) == 0 && cols <= 12288 &&
                                  (long long)rows * cols >= 12ll << 20 && ((reinterpret_cast<uintptr_t>(packed) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
     for (int m0 = 0; m0 < M;) {

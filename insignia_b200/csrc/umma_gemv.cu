@@ -202,6 +202,9 @@ __device__ __forceinline__ void copy8(void *dst, const void *src)
 // its end: z's rows of the in-projection (a tile a head, so that a cluster's four CTAs have their columns' gates at hand) are multiplied here,
 // from the input that the launch before the in-projection left.  The in-projection then has two units a cluster and not three, and the out
 // projection takes digits and not the gated norm: a device-fed token 1010 -> 994 us.
+// One token only: eight warps have one state's 32 columns in registers.  Several sequences have several states, and a verify pass leaves two; their products
+// keep z in the in-projection, and their step (from three sequences on with the digits) is a launch of its own in deltanet.cu.  The gated norm ahead of an out
+// projection (kDGated) is left to them (one and two sequences, verify passes) and, with one token, to the first block, whose input does not come prepared.
 struct DeltaShared {
     float qk[8][2][128]; // per warp: its own copy of the normalised q and k
     float part[2][8][32];
@@ -584,9 +587,9 @@ __global__ void __cluster_dims__(kDCl, 1, 1) __launch_bounds__(kDThreads + ((F &
         if (warp >= 10) {
             // ---- loaders: packed records into what the tensor core reads -------------------------------------------------
             // For plain products on packed records the kernel of gemv_fused.cu dequantises in registers, which bounds it by its ALU pipe; here nothing is
-            // computed on a weight.  Replayed, that kernel -> this one (weights beyond L2): 4096 x 4096, one to four tokens 6.9, 7.6, 8.5, 8.8 -> 5.7, 6.1, 7.3,
-            // 7.8 us; 12352 x 4096 11.3, 12.4, 13.1, 13.4 -> 9.0, 9.4, 10.2, 10.5; 4096 x 12288 12.5, 15.0, 17.3, 19.0 -> 9.4, 10.8, 13.6, 13.6; 248320 x 4096 103,
-            // 118, 117, 118 -> 94, 95, 99, 100 (5.7 TB/s).  With the unswizzled image, whose cells of a row lie 128 and 4096 bytes apart, 191.
+            // computed on a weight.  Replayed, that kernel -> this one (weights beyond L2): 4096 x 4096, one to four tokens 7.0, 7.7, 8.5, 8.9 -> 4.6, 5.2, 6.2,
+            // 6.3 us; 12352 x 4096 11.3, 12.3, 13.0, 13.3 -> 7.2, 7.4, 8.4, 8.6; 4096 x 12288 12.3, 15.0, 17.3, 19.0 -> 7.2, 8.8, 11.6, 11.8; 248320 x 4096, queued, one
+            // and three 104, 119 -> 81, 87.  With the unswizzled image, whose cells of a row lie 128 and 4096 bytes apart, 191.
             // A record holds its rows' 64 bytes one after the other: K-major rows as the tensor core takes them with the 64-byte swizzle, which
             // moves 16-byte cells about within a row.  So every cell goes straight to its place, 512 consecutive bytes of either side a warp.
             // The scale bytes of rows g and g + 8 lie side by side: they come as they are, and the lane that asked for them sorts them when they are there.
